@@ -82,9 +82,9 @@ int sofie_cuda_ctx_h2d(sofie_cuda_ctx *ctx, void *dst_device, const void *src_ho
 /* Pipelined input upload: the input is copied in up to SOFIE_CUDA_MAX_PARTS parts (slices of the batch) on a
  * copy stream of the context, and the launches that read part p are issued after sofie_cuda_ctx_wait_part(p),
  * which makes the context stream wait for that copy only: the model's leading operators work on part p while
- * part p+1 is still crossing PCIe. Copies from pageable host memory fall back to sofie_cuda_ctx_h2d. The
+ * part p+1 is still crossing PCIe. From pageable host memory the call returns when the part has been staged. The
  * caller must not issue the parts of a new inference before the previous one has been fetched
- * (the emitted infer() ends with sofie_cuda_ctx_fetch, which waits). */
+ * (the emitted infer() ends with sofie_cuda_ctx_result_end, which waits). */
 #define SOFIE_CUDA_MAX_PARTS 8
 int sofie_cuda_ctx_h2d_part(sofie_cuda_ctx *ctx, void *dst_device, const void *src_host, size_t bytes, int part);
 int sofie_cuda_ctx_wait_part(sofie_cuda_ctx *ctx, int part);
@@ -96,6 +96,21 @@ int sofie_cuda_ctx_d2h(sofie_cuda_ctx *ctx, void *dst_host, const void *src_devi
  * returns its address; valid until the next fetch. The emitted infer() builds the vector it
  * returns (RModel.cxx:744-801 in the reference) from it in one pass. */
 int sofie_cuda_ctx_fetch(sofie_cuda_ctx *ctx, const void *src_device, size_t bytes, void **host);
+/* The result of one inference brought to the host, whole or part by part (the end of the emitted infer() and inferTo()):
+ * _begin names where it shall go (out_host: pinned memory, which the copies write directly; pageable memory, which the host
+ * fills from the context's pinned buffer; or NULL: anywhere) and its size; _part copies `bytes` bytes at `offset` of it, once
+ * the work enqueued so far is done -- a part that is not the whole runs on a stream of its own, under later parts' kernels and
+ * input copies; _end waits, reports a kernel that gave up as sofie_cuda_ctx_fetch does, and returns the address (out_host, or
+ * pinned memory of the context that stays valid until the next result). At most SOFIE_CUDA_MAX_PARTS parts. */
+int sofie_cuda_ctx_result_begin(sofie_cuda_ctx *ctx, void *out_host, size_t bytes);
+int sofie_cuda_ctx_result_part(sofie_cuda_ctx *ctx, const void *src_device, size_t offset, size_t bytes);
+int sofie_cuda_ctx_result_end(sofie_cuda_ctx *ctx, void **host);
+/* Samples per slice of a batch of `rows` samples whose copies in and out run under the kernels of other slices (`rows` itself:
+ * the batch is better kept whole). in_bytes, out_bytes: per sample; quantum: what a slice has to be a multiple of. */
+size_t sofie_cuda_slice_rows(size_t rows, size_t in_bytes, size_t out_bytes, size_t quantum);
+/* Pinned host memory for results (cudaHostAlloc, portable): sofie_cuda_ctx_result_begin copies straight into it. */
+int sofie_cuda_host_alloc(size_t bytes, void **host);
+int sofie_cuda_host_free(void *host);
 /* A small result tensor placed in mapped pinned host memory: the kernel that computes it writes across PCIe
  * itself and sofie_cuda_ctx_fetch of that pointer only waits for the stream (no device-to-host copy, which
  * costs more than the few kilobytes of a classifier's output are worth). Meant for tensors that no kernel

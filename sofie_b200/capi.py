@@ -100,6 +100,11 @@ SIGNATURES = {
     "sofie_cuda_ctx_h2d": [vp, vp, vp, sz],
     "sofie_cuda_ctx_d2h": [vp, vp, vp, sz],
     "sofie_cuda_ctx_fetch": [vp, vp, sz, C.POINTER(vp)],
+    "sofie_cuda_ctx_result_begin": [vp, vp, sz],
+    "sofie_cuda_ctx_result_part": [vp, vp, sz, sz],
+    "sofie_cuda_ctx_result_end": [vp, C.POINTER(vp)],
+    "sofie_cuda_host_alloc": [sz, C.POINTER(vp)],
+    "sofie_cuda_host_free": [vp],
     "sofie_cuda_ctx_sync": [vp],
     "sofie_cuda_ctx_check": [vp],
     "sofie_cuda_device_check": [C.c_int],
@@ -160,7 +165,8 @@ SIGNATURES = {
     "sofie_cuda_gemm_e4m3_dynamic": [vp, C.POINTER(Fp8GemmDesc), vp, vp, vp, vp, vp, vp],
 }
 STRING_GETTERS = {"sofie_cuda_strerror": [C.c_int], "sofie_cuda_last_error": []}
-SIZE_GETTERS = {"sofie_cuda_mlp_f32_smem": [C.POINTER(MlpDesc)],
+SIZE_GETTERS = {"sofie_cuda_slice_rows": [sz, sz, sz, sz],
+                "sofie_cuda_mlp_f32_smem": [C.POINTER(MlpDesc)],
                 "sofie_cuda_conv_transpose2d_f32_gemm_scratch": [C.POINTER(ConvTranspose2dDesc)]}
 MLP_MAX_LAYERS, MLP_MAX_WIDTH, MLP_MAX_SMEM = 8, 256, 200 * 1024
 

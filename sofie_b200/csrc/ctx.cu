@@ -6,15 +6,10 @@
 // (reference: src/SOFIE_core/src/RModel.cxx:597-604).
 #include "common.cuh"
 #include "contract.cuh"
+#include "host_pool.cuh"
 
-#include <atomic>
-#include <chrono>
-#include <condition_variable>
 #include <cstdlib>
-#include <cstring>
 #include <memory>
-#include <mutex>
-#include <thread>
 #include <utility>
 #include <vector>
 
@@ -89,92 +84,14 @@ uint32_t *device_status_word(cudaStream_t stream)
    return g_status_words[dev];
 }
 
-// Copies between pageable host memory and the pinned staging slots with several threads: one core copies about 12 GB/s,
-// a fifth of what the PCIe link takes. The caller and the helper threads each copy an equal, page-aligned piece of a
-// chunk; copy() returns when all pieces are done. SOFIE_CUDA_COPY_THREADS sets the number of threads (default 4, 1 = the
-// caller alone). A helper spins for a fraction of a millisecond after a chunk (the next chunk of the same transfer comes
-// within that time, and waking a sleeping thread costs as much as its piece of the copy), then sleeps on a condition
-// variable; chunks below 4 MB are copied by the caller alone. The helpers end with the context.
-class HostCopyPool {
-public:
-   explicit HostCopyPool(int helpers) : jobs_(helpers > 0 ? helpers : 0)
-   {
-      for (int i = 0; i < (int)jobs_.size(); i++) threads_.emplace_back([this, i] { work(i); });
-   }
-   ~HostCopyPool()
-   {
-      {
-         std::lock_guard<std::mutex> lock(mu_);
-         stop_.store(true);
-      }
-      wake_.notify_all();
-      for (auto &t : threads_) t.join();
-   }
-   HostCopyPool(const HostCopyPool &) = delete;
-   HostCopyPool &operator=(const HostCopyPool &) = delete;
-
-   void copy(void *dst, const void *src, size_t bytes)
-   {
-      const size_t parts = jobs_.size() + 1;
-      if (parts == 1 || bytes < (size_t(4) << 20)) {
-         std::memcpy(dst, src, bytes);
-         return;
-      }
-      const size_t piece = (((bytes + parts - 1) / parts) + 4095) & ~size_t(4095); // parts x piece >= bytes
-      const size_t mine = piece < bytes ? piece : bytes; // the caller takes the first piece
-      size_t off = mine;
-      for (auto &j : jobs_) {
-         const size_t n = off >= bytes ? 0 : (bytes - off < piece ? bytes - off : piece);
-         j = {static_cast<char *>(dst) + off, static_cast<const char *>(src) + off, n};
-         off += n;
-      }
-      pending_.store((int)jobs_.size(), std::memory_order_relaxed);
-      generation_.fetch_add(1, std::memory_order_release); // publishes the jobs to the helpers that are still spinning
-      {
-         std::lock_guard<std::mutex> lock(mu_);           // ... and to the sleeping ones: no wake-up is lost
-      }
-      wake_.notify_all();
-      std::memcpy(dst, src, mine);
-      // the helpers' pieces are as long as the caller's: they finish at about the same time
-      while (pending_.load(std::memory_order_acquire) != 0) std::this_thread::yield();
-   }
-
-private:
-   struct Job {
-      char *dst;
-      const char *src;
-      size_t bytes;
-   };
-   void work(int index)
-   {
-      unsigned long long seen = 0;
-      for (;;) {
-         const auto t0 = std::chrono::steady_clock::now();
-         while (generation_.load(std::memory_order_acquire) == seen && !stop_.load(std::memory_order_relaxed)) {
-            if (std::chrono::steady_clock::now() - t0 > std::chrono::microseconds(500)) {
-               std::unique_lock<std::mutex> lock(mu_);
-               wake_.wait(lock, [&] { return stop_.load() || generation_.load(std::memory_order_acquire) != seen; });
-               break;
-            }
-            std::this_thread::yield();
-         }
-         if (stop_.load()) return;
-         seen = generation_.load(std::memory_order_acquire);
-         const Job job = jobs_[index];
-         if (job.bytes) std::memcpy(job.dst, job.src, job.bytes);
-         pending_.fetch_sub(1, std::memory_order_release);
-      }
-   }
-   std::vector<Job> jobs_;
-   std::vector<std::thread> threads_;
-   std::mutex mu_;
-   std::condition_variable wake_;
-   std::atomic<unsigned long long> generation_{0};
-   std::atomic<int> pending_{0};
-   std::atomic<bool> stop_{false};
-};
-
 } // namespace sofie
+
+// Pageable host memory crosses PCIe through pinned staging slots: while the copy engine drains some slots the CPU fills
+// the next, so the host's copy and the DMA overlap instead of alternating. The ring is small enough to stay in the host's
+// last-level cache: the filled slot is read by the DMA from there and the host's memory sees the source's bytes alone.
+constexpr int kStagingSlots = 8;
+constexpr size_t kStagingSlot = size_t(2) << 20;
+constexpr size_t kStagingBytes = kStagingSlots * kStagingSlot;
 
 struct sofie_cuda_ctx {
    int device = 0;
@@ -182,13 +99,29 @@ struct sofie_cuda_ctx {
    char *arena = nullptr;
    size_t arena_bytes = 0;
    std::vector<void *> owned;
-   void *staging = nullptr; // pinned: kStagingSlots slots of kStagingSlot bytes, used as a ring
-   size_t staging_bytes = 0;
-   cudaEvent_t staging_event[4] = {}; // the copy out of (h2d) or into (d2h) a slot has completed
-   bool staging_busy[4] = {};         // a copy that read the slot may still be in flight
-   std::unique_ptr<sofie::HostCopyPool> copy_pool; // made with the staging ring
-   void *result = nullptr;  // pinned, grown on demand: where sofie_cuda_ctx_fetch lands device results
+   char *staging = nullptr; // pinned ring, made on first use
+   struct Slot {
+      cudaEvent_t event = nullptr;   // the copy that read the slot has completed, when `recorded`
+      cudaStream_t stream = nullptr; // the stream that copy was issued on
+      bool busy = false, recorded = false;
+   } slots[kStagingSlots];
+   int next_slot = 0;
+   std::unique_ptr<sofie::HostPool> host_pool; // made on first use
+   void *result = nullptr;  // pinned, grown on demand: where results land that were not given a pinned place of their own
    size_t result_bytes = 0;
+   // the result of one inference on its way to the host, between result_begin and result_end
+   struct Landing {
+      bool open = false;
+      char *out = nullptr;    // where the caller wants it (nullptr: anywhere)
+      char *land = nullptr;   // pinned memory the copies write: out, or `result`
+      const char *mapped = nullptr; // the kernels wrote it to host memory themselves
+      size_t bytes = 0;
+      int parts = 0;
+      size_t offset[SOFIE_CUDA_MAX_PARTS], count[SOFIE_CUDA_MAX_PARTS];
+   } landing;
+   cudaStream_t result_stream = nullptr; // results that are copied part by part, under the kernels of later parts
+   cudaEvent_t ready_event = nullptr;    // a part's kernels are done
+   cudaEvent_t landed_event[SOFIE_CUDA_MAX_PARTS] = {};
    cudaGraph_t graph = nullptr;
    cudaGraphExec_t graph_exec = nullptr;
    bool capturing = false;
@@ -235,11 +168,6 @@ struct DeviceGuard {
       if (prev >= 0) cudaSetDevice(prev);
    }
 };
-// Pageable host memory crosses PCIe through pinned staging slots: while the copy engine drains one slot the CPU fills
-// the next, so the host memcpy and the DMA overlap instead of alternating.
-constexpr int kStagingSlots = 4;
-constexpr size_t kStagingSlot = size_t(8) << 20;
-constexpr size_t kStagingBytes = kStagingSlots * kStagingSlot;
 } // namespace
 
 extern "C" {
@@ -340,6 +268,7 @@ int sofie_cuda_ctx_destroy(sofie_cuda_ctx *ctx)
    // nothing of this context may still be running or copying when its memory goes away
    cudaStreamSynchronize(ctx->stream);
    if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
+   if (ctx->result_stream) cudaStreamSynchronize(ctx->result_stream);
    unregister_stream_status(ctx->stream);
    if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
    if (ctx->graph) cudaGraphDestroy(ctx->graph);
@@ -351,8 +280,12 @@ int sofie_cuda_ctx_destroy(sofie_cuda_ctx *ctx)
    splitk_scratch_release(ctx->device, ctx->stream);
    if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
    if (ctx->status) cudaFreeHost(ctx->status);
-   for (cudaEvent_t e : ctx->staging_event)
+   if (ctx->result_stream) cudaStreamDestroy(ctx->result_stream);
+   for (auto &s : ctx->slots)
+      if (s.event) cudaEventDestroy(s.event);
+   for (cudaEvent_t e : ctx->landed_event)
       if (e) cudaEventDestroy(e);
+   if (ctx->ready_event) cudaEventDestroy(ctx->ready_event);
    for (cudaEvent_t e : ctx->marks)
       if (e) cudaEventDestroy(e);
    for (cudaEvent_t e : ctx->part_event)
@@ -415,20 +348,52 @@ int sofie_cuda_ctx_upload(sofie_cuda_ctx *ctx, const void *host, size_t bytes, v
    return SOFIE_CUDA_OK;
 }
 
-static int ensure_staging(sofie_cuda_ctx *ctx)
+static int ensure_pool(sofie_cuda_ctx *ctx)
 {
-   if (ctx->staging) return SOFIE_CUDA_OK;
-   SOFIE_CUDA_TRY(cudaMallocHost(&ctx->staging, kStagingBytes));
-   ctx->staging_bytes = kStagingBytes;
-   for (auto &e : ctx->staging_event) SOFIE_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-   int threads = 4;
-   if (const char *e = std::getenv("SOFIE_CUDA_COPY_THREADS")) threads = std::atoi(e);
+   if (ctx->host_pool) return SOFIE_CUDA_OK;
+   // eight threads keep the link busy from pageable memory (110 GB/s into the ring; four 54 GB/s, with nothing to spare);
+   // half the cores of a smaller host
    const int cores = (int)std::thread::hardware_concurrency();
+   int threads = cores / 2 < 8 ? cores / 2 : 8;
+   if (const char *e = std::getenv("SOFIE_CUDA_COPY_THREADS")) threads = std::atoi(e);
    if (cores > 0 && threads > cores) threads = cores;
    if (threads < 1) threads = 1;
    if (threads > 16) threads = 16;
-   ctx->copy_pool.reset(new HostCopyPool(threads - 1));
+   ctx->host_pool.reset(new HostPool(threads - 1));
    return SOFIE_CUDA_OK;
+}
+
+static int ensure_staging(sofie_cuda_ctx *ctx)
+{
+   int rc = ensure_pool(ctx);
+   if (rc || ctx->staging) return rc;
+   void *p = nullptr;
+   SOFIE_CUDA_TRY(cudaMallocHost(&p, kStagingBytes));
+   ctx->staging = static_cast<char *>(p);
+   for (auto &s : ctx->slots) SOFIE_CUDA_TRY(cudaEventCreateWithFlags(&s.event, cudaEventDisableTiming));
+   return SOFIE_CUDA_OK;
+}
+
+// The next slot of the ring, once the copy that last read it is done.
+static int take_slot(sofie_cuda_ctx *ctx, sofie_cuda_ctx::Slot **slot, char **mem)
+{
+   const int i = ctx->next_slot;
+   ctx->next_slot = (i + 1) % kStagingSlots;
+   sofie_cuda_ctx::Slot &s = ctx->slots[i];
+   if (s.busy) {
+      if (s.recorded) SOFIE_CUDA_TRY(cudaEventSynchronize(s.event));
+      else SOFIE_CUDA_TRY(cudaStreamSynchronize(s.stream));
+      s.busy = false;
+   }
+   *slot = &s;
+   *mem = ctx->staging + (size_t)i * kStagingSlot;
+   return SOFIE_CUDA_OK;
+}
+
+// every copy of this context has completed (its streams were waited for): all slots are free
+static void slots_free(sofie_cuda_ctx *ctx)
+{
+   for (auto &s : ctx->slots) s.busy = false;
 }
 
 // Pageable host memory is staged through one pinned buffer in chunks; memory the caller already
@@ -443,6 +408,32 @@ static bool is_pinned(const void *p)
    return attr.type == cudaMemoryTypeHost;
 }
 
+// Pageable memory to the device on `stream`; returns when the last piece has been staged.
+static int stage_in(sofie_cuda_ctx *ctx, void *dst, const void *src, size_t bytes, cudaStream_t stream)
+{
+   int rc = ensure_staging(ctx);
+   if (rc) return rc;
+   // pieces small enough that the DMA of the first starts early, large enough for its fixed cost (about 3 us of host time)
+   size_t piece = bytes / 4;
+   piece = piece < (size_t(128) << 10) ? (size_t(128) << 10) : (piece > kStagingSlot ? kStagingSlot : ((piece + 4095) & ~size_t(4095)));
+   // an event per slot only where the ring can come round before the stream is waited for anyway
+   const bool record = bytes > (size_t(1) << 20);
+   for (size_t done = 0; done < bytes;) {
+      const size_t n = bytes - done < piece ? bytes - done : piece;
+      sofie_cuda_ctx::Slot *slot = nullptr;
+      char *mem = nullptr;
+      if ((rc = take_slot(ctx, &slot, &mem))) return rc;
+      ctx->host_pool->copy(mem, static_cast<const char *>(src) + done, n);
+      SOFIE_CUDA_TRY(cudaMemcpyAsync(static_cast<char *>(dst) + done, mem, n, cudaMemcpyHostToDevice, stream));
+      slot->busy = true;
+      slot->stream = stream;
+      slot->recorded = record;
+      if (record) SOFIE_CUDA_TRY(cudaEventRecord(slot->event, stream));
+      done += n;
+   }
+   return SOFIE_CUDA_OK;
+}
+
 int sofie_cuda_ctx_h2d(sofie_cuda_ctx *ctx, void *dst, const void *src, size_t bytes)
 {
    SOFIE_REQUIRE(ctx && dst && src, "NULL argument");
@@ -452,29 +443,14 @@ int sofie_cuda_ctx_h2d(sofie_cuda_ctx *ctx, void *dst, const void *src, size_t b
       SOFIE_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
       return SOFIE_CUDA_OK;
    }
-   int rc = ensure_staging(ctx);
-   if (rc) return rc;
-   size_t done = 0;
-   bool used[kStagingSlots] = {};
-   for (int slot = 0; done < bytes; slot = (slot + 1) % kStagingSlots) {
-      const size_t chunk = bytes - done < kStagingSlot ? bytes - done : kStagingSlot;
-      char *stage = static_cast<char *>(ctx->staging) + (size_t)slot * kStagingSlot;
-      // a slot is refilled only after the copy that last read it has finished (also a copy of an earlier call)
-      if (used[slot] || ctx->staging_busy[slot]) SOFIE_CUDA_TRY(cudaEventSynchronize(ctx->staging_event[slot]));
-      ctx->copy_pool->copy(stage, static_cast<const char *>(src) + done, chunk);
-      SOFIE_CUDA_TRY(cudaMemcpyAsync(static_cast<char *>(dst) + done, stage, chunk, cudaMemcpyHostToDevice, ctx->stream));
-      SOFIE_CUDA_TRY(cudaEventRecord(ctx->staging_event[slot], ctx->stream));
-      used[slot] = ctx->staging_busy[slot] = true;
-      done += chunk;
-   }
-   return SOFIE_CUDA_OK;
+   return stage_in(ctx, dst, src, bytes, ctx->stream);
 }
 
 int sofie_cuda_selftest_host_copy(void *dst, const void *src, size_t bytes, size_t chunk, int threads, int repeats)
 {
    SOFIE_REQUIRE((dst && src) || bytes == 0, "NULL buffer");
    SOFIE_REQUIRE(chunk > 0 && threads >= 1 && threads <= 16 && repeats >= 1, "bad chunk size, thread count or repeat count");
-   HostCopyPool pool(threads - 1);
+   HostPool pool(threads - 1);
    for (int r = 0; r < repeats; r++)
       for (size_t done = 0; done < bytes; done += chunk)
          pool.copy(static_cast<char *>(dst) + done, static_cast<const char *>(src) + done, bytes - done < chunk ? bytes - done : chunk);
@@ -488,17 +464,21 @@ int sofie_cuda_ctx_h2d_part(sofie_cuda_ctx *ctx, void *dst, const void *src, siz
    SOFIE_REQUIRE(!ctx->capturing, "input copies are not part of the captured graph");
    DeviceGuard guard(ctx->device);
    if (!ctx->part_event[part]) SOFIE_CUDA_TRY(cudaEventCreateWithFlags(&ctx->part_event[part], cudaEventDisableTiming));
-   if (!is_pinned(src)) {
-      // pageable memory goes through the staging ring on the compute stream; the call returns when the part has been
-      // staged, so the kernels the caller launches next for this part run while the host stages the following one.
-      // The event only keeps sofie_cuda_ctx_wait_part valid
-      int rc = sofie_cuda_ctx_h2d(ctx, dst, src, bytes);
-      if (rc) return rc;
-      SOFIE_CUDA_TRY(cudaEventRecord(ctx->part_event[part], ctx->stream));
-      return SOFIE_CUDA_OK;
-   }
    if (!ctx->copy_stream) SOFIE_CUDA_TRY(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
-   SOFIE_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->copy_stream));
+   if (part == 0) {
+      // kernels of an earlier pass that was not waited for may still read what this copy overwrites
+      if (!ctx->ready_event) SOFIE_CUDA_TRY(cudaEventCreateWithFlags(&ctx->ready_event, cudaEventDisableTiming));
+      SOFIE_CUDA_TRY(cudaEventRecord(ctx->ready_event, ctx->stream));
+      SOFIE_CUDA_TRY(cudaStreamWaitEvent(ctx->copy_stream, ctx->ready_event, 0));
+   }
+   // pinned memory is copied by the DMA engine alone; from pageable memory the call returns when the part has been staged, so
+   // the kernels the caller launches next for this part run while the host stages the following one
+   if (is_pinned(src)) {
+      SOFIE_CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->copy_stream));
+   } else {
+      int rc = stage_in(ctx, dst, src, bytes, ctx->copy_stream);
+      if (rc) return rc;
+   }
    SOFIE_CUDA_TRY(cudaEventRecord(ctx->part_event[part], ctx->copy_stream));
    return SOFIE_CUDA_OK;
 }
@@ -525,35 +505,31 @@ int sofie_cuda_ctx_d2h(sofie_cuda_ctx *ctx, void *dst, const void *src, size_t b
    }
    int rc = ensure_staging(ctx);
    if (rc) return rc;
-   // every input copy that used the slots has to be over before results land in them
+   // every copy that used the slots has to be over before results land in them
    SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-   for (auto &b : ctx->staging_busy) b = false;
+   if (ctx->copy_stream) SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->copy_stream));
+   slots_free(ctx);
    // the copies of all slots are queued first, then each is copied out as soon as it has arrived: the host memcpy of
    // one slot overlaps the DMA into the next
    size_t done = 0;
    while (done < bytes) {
       const size_t round = bytes - done < kStagingBytes ? bytes - done : kStagingBytes;
-      int slots = 0;
-      for (size_t off = 0; off < round; off += kStagingSlot, slots++) {
+      int n = 0;
+      for (size_t off = 0; off < round; off += kStagingSlot, n++) {
          const size_t chunk = round - off < kStagingSlot ? round - off : kStagingSlot;
-         SOFIE_CUDA_TRY(cudaMemcpyAsync(static_cast<char *>(ctx->staging) + off, static_cast<const char *>(src) + done + off, chunk,
-                                        cudaMemcpyDeviceToHost, ctx->stream));
-         SOFIE_CUDA_TRY(cudaEventRecord(ctx->staging_event[slots], ctx->stream));
+         SOFIE_CUDA_TRY(cudaMemcpyAsync(ctx->staging + off, static_cast<const char *>(src) + done + off, chunk, cudaMemcpyDeviceToHost, ctx->stream));
+         SOFIE_CUDA_TRY(cudaEventRecord(ctx->slots[n].event, ctx->stream));
       }
-      for (int slot = 0; slot < slots; slot++) {
-         const size_t off = (size_t)slot * kStagingSlot, chunk = round - off < kStagingSlot ? round - off : kStagingSlot;
-         SOFIE_CUDA_TRY(cudaEventSynchronize(ctx->staging_event[slot]));
-         ctx->copy_pool->copy(static_cast<char *>(dst) + done + off, static_cast<char *>(ctx->staging) + off, chunk);
+      for (int i = 0; i < n; i++) {
+         const size_t off = (size_t)i * kStagingSlot, chunk = round - off < kStagingSlot ? round - off : kStagingSlot;
+         SOFIE_CUDA_TRY(cudaEventSynchronize(ctx->slots[i].event));
+         ctx->host_pool->copy(static_cast<char *>(dst) + done + off, ctx->staging + off, chunk);
       }
       done += round;
    }
    return SOFIE_CUDA_OK;
 }
 
-// Device -> pinned host buffer owned by the context, at full link speed; the caller builds its
-// result (the vector Session::infer returns) from the returned pointer in one pass, instead of
-// zero-filling a vector first and then staging the copy through it. The pointer stays valid until
-// the next fetch on this context.
 int sofie_cuda_ctx_host_output(sofie_cuda_ctx *ctx, size_t bytes, void **dptr)
 {
    SOFIE_REQUIRE(ctx && dptr, "NULL argument");
@@ -573,6 +549,130 @@ int sofie_cuda_ctx_host_output(sofie_cuda_ctx *ctx, size_t bytes, void **dptr)
    return SOFIE_CUDA_OK;
 }
 
+static int ensure_result(sofie_cuda_ctx *ctx, size_t bytes)
+{
+   if (bytes <= ctx->result_bytes) return SOFIE_CUDA_OK;
+   if (ctx->result) cudaFreeHost(ctx->result);
+   ctx->result = nullptr;
+   ctx->result_bytes = 0;
+   SOFIE_CUDA_TRY(cudaMallocHost(&ctx->result, bytes));
+   ctx->result_bytes = bytes;
+   return SOFIE_CUDA_OK;
+}
+
+int sofie_cuda_ctx_result_begin(sofie_cuda_ctx *ctx, void *out_host, size_t bytes)
+{
+   SOFIE_REQUIRE(ctx != nullptr, "NULL context");
+   SOFIE_REQUIRE(!ctx->capturing, "result copies are not part of the captured graph");
+   ctx->landing = {};
+   ctx->landing.open = true;
+   ctx->landing.out = static_cast<char *>(out_host);
+   ctx->landing.bytes = bytes;
+   return SOFIE_CUDA_OK;
+}
+
+int sofie_cuda_ctx_result_part(sofie_cuda_ctx *ctx, const void *src, size_t offset, size_t bytes)
+{
+   SOFIE_REQUIRE(ctx && src, "NULL argument");
+   auto &l = ctx->landing;
+   SOFIE_REQUIRE(l.open && offset <= l.bytes && bytes <= l.bytes - offset, "part [%zu, +%zu) of a result of %zu bytes", offset, bytes, l.bytes);
+   SOFIE_REQUIRE(l.parts < SOFIE_CUDA_MAX_PARTS, "more than %d parts", SOFIE_CUDA_MAX_PARTS);
+   const char *s8 = static_cast<const char *>(src);
+   for (auto &h : ctx->host_outputs)
+      if (s8 >= h.first && s8 + bytes <= h.first + h.second) {
+         l.mapped = s8 - offset; // the kernels write it to host memory themselves
+         return SOFIE_CUDA_OK;
+      }
+   if (bytes == 0) return SOFIE_CUDA_OK;
+   DeviceGuard guard(ctx->device);
+   if (!l.land) {
+      if (l.out && is_pinned(l.out)) {
+         l.land = l.out;
+      } else {
+         int rc = ensure_result(ctx, l.bytes);
+         if (rc) return rc;
+         l.land = static_cast<char *>(ctx->result);
+      }
+   }
+   cudaStream_t stream = ctx->stream;
+   if (bytes != l.bytes) {
+      // one part of several: on a stream of its own, so that the copy out runs beside the later parts' kernels and copies in
+      if (!ctx->result_stream) SOFIE_CUDA_TRY(cudaStreamCreateWithFlags(&ctx->result_stream, cudaStreamNonBlocking));
+      if (!ctx->ready_event) SOFIE_CUDA_TRY(cudaEventCreateWithFlags(&ctx->ready_event, cudaEventDisableTiming));
+      SOFIE_CUDA_TRY(cudaEventRecord(ctx->ready_event, ctx->stream));
+      SOFIE_CUDA_TRY(cudaStreamWaitEvent(ctx->result_stream, ctx->ready_event, 0));
+      stream = ctx->result_stream;
+   }
+   SOFIE_CUDA_TRY(cudaMemcpyAsync(l.land + offset, src, bytes, cudaMemcpyDeviceToHost, stream));
+   if (l.out && l.land != l.out && bytes != l.bytes) {
+      cudaEvent_t &e = ctx->landed_event[l.parts];
+      if (!e) SOFIE_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      SOFIE_CUDA_TRY(cudaEventRecord(e, stream));
+   }
+   l.offset[l.parts] = offset;
+   l.count[l.parts++] = bytes;
+   return SOFIE_CUDA_OK;
+}
+
+int sofie_cuda_ctx_result_end(sofie_cuda_ctx *ctx, void **host)
+{
+   SOFIE_REQUIRE(ctx && host, "NULL argument");
+   auto &l = ctx->landing;
+   SOFIE_REQUIRE(l.open, "no result was begun");
+   l.open = false;
+   DeviceGuard guard(ctx->device);
+   const bool carry = l.out && l.land && l.land != l.out; // the caller's memory is pageable: the host carries the bytes over
+   if (carry) {
+      int rc = ensure_pool(ctx);
+      if (rc) return rc;
+      if (l.parts > 1)
+         for (int i = 0; i < l.parts; i++) { // each part as soon as it has landed, under the copies of the later ones
+            SOFIE_CUDA_TRY(cudaEventSynchronize(ctx->landed_event[i]));
+            ctx->host_pool->copy(l.out + l.offset[i], l.land + l.offset[i], l.count[i]);
+         }
+   }
+   SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+   if (ctx->result_stream && l.parts > 1) SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->result_stream));
+   slots_free(ctx); // the stream has waited for every part that was copied in
+   if (carry && l.parts == 1) ctx->host_pool->copy(l.out, l.land, l.bytes);
+   if (l.mapped && l.out) std::memcpy(l.out, l.mapped, l.bytes);
+   *host = l.out ? l.out : (l.mapped ? const_cast<char *>(l.mapped) : l.land);
+   return report_status(ctx);
+}
+
+size_t sofie_cuda_slice_rows(size_t rows, size_t in_bytes, size_t out_bytes, size_t quantum)
+{
+   static const int forced = [] { const char *e = std::getenv("SOFIE_CUDA_SLICES"); return e ? std::atoi(e) : 0; }();
+   if (quantum == 0) quantum = 1;
+   const size_t total = rows * (in_bytes > out_bytes ? in_bytes : out_bytes);
+   // A slice costs its launches and two copies' fixed cost again (about 10 us each): from 4 MB of traffic on, in slices of at
+   // least 2 MB (38 us of PCIe)
+   size_t parts = forced > 0 ? (size_t)forced : (total < (size_t(4) << 20) ? 1 : total >> 21);
+   if (parts > 8) parts = 8;
+   if (parts <= 1) return rows;
+   const size_t per = (rows + parts - 1) / parts;
+   return (per + quantum - 1) / quantum * quantum;
+}
+
+int sofie_cuda_host_alloc(size_t bytes, void **host)
+{
+   SOFIE_REQUIRE(host && bytes > 0, "NULL argument or no bytes");
+   void *p = nullptr;
+   SOFIE_CUDA_TRY(cudaHostAlloc(&p, bytes, cudaHostAllocPortable));
+   *host = p;
+   return SOFIE_CUDA_OK;
+}
+
+int sofie_cuda_host_free(void *host)
+{
+   if (host) SOFIE_CUDA_TRY(cudaFreeHost(host));
+   return SOFIE_CUDA_OK;
+}
+
+// Device -> pinned host buffer owned by the context, at full link speed; the caller builds its
+// result (the vector Session::infer returns) from the returned pointer in one pass, instead of
+// zero-filling a vector first and then staging the copy through it. The pointer stays valid until
+// the next fetch on this context.
 int sofie_cuda_ctx_fetch(sofie_cuda_ctx *ctx, const void *src, size_t bytes, void **host)
 {
    SOFIE_REQUIRE(ctx && src && host, "NULL argument");
@@ -587,13 +687,8 @@ int sofie_cuda_ctx_fetch(sofie_cuda_ctx *ctx, const void *src, size_t bytes, voi
          return report_status(ctx);
       }
    }
-   if (bytes > ctx->result_bytes) {
-      if (ctx->result) cudaFreeHost(ctx->result);
-      ctx->result = nullptr;
-      ctx->result_bytes = 0;
-      SOFIE_CUDA_TRY(cudaMallocHost(&ctx->result, bytes));
-      ctx->result_bytes = bytes;
-   }
+   int rc = ensure_result(ctx, bytes);
+   if (rc) return rc;
    if (bytes) SOFIE_CUDA_TRY(cudaMemcpyAsync(ctx->result, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
    SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
    *host = ctx->result;

@@ -1,0 +1,144 @@
+// Helper threads of one context for the host's share of a transfer: moving bytes between the caller's pageable memory and
+// pinned memory. One core moves 14 GB/s on the Xeon hosts measured, a quarter of what the PCIe link takes (55 GB/s each way);
+// four reach 54 GB/s and eight 110 GB/s as long as the pinned side stays in the last-level cache.
+#pragma once
+
+#include <atomic>
+#include <chrono>
+#include <condition_variable>
+#include <cstring>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+namespace sofie {
+
+// run() cuts a job into numbered pieces that the caller and the helpers claim one after the other, so a helper that is still
+// asleep or was descheduled delays nothing but the piece it holds. A claim carries the job's generation: a helper that comes
+// late finds another generation (or no piece left) and touches nothing of the next job. Helpers spin for half a millisecond
+// after a job (the next one of the same transfer comes within that time, and waking a sleeping thread costs tens of
+// microseconds), then sleep on a condition variable. They end with the pool.
+class HostPool {
+public:
+   using PieceFn = void (*)(void *arg, size_t piece);
+   explicit HostPool(int helpers)
+   {
+      for (int i = 0; i < helpers; i++) threads_.emplace_back([this] { helper(); });
+   }
+   ~HostPool()
+   {
+      {
+         std::lock_guard<std::mutex> lock(mu_);
+         stop_.store(true);
+      }
+      wake_.notify_all();
+      for (auto &t : threads_) t.join();
+   }
+   HostPool(const HostPool &) = delete;
+   HostPool &operator=(const HostPool &) = delete;
+
+   // fn(arg, i) for every i below `pieces` (at most 2^31), in any order; returns when all are done. One caller at a time.
+   void run(PieceFn fn, void *arg, size_t pieces)
+   {
+      if (threads_.empty() || pieces <= 1) {
+         for (size_t i = 0; i < pieces; i++) fn(arg, i);
+         return;
+      }
+      // a helper that still holds the last job's ticket must not claim with the new job's piece count: the ticket is closed
+      // (odd generation, no piece can be claimed) while the job's fields change
+      ticket_.store(((uint64_t)++generation_ << 32) | 0xFFFFFFFFu, std::memory_order_seq_cst);
+      std::atomic_thread_fence(std::memory_order_seq_cst);
+      fn_ = fn, arg_ = arg;
+      pieces_.store((uint32_t)pieces, std::memory_order_relaxed);
+      done_.store(0, std::memory_order_relaxed);
+      const uint32_t gen = ++generation_;
+      ticket_.store((uint64_t)gen << 32, std::memory_order_seq_cst);
+      if (sleepers_.load(std::memory_order_seq_cst) > 0) {
+         std::lock_guard<std::mutex> lock(mu_);
+         wake_.notify_all();
+      }
+      claim(gen);
+      while (done_.load(std::memory_order_acquire) != (uint32_t)pieces) relax();
+   }
+
+   // A copy below kAloneBytes is the caller's alone: two threads' hand-over costs as much as it saves.
+   void copy(void *dst, const void *src, size_t bytes)
+   {
+      if (threads_.empty() || bytes < kAloneBytes) {
+         std::memcpy(dst, src, bytes);
+         return;
+      }
+      CopyJob job{static_cast<char *>(dst), static_cast<const char *>(src), bytes, kPieceBytes};
+      // enough pieces that every thread gets several, each still long enough for the prefetchers
+      while (job.piece > size_t(32) << 10 && bytes / job.piece < 3 * (threads_.size() + 1)) job.piece >>= 1;
+      run(copy_piece, &job, (bytes + job.piece - 1) / job.piece);
+   }
+
+   static constexpr size_t kAloneBytes = size_t(192) << 10;
+   static constexpr size_t kPieceBytes = size_t(256) << 10;
+
+private:
+   struct CopyJob {
+      char *dst;
+      const char *src;
+      size_t bytes, piece;
+   };
+   static void copy_piece(void *arg, size_t i)
+   {
+      const CopyJob &j = *static_cast<CopyJob *>(arg);
+      const size_t off = i * j.piece;
+      std::memcpy(j.dst + off, j.src + off, j.bytes - off < j.piece ? j.bytes - off : j.piece);
+   }
+   static void relax()
+   {
+#if defined(__x86_64__)
+      __builtin_ia32_pause();
+#else
+      std::this_thread::yield();
+#endif
+   }
+   // takes pieces of job `gen` until none is left; the job's fields are stable while one of its pieces is not done
+   void claim(uint32_t gen)
+   {
+      uint64_t t = ticket_.load(std::memory_order_acquire);
+      for (;;) {
+         if ((uint32_t)(t >> 32) != gen || (uint32_t)t >= pieces_.load(std::memory_order_relaxed)) return;
+         if (!ticket_.compare_exchange_weak(t, t + 1, std::memory_order_acq_rel, std::memory_order_acquire)) continue;
+         fn_(arg_, (uint32_t)t);
+         done_.fetch_add(1, std::memory_order_release);
+         t = ticket_.load(std::memory_order_acquire);
+      }
+   }
+   void helper()
+   {
+      uint32_t seen = 0;
+      auto news = [&] { return stop_.load(std::memory_order_relaxed) || (uint32_t)(ticket_.load(std::memory_order_seq_cst) >> 32) != seen; };
+      for (;;) {
+         const auto t0 = std::chrono::steady_clock::now();
+         while (!news()) {
+            for (int i = 0; i < 32 && !news(); i++) relax();
+            if (std::chrono::steady_clock::now() - t0 < std::chrono::microseconds(500)) continue;
+            std::unique_lock<std::mutex> lock(mu_);
+            sleepers_.fetch_add(1, std::memory_order_seq_cst); // before the last look: run() reads it after it has published
+            wake_.wait(lock, news);
+            sleepers_.fetch_sub(1, std::memory_order_relaxed);
+         }
+         if (stop_.load()) return;
+         seen = (uint32_t)(ticket_.load(std::memory_order_acquire) >> 32);
+         claim(seen);
+      }
+   }
+   std::vector<std::thread> threads_;
+   std::mutex mu_;
+   std::condition_variable wake_;
+   PieceFn fn_ = nullptr;
+   void *arg_ = nullptr;
+   std::atomic<uint32_t> pieces_{0};
+   uint32_t generation_ = 0;
+   std::atomic<uint64_t> ticket_{0}; // generation of the job in the upper half, its next piece in the lower
+   std::atomic<uint32_t> done_{0};
+   std::atomic<int> sleepers_{0};
+   std::atomic<bool> stop_{false};
+};
+
+} // namespace sofie

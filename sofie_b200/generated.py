@@ -3,8 +3,8 @@
     ONNX file --RModelParser_ONNX::Parse / RModel::Generate / OutputGenerated-->  <name>.hxx + <name>.dat
     <name>.hxx --g++ (any C++17 compiler), -lSOFIE_cuda-->  shared object with the emitted Session
 
-The emitted `Session(std::string)` / `std::vector<float> infer(float*)` are reached from Python through
-three extern "C" trampolines compiled next to the header. Used by the tests and by the end-to-end leg
+The emitted `Session(std::string)` / `infer(float*)` (as its twin `inferTo`, which writes into the caller's memory) are
+reached from Python through extern "C" trampolines compiled next to the header. Used by the tests and by the end-to-end leg
 of the benchmark; nothing here computes anything itself.
 """
 from __future__ import annotations
@@ -17,11 +17,13 @@ import os
 import shutil
 import subprocess
 import tempfile
+import threading
+import weakref
 from pathlib import Path
 
 import numpy as np
 
-from . import _build
+from . import _build, capi
 
 ROOT = Path(__file__).resolve().parent.parent
 HOST = Path(__file__).resolve().parent / "host"
@@ -39,10 +41,9 @@ extern "C" void *sofie_session_create(const char *dat, char *err, int errlen) {{
 }}
 extern "C" long sofie_session_infer(void *s, {in_type} **xs, {out_type} *y, long ny, char *err, int errlen) {{
    try {{
-      auto out = static_cast<Session *>(s)->infer({args});
-      if ((long)out.size() > ny) {{ set_err(err, errlen, "output buffer too small"); return -(long)out.size(); }}
-      std::memcpy(y, out.data(), out.size() * sizeof({out_type}));
-      return (long)out.size();
+      const long n = (long)static_cast<Session *>(s)->inferTo({args}y, (size_t)ny);
+      if (n > ny) {{ set_err(err, errlen, "output buffer too small"); return -n; }}
+      return n;
    }} catch (const std::exception &e) {{ set_err(err, errlen, e.what()); return -1; }}
 }}
 extern "C" void sofie_session_destroy(void *s) {{ delete static_cast<Session *>(s); }}
@@ -107,10 +108,9 @@ extern "C" void *sofie_session_create_bs(const char *dat, long max_batch, char *
 }}
 extern "C" long sofie_session_infer_bs(void *s, long bs, {in_type} **xs, {out_type} *y, long ny, char *err, int errlen) {{
    try {{
-      auto out = static_cast<Session *>(s)->infer((size_t)bs, {args});
-      if ((long)out.size() > ny) {{ set_err(err, errlen, "output buffer too small"); return -(long)out.size(); }}
-      std::memcpy(y, out.data(), out.size() * sizeof({out_type}));
-      return (long)out.size();
+      const long n = (long)static_cast<Session *>(s)->inferTo((size_t)bs, {args}y, (size_t)ny);
+      if (n > ny) {{ set_err(err, errlen, "output buffer too small"); return -n; }}
+      return n;
    }} catch (const std::exception &e) {{ set_err(err, errlen, e.what()); return -1; }}
 }}
 extern "C" void sofie_session_destroy(void *s) {{ delete static_cast<Session *>(s); }}
@@ -187,7 +187,7 @@ def compile_session(hxx: Path, name: str, in_type="float", out_type="float") -> 
         if fresh():
             return so
         src = hxx.with_name(hxx.stem + "_trampoline.cxx")
-        args = ", ".join(f"xs[{i}]" for i in range(count_inputs(hxx)))
+        args = "".join(f"xs[{i}], " for i in range(count_inputs(hxx)))
         template = TRAMPOLINE_DYN if is_dynamic(hxx) else TRAMPOLINE
         src.write_text(template.format(header=hxx.name, name=name, in_type=in_type, out_type=out_type, args=args))
         tmp = so.with_name(f".{so.name}.{os.getpid()}.tmp")
@@ -199,6 +199,67 @@ def compile_session(hxx: Path, name: str, in_type="float", out_type="float") -> 
             raise RuntimeError(f"compiling the emitted header failed:\n{r.stdout}")
         os.replace(tmp, so)
     return so
+
+
+class _PinnedBuffer:
+    """Pinned host memory for one result; freed when neither the Session nor an array over it is left."""
+
+    def __init__(self, nbytes: int):
+        self.nbytes = nbytes
+        self.ptr = C.c_void_p()
+        capi.call("sofie_cuda_host_alloc", nbytes, C.byref(self.ptr))
+        self.free = capi.load().sofie_cuda_host_free
+        self.array = None          # weak reference to the array handed out over it; views of that array keep it alive
+
+    def __del__(self):
+        if getattr(self, "free", None) is not None and self.ptr:
+            self.free(self.ptr)
+
+    def lend(self, n: int, dtype) -> np.ndarray:
+        mem = (C.c_char * (n * dtype.itemsize)).from_address(self.ptr.value)
+        mem.owner = self
+        a = np.frombuffer(mem, dtype, n)
+        self.array = weakref.ref(a)
+        return a
+
+    def idle(self) -> bool:
+        return self.array is None or self.array() is None
+
+
+class _ResultArrays:
+    """The arrays infer() returns. From kPinnedFrom bytes on they lie in pinned memory, which the device copies the result into
+    directly: a fresh np.empty of that size is memory the kernel hands out page by page on first touch (measured: 2 GB/s, against
+    55 GB/s of the copy itself), and the result would have to be carried over from pinned memory besides. A buffer comes back when
+    the array over it (and every view of it) is gone, and is used again; a program that keeps more than kBuffers results of one
+    Session gets ordinary arrays from then on, so pinned memory stays bounded by kBuffers results per Session."""
+    kPinnedFrom, kBuffers = 128 << 10, 3
+
+    def __init__(self):
+        self.buffers = []
+        self.lock = threading.Lock()
+
+    def new(self, n: int, dtype) -> np.ndarray:
+        dtype = np.dtype(dtype)
+        nbytes = n * dtype.itemsize
+        if nbytes < self.kPinnedFrom:
+            return np.empty(n, dtype)
+        with self.lock:
+            spare = None
+            for b in self.buffers:
+                if b.idle():
+                    if b.nbytes >= nbytes:
+                        return b.lend(n, dtype)
+                    spare = b
+            if spare is not None:
+                self.buffers.remove(spare)      # too small for this batch: its place goes to a larger one
+            if len(self.buffers) < self.kBuffers:
+                try:
+                    b = _PinnedBuffer(nbytes)
+                except capi.SofieCudaError:
+                    return np.empty(n, dtype)   # no pinned memory to be had: the result is carried over by the host
+                self.buffers.append(b)
+                return b.lend(n, dtype)
+        return np.empty(n, dtype)
 
 
 class DynamicSession:
@@ -216,14 +277,15 @@ class DynamicSession:
         if not self.handle:
             raise RuntimeError(self.err.value.decode())
         self.max_batch, self.out_per_sample = max_batch, out_per_sample
+        self.results = _ResultArrays()
 
     def infer(self, x: np.ndarray) -> np.ndarray:
         """x: [batch, ...] float32; returns batch * out_per_sample floats."""
         x = np.ascontiguousarray(x, np.float32)
         bs = x.shape[0]
-        y = np.empty(max(1, bs * self.out_per_sample), np.float32)
-        ptrs = (C.c_void_p * 1)(x.ctypes.data_as(C.c_void_p))
-        n = self.lib.sofie_session_infer_bs(self.handle, bs, ptrs, y.ctypes.data_as(C.c_void_p), y.size, self.err, 1024)
+        y = self.results.new(max(1, bs * self.out_per_sample), np.float32)
+        ptrs = (C.c_void_p * 1)(x.ctypes.data)
+        n = self.lib.sofie_session_infer_bs(self.handle, bs, ptrs, y.ctypes.data, y.size, self.err, 1024)
         if n != bs * self.out_per_sample:
             raise RuntimeError(f"infer failed ({n}): {self.err.value.decode()}")
         return y[:n]
@@ -282,13 +344,14 @@ class GeneratedSession:
         if not self.handle:
             raise RuntimeError(self.err.value.decode())
         self.out_elems, self.out_dtype = out_elems, out_dtype
+        self.results = _ResultArrays()
 
     def infer(self, x, out: np.ndarray | None = None) -> np.ndarray:
         """x: one array, or a list of arrays for a model with several inputs (in the order of infer())."""
         xs = [np.ascontiguousarray(a) for a in (x if isinstance(x, (list, tuple)) else [x])]
-        ptrs = (C.c_void_p * max(1, len(xs)))(*[a.ctypes.data_as(C.c_void_p) for a in xs])
-        y = out if out is not None else np.empty(self.out_elems, self.out_dtype)
-        n = self.lib.sofie_session_infer(self.handle, ptrs, y.ctypes.data_as(C.c_void_p), self.out_elems, self.err, 1024)
+        ptrs = (C.c_void_p * max(1, len(xs)))(*[a.ctypes.data for a in xs])
+        y = out if out is not None else self.results.new(self.out_elems, self.out_dtype)
+        n = self.lib.sofie_session_infer(self.handle, ptrs, y.ctypes.data, self.out_elems, self.err, 1024)
         if n != self.out_elems:
             raise RuntimeError(f"infer failed ({n}): {self.err.value.decode()}")
         return y

@@ -24,6 +24,26 @@ inline std::string DevSlice(const std::string &name, size_t elems, size_t parts)
    return parts > 1 ? "(" + Dev(name) + " + (size_t)part * " + std::to_string(elems / parts) + ")" : Dev(name);
 }
 
+// Launches on a range of samples instead of one of a fixed number of slices: the text of one-sample slices (parts = the batch,
+// so that `part` is the index of a sample) with every count multiplied by `count`, both variables of the emitted code.
+inline bool &RangeMode()
+{
+   static bool on = false;
+   return on;
+}
+// what slice `part` holds of a quantity that is `total` over the whole batch, as a field of a descriptor
+inline std::string Count(size_t total, size_t parts)
+{
+   const std::string n = std::to_string(total / parts);
+   return RangeMode() ? "static_cast<int32_t>(" + n + " * count)" : n;
+}
+// the same as an element count (size_t)
+inline std::string CountLong(size_t total, size_t parts)
+{
+   const std::string n = std::to_string(total / parts);
+   return RangeMode() ? "(" + n + " * count)" : n;
+}
+
 inline std::string CType(ETensorType t)
 {
    switch (t) {

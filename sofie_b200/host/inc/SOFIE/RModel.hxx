@@ -59,6 +59,8 @@ private:
    bool fNeverPipelinedUpload = false;
    size_t fUploadParts = 4;                  // parts of a pipelined input upload (at most SOFIE_CUDA_MAX_PARTS)
    std::vector<size_t> fSlicedOps;           // operators launched once per uploaded part, in execution order
+   size_t fRangeBatch = 0;                   // samples of the batch when every operator can be launched on a range of it, else 0
+   size_t fRangeQuantum = 1;                 // such a range starts at a multiple of this many samples
    // Run-time batch: Generate() without a batch size on a model whose inputs carry a batch parameter in their first
    // dimension keeps that parameter in the emitted Session (reference: RModel.cxx:680-713, 876-884). Shapes are then
    // inferred with the batch set to a large prime; a number of the emitted text that is a multiple of it scales with the
@@ -172,6 +174,8 @@ public:
 protected:
    void PlanDevice();
    void PlanSlices();
+   void PlanRange(size_t head);
+   void GenerateUpload(bool pipelined, const std::string &result, size_t resultLen);
    void PlanArena();
    void GenerateSessionCode();
    void GenerateSessionMembers();

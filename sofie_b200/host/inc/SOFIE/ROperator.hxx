@@ -47,7 +47,8 @@ public:
    // Pipelined input upload: an operator that treats the samples of a batch independently can be launched
    // on slice `part` of `parts` equal, contiguous slices of its batch-shaped inputs and outputs (`part` is a
    // variable of the emitted code), so that the model works on one slice while the next is still being copied.
-   // Constant inputs (weights, tables) are read whole by every slice.
+   // Constant inputs (weights, tables) are read whole by every slice. With EMIT::RangeMode() on and `parts` = the batch the
+   // text is a launch on `count` samples from sample `part` on, both variables of the emitted code.
    virtual bool CanSliceBatch(size_t /*parts*/) const { return false; }
    virtual std::string GenerateBatchSlice(std::string /*OpName*/, size_t /*parts*/) { return ""; }
 

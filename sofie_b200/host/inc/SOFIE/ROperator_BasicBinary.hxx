@@ -100,13 +100,13 @@ private:
       OpName = "op_" + OpName;
       if (fShapeY.empty() && ConvertShapeToLength(fShapeY) != 1)
          throw std::runtime_error("SOFIE Binary Op called to Generate without being initialized first");
-      std::vector<size_t> out4(4 - fShapeY.size(), 1);
-      out4.insert(out4.end(), fShapeY.begin(), fShapeY.end());
+      std::vector<std::string> out4(4 - fShapeY.size(), "1");
+      for (size_t n : fShapeY) out4.push_back(std::to_string(n));
       auto sa = Strides(fShapeA, fShapeY), sb = Strides(fShapeB, fShapeY);
       std::string a = EMIT::Dev(fNA), b = EMIT::Dev(fNB), y = EMIT::Dev(fNY);
       if (parts > 1) {
          const size_t lead = 4 - fShapeY.size(), rows = fShapeY[0] / parts;
-         out4[lead] = rows;
+         out4[lead] = EMIT::Count(fShapeY[0], parts);
          if (sa[lead]) a = "(" + a + " + (size_t)part * " + std::to_string((size_t)sa[lead] * rows) + ")";
          if (sb[lead]) b = "(" + b + " + (size_t)part * " + std::to_string((size_t)sb[lead] * rows) + ")";
          y = EMIT::DevSlice(fNY, ConvertShapeToLength(fShapeY), parts);

@@ -60,7 +60,7 @@ private:
       const size_t n = ConvertShapeToLength(fShape);
       out << "\n" << SP << "//------ " << fOpLabel << " " << OpName << (parts > 1 ? ", one slice of the batch" : "") << "\n";
       out << EMIT::Call(SP, "sofie_cuda_unary_f32(fStream, " + std::to_string(fCode) + ", " + EMIT::FloatLit(fAlpha) + ", " +
-                               EMIT::DevSlice(fNX, n, parts) + ", " + EMIT::DevSlice(fNY, n, parts) + ", " + std::to_string(n / parts) + ")");
+                               EMIT::DevSlice(fNX, n, parts) + ", " + EMIT::DevSlice(fNY, n, parts) + ", " + EMIT::CountLong(n, parts) + ")");
       return out.str();
    }
 };

@@ -294,7 +294,7 @@ private:
       std::stringstream out;
       out << "\n" << SP << "//----  operator Conv " << OpName << (fFusedRelu ? " + Relu" : "") << (fFusedPool ? " + MaxPool2x2" : "")
           << " -> " << fNOut << " " << ConvertShapeToString(fShapeOut) << (fLayoutY == ELayout::NHWC ? " (NHWC)" : "");
-      if (parts > 1) out << ", one of " << parts << " slices of the batch";
+      if (parts > 1) out << (EMIT::RangeMode() ? std::string(", a range of the batch") : ", one of " + std::to_string(parts) + " slices of the batch");
       out << "\n";
       out << SP << "{\n";
       std::string x = EMIT::Dev(fNX), y = EMIT::Dev(fNOut);
@@ -304,7 +304,7 @@ private:
          y += " + (size_t)part * " + std::to_string(ConvertShapeToLength(fShapeOut) / parts);
       }
       if (fAttr.volume) {
-         out << SP << SP << "const sofie_conv3d_desc d = {" << fShapeX[0] / parts << ", " << fShapeX[1] << ", " << fShapeX[2] << ", " << fShapeX[3]
+         out << SP << SP << "const sofie_conv3d_desc d = {" << EMIT::Count(fShapeX[0], parts) << ", " << fShapeX[1] << ", " << fShapeX[2] << ", " << fShapeX[3]
              << ", " << fShapeX[4] << ", " << fShapeW[0] << ", " << fAttr.k3[0] << ", " << fAttr.k3[1] << ", " << fAttr.k3[2] << ", "
              << fAttr.pad3[0] << ", " << fAttr.pad3[1] << ", " << fAttr.pad3[2] << ", " << fAttr.s3[0] << ", " << fAttr.s3[1] << ", "
              << fAttr.s3[2] << ", " << fAttr.d3[0] << ", " << fAttr.d3[1] << ", " << fAttr.d3[2] << ", " << fAttr.group << ", "
@@ -316,7 +316,7 @@ private:
       }
       // a 1-D convolution runs as an image of height 1
       const size_t H = fAttr.oneD ? 1 : fShapeX[2], W = fAttr.oneD ? fShapeX[2] : fShapeX[3];
-      out << SP << SP << "const sofie_conv2d_desc d = {" << fShapeX[0] / parts << ", " << fShapeX[1] << ", " << H << ", "
+      out << SP << SP << "const sofie_conv2d_desc d = {" << EMIT::Count(fShapeX[0], parts) << ", " << fShapeX[1] << ", " << H << ", "
           << W << ", " << fShapeW[0] << ", " << fAttr.kH << ", " << fAttr.kW << ", " << fAttr.padH << ", " << fAttr.padW
           << ", " << fAttr.sH << ", " << fAttr.sW << ", " << fAttr.dH << ", " << fAttr.dW << ", " << fAttr.group << ", "
           << (int)fLayoutX << ", " << (int)fLayoutY << ", " << (fPacked ? 1 : 0) << ", " << (fFusedRelu ? 1 : 0) << ", "

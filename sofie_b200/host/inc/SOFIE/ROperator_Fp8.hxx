@@ -64,7 +64,7 @@ private:
       const size_t n = ConvertShapeToLength(fShape);
       out << "\n" << SP << "//------ QuantizeLinear (E4M3) op_" << OpName << (parts > 1 ? ", one slice of the batch" : "") << "\n";
       out << EMIT::Call(SP, std::string(fInType == ETensorType::FLOAT ? "sofie_cuda_quantize_e4m3_f32" : "sofie_cuda_quantize_e4m3_bf16") +
-                               "(fStream, " + EMIT::DevSlice(fNX, n, parts) + ", " + EMIT::DevSlice(fNY, n, parts) + ", " + std::to_string(n / parts) + ", " +
+                               "(fStream, " + EMIT::DevSlice(fNX, n, parts) + ", " + EMIT::DevSlice(fNY, n, parts) + ", " + EMIT::CountLong(n, parts) + ", " +
                                EMIT::FloatLit(fScale) + ")");
       return out.str();
    }
@@ -216,7 +216,7 @@ private:
           << (fOutScale > 0.f ? " -> E4M3" : (fNYFloat.empty() ? " -> bfloat16" : " -> bfloat16 -> float (Cast fused)"))
           << (parts > 1 ? ", one slice of the rows" : "") << "\n";
       out << SP << "{\n";
-      out << SP << SP << "const sofie_fp8_gemm_desc d = {" << fShapeA[0] / parts << ", " << fShapeW[0] << ", " << fShapeA[1] << ", "
+      out << SP << SP << "const sofie_fp8_gemm_desc d = {" << EMIT::Count(fShapeA[0], parts) << ", " << fShapeW[0] << ", " << fShapeA[1] << ", "
           << EMIT::FloatLit(fAScale) << ", " << EMIT::FloatLit(fWScale) << ", " << (fRelu ? 1 : 0) << ", " << EMIT::FloatLit(fOutScale) << "};\n";
       const std::string bias = fNB.empty() ? std::string("nullptr") : EMIT::Dev(fNB);
       const size_t lenA = fShapeA[0] * fShapeA[1], lenY = fShapeA[0] * fShapeW[0];

@@ -244,7 +244,7 @@ private:
             w += (l ? ", " : "") + EMIT::Dev(layers[l]->fNBdev);
             b += (l ? ", " : "") + (layers[l]->fBiasKind ? EMIT::Dev(layers[l]->fNCdev) : std::string("nullptr"));
          }
-         out << SP << SP << "const sofie_mlp_desc d = {" << M << ", " << layers.size() << ", {" << dims << "}, {" << relu << "}, {" << nk << "}};\n";
+         out << SP << SP << "const sofie_mlp_desc d = {" << EMIT::Count(fM, parts) << ", " << layers.size() << ", {" << dims << "}, {" << relu << "}, {" << nk << "}};\n";
          out << SP << SP << "const float * const w[] = {" << w << "};\n";
          out << SP << SP << "const float * const b[] = {" << b << "};\n";
          out << EMIT::Call(SP + SP, "sofie_cuda_mlp_f32(fStream, &d, " + EMIT::DevSlice(fNA, fM * fK, parts) + ", w, b, " +
@@ -268,7 +268,7 @@ private:
       out << "\n" << SP << "//--------- Gemm " << opName << ": [" << M << "," << fK << "] x [" << fK << "," << fN << "]"
           << (parts > 1 ? ", one slice of the rows" : "") << "\n";
       out << SP << "{\n";
-      out << SP << SP << "const sofie_gemm_f32_desc d = {" << M << ", " << fN << ", " << fK << ", " << fAttrTransA << ", "
+      out << SP << SP << "const sofie_gemm_f32_desc d = {" << EMIT::Count(fM, parts) << ", " << fN << ", " << fK << ", " << fAttrTransA << ", "
           << fEmitTransB << ", " << EMIT::FloatLit(fAttrAlpha) << ", " << EMIT::FloatLit(fBiasKind ? fAttrBeta : 0.f) << ", "
           << fBiasKind << ", " << (fActivation == EActivationType::RELU ? 1 : 0) << "};\n";
       out << EMIT::Call(SP + SP, "sofie_cuda_gemm_f32(fStream, &d, " + EMIT::DevSlice(fNA, fM * fK, parts) + ", " + EMIT::Dev(fNBdev) + ", " +

@@ -184,13 +184,13 @@ private:
       }
       if (fType == ETensorType::UINT8) {
          out << EMIT::Call(SP, "sofie_cuda_maxpool2d_u8(fStream, " + x + ", " + y + ", " +
-                                  std::to_string(fShape4[0] / parts) + ", " + std::to_string(fShape4[1]) + ", " + std::to_string(fShape4[2]) +
+                                  EMIT::Count(fShape4[0], parts) + ", " + std::to_string(fShape4[1]) + ", " + std::to_string(fShape4[2]) +
                                   ", " + std::to_string(fShape4[3]) + ", " + std::to_string(fKH) + ", " + std::to_string(fKW) + ", " +
                                   std::to_string(fSH) + ", " + std::to_string(fSW) + ", " + std::to_string((int)fLayout) + ")");
          return out.str();
       }
       out << SP << "{\n";
-      out << SP << SP << "const sofie_pool2d_desc d = {" << (fPoolMode == MaxPool ? 0 : 1) << ", " << fShape4[0] / parts << ", " << fShape4[1]
+      out << SP << SP << "const sofie_pool2d_desc d = {" << (fPoolMode == MaxPool ? 0 : 1) << ", " << EMIT::Count(fShape4[0], parts) << ", " << fShape4[1]
           << ", " << fShape4[2] << ", " << fShape4[3] << ", " << fKH << ", " << fKW << ", " << fSH << ", " << fSW << ", {" << fPads[0]
           << ", " << fPads[1] << ", " << fPads[2] << ", " << fPads[3] << "}, " << fAttr.count_include_pad << ", " << (int)fLayout << "};\n";
       out << EMIT::Call(SP + SP, "sofie_cuda_pool2d_f32(fStream, &d, " + x + ", " + y + ")");

@@ -83,7 +83,7 @@ private:
       const size_t n = ConvertShapeToLength(fShape);
       out << "\n" << SP << "//------ QuantizeLinear op_" << OpName << (parts > 1 ? ", one slice of the batch" : "") << "\n";
       out << EMIT::Call(SP, "sofie_cuda_quantize_u8(fStream, " + EMIT::DevSlice(fNX, n, parts) + ", " + EMIT::DevSlice(fNY, n, parts) + ", " +
-                               std::to_string(n / parts) + ", " + EMIT::FloatLit(fScale) + ", " + std::to_string(fZp) + ")");
+                               EMIT::CountLong(n, parts) + ", " + EMIT::FloatLit(fScale) + ", " + std::to_string(fZp) + ")");
       return out.str();
    }
 };
@@ -264,7 +264,7 @@ private:
       out << "\n" << SP << "//--------- QLinearMatMul op_" << OpName << (fRelu ? " + Relu" : "") << ": [" << m << "," << fK << "] x [" << fK
           << "," << fN << "]" << (parts > 1 ? ", one slice of the rows" : "") << "\n";
       out << SP << "{\n";
-      out << SP << SP << "const sofie_qgemm_desc d = {" << m << ", " << fN << ", " << fK << ", 1, " << fYZp << ", " << (fRelu ? 1 : 0) << "};\n";
+      out << SP << SP << "const sofie_qgemm_desc d = {" << EMIT::Count(fM, parts) << ", " << fN << ", " << fK << ", 1, " << fYZp << ", " << (fRelu ? 1 : 0) << "};\n";
       const std::string a = EMIT::DevSlice(fNA, fM * fK, parts);
       if (!fNYFloat.empty())
          out << EMIT::Call(SP + SP, "sofie_cuda_qlinear_matmul_f32(fStream, &d, " + a + ", " + EMIT::Dev(fNBdev) + ", " +
@@ -413,7 +413,7 @@ private:
           << fNOut << " " << ConvertShapeToString(fShapeOut) << (fLayoutY == ELayout::NHWC ? " (NHWC)" : "")
           << (parts > 1 ? ", one slice of the batch" : "") << "\n";
       out << SP << "{\n";
-      out << SP << SP << "const sofie_qconv2d_desc d = {" << fShapeX[0] / parts << ", " << fShapeX[1] << ", " << fShapeX[2] << ", " << fShapeX[3]
+      out << SP << SP << "const sofie_qconv2d_desc d = {" << EMIT::Count(fShapeX[0], parts) << ", " << fShapeX[1] << ", " << fShapeX[2] << ", " << fShapeX[3]
           << ", " << fShapeW[0] << ", " << fAttr.kH << ", " << fAttr.kW << ", " << fAttr.padH << ", " << fAttr.padW << ", " << fAttr.sH
           << ", " << fAttr.sW << ", " << (int)fLayoutX << ", " << (int)fLayoutY << ", " << (fPacked ? 1 : 0) << ", " << fXZp << ", "
           << fYZp << ", " << (fRelu ? 1 : 0) << ", " << fPool << "};\n";

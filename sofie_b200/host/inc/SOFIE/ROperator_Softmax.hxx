@@ -63,7 +63,7 @@ private:
       std::stringstream out;
       const size_t n = ConvertShapeToLength(fShape);
       out << "\n" << SP << "//------ SOFTMAX - " << rank << "  " << n << "  " << axis << (parts > 1 ? ", one slice of the batch" : "") << "\n";
-      out << EMIT::Call(SP, "sofie_cuda_softmax_f32(fStream, " + EMIT::DevSlice(fNX, n, parts) + ", " + EMIT::DevSlice(fNY, n, parts) + ", " + std::to_string(outer / parts) +
+      out << EMIT::Call(SP, "sofie_cuda_softmax_f32(fStream, " + EMIT::DevSlice(fNX, n, parts) + ", " + EMIT::DevSlice(fNY, n, parts) + ", " + EMIT::CountLong(outer, parts) +
                                ", " + std::to_string(fShape[axis]) + ", " + std::to_string(inner) + ")");
       return out.str();
    }

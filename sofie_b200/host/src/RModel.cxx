@@ -430,16 +430,21 @@ void RModel::PlanSlices()
    // What is left after the last copy is one part's share of the kernels: eight parts from 128 MB on, four below.
    fSlicedOps.clear();
    fUploadParts = 4;
+   fRangeBatch = 0;
+   fRangeQuantum = 1;
    size_t head = fOperators.size();
    for (size_t i = 0; i < fOperators.size(); i++)
       if (!fOperators[i]->IsFusedAway()) {
          head = i;
          break;
       }
-   if (head >= fOperators.size() || fInputTensorNames.size() != 1 || fNeverPipelinedUpload || fDynamicBatch) return;
+   if (head >= fOperators.size() || fInputTensorNames.size() != 1 || fNeverPipelinedUpload) return;
    const std::string &in = fInputTensorNames[0];
    const size_t inBytes = ConvertShapeToLength(GetTensorShape(in)) * GetTypeSize(GetTensorType(in));
-   if (inBytes < (fForcePipelinedUpload ? 0 : size_t(32) << 20)) return;
+   if (fDynamicBatch || inBytes < (fForcePipelinedUpload ? 0 : size_t(32) << 20)) {
+      PlanRange(head);
+      return;
+   }
    auto prefix = [&](size_t parts) {
       std::vector<size_t> sliced;
       // every slice of a tensor starts on a 256-byte boundary, like the tensor itself
@@ -480,6 +485,49 @@ void RModel::PlanSlices()
          fUploadParts = 8;
       }
    }
+   if (fSlicedOps.empty()) PlanRange(head);
+}
+
+// Batches that do not split into equal parts, whose size is known at run time only, or that are between a few and 32 MB: when
+// every operator treats the samples independently, the emitted infer() cuts the batch into ranges of samples
+// (sofie_cuda_slice_rows: how many, by the bytes that cross PCIe) and each range is copied in, computed and copied out beside
+// the others. A batch that is not worth cutting runs as the captured graph of the whole.
+void RModel::PlanRange(size_t head)
+{
+   const std::string &in = fInputTensorNames[0];
+   const auto &inShape = GetTensorShape(in);
+   if (inShape.empty() || inShape[0] < 2 || fOutputTensorNames.size() != 1) return;
+   const size_t batch = inShape[0];
+   auto bytes_of = [&](const std::string &n) { return ConvertShapeToLength(GetTensorShape(n)) * GetTypeSize(GetTensorType(n)); };
+   if (!fDynamicBatch && std::max(bytes_of(in), bytes_of(fOutputTensorNames[0])) < (size_t(4) << 20)) return;
+   // every range of a tensor starts on a 256-byte boundary, like the tensor itself; rows of matrices in whole tiles of 128
+   size_t quantum = inShape.size() == 2 ? 128 : 1;
+   auto ranges = [&](const std::string &n) {
+      const size_t b = bytes_of(n);
+      if (b == 0 || b % batch != 0) return false;
+      while ((b / batch * quantum) % 256 != 0) quantum *= 2;
+      return true;
+   };
+   if (!ranges(in)) return;
+   std::set<std::string> parted{in};
+   for (size_t i = head; i < fOperators.size(); i++) {
+      auto &op = fOperators[i];
+      if (op->IsFusedAway()) continue;
+      bool ok = op->CanSliceBatch(batch);
+      size_t batchInputs = 0;
+      for (auto &n : op->GetOpInputTensors()) {
+         if (IsInitializedTensor(n)) continue;
+         ok = ok && parted.count(n) != 0;
+         batchInputs++;
+      }
+      ok = ok && batchInputs > 0;
+      for (auto &w : op->GetOpOutputTensors()) ok = ok && ranges(w);
+      if (!ok) return;
+      for (auto &w : op->GetOpOutputTensors()) parted.insert(w);
+   }
+   if (!parted.count(fOutputTensorNames[0]) || fOutputTensorNames[0] == in) return;
+   fRangeBatch = batch;
+   fRangeQuantum = quantum;
 }
 
 // Step 5: liveness-based first-fit placement in one arena (256-byte aligned slices).
@@ -540,6 +588,14 @@ void RModel::PlanArena()
       for (auto &in : fInputTensorNames) together(in);
       for (size_t i : fSlicedOps)
          for (auto &out : fOperators[i]->GetOpOutputTensors()) together(out);
+   }
+   // Ranges of a batch run one after the other, so the tensors between the first and the last operator may share bytes as in
+   // the plan of the whole; but later ranges of the input arrive, and earlier ranges of the output leave, meanwhile.
+   if (fRangeBatch) {
+      for (auto &in : fInputTensorNames)
+         if (Slot *s = slot_of(in)) s->last = nOps;
+      for (auto &o : fOutputTensorNames)
+         if (Slot *s = slot_of(o)) s->first = -1;
    }
    fArenaBytes = 0;
    for (size_t i = 0; i < slots.size(); i++) {
@@ -868,6 +924,15 @@ void RModel::GenerateInfer()
       for (size_t i : sliced) fGC += fOperators[i]->GenerateBatchSlice(std::to_string(i), fUploadParts);
       fGC += "}\n\n";
    }
+   if (fRangeBatch) {
+      fGC += "// every operator on the samples [part, part + count)\n";
+      fGC += "void LaunchRange(size_t part, size_t count) {\n";
+      EMIT::RangeMode() = true;
+      for (size_t i = 0; i < fOperators.size(); i++)
+         if (!fOperators[i]->IsFusedAway()) fGC += fOperators[i]->GenerateBatchSlice(std::to_string(i), fRangeBatch);
+      EMIT::RangeMode() = false;
+      fGC += "}\n\n";
+   }
    fGC += pipelined ? "// all other kernel launches of one inference, on the context stream\n"
                     : "// all kernel launches of one inference, on the context stream\n";
    fGC += "void Launch() {\n";
@@ -920,14 +985,85 @@ void RModel::GenerateInfer()
    if (pipelined) fGC += "   for (int part = 0; part < " + std::to_string(fUploadParts) + "; part++) LaunchHead(part);\n";
    fGC += "   Run();\n";
    fGC += "}\n\n";
-   fGC += ret + " infer(" + GenerateInferSignature() + "){\n";
-   if (fDynamicBatch) {
-      // any batch up to the one the Session was built for; the graph is captured again when the batch changes
+   auto checkBatch = [&] {
+      // any batch up to the one the Session was built for
       fGC += "   if (" + fBatchParam + " > fMaxBatch) throw std::runtime_error(\"SOFIE: infer() was called with " + fBatchParam +
              " = \" + std::to_string(" + fBatchParam + ") + \", the Session was constructed for at most \" + std::to_string(fMaxBatch));\n";
-      fGC += "   if (" + fBatchParam + " == 0) return {};\n";
-      fGC += "   if (" + fBatchParam + " != fBatch) { fBatch = " + fBatchParam + "; fGraphReady = false; }\n";
+   };
+   auto upload = [&] {
+      // the graph is captured again when the batch changes
+      if (fDynamicBatch) fGC += "   if (" + fBatchParam + " != fBatch) { fBatch = " + fBatchParam + "; fGraphReady = false; }\n";
+   };
+   const std::string sig = GenerateInferSignature(), args = GenerateInferSignature(false);
+   if (nOut != 1) {
+      fGC += ret + " infer(" + sig + "){\n";
+      if (fDynamicBatch) {
+         checkBatch();
+         fGC += "   if (" + fBatchParam + " == 0) return {};\n";
+      }
+      upload();
+      GenerateUpload(pipelined, "", 0);
+      fGC += "   Run();\n";
+      for (size_t i = 0; i < nOut; i++) {
+         const std::string &o = fOutputTensorNames[i];
+         std::string type = ConvertTypeToString(GetTensorType(o));
+         // the result lands in the context's pinned buffer; the returned vector is built from it in one pass
+         const std::string idx = std::to_string(i), len = std::to_string(ConvertShapeToLength(GetTensorShape(o)));
+         fGC += "   void * host_ret_" + idx + " = nullptr;\n";
+         fGC += "   Check(sofie_cuda_ctx_fetch(fCtx, " + EMIT::Dev(o) + ", " + ByteCount(GetTensorShape(o), GetTensorType(o)) + ", &host_ret_" + idx +
+                "), \"sofie_cuda_ctx_fetch\");\n";
+         fGC += "   std::vector<" + type + "> ret_" + idx + "(static_cast<const " + type + " *>(host_ret_" + idx + "), static_cast<const " + type +
+                " *>(host_ret_" + idx + ") + " + len + ");\n";
+      }
+      fGC += "   return {";
+      for (size_t i = 0; i < nOut; i++) fGC += "ret_" + std::to_string(i) + (i + 1 < nOut ? "," : "");
+      fGC += "};\n}\n";
+      return;
    }
+   // One inference from host to host: `out` is where the result shall go (pinned memory is written by the copy itself), or
+   // nullptr for the context's own pinned memory; returns where it is.
+   const std::string &o = fOutputTensorNames[0];
+   const std::string type = ConvertTypeToString(t0), sep = sig.empty() ? "" : ", ";
+   const size_t outLen = ConvertShapeToLength(GetTensorShape(o)), outBytes = outLen * GetTypeSize(t0);
+   fGC += "const " + type + " * Execute(" + sig + sep + type + " * out) {\n";
+   upload();
+   fGC += "   Check(sofie_cuda_ctx_result_begin(fCtx, out, " + std::to_string(outBytes) + "), \"sofie_cuda_ctx_result_begin\");\n";
+   const bool resultInParts = pipelined && tailOps == 0;
+   GenerateUpload(pipelined, resultInParts ? o : "", outLen);
+   if (fRangeBatch) fGC += "   } else {\n";
+   if (fRangeBatch) GenerateUpload(false, "", 0);
+   fGC += "   Run();\n";
+   if (!resultInParts)
+      fGC += "   Check(sofie_cuda_ctx_result_part(fCtx, " + EMIT::Dev(o) + ", 0, " + std::to_string(outBytes) + "), \"sofie_cuda_ctx_result_part\");\n";
+   if (fRangeBatch) fGC += "   }\n";
+   fGC += "   void * host = nullptr;\n";
+   fGC += "   Check(sofie_cuda_ctx_result_end(fCtx, &host), \"sofie_cuda_ctx_result_end\");\n";
+   fGC += "   return static_cast<const " + type + " *>(host);\n}\n\n";
+   // the returned vector is built from the context's pinned memory in one pass
+   fGC += ret + " infer(" + sig + "){\n";
+   if (fDynamicBatch) {
+      checkBatch();
+      fGC += "   if (" + fBatchParam + " == 0) return {};\n";
+   }
+   fGC += "   const " + type + " * host_ret_0 = Execute(" + args + sep + "nullptr);\n";
+   fGC += "   std::vector<" + type + "> ret_0(host_ret_0, host_ret_0 + " + std::to_string(outLen) + ");\n";
+   fGC += "   return ret_0;\n}\n\n";
+   // The same result into the caller's memory of `capacity` values; returns how many values the result has, and computes
+   // nothing when there is no room for them.
+   fGC += "size_t inferTo(" + sig + sep + type + " * out, size_t capacity) {\n";
+   if (fDynamicBatch) checkBatch();
+   const std::string count = fDynamicBatch ? std::to_string(outLen / kBatchSentinel) + " * " + fBatchParam : std::to_string(outLen);
+   fGC += "   const size_t values = " + count + ";\n";
+   fGC += "   if (values == 0 || values > capacity) return values;\n";
+   fGC += "   Execute(" + args + sep + "out);\n";
+   fGC += "   return values;\n}\n";
+}
+
+// The inputs' way to the device. pipelined: in parts, with the sliced operators launched part by part and, when `result` names a
+// tensor, its part sent back behind them. Without parts but with a range plan: the branch that cuts the batch into ranges, left
+// open at its else.
+void RModel::GenerateUpload(bool pipelined, const std::string &result, size_t resultLen)
+{
    if (pipelined) {
       const std::string &n = fInputTensorNames[0];
       const size_t elems = ConvertShapeToLength(GetTensorShape(n)) / fUploadParts;
@@ -940,31 +1076,37 @@ void RModel::GenerateInfer()
              ", " + std::to_string(elems * GetTypeSize(GetTensorType(n))) + ", part), \"sofie_cuda_ctx_h2d_part\");\n";
       fGC += "      Check(sofie_cuda_ctx_wait_part(fCtx, part), \"sofie_cuda_ctx_wait_part\");\n";
       fGC += "      LaunchHead(part);\n";
+      if (!result.empty()) {
+         const size_t rlen = resultLen / fUploadParts, rbytes = rlen * GetTypeSize(GetTensorType(result));
+         fGC += "      Check(sofie_cuda_ctx_result_part(fCtx, " + EMIT::Dev(result) + " + (size_t)part * " + std::to_string(rlen) + ", (size_t)part * " +
+                std::to_string(rbytes) + ", " + std::to_string(rbytes) + "), \"sofie_cuda_ctx_result_part\");\n";
+      }
       fGC += "   }\n";
-   } else {
-      for (auto &n : fInputTensorNames)
-         fGC += "   Check(sofie_cuda_ctx_h2d(fCtx, " + EMIT::Dev(n) + ", tensor_" + n + ", " + ByteCount(GetTensorShape(n), GetTensorType(n)) +
-                "), \"sofie_cuda_ctx_h2d\");\n";
+      return;
    }
-   fGC += "   Run();\n";
-   for (size_t i = 0; i < nOut; i++) {
-      const std::string &o = fOutputTensorNames[i];
-      std::string type = ConvertTypeToString(GetTensorType(o));
-      // the result lands in the context's pinned buffer; the returned vector is built from it in one pass
-      const std::string idx = std::to_string(i), len = std::to_string(ConvertShapeToLength(GetTensorShape(o)));
-      fGC += "   void * host_ret_" + idx + " = nullptr;\n";
-      fGC += "   Check(sofie_cuda_ctx_fetch(fCtx, " + EMIT::Dev(o) + ", " + ByteCount(GetTensorShape(o), GetTensorType(o)) + ", &host_ret_" + idx +
-             "), \"sofie_cuda_ctx_fetch\");\n";
-      fGC += "   std::vector<" + type + "> ret_" + idx + "(static_cast<const " + type + " *>(host_ret_" + idx + "), static_cast<const " + type +
-             " *>(host_ret_" + idx + ") + " + len + ");\n";
+   if (fRangeBatch && resultLen) {
+      const std::string &n = fInputTensorNames[0], &o = fOutputTensorNames[0];
+      const size_t in1 = ConvertShapeToLength(GetTensorShape(n)) / fRangeBatch, out1 = resultLen / fRangeBatch;
+      const size_t inB = in1 * GetTypeSize(GetTensorType(n)), outB = out1 * GetTypeSize(GetTensorType(o));
+      const std::string batch = std::to_string(fRangeBatch), i1 = std::to_string(in1), o1 = std::to_string(out1);
+      fGC += "   const size_t samples = " + batch + ", rows = sofie_cuda_slice_rows(samples, " + std::to_string(inB) + ", " + std::to_string(outB) + ", " +
+             std::to_string(fRangeQuantum) + ");\n";
+      fGC += "   if (rows < samples) {\n";
+      fGC += "      int index = 0;\n";
+      fGC += "      for (size_t part = 0; part < samples; part += rows, index++) {\n";
+      fGC += "         const size_t count = samples - part < rows ? samples - part : rows;\n";
+      fGC += "         Check(sofie_cuda_ctx_h2d_part(fCtx, " + EMIT::Dev(n) + " + part * " + i1 + ", tensor_" + n + " + part * " + i1 + ", count * " + std::to_string(inB) +
+             ", index), \"sofie_cuda_ctx_h2d_part\");\n";
+      fGC += "         Check(sofie_cuda_ctx_wait_part(fCtx, index), \"sofie_cuda_ctx_wait_part\");\n";
+      fGC += "         LaunchRange(part, count);\n";
+      fGC += "         Check(sofie_cuda_ctx_result_part(fCtx, " + EMIT::Dev(o) + " + part * " + o1 + ", part * " + std::to_string(outB) + ", count * " + std::to_string(outB) +
+             "), \"sofie_cuda_ctx_result_part\");\n";
+      fGC += "      }\n";
+      return;
    }
-   if (nOut == 1) fGC += "   return ret_0;\n";
-   else {
-      fGC += "   return {";
-      for (size_t i = 0; i < nOut; i++) fGC += "ret_" + std::to_string(i) + (i + 1 < nOut ? "," : "");
-      fGC += "};\n";
-   }
-   fGC += "}\n";
+   for (auto &n : fInputTensorNames)
+      fGC += "   Check(sofie_cuda_ctx_h2d(fCtx, " + EMIT::Dev(n) + ", tensor_" + n + ", " + ByteCount(GetTensorShape(n), GetTensorType(n)) +
+             "), \"sofie_cuda_ctx_h2d\");\n";
 }
 
 void RModel::GenerateSessionCode()

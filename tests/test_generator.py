@@ -457,3 +457,19 @@ def test_volume_operators_emit_3d_calls():
     pool = re.search(r"sofie_pool3d_desc d = \{([^;]*)\};", text).group(1)
     assert [int(v) for v in re.findall(r"-?\d+", pool)] == [0, 2, 8, 6, 8, 10, 2, 2, 2, 2, 2, 2, 0, 0, 0, 0, 0, 0, 0]
     generated.compile_session(_emit(m, "volume_b2"), "volume_b2")
+
+
+def test_ranges_of_a_batch_keep_the_arriving_input_and_the_leaving_result_apart():
+    """From 4 MB on (or with a run-time batch) every operator is emitted once more on a range of samples; the input and the result then
+    share no arena bytes with anything, because later ranges arrive and earlier ones leave meanwhile."""
+    m, _ = configs.mlp_i8(batch=4099, with_input=False)
+    text = _emit(m, "c3_b4099").read_text()
+    body = text[text.index("void LaunchRange(size_t part, size_t count)"):text.index("void Launch() {")]
+    assert body.count("sofie_cuda_quantize_u8(") == 1 and body.count("sofie_cuda_qlinear_matmul(fStream") + body.count("sofie_cuda_qlinear_matmul_f32(fStream") == 3 and "(512 * count)" in body
+    assert "sofie_cuda_slice_rows(samples, 2048, 1024, 128)" in text
+    slices = {n: (int(o), int(o) + int(b)) for o, b, n in re.findall(r"sofie_cuda_ctx_arena\(fCtx, (\d+), (\d+), reinterpret_cast<void\*\*>\(&dev_(\w+)\)\)", text)}
+    for edge in ("x", "y"):
+        lo, hi = slices[edge]
+        assert all(h <= lo or hi <= l for n, (l, h) in slices.items() if n != edge), edge
+    small = _emit(configs.mlp_i8(batch=100, with_input=False)[0], "c3_b100").read_text()
+    assert "LaunchRange" not in small and "sofie_cuda_slice_rows" not in small

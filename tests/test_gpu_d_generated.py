@@ -324,3 +324,48 @@ def test_batch_sharded_over_sessions_with_the_helper(cuda_device, tmp_path):
     ref = run_model.run(m, x).ravel()
     assert np.array_equal(y.view(np.uint32), ref.view(np.uint32))
     assert np.array_equal(y7.view(np.uint32), ref[:14].view(np.uint32))
+
+
+@pytest.mark.parametrize("key,batch,dynamic", [("C3", 4099, False), ("C3", 4099, True), ("C2", 1003, True), ("RES", 1001, False)])
+def test_batch_cut_into_ranges_of_samples(key, batch, dynamic, cuda_device):
+    """Batches that do not split into equal parts, from 4 MB of input on: infer() cuts them into ranges (the last one short). The result
+    is that of the whole batch (the same model emitted with one upload), from pageable and from pinned memory, into a fresh array, into
+    memory of the caller, and for more results kept alive than a Session lends pinned buffers for."""
+    import torch
+    build = configs.resblock_f32 if key == "RES" else configs.BUILDERS[key]
+    m, x = build(batch=batch)
+    whole = generated.session_from_model(m, f"{key.lower()}_b{batch}_whole", pipelined=False).infer(x)
+    if dynamic:
+        s = generated.dynamic_session_from_model(m, f"{key.lower()}_dyn_range", batch + 5)
+    else:
+        s = generated.session_from_model(m, f"{key.lower()}_b{batch}_range")
+    assert "void LaunchRange(size_t part, size_t count)" in s.hxx.read_text()
+    assert capi_slice_rows(batch, x[0].nbytes) < batch
+
+    def check(y):
+        if key == "C3":
+            assert np.array_equal(np.asarray(y).view(np.uint32), whole.view(np.uint32))
+        else:
+            assert rel_err(np.asarray(y), whole) <= 1e-5
+    kept = [s.infer(x) for _ in range(5)]
+    xp = torch.from_numpy(x).pin_memory().numpy()
+    kept.append(s.infer(xp))
+    for y in kept:
+        check(y)
+    for a in range(len(kept)):
+        for b in range(a):
+            assert not np.shares_memory(kept[a], kept[b])
+    part = kept[0][7:9]
+    want = part.copy()
+    del kept, y                                  # a view keeps its buffer: the next results land elsewhere
+    again = [s.infer(x[::-1].copy()) for _ in range(4)]
+    assert np.array_equal(part, want) and len(again) == 4
+    if not dynamic:
+        out = np.full(whole.size, np.nan, np.float32)
+        assert s.infer(x, out) is out
+        check(out)
+
+
+def capi_slice_rows(rows, in_bytes):
+    from sofie_b200 import capi
+    return capi.load().sofie_cuda_slice_rows(rows, in_bytes, 0, 128)
