@@ -88,6 +88,22 @@ int sofie_cuda_ctx_h2d(sofie_cuda_ctx *ctx, void *dst_device, const void *src_ho
 #define SOFIE_CUDA_MAX_PARTS 8
 int sofie_cuda_ctx_h2d_part(sofie_cuda_ctx *ctx, void *dst_device, const void *src_host, size_t bytes, int part);
 int sofie_cuda_ctx_wait_part(sofie_cuda_ctx *ctx, int part);
+/* A float input that the model only reads to quantise it, when it lies in pageable memory (sofie_cuda_ctx_pageable: 1): the host,
+ * which has to move every float into pinned memory anyway, quantises while it does, and a quarter of the bytes cross PCIe. dst
+ * receives the n bytes the first operator would have written (kind SOFIE_CUDA_STAGE_U8: sofie_cuda_quantize_u8's, STAGE_E4M3:
+ * sofie_cuda_quantize_e4m3_f32's, bit for bit). part < 0: on the context stream; else as part `part` on the copy stream. */
+#define SOFIE_CUDA_STAGE_COPY 0
+#define SOFIE_CUDA_STAGE_U8 1
+#define SOFIE_CUDA_STAGE_E4M3 2
+int sofie_cuda_ctx_pageable(sofie_cuda_ctx *ctx, const void *src_host);
+int sofie_cuda_ctx_h2d_quantized(sofie_cuda_ctx *ctx, uint8_t *dst_device, const float *src_host, size_t n, int kind, float scale, int32_t zp, int part);
+/* Lets the helper threads start on the next part (`bytes`: of its destination) while the caller launches the kernels of this one;
+ * nothing is done for pinned memory. The source must stay as it is until that part's copy call, or until
+ * sofie_cuda_ctx_stage_settle, after which no helper reads it. */
+int sofie_cuda_ctx_stage_ahead(sofie_cuda_ctx *ctx, const void *src_host, size_t bytes, int kind, float scale, int32_t zp);
+int sofie_cuda_ctx_stage_settle(sofie_cuda_ctx *ctx);
+/* Self test of that quantisation on plain host memory (needs no GPU). */
+int sofie_cuda_selftest_host_quantize(uint8_t *dst, const float *src, size_t n, int kind, float scale, int32_t zp);
 /* Device -> host; returns after the data has arrived (last statement of the emitted infer(),
  * replaces `return std::vector<float>(tensor_y, tensor_y + n)`,
  * reference: src/SOFIE_core/src/RModel.cxx:717-740). */

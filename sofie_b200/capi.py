@@ -116,6 +116,11 @@ SIGNATURES = {
     "sofie_cuda_ctx_host_output": [vp, sz, C.POINTER(vp)],
     "sofie_cuda_ctx_h2d_part": [vp, vp, vp, sz, C.c_int],
     "sofie_cuda_ctx_wait_part": [vp, C.c_int],
+    "sofie_cuda_ctx_pageable": [vp, vp],
+    "sofie_cuda_ctx_h2d_quantized": [vp, vp, vp, sz, C.c_int, f32, i32, C.c_int],
+    "sofie_cuda_ctx_stage_ahead": [vp, vp, sz, C.c_int, f32, i32],
+    "sofie_cuda_ctx_stage_settle": [vp],
+    "sofie_cuda_selftest_host_quantize": [vp, vp, sz, C.c_int, f32, i32],
     "sofie_cuda_ctx_graph_begin": [vp],
     "sofie_cuda_ctx_graph_end": [vp],
     "sofie_cuda_ctx_graph_launch": [vp],

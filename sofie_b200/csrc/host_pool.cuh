@@ -13,7 +13,7 @@
 
 namespace sofie {
 
-// run() cuts a job into numbered pieces that the caller and the helpers claim one after the other, so a helper that is still
+// A job is cut into numbered pieces that the caller and the helpers claim one after the other, so a helper that is still
 // asleep or was descheduled delays nothing but the piece it holds. A claim carries the job's generation: a helper that comes
 // late finds another generation (or no piece left) and touches nothing of the next job. Helpers spin for half a millisecond
 // after a job (the next one of the same transfer comes within that time, and waking a sleeping thread costs tens of
@@ -37,11 +37,13 @@ public:
    HostPool(const HostPool &) = delete;
    HostPool &operator=(const HostPool &) = delete;
 
-   // fn(arg, i) for every i below `pieces` (at most 2^31), in any order; returns when all are done. One caller at a time.
-   void run(PieceFn fn, void *arg, size_t pieces)
+   // Starts fn(arg, i) for every i below `pieces` (at most 2^31), in any order, on the helpers; `arg` stays valid until
+   // finish(), which takes part in what is left and returns when all is done. One caller at a time, one job at a time.
+   void begin(PieceFn fn, void *arg, size_t pieces)
    {
-      if (threads_.empty() || pieces <= 1) {
-         for (size_t i = 0; i < pieces; i++) fn(arg, i);
+      finish();
+      if (threads_.empty() || pieces <= 1) { // nothing to share: the caller does it in finish()
+         own_fn_ = fn, own_arg_ = arg, own_pieces_ = pieces;
          return;
       }
       // a helper that still holds the last job's ticket must not claim with the new job's piece count: the ticket is closed
@@ -51,15 +53,28 @@ public:
       fn_ = fn, arg_ = arg;
       pieces_.store((uint32_t)pieces, std::memory_order_relaxed);
       done_.store(0, std::memory_order_relaxed);
-      const uint32_t gen = ++generation_;
-      ticket_.store((uint64_t)gen << 32, std::memory_order_seq_cst);
+      open_ = true;
+      ticket_.store((uint64_t)++generation_ << 32, std::memory_order_seq_cst);
       if (sleepers_.load(std::memory_order_seq_cst) > 0) {
          std::lock_guard<std::mutex> lock(mu_);
          wake_.notify_all();
       }
-      claim(gen);
-      while (done_.load(std::memory_order_acquire) != (uint32_t)pieces) relax();
    }
+   void finish()
+   {
+      for (size_t i = 0; i < own_pieces_; i++) own_fn_(own_arg_, i);
+      own_pieces_ = 0;
+      if (!open_) return;
+      claim(generation_);
+      while (done_.load(std::memory_order_acquire) != pieces_.load(std::memory_order_relaxed)) relax();
+      open_ = false;
+   }
+   void run(PieceFn fn, void *arg, size_t pieces)
+   {
+      begin(fn, arg, pieces);
+      finish();
+   }
+   size_t threads() const { return threads_.size() + 1; }
 
    // A copy below kAloneBytes is the caller's alone: two threads' hand-over costs as much as it saves.
    void copy(void *dst, const void *src, size_t bytes)
@@ -119,7 +134,7 @@ private:
             for (int i = 0; i < 32 && !news(); i++) relax();
             if (std::chrono::steady_clock::now() - t0 < std::chrono::microseconds(500)) continue;
             std::unique_lock<std::mutex> lock(mu_);
-            sleepers_.fetch_add(1, std::memory_order_seq_cst); // before the last look: run() reads it after it has published
+            sleepers_.fetch_add(1, std::memory_order_seq_cst); // before the last look: begin() reads it after it has published
             wake_.wait(lock, news);
             sleepers_.fetch_sub(1, std::memory_order_relaxed);
          }
@@ -131,8 +146,10 @@ private:
    std::vector<std::thread> threads_;
    std::mutex mu_;
    std::condition_variable wake_;
-   PieceFn fn_ = nullptr;
-   void *arg_ = nullptr;
+   PieceFn fn_ = nullptr, own_fn_ = nullptr;
+   void *arg_ = nullptr, *own_arg_ = nullptr;
+   size_t own_pieces_ = 0;
+   bool open_ = false;
    std::atomic<uint32_t> pieces_{0};
    uint32_t generation_ = 0;
    std::atomic<uint64_t> ticket_{0}; // generation of the job in the upper half, its next piece in the lower

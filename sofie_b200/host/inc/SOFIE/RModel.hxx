@@ -59,6 +59,8 @@ private:
    bool fNeverPipelinedUpload = false;
    size_t fUploadParts = 4;                  // parts of a pipelined input upload (at most SOFIE_CUDA_MAX_PARTS)
    std::vector<size_t> fSlicedOps;           // operators launched once per uploaded part, in execution order
+   ROperator::StagedQuantization fStaged;    // the input's only reader quantises it: the host can do that while it stages the input
+   size_t fStagedOp = 0;                     // that operator
    size_t fRangeBatch = 0;                   // samples of the batch when every operator can be launched on a range of it, else 0
    size_t fRangeQuantum = 1;                 // such a range starts at a multiple of this many samples
    // Run-time batch: Generate() without a batch size on a model whose inputs carry a batch parameter in their first
@@ -175,6 +177,8 @@ protected:
    void PlanDevice();
    void PlanSlices();
    void PlanRange(size_t head);
+   void PlanStaged();
+   std::string LaunchText(size_t op, const std::string &text) const;
    void GenerateUpload(bool pipelined, const std::string &result, size_t resultLen);
    void PlanArena();
    void GenerateSessionCode();

@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "SOFIE/SOFIE_common.hxx"
+#include "sofie_cuda.h" // SOFIE_CUDA_STAGE_*
 
 namespace SOFIE {
 
@@ -51,6 +52,15 @@ public:
    // text is a launch on `count` samples from sample `part` on, both variables of the emitted code.
    virtual bool CanSliceBatch(size_t /*parts*/) const { return false; }
    virtual std::string GenerateBatchSlice(std::string /*OpName*/, size_t /*parts*/) { return ""; }
+
+   // An operator that only quantises its float input can be taken over by the host's pass over a pageable model input: what that
+   // pass has to produce (kind SOFIE_CUDA_STAGE_*, 0: it cannot)
+   struct StagedQuantization {
+      int kind = 0;
+      float scale = 1.f;
+      int zp = 0;
+   };
+   virtual StagedQuantization GetStagedQuantization() const { return {}; }
 
    const std::vector<std::string> &GetOpInputTensors() const { return fInputTensorNames; }
    const std::vector<std::string> &GetOpOutputTensors() const { return fOutputTensorNames; }

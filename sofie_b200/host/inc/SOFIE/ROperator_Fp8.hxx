@@ -54,6 +54,10 @@ public:
       model.AddIntermediateTensor(fNY, ETensorType::FLOAT8E4M3FN, fShape);
    }
    bool CanSliceBatch(size_t parts) const override { return parts > 0 && !fShape.empty() && fShape[0] % parts == 0; }
+   StagedQuantization GetStagedQuantization() const override
+   {
+      return fInType == ETensorType::FLOAT ? StagedQuantization{SOFIE_CUDA_STAGE_E4M3, fScale, 0} : StagedQuantization{};
+   }
    std::string GenerateBatchSlice(std::string OpName, size_t parts) override { return GenerateCall(OpName, parts); }
    std::string Generate(std::string OpName) override { return GenerateCall(OpName, 1); }
 

@@ -73,6 +73,7 @@ public:
    }
    void PlanDevice(RModel &model) override { model.SetTensorLayout(fNY, model.GetTensorLayout(model.ResolveAlias(fNX))); }
    bool CanSliceBatch(size_t parts) const override { return parts > 0 && !fShape.empty() && fShape[0] % parts == 0; }
+   StagedQuantization GetStagedQuantization() const override { return {SOFIE_CUDA_STAGE_U8, fScale, fZp}; }
    std::string GenerateBatchSlice(std::string OpName, size_t parts) override { return GenerateCall(OpName, parts); }
    std::string Generate(std::string OpName) override { return GenerateCall(OpName, 1); }
 

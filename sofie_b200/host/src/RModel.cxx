@@ -310,6 +310,7 @@ void RModel::Initialize(int batchSize, bool verbose)
       op->Initialize(*this);
    }
    PlanDevice();
+   PlanStaged();
    PlanSlices();
    PlanArena();
    fIsInitialized = true;
@@ -416,6 +417,32 @@ void RModel::PlanDevice()
       head->AbsorbChain(tail);
       for (auto *g : tail) g->SetFusedAway();
    }
+}
+
+// A quantised network's first operator, when it is the only reader of the model's one float input: with that input in pageable
+// memory the host quantises it on its way into pinned memory, the operator's output arrives instead of its input and the
+// operator is not launched.
+void RModel::PlanStaged()
+{
+   fStaged = {};
+   if (fInputTensorNames.size() != 1) return;
+   const std::string &in = fInputTensorNames[0];
+   if (GetTensorType(in) != ETensorType::FLOAT || IsModelOutput(in) || Consumers(in).size() != 1) return;
+   for (size_t i = 0; i < fOperators.size(); i++) {
+      if (fOperators[i]->IsFusedAway()) continue;
+      const auto &reads = fOperators[i]->GetOpInputTensors();
+      if (std::find(reads.begin(), reads.end(), in) != reads.end()) {
+         fStaged = fOperators[i]->GetStagedQuantization();
+         fStagedOp = i;
+      }
+      return; // only the operator that runs first
+   }
+}
+
+// The launch of an operator as it stands in the emitted code: nothing where the host has done its work.
+std::string RModel::LaunchText(size_t op, const std::string &text) const
+{
+   return fStaged.kind && op == fStagedOp ? "   if (!fConverted) {\n" + text + "   }\n" : text;
 }
 
 // Step 4: which operators run once per uploaded part of the input.
@@ -730,6 +757,10 @@ void RModel::GenerateSessionMembers()
       fGC += "size_t fBatch = 0;      // batch of the current / last infer(); the captured graph is the one of this batch\n";
       fGC += "size_t fMaxBatch = 0;   // the batch the Session was constructed for: the arena holds that many samples\n";
    }
+   if (fStaged.kind) {
+      fSessionMembers.push_back("fConverted");
+      fGC += "bool fConverted = false;   // the last input was quantised by the host while it was staged\n";
+   }
    auto pointer = [this](ETensorType type, const std::string &name) {
       fGC += EMIT::CType(type) + " * " + EMIT::Dev(name) + " = nullptr;\n";
       fSessionMembers.push_back(EMIT::Dev(name));
@@ -921,7 +952,7 @@ void RModel::GenerateInfer()
    if (pipelined) {
       fGC += "// the leading operators on one slice of the batch: launched as soon as that slice of the input has arrived\n";
       fGC += "void LaunchHead(int part) {\n";
-      for (size_t i : sliced) fGC += fOperators[i]->GenerateBatchSlice(std::to_string(i), fUploadParts);
+      for (size_t i : sliced) fGC += LaunchText(i, fOperators[i]->GenerateBatchSlice(std::to_string(i), fUploadParts));
       fGC += "}\n\n";
    }
    if (fRangeBatch) {
@@ -929,7 +960,7 @@ void RModel::GenerateInfer()
       fGC += "void LaunchRange(size_t part, size_t count) {\n";
       EMIT::RangeMode() = true;
       for (size_t i = 0; i < fOperators.size(); i++)
-         if (!fOperators[i]->IsFusedAway()) fGC += fOperators[i]->GenerateBatchSlice(std::to_string(i), fRangeBatch);
+         if (!fOperators[i]->IsFusedAway()) fGC += LaunchText(i, fOperators[i]->GenerateBatchSlice(std::to_string(i), fRangeBatch));
       EMIT::RangeMode() = false;
       fGC += "}\n\n";
    }
@@ -942,7 +973,7 @@ void RModel::GenerateInfer()
       if (fOperators[i]->IsFusedAway() || isSliced(i)) continue;
       if (fVerbose) std::cout << "Generating code for operator .... " << i << std::endl;
       fGC += "   Check(sofie_cuda_ctx_mark(fCtx, " + std::to_string(i) + "), \"sofie_cuda_ctx_mark\");\n";
-      fGC += fOperators[i]->Generate(std::to_string(i));
+      fGC += LaunchText(i, fOperators[i]->Generate(std::to_string(i)));
       lastMark = i + 1;
    }
    fGC += "   Check(sofie_cuda_ctx_mark(fCtx, " + std::to_string(lastMark) + "), \"sofie_cuda_ctx_mark\");\n";
@@ -993,6 +1024,11 @@ void RModel::GenerateInfer()
    auto upload = [&] {
       // the graph is captured again when the batch changes
       if (fDynamicBatch) fGC += "   if (" + fBatchParam + " != fBatch) { fBatch = " + fBatchParam + "; fGraphReady = false; }\n";
+      // ... and when the first operator's work moves between the host and the device
+      if (fStaged.kind) {
+         fGC += "   const bool converted = sofie_cuda_ctx_pageable(fCtx, tensor_" + fInputTensorNames[0] + ") != 0;\n";
+         fGC += "   if (converted != fConverted) { fConverted = converted; fGraphReady = false; }\n";
+      }
    };
    const std::string sig = GenerateInferSignature(), args = GenerateInferSignature(false);
    if (nOut != 1) {
@@ -1064,16 +1100,41 @@ void RModel::GenerateInfer()
 // open at its else.
 void RModel::GenerateUpload(bool pipelined, const std::string &result, size_t resultLen)
 {
+   const std::string n = fInputTensorNames.empty() ? std::string() : fInputTensorNames[0];
+   const size_t size = n.empty() ? 0 : GetTypeSize(GetTensorType(n));
+   const std::string how = fStaged.kind ? std::to_string(fStaged.kind) + ", " + EMIT::FloatLit(fStaged.scale) + ", " + std::to_string(fStaged.zp) : "";
+   const std::string q = fStaged.kind ? EMIT::Dev(fOperators[fStagedOp]->GetOpOutputTensors()[0]) : "";
+   // one part: `at` elements from the start, `elems` of them; `next`, `nextElems`: the part behind it, where `more` is true
+   auto part = [&](const std::string &SP, const std::string &copy, const std::string &at, const std::string &elems, const std::string &index, const std::string &more,
+                   const std::string &next, const std::string &nextElems) {
+      if (fStaged.kind) {
+         fGC += SP + "if (fConverted) {\n";
+         fGC += SP + "   Check(sofie_cuda_ctx_h2d_quantized(fCtx, " + q + " + " + at + ", tensor_" + n + " + " + at + ", " + elems + ", " + how + ", " + index +
+                "), \"sofie_cuda_ctx_h2d_quantized\");\n";
+         if (!more.empty())
+            fGC += SP + "   if (" + more + ") Check(sofie_cuda_ctx_stage_ahead(fCtx, tensor_" + n + " + " + next + ", " + nextElems + ", " + how +
+                   "), \"sofie_cuda_ctx_stage_ahead\");\n";
+         fGC += SP + "} else\n";
+      }
+      fGC += SP + copy;
+      if (!fStaged.kind && !more.empty())
+         fGC += SP + "if (" + more + ") Check(sofie_cuda_ctx_stage_ahead(fCtx, tensor_" + n + " + " + next + ", " + nextElems + " * " + std::to_string(size) +
+                ", 0, 1.0f, 0), \"sofie_cuda_ctx_stage_ahead\");\n";
+   };
+   // the helpers read the caller's input ahead of the launches: not beyond this call, whatever ends it
+   const std::string settle = "struct Settle { sofie_cuda_ctx * c; ~Settle() { sofie_cuda_ctx_stage_settle(c); } } settle{fCtx};\n";
    if (pipelined) {
-      const std::string &n = fInputTensorNames[0];
       const size_t elems = ConvertShapeToLength(GetTensorShape(n)) / fUploadParts;
       const std::string parts = std::to_string(fUploadParts), slice = std::to_string(elems);
       // one loop: from pinned memory every call only enqueues (the copy of a part takes far longer than enqueueing the launches
       // behind it, so the copy stream never runs dry); from pageable memory the copy call returns when the part has been staged,
       // and the kernels of that part run while the host stages the next one
+      fGC += "   " + settle;
       fGC += "   for (int part = 0; part < " + parts + "; part++) {\n";
-      fGC += "      Check(sofie_cuda_ctx_h2d_part(fCtx, " + EMIT::Dev(n) + " + (size_t)part * " + slice + ", tensor_" + n + " + (size_t)part * " + slice +
-             ", " + std::to_string(elems * GetTypeSize(GetTensorType(n))) + ", part), \"sofie_cuda_ctx_h2d_part\");\n";
+      part("      ",
+           "Check(sofie_cuda_ctx_h2d_part(fCtx, " + EMIT::Dev(n) + " + (size_t)part * " + slice + ", tensor_" + n + " + (size_t)part * " + slice + ", " +
+              std::to_string(elems * size) + ", part), \"sofie_cuda_ctx_h2d_part\");\n",
+           "(size_t)part * " + slice, slice, "part", "part + 1 < " + parts, "(size_t)(part + 1) * " + slice, slice);
       fGC += "      Check(sofie_cuda_ctx_wait_part(fCtx, part), \"sofie_cuda_ctx_wait_part\");\n";
       fGC += "      LaunchHead(part);\n";
       if (!result.empty()) {
@@ -1085,18 +1146,21 @@ void RModel::GenerateUpload(bool pipelined, const std::string &result, size_t re
       return;
    }
    if (fRangeBatch && resultLen) {
-      const std::string &n = fInputTensorNames[0], &o = fOutputTensorNames[0];
+      const std::string &o = fOutputTensorNames[0];
       const size_t in1 = ConvertShapeToLength(GetTensorShape(n)) / fRangeBatch, out1 = resultLen / fRangeBatch;
-      const size_t inB = in1 * GetTypeSize(GetTensorType(n)), outB = out1 * GetTypeSize(GetTensorType(o));
-      const std::string batch = std::to_string(fRangeBatch), i1 = std::to_string(in1), o1 = std::to_string(out1);
-      fGC += "   const size_t samples = " + batch + ", rows = sofie_cuda_slice_rows(samples, " + std::to_string(inB) + ", " + std::to_string(outB) + ", " +
-             std::to_string(fRangeQuantum) + ");\n";
+      const size_t inB = in1 * size, outB = out1 * GetTypeSize(GetTensorType(o));
+      const std::string i1 = std::to_string(in1), o1 = std::to_string(out1);
+      fGC += "   const size_t samples = " + std::to_string(fRangeBatch) + ", rows = sofie_cuda_slice_rows(samples, " + std::to_string(inB) + ", " + std::to_string(outB) +
+             ", " + std::to_string(fRangeQuantum) + ");\n";
       fGC += "   if (rows < samples) {\n";
       fGC += "      int index = 0;\n";
+      fGC += "      " + settle;
       fGC += "      for (size_t part = 0; part < samples; part += rows, index++) {\n";
-      fGC += "         const size_t count = samples - part < rows ? samples - part : rows;\n";
-      fGC += "         Check(sofie_cuda_ctx_h2d_part(fCtx, " + EMIT::Dev(n) + " + part * " + i1 + ", tensor_" + n + " + part * " + i1 + ", count * " + std::to_string(inB) +
-             ", index), \"sofie_cuda_ctx_h2d_part\");\n";
+      fGC += "         const size_t next = part + rows, count = samples - part < rows ? samples - part : rows;\n";
+      part("         ",
+           "Check(sofie_cuda_ctx_h2d_part(fCtx, " + EMIT::Dev(n) + " + part * " + i1 + ", tensor_" + n + " + part * " + i1 + ", count * " + std::to_string(inB) +
+              ", index), \"sofie_cuda_ctx_h2d_part\");\n",
+           "part * " + i1, "count * " + i1, "index", "next < samples", "next * " + i1, "(samples - next < rows ? samples - next : rows) * " + i1);
       fGC += "         Check(sofie_cuda_ctx_wait_part(fCtx, index), \"sofie_cuda_ctx_wait_part\");\n";
       fGC += "         LaunchRange(part, count);\n";
       fGC += "         Check(sofie_cuda_ctx_result_part(fCtx, " + EMIT::Dev(o) + " + part * " + o1 + ", part * " + std::to_string(outB) + ", count * " + std::to_string(outB) +
@@ -1104,9 +1168,12 @@ void RModel::GenerateUpload(bool pipelined, const std::string &result, size_t re
       fGC += "      }\n";
       return;
    }
-   for (auto &n : fInputTensorNames)
-      fGC += "   Check(sofie_cuda_ctx_h2d(fCtx, " + EMIT::Dev(n) + ", tensor_" + n + ", " + ByteCount(GetTensorShape(n), GetTensorType(n)) +
-             "), \"sofie_cuda_ctx_h2d\");\n";
+   for (auto &in : fInputTensorNames) {
+      const std::string copy = "Check(sofie_cuda_ctx_h2d(fCtx, " + EMIT::Dev(in) + ", tensor_" + in + ", " + ByteCount(GetTensorShape(in), GetTensorType(in)) +
+                               "), \"sofie_cuda_ctx_h2d\");\n";
+      if (fStaged.kind) part("   ", copy, "0", std::to_string(ConvertShapeToLength(GetTensorShape(in))), "-1", "", "", "");
+      else fGC += "   " + copy;
+   }
 }
 
 void RModel::GenerateSessionCode()

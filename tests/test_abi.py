@@ -101,3 +101,32 @@ def test_threaded_host_copy_moves_every_byte(threads):
         capi.call("sofie_cuda_selftest_host_copy", 0, 0, 16, 1 << 20, 1, 1)
     with pytest.raises(RuntimeError):
         capi.call("sofie_cuda_selftest_host_copy", dst.ctypes.data, src.ctypes.data, 16, 1 << 20, 0, 1)
+
+
+@pytest.mark.parametrize("kind,zp", [(1, 0), (1, 128), (1, 255), (2, 0)])
+def test_host_quantisation_gives_the_operators_bytes(kind, zp):
+    """What the host makes of a pageable input while it stages it, against the oracle's QuantizeLinear: every tie and its neighbours, both
+    saturations, infinities, subnormals, lengths around the vector width. A NaN takes the lower bound / the E4M3 NaN."""
+    import numpy as np
+    from oracle import cpu_oracle as o
+    rng = np.random.default_rng(kind)
+    for scale in (0.02, 1.0, 8.0 / 255.0, 3e-3, 1e-30):
+        if kind == 1:
+            ties = (np.arange(-300, 300) + 0.5).astype(np.float32) * np.float32(scale)
+        else:
+            codes = o.e4m3_table()[:127].astype(np.float32)
+            ties = np.concatenate([codes, (codes[1:] + codes[:-1]) / 2]) * np.float32(scale)
+            ties = np.concatenate([ties, -ties])
+        x = np.concatenate([ties, np.nextafter(ties, np.float32(np.inf)), np.nextafter(ties, np.float32(-np.inf)),
+                            np.array([0.0, -0.0, np.inf, -np.inf, 3e38, -3e38, 1e-45, 1e-39], np.float32), (rng.standard_normal(5000) * 100 * scale).astype(np.float32)])
+        want = o.quantize_u8(x, scale, zp) if kind == 1 else o.quantize_e4m3(x, scale)
+        for n in (x.size, 0, 1, 15, 16, 17, 63, 65):
+            y = np.full(n + 64, 0xA5, np.uint8)
+            capi.call("sofie_cuda_selftest_host_quantize", y.ctypes.data, x.ctypes.data, n, kind, scale, zp)
+            assert np.array_equal(y[:n], want[:n]) and (y[n:] == 0xA5).all()
+    nan = np.full(1, np.nan, np.float32)
+    y = np.zeros(1, np.uint8)
+    capi.call("sofie_cuda_selftest_host_quantize", y.ctypes.data, nan.ctypes.data, 1, kind, 1.0, zp)
+    assert y[0] == (0 if kind == 1 else 0x7F)
+    with pytest.raises(RuntimeError):
+        capi.call("sofie_cuda_selftest_host_quantize", y.ctypes.data, nan.ctypes.data, 1, kind, 0.0, zp)
