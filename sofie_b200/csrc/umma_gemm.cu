@@ -819,7 +819,14 @@ static int launch_umma_gemm(cudaStream_t s, const void *A, const void *B, const 
 int launch_gemm_f32_umma(cudaStream_t s, const sofie_gemm_f32_desc &d, const float *A, const float *B, const float *C,
                          float *Y)
 {
-   if (d.transA || !d.transB) return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "tensor-core GEMM takes A[M,K] and B[N,K]");
+   auto aligned = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+   const bool tma = !d.transA && d.transB && d.K % 4 == 0 && aligned(A) && aligned(B); // rows TMA can fetch
+   if (!tma && (long long)d.M * d.N * d.K <= 32768)
+      return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "a product this small of rows TMA cannot fetch is faster on the CUDA cores (3.2 against 3.5 us)");
+   // The kernel below overlaps a tile's epilogue with the next one's MMAs, which pays where a CTA has several tiles and each is short:
+   // 100000 x 10 x 128 20 us against 29, 100000 x 128 x 128 48 against 54. Longer K or fewer tiles are the other kernel's, whose
+   // stages are cheaper and which splits K.
+   if (!tma || d.K >= 1024 || (long long)ceil_div(d.M, umma::kBM) * ceil_div(d.N, 64) < 2 * kNumSMs) return launch_gemm_f32_any(s, d, A, B, C, Y);
    umma::GemmEpilogue ep = {};
    ep.alpha = d.alpha;
    ep.beta = d.beta;

@@ -45,6 +45,30 @@ def test_gemm_f32_3xtf32(M, N, K, bias, relu):
     assert rel_err(y.cpu().numpy(), ref) <= 1e-5
 
 
+# every way an operand can lie (rows of 16-byte multiples or not, K or the rows contiguous, an unaligned base) at the edges of the
+# tiles (32 / 64 / 128 columns, 128 rows, 32 of K), one cluster rank to eight, several tiles per CTA, more than one promoted unit
+@pytest.mark.parametrize("M,N,K,tA,tB,bias", [(129, 33, 31, 0, 1, 1), (127, 31, 33, 1, 0, 2), (128, 64, 32, 1, 1, 0), (200, 65, 4100, 0, 0, 1), (33, 1000, 2501, 1, 1, 1),
+                                              (1, 130, 1025, 0, 1, 2), (1000, 777, 1333, 1, 0, 2), (2500, 1029, 289, 0, 0, 1), (5000, 512, 270, 0, 1, 1),
+                                              (1300, 2050, 515, 1, 0, 1), (40000, 72, 64, 0, 1, 1), (64, 129, 257, 0, 1, 1)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_gemm_f32_any_layout(M, N, K, tA, tB, bias, offset):
+    rng = np.random.default_rng(M + N + K)
+
+    def place(a):     # `offset` floats behind a 16-byte boundary
+        buf = torch.empty(a.size + 4, device="cuda")
+        v = buf[offset: offset + a.size].view(a.shape)
+        v.copy_(torch.from_numpy(a))
+        return v
+    A = rng.standard_normal((K, M) if tA else (M, K)).astype(np.float32)
+    B = rng.standard_normal((N, K) if tB else (K, N)).astype(np.float32)
+    Cb = None if bias == 0 else rng.standard_normal((N,) if bias == 1 else (M, N)).astype(np.float32)
+    ref = o.gemm_f32(A, B, Cb, transA=tA, transB=tB, alpha=1.25, beta=0.5, relu=True)
+    out = place(np.full((M, N), np.nan, np.float32))
+    y = ops.gemm_f32(place(A), place(B), None if Cb is None else place(Cb), transA=tA, transB=tB, alpha=1.25, beta=0.5, relu=True, out=out)
+    assert ops.last_engine() == capi.ENGINE_TCGEN05
+    assert rel_err(y.cpu().numpy(), ref) <= 1e-5
+
+
 def test_gemm_f32_shape_outside_tensor_core_kernel_is_refused_when_forced():
     A, B = torch.zeros((8, 6), device="cuda"), torch.zeros((4, 6), device="cuda")   # K*4 not a multiple of 16
     with pytest.raises(capi.SofieCudaError) as e:
