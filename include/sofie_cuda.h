@@ -132,6 +132,9 @@ int sofie_cuda_host_free(void *host);
  * costs more than the few kilobytes of a classifier's output are worth). Meant for tensors that no kernel
  * reads; the memory is zero-initialised and owned by the context. */
 int sofie_cuda_ctx_host_output(sofie_cuda_ctx *ctx, size_t bytes, void **dptr);
+/* The counterpart for a small input whose one reader loads every element once: it lies in mapped pinned host memory,
+ * sofie_cuda_ctx_h2d of that pointer is a plain store by the host, and the kernel fetches it across PCIe with its other operands. */
+int sofie_cuda_ctx_host_input(sofie_cuda_ctx *ctx, size_t bytes, void **dptr);
 int sofie_cuda_ctx_sync(sofie_cuda_ctx *ctx);
 /* Waits for the context's stream, then reads and clears the context's status word, which a kernel whose
  * bounded wait ran out has set (SOFIE_CUDA_ERR_DEVICE; the kernel itself ended normally and the context

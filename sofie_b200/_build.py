@@ -93,6 +93,92 @@ def _compile_and_link(fp: str, verbose: bool) -> Path:
     return LIB
 
 
+# ---- Python extension modules: the operator calls on torch tensors (over libSOFIE_cuda) and the calls of emitted Sessions ---------
+CSRC_PY = Path(__file__).resolve().parent / "csrc_py"
+OPS_LIB = LIBDIR / "_ops.so"
+SESSION_LIB = LIBDIR / "_session.so"
+
+
+def _build_extension(target: Path, sources: list[Path], tag: str, command) -> Path:
+    """Run command(temporary output) unless `target` is the build of these sources and this tag."""
+    import sysconfig
+    h = hashlib.sha256(f"{tag} {sysconfig.get_config_var('EXT_SUFFIX')}".encode())
+    for p in sources:
+        h.update(p.read_bytes())
+    fp, stamp = h.hexdigest(), target.with_suffix(".stamp")
+
+    def current():
+        return target.exists() and stamp.exists() and stamp.read_text().strip() == fp
+    if current():
+        return target
+    LIBDIR.mkdir(parents=True, exist_ok=True)
+    with open(LIBDIR / f".{target.stem}.lock", "a+") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        try:
+            if current():
+                return target
+            tmp = target.with_name(f".{target.name}.{os.getpid()}.tmp")
+            r = subprocess.run(command(tmp), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+            if r.returncode != 0:
+                tmp.unlink(missing_ok=True)
+                raise RuntimeError(f"building {target.name} failed:\n{r.stdout}")
+            os.replace(tmp, target)
+            stamp.write_text(fp)
+            return target
+        finally:
+            fcntl.flock(lock, fcntl.LOCK_UN)
+
+
+def build_ops() -> Path:
+    """csrc_py/ops_native.cpp against the installed torch (headers and libraries) and libSOFIE_cuda."""
+    import torch
+    lib = build()
+    src = CSRC_PY / "ops_native.cpp"
+
+    def command(out):
+        import sysconfig
+        from torch.utils import cpp_extension
+        cuda = Path(_nvcc()).resolve().parent.parent
+        inc = [*cpp_extension.include_paths(), str(cuda / "include"), sysconfig.get_paths()["include"], str(ROOT / "include")]
+        libs = cpp_extension.library_paths()
+        return ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+                *[f for d in inc for f in ("-isystem", d)], str(src), "-o", str(out), *[f"-L{d}" for d in libs], f"-L{lib.parent}",
+                "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-lSOFIE_cuda", "-Wl,-rpath,$ORIGIN",
+                *[f"-Wl,-rpath,{d}" for d in libs]]
+    return _build_extension(OPS_LIB, [src, ROOT / "include" / "sofie_cuda.h"], torch.__version__, command)
+
+
+def build_session() -> Path:
+    """csrc_py/session_native.c: Python's headers alone."""
+    import sysconfig
+    src = CSRC_PY / "session_native.c"
+    return _build_extension(SESSION_LIB, [src], "", lambda out: ["gcc", "-O2", "-fPIC", "-shared", "-I", sysconfig.get_paths()["include"], str(src), "-o", str(out)])
+
+
+_loaded = {}
+
+
+def _load_extension(name: str, build_it):
+    if name not in _loaded:
+        import importlib.machinery
+        import importlib.util
+        path = str(build_it())
+        spec = importlib.util.spec_from_file_location(name, path, loader=importlib.machinery.ExtensionFileLoader(name, path))
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _loaded[name] = module
+    return _loaded[name]
+
+
+def load_ops():
+    """The operator calls (built first when absent or stale); torch is imported before them, libSOFIE_cuda with them."""
+    return _load_extension("_ops", build_ops)
+
+
+def load_session():
+    return _load_extension("_session", build_session)
+
+
 if __name__ == "__main__":
     import sys
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))

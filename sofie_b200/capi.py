@@ -114,6 +114,7 @@ SIGNATURES = {
     "sofie_cuda_ctx_mark": [vp, C.c_int],
     "sofie_cuda_ctx_timers_read": [vp, vp, C.c_int, C.POINTER(C.c_int)],
     "sofie_cuda_ctx_host_output": [vp, sz, C.POINTER(vp)],
+    "sofie_cuda_ctx_host_input": [vp, sz, C.POINTER(vp)],
     "sofie_cuda_ctx_h2d_part": [vp, vp, vp, sz, C.c_int],
     "sofie_cuda_ctx_wait_part": [vp, C.c_int],
     "sofie_cuda_ctx_pageable": [vp, vp],

@@ -4,6 +4,8 @@
 // emits for each operator (cited per case), evaluated in the same precision.
 #include "common.cuh"
 
+#include <utility>
+
 namespace sofie {
 namespace {
 
@@ -17,9 +19,10 @@ inline int act_grid(size_t items)
    return blocks ? (int)blocks : 1;
 }
 
-__device__ __forceinline__ float unary_apply(int op, float x, float alpha)
+template <int OP>
+__device__ __forceinline__ float unary_apply(float x, float alpha)
 {
-   switch (op) {
+   switch (OP) {
    case SOFIE_UNARY_SIGMOID: return __fdiv_rn(1.f, __fadd_rn(1.f, expf(-x)));          // ROperator_Sigmoid.hxx:59
    case SOFIE_UNARY_TANH: return tanhf(x);                                             // ROperator_Tanh.hxx:60
    case SOFIE_UNARY_LEAKY_RELU: return x >= 0.f ? x : __fmul_rn(alpha, x);             // ROperator_LeakyRelu.hxx:73
@@ -41,17 +44,28 @@ __device__ __forceinline__ float unary_apply(int op, float x, float alpha)
    }
 }
 
-__global__ void unary_f32_kernel(int op, float alpha, const float *__restrict__ X, float *__restrict__ Y, size_t n, bool vec)
+template <int OP>
+__global__ void __launch_bounds__(kActThreads) unary_f32_kernel(float alpha, const float *__restrict__ X, float *__restrict__ Y, size_t n, bool vec)
 {
+   griddep_launch_dependents();
+   griddep_wait(); // X is the previous kernel's output
    const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nthreads = (size_t)gridDim.x * blockDim.x;
    const size_t n4 = vec ? n / 4 : 0;
 #pragma unroll 2
    for (size_t i = tid; i < n4; i += nthreads) {
       const float4 v = reinterpret_cast<const float4 *>(X)[i];
       reinterpret_cast<float4 *>(Y)[i] =
-         make_float4(unary_apply(op, v.x, alpha), unary_apply(op, v.y, alpha), unary_apply(op, v.z, alpha), unary_apply(op, v.w, alpha));
+         make_float4(unary_apply<OP>(v.x, alpha), unary_apply<OP>(v.y, alpha), unary_apply<OP>(v.z, alpha), unary_apply<OP>(v.w, alpha));
    }
-   for (size_t i = n4 * 4 + tid; i < n; i += nthreads) Y[i] = unary_apply(op, X[i], alpha);
+   for (size_t i = n4 * 4 + tid; i < n; i += nthreads) Y[i] = unary_apply<OP>(X[i], alpha);
+}
+
+using UnaryKernel = void (*)(float, const float *, float *, size_t, bool);
+template <int... OP>
+UnaryKernel unary_kernel(int op, std::integer_sequence<int, OP...>)
+{
+   static constexpr UnaryKernel table[] = {unary_f32_kernel<OP>...};
+   return table[op];
 }
 
 __device__ __forceinline__ float binary_apply(int op, float a, float b)
@@ -67,6 +81,8 @@ __device__ __forceinline__ float binary_apply(int op, float a, float b)
 __global__ void binary_same_f32_kernel(int op, const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ Y, size_t n,
                                        bool vec)
 {
+   griddep_launch_dependents();
+   griddep_wait();
    const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nthreads = (size_t)gridDim.x * blockDim.x;
    const size_t n4 = vec ? n / 4 : 0;
 #pragma unroll 2
@@ -78,11 +94,81 @@ __global__ void binary_same_f32_kernel(int op, const float *__restrict__ A, cons
    for (size_t i = n4 * 4 + tid; i < n; i += nthreads) Y[i] = binary_apply(op, A[i], B[i]);
 }
 
-// General form: the output index is split into up to four coordinates; a broadcast dimension of an
-// operand has stride 0.
-__global__ void binary_bcast_f32_kernel(sofie_binary_desc d, const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ Y,
-                                        size_t n)
+// Broadcasting. The dimensions are merged as far as both operands allow (an [N,C,H,W] tensor and a [C,1,1] one become [N,C,HW]); a
+// thread writes four consecutive outputs. An operand that lies like the output is read as one 16-byte word, the other by
+// coordinates: those of the first output by multiplications (FastDiv), the next ones by counting on. Measured on [512,16,64,64]
+// times [16,1,1]: 250 us with four 64-bit divisions per element, 43 us here (a copy of the bytes takes 41).
+struct BcastDims {
+   FastDiv shape[4]; // innermost first
+   uint32_t a[4], b[4];
+};
+template <bool A_DENSE, bool B_DENSE>
+__global__ void __launch_bounds__(kActThreads) binary_bcast_f32_kernel(BcastDims d, int op, const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ Y,
+                                                                      uint32_t n, bool vec)
 {
+   griddep_launch_dependents();
+   griddep_wait();
+   const uint32_t nthreads = gridDim.x * blockDim.x;
+   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += nthreads * 4) {
+      uint32_t c[4], rem = i, ao = 0, bo = 0;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+         if (k < 3) rem = d.shape[k].divmod(rem, c[k]);
+         else c[k] = rem;
+         if (!A_DENSE) ao += c[k] * d.a[k];
+         if (!B_DENSE) bo += c[k] * d.b[k];
+      }
+      const bool full = vec && i + 4 <= n;
+      float a[4], b[4], y[4];
+      if (A_DENSE && full) {
+         const float4 v = *reinterpret_cast<const float4 *>(A + i);
+         a[0] = v.x, a[1] = v.y, a[2] = v.z, a[3] = v.w;
+      }
+      if (B_DENSE && full) {
+         const float4 v = *reinterpret_cast<const float4 *>(B + i);
+         b[0] = v.x, b[1] = v.y, b[2] = v.z, b[3] = v.w;
+      }
+      if (full && c[0] + 4 <= d.shape[0].d && (A_DENSE || d.a[0] == 0) && (B_DENSE || d.b[0] == 0)) {
+         // one run of the innermost dimension, along which the broadcast operand stands still
+         if (!A_DENSE) a[0] = a[1] = a[2] = a[3] = A[ao];
+         if (!B_DENSE) b[0] = b[1] = b[2] = b[3] = B[bo];
+      } else {
+#pragma unroll
+         for (int j = 0; j < 4; j++) {
+            if (i + j >= n) break;
+            if (A_DENSE ? !full : true) a[j] = A[A_DENSE ? i + j : ao];
+            if (B_DENSE ? !full : true) b[j] = B[B_DENSE ? i + j : bo];
+            // the next coordinate: one step along the innermost dimension, carried outwards
+            ao += d.a[0], bo += d.b[0];
+            c[0]++;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+               if (c[k] != d.shape[k].d) break;
+               ao += d.a[k + 1] - c[k] * d.a[k];
+               bo += d.b[k + 1] - c[k] * d.b[k];
+               c[k] = 0;
+               c[k + 1]++;
+            }
+         }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) y[j] = binary_apply(op, a[j], b[j]);
+      if (full) {
+         *reinterpret_cast<float4 *>(Y + i) = make_float4(y[0], y[1], y[2], y[3]);
+      } else {
+#pragma unroll
+         for (int j = 0; j < 4; j++)
+            if (i + j < n) Y[i + j] = y[j];
+      }
+   }
+}
+
+// The same without the limit of 2^31 elements: the output index is split into up to four coordinates; a broadcast dimension of an
+// operand has stride 0.
+__global__ void binary_bcast_large_f32_kernel(sofie_binary_desc d, const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ Y, size_t n)
+{
+   griddep_launch_dependents();
+   griddep_wait();
    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
       size_t rem = i, ao = 0, bo = 0;
 #pragma unroll
@@ -98,13 +184,62 @@ __global__ void binary_bcast_f32_kernel(sofie_binary_desc d, const float *__rest
 
 // y = ((x - mean[c]) * scale[c]) + bias[c], optional Relu; the three steps are separate roundings as
 // in the emitted scopy / saxpy / multiply / saxpy sequence (ROperator_BatchNormalization.hxx:200-226).
-__global__ void batchnorm_f32_kernel(sofie_batchnorm_desc d, const float *__restrict__ X, const float *__restrict__ scale,
-                                     const float *__restrict__ bias, const float *__restrict__ mean, float *__restrict__ Y, size_t n)
+__device__ __forceinline__ float batchnorm_apply(float x, float mean, float scale, float bias, int relu)
 {
+   const float y = __fadd_rn(__fmul_rn(__fsub_rn(x, mean), scale), bias);
+   return relu ? relu_ref(y) : y;
+}
+
+// Four consecutive elements per thread. `inner` elements in a row share a channel (HW, or 1 with the channels innermost). Measured
+// on [512,16,64,64]: 116 us with 64-bit divisions per element, 42 us here.
+__global__ void __launch_bounds__(kActThreads) batchnorm_f32_kernel(FastDiv inner, FastDiv channels, const float *__restrict__ X, const float *__restrict__ scale,
+                                                                   const float *__restrict__ bias, const float *__restrict__ mean, float *__restrict__ Y, uint32_t n, int relu, bool vec)
+{
+   griddep_launch_dependents();
+   griddep_wait();
+   const uint32_t nthreads = gridDim.x * blockDim.x;
+   for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += nthreads * 4) {
+      uint32_t in, c;
+      channels.divmod(inner.divmod(i, in), c);
+      const bool full = vec && i + 4 <= n;
+      float x[4] = {};
+      if (full) {
+         const float4 v = *reinterpret_cast<const float4 *>(X + i);
+         x[0] = v.x, x[1] = v.y, x[2] = v.z, x[3] = v.w;
+      }
+      if (full && in + 4 <= inner.d) {
+         const float m = mean[c], s = scale[c], b = bias[c];
+#pragma unroll
+         for (int j = 0; j < 4; j++) x[j] = batchnorm_apply(x[j], m, s, b, relu);
+      } else {
+#pragma unroll
+         for (int j = 0; j < 4; j++) {
+            if (i + j >= n) break;
+            if (!full) x[j] = X[i + j];
+            x[j] = batchnorm_apply(x[j], mean[c], scale[c], bias[c], relu);
+            if (++in == inner.d) {
+               in = 0;
+               if (++c == channels.d) c = 0;
+            }
+         }
+      }
+      if (full) {
+         *reinterpret_cast<float4 *>(Y + i) = make_float4(x[0], x[1], x[2], x[3]);
+      } else {
+#pragma unroll
+         for (int j = 0; j < 4; j++)
+            if (i + j < n) Y[i + j] = x[j];
+      }
+   }
+}
+__global__ void batchnorm_large_f32_kernel(sofie_batchnorm_desc d, const float *__restrict__ X, const float *__restrict__ scale,
+                                           const float *__restrict__ bias, const float *__restrict__ mean, float *__restrict__ Y, size_t n)
+{
+   griddep_launch_dependents();
+   griddep_wait();
    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
       const int c = d.layout == SOFIE_LAYOUT_NHWC ? (int)(i % (size_t)d.C) : (int)((i / (size_t)d.HW) % (size_t)d.C);
-      float y = __fadd_rn(__fmul_rn(__fsub_rn(X[i], mean[c]), scale[c]), bias[c]);
-      Y[i] = d.relu ? relu_ref(y) : y;
+      Y[i] = batchnorm_apply(X[i], mean[c], scale[c], bias[c], d.relu);
    }
 }
 
@@ -121,8 +256,8 @@ extern "C" int sofie_cuda_unary_f32(void *stream, int32_t op, float alpha, const
    if (n == 0) return SOFIE_CUDA_OK;
    SOFIE_REQUIRE(X && Y, "NULL tensor");
    const bool vec = aligned16(X) && aligned16(Y);
-   unary_f32_kernel<<<act_grid(vec ? n / 4 + 1 : n), kActThreads, 0, as_stream(stream)>>>(op, alpha, X, Y, n, vec);
-   SOFIE_LAUNCH_CHECK("unary_f32_kernel");
+   const UnaryKernel kernel = unary_kernel(op, std::make_integer_sequence<int, SOFIE_UNARY_SIN + 1>());
+   SOFIE_CUDA_TRY(launch_dependent(kernel, dim3(act_grid(vec ? n / 4 + 1 : n)), dim3(kActThreads), 0, as_stream(stream), alpha, X, Y, n, vec));
    return SOFIE_CUDA_OK;
 }
 
@@ -144,11 +279,37 @@ extern "C" int sofie_cuda_binary_f32(void *stream, const sofie_binary_desc *d, c
    cudaStream_t s = as_stream(stream);
    if (same) {
       const bool vec = aligned16(A) && aligned16(B) && aligned16(Y);
-      binary_same_f32_kernel<<<act_grid(vec ? n / 4 + 1 : n), kActThreads, 0, s>>>(d->op, A, B, Y, n, vec);
-   } else {
-      binary_bcast_f32_kernel<<<act_grid(n), kActThreads, 0, s>>>(*d, A, B, Y, n);
+      SOFIE_CUDA_TRY(launch_dependent(binary_same_f32_kernel, dim3(act_grid(vec ? n / 4 + 1 : n)), dim3(kActThreads), 0, s, d->op, A, B, Y, n, vec));
+      return SOFIE_CUDA_OK;
    }
-   SOFIE_LAUNCH_CHECK("binary_f32_kernel");
+   if (n >= (size_t(1) << 31) - 4096 * 1024) {
+      SOFIE_CUDA_TRY(launch_dependent(binary_bcast_large_f32_kernel, dim3(act_grid(n)), dim3(kActThreads), 0, s, *d, A, B, Y, n));
+      return SOFIE_CUDA_OK;
+   }
+   // merge dimensions, innermost first: the next one continues the current one where both operands' strides do
+   BcastDims b;
+   int64_t shape[4] = {1, 1, 1, 1}, as[4] = {}, bs[4] = {};
+   int dims = 0;
+   for (int k = 3; k >= 0; k--) {
+      if (d->shape[k] == 1) continue;
+      if (dims && d->a_stride[k] == as[dims - 1] * shape[dims - 1] && d->b_stride[k] == bs[dims - 1] * shape[dims - 1]) {
+         shape[dims - 1] *= d->shape[k];
+         continue;
+      }
+      shape[dims] = d->shape[k], as[dims] = d->a_stride[k], bs[dims] = d->b_stride[k];
+      dims++;
+   }
+   bool a_dense = true, b_dense = true;
+   int64_t run = 1;
+   for (int k = 0; k < 4; k++) {
+      b.shape[k] = FastDiv((uint32_t)shape[k]);
+      b.a[k] = (uint32_t)as[k], b.b[k] = (uint32_t)bs[k];
+      if (k < dims) a_dense = a_dense && as[k] == run, b_dense = b_dense && bs[k] == run;
+      run *= shape[k];
+   }
+   const bool vec = aligned16(Y) && (!a_dense || aligned16(A)) && (!b_dense || aligned16(B));
+   auto kernel = a_dense ? binary_bcast_f32_kernel<true, false> : (b_dense ? binary_bcast_f32_kernel<false, true> : binary_bcast_f32_kernel<false, false>);
+   SOFIE_CUDA_TRY(launch_dependent(kernel, dim3(act_grid(n / 4 + 1)), dim3(kActThreads), 0, s, b, d->op, A, B, Y, (uint32_t)n, vec));
    return SOFIE_CUDA_OK;
 }
 
@@ -161,7 +322,12 @@ extern "C" int sofie_cuda_batchnorm_f32(void *stream, const sofie_batchnorm_desc
    const size_t n = (size_t)d->N * d->C * d->HW;
    if (n == 0) return SOFIE_CUDA_OK;
    SOFIE_REQUIRE(X && Y && scale && bias && mean, "NULL tensor");
-   batchnorm_f32_kernel<<<act_grid(n), kActThreads, 0, as_stream(stream)>>>(*d, X, scale, bias, mean, Y, n);
-   SOFIE_LAUNCH_CHECK("batchnorm_f32_kernel");
+   if (n >= (size_t(1) << 31) - 4096 * 1024) {
+      SOFIE_CUDA_TRY(launch_dependent(batchnorm_large_f32_kernel, dim3(act_grid(n)), dim3(kActThreads), 0, as_stream(stream), *d, X, scale, bias, mean, Y, n));
+      return SOFIE_CUDA_OK;
+   }
+   const FastDiv inner(d->layout == SOFIE_LAYOUT_NHWC ? 1 : (uint32_t)d->HW), channels((uint32_t)d->C);
+   SOFIE_CUDA_TRY(launch_dependent(batchnorm_f32_kernel, dim3(act_grid(n / 4 + 1)), dim3(kActThreads), 0, as_stream(stream), inner, channels, X, scale, bias, mean, Y,
+                                   (uint32_t)n, d->relu, aligned16(X) && aligned16(Y)));
    return SOFIE_CUDA_OK;
 }

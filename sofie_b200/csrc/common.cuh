@@ -88,6 +88,47 @@ __host__ __device__ constexpr T ceil_div(T a, T b)
    return (a + b - 1) / b;
 }
 
+// ---- division of 32-bit indices by a number known at launch ---------------------------------------
+// q = floor(n / d) for n < 2^31 as one multiplication and a shift: with p = 31 + ceil(log2 d) and m = ceil(2^p / d), which fits in
+// 32 bits, floor(n * m / 2^p) is exact (round-up method).
+struct FastDiv {
+   uint32_t d = 1, m = 0, s = 0;
+   FastDiv() = default;
+   explicit FastDiv(uint32_t divisor) : d(divisor)
+   {
+      if (d <= 1) return; // n / 1: no multiplication
+      uint32_t log = 0;
+      while ((uint64_t(1) << log) < d) log++;
+      m = (uint32_t)(((uint64_t(1) << (31 + log)) + d - 1) / d);
+      s = log - 1;
+   }
+   __device__ __forceinline__ uint32_t div(uint32_t n) const { return d <= 1 ? n : __umulhi(n, m) >> s; }
+   __device__ __forceinline__ uint32_t divmod(uint32_t n, uint32_t &rem) const
+   {
+      const uint32_t q = div(n);
+      rem = n - q * d;
+      return q;
+   }
+};
+
+// Dynamic shared memory above 48 KB has to be allowed per kernel and device once; the launchers call this on every launch.
+inline cudaError_t allow_smem(const void *kernel, int bytes)
+{
+   struct Done {
+      const void *kernel = nullptr;
+      int device = -1, bytes = 0;
+   };
+   static thread_local Done table[128];
+   int dev = 0;
+   cudaError_t err = cudaGetDevice(&dev);
+   if (err != cudaSuccess) return err;
+   Done &e = table[(reinterpret_cast<uintptr_t>(kernel) >> 4) % 128];
+   if (e.kernel == kernel && e.device == dev && e.bytes >= bytes) return cudaSuccess;
+   err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+   if (err == cudaSuccess) e = {kernel, dev, bytes};
+   return err;
+}
+
 // ---- requantisation recipe shared by every int8 kernel -------------------------------------------
 // q = clamp(rne((float)acc * mult), qmin - zp, qmax - zp) + zp, with no FMA contraction, so a CPU
 // evaluating nearbyintf((float)acc * mult) under the default rounding mode gets the same bits.

@@ -89,7 +89,7 @@ public:
       run(copy_piece, &job, (bytes + job.piece - 1) / job.piece);
    }
 
-   static constexpr size_t kAloneBytes = size_t(192) << 10;
+   static constexpr size_t kAloneBytes = size_t(96) << 10;
    static constexpr size_t kPieceBytes = size_t(256) << 10;
 
 private:

@@ -203,7 +203,7 @@ int launch_conv_direct(cudaStream_t s, const ConvGeom &g, const TX *X, const TW 
    size_t smem = (size_t)cg * g.kH * g.kW * kConvOCB * sizeof(TW);
    if (smem > 200 * 1024) return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "convolution weights slice of %zu bytes exceeds shared memory", smem);
    auto kern = conv2d_direct_kernel<TX, TW, TACC, TY, Epi>;
-   if (smem > 48 * 1024) SOFIE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+   if (smem > 48 * 1024) SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), (int)smem));
    size_t positions = (size_t)g.N * g.pH * g.pW;
    if (positions == 0) return SOFIE_CUDA_OK;
    int gy = g.group * ceil_div(og, kConvOCB);

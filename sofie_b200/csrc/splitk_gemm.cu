@@ -109,32 +109,33 @@ __global__ void gemm_f32_splitk_reduce_kernel(sofie_gemm_f32_desc d, int splits,
 // the two launches of the split-K pair and its scratch round trip cost more than the arithmetic.
 // four rows per block measured best inside the C2 step (72.3 us against 73.7 with two and 74.8 with eight)
 constexpr int kRowBlockRows = 4;
-constexpr int kRowBlockMaxRows = 2048; // beyond this B would be re-read from L2 too often: split-K instead
+// Larger batches with up to ten columns: eight rows per block halve what is read of B out of L2
+constexpr int kRowBlockManyRows = 8, kRowBlockManyFrom = 2048, kRowBlockManyMaxN = 10;
 
-template <int NN>
+template <int NN, int ROWS>
 __global__ void __launch_bounds__(256)
 gemm_f32_rowblock_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, const float *__restrict__ B, const float *__restrict__ C,
                          float *__restrict__ Y)
 {
-   __shared__ float s_part[8][kRowBlockRows][NN];
+   __shared__ float s_part[8][ROWS][NN];
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-   const int m0 = blockIdx.x * kRowBlockRows, K = d.K;
+   const int m0 = blockIdx.x * ROWS, K = d.K;
    griddep_launch_dependents();
    griddep_wait(); // A is the previous kernel's output
-   float acc[kRowBlockRows][NN];
+   float acc[ROWS][NN];
 #pragma unroll
-   for (int r = 0; r < kRowBlockRows; r++)
+   for (int r = 0; r < ROWS; r++)
 #pragma unroll
       for (int n = 0; n < NN; n++) acc[r][n] = 0.f;
-   const float *arow[kRowBlockRows];
+   const float *arow[ROWS];
 #pragma unroll
-   for (int r = 0; r < kRowBlockRows; r++) arow[r] = A + (size_t)min(m0 + r, d.M - 1) * K; // rows past M repeat the last one, not stored
+   for (int r = 0; r < ROWS; r++) arow[r] = A + (size_t)min(m0 + r, d.M - 1) * K; // rows past M repeat the last one, not stored
    for (int k = threadIdx.x * 4; k < K; k += 1024) {
       float4 b[NN];
 #pragma unroll
       for (int n = 0; n < NN; n++) b[n] = __ldg(reinterpret_cast<const float4 *>(B + (size_t)n * K + k));
 #pragma unroll
-      for (int r = 0; r < kRowBlockRows; r++) {
+      for (int r = 0; r < ROWS; r++) {
          const float4 a = *reinterpret_cast<const float4 *>(arow[r] + k);
 #pragma unroll
          for (int n = 0; n < NN; n++) {
@@ -146,7 +147,7 @@ gemm_f32_rowblock_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, con
       }
    }
 #pragma unroll
-   for (int r = 0; r < kRowBlockRows; r++)
+   for (int r = 0; r < ROWS; r++)
 #pragma unroll
       for (int n = 0; n < NN; n++) {
          float v = acc[r][n];
@@ -155,8 +156,8 @@ gemm_f32_rowblock_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, con
          if (lane == 0) s_part[warp][r][n] = v;
       }
    __syncthreads();
-   if (threadIdx.x < kRowBlockRows * NN) {
-      const int r = threadIdx.x / NN, n = threadIdx.x - r * NN, m = m0 + r;
+   for (int i = threadIdx.x; i < ROWS * NN; i += 256) {
+      const int r = i / NN, n = i - r * NN, m = m0 + r;
       if (m < d.M) {
          float sum = 0.f;
 #pragma unroll
@@ -172,21 +173,29 @@ gemm_f32_rowblock_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, con
 bool rowblock_shape_ok(const sofie_gemm_f32_desc &d, const float *A, const float *B)
 {
    static const bool enabled = [] { const char *e = getenv("SOFIE_CUDA_GEMM_ROWBLOCK"); return !e || atoi(e) != 0; }();
-   return enabled && !d.transA && d.transB && d.N <= kSplitKMaxN && d.K >= 1024 && d.K % 4 == 0 && d.M <= kRowBlockMaxRows &&
+   return enabled && !d.transA && d.transB && d.N <= kSplitKMaxN && d.K >= 1024 && d.K % 4 == 0 && d.M <= (d.N <= 4 ? (1 << 30) : (d.N <= kRowBlockManyMaxN ? 5000 : kRowBlockManyFrom)) &&
           (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0;
 }
 
 int launch_gemm_f32_rowblock(cudaStream_t s, const sofie_gemm_f32_desc &d, const float *A, const float *B, const float *C, float *Y)
 {
    if (!rowblock_shape_ok(d, A, B)) return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "not a row-block GEMM shape");
-   const dim3 grid(ceil_div(d.M, kRowBlockRows)), block(256);
-#define SOFIE_ROWBLOCK(NN) \
-   case NN: SOFIE_CUDA_TRY(launch_dependent(gemm_f32_rowblock_kernel<NN>, grid, block, 0, s, d, A, B, C, Y)); break
+   const bool many = d.M > kRowBlockManyFrom;
+   const dim3 grid(ceil_div(d.M, many ? kRowBlockManyRows : kRowBlockRows)), block(256);
+#define SOFIE_ROWBLOCK(NN)                                                                                                              \
+   case NN:                                                                                                                             \
+      if constexpr (NN <= kRowBlockManyMaxN) {                                                                                          \
+         if (many) {                                                                                                                    \
+            SOFIE_CUDA_TRY(launch_dependent(gemm_f32_rowblock_kernel<NN, kRowBlockManyRows>, grid, block, 0, s, d, A, B, C, Y));       \
+            break;                                                                                                                      \
+         }                                                                                                                              \
+      }                                                                                                                                 \
+      SOFIE_CUDA_TRY(launch_dependent(gemm_f32_rowblock_kernel<NN, kRowBlockRows>, grid, block, 0, s, d, A, B, C, Y));                 \
+      break
    switch (d.N) {
       SOFIE_ROWBLOCK(1); SOFIE_ROWBLOCK(2); SOFIE_ROWBLOCK(3); SOFIE_ROWBLOCK(4); SOFIE_ROWBLOCK(5); SOFIE_ROWBLOCK(6);
       SOFIE_ROWBLOCK(7); SOFIE_ROWBLOCK(8); SOFIE_ROWBLOCK(9); SOFIE_ROWBLOCK(10); SOFIE_ROWBLOCK(11); SOFIE_ROWBLOCK(12);
-      SOFIE_ROWBLOCK(13); SOFIE_ROWBLOCK(14); SOFIE_ROWBLOCK(15);
-   default: SOFIE_CUDA_TRY(launch_dependent(gemm_f32_rowblock_kernel<16>, grid, block, 0, s, d, A, B, C, Y)); break;
+      SOFIE_ROWBLOCK(13); SOFIE_ROWBLOCK(14); SOFIE_ROWBLOCK(15); SOFIE_ROWBLOCK(16);
    }
 #undef SOFIE_ROWBLOCK
    set_last_engine(SOFIE_ENGINE_SIMT);

@@ -871,7 +871,7 @@ static int launch_conv_patch(cudaStream_t s, const ConvGeom &g, const void *X, c
    if (!status) return fail(SOFIE_CUDA_ERR_CUDA, "cannot allocate the device status word");
    const int grid = tg.num_tiles < kNumSMs ? tg.num_tiles : kNumSMs;
    auto kern = umma_conv3x3_patch_kernel<KIND, BN, KPS, G>;
-   SOFIE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+   SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), smem));
    SOFIE_CUDA_TRY(launch_dependent(kern, dim3(grid), dim3(kPatchThreads<KIND>), smem, s, tmX, tmW, ep, tg, pl, status));
    SOFIE_LAUNCH_CHECK("umma_conv3x3_patch_kernel");
    set_last_engine(SOFIE_ENGINE_TCGEN05);
@@ -931,7 +931,7 @@ static int launch_conv_tps_rw(cudaStream_t s, const CUtensorMap &tmX, const CUte
    tg.stages = stages;
    const int smem = w_bytes + stages * STAGE_BYTES + 1024;
    auto kern = umma_conv3x3_kernel<KIND, BN, CB, TPS, RW>;
-   SOFIE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+   SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), smem));
    uint32_t *status = device_status_word(s);
    if (!status) return fail(SOFIE_CUDA_ERR_CUDA, "cannot allocate the device status word");
    const int grid = tg.num_tiles < kNumSMs ? tg.num_tiles : kNumSMs;

@@ -567,7 +567,7 @@ int launch_first_pool_conv(cudaStream_t s, const ConvGeom &g, const uint8_t *X, 
    if (!status) return fail(SOFIE_CUDA_ERR_CUDA, "cannot allocate the device status word");
    const int grid = p.num_tiles < kNumSMs ? p.num_tiles : kNumSMs;
    auto kern = umma_qconv3x3_first_pool_kernel<BN>;
-   SOFIE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+   SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), smem));
    SOFIE_CUDA_TRY(launch_dependent(kern, dim3(grid), dim3(kFirstThreads), smem, s, tmX, W, p, status));
    SOFIE_LAUNCH_CHECK("umma_qconv3x3_first_pool_kernel");
    set_last_engine(SOFIE_ENGINE_TCGEN05);
@@ -608,7 +608,7 @@ int launch_pool_conv(cudaStream_t s, const ConvGeom &g, const uint8_t *X, const 
    if (!status) return fail(SOFIE_CUDA_ERR_CUDA, "cannot allocate the device status word");
    const int grid = p.num_tiles < kNumSMs ? p.num_tiles : kNumSMs;
    auto kern = umma_qconv3x3_pool_kernel<BN, KPS>;
-   SOFIE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+   SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), smem));
    SOFIE_CUDA_TRY(launch_dependent(kern, dim3(grid), dim3(kPoolThreads), smem, s, tmX, tmW, p, status));
    SOFIE_LAUNCH_CHECK("umma_qconv3x3_pool_kernel");
    set_last_engine(SOFIE_ENGINE_TCGEN05);

@@ -5,9 +5,9 @@
 //   * sixteen worker warps read the operands themselves, split them in registers and write the hi / lo tiles where the MMA's
 //     swizzled K-major descriptors expect them. A unit of work is four consecutive K of one row: one 16-byte load, four scalar loads
 //     (rows that are not 16-byte multiples), or four loads of consecutive rows (K is not the contiguous dimension), always one
-//     conflict-free 16-byte store per tile. Two groups of eight warps take the stages alternately: while one splits and stores, the
-//     other's loads are in flight (one group with two stages of loads in flight was bound by their latency: 2500 clocks a stage).
-//     The same warps add the partial sums up in registers and write the tile.
+//     conflict-free 16-byte store per tile. Groups of them take the stages in turn: while one splits and stores, the others' loads
+//     are in flight (one group with two stages of loads in flight was bound by their latency: 2500 clocks a stage). The same warps
+//     add the partial sums up in registers and write the tile.
 //   * B's hi and lo tiles lie side by side as one operand of twice the width: A_hi x [B_hi | B_lo] and A_lo x B_hi are two MMAs per
 //     K step instead of three, with a sixth less shared memory read.
 //   * a cluster of S CTAs shares one output tile: each takes a S-th of K, leaves its partial tile in shared memory, and adds up and
@@ -26,8 +26,10 @@ namespace {
 
 constexpr int kAnyBM = 128;             // rows of the tile = TMEM lanes
 constexpr int kAnyKE = 32;              // floats of K per stage = one 128-byte swizzle row
-constexpr int kAnyGroups = 2, kAnyGroupWarps = 8;
-constexpr int kAnyWorkers = kAnyGroups * kAnyGroupWarps * 32;
+constexpr int kAnyWorkers = 16 * 32;
+// Groups of worker warps that take the stages in turn. Four were 5 to 10 % faster at 32 columns with a long K and as much slower with a
+// short one (the pipeline takes longer to start), and spilled at 64 columns.
+constexpr int kAnyGroups = 2;
 constexpr int kAnyThreads = kAnyWorkers + 32; // and the warp that issues the MMAs
 constexpr int kAnyPromote = 8;          // stages accumulated in one TMEM buffer: 256 elements of K
 constexpr int kAnyMaxStages = 5;
@@ -60,15 +62,15 @@ __device__ __forceinline__ void any_split(float x, float &h, float &l)
 }
 
 // One thread's share of the tiles of an operand with R rows: U units, a unit being K chunk `c` (four floats) of row `r`.
-//   K contiguous: eight lanes cover the 128 bytes of one row; the thread's units are 32 rows apart, in the same chunk.
-//   Rows contiguous: lanes cover consecutive rows; the thread's units are in one row, 256 / R chunks apart.
+//   K contiguous: eight lanes cover the 128 bytes of one row; the thread's units are T / 8 rows apart, in the same chunk.
+//   Rows contiguous: lanes cover consecutive rows; the thread's units are in one row, T / R chunks apart (T threads per group).
 // Either way the 16-byte stores of eight lanes fall into eight different bank groups, and everything that depends on the thread is
 // worked out once per tile: the loops below are a load, an addition and the split per unit (with the addresses taken from the unit
 // number the loaders were bound by instruction issue).
-template <int R>
+template <int R, int T>
 struct AnyLoader {
-   static constexpr int U = R * 8 / (kAnyGroupWarps * 32);
-   static constexpr int kChunkStep = kAnyGroupWarps * 32 / R; // rows contiguous: chunks between the units of a thread
+   static constexpr int U = R * 8 / T;
+   static constexpr int kRowStep = T / 8, kChunkStep = T / R; // between the units of a thread
    const float *p = nullptr; // the thread's first element at K = 0 of the tile
    uint32_t at = 0;          // byte offset of its first unit in the tile
    uint32_t ok = 0;          // bit i: the row of unit i exists
@@ -89,7 +91,7 @@ struct AnyLoader {
          const int r = row0 + (t >> 3);
          ok = 0;
 #pragma unroll
-         for (int i = 0; i < U; i++) ok |= (r + 32 * i < o.rows ? 1u : 0u) << i;
+         for (int i = 0; i < U; i++) ok |= (r + kRowStep * i < o.rows ? 1u : 0u) << i;
          p = o.p + (long long)r * o.ld + 4 * (t & 7);
       }
    }
@@ -111,7 +113,7 @@ struct AnyLoader {
          }
       } else {
          const float *q = p + k0;
-         const long long step = 32 * o.ld;
+         const long long step = kRowStep * o.ld;
          const int left = kend - k0 - 4 * (t & 7);
          if (o.mode == kVecK) { // K % 4 == 0 and kend % 4 == 0
 #pragma unroll
@@ -136,8 +138,8 @@ struct AnyLoader {
    {
 #pragma unroll
       for (int i = 0; i < U; i++) {
-         // units 32 rows apart keep their place in the swizzle pattern; chunks kChunkStep apart flip its upper bits
-         const uint32_t off = o.mode == kRowsContiguous ? (at ^ (uint32_t)(i * kChunkStep * 16)) : (at + (uint32_t)(i * 32 * 128));
+         // units a multiple of 8 rows apart keep their place in the swizzle pattern; chunks kChunkStep apart flip its upper bits
+         const uint32_t off = o.mode == kRowsContiguous ? (at ^ (uint32_t)(i * kChunkStep * 16)) : (at + (uint32_t)(i * kRowStep * 128));
          float4 h, l;
          any_split(v[i].x, h.x, l.x);
          any_split(v[i].y, h.y, l.y);
@@ -225,6 +227,7 @@ __global__ void __launch_bounds__(kAnyThreads, 1)
 umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, uint32_t *status)
 {
    using L = AnySmem<BN>;
+   constexpr int G = kAnyGroups, GT = kAnyWorkers / G; // groups and their threads
    constexpr int QUARTER = BN / 4;       // columns of the tile a worker warp adds up
    constexpr uint32_t TMEM_COLS = 4 * BN; // two buffers of [hi x hi | the cross terms]
    extern __shared__ unsigned char smem_raw[];
@@ -252,7 +255,7 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
 
    if (threadIdx.x == 0) {
       for (int s = 0; s < L::kStages; s++) {
-         mbar_init(&full_bar[s], kAnyGroupWarps);
+         mbar_init(&full_bar[s], GT / 32);
          mbar_init(&empty_bar[s], 1);
       }
       for (int b = 0; b < 2; b++) {
@@ -274,14 +277,14 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
 
    if (warp < kAnyWorkers / 32) {
       // ---------------- workers ----------------
-      const int group = warp / kAnyGroupWarps, t = threadIdx.x - group * (kAnyGroupWarps * 32);
+      const int group = threadIdx.x / GT, t = threadIdx.x % GT;
       const int lane_base = (warp & 3) * 32, col_base = (warp >> 2) * QUARTER;
       const uint32_t t_row = tmem_base + ((uint32_t)lane_base << 16) + (uint32_t)col_base;
-      AnyLoader<kAnyBM> la;
-      AnyLoader<BN> lb;
+      AnyLoader<kAnyBM, GT> la;
+      AnyLoader<BN, GT> lb;
       la.place(A, t);
       lb.place(B, t);
-      // Stages are numbered through all tiles of this CTA; the group's own are every other one. `lt`, `lk`: the stage whose loads are
+      // Stages are numbered through all tiles of this CTA; the group's own are every G-th. `lt`, `lk`: the stage whose loads are
       // issued next; g: the stage the group stores next.
       int lt = tile0, lk = group, placed = -1;
       auto load = [&] {
@@ -297,7 +300,7 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
          }
          la.load(A, (kb0 + lk) * kAnyKE, kend, t);
          lb.load(B, (kb0 + lk) * kAnyKE, kend, t);
-         lk += kAnyGroups;
+         lk += G;
       };
       load();
       int g = group, s = group % L::kStages, u = 0, first = 0; // first: number of the current tile's first stage
@@ -328,7 +331,7 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
             u++;
          };
          int unit = 0; // units of this tile already added up
-         for (; g < first + kbn; g += kAnyGroups) {
+         for (; g < first + kbn; g += G) {
             // the partial sum of a unit is collected a ring's length after its last stage was stored: its MMAs are done by then
             if (g - first >= (unit + 1) * kAnyPromote + L::kStages) {
                promote();
@@ -343,7 +346,7 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
                if (lane == 0) mbar_arrive(&full_bar[s]);
             }
             load();
-            for (int i = 0; i < kAnyGroups; i++) ring_next(s, ph, L::kStages);
+            for (int i = 0; i < G; i++) ring_next(s, ph, L::kStages);
          }
          for (; unit < units; unit++) promote();
          workers_sync(); // all units added up: the tile's MMAs are done and its stages free
@@ -413,13 +416,7 @@ int launch_any(cudaStream_t s, const AnyOperand &A, const AnyOperand &B, const A
 {
    using L = AnySmem<BN>;
    auto kern = umma_gemm_any_kernel<BN>;
-   static thread_local int configured = -1; // the device this thread last set the attribute on
-   int dev = 0;
-   SOFIE_CUDA_TRY(cudaGetDevice(&dev));
-   if (configured != dev) {
-      SOFIE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes));
-      configured = dev;
-   }
+   SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), L::kBytes));
    uint32_t *status = device_status_word(s);
    if (!status) return fail(SOFIE_CUDA_ERR_CUDA, "cannot allocate the device status word");
    const int tiles = ceil_div(A.rows, kAnyBM) * ceil_div(B.rows, BN);

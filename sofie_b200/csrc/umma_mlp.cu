@@ -437,7 +437,7 @@ int launch_mlp_f32_umma(cudaStream_t s, const sofie_mlp_desc *d, const float *X,
    const int grid = slabs < kNumSMs ? slabs : kNumSMs;
    const int x_vec = d->dims[0] % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
    auto kern = umma_mlp_kernel;
-   SOFIE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+   SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), smem));
    SOFIE_CUDA_TRY(launch_dependent(kern, dim3(grid), dim3(kMlpTcThreads), smem, s, pl, X, Y, x_vec, status));
    SOFIE_LAUNCH_CHECK("umma_mlp_kernel");
    set_last_engine(SOFIE_ENGINE_TCGEN05);

@@ -239,6 +239,8 @@ class _ResultArrays:
         self.lock = threading.Lock()
 
     def new(self, n: int, dtype) -> np.ndarray:
+        if n * 8 < self.kPinnedFrom:
+            return np.empty(n, dtype)
         dtype = np.dtype(dtype)
         nbytes = n * dtype.itemsize
         if nbytes < self.kPinnedFrom:
@@ -345,9 +347,18 @@ class GeneratedSession:
             raise RuntimeError(self.err.value.decode())
         self.out_elems, self.out_dtype = out_elems, out_dtype
         self.results = _ResultArrays()
+        self._call = _build.load_session().infer
+        self._infer = C.cast(self.lib.sofie_session_infer, C.c_void_p).value
+        self._err = C.addressof(self.err)
 
     def infer(self, x, out: np.ndarray | None = None) -> np.ndarray:
         """x: one array, or a list of arrays for a model with several inputs (in the order of infer())."""
+        if type(x) is np.ndarray and x.flags.c_contiguous:
+            y = out if out is not None else self.results.new(self.out_elems, self.out_dtype)
+            n = self._call(self._infer, self.handle, x, y, self.out_elems, self._err, 1024)
+            if n != self.out_elems:
+                raise RuntimeError(f"infer failed ({n}): {self.err.value.decode()}")
+            return y
         xs = [np.ascontiguousarray(a) for a in (x if isinstance(x, (list, tuple)) else [x])]
         ptrs = (C.c_void_p * max(1, len(xs)))(*[a.ctypes.data for a in xs])
         y = out if out is not None else self.results.new(self.out_elems, self.out_dtype)

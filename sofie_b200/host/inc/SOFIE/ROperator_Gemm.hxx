@@ -74,6 +74,7 @@ public:
       return fPlainInput && fNBdev != fNB && fAttrAlpha == 1.f && !fAttrTransA && (fBiasKind == 0 || (fBiasKind == 1 && fAttrBeta == 1.f)) &&
              fK <= 256 && fN <= 256 && fM <= kMlpFusedMaxRows && fShapeA.size() == 2 && fStack == 1;
    }
+   bool IsChain() const { return !fChain.empty(); }
    void AbsorbChain(const std::vector<ROperator_Gemm<T> *> &tail)
    {
       fChain = tail;

@@ -11,7 +11,7 @@ import ctypes as C
 import numpy as np
 import torch
 
-from . import capi
+from . import _build, capi
 from .capi import LAYOUT_NCHW, LAYOUT_NHWC
 
 
@@ -26,6 +26,18 @@ def _p(t) -> C.c_void_p:
     return C.c_void_p(t.data_ptr())
 
 
+_module = None
+
+
+def _native():
+    """The extension module with the calls that are made often (csrc_py/ops_native.cpp); the others below go through ctypes."""
+    global _module
+    if _module is None:
+        capi.load()
+        _module = _build.load_ops()
+    return _module
+
+
 def set_engine(engine: int) -> None:
     capi.call("sofie_cuda_set_engine", engine)
 
@@ -36,18 +48,7 @@ def last_engine() -> int:
 
 def gemm_f32(A, B, C_=None, *, transA=0, transB=0, alpha=1.0, beta=1.0, relu=False, out=None):
     """ONNX Gemm / MatMul: Y = alpha*op(A)*op(B) + beta*broadcast(C), optional Relu."""
-    M = A.shape[1] if transA else A.shape[0]
-    K = A.shape[0] if transA else A.shape[1]
-    N = B.shape[0] if transB else B.shape[1]
-    assert (B.shape[1] if transB else B.shape[0]) == K
-    bias_kind = 0
-    if C_ is not None:
-        bias_kind = 1 if C_.numel() == N else 2
-        assert C_.numel() in (N, M * N)
-    Y = out if out is not None else torch.empty((M, N), dtype=torch.float32, device=A.device)
-    d = capi.GemmF32Desc(M, N, K, int(transA), int(transB), float(alpha), float(beta), bias_kind, int(relu))
-    capi.call("sofie_cuda_gemm_f32", _stream(), C.byref(d), _p(A), _p(B), _p(C_), _p(Y))
-    return Y
+    return _native().gemm_f32(A, B, C_, transA, transB, alpha, beta, relu, out)
 
 
 def conv_out_hw(H, W, kH, kW, pad, stride, dil=(1, 1)):
@@ -59,20 +60,7 @@ def conv_out_hw(H, W, kH, kW, pad, stride, dil=(1, 1)):
 def conv2d_f32(X, W, bias=None, *, shape=None, pad=(0, 0), stride=(1, 1), dil=(1, 1), group=1, relu=False, pool=0,
                x_layout=LAYOUT_NCHW, y_layout=LAYOUT_NCHW, w_packed=False, kernel=None, out=None):
     """ONNX Conv (+Relu, +MaxPool 2x2). `shape` = (N, C, H, W) of the logical input."""
-    N, Cin, H, Wd = shape if shape is not None else X.shape
-    if w_packed:
-        Cout, kH, kW = W.shape[0], kernel[0], kernel[1]
-    else:
-        Cout, kH, kW = W.shape[0], W.shape[2], W.shape[3]
-    oH, oW = conv_out_hw(H, Wd, kH, kW, pad, stride, dil)
-    if pool == 2:
-        oH, oW = oH // 2, oW // 2
-    yshape = (N, oH, oW, Cout) if y_layout == LAYOUT_NHWC else (N, Cout, oH, oW)
-    Y = out if out is not None else torch.empty(yshape, dtype=torch.float32, device=X.device)
-    d = capi.Conv2dDesc(N, Cin, H, Wd, Cout, kH, kW, pad[0], pad[1], stride[0], stride[1], dil[0], dil[1], group,
-                        x_layout, y_layout, int(w_packed), int(relu), pool)
-    capi.call("sofie_cuda_conv2d_f32", _stream(), C.byref(d), _p(X), _p(W), _p(bias), _p(Y))
-    return Y
+    return _native().conv2d_f32(X, W, bias, shape, pad, stride, dil, group, relu, pool, x_layout, y_layout, w_packed, kernel, out)
 
 
 def conv2d_pack_f32(W):
@@ -84,22 +72,12 @@ def conv2d_pack_f32(W):
 
 
 def relu_f32(X, out=None):
-    Y = out if out is not None else torch.empty_like(X)
-    capi.call("sofie_cuda_relu_f32", _stream(), _p(X), _p(Y), X.numel())
-    return Y
+    return _native().relu_f32(X, out)
 
 
 def pool2d_f32(X, *, mode=0, kernel=(2, 2), stride=(2, 2), pads=(0, 0, 0, 0), count_include_pad=0,
                layout=LAYOUT_NCHW, shape=None):
-    N, Cc, H, W = shape if shape is not None else X.shape
-    oH = -(-(H + pads[0] + pads[2] - kernel[0] + 1) // stride[0])
-    oW = -(-(W + pads[1] + pads[3] - kernel[1] + 1) // stride[1])
-    yshape = (N, oH, oW, Cc) if layout == LAYOUT_NHWC else (N, Cc, oH, oW)
-    Y = torch.empty(yshape, dtype=torch.float32, device=X.device)
-    d = capi.Pool2dDesc(mode, N, Cc, H, W, kernel[0], kernel[1], stride[0], stride[1], (capi.i32 * 4)(*pads),
-                        count_include_pad, layout)
-    capi.call("sofie_cuda_pool2d_f32", _stream(), C.byref(d), _p(X), _p(Y))
-    return Y
+    return _native().pool2d_f32(X, mode, kernel, stride, pads, count_include_pad, layout, shape)
 
 
 def pool3d_f32(X, *, mode=0, kernel=(2, 2, 2), stride=(2, 2, 2), pads=(0, 0, 0, 0, 0, 0), count_include_pad=0):
@@ -124,12 +102,7 @@ def conv3d_f32(X, W, bias=None, *, pad=(0, 0, 0), stride=(1, 1, 1), dil=(1, 1, 1
 
 
 def softmax_f32(X, axis=-1):
-    axis = axis % X.dim()
-    outer = int(np.prod(X.shape[:axis], dtype=np.int64))
-    inner = int(np.prod(X.shape[axis + 1:], dtype=np.int64))
-    Y = torch.empty_like(X)
-    capi.call("sofie_cuda_softmax_f32", _stream(), _p(X), _p(Y), outer, X.shape[axis], inner)
-    return Y
+    return _native().softmax_f32(X, axis)
 
 
 def conv_transpose2d_f32(X, W, bias=None, pad=(0, 0), stride=(1, 1), dil=(1, 1), out_pad=(0, 0), relu=False, product_form=False):
@@ -224,59 +197,24 @@ BINARY_OPS = {"Add": 0, "Sub": 1, "Mul": 2, "Div": 3}
 
 
 def unary_f32(X, op, alpha=0.0):
-    Y = torch.empty_like(X)
-    capi.call("sofie_cuda_unary_f32", _stream(), UNARY_OPS[op], float(alpha), _p(X), _p(Y), X.numel())
-    return Y
-
-
-def binary_strides(a_shape, b_shape):
-    """Output shape and the rank-4 shape / element strides (0 along broadcast dimensions) of A op B."""
-    out = tuple(torch.broadcast_shapes(tuple(a_shape), tuple(b_shape)))
-    if len(out) > 4:
-        raise ValueError("binary operators are built for rank <= 4")
-
-    def strides(shape):
-        shape = (1,) * (len(out) - len(shape)) + tuple(shape)
-        st, dense = [], 1
-        for d in reversed(shape):
-            st.append(0 if d == 1 else dense)
-            dense *= d
-        return [0] * (4 - len(out)) + list(reversed(st))
-
-    return out, [1] * (4 - len(out)) + list(out), strides(a_shape), strides(b_shape)
+    return _native().unary_f32(X, UNARY_OPS[op], alpha)
 
 
 def binary_f32(A, B, op):
-    out, shape4, sa, sb = binary_strides(A.shape, B.shape)
-    Y = torch.empty(out, dtype=torch.float32, device=A.device)
-    i64 = C.c_int64 * 4
-    d = capi.BinaryDesc(BINARY_OPS[op], i64(*shape4), i64(*sa), i64(*sb))
-    capi.call("sofie_cuda_binary_f32", _stream(), C.byref(d), _p(A), _p(B), _p(Y))
-    return Y
+    return _native().binary_f32(A, B, BINARY_OPS[op])
 
 
 def batchnorm_f32(X, scale, bias, mean, N, Cc, HW, layout=LAYOUT_NCHW, relu=False):
     """scale is the folded gamma / sqrt(var + eps)."""
-    Y = torch.empty_like(X)
-    d = capi.BatchNormDesc(N, Cc, HW, layout, int(relu))
-    capi.call("sofie_cuda_batchnorm_f32", _stream(), C.byref(d), _p(X), _p(scale), _p(bias), _p(mean), _p(Y))
-    return Y
+    return _native().batchnorm_f32(X, scale, bias, mean, N, Cc, HW, layout, relu)
 
 
 def nchw_to_nhwc(X):
-    N, Cc, H, W = X.shape
-    Y = torch.empty((N, H, W, Cc), dtype=X.dtype, device=X.device)
-    fn = "sofie_cuda_nchw_to_nhwc_f32" if X.dtype == torch.float32 else "sofie_cuda_nchw_to_nhwc_u8"
-    capi.call(fn, _stream(), _p(X), _p(Y), N, Cc, H, W)
-    return Y
+    return _native().change_layout(X, True)
 
 
 def nhwc_to_nchw(X):
-    N, H, W, Cc = X.shape
-    Y = torch.empty((N, Cc, H, W), dtype=X.dtype, device=X.device)
-    fn = "sofie_cuda_nhwc_to_nchw_f32" if X.dtype == torch.float32 else "sofie_cuda_nhwc_to_nchw_u8"
-    capi.call(fn, _stream(), _p(X), _p(Y), N, Cc, H, W)
-    return Y
+    return _native().change_layout(X, False)
 
 
 def transpose2d(X):
@@ -289,15 +227,11 @@ def transpose2d(X):
 
 # ---------------------------------------------------------------- int8 -------------------------
 def quantize_u8(X, scale, zp):
-    Y = torch.empty(X.shape, dtype=torch.uint8, device=X.device)
-    capi.call("sofie_cuda_quantize_u8", _stream(), _p(X), _p(Y), X.numel(), float(scale), int(zp))
-    return Y
+    return _native().quantize_u8(X, scale, zp)
 
 
 def dequantize_u8(X, scale, zp):
-    Y = torch.empty(X.shape, dtype=torch.float32, device=X.device)
-    capi.call("sofie_cuda_dequantize_u8", _stream(), _p(X), _p(Y), X.numel(), float(scale), int(zp))
-    return Y
+    return _native().dequantize_u8(X, scale, zp)
 
 
 def qlinear_prepare(W_host: np.ndarray, w_is_nk: bool, a_scale, a_zp, w_scale_host: np.ndarray, y_scale,
@@ -322,40 +256,17 @@ def qlinear_prepare(W_host: np.ndarray, w_is_nk: bool, a_scale, a_zp, w_scale_ho
 
 
 def qlinear_matmul(A, W, mult, corr, *, w_is_nk=True, y_zp=0, relu=False):
-    M, K = A.shape
-    N = W.shape[0] if w_is_nk else W.shape[1]
-    Y = torch.empty((M, N), dtype=torch.uint8, device=A.device)
-    d = capi.QGemmDesc(M, N, K, int(w_is_nk), int(y_zp), int(relu))
-    capi.call("sofie_cuda_qlinear_matmul", _stream(), C.byref(d), _p(A), _p(W), _p(mult), _p(corr), _p(Y))
-    return Y
+    return _native().qlinear_matmul(A, W, mult, corr, w_is_nk, y_zp, relu, None)
 
 
 def qlinear_matmul_f32(A, W, mult, corr, y_scale, *, w_is_nk=True, y_zp=0, relu=False):
     """QLinearMatMul + DequantizeLinear (same zero point) in one pass: float32 (q - y_zp) * y_scale."""
-    M, K = A.shape
-    N = W.shape[0] if w_is_nk else W.shape[1]
-    Y = torch.empty((M, N), dtype=torch.float32, device=A.device)
-    d = capi.QGemmDesc(M, N, K, int(w_is_nk), int(y_zp), int(relu))
-    capi.call("sofie_cuda_qlinear_matmul_f32", _stream(), C.byref(d), _p(A), _p(W), _p(mult), _p(corr), float(y_scale), _p(Y))
-    return Y
+    return _native().qlinear_matmul(A, W, mult, corr, w_is_nk, y_zp, relu, y_scale)
 
 
 def qlinear_conv2d(X, W, mult, bias=None, *, shape=None, pad=(0, 0), stride=(1, 1), x_zp=0, y_zp=0, relu=False,
                    pool=0, x_layout=LAYOUT_NCHW, y_layout=LAYOUT_NCHW, w_packed=False, kernel=None):
-    N, Cin, H, Wd = shape if shape is not None else X.shape
-    if w_packed:
-        Cout, kH, kW = W.shape[0], kernel[0], kernel[1]
-    else:
-        Cout, kH, kW = W.shape[0], W.shape[2], W.shape[3]
-    oH, oW = conv_out_hw(H, Wd, kH, kW, pad, stride)
-    if pool == 2:
-        oH, oW = oH // 2, oW // 2
-    yshape = (N, oH, oW, Cout) if y_layout == LAYOUT_NHWC else (N, Cout, oH, oW)
-    Y = torch.empty(yshape, dtype=torch.uint8, device=X.device)
-    d = capi.QConv2dDesc(N, Cin, H, Wd, Cout, kH, kW, pad[0], pad[1], stride[0], stride[1], x_layout, y_layout,
-                         int(w_packed), int(x_zp), int(y_zp), int(relu), pool)
-    capi.call("sofie_cuda_qlinear_conv2d", _stream(), C.byref(d), _p(X), _p(W), _p(mult), _p(bias), _p(Y))
-    return Y
+    return _native().qlinear_conv2d(X, W, mult, bias, shape, pad, stride, x_zp, y_zp, relu, pool, x_layout, y_layout, w_packed, kernel)
 
 
 def qconv2d_pack_i8(W):
@@ -367,24 +278,12 @@ def qconv2d_pack_i8(W):
 
 
 def maxpool2d_u8(X, *, kernel=(2, 2), stride=(2, 2), layout=LAYOUT_NCHW, shape=None):
-    N, Cc, H, W = shape if shape is not None else X.shape
-    oH, oW = (H - kernel[0]) // stride[0] + 1, (W - kernel[1]) // stride[1] + 1
-    yshape = (N, oH, oW, Cc) if layout == LAYOUT_NHWC else (N, Cc, oH, oW)
-    Y = torch.empty(yshape, dtype=torch.uint8, device=X.device)
-    capi.call("sofie_cuda_maxpool2d_u8", _stream(), _p(X), _p(Y), N, Cc, H, W, kernel[0], kernel[1], stride[0],
-              stride[1], layout)
-    return Y
+    return _native().maxpool2d_u8(X, kernel, stride, layout, shape)
 
 
 # ---------------------------------------------------------------- FP8 --------------------------
 def quantize_e4m3(X, scale):
-    Y = torch.empty(X.shape, dtype=torch.uint8, device=X.device)
-    if X.dtype == torch.float32:
-        capi.call("sofie_cuda_quantize_e4m3_f32", _stream(), _p(X), _p(Y), X.numel(), float(scale))
-    else:
-        assert X.dtype in (torch.bfloat16, torch.uint16, torch.int16)
-        capi.call("sofie_cuda_quantize_e4m3_bf16", _stream(), _p(X), _p(Y), X.numel(), float(scale))
-    return Y
+    return _native().quantize_e4m3(X, scale)
 
 
 def cast_bf16_f32(X):
@@ -407,20 +306,9 @@ def amax_f32(X):
 
 def gemm_e4m3(A, W, bias=None, *, a_scale=1.0, w_scale=1.0, relu=False, q_scale=0.0, want_bf16=True):
     """A [M,K] and W [N,K] are uint8 tensors holding E4M3 codes. Returns (bf16 Y or None, E4M3 Yq or None)."""
-    M, K = A.shape
-    N = W.shape[0]
-    Y = torch.empty((M, N), dtype=torch.bfloat16, device=A.device) if want_bf16 else None
-    Yq = torch.empty((M, N), dtype=torch.uint8, device=A.device) if q_scale > 0 else None
-    d = capi.Fp8GemmDesc(M, N, K, float(a_scale), float(w_scale), int(relu), float(q_scale))
-    capi.call("sofie_cuda_gemm_e4m3", _stream(), C.byref(d), _p(A), _p(W), _p(bias), _p(Y), _p(Yq))
-    return Y, Yq
+    return _native().gemm_e4m3(A, W, bias, a_scale, w_scale, relu, q_scale, want_bf16, False)
 
 
 def gemm_e4m3_f32(A, W, bias=None, *, a_scale=1.0, w_scale=1.0, relu=False):
     """The FP8 product with the bf16-rounded result written as float32 (Fp8Gemm + Cast in one pass)."""
-    M, K = A.shape
-    N = W.shape[0]
-    Y = torch.empty((M, N), dtype=torch.float32, device=A.device)
-    d = capi.Fp8GemmDesc(M, N, K, float(a_scale), float(w_scale), int(relu), 0.0)
-    capi.call("sofie_cuda_gemm_e4m3_f32", _stream(), C.byref(d), _p(A), _p(W), _p(bias), _p(Y))
-    return Y
+    return _native().gemm_e4m3(A, W, bias, a_scale, w_scale, relu, 0.0, True, True)

@@ -688,3 +688,62 @@ def test_many_contexts_one_after_another_share_the_splitk_scratch_pool():
     finally:
         for ctx in alive:
             capi.call("sofie_cuda_ctx_destroy", ctx)
+
+
+@pytest.mark.parametrize("a,b,op", [((3, 5, 7, 9), (5, 1, 1), "Mul"), ((2, 16, 8, 12), (16, 1, 1), "Add"), ((4, 6, 5), (5,), "Sub"), ((33, 1), (1, 47), "Div"),
+                                    ((1, 3, 1, 5), (4, 1, 6, 1), "Add"), ((7, 130), (7, 1), "Mul"), ((2, 3, 4, 5), (2, 1, 4, 1), "Sub"), ((1,), (257, 3), "Mul"),
+                                    ((513, 8), (1, 8), "Div")])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_broadcast_shapes_and_unaligned_tensors(a, b, op, offset):
+    """Merged dimensions, runs that end inside a thread's four outputs, either operand dense, none dense, an unaligned base."""
+    rng = np.random.default_rng(len(a) * 10 + len(b))
+
+    def place(shape):
+        x = rng.uniform(0.5, 2.0, shape).astype(np.float32)
+        buf = torch.empty(x.size + 4, device="cuda")
+        v = buf[offset: offset + x.size].view(shape)
+        v.copy_(torch.from_numpy(x))
+        return x, v
+    xa, va = place(a)
+    xb, vb = place(b)
+    want = {"Add": np.add, "Sub": np.subtract, "Mul": np.multiply, "Div": np.divide}[op](xa, xb)
+    got = ops.binary_f32(va, vb, op).cpu().numpy()
+    assert got.shape == want.shape and np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
+@pytest.mark.parametrize("N,C,H,W", [(1, 1, 1, 1), (3, 1, 7, 9), (2, 3, 51, 67), (5, 3, 6, 6), (2, 24, 9, 13), (1, 64, 33, 31), (300, 16, 4, 4), (2, 65, 5, 7), (40000, 2, 1, 3), (2, 33, 64, 64)])
+@pytest.mark.parametrize("dtype", ["f32", "u8"])
+def test_layout_change_of_every_channel_count(N, C, H, W, dtype):
+    rng = np.random.default_rng(N + C)
+    x = rng.standard_normal((N, C, H, W)).astype(np.float32) if dtype == "f32" else rng.integers(0, 256, (N, C, H, W)).astype(np.uint8)
+    y = ops.nchw_to_nhwc(dev(x))
+    assert np.array_equal(y.cpu().numpy(), x.transpose(0, 2, 3, 1))
+    assert np.array_equal(ops.nhwc_to_nchw(y).cpu().numpy(), x)
+
+
+@pytest.mark.parametrize("N,C,HW,layout,relu", [(3, 5, 63, 0, 1), (2, 16, 64, 0, 0), (5, 7, 1, 0, 1), (4, 6, 35, 1, 0), (1, 1, 5, 0, 0), (3, 130, 6, 1, 1)])
+def test_batchnorm_channels_that_change_inside_four_elements(N, C, HW, layout, relu):
+    rng = np.random.default_rng(N * C)
+    x = rng.standard_normal((N, C, HW) if layout == 0 else (N, HW, C)).astype(np.float32)
+    s, b, m = (rng.standard_normal(C).astype(np.float32) for _ in range(3))
+    ax = (slice(None), None) if layout == 0 else (slice(None),)
+    want = ((x - m[ax]) * s[ax]) + b[ax]
+    want = np.where(want > 0, want, np.float32(0)) if relu else want
+    got = ops.batchnorm_f32(dev(x), dev(s), dev(b), dev(m), N, C, HW, layout=layout, relu=bool(relu)).cpu().numpy()
+    assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("rows,n", [(5, 33), (300, 77), (7, 129), (9, 385), (4, 1001), (3, 1025), (2, 2049), (1000, 127)])
+def test_softmax_rows_of_every_length_class(rows, n):
+    x = np.random.default_rng(n).standard_normal((rows, n)).astype(np.float32) * 3
+    assert rel_err(ops.softmax_f32(dev(x)).cpu().numpy(), o.softmax_f32(x, axis=-1)) <= FP32_TOL
+
+
+@pytest.mark.parametrize("shape,k,s,pads,mode", [((2, 3, 7, 9), 2, 2, (0, 0, 0, 0), 0), ((2, 3, 7, 9), 2, 2, (1, 1, 1, 1), 1), ((1, 5, 51, 67), 2, 2, (0, 0, 0, 0), 1), ((3, 4, 6, 5), 3, 1, (1, 1, 1, 1), 0)])
+def test_pool2d_odd_images(shape, k, s, pads, mode):
+    x = np.random.default_rng(k).standard_normal(shape).astype(np.float32)
+    want = o.pool2d_f32(x, mode=mode, kernel=(k, k), stride=(s, s), pads=pads)
+    for layout in (0, 1):
+        t = dev(x if layout == 0 else x.transpose(0, 2, 3, 1))
+        got = ops.pool2d_f32(t, mode=mode, kernel=(k, k), stride=(s, s), pads=pads, layout=layout, shape=shape).cpu().numpy()
+        assert rel_err(got if layout == 0 else got.transpose(0, 3, 1, 2), want) <= FP32_TOL
