@@ -152,6 +152,33 @@ __device__ __forceinline__ int requant_u8(int acc, float mult, int y_zp, int rel
    return __float_as_int(__fadd_rn(v, 12582912.f)) - 0x4B400000 + y_zp;
 }
 
+// ---- two fp32 values per instruction, each rounded as by the scalar one ------------------------
+__device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi)
+{
+   uint64_t v;
+   asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+   return v;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b)
+{
+   uint64_t v;
+   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+   return v;
+}
+__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b)
+{
+   uint64_t v;
+   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+   return v;
+}
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c)
+{
+   uint64_t v;
+   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+   return v;
+}
+
 __device__ __forceinline__ float relu_ref(float v)
 {
    // The reference's `x > 0 ? x : 0`: NaN and -0 both become +0.

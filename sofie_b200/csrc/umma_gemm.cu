@@ -143,12 +143,7 @@ struct GemmSmem {
 // (or on) a rounding boundary of E4M3; every such boundary, in the normal and the subnormal range,
 // is an fp32 number whose low 19 mantissa bits are zero. So the product is used unless its low 19
 // bits are within a few units of zero (about one value in 10^5), where the real division runs.
-__device__ __forceinline__ float div_for_e4m3(float x, float scale, float inv_scale)
-{
-   const float q = __fmul_rn(x, inv_scale);
-   if (((__float_as_uint(q) + 4u) & 0x7FFFFu) < 9u) return __fdiv_rn(x, scale);
-   return q;
-}
+// The epilogue below tests eight values at a time.
 
 // Epilogue of 32 consecutive columns of one output row: r[j] is the raw accumulator of column
 // col0 + j (fp32 bits, or int32 for kI8). The per-column constants (bias, multiplier, correction) are
@@ -241,33 +236,60 @@ __device__ __forceinline__ void store_row_chunk(const GemmEpilogue &ep, const ui
          for (int j = 0; j < 32; j++) if (j < ncols) y[j] = (uint8_t)(packed[j >> 2] >> (8 * (j & 3)));
       }
    } else {
-      // y = acc * scale (+ bias) (Relu) -> bf16 (round to nearest even) -> optional E4M3 of bf16(y) / q_scale.
-      // Both conversions use the paired hardware instructions (two values per instruction).
+      // y = acc * scale (+ bias) -> bf16 (round to nearest even) -> Relu -> optional E4M3 of bf16(y) / q_scale, two values per
+      // instruction throughout (Relu commutes with the rounding; max gives +0 for NaN and -0 as relu_ref does). The quotient is taken
+      // as described above, with one test per eight values: of the smallest distance to a rounding boundary. A zero would look like
+      // one, and after Relu half of the values are zero, so there the product has 1e-30 added: no other value's E4M3 changes (the
+      // smallest boundary is 2^-10), and y is never negative. Without Relu the addend is -0, which changes nothing.
+      // Bound by issue slots: with a test per value, which sent every zero through the division, the drain of a 256 x 256 tile took
+      // longer than its MMAs at K = 1024 and slowed them at K = 4096. 65536 x 4096 x 4096 1083 -> 836 us (2031 -> 2632 TFLOP/s),
+      // 262144 x 1024 x 1024 988 -> 304 us; back to back the first one runs into the power limit (1198 -> 948 us).
       uint32_t hb[16], qb[8];
       const float scale = ep.a_scale_dev ? __fmul_rn(__ldg(ep.a_scale_dev), ep.w_scale) : ep.scale;
+      const uint64_t scale2 = pack_f32x2(scale, scale), inv2 = pack_f32x2(ep.q_inv, ep.q_inv);
+      const float off_zero = ep.relu ? 1e-30f : -0.f;
+      const uint64_t off2 = pack_f32x2(off_zero, off_zero);
+      const ulonglong2 *cf2 = reinterpret_cast<const ulonglong2 *>(cf);
 #pragma unroll
-      for (int j4 = 0; j4 < 8; j4++) {
-         const float4 c = cf4[j4];
-         const float cc[4] = {c.x, c.y, c.z, c.w};
-         float yv[4];
+      for (int j8 = 0; j8 < 4; j8++) {
 #pragma unroll
-         for (int t = 0; t < 4; t++) {
-            float y = __fmul_rn(__uint_as_float(r[4 * j4 + t]), scale);
-            if (ep.bias) y = __fadd_rn(y, cc[t]);
-            yv[t] = ep.relu ? relu_ref(y) : y;
+         for (int p = 0; p < 4; p++) {
+            const int j = 8 * j8 + 2 * p;
+            uint64_t y = mul_f32x2(pack_f32x2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), scale2);
+            if (ep.bias) {
+               const ulonglong2 c = cf2[j >> 2];
+               y = add_f32x2(y, (p & 1) ? c.y : c.x);
+            }
+            float y0, y1;
+            unpack_f32x2(y, y0, y1);
+            uint32_t h;
+            // cvt packs {hi, lo}: the first source lands in the upper half
+            asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(y1), "f"(y0));
+            if (ep.relu) asm("max.bf16x2 %0, %0, %1;" : "+r"(h) : "r"(0u));
+            hb[j >> 1] = h;
          }
-         // cvt packs {hi, lo}: the first source lands in the upper half
-         asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hb[2 * j4]) : "f"(yv[1]), "f"(yv[0]));
-         asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(hb[2 * j4 + 1]) : "f"(yv[3]), "f"(yv[2]));
          if (ep.Yq) {
-            const float d0 = div_for_e4m3(__uint_as_float(hb[2 * j4] << 16), ep.q_scale, ep.q_inv);
-            const float d1 = div_for_e4m3(__uint_as_float(hb[2 * j4] & 0xFFFF0000u), ep.q_scale, ep.q_inv);
-            const float d2 = div_for_e4m3(__uint_as_float(hb[2 * j4 + 1] << 16), ep.q_scale, ep.q_inv);
-            const float d3 = div_for_e4m3(__uint_as_float(hb[2 * j4 + 1] & 0xFFFF0000u), ep.q_scale, ep.q_inv);
-            uint16_t lo, hi;
-            asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(lo) : "f"(d1), "f"(d0));
-            asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(hi) : "f"(d3), "f"(d2));
-            qb[j4] = (uint32_t)lo | ((uint32_t)hi << 16);
+            float d[8];
+            uint32_t nearest = 0xFFFFFFFFu;
+#pragma unroll
+            for (int p = 0; p < 4; p++) {
+               const uint32_t h = hb[4 * j8 + p];
+               unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(h << 16), __uint_as_float(h & 0xFFFF0000u)), inv2, off2), d[2 * p], d[2 * p + 1]);
+               nearest = min(nearest, min((__float_as_uint(d[2 * p]) + 4u) & 0x7FFFFu, (__float_as_uint(d[2 * p + 1]) + 4u) & 0x7FFFFu));
+            }
+            if (nearest < 9u) {
+#pragma unroll
+               for (int p = 0; p < 4; p++) {
+                  const uint32_t h = hb[4 * j8 + p];
+                  d[2 * p] = __fdiv_rn(__uint_as_float(h << 16), ep.q_scale);
+                  d[2 * p + 1] = __fdiv_rn(__uint_as_float(h & 0xFFFF0000u), ep.q_scale);
+               }
+            }
+            uint16_t e[4];
+#pragma unroll
+            for (int p = 0; p < 4; p++) asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(e[p]) : "f"(d[2 * p + 1]), "f"(d[2 * p]));
+            qb[2 * j8] = (uint32_t)e[0] | ((uint32_t)e[1] << 16);
+            qb[2 * j8 + 1] = (uint32_t)e[2] | ((uint32_t)e[3] << 16);
          }
       }
       if (ep.Ybf16) {

@@ -154,6 +154,27 @@ def test_gemm_e4m3_pair_kernel():
     assert np.array_equal(Yq.cpu().numpy(), o.quantize_e4m3(y, 0.01))
 
 
+# The E4M3 output takes eight quotients at a time and divides only where one of them lies near a rounding boundary: with a scale of
+# 0.01 or 0.25 many do, zeros (whole rows of them, some biases too) must not count as such nor change their sign, and 3e-39 has an
+# infinite reciprocal. Sizes of the one-CTA kernel (ragged) and of the pair kernel.
+@pytest.mark.parametrize("M,N,K", [(300, 72, 144), (18900, 1000, 128)])
+@pytest.mark.parametrize("relu", [False, True])
+def test_gemm_e4m3_output_bytes(relu, M, N, K):
+    rng = np.random.default_rng(M + N)
+    X = rng.standard_normal((M, K)).astype(np.float32)
+    X[::7] = 0
+    Wf = (rng.standard_normal((N, K)) * 0.02).astype(np.float32)
+    bias = np.where(rng.random(N) < 0.3, 0, rng.standard_normal(N) * 0.02).astype(np.float32)
+    sa, sw = float(np.abs(X).max() / 448), float(np.abs(Wf).max() / 448)
+    Aq, Wq = o.quantize_e4m3(X, sa), o.quantize_e4m3(Wf, sw)
+    ref = o.bf16_bits_to_f32(o.gemm_e4m3(Aq, sa, Wq, sw, bias, relu=relu))
+    for scale in (0.01, 0.01137, 0.25, 1e-6) + ((3e-39,) if M == 300 else ()):
+        Y, Yq = ops.gemm_e4m3(dev(Aq), dev(Wq), dev(bias), a_scale=sa, w_scale=sw, relu=relu, q_scale=scale)
+        y = Y.float().cpu().numpy()
+        assert rel_err(y, ref) <= 8e-3
+        assert np.array_equal(Yq.cpu().numpy(), o.quantize_e4m3(y, scale))
+
+
 # ------------------------------------------------------------------------------------ implicit-GEMM convolution
 CONV_TC = [
     # N, C, H, W, Cout, relu, pool
