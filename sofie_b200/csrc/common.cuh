@@ -179,6 +179,14 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
    return v;
 }
 
+// 32 bytes of a 32-byte aligned row in one store: a whole sector per thread
+__device__ __forceinline__ void store_f32x8(float *p, const float *v)
+{
+   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]),
+                "f"(v[5]), "f"(v[6]), "f"(v[7])
+                : "memory");
+}
+
 __device__ __forceinline__ float relu_ref(float v)
 {
    // The reference's `x > 0 ? x : 0`: NaN and -0 both become +0.

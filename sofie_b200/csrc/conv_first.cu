@@ -335,6 +335,9 @@ qconv3x3_first_c1_pool_kernel(ConvGeom g, const uint8_t *__restrict__ X, const i
 // the shared-memory pipe off the critical path. A block of 128 threads covers 16 rows x 32 columns of
 // convolution outputs; blocks are kept that small so that four fit on an SM and the load, compute and
 // store phases of different blocks overlap.
+// Bound by issue slots: packed FMAs take two channels at a time (each product and sum is rounded as the scalar ones were), a pixel's
+// eight channels leave as one 32-byte store, and the next tile is fetched under this one. 8192 x 3 x 32 x 32 to 16 channels:
+// 270 -> 218 us (its bytes take 97).
 // VEC: NCHW input whose width is a multiple of 4 (and a 16-byte aligned base): the tile is staged with 16-byte
 // asynchronous copies of whole words of the image rows (a tile starts on a multiple of 32 columns, so a word is
 // either inside the image or entirely padding, which the copy zero-fills); the patch then starts at column 3.
@@ -349,26 +352,24 @@ conv3x3_first_f32_kernel(ConvGeom g, const float *__restrict__ X, const float *_
    constexpr int OCC = 8;
    constexpr int TW4 = 10;                       // VEC: 16-byte words per tile row, image columns ux0*2 - 4 .. ux0*2 + 35
    constexpr int TSW = VEC ? 4 * TW4 : TS + 1;   // row stride of the tile in floats
-   constexpr int COL0 = VEC ? 3 : 0;             // tile column of the patch's first input column
-   __shared__ __align__(16) float tile[C][TSH][TSW];
+   constexpr int BUFS = VEC ? 2 : 1;             // VEC: the next tile is fetched while this one is computed
+   __shared__ __align__(16) float tile[BUFS][C][TSH][TSW];
    __shared__ float4 s_w[K][kFirstMaxCout / 4]; // [tap][channel / 4]
-   __shared__ float s_bias[kFirstMaxCout];
+   __shared__ __align__(16) float s_bias[kFirstMaxCout];
 
    const int tid = threadIdx.x;
    const int ty = tid / 16, tx = tid % 16;
    bool weights_staged = false;
-   for (long long tile_id = blockIdx.x; tile_id < num_tiles; tile_id += gridDim.x) {
-      int n, uy0, ux0; // origin in units of 2 x 2 outputs
-      first_tile_origin(g, tile_id, tiles_x, tiles_y, n, uy0, ux0);
+   auto origin = [&](long long id, int &n, int &uy0, int &ux0) { // in units of 2 x 2 outputs
+      first_tile_origin(g, id, tiles_x, tiles_y, n, uy0, ux0);
       uy0 = uy0 / 16 * kFirstF32UnitsY; // this kernel's tiles are 8 units tall
-      const int ih0 = uy0 * 2 - 1, iw0 = ux0 * 2 - 1;
-      // all loads of a thread are issued before the first store, so their latencies overlap
-      constexpr int kLoads = VEC ? 1 : (C * TSH * TS + kFirstF32Threads - 1) / kFirstF32Threads;
-      float staged[kLoads];
-      if constexpr (VEC) {
-         __syncthreads(); // the previous tile is no longer read: the copies below write the tile directly
+   };
+   auto copy_tile = [&](long long id, int buf) {
+      if (id < num_tiles) {
+         int n, uy0, ux0;
+         origin(id, n, uy0, ux0);
          constexpr int kPieces = C * TSH * TW4;
-         const int wc0 = (ux0 * 2 - 4) >> 2, wcols = g.W >> 2;
+         const int ih0 = uy0 * 2 - 1, wc0 = (ux0 * 2 - 4) >> 2, wcols = g.W >> 2;
 #pragma unroll
          for (int j = 0; j < (kPieces + kFirstF32Threads - 1) / kFirstF32Threads; j++) {
             const int i = tid + j * kFirstF32Threads;
@@ -377,25 +378,40 @@ conv3x3_first_f32_kernel(ConvGeom g, const float *__restrict__ X, const float *_
                const int ih = ih0 + r, wc = wc0 + w;
                const bool ok = ih >= 0 && ih < g.H && wc >= 0 && wc < wcols;
                const float *src = X + (((size_t)n * C + c) * g.H + (ok ? ih : 0)) * g.W + 4 * (ok ? wc : 0);
-               const unsigned dst = (unsigned)__cvta_generic_to_shared(&tile[c][r][4 * w]);
+               const unsigned dst = (unsigned)__cvta_generic_to_shared(&tile[buf][c][r][4 * w]);
                const int bytes = ok ? 16 : 0; // zero-filled when the word lies outside the image
                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
             }
          }
+      }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+   };
+   if constexpr (VEC) copy_tile(blockIdx.x, 0);
+   int buf = 0;
+   for (long long tile_id = blockIdx.x; tile_id < num_tiles; tile_id += gridDim.x, buf ^= BUFS - 1) {
+      int n, uy0, ux0;
+      origin(tile_id, n, uy0, ux0);
+      // all loads of a thread are issued before the first store, so their latencies overlap
+      constexpr int kLoads = VEC ? 1 : (C * TSH * TS + kFirstF32Threads - 1) / kFirstF32Threads;
+      float staged[kLoads];
+      if constexpr (VEC) {
+         __syncthreads(); // the tile before this one is no longer read: its buffer is the next tile's
+         copy_tile(tile_id + gridDim.x, buf ^ 1);
          staged[0] = 0.f;
       } else {
+         const int ih0 = uy0 * 2 - 1, iw0 = ux0 * 2 - 1;
 #pragma unroll
-      for (int j = 0; j < kLoads; j++) {
-         const int i = tid + j * kFirstF32Threads;
-         const int c = i / (TSH * TS), rem = i % (TSH * TS), r = rem / TS, col = rem % TS;
-         const int ih = ih0 + r, iw = iw0 + col;
-         float v = 0.f;
-         if (i < C * TSH * TS && ih >= 0 && ih < g.H && iw >= 0 && iw < g.W) {
-            const size_t xi = g.x_nhwc ? (((size_t)n * g.H + ih) * g.W + iw) * C + c : (((size_t)n * C + c) * g.H + ih) * g.W + iw;
-            v = __ldg(X + xi);
+         for (int j = 0; j < kLoads; j++) {
+            const int i = tid + j * kFirstF32Threads;
+            const int c = i / (TSH * TS), rem = i % (TSH * TS), r = rem / TS, col = rem % TS;
+            const int ih = ih0 + r, iw = iw0 + col;
+            float v = 0.f;
+            if (i < C * TSH * TS && ih >= 0 && ih < g.H && iw >= 0 && iw < g.W) {
+               const size_t xi = g.x_nhwc ? (((size_t)n * g.H + ih) * g.W + iw) * C + c : (((size_t)n * C + c) * g.H + ih) * g.W + iw;
+               v = __ldg(X + xi);
+            }
+            staged[j] = v;
          }
-         staged[j] = v;
-      }
       }
       if (!weights_staged) {
          // The weights are fetched while the loads of the first tile are still in flight.
@@ -412,54 +428,72 @@ conv3x3_first_f32_kernel(ConvGeom g, const float *__restrict__ X, const float *_
          weights_staged = true;
       }
       if constexpr (VEC) {
-         asm volatile("cp.async.wait_all;\n" ::: "memory");
+         asm volatile("cp.async.wait_group 1;\n" ::: "memory"); // all but the copies of the next tile
       } else {
          __syncthreads(); // weights staged / the previous tile is no longer read
 #pragma unroll
          for (int j = 0; j < kLoads; j++) {
             const int i = tid + j * kFirstF32Threads;
-            if (i < C * TSH * TS) tile[i / (TSH * TS)][(i % (TSH * TS)) / TS][i % TS] = staged[j];
+            if (i < C * TSH * TS) tile[0][i / (TSH * TS)][(i % (TSH * TS)) / TS][i % TS] = staged[j];
          }
       }
       __syncthreads(); // tile and weights are in shared memory
       const int oh0 = (uy0 + ty) * 2, ow0 = (ux0 + tx) * 2; // top-left convolution output of this thread
       if (oh0 >= g.oH || ow0 >= g.oW) continue;
+#pragma unroll 1
       for (int oc0 = 0; oc0 < g.Cout; oc0 += OCC) {
-         float acc[4][OCC];
+         uint64_t acc2[4][OCC / 2]; // two neighbouring channels each
 #pragma unroll
          for (int q = 0; q < 4; q++)
 #pragma unroll
-            for (int o = 0; o < OCC; o++) acc[q][o] = 0.f;
+            for (int o = 0; o < OCC / 2; o++) acc2[q][o] = 0;
 #pragma unroll
          for (int c = 0; c < C; c++) {
-            float win[4][4]; // the 4 x 4 inputs under the 2 x 2 outputs
+            uint64_t win[4][4]; // the 4 x 4 inputs under the 2 x 2 outputs, each twice
 #pragma unroll
-            for (int r = 0; r < 4; r++)
+            for (int r = 0; r < 4; r++) {
+               float v[4];
+               if constexpr (VEC) {
+                  // columns 3 + 2 tx ... 6 + 2 tx, read as aligned pairs
+                  const float *p = &tile[buf][c][ty * 2 + r][tx * 2 + 2];
+                  const float2 a = *reinterpret_cast<const float2 *>(p), b = *reinterpret_cast<const float2 *>(p + 2);
+                  v[0] = a.y, v[1] = b.x, v[2] = b.y, v[3] = p[4];
+               } else {
 #pragma unroll
-               for (int t = 0; t < 4; t++) win[r][t] = tile[c][ty * 2 + r][COL0 + tx * 2 + t];
+                  for (int t = 0; t < 4; t++) v[t] = tile[0][c][ty * 2 + r][tx * 2 + t];
+               }
+#pragma unroll
+               for (int t = 0; t < 4; t++) win[r][t] = pack_f32x2(v[t], v[t]);
+            }
 #pragma unroll
             for (int rt = 0; rt < 9; rt++) {
                const int r = rt / 3, t = rt % 3;
 #pragma unroll
                for (int o4 = 0; o4 < OCC / 4; o4++) {
-                  const float4 w = s_w[c * 9 + rt][oc0 / 4 + o4];
+                  const ulonglong2 w = *reinterpret_cast<const ulonglong2 *>(&s_w[c * 9 + rt][oc0 / 4 + o4]);
 #pragma unroll
                   for (int q = 0; q < 4; q++) {
-                     const float xv = win[(q >> 1) + r][(q & 1) + t];
-                     acc[q][4 * o4 + 0] = fmaf(xv, w.x, acc[q][4 * o4 + 0]);
-                     acc[q][4 * o4 + 1] = fmaf(xv, w.y, acc[q][4 * o4 + 1]);
-                     acc[q][4 * o4 + 2] = fmaf(xv, w.z, acc[q][4 * o4 + 2]);
-                     acc[q][4 * o4 + 3] = fmaf(xv, w.w, acc[q][4 * o4 + 3]);
+                     const uint64_t xv = win[(q >> 1) + r][(q & 1) + t];
+                     acc2[q][2 * o4 + 0] = fma_f32x2(xv, w.x, acc2[q][2 * o4 + 0]);
+                     acc2[q][2 * o4 + 1] = fma_f32x2(xv, w.y, acc2[q][2 * o4 + 1]);
                   }
                }
             }
          }
+         float acc[4][OCC];
+#pragma unroll
+         for (int q = 0; q < 4; q++)
+#pragma unroll
+            for (int o = 0; o < OCC / 2; o++) unpack_f32x2(acc2[q][o], acc[q][2 * o], acc[q][2 * o + 1]);
          // one stored pixel (pooled) or four
          auto store_pixel = [&](const float *v, int ph, int pw) {
             const size_t opix = ((size_t)n * g.pH + ph) * g.pW + pw;
             if (g.y_nhwc) {
                float *y = Y + opix * g.Cout + oc0;
-               if (oc0 + OCC <= g.Cout && ((reinterpret_cast<uintptr_t>(y) & 15) == 0)) {
+               if (oc0 + OCC <= g.Cout && ((reinterpret_cast<uintptr_t>(y) & 31) == 0)) {
+                  static_assert(OCC == 8, "one 32-byte store");
+                  store_f32x8(y, v);
+               } else if (oc0 + OCC <= g.Cout && ((reinterpret_cast<uintptr_t>(y) & 15) == 0)) {
 #pragma unroll
                   for (int o = 0; o < OCC; o += 4) *reinterpret_cast<float4 *>(y + o) = make_float4(v[o], v[o + 1], v[o + 2], v[o + 3]);
                } else {
