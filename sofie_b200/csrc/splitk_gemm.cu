@@ -109,8 +109,7 @@ __global__ void gemm_f32_splitk_reduce_kernel(sofie_gemm_f32_desc d, int splits,
 // the two launches of the split-K pair and its scratch round trip cost more than the arithmetic.
 // four rows per block measured best inside the C2 step (72.3 us against 73.7 with two and 74.8 with eight)
 constexpr int kRowBlockRows = 4;
-// Larger batches with up to ten columns: eight rows per block halve what is read of B out of L2
-constexpr int kRowBlockManyRows = 8, kRowBlockManyFrom = 2048, kRowBlockManyMaxN = 10;
+constexpr int kRowBlockMaxRows = 2048; // more rows go to gemm_f32_rows_kernel
 
 template <int NN, int ROWS>
 __global__ void __launch_bounds__(256)
@@ -170,32 +169,106 @@ gemm_f32_rowblock_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, con
    }
 }
 
+// ------------------------------------------------------------------------------------------------
+// The same shapes with many rows, where A (K >= 1024, once through memory) is all that counts. A block owns 8 x ROWS rows, a warp
+// ROWS of them, whose lanes split K in 16-byte steps. B is staged chunk by chunk (256 of K, asynchronously, two buffers) and shared by the block's rows: 10 KB out
+// of L2 for 32 KB of A. The rows' loads of a chunk are issued before the wait for it.
+// 8192 x 10 x 4096: 62 -> 46 us, 4096 x 10 x 4096 90 (before the tensor-core kernel of any layout) -> 35 us.
+constexpr int kRowsChunk = 256;
+template <int NN, int ROWS>
+__global__ void __launch_bounds__(256, 2)
+gemm_f32_rows_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, const float *__restrict__ B, const float *__restrict__ C,
+                     float *__restrict__ Y)
+{
+   __shared__ __align__(16) float s_b[2][NN][kRowsChunk];
+   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); // known to be the same in all lanes
+   const int m0 = (blockIdx.x * 8 + warp) * ROWS, K = d.K;
+   griddep_launch_dependents();
+   griddep_wait(); // A is the previous kernel's output
+   auto copy_b = [&](int k0, int buf) {
+      for (int i = threadIdx.x; i < NN * (kRowsChunk / 4); i += 256) {
+         const int n = i / (kRowsChunk / 4), k = k0 + 4 * (i % (kRowsChunk / 4));
+         const bool in = k < K; // K % 4 == 0: a piece lies inside or outside; zeros outside
+         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((unsigned)__cvta_generic_to_shared(&s_b[buf][n][4 * (i % (kRowsChunk / 4))])),
+                      "l"(B + (size_t)n * K + (in ? k : 0)), "r"(in ? 16 : 0)
+                      : "memory");
+      }
+      asm volatile("cp.async.commit_group;\n" ::: "memory");
+   };
+   float acc[ROWS][NN];
+#pragma unroll
+   for (int r = 0; r < ROWS; r++)
+#pragma unroll
+      for (int n = 0; n < NN; n++) acc[r][n] = 0.f;
+   const float *a0 = A + (size_t)min(m0, d.M - 1) * K + 4 * lane;
+   const int last = d.M - 1 - m0; // rows past M repeat the last one (or all are it), not stored
+   copy_b(0, 0);
+   int buf = 0;
+   for (int k0 = 0; k0 < K; k0 += kRowsChunk, buf ^= 1) {
+      float4 a[kRowsChunk / 128][ROWS];
+#pragma unroll
+      for (int h = 0; h < kRowsChunk / 128; h++)
+#pragma unroll
+         for (int r = 0; r < ROWS; r++) {
+            a[h][r] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (k0 + 128 * h + 4 * lane < K) a[h][r] = *reinterpret_cast<const float4 *>(a0 + (size_t)max(min(r, last), 0) * K + k0 + 128 * h);
+         }
+      copy_b(k0 + kRowsChunk, buf ^ 1); // past the end: zeros nobody reads
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+      __syncthreads();
+#pragma unroll
+      for (int h = 0; h < kRowsChunk / 128; h++)
+#pragma unroll
+         for (int n = 0; n < NN; n++) {
+            const float4 b = *reinterpret_cast<const float4 *>(&s_b[buf][n][128 * h + 4 * lane]);
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) acc[r][n] = fmaf(a[h][r].w, b.w, fmaf(a[h][r].z, b.z, fmaf(a[h][r].y, b.y, fmaf(a[h][r].x, b.x, acc[r][n]))));
+         }
+      __syncthreads(); // this buffer is the one after next's
+   }
+#pragma unroll
+   for (int r = 0; r < ROWS; r++)
+#pragma unroll
+      for (int n = 0; n < NN; n++) {
+         float v = acc[r][n];
+#pragma unroll
+         for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+         const int m = m0 + r;
+         if (lane == n && m < d.M) {
+            float y = d.alpha * v;
+            if (d.bias_kind == 1) y += d.beta * C[n];
+            else if (d.bias_kind == 2) y += d.beta * C[(size_t)m * NN + n];
+            Y[(size_t)m * NN + n] = d.relu ? relu_ref(y) : y;
+         }
+      }
+}
+
 bool rowblock_shape_ok(const sofie_gemm_f32_desc &d, const float *A, const float *B)
 {
    static const bool enabled = [] { const char *e = getenv("SOFIE_CUDA_GEMM_ROWBLOCK"); return !e || atoi(e) != 0; }();
-   return enabled && !d.transA && d.transB && d.N <= kSplitKMaxN && d.K >= 1024 && d.K % 4 == 0 && d.M <= (d.N <= 4 ? (1 << 30) : (d.N <= kRowBlockManyMaxN ? 5000 : kRowBlockManyFrom)) &&
+   // Rows kernel against the tensor-core one, whose time hardly depends on N (us): 8192 x 10 x 4096 46 / 62, 32768 x 10 x 4096 143 / 174,
+   // 32768 x 16 x 4096 174 / 175, 32768 x 4 x 1024 41 / 52, 32768 x 10 x 1024 54 / 52, 32768 x 16 x 1024 66 / 54
+   const bool rows = d.M <= kRowBlockMaxRows || d.N <= 4 || d.K >= 2048 || d.M <= 16384;
+   return enabled && rows && !d.transA && d.transB && d.N <= kSplitKMaxN && d.K >= 1024 && d.K % 4 == 0 &&
           (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (reinterpret_cast<uintptr_t>(B) & 15) == 0;
 }
 
 int launch_gemm_f32_rowblock(cudaStream_t s, const sofie_gemm_f32_desc &d, const float *A, const float *B, const float *C, float *Y)
 {
    if (!rowblock_shape_ok(d, A, B)) return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "not a row-block GEMM shape");
-   const bool many = d.M > kRowBlockManyFrom;
-   const dim3 grid(ceil_div(d.M, many ? kRowBlockManyRows : kRowBlockRows)), block(256);
 #define SOFIE_ROWBLOCK(NN)                                                                                                              \
-   case NN:                                                                                                                             \
-      if constexpr (NN <= kRowBlockManyMaxN) {                                                                                          \
-         if (many) {                                                                                                                    \
-            SOFIE_CUDA_TRY(launch_dependent(gemm_f32_rowblock_kernel<NN, kRowBlockManyRows>, grid, block, 0, s, d, A, B, C, Y));       \
-            break;                                                                                                                      \
-         }                                                                                                                              \
-      }                                                                                                                                 \
-      SOFIE_CUDA_TRY(launch_dependent(gemm_f32_rowblock_kernel<NN, kRowBlockRows>, grid, block, 0, s, d, A, B, C, Y));                 \
-      break
+   case NN: {                                                                                                                           \
+      constexpr int rows = 4; /* of a warp */                                                                                           \
+      if (d.M > kRowBlockMaxRows)                                                                                                       \
+         SOFIE_CUDA_TRY(launch_dependent(gemm_f32_rows_kernel<NN, rows>, dim3(ceil_div(d.M, 8 * rows)), dim3(256), 0, s, d, A, B, C, Y)); \
+      else                                                                                                                              \
+         SOFIE_CUDA_TRY(launch_dependent(gemm_f32_rowblock_kernel<NN, kRowBlockRows>, dim3(ceil_div(d.M, kRowBlockRows)), dim3(256), 0, s, d, A, B, C, Y)); \
+      break;                                                                                                                            \
+   }
    switch (d.N) {
-      SOFIE_ROWBLOCK(1); SOFIE_ROWBLOCK(2); SOFIE_ROWBLOCK(3); SOFIE_ROWBLOCK(4); SOFIE_ROWBLOCK(5); SOFIE_ROWBLOCK(6);
-      SOFIE_ROWBLOCK(7); SOFIE_ROWBLOCK(8); SOFIE_ROWBLOCK(9); SOFIE_ROWBLOCK(10); SOFIE_ROWBLOCK(11); SOFIE_ROWBLOCK(12);
-      SOFIE_ROWBLOCK(13); SOFIE_ROWBLOCK(14); SOFIE_ROWBLOCK(15); SOFIE_ROWBLOCK(16);
+      SOFIE_ROWBLOCK(1) SOFIE_ROWBLOCK(2) SOFIE_ROWBLOCK(3) SOFIE_ROWBLOCK(4) SOFIE_ROWBLOCK(5) SOFIE_ROWBLOCK(6)
+      SOFIE_ROWBLOCK(7) SOFIE_ROWBLOCK(8) SOFIE_ROWBLOCK(9) SOFIE_ROWBLOCK(10) SOFIE_ROWBLOCK(11) SOFIE_ROWBLOCK(12)
+      SOFIE_ROWBLOCK(13) SOFIE_ROWBLOCK(14) SOFIE_ROWBLOCK(15) SOFIE_ROWBLOCK(16)
    }
 #undef SOFIE_ROWBLOCK
    set_last_engine(SOFIE_ENGINE_SIMT);

@@ -650,6 +650,21 @@ def test_context_arena_upload_copy_and_graph():
         capi.call("sofie_cuda_ctx_destroy", ctx)
 
 
+@pytest.mark.parametrize("M,N,K", [(2049, 1, 1024), (2081, 10, 1028), (2100, 16, 1276), (4000, 7, 1532), (2064, 11, 2048)])
+@pytest.mark.parametrize("bias_kind", [0, 1, 2])
+def test_gemm_f32_many_rows_few_columns(M, N, K, bias_kind):
+    """More than 2048 rows: the kernel whose warps own four rows each. Rows that end within a warp's four and within a block's 32, K that
+    ends within a lane's step of a chunk; against float64, within the error of K / 32 sums in a row (each of a lane) and five more."""
+    rng = np.random.default_rng(M + N + K)
+    A, B = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32)
+    C = [None, rng.standard_normal(N).astype(np.float32), rng.standard_normal((M, N)).astype(np.float32)][bias_kind]
+    ref = 0.75 * (A.astype(np.float64) @ B.astype(np.float64).T) + (0 if C is None else 1.5 * C.astype(np.float64))
+    y = ops.gemm_f32(dev(A), dev(B), None if C is None else dev(C), transB=1, alpha=0.75, beta=1.5, relu=bias_kind == 1).cpu().numpy()
+    if bias_kind == 1:
+        ref = np.maximum(ref, 0)
+    assert np.abs(y - ref).max() <= (K / 32 + 8) * 2.0 ** -24 * np.abs(A).astype(np.float64).dot(np.abs(B).T.astype(np.float64)).max() + 2.0 ** -22 * np.abs(ref).max()
+
+
 def test_many_contexts_one_after_another_share_the_splitk_scratch_pool():
     """Each context's stream borrows a split-K scratch buffer from a pool of 16 and gives it back when the
     context is destroyed: far more than 16 contexts can come and go, and 16 can be alive at once."""
