@@ -160,18 +160,6 @@ __device__ __forceinline__ uint64_t pack_f32x2(float lo, float hi)
    return v;
 }
 __device__ __forceinline__ void unpack_f32x2(uint64_t v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b)
-{
-   uint64_t v;
-   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-   return v;
-}
-__device__ __forceinline__ uint64_t add_f32x2(uint64_t a, uint64_t b)
-{
-   uint64_t v;
-   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-   return v;
-}
 __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c)
 {
    uint64_t v;

@@ -237,31 +237,30 @@ __device__ __forceinline__ void store_row_chunk(const GemmEpilogue &ep, const ui
       }
    } else {
       // y = acc * scale (+ bias) -> bf16 (round to nearest even) -> Relu -> optional E4M3 of bf16(y) / q_scale, two values per
-      // instruction throughout (Relu commutes with the rounding; max gives +0 for NaN and -0 as relu_ref does). The quotient is taken
+      // instruction from the rounding on (Relu commutes with the rounding; max gives +0 for NaN and -0 as relu_ref does). The quotient is taken
       // as described above, with one test per eight values: of the smallest distance to a rounding boundary. A zero would look like
-      // one, and after Relu half of the values are zero, so there the product has 1e-30 added: no other value's E4M3 changes (the
-      // smallest boundary is 2^-10), and y is never negative. Without Relu the addend is -0, which changes nothing.
+      // one, and after Relu half of the values are zero, so there the product has 1e-30 (of the scale's sign) added: no other value's E4M3 changes (the
+      // smallest boundary is 2^-10), and y is never negative. Without Relu the addend is -0: zeros are divided and keep their sign.
       // Bound by issue slots: with a test per value, which sent every zero through the division, the drain of a 256 x 256 tile took
       // longer than its MMAs at K = 1024 and slowed them at K = 4096. 65536 x 4096 x 4096 1083 -> 836 us (2031 -> 2632 TFLOP/s),
       // 262144 x 1024 x 1024 988 -> 304 us; back to back the first one runs into the power limit (1198 -> 948 us).
       uint32_t hb[16], qb[8];
       const float scale = ep.a_scale_dev ? __fmul_rn(__ldg(ep.a_scale_dev), ep.w_scale) : ep.scale;
-      const uint64_t scale2 = pack_f32x2(scale, scale), inv2 = pack_f32x2(ep.q_inv, ep.q_inv);
-      const float off_zero = ep.relu ? 1e-30f : -0.f;
+      const uint64_t inv2 = pack_f32x2(ep.q_inv, ep.q_inv);
+      const float off_zero = ep.relu ? copysignf(1e-30f, ep.q_inv) : -0.f;
       const uint64_t off2 = pack_f32x2(off_zero, off_zero);
-      const ulonglong2 *cf2 = reinterpret_cast<const ulonglong2 *>(cf);
+      const float2 *cf2 = reinterpret_cast<const float2 *>(cf);
 #pragma unroll
       for (int j8 = 0; j8 < 4; j8++) {
 #pragma unroll
          for (int p = 0; p < 4; p++) {
             const int j = 8 * j8 + 2 * p;
-            uint64_t y = mul_f32x2(pack_f32x2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), scale2);
+            // scalar: the packed product and sum come out of the assembler as one rounding
+            float y0 = __fmul_rn(__uint_as_float(r[j]), scale), y1 = __fmul_rn(__uint_as_float(r[j + 1]), scale);
             if (ep.bias) {
-               const ulonglong2 c = cf2[j >> 2];
-               y = add_f32x2(y, (p & 1) ? c.y : c.x);
+               const float2 c = cf2[j >> 1];
+               y0 = __fadd_rn(y0, c.x), y1 = __fadd_rn(y1, c.y);
             }
-            float y0, y1;
-            unpack_f32x2(y, y0, y1);
             uint32_t h;
             // cvt packs {hi, lo}: the first source lands in the upper half
             asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(y1), "f"(y0));
