@@ -4,6 +4,7 @@
 // emits for each operator (cited per case), evaluated in the same precision.
 #include "common.cuh"
 
+#include <initializer_list>
 #include <utility>
 
 namespace sofie {
@@ -78,20 +79,31 @@ __device__ __forceinline__ float binary_apply(int op, float a, float b)
    }
 }
 
+// Two tensors in, one out: 32-byte accesses keep more in flight. 134 MB tensors 71.7 -> 67.6 us (6.0 TB/s), 1 GB tensors 513 -> 487 us;
+// for one tensor in they gain nothing (Relu 49.2 us both ways) or lose (Sigmoid 51.1 -> 55.3 us), so those stay with 16 bytes.
 __global__ void binary_same_f32_kernel(int op, const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ Y, size_t n,
-                                       bool vec)
+                                       int vec)
 {
    griddep_launch_dependents();
    griddep_wait();
    const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nthreads = (size_t)gridDim.x * blockDim.x;
-   const size_t n4 = vec ? n / 4 : 0;
+   const size_t n4 = vec == 4 ? n / 4 : 0, n8 = vec == 8 ? n / 8 : 0;
+#pragma unroll 2
+   for (size_t i = tid; i < n8; i += nthreads) {
+      float a[8], b[8];
+      load_f32x8(A + 8 * i, a);
+      load_f32x8(B + 8 * i, b);
+#pragma unroll
+      for (int j = 0; j < 8; j++) a[j] = binary_apply(op, a[j], b[j]);
+      store_f32x8(Y + 8 * i, a);
+   }
 #pragma unroll 2
    for (size_t i = tid; i < n4; i += nthreads) {
       const float4 a = reinterpret_cast<const float4 *>(A)[i], b = reinterpret_cast<const float4 *>(B)[i];
       reinterpret_cast<float4 *>(Y)[i] =
          make_float4(binary_apply(op, a.x, b.x), binary_apply(op, a.y, b.y), binary_apply(op, a.z, b.z), binary_apply(op, a.w, b.w));
    }
-   for (size_t i = n4 * 4 + tid; i < n; i += nthreads) Y[i] = binary_apply(op, A[i], B[i]);
+   for (size_t i = n8 * 8 + n4 * 4 + tid; i < n; i += nthreads) Y[i] = binary_apply(op, A[i], B[i]);
 }
 
 // Broadcasting. The dimensions are merged as far as both operands allow (an [N,C,H,W] tensor and a [C,1,1] one become [N,C,HW]); a
@@ -243,6 +255,13 @@ __global__ void batchnorm_large_f32_kernel(sofie_batchnorm_desc d, const float *
    }
 }
 
+// floats per access: as wide as all of the pointers allow
+inline int access_width(std::initializer_list<const void *> pointers)
+{
+   uintptr_t bits = 0;
+   for (const void *p : pointers) bits |= reinterpret_cast<uintptr_t>(p);
+   return (bits & 31) == 0 ? 8 : ((bits & 15) == 0 ? 4 : 1);
+}
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 } // namespace
@@ -278,8 +297,8 @@ extern "C" int sofie_cuda_binary_f32(void *stream, const sofie_binary_desc *d, c
    SOFIE_REQUIRE(A && B && Y, "NULL tensor");
    cudaStream_t s = as_stream(stream);
    if (same) {
-      const bool vec = aligned16(A) && aligned16(B) && aligned16(Y);
-      SOFIE_CUDA_TRY(launch_dependent(binary_same_f32_kernel, dim3(act_grid(vec ? n / 4 + 1 : n)), dim3(kActThreads), 0, s, d->op, A, B, Y, n, vec));
+      const int vec = access_width({A, B, Y});
+      SOFIE_CUDA_TRY(launch_dependent(binary_same_f32_kernel, dim3(act_grid(n / vec + 1)), dim3(kActThreads), 0, s, d->op, A, B, Y, n, vec));
       return SOFIE_CUDA_OK;
    }
    if (n >= (size_t(1) << 31) - 4096 * 1024) {

@@ -167,6 +167,13 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
    return v;
 }
 
+// 32 bytes of a 32-byte aligned row in one load
+__device__ __forceinline__ void load_f32x8(const float *p, float (&v)[8])
+{
+   asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                : "l"(p));
+}
 // 32 bytes of a 32-byte aligned row in one store: a whole sector per thread
 __device__ __forceinline__ void store_f32x8(float *p, const float *v)
 {

@@ -650,6 +650,15 @@ def test_context_arena_upload_copy_and_graph():
         capi.call("sofie_cuda_ctx_destroy", ctx)
 
 
+@pytest.mark.parametrize("n", [1, 7, 8, 17, 4099])
+@pytest.mark.parametrize("skip", [0, 4, 1])
+def test_binary_access_widths(n, skip):
+    """Bases on 32, 16 and 4 bytes take accesses of eight, four and one floats; every length leaves its own remainder."""
+    rng = np.random.default_rng(n + skip)
+    a, b = (rng.standard_normal(n + skip).astype(np.float32) for _ in range(2))
+    assert np.array_equal(ops.binary_f32(dev(a)[skip:], dev(b)[skip:], "Add").cpu().numpy(), (a + b)[skip:])
+
+
 @pytest.mark.parametrize("M,N,K", [(2049, 1, 1024), (2081, 10, 1028), (2100, 16, 1276), (4000, 7, 1532), (2064, 11, 2048)])
 @pytest.mark.parametrize("bias_kind", [0, 1, 2])
 def test_gemm_f32_many_rows_few_columns(M, N, K, bias_kind):
