@@ -617,12 +617,18 @@ void RModel::PlanArena()
          for (auto &out : fOperators[i]->GetOpOutputTensors()) together(out);
    }
    // Ranges of a batch run one after the other, so the tensors between the first and the last operator may share bytes as in
-   // the plan of the whole; but later ranges of the input arrive, and earlier ranges of the output leave, meanwhile.
+   // the plan of the whole; but later ranges of the input arrive, and earlier ranges of the output leave, meanwhile. What arrives
+   // from pageable memory is not the input but what the first operator makes of it.
    if (fRangeBatch) {
       for (auto &in : fInputTensorNames)
          if (Slot *s = slot_of(in)) s->last = nOps;
       for (auto &o : fOutputTensorNames)
          if (Slot *s = slot_of(o)) s->first = -1;
+      if (fStaged.kind)
+         if (Slot *s = slot_of(fOperators[fStagedOp]->GetOpOutputTensors()[0])) {
+            s->first = -1;
+            s->last = nOps;
+         }
    }
    fArenaBytes = 0;
    for (size_t i = 0; i < slots.size(); i++) {

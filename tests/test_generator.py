@@ -473,3 +473,22 @@ def test_ranges_of_a_batch_keep_the_arriving_input_and_the_leaving_result_apart(
         assert all(h <= lo or hi <= l for n, (l, h) in slices.items() if n != edge), edge
     small = _emit(configs.mlp_i8(batch=100, with_input=False)[0], "c3_b100").read_text()
     assert "LaunchRange" not in small and "sofie_cuda_slice_rows" not in small
+
+
+@pytest.mark.parametrize("dims", [(1024, 1024, 512, 256, 10), (512, 1024, 1024, 1024, 256)])
+@pytest.mark.parametrize("dynamic", [False, True])
+def test_what_arrives_from_pageable_memory_shares_no_bytes_with_activations(dims, dynamic):
+    """The host quantises a pageable input while it stages it: the first operator's output arrives range by range, on the copy stream,
+    while earlier ranges are computed. It has to lie apart from everything, as the input it stands for."""
+    m, _ = configs.mlp_i8(batch=4096, dims=dims, with_input=False)
+    onnx = onnx_wire.model_to_onnx(m, batch_param="bs") if dynamic else onnx_wire.model_to_onnx(m)
+    text = generated.emit(onnx, "c3_arriving" + ("_dyn" if dynamic else "")).read_text()
+    assert "sofie_cuda_ctx_h2d_quantized(fCtx, dev_q0 + part * " in text
+    slices = {}
+    for off, size, name in re.findall(r"sofie_cuda_ctx_arena\(fCtx, ([^,]+), ([^,]+), reinterpret_cast<void\*\*>\(&dev_(\w+)\)\)", text):
+        o, b = (int(re.search(r"\d+", v).group()) for v in (off, size))      # with a run-time batch: per sample
+        slices[name] = (o, o + b)
+    assert {"x", "q0", "q1", "q2", "q3"} <= set(slices)
+    for edge in ("x", "q0", "q4" if "q4" in slices else "y"):
+        lo, hi = slices[edge]
+        assert all(h <= lo or hi <= l for n, (l, h) in slices.items() if n != edge), edge

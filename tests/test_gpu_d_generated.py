@@ -369,3 +369,16 @@ def test_batch_cut_into_ranges_of_samples(key, batch, dynamic, cuda_device):
 def capi_slice_rows(rows, in_bytes):
     from sofie_b200 import capi
     return capi.load().sofie_cuda_slice_rows(rows, in_bytes, 0, 128)
+
+
+@pytest.mark.parametrize("dynamic", [False, True])
+def test_ranges_of_a_network_whose_layers_shrink(dynamic, cuda_device):
+    """A quantised network whose later activations would fit over the quantised input: from pageable memory, call after call, bit for bit
+    the result of the whole batch in one piece."""
+    batch = 4096
+    m, x = configs.mlp_i8(batch=batch, dims=(1024, 1024, 512, 256, 10))
+    whole = generated.session_from_model(m, "c3_shrink_whole", pipelined=False).infer(x)
+    s = generated.dynamic_session_from_model(m, "c3_shrink_dyn", batch) if dynamic else generated.session_from_model(m, "c3_shrink")
+    assert capi_slice_rows(batch, x[0].nbytes) < batch
+    for _ in range(200):
+        assert np.array_equal(s.infer(x).view(np.uint32), whole.view(np.uint32))
