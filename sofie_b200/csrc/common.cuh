@@ -6,6 +6,9 @@
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
+#include <utility>
 
 #include "sofie_cuda.h"
 
@@ -111,21 +114,25 @@ struct FastDiv {
    }
 };
 
-// Dynamic shared memory above 48 KB has to be allowed per kernel and device once; the launchers call this on every launch.
+// Dynamic shared memory above 48 KB has to be allowed per kernel and device; the launchers call this on every launch. The allowance
+// belongs to the function, for all threads of the process, and setting a smaller one lowers it: it is only ever raised here, under
+// one lock, so that no thread's launch (nor the replay of a kernel captured earlier) is refused because another needed less.
 inline cudaError_t allow_smem(const void *kernel, int bytes)
 {
-   struct Done {
-      const void *kernel = nullptr;
-      int device = -1, bytes = 0;
-   };
-   static thread_local Done table[128];
+   static std::mutex mu;
+   static std::map<std::pair<const void *, int>, int> allowed;
    int dev = 0;
    cudaError_t err = cudaGetDevice(&dev);
    if (err != cudaSuccess) return err;
-   Done &e = table[(reinterpret_cast<uintptr_t>(kernel) >> 4) % 128];
-   if (e.kernel == kernel && e.device == dev && e.bytes >= bytes) return cudaSuccess;
-   err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-   if (err == cudaSuccess) e = {kernel, dev, bytes};
+   try {
+      std::lock_guard<std::mutex> lock(mu);
+      int &now = allowed[{kernel, dev}];
+      if (now >= bytes) return cudaSuccess;
+      err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      if (err == cudaSuccess) now = bytes;
+   } catch (...) {
+      return cudaErrorMemoryAllocation; // the callers are C functions
+   }
    return err;
 }
 

@@ -989,7 +989,7 @@ int sofie_cuda_ctx_graph_end(sofie_cuda_ctx *ctx)
    SOFIE_CUDA_TRY(cudaStreamEndCapture(ctx->stream, &ctx->graph));
    SOFIE_CUDA_TRY(cudaGraphInstantiate(&ctx->graph_exec, ctx->graph, 0));
    // A graph of one kernel saves nothing and its launch costs twice a kernel's (4.5 against 2.2 us of host time): the kernel
-   // is launched with the parameters the graph holds
+   // is launched with the parameters the graph holds (its shared memory was allowed when it was captured, and stays so: allow_smem)
    ctx->only_kernel = {};
    size_t nodes = 0;
    SOFIE_CUDA_TRY(cudaGraphGetNodes(ctx->graph, nullptr, &nodes));

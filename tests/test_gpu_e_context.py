@@ -115,3 +115,40 @@ def test_operator_timers_and_run_resident_of_the_emitted_session(cuda_device, mo
     plain.run_resident()
     capi.call("sofie_cuda_ctx_check", plain.ctx)
     assert np.array_equal(plain.infer(x), y0)
+
+
+def test_shared_memory_allowed_for_one_network_survives_a_smaller_one_on_another_thread(cuda_device):
+    """The allowance of a kernel's dynamic shared memory belongs to the process: a thread whose network needs less must not take it away
+    from one whose network needs more, neither for operator calls nor for the replay of a captured Session of one kernel."""
+    import threading
+    from sofie_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(5)
+
+    def net(width):
+        w = [torch.randn(width, 64, device="cuda", generator=g), torch.randn(10, width, device="cuda", generator=g)]
+        x = torch.randn(40, 64, device="cuda", generator=g)
+        return lambda: ops.mlp_f32(x, w, [None, None], [1, 0], [1, 1]).cpu()
+    large, small = net(240), net(96)
+    sessions = {}
+    for width in (240, 96):
+        m, x = configs.mlp_f32(batch=40, dims=(64, width, 10))
+        s = generated.session_from_model(m, f"c1_smem_{width}")
+        sessions[width] = (s, x)
+    first = {}
+
+    def elsewhere(f):
+        box = []
+        t = threading.Thread(target=lambda: box.append(f()))
+        t.start()
+        t.join()
+        assert box, "the call on the other thread failed"
+        return box[0]
+    first["large"] = large()
+    s, x = sessions[240]
+    first[240] = [s.infer(x) for _ in range(3)][-1]      # the third is a replay
+    for _ in range(2):
+        elsewhere(small)
+        s2, x2 = sessions[96]
+        elsewhere(lambda: s2.infer(x2))
+        assert torch.equal(large(), first["large"])
+        assert np.array_equal(s.infer(x), first[240])
