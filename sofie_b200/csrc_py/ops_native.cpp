@@ -50,6 +50,16 @@ int64_t integer(PyObject *o)
    return v;
 }
 int32_t i32(PyObject *o) { return static_cast<int32_t>(integer(o)); }
+// what int(o) gives: a zero point may come as a float or as a NumPy or torch scalar
+int32_t as_int32(PyObject *o)
+{
+   PyObject *v = PyNumber_Long(o);
+   if (!v) throw Raised();
+   const long long n = PyLong_AsLongLong(v);
+   Py_DECREF(v);
+   if (n == -1 && PyErr_Occurred()) throw Raised();
+   return static_cast<int32_t>(n);
+}
 float f32(PyObject *o)
 {
    const double v = PyFloat_AsDouble(o);
@@ -62,13 +72,15 @@ bool truth(PyObject *o)
    if (v < 0) throw Raised();
    return v != 0;
 }
+// The first N of a sequence of integers: of exactly N, or of N or more.
 template <size_t N>
-std::array<int32_t, N> ints(PyObject *o)
+std::array<int32_t, N> ints(PyObject *o, bool exactly)
 {
    PyObject *s = PySequence_Fast(o, "a sequence of integers is expected");
    if (!s) throw Raised();
    std::array<int32_t, N> v{};
-   const bool fits = PySequence_Fast_GET_SIZE(s) == (Py_ssize_t)N;
+   const Py_ssize_t size = PySequence_Fast_GET_SIZE(s);
+   const bool fits = exactly ? size == (Py_ssize_t)N : size >= (Py_ssize_t)N;
    try {
       for (size_t i = 0; fits && i < N; i++) v[i] = i32(PySequence_Fast_GET_ITEM(s, i));
    } catch (...) {
@@ -76,15 +88,32 @@ std::array<int32_t, N> ints(PyObject *o)
       throw;
    }
    Py_DECREF(s);
-   if (!fits) raise(PyExc_ValueError, "a sequence of another length is expected");
+   if (!fits) raise(exactly ? PyExc_ValueError : PyExc_IndexError, "a sequence of another length is expected");
    return v;
 }
+std::array<int32_t, 2> pair(PyObject *o) { return ints<2>(o, false); } // of a longer padding or kernel, the first two
+// the extents of a tensor of rank N
+template <size_t N>
+std::array<int32_t, N> extents(const at::Tensor &t)
+{
+   if (t.dim() != (int64_t)N) raise(PyExc_ValueError, "a tensor of another rank is expected");
+   std::array<int32_t, N> v;
+   for (size_t i = 0; i < N; i++) v[i] = (int32_t)t.size((int64_t)i);
+   return v;
+}
+std::array<int32_t, 4> image_shape(PyObject *shape, const at::Tensor &X) { return shape != Py_None ? ints<4>(shape, true) : extents<4>(X); }
 
 void *stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
 at::Tensor make(at::IntArrayRef shape, at::ScalarType type, const at::Tensor &like)
 {
    return at::Tensor(at::detail::empty_cuda(shape, type, like.device(), std::nullopt));
+}
+// the result of an operator on 32-bit values: of X's type; a type of fewer bytes holds less than the kernel would read and write
+at::Tensor make_like(const at::Tensor &X)
+{
+   if (X.element_size() < 4) raise(PyExc_AssertionError, "a tensor of float32 values is expected");
+   return make(X.sizes(), X.scalar_type(), X);
 }
 at::Tensor make_or(PyObject *out, at::IntArrayRef shape, at::ScalarType type, const at::Tensor &like)
 {
@@ -148,15 +177,11 @@ ConvShape conv_shape(const at::Tensor &X, const at::Tensor &W, PyObject *shape, 
                      const std::array<int32_t, 2> &stride, const std::array<int32_t, 2> &dil, int32_t pool, int32_t y_layout)
 {
    ConvShape c;
-   if (shape != Py_None) {
-      const auto s = ints<4>(shape);
-      c.N = s[0], c.C = s[1], c.H = s[2], c.W = s[3];
-   } else {
-      c.N = (int32_t)X.size(0), c.C = (int32_t)X.size(1), c.H = (int32_t)X.size(2), c.W = (int32_t)X.size(3);
-   }
+   const auto s = image_shape(shape, X);
+   c.N = s[0], c.C = s[1], c.H = s[2], c.W = s[3];
    c.Cout = (int32_t)W.size(0);
    if (packed) {
-      const auto k = ints<2>(kernel);
+      const auto k = pair(kernel);
       c.kH = k[0], c.kW = k[1];
    } else {
       c.kH = (int32_t)W.size(2), c.kW = (int32_t)W.size(3);
@@ -174,7 +199,7 @@ ConvShape conv_shape(const at::Tensor &X, const at::Tensor &W, PyObject *shape, 
 PyObject *conv2d_f32(Args a)
 {
    const at::Tensor &X = tensor(a[0]), &W = tensor(a[1]);
-   const auto pad = ints<2>(a[4]), stride = ints<2>(a[5]), dil = ints<2>(a[6]);
+   const auto pad = pair(a[4]), stride = pair(a[5]), dil = pair(a[6]);
    require(stride[0] > 0 && stride[1] > 0, "strides must be positive");
    const int32_t pool = i32(a[9]), yl = i32(a[11]);
    const bool packed = truth(a[12]);
@@ -193,14 +218,14 @@ PyObject *conv2d_f32(Args a)
 PyObject *qlinear_conv2d(Args a)
 {
    const at::Tensor &X = tensor(a[0]), &W = tensor(a[1]);
-   const auto pad = ints<2>(a[5]), stride = ints<2>(a[6]);
+   const auto pad = pair(a[5]), stride = pair(a[6]);
    require(stride[0] > 0 && stride[1] > 0, "strides must be positive");
    const int32_t pool = i32(a[10]), yl = i32(a[12]);
    const bool packed = truth(a[13]);
    const ConvShape c = conv_shape(X, W, a[4], a[14], packed, pad, stride, {1, 1}, pool, yl);
    at::Tensor Y = make(c.y, at::kByte, X);
    const sofie_qconv2d_desc d = {c.N, c.C, c.H, c.W, c.Cout, c.kH, c.kW, pad[0], pad[1], stride[0], stride[1], i32(a[11]), yl, packed,
-                                 i32(a[7]), i32(a[8]), truth(a[9]), pool};
+                                 as_int32(a[7]), as_int32(a[8]), truth(a[9]), pool};
    void *const s = ::stream();
    const uint8_t *pX = as<uint8_t>(X);
    const int8_t *pW = as<int8_t>(W);
@@ -215,7 +240,7 @@ PyObject *qlinear_conv2d(Args a)
 PyObject *relu_f32(Args a)
 {
    const at::Tensor &X = tensor(a[0]);
-   at::Tensor Y = make_or(a[1], X.sizes(), at::kFloat, X);
+   at::Tensor Y = a[1] == Py_None ? make_like(X) : tensor(a[1]);
    void *const s = stream();
    const float *pX = as<float>(X);
    float *pY = as<float>(Y);
@@ -228,7 +253,7 @@ PyObject *relu_f32(Args a)
 PyObject *unary_f32(Args a)
 {
    const at::Tensor &X = tensor(a[0]);
-   at::Tensor Y = make(X.sizes(), at::kFloat, X);
+   at::Tensor Y = make_like(X);
    void *const s = stream();
    const int32_t op = i32(a[1]);
    const float alpha = f32(a[2]);
@@ -268,7 +293,7 @@ PyObject *binary_f32(Args a)
 PyObject *batchnorm_f32(Args a)
 {
    const at::Tensor &X = tensor(a[0]);
-   at::Tensor Y = make(X.sizes(), at::kFloat, X);
+   at::Tensor Y = make_like(X);
    const sofie_batchnorm_desc d = {i32(a[4]), i32(a[5]), i32(a[6]), i32(a[7]), truth(a[8])};
    void *const s = stream();
    const float *pX = as<float>(X), *ps = as<float>(a[1]), *pb = as<float>(a[2]), *pm = as<float>(a[3]);
@@ -281,12 +306,10 @@ PyObject *batchnorm_f32(Args a)
 PyObject *pool2d_f32(Args a)
 {
    const at::Tensor &X = tensor(a[0]);
-   const auto k = ints<2>(a[2]), st = ints<2>(a[3]);
-   const auto p = ints<4>(a[4]);
+   const auto k = pair(a[2]), st = pair(a[3]);
+   const auto p = ints<4>(a[4], true);
    require(st[0] > 0 && st[1] > 0, "strides must be positive");
-   std::array<int32_t, 4> n;
-   if (a[7] != Py_None) n = ints<4>(a[7]);
-   else n = {(int32_t)X.size(0), (int32_t)X.size(1), (int32_t)X.size(2), (int32_t)X.size(3)};
+   const auto n = image_shape(a[7], X);
    auto out = [&](int i) {
       const int64_t v = n[2 + i] + p[i] + p[2 + i] - k[i] + 1;
       return v <= 0 ? int64_t(0) : (v + st[i] - 1) / st[i];
@@ -306,11 +329,9 @@ PyObject *pool2d_f32(Args a)
 PyObject *maxpool2d_u8(Args a)
 {
    const at::Tensor &X = tensor(a[0]);
-   const auto k = ints<2>(a[1]), st = ints<2>(a[2]);
+   const auto k = pair(a[1]), st = pair(a[2]);
    require(st[0] > 0 && st[1] > 0, "strides must be positive");
-   std::array<int32_t, 4> n;
-   if (a[4] != Py_None) n = ints<4>(a[4]);
-   else n = {(int32_t)X.size(0), (int32_t)X.size(1), (int32_t)X.size(2), (int32_t)X.size(3)};
+   const auto n = image_shape(a[4], X);
    const int64_t oH = n[2] < k[0] ? 0 : (n[2] - k[0]) / st[0] + 1, oW = n[3] < k[1] ? 0 : (n[3] - k[1]) / st[1] + 1;
    const int32_t layout = i32(a[3]);
    at::Tensor Y = layout == SOFIE_LAYOUT_NHWC ? make({n[0], oH, oW, n[1]}, at::kByte, X) : make({n[0], n[1], oH, oW}, at::kByte, X);
@@ -332,7 +353,7 @@ PyObject *softmax_f32(Args a)
    for (int64_t i = 0; i < axis; i++) outer *= (size_t)X.size(i);
    for (int64_t i = axis + 1; i < rank; i++) inner *= (size_t)X.size(i);
    const size_t len = (size_t)X.size(axis);
-   at::Tensor Y = make(X.sizes(), at::kFloat, X);
+   at::Tensor Y = make_like(X);
    void *const s = stream();
    const float *pX = as<float>(X);
    float *pY = as<float>(Y);
@@ -365,7 +386,7 @@ PyObject *quantize_u8(Args a)
    at::Tensor Y = make(X.sizes(), at::kByte, X);
    void *const s = stream();
    const float scale = f32(a[1]);
-   const int32_t zp = i32(a[2]);
+   const int32_t zp = as_int32(a[2]);
    const float *pX = as<float>(X);
    uint8_t *pY = as<uint8_t>(Y);
    const size_t n = (size_t)X.numel();
@@ -379,7 +400,7 @@ PyObject *dequantize_u8(Args a)
    at::Tensor Y = make(X.sizes(), at::kFloat, X);
    void *const s = stream();
    const float scale = f32(a[1]);
-   const int32_t zp = i32(a[2]);
+   const int32_t zp = as_int32(a[2]);
    const uint8_t *pX = as<uint8_t>(X);
    float *pY = as<float>(Y);
    const size_t n = (size_t)X.numel();
@@ -410,9 +431,10 @@ PyObject *qlinear_matmul(Args a)
 {
    const at::Tensor &A = tensor(a[0]), &W = tensor(a[1]);
    const bool nk = truth(a[4]), to_f32 = a[7] != Py_None;
-   const int64_t M = A.size(0), K = A.size(1), N = W.size(nk ? 0 : 1);
+   const auto mk = extents<2>(A);
+   const int64_t M = mk[0], K = mk[1], N = W.size(nk ? 0 : 1);
    at::Tensor Y = make({M, N}, to_f32 ? at::kFloat : at::kByte, A);
-   const sofie_qgemm_desc d = {(int32_t)M, (int32_t)N, (int32_t)K, nk, i32(a[5]), truth(a[6])};
+   const sofie_qgemm_desc d = {(int32_t)M, (int32_t)N, (int32_t)K, nk, as_int32(a[5]), truth(a[6])};
    void *const s = stream();
    const uint8_t *pA = as<uint8_t>(A);
    const int8_t *pW = as<int8_t>(W);
@@ -432,7 +454,8 @@ PyObject *qlinear_matmul(Args a)
 PyObject *gemm_e4m3(Args a)
 {
    const at::Tensor &A = tensor(a[0]), &W = tensor(a[1]);
-   const int64_t M = A.size(0), K = A.size(1), N = W.size(0);
+   const auto mk = extents<2>(A);
+   const int64_t M = mk[0], K = mk[1], N = W.size(0);
    const sofie_fp8_gemm_desc d = {(int32_t)M, (int32_t)N, (int32_t)K, f32(a[3]), f32(a[4]), truth(a[5]), f32(a[6])};
    void *const s = stream();
    const uint8_t *pA = as<uint8_t>(A), *pW = as<uint8_t>(W);
@@ -450,10 +473,10 @@ PyObject *gemm_e4m3(Args a)
    uint8_t *pq = Yq.defined() ? as<uint8_t>(Yq) : nullptr;
    SOFIE_CALL(sofie_cuda_gemm_e4m3, s, &d, pA, pW, pb, pY, pq);
    PyObject *y = Y.defined() ? THPVariable_Wrap(Y) : Py_NewRef(Py_None), *q = Yq.defined() ? THPVariable_Wrap(Yq) : Py_NewRef(Py_None);
-   PyObject *pair = PyTuple_New(2);
-   PyTuple_SET_ITEM(pair, 0, y);
-   PyTuple_SET_ITEM(pair, 1, q);
-   return pair;
+   PyObject *both = PyTuple_New(2);
+   PyTuple_SET_ITEM(both, 0, y);
+   PyTuple_SET_ITEM(both, 1, q);
+   return both;
 }
 
 template <PyObject *(*F)(Args), int N>

@@ -200,6 +200,19 @@ def unary_f32(X, op, alpha=0.0):
     return _native().unary_f32(X, UNARY_OPS[op], alpha)
 
 
+def binary_strides(a_shape, b_shape):
+    """Output shape and the rank-4 shape / element strides (0 along broadcast dimensions) of A op B: the descriptor binary_f32 passes."""
+    out = tuple(torch.broadcast_shapes(tuple(a_shape), tuple(b_shape)))
+    if len(out) > 4:
+        raise ValueError("binary operators are built for rank <= 4")
+
+    def strides(shape):
+        shape = (1,) * (4 - len(shape)) + tuple(shape)
+        return [0 if n == 1 else int(np.prod(shape[i + 1:], dtype=np.int64)) for i, n in enumerate(shape)]
+
+    return out, [1] * (4 - len(out)) + list(out), strides(a_shape), strides(b_shape)
+
+
 def binary_f32(A, B, op):
     return _native().binary_f32(A, B, BINARY_OPS[op])
 
@@ -261,7 +274,7 @@ def qlinear_matmul(A, W, mult, corr, *, w_is_nk=True, y_zp=0, relu=False):
 
 def qlinear_matmul_f32(A, W, mult, corr, y_scale, *, w_is_nk=True, y_zp=0, relu=False):
     """QLinearMatMul + DequantizeLinear (same zero point) in one pass: float32 (q - y_zp) * y_scale."""
-    return _native().qlinear_matmul(A, W, mult, corr, w_is_nk, y_zp, relu, y_scale)
+    return _native().qlinear_matmul(A, W, mult, corr, w_is_nk, y_zp, relu, float(y_scale))
 
 
 def qlinear_conv2d(X, W, mult, bias=None, *, shape=None, pad=(0, 0), stride=(1, 1), x_zp=0, y_zp=0, relu=False,

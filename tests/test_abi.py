@@ -130,3 +130,41 @@ def test_host_quantisation_gives_the_operators_bytes(kind, zp):
     assert y[0] == (0 if kind == 1 else 0x7F)
     with pytest.raises(RuntimeError):
         capi.call("sofie_cuda_selftest_host_quantize", y.ctypes.data, nan.ctypes.data, 1, kind, 0.0, zp)
+
+
+def test_operator_calls_refuse_what_they_refused():
+    """Tensors of another rank, short sequences and a missing scale are refused before anything is launched (or a device is needed)."""
+    import torch
+    from sofie_b200 import ops
+    image, weights, row = torch.zeros(2, 3, 4, 4, 1), torch.zeros(2, 3, 3, 3), torch.zeros(4)
+    bytes3, wi = torch.zeros(2, 3, 4, dtype=torch.uint8), torch.zeros(4, 3, dtype=torch.int8)
+    for call in (lambda: ops.conv2d_f32(image, weights), lambda: ops.conv2d_f32(torch.zeros(2, 3, 4, 4), weights, shape=(2, 3, 4)),
+                 lambda: ops.qlinear_conv2d(image, weights, row), lambda: ops.pool2d_f32(image), lambda: ops.maxpool2d_u8(image),
+                 lambda: ops.pool2d_f32(torch.zeros(2, 3, 4, 4), pads=(0, 0, 0)), lambda: ops.qlinear_matmul(bytes3, wi, row, row),
+                 lambda: ops.gemm_e4m3(bytes3, wi.view(torch.uint8)), lambda: ops.gemm_e4m3_f32(bytes3, wi.view(torch.uint8))):
+        with pytest.raises(ValueError):
+            call()
+    with pytest.raises(IndexError):
+        ops.conv2d_f32(torch.zeros(2, 3, 4, 4), weights, pad=(1,))
+    for call in (ops.relu_f32, ops.softmax_f32, lambda t: ops.unary_f32(t, "Exp")):
+        with pytest.raises(AssertionError):
+            call(torch.zeros(4, dtype=torch.bfloat16))
+    for call in (lambda: ops.qlinear_matmul_f32(bytes3[0], wi, row, row, None), lambda: ops.conv2d_f32(torch.zeros(2, 3, 4, 4), weights, pad=(1.5, 1.0))):
+        with pytest.raises(TypeError):
+            call()
+
+
+@pytest.mark.parametrize("a,b", [((2, 3, 4, 5), (3, 1, 1)), ((7,), (4, 1)), ((1, 6), (5, 1, 6)), ((), (2, 2)), ((0, 3), (1,))])
+def test_strides_of_a_broadcast_operand(a, b):
+    import torch
+    from sofie_b200 import ops
+    out, shape4, sa, sb = ops.binary_strides(a, b)
+    assert out == tuple(torch.broadcast_shapes(a, b)) and shape4 == [1] * (4 - len(out)) + list(out)
+    for operand, strides in ((a, sa), (b, sb)):
+        full = (1,) * (4 - len(operand)) + tuple(operand)
+        want = torch.empty(operand).reshape(full).stride()
+        assert all(s == (0 if n == 1 else w) for n, s, w in zip(full, strides, want) if 0 not in operand)
+    with pytest.raises(ValueError):
+        ops.binary_strides((1, 1, 1, 1, 2), (1,))
+    with pytest.raises(RuntimeError):
+        ops.binary_strides((2,), (3,))

@@ -771,3 +771,24 @@ def test_pool2d_odd_images(shape, k, s, pads, mode):
         t = dev(x if layout == 0 else x.transpose(0, 2, 3, 1))
         got = ops.pool2d_f32(t, mode=mode, kernel=(k, k), stride=(s, s), pads=pads, layout=layout, shape=shape).cpu().numpy()
         assert rel_err(got if layout == 0 else got.transpose(0, 3, 1, 2), want) <= FP32_TOL
+
+
+def test_operator_calls_take_the_arguments_they_took(cuda_device):
+    """Zero points of any number type, paddings and kernels longer than two, and results of the input's type."""
+    g = torch.Generator(device="cuda").manual_seed(11)
+    x = torch.randn(3, 5, 8, 8, device="cuda", generator=g)
+    q = ops.quantize_u8(x, 0.02, 128)
+    for zp in (128.0, np.float32(128), np.int64(128), torch.tensor(128)):
+        assert torch.equal(ops.quantize_u8(x, 0.02, zp), q)
+        assert torch.equal(ops.dequantize_u8(q, 0.02, zp), ops.dequantize_u8(q, 0.02, 128))
+    w = torch.randn(4, 5, 3, 3, device="cuda", generator=g)
+    assert torch.equal(ops.conv2d_f32(x, w, pad=[1, 1, 1, 1], stride=(1, 1, 7), dil=np.array([1, 1])), ops.conv2d_f32(x, w, pad=(1, 1)))
+    assert torch.equal(ops.pool2d_f32(x, kernel=(2, 2, 2), stride=[2, 2]), ops.pool2d_f32(x))
+    wi = np.random.default_rng(3).integers(-127, 128, (6, 64), dtype=np.int8)
+    mult, corr = ops.qlinear_prepare(wi, True, 0.02, 128, np.full(6, 0.01, np.float32), 0.05, None, "cuda")
+    a, wd = q.view(15, 64), torch.from_numpy(wi).cuda()
+    assert torch.equal(ops.qlinear_matmul(a, wd, mult, corr, y_zp=128.0), ops.qlinear_matmul(a, wd, mult, corr, y_zp=128))
+    assert torch.equal(ops.qlinear_matmul_f32(a, wd, mult, corr, np.float64(0.05), y_zp=128.0), ops.qlinear_matmul_f32(a, wd, mult, corr, 0.05, y_zp=128))
+    bits = torch.zeros(16, dtype=torch.int32, device="cuda")
+    for f in (ops.relu_f32, ops.softmax_f32, lambda t: ops.unary_f32(t, "Neg")):
+        assert f(bits).dtype == torch.int32 and f(x).dtype == torch.float32
