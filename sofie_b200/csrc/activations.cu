@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(kActThreads) binary_bcast_f32_kernel(BcastDims
    }
 }
 
-// The same without the limit of 2^31 elements: the output index is split into up to four coordinates; a broadcast dimension of an
+// The same without the limits of 2^31 outputs and 32-bit offsets: the output index is split into up to four coordinates; a broadcast dimension of an
 // operand has stride 0.
 __global__ void binary_bcast_large_f32_kernel(sofie_binary_desc d, const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ Y, size_t n)
 {
@@ -301,7 +301,16 @@ extern "C" int sofie_cuda_binary_f32(void *stream, const sofie_binary_desc *d, c
       SOFIE_CUDA_TRY(launch_dependent(binary_same_f32_kernel, dim3(act_grid(n / vec + 1)), dim3(kActThreads), 0, s, d->op, A, B, Y, n, vec));
       return SOFIE_CUDA_OK;
    }
-   if (n >= (size_t(1) << 31) - 4096 * 1024) {
+   // coordinates of the outputs and offsets of the operands in 32 bits, where they fit: an operand may be a view of something larger
+   uint64_t last_a = 0, last_b = 0;
+   bool narrow = n < (size_t(1) << 31) - 4096 * 1024;
+   for (int k = 0; k < 4; k++) {
+      if (d->shape[k] == 1) continue;
+      narrow = narrow && d->a_stride[k] <= UINT32_MAX && d->b_stride[k] <= UINT32_MAX;
+      last_a += (uint64_t)(d->shape[k] - 1) * (uint64_t)d->a_stride[k];
+      last_b += (uint64_t)(d->shape[k] - 1) * (uint64_t)d->b_stride[k];
+   }
+   if (!narrow || last_a > UINT32_MAX || last_b > UINT32_MAX) {
       SOFIE_CUDA_TRY(launch_dependent(binary_bcast_large_f32_kernel, dim3(act_grid(n)), dim3(kActThreads), 0, s, *d, A, B, Y, n));
       return SOFIE_CUDA_OK;
    }

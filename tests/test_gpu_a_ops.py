@@ -792,3 +792,20 @@ def test_operator_calls_take_the_arguments_they_took(cuda_device):
     bits = torch.zeros(16, dtype=torch.int32, device="cuda")
     for f in (ops.relu_f32, ops.softmax_f32, lambda t: ops.unary_f32(t, "Neg")):
         assert f(bits).dtype == torch.int32 and f(x).dtype == torch.float32
+
+
+@pytest.mark.parametrize("where", ["a", "b"])
+def test_binary_operand_that_spans_more_than_32_bits(where, cuda_device):
+    """The strides of a descriptor are 64-bit numbers: rows of a view 2^32 elements apart, and just below."""
+    big = torch.empty((1 << 32) + 64, device="cuda")
+    other = torch.arange(12, device="cuda", dtype=torch.float32) + 1.
+    for stride in ((1 << 32) + 5, 1 << 32, (1 << 32) - 7):
+        big[:6], big[stride:stride + 6] = torch.arange(6.) + 10., torch.arange(6.) + 100.
+        i64 = C.c_int64 * 4
+        view, dense = i64(stride, 0, 3, 1), i64(6, 0, 3, 1)
+        d = capi.BinaryDesc(ops.BINARY_OPS["Sub"], i64(2, 1, 2, 3), view if where == "a" else dense, dense if where == "a" else view)
+        y = torch.empty(12, device="cuda")
+        p = [C.c_void_p(t.data_ptr()) for t in ((big, other) if where == "a" else (other, big))]
+        capi.call("sofie_cuda_binary_f32", C.c_void_p(torch.cuda.current_stream().cuda_stream), C.byref(d), *p, C.c_void_p(y.data_ptr()))
+        rows = torch.cat([big[:6], big[stride:stride + 6]])
+        assert torch.equal(y, rows - other if where == "a" else other - rows)
