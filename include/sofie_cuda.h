@@ -97,6 +97,8 @@ int sofie_cuda_ctx_wait_part(sofie_cuda_ctx *ctx, int part);
 #define SOFIE_CUDA_STAGE_E4M3 2
 int sofie_cuda_ctx_pageable(sofie_cuda_ctx *ctx, const void *src_host);
 int sofie_cuda_ctx_h2d_quantized(sofie_cuda_ctx *ctx, uint8_t *dst_device, const float *src_host, size_t n, int kind, float scale, int32_t zp, int part);
+/* The floats that the n quantised values on the device stand for; quantised again they are the same bytes. */
+int sofie_cuda_ctx_unquantize(sofie_cuda_ctx *ctx, const uint8_t *src_device, float *dst_device, size_t n, int kind, float scale, int32_t zp);
 /* Lets the helper threads start on the next part (`bytes`: of its destination) while the caller launches the kernels of this one;
  * nothing is done for pinned memory. The source must stay as it is until that part's copy call, or until
  * sofie_cuda_ctx_stage_settle, after which no helper reads it. */
@@ -537,6 +539,8 @@ int sofie_cuda_nhwc_to_nchw_u8(void *stream, const uint8_t *X, uint8_t *Y, int32
 
 /* y = e4m3(x / scale), round to nearest even, saturating. */
 int sofie_cuda_quantize_e4m3_f32(void *stream, const float *X, uint8_t *Y, size_t n, float scale);
+/* y = (value of the code x) * scale; quantising the result with the same scale gives the code again. */
+int sofie_cuda_dequantize_e4m3_f32(void *stream, const uint8_t *X, float *Y, size_t n, float scale);
 int sofie_cuda_quantize_e4m3_bf16(void *stream, const uint16_t *X, uint8_t *Y, size_t n, float scale);
 int sofie_cuda_cast_bf16_f32(void *stream, const uint16_t *X, float *Y, size_t n);
 int sofie_cuda_cast_f32_bf16(void *stream, const float *X, uint16_t *Y, size_t n);

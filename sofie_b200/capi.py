@@ -119,6 +119,7 @@ SIGNATURES = {
     "sofie_cuda_ctx_wait_part": [vp, C.c_int],
     "sofie_cuda_ctx_pageable": [vp, vp],
     "sofie_cuda_ctx_h2d_quantized": [vp, vp, vp, sz, C.c_int, f32, i32, C.c_int],
+    "sofie_cuda_ctx_unquantize": [vp, vp, vp, sz, C.c_int, f32, i32],
     "sofie_cuda_ctx_stage_ahead": [vp, vp, sz, C.c_int, f32, i32],
     "sofie_cuda_ctx_stage_settle": [vp],
     "sofie_cuda_selftest_host_quantize": [vp, vp, sz, C.c_int, f32, i32],
@@ -160,6 +161,7 @@ SIGNATURES = {
     "sofie_cuda_nchw_to_nhwc_u8": [vp, vp, vp, i32, i32, i32, i32],
     "sofie_cuda_nhwc_to_nchw_u8": [vp, vp, vp, i32, i32, i32, i32],
     "sofie_cuda_quantize_e4m3_f32": [vp, vp, vp, sz, f32],
+    "sofie_cuda_dequantize_e4m3_f32": [vp, vp, vp, sz, f32],
     "sofie_cuda_quantize_e4m3_bf16": [vp, vp, vp, sz, f32],
     "sofie_cuda_cast_bf16_f32": [vp, vp, vp, sz],
     "sofie_cuda_cast_f32_bf16": [vp, vp, vp, sz],

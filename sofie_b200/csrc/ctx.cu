@@ -621,6 +621,14 @@ int sofie_cuda_ctx_h2d_quantized(sofie_cuda_ctx *ctx, uint8_t *dst, const float 
    return SOFIE_CUDA_OK;
 }
 
+int sofie_cuda_ctx_unquantize(sofie_cuda_ctx *ctx, const uint8_t *src, float *dst, size_t n, int kind, float scale, int32_t zp)
+{
+   SOFIE_REQUIRE(ctx && src && dst, "NULL argument");
+   SOFIE_REQUIRE(kind == SOFIE_CUDA_STAGE_U8 || kind == SOFIE_CUDA_STAGE_E4M3, "no quantisation named");
+   DeviceGuard guard(ctx->device);
+   return kind == SOFIE_CUDA_STAGE_U8 ? sofie_cuda_dequantize_u8(ctx->stream, src, dst, n, scale, zp) : sofie_cuda_dequantize_e4m3_f32(ctx->stream, src, dst, n, scale);
+}
+
 int sofie_cuda_ctx_stage_ahead(sofie_cuda_ctx *ctx, const void *src, size_t bytes, int kind, float scale, int32_t zp)
 {
    SOFIE_REQUIRE(ctx && src, "NULL argument");

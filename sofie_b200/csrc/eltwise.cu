@@ -3,6 +3,7 @@
 // pointers allow it, grids sized as a multiple of the SM count.
 #include "common.cuh"
 
+#include <cuda_fp16.h>
 #include <cuda_fp8.h>
 #include <cfloat>
 
@@ -575,6 +576,15 @@ __device__ __forceinline__ uint8_t to_e4m3(float x)
    return (uint8_t)__nv_cvt_float_to_fp8(x, __NV_SATFINITE, __NV_E4M3);
 }
 
+// y = value of the E4M3 code times scale. Off every timed path (a Session's input brought back from its codes): one value per thread.
+__global__ void dequantize_e4m3_kernel(const uint8_t *__restrict__ X, float *__restrict__ Y, size_t n, float scale)
+{
+   griddep_launch_dependents();
+   griddep_wait(); // X is the previous kernel's output
+   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+      Y[i] = __fmul_rn(__half2float(__half(__nv_cvt_fp8_to_halfraw(X[i], __NV_E4M3))), scale);
+}
+
 // Scalar forms: the tail of a tensor and unaligned tensors.
 template <typename In>
 __global__ void quantize_e4m3_kernel(const In *__restrict__ X, uint8_t *__restrict__ Y, size_t begin, size_t n, float scale_in,
@@ -896,6 +906,13 @@ int sofie_cuda_quantize_e4m3_f32(void *stream, const float *X, uint8_t *Y, size_
    SOFIE_REQUIRE(X && Y && scale > 0.f, "bad arguments");
    if (n == 0) return SOFIE_CUDA_OK;
    return launch_quantize_e4m3<float>(as_stream(stream), X, Y, n, scale);
+}
+int sofie_cuda_dequantize_e4m3_f32(void *stream, const uint8_t *X, float *Y, size_t n, float scale)
+{
+   SOFIE_REQUIRE(X && Y && scale > 0.f, "bad arguments");
+   if (n == 0) return SOFIE_CUDA_OK;
+   SOFIE_CUDA_TRY(launch_dependent(dequantize_e4m3_kernel, dim3(grid_for(n)), dim3(kThreads), 0, as_stream(stream), X, Y, n, scale));
+   return SOFIE_CUDA_OK;
 }
 int sofie_cuda_quantize_e4m3_bf16(void *stream, const uint16_t *X, uint8_t *Y, size_t n, float scale)
 {

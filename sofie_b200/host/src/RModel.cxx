@@ -624,11 +624,14 @@ void RModel::PlanArena()
          if (Slot *s = slot_of(in)) s->last = nOps;
       for (auto &o : fOutputTensorNames)
          if (Slot *s = slot_of(o)) s->first = -1;
-      if (fStaged.kind)
-         if (Slot *s = slot_of(fOperators[fStagedOp]->GetOpOutputTensors()[0])) {
-            s->first = -1;
-            s->last = nOps;
-         }
+   }
+   // (RunResident goes back to it, and to the input that it restores from it, after the last operator.)
+   if (fStaged.kind) {
+      if (Slot *s = slot_of(fOperators[fStagedOp]->GetOpOutputTensors()[0])) {
+         if (fRangeBatch) s->first = -1;
+         s->last = nOps;
+      }
+      if (Slot *s = slot_of(fInputTensorNames[0])) s->last = nOps;
    }
    fArenaBytes = 0;
    for (size_t i = 0; i < slots.size(); i++) {
@@ -1030,7 +1033,17 @@ void RModel::GenerateInfer()
    }
    // Every kernel of one inference on the inputs of the previous infer() call, which are still on the device:
    // no copy in either direction and no wait (for callers that time or pipeline the device work themselves).
+   // Where the host quantised that input, the first call brings the floats back, so that the first operator has its input too.
    fGC += "void RunResident() {\n";
+   if (fStaged.kind) {
+      // the last input came quantised: its values are on the device as the first operator's output, and the values those stand for
+      // quantise to the same bytes again
+      const std::string &in = fInputTensorNames[0], &q = fOperators[fStagedOp]->GetOpOutputTensors()[0];
+      fGC += "   if (fConverted) {\n";
+      fGC += "      Check(sofie_cuda_ctx_unquantize(fCtx, " + EMIT::Dev(q) + ", " + EMIT::Dev(in) + ", " + std::to_string(ConvertShapeToLength(GetTensorShape(in))) + ", " +
+             std::to_string(fStaged.kind) + ", " + EMIT::FloatLit(fStaged.scale) + ", " + std::to_string(fStaged.zp) + "), \"sofie_cuda_ctx_unquantize\");\n";
+      fGC += "      fConverted = false;\n      fGraphReady = false;\n   }\n";
+   }
    if (pipelined) fGC += "   for (int part = 0; part < " + std::to_string(fUploadParts) + "; part++) LaunchHead(part);\n";
    fGC += "   Run();\n";
    fGC += "}\n\n";

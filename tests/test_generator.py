@@ -492,3 +492,23 @@ def test_what_arrives_from_pageable_memory_shares_no_bytes_with_activations(dims
     for edge in ("x", "q0", "q4" if "q4" in slices else "y"):
         lo, hi = slices[edge]
         assert all(h <= lo or hi <= l for n, (l, h) in slices.items() if n != edge), edge
+
+
+@pytest.mark.parametrize("dynamic", [False, True])
+def test_run_resident_has_its_input_after_a_quantised_upload(dynamic):
+    """After an infer() from pageable memory the device holds the quantised input only: RunResident() restores the floats first, and the
+    quantised tensor keeps its bytes until then."""
+    m, _ = configs.mlp_i8(batch=64, dims=(512, 256, 128, 64, 10), with_input=False)
+    onnx = onnx_wire.model_to_onnx(m, batch_param="bs") if dynamic else onnx_wire.model_to_onnx(m)
+    text = generated.emit(onnx, "c3_resident_plan" + ("_dyn" if dynamic else "")).read_text()
+    body = text[text.index("void RunResident() {"):]
+    body = body[:body.index("\n}\n")]
+    assert re.search(r"if \(fConverted\) \{\n\s+Check\(sofie_cuda_ctx_unquantize\(fCtx, dev_q0, dev_x, ", body)
+    assert body.index("fConverted = false;") < body.index("Run();")
+    slices = {}
+    for off, size, name in re.findall(r"sofie_cuda_ctx_arena\(fCtx, ([^,]+), ([^,]+), reinterpret_cast<void\*\*>\(&dev_(\w+)\)\)", text):
+        o, b = (int(re.search(r"\d+", v).group()) for v in (off, size))
+        slices[name] = (o, o + b)
+    for kept in ("q0", "x"):
+        lo, hi = slices[kept]
+        assert all(h <= lo or hi <= l for n, (l, h) in slices.items() if n != kept), kept

@@ -2,6 +2,7 @@
 ends by itself, reports once, and the context keeps computing), the per-operator device timers of the emitted
 Launch(), Session::RunResident, and two Sessions that do not see each other's failures."""
 import ctypes as C
+import re
 
 import numpy as np
 import pytest
@@ -152,3 +153,46 @@ def test_shared_memory_allowed_for_one_network_survives_a_smaller_one_on_another
         elsewhere(lambda: s2.infer(x2))
         assert torch.equal(large(), first["large"])
         assert np.array_equal(s.infer(x), first[240])
+
+
+@pytest.mark.parametrize("kind", ["u8", "u8 ranges", "e4m3"])
+def test_run_resident_after_an_input_the_host_quantised(kind, cuda_device):
+    """RunResident() runs every kernel of one inference, QuantizeLinear too, on the last infer()'s input -- also when that input was
+    pageable and only its quantised form is on the device. The result of every repetition is the one infer() gave."""
+    if kind == "e4m3":
+        m, x = configs.gemm_chain_fp8(rows=64, width=256, layers=4)
+        x[0, :8] = [0., -0., 1e9, -1e9, 1e-9, -1e-9, np.nan, 3.]
+        s = generated.session_from_model(m, "c4_resident", fp8_scales=configs.calibrate_fp8_scales(m, np.nan_to_num(x)))
+    else:
+        m, x = configs.mlp_i8(batch=4096 if "ranges" in kind else 100, dims=(512, 256, 128, 64, 10))
+        x[0, :6] = [0., 1e9, -1e9, np.nan, np.inf, -np.inf]
+        s = generated.session_from_model(m, f"c3_resident_{m.batch()}")
+    y = s.infer(x)
+    text = s.hxx.read_text()
+    where = re.search(r"sofie_cuda_ctx_(arena|host_output)\(fCtx, (\d+)[^&]*&dev_" + m.output_name + r"\)", text)
+    out = C.c_void_p()
+    if where.group(1) == "arena":
+        capi.call("sofie_cuda_ctx_arena", s.ctx, int(where.group(2)), y.nbytes, C.byref(out))
+    for _ in range(3):
+        s.run_resident()
+        capi.call("sofie_cuda_ctx_check", s.ctx)
+        if where.group(1) == "arena":
+            again = np.empty_like(y)
+            capi.call("sofie_cuda_ctx_d2h", s.ctx, again.ctypes.data_as(C.c_void_p), out, y.nbytes)
+            assert np.array_equal(again.view(np.uint32), y.view(np.uint32))
+    for _ in range(2):
+        assert np.array_equal(s.infer(x).view(np.uint32), y.view(np.uint32))
+
+
+def test_e4m3_codes_and_their_values(cuda_device):
+    from sofie_b200 import ops
+    codes = torch.arange(256, dtype=torch.uint8, device="cuda")
+    for scale in (1.0, 0.0123, 3.7e5):
+        v = torch.empty(256, device="cuda")
+        capi.call("sofie_cuda_dequantize_e4m3_f32", None, C.c_void_p(codes.data_ptr()), C.c_void_p(v.data_ptr()), 256, scale)
+        torch.cuda.synchronize()
+        want = codes.view(torch.float8_e4m3fn).float() * scale
+        assert torch.equal(v.nan_to_num(-7.), want.nan_to_num(-7.))
+        back = ops.quantize_e4m3(v, scale)
+        number = (codes & 127) != 127
+        assert torch.equal(back[number], codes[number]) and bool((back[~number] & 127 == 127).all())
