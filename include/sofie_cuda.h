@@ -178,6 +178,9 @@ int sofie_cuda_ctx_graph_begin(sofie_cuda_ctx *ctx);
 int sofie_cuda_ctx_graph_end(sofie_cuda_ctx *ctx);
 int sofie_cuda_ctx_graph_launch(sofie_cuda_ctx *ctx);
 int sofie_cuda_ctx_graph_ready(sofie_cuda_ctx *ctx, int *ready);
+/* Sets the captured graph aside and brings the one set aside before back (none at first): a Session whose launches differ between two
+ * kinds of input keeps a graph for each. */
+int sofie_cuda_ctx_graph_swap(sofie_cuda_ctx *ctx);
 
 /* ------------------------------------------------------------------ fp32 contractions ------- */
 #define SOFIE_LAYOUT_NCHW 0

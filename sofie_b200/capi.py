@@ -126,6 +126,7 @@ SIGNATURES = {
     "sofie_cuda_ctx_graph_begin": [vp],
     "sofie_cuda_ctx_graph_end": [vp],
     "sofie_cuda_ctx_graph_launch": [vp],
+    "sofie_cuda_ctx_graph_swap": [vp],
     "sofie_cuda_ctx_graph_ready": [vp, C.POINTER(C.c_int)],
     "sofie_cuda_last_engine": [],
     "sofie_cuda_set_engine": [C.c_int],

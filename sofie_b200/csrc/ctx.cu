@@ -133,9 +133,11 @@ struct sofie_cuda_ctx {
    cudaStream_t result_stream = nullptr; // results that are copied part by part, under the kernels of later parts
    cudaEvent_t ready_event = nullptr;    // a part's kernels are done
    cudaEvent_t landed_event[SOFIE_CUDA_MAX_PARTS] = {};
-   cudaGraph_t graph = nullptr;
-   cudaGraphExec_t graph_exec = nullptr;
-   cudaKernelNodeParams only_kernel = {}; // the captured graph's one kernel (func set), launched without the graph
+   struct Captured {
+      cudaGraph_t graph = nullptr;
+      cudaGraphExec_t exec = nullptr;
+      cudaKernelNodeParams only_kernel = {}; // the graph's one kernel (func set), launched without the graph
+   } captured, kept; // kept: set aside by sofie_cuda_ctx_graph_swap
    bool capturing = false;
    // small results written by the last kernel straight into mapped pinned host memory (no device-to-host copy)
    std::vector<std::pair<char *, size_t>> host_outputs;
@@ -287,8 +289,10 @@ int sofie_cuda_ctx_destroy(sofie_cuda_ctx *ctx)
    if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
    if (ctx->result_stream) cudaStreamSynchronize(ctx->result_stream);
    unregister_stream_status(ctx->stream);
-   if (ctx->graph_exec) cudaGraphExecDestroy(ctx->graph_exec);
-   if (ctx->graph) cudaGraphDestroy(ctx->graph);
+   for (auto *g : {&ctx->captured, &ctx->kept}) {
+      if (g->exec) cudaGraphExecDestroy(g->exec);
+      if (g->graph) cudaGraphDestroy(g->graph);
+   }
    for (void *p : ctx->owned) cudaFree(p);
    if (ctx->arena) cudaFree(ctx->arena);
    for (auto &h : ctx->host_outputs) cudaFreeHost(h.first);
@@ -927,7 +931,7 @@ int sofie_cuda_device_check(int device)
 int sofie_cuda_ctx_timers(sofie_cuda_ctx *ctx, int on)
 {
    SOFIE_REQUIRE(ctx, "NULL ctx");
-   SOFIE_REQUIRE(!ctx->capturing && !ctx->graph_exec, "switch the timers before the first inference is captured");
+   SOFIE_REQUIRE(!ctx->capturing && !ctx->captured.exec && !ctx->kept.exec, "switch the timers before the first inference is captured");
    ctx->timers_on = on != 0;
    return SOFIE_CUDA_OK;
 }
@@ -974,15 +978,9 @@ int sofie_cuda_ctx_graph_begin(sofie_cuda_ctx *ctx)
    SOFIE_REQUIRE(ctx, "NULL ctx");
    SOFIE_REQUIRE(!ctx->capturing, "graph capture already in progress");
    DeviceGuard guard(ctx->device);
-   if (ctx->graph_exec) {
-      cudaGraphExecDestroy(ctx->graph_exec);
-      ctx->graph_exec = nullptr;
-   }
-   if (ctx->graph) {
-      cudaGraphDestroy(ctx->graph);
-      ctx->graph = nullptr;
-      ctx->only_kernel = {};
-   }
+   if (ctx->captured.exec) cudaGraphExecDestroy(ctx->captured.exec);
+   if (ctx->captured.graph) cudaGraphDestroy(ctx->captured.graph);
+   ctx->captured = {};
    SOFIE_CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
    ctx->capturing = true;
    return SOFIE_CUDA_OK;
@@ -994,22 +992,23 @@ int sofie_cuda_ctx_graph_end(sofie_cuda_ctx *ctx)
    SOFIE_REQUIRE(ctx->capturing, "no graph capture in progress");
    DeviceGuard guard(ctx->device);
    ctx->capturing = false;
-   SOFIE_CUDA_TRY(cudaStreamEndCapture(ctx->stream, &ctx->graph));
-   SOFIE_CUDA_TRY(cudaGraphInstantiate(&ctx->graph_exec, ctx->graph, 0));
+   auto &g = ctx->captured;
+   SOFIE_CUDA_TRY(cudaStreamEndCapture(ctx->stream, &g.graph));
+   SOFIE_CUDA_TRY(cudaGraphInstantiate(&g.exec, g.graph, 0));
    // A graph of one kernel saves nothing and its launch costs twice a kernel's (4.5 against 2.2 us of host time): the kernel
    // is launched with the parameters the graph holds (its shared memory was allowed when it was captured, and stays so: allow_smem)
-   ctx->only_kernel = {};
+   g.only_kernel = {};
    size_t nodes = 0;
-   SOFIE_CUDA_TRY(cudaGraphGetNodes(ctx->graph, nullptr, &nodes));
+   SOFIE_CUDA_TRY(cudaGraphGetNodes(g.graph, nullptr, &nodes));
    if (nodes == 1) {
       cudaGraphNode_t node;
       cudaGraphNodeType type;
-      SOFIE_CUDA_TRY(cudaGraphGetNodes(ctx->graph, &node, &nodes));
+      SOFIE_CUDA_TRY(cudaGraphGetNodes(g.graph, &node, &nodes));
       SOFIE_CUDA_TRY(cudaGraphNodeGetType(node, &type));
       cudaKernelNodeAttrValue cluster = {};
       if (type == cudaGraphNodeTypeKernel && cudaGraphKernelNodeGetAttribute(node, cudaLaunchAttributeClusterDimension, &cluster) == cudaSuccess &&
           cluster.clusterDim.x * cluster.clusterDim.y * cluster.clusterDim.z <= 1) { // a plain launch has no cluster dimensions
-         if (cudaGraphKernelNodeGetParams(node, &ctx->only_kernel) != cudaSuccess) ctx->only_kernel = {};
+         if (cudaGraphKernelNodeGetParams(node, &g.only_kernel) != cudaSuccess) g.only_kernel = {};
       }
       cudaGetLastError();
    }
@@ -1019,18 +1018,26 @@ int sofie_cuda_ctx_graph_end(sofie_cuda_ctx *ctx)
 int sofie_cuda_ctx_graph_launch(sofie_cuda_ctx *ctx)
 {
    SOFIE_REQUIRE(ctx, "NULL ctx");
-   SOFIE_REQUIRE(ctx->graph_exec != nullptr, "no captured graph");
+   SOFIE_REQUIRE(ctx->captured.exec != nullptr, "no captured graph");
    DeviceGuard guard(ctx->device);
-   const cudaKernelNodeParams &k = ctx->only_kernel;
+   const cudaKernelNodeParams &k = ctx->captured.only_kernel;
    if (k.func && k.kernelParams) SOFIE_CUDA_TRY(cudaLaunchKernel(k.func, k.gridDim, k.blockDim, k.kernelParams, k.sharedMemBytes, ctx->stream));
-   else SOFIE_CUDA_TRY(cudaGraphLaunch(ctx->graph_exec, ctx->stream));
+   else SOFIE_CUDA_TRY(cudaGraphLaunch(ctx->captured.exec, ctx->stream));
    return SOFIE_CUDA_OK;
 }
 
 int sofie_cuda_ctx_graph_ready(sofie_cuda_ctx *ctx, int *ready)
 {
    SOFIE_REQUIRE(ctx && ready, "NULL argument");
-   *ready = ctx->graph_exec != nullptr;
+   *ready = ctx->captured.exec != nullptr;
+   return SOFIE_CUDA_OK;
+}
+
+int sofie_cuda_ctx_graph_swap(sofie_cuda_ctx *ctx)
+{
+   SOFIE_REQUIRE(ctx, "NULL ctx");
+   SOFIE_REQUIRE(!ctx->capturing, "graph capture in progress");
+   std::swap(ctx->captured, ctx->kept);
    return SOFIE_CUDA_OK;
 }
 

@@ -771,6 +771,8 @@ void RModel::GenerateSessionMembers()
    if (fStaged.kind) {
       fSessionMembers.push_back("fConverted");
       fGC += "bool fConverted = false;   // the last input was quantised by the host while it was staged\n";
+      fSessionMembers.push_back("fOtherGraphReady");
+      fGC += "bool fOtherGraphReady = false;   // the graph of the other kind of input (fConverted or not) is captured\n";
    }
    auto pointer = [this](ETensorType type, const std::string &name) {
       fGC += EMIT::CType(type) + " * " + EMIT::Dev(name) + " = nullptr;\n";
@@ -1031,6 +1033,15 @@ void RModel::GenerateInfer()
    fGC += "   }\n";
    fGC += "}\n\n";
    }
+   if (fStaged.kind) {
+      fGC += "// whether the host or the device does the first operator's work: each has a graph of its own\n";
+      fGC += "void SetConverted(bool converted) {\n";
+      fGC += "   if (converted == fConverted) return;\n";
+      fGC += "   Check(sofie_cuda_ctx_graph_swap(fCtx), \"sofie_cuda_ctx_graph_swap\");\n";
+      fGC += "   std::swap(fGraphReady, fOtherGraphReady);\n";
+      fGC += "   fConverted = converted;\n";
+      fGC += "}\n\n";
+   }
    // Every kernel of one inference on the inputs of the previous infer() call, which are still on the device:
    // no copy in either direction and no wait (for callers that time or pipeline the device work themselves).
    // Where the host quantised that input, the first call brings the floats back, so that the first operator has its input too.
@@ -1042,7 +1053,7 @@ void RModel::GenerateInfer()
       fGC += "   if (fConverted) {\n";
       fGC += "      Check(sofie_cuda_ctx_unquantize(fCtx, " + EMIT::Dev(q) + ", " + EMIT::Dev(in) + ", " + std::to_string(ConvertShapeToLength(GetTensorShape(in))) + ", " +
              std::to_string(fStaged.kind) + ", " + EMIT::FloatLit(fStaged.scale) + ", " + std::to_string(fStaged.zp) + "), \"sofie_cuda_ctx_unquantize\");\n";
-      fGC += "      fConverted = false;\n      fGraphReady = false;\n   }\n";
+      fGC += "      SetConverted(false);\n   }\n";
    }
    if (pipelined) fGC += "   for (int part = 0; part < " + std::to_string(fUploadParts) + "; part++) LaunchHead(part);\n";
    fGC += "   Run();\n";
@@ -1054,12 +1065,9 @@ void RModel::GenerateInfer()
    };
    auto upload = [&] {
       // the graph is captured again when the batch changes
+      if (fDynamicBatch && fStaged.kind) fGC += "   if (" + fBatchParam + " != fBatch) fOtherGraphReady = false;\n";
       if (fDynamicBatch) fGC += "   if (" + fBatchParam + " != fBatch) { fBatch = " + fBatchParam + "; fGraphReady = false; }\n";
-      // ... and when the first operator's work moves between the host and the device
-      if (fStaged.kind) {
-         fGC += "   const bool converted = sofie_cuda_ctx_pageable(fCtx, tensor_" + fInputTensorNames[0] + ") != 0;\n";
-         fGC += "   if (converted != fConverted) { fConverted = converted; fGraphReady = false; }\n";
-      }
+      if (fStaged.kind) fGC += "   SetConverted(sofie_cuda_ctx_pageable(fCtx, tensor_" + fInputTensorNames[0] + ") != 0);\n";
    };
    const std::string sig = GenerateInferSignature(), args = GenerateInferSignature(false);
    if (nOut != 1) {

@@ -504,7 +504,7 @@ def test_run_resident_has_its_input_after_a_quantised_upload(dynamic):
     body = text[text.index("void RunResident() {"):]
     body = body[:body.index("\n}\n")]
     assert re.search(r"if \(fConverted\) \{\n\s+Check\(sofie_cuda_ctx_unquantize\(fCtx, dev_q0, dev_x, ", body)
-    assert body.index("fConverted = false;") < body.index("Run();")
+    assert body.index("SetConverted(false);") < body.index("Run();")
     slices = {}
     for off, size, name in re.findall(r"sofie_cuda_ctx_arena\(fCtx, ([^,]+), ([^,]+), reinterpret_cast<void\*\*>\(&dev_(\w+)\)\)", text):
         o, b = (int(re.search(r"\d+", v).group()) for v in (off, size))
@@ -512,3 +512,14 @@ def test_run_resident_has_its_input_after_a_quantised_upload(dynamic):
     for kept in ("q0", "x"):
         lo, hi = slices[kept]
         assert all(h <= lo or hi <= l for n, (l, h) in slices.items() if n != kept), kept
+
+
+def test_inputs_of_both_kinds_keep_their_graphs():
+    """Alternating between a pageable and a pinned input swaps the two captured graphs; only another batch captures again."""
+    m, _ = configs.mlp_i8(batch=64, with_input=False)
+    for param in (None, "bs"):
+        text = generated.emit(onnx_wire.model_to_onnx(m, batch_param=param) if param else onnx_wire.model_to_onnx(m), "c3_graphs" + ("_dyn" if param else "")).read_text()
+        body = text[text.index("void SetConverted(bool converted) {"):]
+        body = body[:body.index("\n}\n")]
+        assert "sofie_cuda_ctx_graph_swap(fCtx)" in body and "std::swap(fGraphReady, fOtherGraphReady);" in body and "= false" not in body
+        assert text.count("fGraphReady = false") == (2 if param else 1) and ("fOtherGraphReady = false;" in text)

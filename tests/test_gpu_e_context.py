@@ -196,3 +196,23 @@ def test_e4m3_codes_and_their_values(cuda_device):
         back = ops.quantize_e4m3(v, scale)
         number = (codes & 127) != 127
         assert torch.equal(back[number], codes[number]) and bool((back[~number] & 127 == 127).all())
+
+
+def test_pinned_and_pageable_inputs_in_turn(cuda_device):
+    """Each kind of input has a graph of its own (with and without QuantizeLinear); results are the same bytes, and so after another batch."""
+    m, x = configs.mlp_i8(batch=96, dims=(512, 256, 128, 64, 10))
+    pinned = torch.from_numpy(x).pin_memory().numpy()
+    s = generated.session_from_model(m, "c3_turns")
+    want = s.infer(pinned)
+    ready = C.c_int()
+    for i in range(9):
+        assert np.array_equal(s.infer(x if i % 2 else pinned).view(np.uint32), want.view(np.uint32))
+        if i == 1:
+            capi.call("sofie_cuda_ctx_graph_swap", s.ctx)
+            capi.call("sofie_cuda_ctx_graph_ready", s.ctx, C.byref(ready))
+            assert ready.value                    # the pinned input's graph is still there
+            capi.call("sofie_cuda_ctx_graph_swap", s.ctx)
+    d = generated.dynamic_session_from_model(m, "c3_turns_dyn", 96)
+    for n in (96, 50, 96):
+        for source in (x, pinned, x):
+            assert np.array_equal(d.infer(source[:n]).view(np.uint32), want.view(np.uint32)[:n * 10])
