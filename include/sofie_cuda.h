@@ -170,6 +170,7 @@ int sofie_cuda_selftest_host_copy(void *dst, const void *src, size_t bytes, size
  * serialise the kernels around them (no overlap of one kernel's prologue with the previous kernel's tail),
  * so a timed Session is a little slower than an untimed one: use it to see where a step's time goes. */
 int sofie_cuda_ctx_timers(sofie_cuda_ctx *ctx, int on);
+int sofie_cuda_ctx_timed(sofie_cuda_ctx *ctx); /* 1 when the timers are on: the emitted infer() then launches every operator once, on the whole batch */
 int sofie_cuda_ctx_mark(sofie_cuda_ctx *ctx, int slot);
 int sofie_cuda_ctx_timers_read(sofie_cuda_ctx *ctx, float *ms, int n, int *count);
 /* Capture of the kernel sequence of one infer() into a CUDA graph: begin, run the launchers on

@@ -936,6 +936,8 @@ int sofie_cuda_ctx_timers(sofie_cuda_ctx *ctx, int on)
    return SOFIE_CUDA_OK;
 }
 
+int sofie_cuda_ctx_timed(sofie_cuda_ctx *ctx) { return ctx && ctx->timers_on; }
+
 int sofie_cuda_ctx_mark(sofie_cuda_ctx *ctx, int slot)
 {
    SOFIE_REQUIRE(ctx, "NULL ctx");

@@ -1067,7 +1067,7 @@ void RModel::GenerateInfer()
       // the graph is captured again when the batch changes
       if (fDynamicBatch && fStaged.kind) fGC += "   if (" + fBatchParam + " != fBatch) fOtherGraphReady = false;\n";
       if (fDynamicBatch) fGC += "   if (" + fBatchParam + " != fBatch) { fBatch = " + fBatchParam + "; fGraphReady = false; }\n";
-      if (fStaged.kind) fGC += "   SetConverted(sofie_cuda_ctx_pageable(fCtx, tensor_" + fInputTensorNames[0] + ") != 0);\n";
+      if (fStaged.kind) fGC += "   SetConverted(sofie_cuda_ctx_pageable(fCtx, tensor_" + fInputTensorNames[0] + ") && !sofie_cuda_ctx_timed(fCtx));\n";
    };
    const std::string sig = GenerateInferSignature(), args = GenerateInferSignature(false);
    if (nOut != 1) {
@@ -1189,7 +1189,9 @@ void RModel::GenerateUpload(bool pipelined, const std::string &result, size_t re
       const size_t in1 = ConvertShapeToLength(GetTensorShape(n)) / fRangeBatch, out1 = resultLen / fRangeBatch;
       const size_t inB = in1 * size, outB = out1 * GetTypeSize(GetTensorType(o));
       const std::string i1 = std::to_string(in1), o1 = std::to_string(out1);
-      fGC += "   const size_t samples = " + std::to_string(fRangeBatch) + ", rows = sofie_cuda_slice_rows(samples, " + std::to_string(inB) + ", " + std::to_string(outB) +
+      fGC += "   const size_t samples = " + std::to_string(fRangeBatch) + ";\n";
+      // with the device timers on every operator runs once, between its marks
+      fGC += "   const size_t rows = sofie_cuda_ctx_timed(fCtx) ? samples : sofie_cuda_slice_rows(samples, " + std::to_string(inB) + ", " + std::to_string(outB) +
              ", " + std::to_string(fRangeQuantum) + ");\n";
       fGC += "   if (rows < samples) {\n";
       fGC += "      int index = 0;\n";

@@ -216,3 +216,20 @@ def test_pinned_and_pageable_inputs_in_turn(cuda_device):
     for n in (96, 50, 96):
         for source in (x, pinned, x):
             assert np.array_equal(d.infer(source[:n]).view(np.uint32), want.view(np.uint32)[:n * 10])
+
+
+def test_operator_timers_of_a_session_that_cuts_its_batch(cuda_device, monkeypatch):
+    """With the timers on a batch that would be cut into ranges, from memory whose quantisation the host would take over, is launched
+    operator by operator: one interval for each, QuantizeLinear's among them, and the same result."""
+    m, x = configs.mlp_i8(batch=4099)
+    y0 = generated.session_from_model(m, "c3_b4099_timed").infer(x)
+    monkeypatch.setenv("SOFIE_CUDA_TIMERS", "1")
+    timed = generated.session_from_model(m, "c3_b4099_timed")
+    monkeypatch.delenv("SOFIE_CUDA_TIMERS")
+    plan = generated.launch_plan(timed.hxx)
+    assert plan[0]["calls"] == ["sofie_cuda_quantize_u8"]
+    n, ms = C.c_int(-1), (C.c_float * len(plan))()
+    for _ in range(3):
+        assert np.array_equal(timed.infer(x).view(np.uint32), y0.view(np.uint32))
+        capi.call("sofie_cuda_ctx_timers_read", timed.ctx, ms, len(plan), C.byref(n))
+        assert n.value == len(plan) and all(0.0 <= t < 50.0 for t in ms) and ms[0] > 0.0
