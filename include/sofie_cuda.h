@@ -104,6 +104,8 @@ int sofie_cuda_ctx_unquantize(sofie_cuda_ctx *ctx, const uint8_t *src_device, fl
  * sofie_cuda_ctx_stage_settle, after which no helper reads it. */
 int sofie_cuda_ctx_stage_ahead(sofie_cuda_ctx *ctx, const void *src_host, size_t bytes, int kind, float scale, int32_t zp);
 int sofie_cuda_ctx_stage_settle(sofie_cuda_ctx *ctx);
+/* Self test of failures on the host: the nth copy out of the staging ring from now on is refused (0: none). */
+int sofie_cuda_selftest_fail_copy(sofie_cuda_ctx *ctx, int nth);
 /* Self test of that quantisation on plain host memory (needs no GPU). */
 int sofie_cuda_selftest_host_quantize(uint8_t *dst, const float *src, size_t n, int kind, float scale, int32_t zp);
 /* Device -> host; returns after the data has arrived (last statement of the emitted infer(),
@@ -123,6 +125,9 @@ int sofie_cuda_ctx_fetch(sofie_cuda_ctx *ctx, const void *src_device, size_t byt
 int sofie_cuda_ctx_result_begin(sofie_cuda_ctx *ctx, void *out_host, size_t bytes);
 int sofie_cuda_ctx_result_part(sofie_cuda_ctx *ctx, const void *src_device, size_t offset, size_t bytes);
 int sofie_cuda_ctx_result_end(sofie_cuda_ctx *ctx, void **host);
+/* After a failure between _begin and _end: returns when no copy of this inference reads or writes the caller's memory any more.
+ * Does nothing after _end. */
+int sofie_cuda_ctx_result_abort(sofie_cuda_ctx *ctx);
 /* Samples per slice of a batch of `rows` samples whose copies in and out run under the kernels of other slices (`rows` itself:
  * the batch is better kept whole). in_bytes, out_bytes: per sample; quantum: what a slice has to be a multiple of. */
 size_t sofie_cuda_slice_rows(size_t rows, size_t in_bytes, size_t out_bytes, size_t quantum);

@@ -118,6 +118,7 @@ struct sofie_cuda_ctx {
    } fills[2];
    int next_fill = 0;
    Fill *ahead = nullptr; // begun by sofie_cuda_ctx_stage_ahead for a copy that is yet to be asked for
+   int fail_copy = 0;     // self test: the fail_copy-th staged copy from now on is refused (0: none)
    void *result = nullptr;  // pinned, grown on demand: where results land that were not given a pinned place of their own
    size_t result_bytes = 0;
    // the result of one inference on its way to the host, between result_begin and result_end
@@ -487,9 +488,7 @@ static int pull(cudaStream_t stream, void *dst, const void *src, size_t bytes)
    return SOFIE_CUDA_OK;
 }
 
-// Pageable memory to the device on `stream` (`bytes`: of the destination); returns when the last byte of the source has been
-// read. While the copy of one slot is issued the helpers fill the next.
-static int stage_in(sofie_cuda_ctx *ctx, const HostConvert &how, void *dst, const void *src_v, size_t bytes, cudaStream_t stream)
+static int stage_slots(sofie_cuda_ctx *ctx, const HostConvert &how, void *dst, const void *src_v, size_t bytes, cudaStream_t stream)
 {
    int rc = ensure_staging(ctx);
    if (rc || bytes == 0) return rc;
@@ -516,7 +515,8 @@ static int stage_in(sofie_cuda_ctx *ctx, const HostConvert &how, void *dst, cons
       sofie_cuda_ctx::Fill *now = cur;
       const size_t next = done + now->bytes;
       if (next < bytes && (rc = begin_fill(ctx, how, src + next * how.ratio(), bytes - next < step ? bytes - next : step, &cur))) return rc;
-      if (small && now->bytes == bytes) rc = pull(stream, dst, now->mem, bytes);
+      if (ctx->fail_copy > 0 && --ctx->fail_copy == 0) rc = fail(SOFIE_CUDA_ERR_CUDA, "staged copy refused (self test)");
+      else if (small && now->bytes == bytes) rc = pull(stream, dst, now->mem, bytes);
       else SOFIE_CUDA_TRY(cudaMemcpyAsync(static_cast<char *>(dst) + done, now->mem, now->bytes, cudaMemcpyHostToDevice, stream));
       if (rc) return rc;
       now->slot->busy = true;
@@ -526,6 +526,15 @@ static int stage_in(sofie_cuda_ctx *ctx, const HostConvert &how, void *dst, cons
       done = next;
    }
    return SOFIE_CUDA_OK;
+}
+
+// Pageable memory to the device on `stream` (`bytes`: of the destination); returns when the last byte of the source has been
+// read, or with an error, after which no helper reads the source either. While the copy of one slot is issued the helpers fill the next.
+static int stage_in(sofie_cuda_ctx *ctx, const HostConvert &how, void *dst, const void *src, size_t bytes, cudaStream_t stream)
+{
+   const int rc = stage_slots(ctx, how, dst, src, bytes, stream);
+   if (rc) settle(ctx);
+   return rc;
 }
 
 int sofie_cuda_ctx_h2d(sofie_cuda_ctx *ctx, void *dst, const void *src, size_t bytes)
@@ -547,6 +556,13 @@ int sofie_cuda_ctx_h2d(sofie_cuda_ctx *ctx, void *dst, const void *src, size_t b
       return SOFIE_CUDA_OK;
    }
    return stage_in(ctx, HostConvert(), dst, src, bytes, ctx->stream);
+}
+
+int sofie_cuda_selftest_fail_copy(sofie_cuda_ctx *ctx, int nth)
+{
+   SOFIE_REQUIRE(ctx && nth >= 0, "NULL context or negative count");
+   ctx->fail_copy = nth;
+   return SOFIE_CUDA_OK;
 }
 
 int sofie_cuda_selftest_host_copy(void *dst, const void *src, size_t bytes, size_t chunk, int threads, int repeats)
@@ -812,7 +828,6 @@ int sofie_cuda_ctx_result_end(sofie_cuda_ctx *ctx, void **host)
    SOFIE_REQUIRE(ctx && host, "NULL argument");
    auto &l = ctx->landing;
    SOFIE_REQUIRE(l.open, "no result was begun");
-   l.open = false;
    settle(ctx);
    DeviceGuard guard(ctx->device);
    const bool carry = l.out && l.land && l.land != l.out; // the caller's memory is pageable: the host carries the bytes over
@@ -826,12 +841,31 @@ int sofie_cuda_ctx_result_end(sofie_cuda_ctx *ctx, void **host)
          }
    }
    SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-   if (ctx->result_stream && l.parts > 1) SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->result_stream));
+   if (ctx->result_stream) SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->result_stream));
+   l.open = false;
    slots_free(ctx); // the stream has waited for every part that was copied in
-   if (carry && l.parts == 1) ctx->host_pool->copy(l.out, l.land, l.bytes);
+   if (carry && l.parts == 1) ctx->host_pool->copy(l.out + l.offset[0], l.land + l.offset[0], l.count[0]);
    if (l.mapped && l.out) std::memcpy(l.out, l.mapped, l.bytes);
    *host = l.out ? l.out : (l.mapped ? const_cast<char *>(l.mapped) : l.land);
    return report_status(ctx);
+}
+
+int sofie_cuda_ctx_result_abort(sofie_cuda_ctx *ctx)
+{
+   SOFIE_REQUIRE(ctx, "NULL ctx");
+   if (!ctx->landing.open) return SOFIE_CUDA_OK;
+   ctx->landing.open = false;
+   settle(ctx);
+   DeviceGuard guard(ctx->device);
+   // inputs on their way out of the caller's memory, and results on their way into it
+   cudaError_t err = cudaStreamSynchronize(ctx->stream);
+   for (cudaStream_t s : {ctx->copy_stream, ctx->result_stream}) {
+      const cudaError_t e = s ? cudaStreamSynchronize(s) : cudaSuccess;
+      if (err == cudaSuccess) err = e;
+   }
+   SOFIE_CUDA_TRY(err);
+   slots_free(ctx);
+   return SOFIE_CUDA_OK;
 }
 
 size_t sofie_cuda_slice_rows(size_t rows, size_t in_bytes, size_t out_bytes, size_t quantum)

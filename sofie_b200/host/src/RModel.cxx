@@ -1103,6 +1103,8 @@ void RModel::GenerateInfer()
    fGC += "const " + type + " * Execute(" + sig + sep + type + " * out) {\n";
    upload();
    fGC += "   Check(sofie_cuda_ctx_result_begin(fCtx, out, " + std::to_string(outBytes) + "), \"sofie_cuda_ctx_result_begin\");\n";
+   // whatever ends this call, no copy of it is on its way from or to the caller's memory afterwards
+   fGC += "   struct Abort { sofie_cuda_ctx * c; ~Abort() { sofie_cuda_ctx_result_abort(c); } } abort{fCtx};\n";
    const bool resultInParts = pipelined && tailOps == 0;
    GenerateUpload(pipelined, resultInParts ? o : "", outLen);
    if (fRangeBatch) fGC += "   } else {\n";

@@ -233,3 +233,57 @@ def test_operator_timers_of_a_session_that_cuts_its_batch(cuda_device, monkeypat
         assert np.array_equal(timed.infer(x).view(np.uint32), y0.view(np.uint32))
         capi.call("sofie_cuda_ctx_timers_read", timed.ctx, ms, len(plan), C.byref(n))
         assert n.value == len(plan) and all(0.0 <= t < 50.0 for t in ms) and ms[0] > 0.0
+
+
+_READ_AFTER_FAILURE = r"""
+import ctypes as C, mmap, sys, time
+sys.path.insert(0, sys.argv[1])
+from sofie_b200 import capi
+libc = C.CDLL(None, use_errno=True)
+libc.mprotect.argtypes = [C.c_void_p, C.c_size_t, C.c_int]
+ctx, dst, size = C.c_void_p(), C.c_void_p(), 64 << 20
+capi.call("sofie_cuda_ctx_create", C.byref(ctx), -1, size)
+capi.call("sofie_cuda_ctx_arena", ctx, 0, size, C.byref(dst))
+m = mmap.mmap(-1, size)
+src = C.addressof(C.c_char.from_buffer(m))
+C.memset(src, 1, size)
+lib = capi.load()
+for i in range(40):
+    capi.call("sofie_cuda_selftest_fail_copy", ctx, 1 + i % 5)
+    rc = (lib.sofie_cuda_ctx_h2d(ctx, dst, src, size) if i % 2 else lib.sofie_cuda_ctx_h2d_quantized(ctx, dst, src, size // 4, 1, 0.1, 3, -1))
+    assert libc.mprotect(src, size, 0) == 0          # the caller's memory goes away: a reader would be killed
+    assert rc == capi.ERR_CUDA, rc
+    time.sleep(0.002)
+    assert libc.mprotect(src, size, 3) == 0
+capi.call("sofie_cuda_ctx_h2d", ctx, dst, src, size)
+capi.call("sofie_cuda_ctx_sync", ctx)
+capi.call("sofie_cuda_ctx_destroy", ctx)
+print("ok")
+"""
+
+
+def test_no_helper_reads_the_source_of_a_copy_that_failed(cuda_device, tmp_path):
+    import subprocess
+    import sys
+    from pathlib import Path
+    script = tmp_path / "read_after_failure.py"
+    script.write_text(_READ_AFTER_FAILURE)
+    r = subprocess.run([sys.executable, str(script), str(Path(__file__).resolve().parents[1])], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), (r.returncode, r.stdout[-2000:])
+
+
+def test_no_copy_writes_the_result_of_an_inference_that_failed(cuda_device):
+    """infer() into pinned memory of the caller that fails between two ranges: earlier ranges' results are not on their way any more."""
+    import time
+    m, x = configs.mlp_i8(batch=16387)
+    s = generated.session_from_model(m, "c3_b16387")
+    want = s.infer(x)
+    out = torch.empty(want.size, pin_memory=True).numpy()
+    for nth in (5, 6, 8, 10):                   # the first range is copied in four pieces, each later one in one
+        capi.call("sofie_cuda_selftest_fail_copy", s.ctx, nth)
+        with pytest.raises(RuntimeError):
+            s.infer(x, out)
+        out.fill(-12345.)
+        time.sleep(0.02)
+        assert (out == -12345.).all()
+        assert s.infer(x, out) is out and np.array_equal(out.view(np.uint32), want.view(np.uint32))
