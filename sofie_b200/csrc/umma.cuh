@@ -153,7 +153,7 @@ __device__ __forceinline__ void tc_commit(uint64_t *bar)
                 : "memory");
 }
 
-enum Kind { kTF32 = 0, kI8 = 1, kF8 = 2 };
+enum Kind { kTF32 = 0, kI8 = 1, kF8 = 2, kBF16 = 3 };
 
 template <int KIND>
 __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
@@ -162,6 +162,11 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_
    if constexpr (KIND == kTF32) {
       asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                    "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+                   "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+                   : "memory");
+   } else if constexpr (KIND == kBF16) { // both operands
+      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                   "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
                    "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
                    : "memory");
    } else if constexpr (KIND == kI8) {
@@ -346,8 +351,8 @@ template <int KIND>
 __host__ __device__ constexpr uint32_t make_idesc(int M, int N)
 {
    uint32_t c_fmt = (KIND == kI8) ? 2u : 1u;
-   uint32_t a_fmt = (KIND == kTF32) ? 2u : 0u;                       // tf32 | uint8 | e4m3
-   uint32_t b_fmt = (KIND == kTF32) ? 2u : ((KIND == kI8) ? 1u : 0u); // tf32 | int8  | e4m3
+   uint32_t a_fmt = (KIND == kTF32) ? 2u : (KIND == kBF16 ? 1u : 0u);                     // tf32 | bf16 | uint8 | e4m3
+   uint32_t b_fmt = (KIND == kTF32) ? 2u : ((KIND == kI8 || KIND == kBF16) ? 1u : 0u);    // tf32 | bf16 | int8  | e4m3
    return (c_fmt << 4) | (a_fmt << 7) | (b_fmt << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 

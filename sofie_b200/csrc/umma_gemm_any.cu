@@ -1,21 +1,22 @@
 // fp32 tensor-core GEMM for the operands TMA cannot fetch -- a transposed A, B stored [K,N], rows that are not multiples of 16
-// bytes, unaligned bases -- and for few tiles with a long K. The same arithmetic as the TMA kernel of umma_gemm.cu (3xTF32: every
-// value split into hi = tf32(x) and lo = x - hi, lo*hi + hi*lo + hi*hi into a TMEM accumulator, promoted to fp32 registers every 256
-// elements of K), with two differences:
-//   * sixteen worker warps read the operands themselves, split them in registers and write the hi / lo tiles where the MMA's
-//     swizzled K-major descriptors expect them. A unit of work is four consecutive K of one row: one 16-byte load, four scalar loads
-//     (rows that are not 16-byte multiples), or four loads of consecutive rows (K is not the contiguous dimension), always one
-//     conflict-free 16-byte store per tile. Groups of them take the stages in turn: while one splits and stores, the others' loads
-//     are in flight (one group with two stages of loads in flight was bound by their latency: 2500 clocks a stage). The same warps
-//     add the partial sums up in registers and write the tile.
-//   * B's hi and lo tiles lie side by side as one operand of twice the width: A_hi x [B_hi | B_lo] and A_lo x B_hi are two MMAs per
-//     K step instead of three, with a sixth less shared memory read.
+// bytes, unaligned bases -- and for few tiles with a long K. Without it these products are chains of fp32 FMAs on the CUDA cores, and
+// its results are no further from the exact ones than theirs: every value is split into three bfloat16 parts that add up to it (8 + 8 + 8
+// bits), and the six products of parts that reach into 24 bits are summed by the tensor core, the leading ones apart from the others
+// (what is dropped is below 2^-25 of a product). The tensor core's sums truncate, so they are added to fp32 registers every few stages:
+// every 96 elements of K below K = 256, where a chain of FMAs has made few roundings too, every 128 up to K = 1023, every 256 from there.
+// Error against float64 over that of the chain of FMAs, N(0,1) operands: 0.57 at K = 8, 0.4 to 0.6 at K = 128, 0.2 to 0.4 at K = 800,
+// below 0.3 beyond; the same with operands of one sign: 0.66, 0.9, 0.4, 0.3. (Two TF32 parts, 22 bits, and sums of 256: 1.7, 1.7, 0.7, 0.6.)
+//   * sixteen worker warps read the operands themselves, split them in registers and write the parts where the MMA's swizzled K-major
+//     descriptors expect them. A unit of work is eight consecutive K of one row: two 16-byte loads, eight scalar loads (rows that are
+//     not 16-byte multiples), or eight loads of consecutive rows (K is not the contiguous dimension), always one conflict-free
+//     16-byte store per part. Groups of them take the stages in turn: while one splits and stores, the others' loads are in flight
+//     (one group with two stages of loads in flight was bound by their latency). The same warps add the partial sums up in registers
+//     and write the tile.
+//   * B's parts lie one behind the other, so that the first instruction of a K step multiplies A's first part with two of B's at once,
+//     into neighbouring columns of the accumulator.
 //   * a cluster of S CTAs shares one output tile: each takes a S-th of K, leaves its partial tile in shared memory, and adds up and
 //     writes a S-th of the rows out of all of them (distributed shared memory, fixed order). No scratch buffer, one launch.
-// Measured on B200 (in a graph, back to back): 1000 x 777 x 1333 with A transposed 211 us on the CUDA cores, 35 here; 200 x 200 x 4000
-// 85 us on one CTA per 128 x 64 tile, 15 here; 4096 x 4096 x 2048 603 us by the TMA kernel (128 x 64 tiles), 440 here (157 TFLOP/s of
-// the 273 that bf16 / 6 leaves): what bounds it is the workers' chain of loading, splitting and storing (1860 clocks a stage, of which
-// the MMAs take 770 and their issue 700).
+// What bounds it is the workers' chain of loading, splitting and storing; the MMAs of a stage take 770 clocks at 128 columns.
 // The tile goes out through shared memory, so stores (and a bias of the output's shape) are contiguous along rows for every N.
 #include "umma.cuh"
 #include "contract.cuh"
@@ -25,23 +26,24 @@ namespace umma {
 namespace {
 
 constexpr int kAnyBM = 128;             // rows of the tile = TMEM lanes
-constexpr int kAnyKE = 32;              // floats of K per stage = one 128-byte swizzle row
+constexpr int kAnyKE = 32;              // floats of K per stage: one 64-byte swizzle row of each of the three parts
+constexpr int kAnyRow = kAnyKE * 2;
 constexpr int kAnyWorkers = 16 * 32;
 // Groups of worker warps that take the stages in turn. Four were 5 to 10 % faster at 32 columns with a long K and as much slower with a
 // short one (the pipeline takes longer to start), and spilled at 64 columns.
 constexpr int kAnyGroups = 2;
 constexpr int kAnyThreads = kAnyWorkers + 32; // and the warp that issues the MMAs
-constexpr int kAnyPromote = 8;          // stages accumulated in one TMEM buffer: 256 elements of K
 constexpr int kAnyMaxStages = 5;
 
 template <int BN>
 struct AnySmem {
-   static constexpr int kA = kAnyBM * 128, kB = BN * 128;
-   static constexpr int kStage = 2 * (kA + kB);                       // hi and lo
+   static constexpr int kA = kAnyBM * kAnyRow, kB = BN * kAnyRow;
+   static constexpr int kStage = 3 * (kA + kB);                       // the three parts of both operands
    static constexpr int kPitch = BN + 4;                              // floats per row of the outgoing tile, which takes the
    static constexpr int kTile = kAnyBM * kPitch * 4;                  // place of the stages when their MMAs are done
-   static constexpr int kStages = BN == 128 ? 3 : (BN == 64 ? 4 : 5);
+   static constexpr int kStages = BN == 128 ? 4 : 5;
    static_assert(kTile <= kStages * kStage, "the tile fits in the stages");
+   static_assert(kB % 512 == 0, "parts start on whole swizzle atoms");
    static constexpr int kBytes = kStages * kStage + 1024;
 };
 
@@ -53,100 +55,110 @@ struct AnyOperand {
    int rows, mode;
 };
 
-__device__ __forceinline__ void any_split(float x, float &h, float &l)
+// Two values in three bfloat16 parts each, packed: round, take off, twice. Both remainders are exact, and the second has at most
+// seven bits, so that its upper half is all of it: p0 + p1 + p2 is the value itself.
+__device__ __forceinline__ uint32_t any_part(float lo, float hi)
 {
-   uint32_t w;
-   asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(w) : "f"(x));
-   h = __uint_as_float(w);
-   l = x - h;
+   uint32_t p;
+   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p) : "f"(hi), "f"(lo)); // the first source lands in the upper half
+   return p;
+}
+__device__ __forceinline__ void any_split(float x, float y, uint32_t &p0, uint32_t &p1, uint32_t &p2)
+{
+   p0 = any_part(x, y);
+   x -= __uint_as_float(p0 << 16), y -= __uint_as_float(p0 & 0xFFFF0000u);
+   p1 = any_part(x, y);
+   x -= __uint_as_float(p1 << 16), y -= __uint_as_float(p1 & 0xFFFF0000u);
+   p2 = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
 }
 
-// One thread's share of the tiles of an operand with R rows: U units, a unit being K chunk `c` (four floats) of row `r`.
-//   K contiguous: eight lanes cover the 128 bytes of one row; the thread's units are T / 8 rows apart, in the same chunk.
+// One thread's share of the tiles of an operand with R rows: U units, a unit being K chunk `c` (eight floats) of row `r`.
+//   K contiguous: four lanes cover the 128 bytes of one row; the thread's units are T / 4 rows apart, in the same chunk.
 //   Rows contiguous: lanes cover consecutive rows; the thread's units are in one row, T / R chunks apart (T threads per group).
 // Either way the 16-byte stores of eight lanes fall into eight different bank groups, and everything that depends on the thread is
-// worked out once per tile: the loops below are a load, an addition and the split per unit (with the addresses taken from the unit
-// number the loaders were bound by instruction issue).
+// worked out once per tile: the loops below are the loads, an addition and the split per unit (with the addresses taken from the unit
+// number the loaders were bound by instruction issue). With 32 rows half of the threads have no unit.
 template <int R, int T>
 struct AnyLoader {
-   static constexpr int U = R * 8 / T;
-   static constexpr int kRowStep = T / 8, kChunkStep = T / R; // between the units of a thread
+   static constexpr int U = R * 4 / T > 0 ? R * 4 / T : 1;
+   static constexpr bool kAll = R * 4 >= T;                       // every thread has a unit
+   static constexpr int kRowStep = T / 4, kChunkStep = T / R;     // between the units of a thread
    const float *p = nullptr; // the thread's first element at K = 0 of the tile
    uint32_t at = 0;          // byte offset of its first unit in the tile
    uint32_t ok = 0;          // bit i: the row of unit i exists
-   float4 v[U];
+   float v[U][8];
 
    __device__ __forceinline__ void place(const AnyOperand &o, int t)
    {
-      const int r = o.mode == kRowsContiguous ? (t & (R - 1)) : (t >> 3), c = o.mode == kRowsContiguous ? t / R : (t & 7);
-      at = (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); // the 128-byte swizzle the descriptors name
+      const int r = o.mode == kRowsContiguous ? (t & (R - 1)) : (t >> 2), c = o.mode == kRowsContiguous ? t / R : (t & 3);
+      at = (uint32_t)(r * kAnyRow + ((c ^ ((r >> 1) & 3)) << 4)); // the 64-byte swizzle the descriptors name
    }
    __device__ __forceinline__ void tile(const AnyOperand &o, int row0, int t)
    {
       if (o.mode == kRowsContiguous) {
          const int r = row0 + (t & (R - 1));
-         ok = r < o.rows ? ~0u : 0u;
-         p = o.p + r + (long long)(4 * (t / R)) * o.ld;
+         ok = r < o.rows && (kAll || t < R * 4) ? ~0u : 0u;
+         p = o.p + r + (long long)(8 * (t / R)) * o.ld;
       } else {
-         const int r = row0 + (t >> 3);
+         const int r = row0 + (t >> 2);
          ok = 0;
 #pragma unroll
-         for (int i = 0; i < U; i++) ok |= (r + kRowStep * i < o.rows ? 1u : 0u) << i;
-         p = o.p + (long long)r * o.ld + 4 * (t & 7);
+         for (int i = 0; i < U; i++) ok |= (r + kRowStep * i < o.rows && (kAll || t < R * 4) ? 1u : 0u) << i;
+         p = o.p + (long long)r * o.ld + 8 * (t & 3);
       }
    }
    // the units of the stage that starts at element k0 of K; K ends at kend
    __device__ __forceinline__ void load(const AnyOperand &o, int k0, int kend, int t)
    {
+#pragma unroll
+      for (int i = 0; i < U; i++)
+#pragma unroll
+         for (int j = 0; j < 8; j++) v[i][j] = 0.f;
       if (o.mode == kRowsContiguous) {
          const float *q = p + (long long)k0 * o.ld;
-         const long long step = (long long)(4 * kChunkStep) * o.ld;
-         int left = kend - k0 - 4 * (t / R); // elements of K from the thread's first chunk on
+         int left = ok ? kend - k0 - 8 * (t / R) : 0; // elements of K from the thread's first chunk on
 #pragma unroll
-         for (int i = 0; i < U; i++, q += step, left -= 4 * kChunkStep) {
-            const float *q1 = q + o.ld, *q2 = q1 + o.ld, *q3 = q2 + o.ld;
-            v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (ok && left > 0) v[i].x = *q;
-            if (ok && left > 1) v[i].y = *q1;
-            if (ok && left > 2) v[i].z = *q2;
-            if (ok && left > 3) v[i].w = *q3;
+         for (int i = 0; i < U; i++, left -= 8 * kChunkStep) {
+            const float *e = q + (long long)(8 * kChunkStep * i) * o.ld;
+#pragma unroll
+            for (int j = 0; j < 8; j++, e += o.ld)
+               if (left > j) v[i][j] = *e;
          }
       } else {
          const float *q = p + k0;
          const long long step = kRowStep * o.ld;
-         const int left = kend - k0 - 4 * (t & 7);
+         const int left = kend - k0 - 8 * (t & 3);
          if (o.mode == kVecK) { // K % 4 == 0 and kend % 4 == 0
 #pragma unroll
-            for (int i = 0; i < U; i++, q += step) {
-               v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-               if (((ok >> i) & 1) && left > 0) v[i] = *reinterpret_cast<const float4 *>(q);
-            }
+            for (int i = 0; i < U; i++, q += step)
+#pragma unroll
+               for (int h = 0; h < 8; h += 4)
+                  if (((ok >> i) & 1) && left > h) {
+                     const float4 w = *reinterpret_cast<const float4 *>(q + h);
+                     v[i][h] = w.x, v[i][h + 1] = w.y, v[i][h + 2] = w.z, v[i][h + 3] = w.w;
+                  }
          } else {
 #pragma unroll
-            for (int i = 0; i < U; i++, q += step) {
-               const bool row = (ok >> i) & 1;
-               v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-               if (row && left > 0) v[i].x = q[0];
-               if (row && left > 1) v[i].y = q[1];
-               if (row && left > 2) v[i].z = q[2];
-               if (row && left > 3) v[i].w = q[3];
-            }
+            for (int i = 0; i < U; i++, q += step)
+#pragma unroll
+               for (int j = 0; j < 8; j++)
+                  if (((ok >> i) & 1) && left > j) v[i][j] = q[j];
          }
       }
    }
-   __device__ __forceinline__ void store(const AnyOperand &o, unsigned char *hi, unsigned char *lo)
+   // the parts lie `part` bytes apart
+   __device__ __forceinline__ void store(const AnyOperand &o, unsigned char *p0, int part, int t)
    {
+      if (!kAll && t >= R * 4) return;
 #pragma unroll
       for (int i = 0; i < U; i++) {
-         // units a multiple of 8 rows apart keep their place in the swizzle pattern; chunks kChunkStep apart flip its upper bits
-         const uint32_t off = o.mode == kRowsContiguous ? (at ^ (uint32_t)(i * kChunkStep * 16)) : (at + (uint32_t)(i * kRowStep * 128));
-         float4 h, l;
-         any_split(v[i].x, h.x, l.x);
-         any_split(v[i].y, h.y, l.y);
-         any_split(v[i].z, h.z, l.z);
-         any_split(v[i].w, h.w, l.w);
-         *reinterpret_cast<float4 *>(hi + off) = h;
-         *reinterpret_cast<float4 *>(lo + off) = l;
+         // units a multiple of 8 rows apart keep their place in the swizzle pattern; chunks kChunkStep apart flip its upper bit
+         const uint32_t off = o.mode == kRowsContiguous ? (at ^ (uint32_t)(i * kChunkStep * 16)) : (at + (uint32_t)(i * kRowStep * kAnyRow));
+         uint32_t w[3][4];
+#pragma unroll
+         for (int j = 0; j < 4; j++) any_split(v[i][2 * j], v[i][2 * j + 1], w[0][j], w[1][j], w[2][j]);
+#pragma unroll
+         for (int q = 0; q < 3; q++) *reinterpret_cast<uint4 *>(p0 + q * part + off) = make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]);
       }
    }
 };
@@ -170,6 +182,7 @@ struct AnyEpilogue {
    const float *C;
    float *Y;
    int bias_kind, relu, vec; // vec: rows of Y (and of a full C) start on 16-byte boundaries
+   int unit;                 // stages added up in one TMEM buffer (the tensor core's sums truncate) before they are promoted
 };
 
 __device__ __forceinline__ float any_finish(const AnyEpilogue &ep, float v, float c)
@@ -229,7 +242,7 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
    using L = AnySmem<BN>;
    constexpr int G = kAnyGroups, GT = kAnyWorkers / G; // groups and their threads
    constexpr int QUARTER = BN / 4;       // columns of the tile a worker warp adds up
-   constexpr uint32_t TMEM_COLS = 4 * BN; // two buffers of [hi x hi | the cross terms]
+   constexpr uint32_t TMEM_COLS = 4 * BN; // two buffers of [the leading products | the smaller ones]
    extern __shared__ unsigned char smem_raw[];
    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
    float *tile_out = reinterpret_cast<float *>(smem);
@@ -246,12 +259,10 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
    const int nkb = (K + kAnyKE - 1) / kAnyKE;
    const int kb0 = (int)((long long)nkb * rank / S), kbn = (int)((long long)nkb * (rank + 1) / S) - kb0; // this rank's stages of a tile
    const int kend = min(K, (kb0 + kbn) * kAnyKE);
-   const int units = (kbn + kAnyPromote - 1) / kAnyPromote;
+   const int unit_stages = ep.unit, units = (kbn + unit_stages - 1) / unit_stages;
    const int tile0 = blockIdx.x / S, tile_step = gridDim.x / S;
-   auto a_hi = [&](int s) { return smem + s * L::kStage; };
-   auto a_lo = [&](int s) { return smem + s * L::kStage + L::kA; };
-   auto b_hi = [&](int s) { return smem + s * L::kStage + 2 * L::kA; };
-   auto b_lo = [&](int s) { return smem + s * L::kStage + 2 * L::kA + L::kB; };
+   auto a_part = [&](int s, int q) { return smem + s * L::kStage + q * L::kA; };
+   auto b_part = [&](int s, int q) { return smem + s * L::kStage + 3 * L::kA + q * L::kB; };
 
    if (threadIdx.x == 0) {
       for (int s = 0; s < L::kStages; s++) {
@@ -333,13 +344,13 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
          int unit = 0; // units of this tile already added up
          for (; g < first + kbn; g += G) {
             // the partial sum of a unit is collected a ring's length after its last stage was stored: its MMAs are done by then
-            if (g - first >= (unit + 1) * kAnyPromote + L::kStages) {
+            if (g - first >= (unit + 1) * unit_stages + L::kStages) {
                promote();
                unit++;
             }
             if (SOFIE_PROF_WAIT(mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g))) {
-               la.store(A, a_hi(s), a_lo(s));
-               lb.store(B, b_hi(s), b_lo(s));
+               la.store(A, a_part(s, 0), L::kA, t);
+               lb.store(B, b_part(s, 0), L::kB, t);
                // visible to the tensor core: before the next loads are issued, because the fence would wait for them
                fence_proxy_async();
                __syncwarp();
@@ -360,12 +371,12 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
       }
    } else if (lane == 0) {
       // ---------------- MMA issuer ----------------
-      constexpr uint32_t idesc_wide = make_idesc<kTF32>(kAnyBM, 2 * BN), idesc = make_idesc<kTF32>(kAnyBM, BN);
+      constexpr uint32_t idesc_wide = make_idesc<kBF16>(kAnyBM, 2 * BN), idesc = make_idesc<kBF16>(kAnyBM, BN);
       int s = 0, u = 0, g = 0;
       uint32_t ph = 0;
       bool ok = true;
       for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
-         for (int kc = 0; kc < kbn && ok; kc += kAnyPromote, u++) {
+         for (int kc = 0; kc < kbn && ok; kc += unit_stages, u++) {
             const int buf = u & 1;
             if (!SOFIE_PROF_WAIT(mbar_wait(&tmem_empty[buf], ((u >> 1) & 1) ^ 1, &abort_flag, status, kStatusWaitAccum, 0x1000 + u))) {
                ok = false;
@@ -373,18 +384,22 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
             }
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + (uint32_t)(buf * 2 * BN);
-            const int kce = min(kbn, kc + kAnyPromote);
+            const int kce = min(kbn, kc + unit_stages);
             for (int kb = kc; kb < kce; kb++, g++, ring_next(s, ph, L::kStages)) {
                ok = SOFIE_PROF_WAIT(mbar_wait(&full_bar[s], ph, &abort_flag, status, kStatusWaitConv, g));
                if (!ok) break;
                tc_fence_after();
-               const uint64_t da = make_smem_desc(smem_u32(a_hi(s)), 128), dal = make_smem_desc(smem_u32(a_lo(s)), 128);
-               const uint64_t db = make_smem_desc(smem_u32(b_hi(s)), 128);
+               const uint64_t da0 = make_smem_desc(smem_u32(a_part(s, 0)), kAnyRow), da1 = make_smem_desc(smem_u32(a_part(s, 1)), kAnyRow);
+               const uint64_t da2 = make_smem_desc(smem_u32(a_part(s, 2)), kAnyRow), db0 = make_smem_desc(smem_u32(b_part(s, 0)), kAnyRow);
+               const uint64_t db1 = make_smem_desc(smem_u32(b_part(s, 1)), kAnyRow), db2 = make_smem_desc(smem_u32(b_part(s, 2)), kAnyRow);
 #pragma unroll
-               for (int k = 0; k < 4; k++) {
+               for (int k = 0; k < 2; k++) {
                   const uint64_t koff = (uint64_t)(2 * k);
-                  tc_mma<kTF32>(d_tmem, da + koff, db + koff, idesc_wide, (kb == kc && k == 0) ? 0u : 1u);
-                  tc_mma<kTF32>(d_tmem + BN, dal + koff, db + koff, idesc, 1);
+                  tc_mma<kBF16>(d_tmem, da0 + koff, db0 + koff, idesc_wide, (kb == kc && k == 0) ? 0u : 1u); // and the second part of B behind it
+                  tc_mma<kBF16>(d_tmem + BN, da1 + koff, db0 + koff, idesc, 1);
+                  tc_mma<kBF16>(d_tmem + BN, da1 + koff, db1 + koff, idesc, 1);
+                  tc_mma<kBF16>(d_tmem + BN, da0 + koff, db2 + koff, idesc, 1);
+                  tc_mma<kBF16>(d_tmem + BN, da2 + koff, db0 + koff, idesc, 1);
                }
                tc_commit(&empty_bar[s]);
             }
@@ -449,7 +464,7 @@ int launch_gemm_f32_any(cudaStream_t s, const sofie_gemm_f32_desc &d, const floa
    const bool vec_k = d.K % 4 == 0;
    const AnyOperand a{A, d.transA ? d.M : d.K, d.M, d.transA ? kRowsContiguous : (vec_k && aligned(A) ? kVecK : kScalarK)};
    const AnyOperand b{B, d.transB ? d.K : d.N, d.N, !d.transB ? kRowsContiguous : (vec_k && aligned(B) ? kVecK : kScalarK)};
-   const AnyEpilogue ep{d.alpha, d.beta, C, Y, d.bias_kind, d.relu, d.N % 4 == 0 && aligned(Y) && (d.bias_kind != 2 || aligned(C))};
+   const AnyEpilogue ep{d.alpha, d.beta, C, Y, d.bias_kind, d.relu, d.N % 4 == 0 && aligned(Y) && (d.bias_kind != 2 || aligned(C)), d.K >= 1024 ? 8 : (d.K >= 256 ? 4 : 3)};
    const int tm = ceil_div(d.M, kAnyBM), nkb = ceil_div(d.K, kAnyKE);
    // Tile width and clusters along K by the time they take: a stage of 32 K costs about 1800 / 1150 / 900 clocks at 128 / 64 / 32
    // columns, a tile's start and end about 6000, the exchange within a cluster 2500 more; clusters of 2 / 4 / 8 found room for

@@ -271,3 +271,25 @@ def test_qconv_pool_with_negative_multipliers(case):
                            x_zp=0, y_zp=100, relu=False, pool=2, x_layout=1, y_layout=1, w_packed=True, kernel=(3, 3)).cpu().numpy()
     assert np.array_equal(y.transpose(0, 3, 1, 2), ref)
     assert len(np.unique(ref)) > 20
+
+
+@pytest.mark.parametrize("sign", ["both", "one"])
+@pytest.mark.parametrize("M,N,K", [(300, 200, 8), (1024, 130, 17), (257, 333, 33), (700, 64, 96), (640, 250, 97), (512, 300, 128), (129, 260, 255), (300, 200, 256),
+                                   (400, 70, 777), (600, 33, 1023), (260, 190, 1333), (100, 600, 4001)])
+def test_gemm_f32_parts_are_no_further_from_float64_than_fma_chains(M, N, K, sign):
+    """Products that run as chains of fp32 FMAs on the CUDA cores when the tensor cores are not used: their error (2-norm, against
+    float64) is the bound for the tensor-core kernel, for every way the operands can lie, below and at the edges of its units of K."""
+    g = torch.Generator(device="cuda").manual_seed(M * N + K)
+    for tA, tB in ((1, 0), (1, 1), (0, 0)):
+        A = torch.randn((K, M) if tA else (M, K), device="cuda", generator=g)
+        B = torch.randn((N, K) if tB else (K, N), device="cuda", generator=g) * K ** -0.5
+        if sign == "one":
+            A, B = A.abs(), B.abs()
+        exact = (A.double().t() if tA else A.double()) @ (B.double().t() if tB else B.double())
+
+        def error(engine):
+            ops.set_engine(engine)
+            y = ops.gemm_f32(A, B, transA=tA, transB=tB)
+            assert ops.last_engine() == engine
+            return float((y.double() - exact).norm())
+        assert error(capi.ENGINE_TCGEN05) <= error(capi.ENGINE_SIMT)
