@@ -6,6 +6,7 @@
 // every 96 elements of K below K = 256, where a chain of FMAs has made few roundings too, every 128 up to K = 1023, every 256 from there.
 // Error against float64 over that of the chain of FMAs, N(0,1) operands: 0.57 at K = 8, 0.4 to 0.6 at K = 128, 0.2 to 0.4 at K = 800,
 // below 0.3 beyond; the same with operands of one sign: 0.66, 0.9, 0.4, 0.3. (Two TF32 parts, 22 bits, and sums of 256: 1.7, 1.7, 0.7, 0.6.)
+// Infinities, NaNs and the ends of fp32's range give what the chain gives (any_doubtful below).
 //   * sixteen worker warps read the operands themselves, split them in registers and write the parts where the MMA's swizzled K-major
 //     descriptors expect them. A unit of work is eight consecutive K of one row: two 16-byte loads, eight scalar loads (rows that are
 //     not 16-byte multiples), or eight loads of consecutive rows (K is not the contiguous dimension), always one conflict-free
@@ -192,6 +193,41 @@ __device__ __forceinline__ float any_finish(const AnyEpilogue &ep, float v, floa
    return ep.relu ? relu_ref(v) : v;
 }
 
+// The parts of an operand that is infinite, not a number or above the largest bfloat16 do not add up to it (Inf - Inf, Inf x 0), and
+// those of one below 2^-110 lose bits to bfloat16's range. The first kind shows in the sum, the second where the sum is tiny too
+// (and not where a factor above 2^14 or more lifts it back into the range; an operand below 2^-134 counts as zero). Such a sum is
+// doubtful: it is taken again as the chain of FMAs that the CUDA-core kernel forms, term by term.
+__device__ __forceinline__ bool any_doubtful(float v)
+{
+   const uint32_t e = __float_as_uint(v) & 0x7FFFFFFFu, tiny = 31u << 23; // 2^-96
+   return e - tiny >= 0x7F800000u - tiny && e != 0u;
+}
+
+// any_write below for a tile with doubtful sums.
+template <int BN>
+__device__ __forceinline__ void any_write_checked(const AnyOperand &A, const AnyOperand &B, int K, const AnyEpilogue &ep, const float *tile, int S, int r0, int rows, int m0, int n0)
+{
+   constexpr int P = AnySmem<BN>::kPitch;
+   const uint32_t base = smem_u32(tile);
+   const long long as = A.mode == kRowsContiguous ? A.ld : 1, ar = A.mode == kRowsContiguous ? 1 : A.ld;
+   const long long bs = B.mode == kRowsContiguous ? B.ld : 1, br = B.mode == kRowsContiguous ? 1 : B.ld;
+#pragma unroll 1
+   for (int i = threadIdx.x; i < rows * BN; i += kAnyWorkers) {
+      const int r = r0 + i / BN, c = i % BN, row = m0 + r, col = n0 + c;
+      if (row >= A.rows || col >= B.rows) continue;
+      float v = 0.f;
+      for (int q = 0; q < S; q++) v += S == 1 ? tile[r * P + c] : ld_cluster_f1(mapa_shared(base + (uint32_t)(r * P + c) * 4, (uint32_t)q));
+      if (any_doubtful(v)) {
+         const float *a = A.p + row * ar, *b = B.p + col * br;
+         v = 0.f;
+#pragma unroll 1
+         for (int k = 0; k < K; k++, a += as, b += bs) v = fmaf(*a, *b, v);
+      }
+      const float bias = ep.bias_kind == 1 ? ep.C[col] : (ep.bias_kind == 2 ? ep.C[(size_t)row * B.rows + col] : 0.f);
+      ep.Y[(size_t)row * B.rows + col] = any_finish(ep, v, bias);
+   }
+}
+
 // Rows [r0, r0 + rows) of the tile at (m0, n0), the sum of the S partial tiles, to global memory.
 template <int BN>
 __device__ __forceinline__ void any_write(const AnyEpilogue &ep, const float *tile, int S, int r0, int rows, int m0, int n0, int M, int N)
@@ -248,7 +284,7 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
    float *tile_out = reinterpret_cast<float *>(smem);
    __shared__ uint64_t full_bar[kAnyMaxStages], empty_bar[kAnyMaxStages], tmem_full[2], tmem_empty[2];
    __shared__ uint32_t tmem_base_holder;
-   __shared__ volatile uint32_t abort_flag;
+   __shared__ volatile uint32_t abort_flag, doubt_flag; // doubt_flag: a sum of this CTA's tile is doubtful
 
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
    SOFIE_PROF_DECL
@@ -274,6 +310,7 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
          mbar_init(&tmem_empty[b], kAnyWorkers / 32);
       }
       abort_flag = 0;
+      doubt_flag = 0;
       fence_mbar_init();
    }
    if (warp == kAnyWorkers / 32) {
@@ -364,10 +401,23 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
          float *mine = tile_out + (lane_base + lane) * L::kPitch + col_base;
 #pragma unroll
          for (int j = 0; j < QUARTER; j += 4) *reinterpret_cast<float4 *>(mine + j) = make_float4(acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+         // any_doubtful() of all of them in three instructions each: an infinity or NaN times 0 stays, 2e - 1 leaves the zeros out
+         float finite = 0.f;
+         uint32_t least = 0xFFFFFFFFu;
+#pragma unroll
+         for (int j = 0; j < QUARTER; j++) {
+            finite = fmaf(acc[j], 0.f, finite);
+            least = min(least, 2 * __float_as_uint(acc[j]) - 1);
+         }
+         if (finite != 0.f || least < 2 * (31u << 23) - 1) doubt_flag = 1;
          workers_sync();
          if (S > 1) break; // one tile per cluster: it is summed up below
-         if (!abort_flag) any_write<BN>(ep, tile_out, 1, 0, kAnyBM, m0, n0, M, N);
+         if (!abort_flag) {
+            if (doubt_flag) any_write_checked<BN>(A, B, K, ep, tile_out, 1, 0, kAnyBM, m0, n0);
+            else any_write<BN>(ep, tile_out, 1, 0, kAnyBM, m0, n0, M, N);
+         }
          workers_sync(); // the tile has been read: its place is the stages' again
+         if (threadIdx.x == 0) doubt_flag = 0; // set again behind the next tile's first workers_sync
       }
    } else if (lane == 0) {
       // ---------------- MMA issuer ----------------
@@ -412,8 +462,13 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
       // every rank's partial tile is complete; each sums up and writes its share of the rows
       __syncwarp();
       cluster_sync_all();
-      if (warp < kAnyWorkers / 32 && !abort_flag)
-         any_write<BN>(ep, tile_out, S, rank * (kAnyBM / S), kAnyBM / S, (tile0 / tiles_n) * kAnyBM, (tile0 % tiles_n) * BN, M, N);
+      if (warp < kAnyWorkers / 32 && !abort_flag) {
+         uint32_t doubt = 0;
+         for (int q = 0; q < S; q++) doubt |= __float_as_uint(ld_cluster_f1(mapa_shared(smem_u32(const_cast<uint32_t *>(&doubt_flag)), (uint32_t)q)));
+         const int r0 = rank * (kAnyBM / S), m0 = (tile0 / tiles_n) * kAnyBM, n0 = (tile0 % tiles_n) * BN;
+         if (doubt) any_write_checked<BN>(A, B, K, ep, tile_out, S, r0, kAnyBM / S, m0, n0);
+         else any_write<BN>(ep, tile_out, S, r0, kAnyBM / S, m0, n0, M, N);
+      }
       __syncwarp();
       cluster_sync_all(); // nobody leaves while its tile is still read
    }

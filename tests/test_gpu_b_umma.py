@@ -293,3 +293,45 @@ def test_gemm_f32_parts_are_no_further_from_float64_than_fma_chains(M, N, K, sig
             assert ops.last_engine() == engine
             return float((y.double() - exact).norm())
         assert error(capi.ENGINE_TCGEN05) <= error(capi.ENGINE_SIMT)
+
+
+@pytest.mark.parametrize("relu", [False, True])
+@pytest.mark.parametrize("M,N,K,bias", [(130, 68, 40, 2), (131, 37, 41, 2), (300, 200, 64, 1), (90, 33, 1500, 0), (257, 130, 2047, 2), (20000, 64, 9, 1)])
+def test_gemm_f32_of_values_the_parts_do_not_hold(M, N, K, bias, relu):
+    """Infinities, NaNs, values that round up to infinity, products that overflow and rows near the bottom of the range: what the chain of
+    FMAs gives (operands below bfloat16's denormals, row 21, count as zeros), for every layout, with one tile and with a cluster along K, whole words and single floats at the output."""
+    rng = np.random.default_rng(M + N + K)
+    for tA, tB in ((1, 0), (1, 1), (0, 0)):
+        A = rng.standard_normal((M, K)).astype(np.float32)
+        B = rng.standard_normal((N, K)).astype(np.float32)
+        A[3, 5], A[7, K - 1], A[11, 0], B[2, 3], B[N - 1, K - 1] = np.inf, -np.inf, np.nan, np.inf, np.nan
+        A[17, 2], A[18, 2], B[5, 7] = 3.4e38, -np.float32(3.4028235e38), 3.4028235e38
+        A[20], A[21], B[9] = A[20] * 1e-35, A[21] * 1e-41, B[9] * 1e-30
+        A[22], B[11] = 0., 0.
+        A[23], B[12] = A[23] * 1e30, B[12] * 1e30
+        a = dev(A.T if tA else A)
+        b = dev(B if tB else B.T)
+        c = {0: None, 1: dev(rng.standard_normal(N).astype(np.float32)), 2: dev(rng.standard_normal((M, N)).astype(np.float32))}[bias]
+
+        def product(engine, in_place):
+            ops.set_engine(engine)
+            out = c.clone() if in_place else None      # the bias and the result may be the same memory
+            y = ops.gemm_f32(a, b, out if in_place else c, transA=tA, transB=tB, alpha=1.5, beta=0.5, relu=relu, out=out)
+            assert ops.last_engine() == engine
+            return y.cpu().numpy()
+        ref = product(capi.ENGINE_SIMT, False)
+        assert relu or not np.isfinite(ref).all()
+        for in_place in ([False, True] if bias == 2 else [False]):
+            y = product(capi.ENGINE_TCGEN05, in_place)
+            assert np.array_equal(np.isnan(y), np.isnan(ref))
+            tiny = np.abs(ref) < 1e-29                 # 1.5 times a sum below 2^-96, as all of its parts are in a row this small
+            tiny[:20], tiny[21:] = False, False
+            assert np.array_equal(y[~np.isfinite(ref)], ref[~np.isfinite(ref)], equal_nan=True)
+            if bias == 0:
+                assert np.array_equal(y[tiny], ref[tiny])
+            # the reference is a chain of K roundings of 2^-24 of a growing sum: a standard deviation of sqrt(K / 6) * 2^-24, of which the
+            # largest of some ten thousand sums may show a dozen (1.1e-6 and 1.8e-5 at K = 2047)
+            ok = np.isfinite(ref) & (np.abs(ref) < 1e6)
+            bound = max(1e-5, 16 * np.sqrt(K / 6) * 2.0 ** -24)
+            scale = np.maximum(np.abs(ref[ok]), np.sqrt(np.mean(ref[ok].astype(np.float64) ** 2)))    # some sums are a thousand times the others
+            assert (np.abs(y[ok].astype(np.float64) - ref[ok]) / scale).max() <= bound
