@@ -58,10 +58,11 @@ int sofie_cuda_gemm_f32(void *stream, const sofie_gemm_f32_desc *d, const float 
    if (d->M == 0) return SOFIE_CUDA_OK; // an empty batch has no rows to compute (and may have NULL A / Y)
    SOFIE_REQUIRE(A && B && Y, "NULL tensor");
    cudaStream_t s = as_stream(stream);
-   // few rows, few columns, long K: split K over the grid. Up to 800 rows, where the tensor-core kernel's tiles of 128 rows lose to it
-   // (24 x 10 x 4096: 7.1 against 13.6 us; 1000 x 10 x 4096: 21.8 against 14.6)
+   // few rows, few columns, long K: split K over the grid, instead of running on two or three SMs. The tensor-core kernel is the faster one
+   // from about 800 rows on (1000 x 10 x 4096 14.6 against 21.8 us, 24 x 10 x 4096 13.6 against 7.1), but split-K's many short chains are
+   // the more precise: 1.0e-7 from float64 at K = 1500 against 1.2e-7, and 0.5e-7 against 1.8e-7 with operands of one sign.
    if (forced_engine() != SOFIE_ENGINE_TCGEN05 && rowblock_shape_ok(*d, A, B)) return launch_gemm_f32_rowblock(s, *d, A, B, C, Y); // one launch, no scratch
-   if (forced_engine() != SOFIE_ENGINE_TCGEN05 && splitk_shape_ok(*d) && (d->M <= 800 || forced_engine() == SOFIE_ENGINE_SIMT) && ceil_div(d->M, 128) < 32) {
+   if (forced_engine() != SOFIE_ENGINE_TCGEN05 && splitk_shape_ok(*d) && ceil_div(d->M, 128) < 32) {
       const int rc = launch_gemm_f32_splitk_auto(s, *d, A, B, C, Y);
       // no scratch buffer to be had (every slot of the pool belongs to another live stream, or the first call on this
       // stream came during a capture, where nothing can be allocated): the general kernels below take the shape too

@@ -809,3 +809,33 @@ def test_binary_operand_that_spans_more_than_32_bits(where, cuda_device):
         capi.call("sofie_cuda_binary_f32", C.c_void_p(torch.cuda.current_stream().cuda_stream), C.byref(d), *p, C.c_void_p(y.data_ptr()))
         rows = torch.cat([big[:6], big[stride:stride + 6]])
         assert torch.equal(y, rows - other if where == "a" else other - rows)
+
+
+@pytest.mark.parametrize("M,N,K", [(2340, 4, 1664), (2100, 16, 1028), (4000, 9, 2048), (3001, 1, 4096)])
+def test_rows_kernel_is_as_precise_as_split_k(M, N, K):
+    """Classifier heads on many rows: no further from float64 than the split-K sums of the same product (here of an unaligned copy)."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    for sign in (False, True):
+        A, B = torch.randn(M, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
+        if sign:
+            A, B = A.abs(), B.abs()
+        shifted = torch.empty(M * K + 1, device="cuda")[1:].view(M, K).copy_(A)
+        exact = A.double() @ B.double().t()
+        rows, split = ops.gemm_f32(A, B, transB=1), ops.gemm_f32(shifted, B, transB=1)
+        assert not torch.equal(rows, split)
+        error = float((rows.double() - exact).norm())
+        if sign: # all that is left are the last few roundings of either: within one of the result
+            assert error <= 2.0 ** -24 * float(exact.norm())
+        else:    # 2-norm of at least two thousand errors each: the ratio scatters by some per cent
+            assert error <= 1.05 * float((split.double() - exact).norm())
+
+
+@pytest.mark.parametrize("M,N,K,transB", [(1567, 9, 1558, 0), (801, 16, 1025, 1), (3968, 1, 3000, 0), (1000, 10, 4096, 0)])
+def test_skinny_products_stay_with_split_k(M, N, K, transB):
+    ops.set_engine(0)
+    g = torch.Generator(device="cuda").manual_seed(M)
+    A, B = torch.randn(M, K, device="cuda", generator=g), torch.randn((N, K) if transB else (K, N), device="cuda", generator=g)
+    y = ops.gemm_f32(A, B, transB=transB)
+    assert ops.last_engine() == capi.ENGINE_SIMT
+    exact = A.double() @ (B.double().t() if transB else B.double())
+    assert float((y.double() - exact).norm() / exact.norm()) <= 2.5e-7     # chains of at most some hundred terms
