@@ -13,8 +13,9 @@ struct ConvGeom {
 
 int launch_gemm_f32_simt(cudaStream_t, const sofie_gemm_f32_desc &, const float *, const float *, const float *, float *);
 int launch_gemm_f32_umma(cudaStream_t, const sofie_gemm_f32_desc &, const float *, const float *, const float *, float *);
-// any layout, alignment and K; long K split over a cluster (umma_gemm_any.cu)
-int launch_gemm_f32_any(cudaStream_t, const sofie_gemm_f32_desc &, const float *, const float *, const float *, float *);
+// any layout, alignment and K; long K split over a cluster (umma_gemm_any.cu). tma: operands the TMA kernel takes too; others are refused
+// where the CUDA-core kernel is the faster one
+int launch_gemm_f32_any(cudaStream_t, const sofie_gemm_f32_desc &, bool tma, const float *, const float *, const float *, float *);
 int launch_qgemm_simt(cudaStream_t, const sofie_qgemm_desc &, const uint8_t *, const int8_t *, const float *,
                       const int32_t *, uint8_t *, float *Yf32, float dq_scale);
 int launch_qgemm_umma(cudaStream_t, const sofie_qgemm_desc &, const uint8_t *, const int8_t *, const float *,

@@ -846,8 +846,10 @@ int launch_gemm_f32_umma(cudaStream_t s, const sofie_gemm_f32_desc &d, const flo
       return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "a product this small of rows TMA cannot fetch is faster on the CUDA cores (3.2 against 3.5 us)");
    // The kernel below overlaps a tile's epilogue with the next one's MMAs, which pays where a CTA has several tiles and each is short:
    // 100000 x 10 x 128 20 us against 29, 100000 x 128 x 128 48 against 54. Longer K or fewer tiles are the other kernel's, whose
-   // stages are cheaper and which splits K.
-   if (!tma || d.K >= 1024 || (long long)ceil_div(d.M, umma::kBM) * ceil_div(d.N, 64) < 2 * kNumSMs) return launch_gemm_f32_any(s, d, A, B, C, Y);
+   // stages are cheaper and which splits K -- unless the rows of Y are short, which this kernel's threads write one each: 500 x 1 x 12 3.8 us
+   // against 5.4, 327 x 2 x 120 5.6 against 6.7, but 163 x 52 x 104 7.8 against 6.1 and 17 x 1 x 236 8.0 against 6.2.
+   const bool few_tiles = (long long)ceil_div(d.M, umma::kBM) * ceil_div(d.N, 64) < 2 * kNumSMs, short_rows = d.N <= 24 && d.K < 224;
+   if (!tma || d.K >= 1024 || (few_tiles && !short_rows)) return launch_gemm_f32_any(s, d, tma, A, B, C, Y);
    umma::GemmEpilogue ep = {};
    ep.alpha = d.alpha;
    ep.beta = d.beta;

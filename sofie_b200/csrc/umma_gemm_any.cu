@@ -512,7 +512,7 @@ int launch_any(cudaStream_t s, const AnyOperand &A, const AnyOperand &B, const A
 } // namespace
 } // namespace umma
 
-int launch_gemm_f32_any(cudaStream_t s, const sofie_gemm_f32_desc &d, const float *A, const float *B, const float *C, float *Y)
+int launch_gemm_f32_any(cudaStream_t s, const sofie_gemm_f32_desc &d, bool tma, const float *A, const float *B, const float *C, float *Y)
 {
    using namespace umma;
    auto aligned = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
@@ -521,20 +521,35 @@ int launch_gemm_f32_any(cudaStream_t s, const sofie_gemm_f32_desc &d, const floa
    const AnyOperand b{B, d.transB ? d.K : d.N, d.N, !d.transB ? kRowsContiguous : (vec_k && aligned(B) ? kVecK : kScalarK)};
    const AnyEpilogue ep{d.alpha, d.beta, C, Y, d.bias_kind, d.relu, d.N % 4 == 0 && aligned(Y) && (d.bias_kind != 2 || aligned(C)), d.K >= 1024 ? 8 : (d.K >= 256 ? 4 : 3)};
    const int tm = ceil_div(d.M, kAnyBM), nkb = ceil_div(d.K, kAnyKE);
-   // Tile width and clusters along K by the time they take: a stage of 32 K costs about 1800 / 1150 / 900 clocks at 128 / 64 / 32
-   // columns, a tile's start and end about 6000, the exchange within a cluster 2500 more; clusters of 2 / 4 / 8 found room for
+   // Tile width and clusters along K by the time they take, in ns (fitted to 450 products, each at every width and cluster size): a stage
+   // of 32 K, a tile's start and end, the exchange within a cluster, and what the write-out takes more where rows of Y are not whole
+   // 16-byte words and where a bias of Y's shape is read. Nothing overlaps a CTA's write-out. Clusters of 2 / 4 / 8 found room for
    // 148 / 140 / 104 CTAs at a time.
-   static const int widths[3] = {128, 64, 32}, cost[3] = {1800, 1150, 900}, room[4] = {kNumSMs, kNumSMs, 140, 104};
+   static const int widths[3] = {128, 64, 32}, stage[3] = {1210, 700, 750}, tile[3] = {4100, 2300, 1500}, scalar[3] = {2000, 1000, 470}, scalar_full[3] = {3500, 1600, 950},
+                    room[4] = {kNumSMs, kNumSMs, 140, 104};
+   const bool vec = d.N % 4 == 0, full = d.bias_kind == 2;
+   const long long bias = full ? (long long)d.M * d.N / 750 : 0;
    int BN = 32, S = 1;
    long long best = -1;
    for (int w = 0; w < 3; w++) {
       if (widths[w] > 32 && widths[w] / 2 >= d.N) continue; // more than half of the tile would be padding
       const long long tiles = (long long)tm * ceil_div(d.N, widths[w]);
+      const int out = vec ? 0 : scalar[w] + (full ? scalar_full[w] : 0);
       for (int i = 0, q = 1; i < 4 && (q == 1 || (nkb >= 2 * q && tiles * q <= 3 * kNumSMs)); i++, q *= 2) {
          const long long waves = (tiles * q + room[i] - 1) / room[i];
-         const long long time = waves * ((long long)ceil_div(nkb, q) * cost[w] + 6000 + (q > 1 ? 2500 : 0));
+         const long long time = 1400 + bias + waves * ((long long)ceil_div(nkb, q) * stage[w] + tile[w] + out / q + (q > 1 ? 2100 : 0));
          if (best < 0 || time < best) best = time, BN = widths[w], S = q;
       }
+   }
+   // What TMA cannot fetch has the CUDA-core kernel beside it: blocks of 64 x 64, steps of 16 K that take 1.9 us alone and 0.45 us (0.65 with
+   // B stored [N,K]) apart on an SM full of them, whose outputs leave while other blocks compute. It wins where the output is what
+   // counts: 16384 x 4093 x 8 with a full bias 163 us against 580, 16384 x 777 x 64 81 against 144; 1000 x 777 x 1333 211 against 38. Over
+   // 620 products the choice is 0.9 % above the faster of the two in the mean, and never more than 5 % above the CUDA-core kernel.
+   if (!tma && forced_engine() != SOFIE_ENGINE_TCGEN05) {
+      const long long blocks = (long long)ceil_div(d.M, 64) * ceil_div(d.N, 64), steps = ceil_div(d.K, 16);
+      const long long alone = 1900 * steps * ((blocks + 3 * kNumSMs - 1) / (3 * kNumSMs));
+      const long long filled = ((d.transB ? 645 : 445) * steps + 800 + (full ? 330 : 0)) * blocks / kNumSMs;
+      if (2200 + (alone > filled ? alone : filled) < best) return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "faster on the CUDA cores");
    }
    if (BN == 128) return launch_any<128>(s, a, b, ep, d.K, S);
    if (BN == 64) return launch_any<64>(s, a, b, ep, d.K, S);

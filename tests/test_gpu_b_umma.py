@@ -335,3 +335,24 @@ def test_gemm_f32_of_values_the_parts_do_not_hold(M, N, K, bias, relu):
             bound = max(1e-5, 16 * np.sqrt(K / 6) * 2.0 ** -24)
             scale = np.maximum(np.abs(ref[ok]), np.sqrt(np.mean(ref[ok].astype(np.float64) ** 2)))    # some sums are a thousand times the others
             assert (np.abs(y[ok].astype(np.float64) - ref[ok]) / scale).max() <= bound
+
+
+@pytest.mark.parametrize("M,N,K,tA,tB,bias,engine", [
+    (16384, 1001, 9, 1, 0, 2, capi.ENGINE_SIMT), (4099, 2050, 8, 0, 0, 0, capi.ENGINE_SIMT), (8000, 777, 40, 1, 1, 2, capi.ENGINE_SIMT),   # output-bound
+    (3190, 824, 9, 0, 1, 1, capi.ENGINE_SIMT), (290, 1431, 10, 0, 0, 1, capi.ENGINE_SIMT),
+    (1000, 777, 1333, 1, 0, 2, capi.ENGINE_TCGEN05), (200, 200, 4000, 1, 1, 1, capi.ENGINE_TCGEN05), (4000, 1000, 500, 0, 0, 0, capi.ENGINE_TCGEN05),
+    (43, 158, 3447, 0, 0, 1, capi.ENGINE_TCGEN05)])
+def test_gemm_f32_takes_the_faster_kernel_where_tma_cannot_fetch(M, N, K, tA, tB, bias, engine):
+    """The choice between the tensor-core kernel and the CUDA-core one, and the result of either."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    A = torch.randn((K, M) if tA else (M, K), device="cuda", generator=g)
+    B = torch.randn((N, K) if tB else (K, N), device="cuda", generator=g) * K ** -0.5
+    C_ = {0: None, 1: torch.randn(N, device="cuda", generator=g), 2: torch.randn(M, N, device="cuda", generator=g)}[bias]
+    exact = 0.75 * ((A.double().t() if tA else A.double()) @ (B.double().t() if tB else B.double())) + (0 if C_ is None else 1.5 * C_.double())
+    ops.set_engine(0)
+    y = ops.gemm_f32(A, B, C_, transA=tA, transB=tB, alpha=0.75, beta=1.5)
+    assert ops.last_engine() == engine
+    assert float((y.double() - exact).norm() / exact.norm()) <= 2e-6     # 24-bit chains of up to 4000 terms: sqrt(K / 6) * 2^-24 = 1.6e-6
+    if engine == capi.ENGINE_SIMT:
+        ops.set_engine(capi.ENGINE_SIMT)
+        assert torch.equal(y, ops.gemm_f32(A, B, C_, transA=tA, transB=tB, alpha=0.75, beta=1.5))
