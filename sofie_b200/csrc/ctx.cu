@@ -843,7 +843,11 @@ int sofie_cuda_ctx_result_end(sofie_cuda_ctx *ctx, void **host)
    SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
    if (ctx->result_stream) SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->result_stream));
    l.open = false;
-   slots_free(ctx); // the stream has waited for every part that was copied in
+   // the stream has waited for every part that was copied in and waited for; a part that was not may still be read out of the ring
+   bool copying = false;
+   for (auto &slot : ctx->slots) copying = copying || (slot.busy && slot.stream == ctx->copy_stream);
+   if (copying) SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->copy_stream));
+   slots_free(ctx);
    if (carry && l.parts == 1) ctx->host_pool->copy(l.out + l.offset[0], l.land + l.offset[0], l.count[0]);
    if (l.mapped && l.out) std::memcpy(l.out, l.mapped, l.bytes);
    *host = l.out ? l.out : (l.mapped ? const_cast<char *>(l.mapped) : l.land);

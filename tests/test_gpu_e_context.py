@@ -287,3 +287,27 @@ def test_no_copy_writes_the_result_of_an_inference_that_failed(cuda_device):
         time.sleep(0.02)
         assert (out == -12345.).all()
         assert s.infer(x, out) is out and np.array_equal(out.view(np.uint32), want.view(np.uint32))
+
+
+def test_a_part_nobody_waited_for_keeps_its_staging_slots(cuda_device):
+    """An input part that is still on its way when a result ends: its bytes in the staging ring are not overwritten by the next copy."""
+    ctx, _ = _ctx(64 << 20)
+    try:
+        n = 24 << 20
+        first, second, result, host = C.c_void_p(), C.c_void_p(), C.c_void_p(), C.c_void_p()
+        for p, off, size in ((first, 0, n), (second, n, n), (result, 2 * n, 256)):
+            capi.call("sofie_cuda_ctx_arena", ctx, off, size, C.byref(p))
+        a, b = np.full(n, 1, np.uint8), np.full(n, 2, np.uint8)
+        for _ in range(60):
+            capi.call("sofie_cuda_ctx_result_begin", ctx, None, 256)
+            capi.call("sofie_cuda_ctx_h2d_part", ctx, first, a.ctypes.data_as(C.c_void_p), n, 0)
+            capi.call("sofie_cuda_ctx_result_part", ctx, result, 0, 256)
+            capi.call("sofie_cuda_ctx_result_end", ctx, C.byref(host))
+            capi.call("sofie_cuda_ctx_h2d_part", ctx, second, b.ctypes.data_as(C.c_void_p), n, 1)
+            capi.call("sofie_cuda_ctx_wait_part", ctx, 0)
+            capi.call("sofie_cuda_ctx_wait_part", ctx, 1)
+            got = np.zeros(n, np.uint8)
+            capi.call("sofie_cuda_ctx_d2h", ctx, got.ctypes.data_as(C.c_void_p), first, n)
+            assert (got == 1).all()
+    finally:
+        capi.call("sofie_cuda_ctx_destroy", ctx)
