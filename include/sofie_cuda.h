@@ -104,6 +104,8 @@ int sofie_cuda_ctx_unquantize(sofie_cuda_ctx *ctx, const uint8_t *src_device, fl
  * sofie_cuda_ctx_stage_settle, after which no helper reads it. */
 int sofie_cuda_ctx_stage_ahead(sofie_cuda_ctx *ctx, const void *src_host, size_t bytes, int kind, float scale, int32_t zp);
 int sofie_cuda_ctx_stage_settle(sofie_cuda_ctx *ctx);
+/* Self test of the helper threads (needs no GPU): helpers[i] = how many the i-th of `transfers` transfers at the same time gets. */
+int sofie_cuda_selftest_host_pools(int transfers, int *helpers);
 /* Self test of failures on the host: the nth copy out of the staging ring from now on is refused (0: none). */
 int sofie_cuda_selftest_fail_copy(sofie_cuda_ctx *ctx, int nth);
 /* Self test of that quantisation on plain host memory (needs no GPU). */

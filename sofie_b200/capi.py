@@ -105,6 +105,7 @@ SIGNATURES = {
     "sofie_cuda_ctx_result_end": [vp, C.POINTER(vp)],
     "sofie_cuda_ctx_result_abort": [vp],
     "sofie_cuda_selftest_fail_copy": [vp, C.c_int],
+    "sofie_cuda_selftest_host_pools": [C.c_int, C.POINTER(C.c_int)],
     "sofie_cuda_host_alloc": [sz, C.POINTER(vp)],
     "sofie_cuda_host_free": [vp],
     "sofie_cuda_ctx_sync": [vp],

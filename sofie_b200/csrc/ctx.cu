@@ -107,7 +107,7 @@ struct sofie_cuda_ctx {
       bool busy = false, recorded = false;
    } slots[kStagingSlots];
    int next_slot = 0;
-   std::unique_ptr<sofie::HostPool> host_pool; // made on first use
+   sofie::HostPool *host_pool = nullptr; // borrowed from the process's while a transfer runs
    // one slot being filled by the pool: `bytes` of the slot from `src`
    struct Fill {
       sofie::HostConvert how;
@@ -273,6 +273,7 @@ int sofie_cuda_ctx_create(sofie_cuda_ctx **out, int device, size_t arena_bytes)
                   "context creation on device %d (arena %zu bytes): %s", device, arena_bytes, cudaGetErrorString(err));
    }
    register_stream_status(ctx->stream, ctx->status);
+   HostPools::get().user_begins();
    if (const char *t = std::getenv("SOFIE_CUDA_TIMERS")) ctx->timers_on = std::atoi(t) != 0;
    *out = ctx;
    return SOFIE_CUDA_OK;
@@ -286,6 +287,7 @@ int sofie_cuda_ctx_destroy(sofie_cuda_ctx *ctx)
    DeviceGuard guard(ctx->device);
    // nothing of this context may still be running or copying when its memory goes away
    settle(ctx);
+   HostPools::get().user_ends();
    cudaStreamSynchronize(ctx->stream);
    if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
    if (ctx->result_stream) cudaStreamSynchronize(ctx->result_stream);
@@ -373,17 +375,15 @@ int sofie_cuda_ctx_upload(sofie_cuda_ctx *ctx, const void *host, size_t bytes, v
 
 static int ensure_pool(sofie_cuda_ctx *ctx)
 {
-   if (ctx->host_pool) return SOFIE_CUDA_OK;
-   // All cores but two, fourteen at most. Measured on a 16-core host, int8 CNN on 16384 images (268 MB of floats quantised while
-   // they are staged): 4.06 ms per call with eight threads, 3.83 with ten, 3.0 with twelve, 2.65 with fourteen.
-   const int cores = (int)std::thread::hardware_concurrency();
-   int threads = cores - 2 < 14 ? cores - 2 : 14;
-   if (const char *e = std::getenv("SOFIE_CUDA_COPY_THREADS")) threads = std::atoi(e);
-   if (cores > 0 && threads > cores) threads = cores;
-   if (threads < 1) threads = 1;
-   if (threads > 16) threads = 16;
-   ctx->host_pool.reset(new HostPool(threads - 1));
-   return SOFIE_CUDA_OK;
+   if (!ctx->host_pool) ctx->host_pool = HostPools::get().borrow();
+   return ctx->host_pool ? SOFIE_CUDA_OK : fail(SOFIE_CUDA_ERR_NOMEM, "no memory for the helper threads");
+}
+
+// No job is left: the helpers are another transfer's.
+static void release_pool(sofie_cuda_ctx *ctx)
+{
+   if (ctx->host_pool) HostPools::get().give_back(ctx->host_pool);
+   ctx->host_pool = nullptr;
 }
 
 static int ensure_staging(sofie_cuda_ctx *ctx)
@@ -464,6 +464,7 @@ static void settle(sofie_cuda_ctx *ctx)
 {
    if (ctx->host_pool) ctx->host_pool->finish();
    ctx->ahead = nullptr;
+   release_pool(ctx);
 }
 
 // A small input's way out of pinned memory: read across PCIe by the SMs themselves. The copy engine takes 10 us and more for 256 KB
@@ -508,7 +509,7 @@ static int stage_slots(sofie_cuda_ctx *ctx, const HostConvert &how, void *dst, c
       ctx->ahead = nullptr;
    } else {
       settle(ctx);
-      if ((rc = begin_fill(ctx, how, src, bytes < step ? bytes : step, &cur))) return rc;
+      if ((rc = ensure_pool(ctx)) || (rc = begin_fill(ctx, how, src, bytes < step ? bytes : step, &cur))) return rc;
    }
    for (size_t done = 0; done < bytes;) {
       ctx->host_pool->finish();
@@ -533,7 +534,7 @@ static int stage_slots(sofie_cuda_ctx *ctx, const HostConvert &how, void *dst, c
 static int stage_in(sofie_cuda_ctx *ctx, const HostConvert &how, void *dst, const void *src, size_t bytes, cudaStream_t stream)
 {
    const int rc = stage_slots(ctx, how, dst, src, bytes, stream);
-   if (rc) settle(ctx);
+   settle(ctx);
    return rc;
 }
 
@@ -556,6 +557,25 @@ int sofie_cuda_ctx_h2d(sofie_cuda_ctx *ctx, void *dst, const void *src, size_t b
       return SOFIE_CUDA_OK;
    }
    return stage_in(ctx, HostConvert(), dst, src, bytes, ctx->stream);
+}
+
+int sofie_cuda_selftest_host_pools(int transfers, int *helpers)
+{
+   SOFIE_REQUIRE(helpers && transfers >= 1 && transfers <= 64, "bad number of transfers");
+   auto &pools = HostPools::get();
+   HostPool *lent[64];
+   pools.user_begins();
+   int rc = SOFIE_CUDA_OK, n = 0;
+   for (; n < transfers; n++) {
+      if (!(lent[n] = pools.borrow())) {
+         rc = fail(SOFIE_CUDA_ERR_NOMEM, "no memory for the helper threads");
+         break;
+      }
+      helpers[n] = (int)lent[n]->threads() - 1;
+   }
+   while (n > 0) pools.give_back(lent[--n]);
+   pools.user_ends();
+   return rc;
 }
 
 int sofie_cuda_selftest_fail_copy(sofie_cuda_ctx *ctx, int nth)
@@ -724,6 +744,7 @@ int sofie_cuda_ctx_d2h(sofie_cuda_ctx *ctx, void *dst, const void *src, size_t b
       }
       done += round;
    }
+   release_pool(ctx);
    return SOFIE_CUDA_OK;
 }
 
@@ -849,6 +870,7 @@ int sofie_cuda_ctx_result_end(sofie_cuda_ctx *ctx, void **host)
    if (copying) SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->copy_stream));
    slots_free(ctx);
    if (carry && l.parts == 1) ctx->host_pool->copy(l.out + l.offset[0], l.land + l.offset[0], l.count[0]);
+   release_pool(ctx);
    if (l.mapped && l.out) std::memcpy(l.out, l.mapped, l.bytes);
    *host = l.out ? l.out : (l.mapped ? const_cast<char *>(l.mapped) : l.land);
    return report_status(ctx);

@@ -168,3 +168,52 @@ def test_strides_of_a_broadcast_operand(a, b):
         ops.binary_strides((1, 1, 1, 1, 2), (1,))
     with pytest.raises(RuntimeError):
         ops.binary_strides((2,), (3,))
+
+
+def test_transfers_share_the_helper_threads_of_the_process():
+    """One transfer may have all cores but two (at most fourteen threads with the caller); transfers at the same time get what is left,
+    three helpers at least; one after the other they use the same threads, and none is left when the last context is gone."""
+    import os
+    import subprocess
+    import sys
+    script = (
+        "import ctypes as C, os, sys\n"
+        "sys.path.insert(0, sys.argv[1])\n"
+        "from sofie_b200 import capi\n"
+        "capi.load()\n"
+        "threads = lambda: len(os.listdir('/proc/self/task'))\n"
+        "before = threads()\n"
+        "h = (C.c_int * 5)()\n"
+        "for n in (1, 1, 5, 1):\n"
+        "    capi.call('sofie_cuda_selftest_host_pools', n, h)\n"
+        "    print(*h[:n])\n"
+        "    assert threads() == before, (threads(), before)\n")
+    r = subprocess.run([sys.executable, "-c", script, str(ROOT)], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout
+    one, again, five, last = [[int(v) for v in line.split()] for line in r.stdout.strip().splitlines()[-4:]]
+    cores = len(os.sched_getaffinity(0))
+    first = max(min(cores - 2, 14), 1) - 1
+    assert one == again == last == [first] and five[0] == first
+    assert all(h == min(first, 3) for h in five[1:]) or cores > 17
+    assert sum(five) <= max(cores - 2, first + 3 * 4)
+
+
+def test_helper_threads_that_cannot_be_started_are_done_without(tmp_path):
+    """A process at its limit of threads (here: of address space, which their stacks need) copies with the threads it gets."""
+    import subprocess
+    import sys
+    script = (
+        "import ctypes as C, resource, sys\n"
+        "sys.path.insert(0, sys.argv[1])\n"
+        "from sofie_b200 import capi\n"
+        "capi.load()\n"
+        "used = int(open('/proc/self/statm').read().split()[0]) * resource.getpagesize()\n"
+        "n = 8 << 20\n"
+        "libc, src, dst = C.CDLL(None), (C.c_char * n)(*[7] * 64), (C.c_char * n)()\n"
+        "used = int(open('/proc/self/statm').read().split()[0]) * resource.getpagesize()\n"
+        "resource.setrlimit(resource.RLIMIT_AS, (used + (20 << 20), used + (20 << 20)))\n"
+        "rc = capi.load().sofie_cuda_selftest_host_copy(dst, src, n, 1 << 20, 16, 3)\n"
+        "assert rc == 0 and libc.memcmp(dst, src, n) == 0\n"
+        "print('ok')\n")
+    r = subprocess.run([sys.executable, "-c", script, str(ROOT)], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), (r.returncode, r.stdout[-2000:])

@@ -311,3 +311,28 @@ def test_a_part_nobody_waited_for_keeps_its_staging_slots(cuda_device):
             assert (got == 1).all()
     finally:
         capi.call("sofie_cuda_ctx_destroy", ctx)
+
+
+def test_sessions_share_the_helper_threads(cuda_device):
+    """Sessions called one after the other add no threads; called at the same time from several threads they give the same results."""
+    import os
+    import threading
+    m, x = configs.mlp_i8(batch=2048)
+    sessions = [generated.session_from_model(m, "c3_b2048_threads") for _ in range(6)]
+    want = sessions[0].infer(x)
+    threads = len(os.listdir("/proc/self/task"))
+    for s in sessions:
+        assert np.array_equal(s.infer(x).view(np.uint32), want.view(np.uint32))
+    assert len(os.listdir("/proc/self/task")) <= threads + 2        # the driver's own, at most
+    wrong = []
+
+    def work(s):
+        for _ in range(50):
+            if not np.array_equal(s.infer(x).view(np.uint32), want.view(np.uint32)):
+                wrong.append(1)
+    workers = [threading.Thread(target=work, args=(s,)) for s in sessions]
+    for t in workers:
+        t.start()
+    for t in workers:
+        t.join()
+    assert not wrong
