@@ -11,7 +11,9 @@
 //               per four k one 16-byte load of its row and one 16-byte load per column
 //   ROWS        32, 16 or 8: the largest that still gives every SM a tile, so that a small batch
 //               spreads over the whole GPU (each block stages the weights from L2 either way)
-// Eight rows have a kernel of their own (mlp_rows8_kernel): what counts there is the time of one tile, from launch to result.
+// A kernel of its own for eight rows (K split over a warp's quarters, 512 threads, two more shuffles and barriers of twice the warps) was
+// slower at every size: 64 -> 128 -> 128 -> 10 9.2 us instead of 8.25 for one row and 9.6 instead of 8.6 for 1024, back to back; 14.3
+// instead of 12.3 after an L2 flush.
 // Staging uses 16-byte asynchronous copies (all of a block's weight bytes in flight at once) when
 // the layout allows it: [N][K] weights, K a multiple of 4, 16-byte aligned pointers. The input
 // tile of the next batch rows is fetched while the layers after the first run.
@@ -34,7 +36,6 @@ struct MlpParams {
    int x_off, x_ld;                 // input tile [ROWS][x_ld]
    int act_off[2], act_ld;          // the two activation buffers [ROWS][act_ld]
    int w_vec[SOFIE_MLP_MAX_LAYERS]; // layer's weights can be staged with 16-byte copies
-   FastDiv kq[SOFIE_MLP_MAX_LAYERS]; // 16-byte pieces of a row
    int x_vec;
 };
 
@@ -240,153 +241,6 @@ mlp_fused_f32_kernel(MlpParams p, const float *__restrict__ X, float *__restrict
    cp_async_wait_all();
 }
 
-// ---- eight rows per tile: the latency of one tile -----------------------------------------------------------------
-// 512 threads: lane = (row lane % 8, quarter of K lane / 8), a warp takes every 16th column. All eight rows of a quarter warp read the
-// same 16 bytes of a weight row, the four quarters the 48 bytes behind them, so a weight load is one shared-memory wavefront for
-// 4 x 8 x 4 products (the mapping above: one for 4 x 4), and a thread's chain of additions is a quarter as long; the quarters are
-// added by two shuffles. The blocks start staging a layer's weights at different places, so that they do not all ask the
-// same L2 slices for the same lines at the same time. 64 -> 128 -> 128 -> 10: one row 9.0 us -> kRow1, 1024 rows 13.1 us -> kRow1024.
-constexpr int kMlpThreads8 = 512, kMlpWarps8 = kMlpThreads8 / 32;
-
-template <int J>
-__device__ __forceinline__ void mlp_layer8(const float *__restrict__ arow, const float *__restrict__ w0, const float *__restrict__ bs, float *__restrict__ nxt, int Kp,
-                                           int ldw, int N4, int warp, int quarter, bool relu)
-{
-   float acc[J];
-#pragma unroll
-   for (int j = 0; j < J; j++) acc[j] = 0.f;
-#pragma unroll 2
-   for (int k = 4 * quarter; k < Kp; k += 16) {
-      const float4 a = *reinterpret_cast<const float4 *>(arow + k);
-#pragma unroll
-      for (int j = 0; j < J; j++) {
-         const float4 wv = *reinterpret_cast<const float4 *>(w0 + (size_t)(j * kMlpWarps8) * ldw + k);
-         acc[j] = fmaf(a.x, wv.x, acc[j]);
-         acc[j] = fmaf(a.y, wv.y, acc[j]);
-         acc[j] = fmaf(a.z, wv.z, acc[j]);
-         acc[j] = fmaf(a.w, wv.w, acc[j]);
-      }
-   }
-#pragma unroll
-   for (int j = 0; j < J; j++) {
-      acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 8);
-      acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], 16);
-      const int n = warp + kMlpWarps8 * j;
-      if (quarter == (j & 3) && n < N4) {
-         const float v = acc[j] + bs[n];
-         nxt[n] = relu ? relu_ref(v) : v;
-      }
-   }
-}
-
-__global__ void __launch_bounds__(kMlpThreads8, 1) mlp_rows8_kernel(MlpParams p, const float *__restrict__ X, float *__restrict__ Y)
-{
-   constexpr int ROWS = 8;
-   extern __shared__ __align__(16) float sm[];
-   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane & 7, quarter = lane >> 3;
-   const int L = p.d.layers, M = p.d.M, tiles = (M + ROWS - 1) / ROWS;
-   auto load_x = [&](int tile) {
-      const int K0 = p.d.dims[0], m0 = tile * ROWS, kq = (K0 + 3) >> 2;
-      float *xin = sm + p.x_off;
-      for (int i = tid; i < ROWS * kq; i += kMlpThreads8) {
-         uint32_t c;
-         const int rr = (int)p.kq[0].divmod((uint32_t)i, c), k = 4 * (int)c;
-         const bool ok = m0 + rr < M;
-         const float *src = X + (size_t)(ok ? m0 + rr : 0) * K0 + k;
-         if (p.x_vec) cp_async16(xin + rr * p.x_ld + k, src, ok);
-         else
-            for (int j = 0; j < 4; j++) xin[rr * p.x_ld + k + j] = ok && k + j < K0 ? __ldg(src + j) : 0.f;
-      }
-   };
-   // copy groups: [input tile + layer 0], [layer 1], ..., [layer L-1]; a layer starts when its own group has landed
-   load_x(blockIdx.x);
-   for (int l = 0; l < L; l++) {
-      const int K = p.d.dims[l], N = p.d.dims[l + 1], Np = (N + 31) & ~31, ld = p.w_ld[l], kq = (K + 3) >> 2;
-      float *wt = sm + p.w_off[l];
-      const float *Wg = p.W[l];
-      if (p.w_vec[l]) {
-         const int total = N * kq;
-         int i = tid + (int)(((long long)blockIdx.x * total) / gridDim.x); // every block begins elsewhere and wraps round
-         if (i >= total) i -= total;
-         for (int done = tid; done < total; done += kMlpThreads8) {
-            uint32_t c;
-            const int n = (int)p.kq[l].divmod((uint32_t)i, c);
-            cp_async16(wt + n * ld + 4 * (int)c, Wg + (size_t)n * K + 4 * (int)c, true);
-            i += kMlpThreads8;
-            while (i >= total) i -= total;
-         }
-         for (int z = tid; z < (Np - N) * ld; z += kMlpThreads8) wt[N * ld + z] = 0.f; // columns past N contribute nothing
-      } else {
-         for (int i = tid; i < Np * kq; i += kMlpThreads8) {
-            // [N][K]: consecutive threads on consecutive K; [K][N]: on consecutive columns
-            int n, c;
-            if (p.d.w_is_nk[l]) {
-               n = i / kq;
-               c = i - n * kq;
-            } else {
-               c = i / Np;
-               n = i - c * Np;
-            }
-            for (int k = 4 * c; k < 4 * c + 4; k++)
-               wt[n * ld + k] = (n < N && k < K) ? __ldg(p.d.w_is_nk[l] ? Wg + (size_t)n * K + k : Wg + (size_t)k * N + n) : 0.f;
-         }
-      }
-      float *bs = sm + p.b_off[l];
-      for (int n = tid; n < Np; n += kMlpThreads8) {
-         if (n < N && p.B[l]) cp_async4(bs + n, p.B[l] + n);
-         else bs[n] = 0.f;
-      }
-      cp_async_commit();
-   }
-   bool first = true;
-   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-      const int m0 = tile * ROWS;
-      if (!first) {
-         cp_async_wait_all();
-         __syncthreads(); // this tile's input has landed; the previous tile's buffers are free
-      }
-      for (int l = 0; l < L; l++) {
-         if (first) {
-            // groups still allowed in flight: the later layers' and, behind layer 0, the next tile's input
-            cp_async_wait_pending(L - 1 - l + (l > 0 ? 1 : 0));
-            __syncthreads();
-         }
-         const int K = p.d.dims[l], N = p.d.dims[l + 1], Kp = (K + 3) & ~3, ldw = p.w_ld[l], lda = l == 0 ? p.x_ld : p.act_ld;
-         const float *arow = sm + (l == 0 ? p.x_off : p.act_off[(l - 1) & 1]) + r * lda;
-         const float *w0 = sm + p.w_off[l] + warp * ldw;
-         const float *bs = sm + p.b_off[l];
-         const bool relu = p.d.relu[l] != 0;
-         const int N4 = (N + 3) & ~3; // the next layer reads k up to its K rounded to 4: columns N .. N4 are written as zeros
-         float *nxt = sm + p.act_off[l & 1] + r * p.act_ld;
-         switch (((N + 31) & ~31) >> 5) { // the column count is a compile-time constant inside: no predicated-off work
-         case 1: mlp_layer8<2>(arow, w0, bs, nxt, Kp, ldw, N4, warp, quarter, relu); break;
-         case 2: mlp_layer8<4>(arow, w0, bs, nxt, Kp, ldw, N4, warp, quarter, relu); break;
-         case 3: mlp_layer8<6>(arow, w0, bs, nxt, Kp, ldw, N4, warp, quarter, relu); break;
-         case 4: mlp_layer8<8>(arow, w0, bs, nxt, Kp, ldw, N4, warp, quarter, relu); break;
-         case 5: mlp_layer8<10>(arow, w0, bs, nxt, Kp, ldw, N4, warp, quarter, relu); break;
-         case 6: mlp_layer8<12>(arow, w0, bs, nxt, Kp, ldw, N4, warp, quarter, relu); break;
-         case 7: mlp_layer8<14>(arow, w0, bs, nxt, Kp, ldw, N4, warp, quarter, relu); break;
-         default: mlp_layer8<16>(arow, w0, bs, nxt, Kp, ldw, N4, warp, quarter, relu); break;
-         }
-         __syncthreads(); // the next layer (or the copy-out) reads what every warp wrote
-         if (l == 0) {
-            if (tile + (int)gridDim.x < tiles) load_x(tile + gridDim.x); // the input buffer is free
-            cp_async_commit(); // committed even when empty: the group count above does not depend on the tile
-         }
-      }
-      first = false;
-      const int N = p.d.dims[L]; // the tile's rows are one contiguous piece of Y
-      const float *out = sm + p.act_off[(L - 1) & 1];
-      const int rows = M - m0 < ROWS ? M - m0 : ROWS;
-      float *Yt = Y + (size_t)m0 * N;
-      for (int i = tid; i < rows * N; i += kMlpThreads8) {
-         const int rr = i / N, n = i - rr * N;
-         Yt[i] = out[rr * p.act_ld + n];
-      }
-   }
-   cp_async_wait_all();
-}
-
 template <int ROWS>
 int launch_mlp(cudaStream_t stream, MlpParams &p, int floats, int maxact, const float *X, float *Y)
 {
@@ -399,13 +253,8 @@ int launch_mlp(cudaStream_t stream, MlpParams &p, int floats, int maxact, const 
    floats += 2 * ROWS * p.act_ld;
    const size_t smem = (size_t)floats * sizeof(float);
    const int tiles = (p.d.M + ROWS - 1) / ROWS, blocks = tiles < kNumSMs ? tiles : kNumSMs;
-   if constexpr (ROWS == 8) {
-      SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(mlp_rows8_kernel), (int)smem));
-      mlp_rows8_kernel<<<blocks, kMlpThreads8, smem, stream>>>(p, X, Y);
-   } else {
-      SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(mlp_fused_f32_kernel<ROWS>), (int)smem));
-      mlp_fused_f32_kernel<ROWS><<<blocks, kMlpThreads, smem, stream>>>(p, X, Y);
-   }
+   SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(mlp_fused_f32_kernel<ROWS>), (int)smem));
+   mlp_fused_f32_kernel<ROWS><<<blocks, kMlpThreads, smem, stream>>>(p, X, Y);
    SOFIE_LAUNCH_CHECK("mlp_fused_f32_kernel");
    return SOFIE_CUDA_OK;
 }
@@ -442,7 +291,6 @@ extern "C" int sofie_cuda_mlp_f32(void *stream, const sofie_mlp_desc *d, const f
       p.W[l] = W[l];
       p.B[l] = B ? B[l] : nullptr;
       p.w_vec[l] = d->w_is_nk[l] && K % 4 == 0 && (reinterpret_cast<uintptr_t>(W[l]) & 15) == 0;
-      p.kq[l] = FastDiv((uint32_t)((K + 3) >> 2));
       p.w_ld[l] = padded_ld(K);
       p.w_off[l] = floats;
       floats += Np * p.w_ld[l];
