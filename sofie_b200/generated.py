@@ -13,6 +13,7 @@ import contextlib
 import ctypes as C
 import fcntl
 import hashlib
+import mmap
 import os
 import shutil
 import subprocess
@@ -23,7 +24,7 @@ from pathlib import Path
 
 import numpy as np
 
-from . import _build, capi
+from . import _build
 
 ROOT = Path(__file__).resolve().parent.parent
 HOST = Path(__file__).resolve().parent / "host"
@@ -201,24 +202,21 @@ def compile_session(hxx: Path, name: str, in_type="float", out_type="float") -> 
     return so
 
 
-class _PinnedBuffer:
-    """Pinned host memory for one result; freed when neither the Session nor an array over it is left."""
+class _Buffer:
+    """Memory for one result; kept by the Session and by the array over it. Mapped apart from the heap, whose blocks come and go."""
 
     def __init__(self, nbytes: int):
         self.nbytes = nbytes
-        self.ptr = C.c_void_p()
-        capi.call("sofie_cuda_host_alloc", nbytes, C.byref(self.ptr))
-        self.free = capi.load().sofie_cuda_host_free
+        self.memory = mmap.mmap(-1, nbytes, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+        if hasattr(mmap, "MADV_HUGEPAGE"):
+            try:
+                self.memory.madvise(mmap.MADV_HUGEPAGE)
+            except OSError:
+                pass                   # a kernel without them
         self.array = None          # weak reference to the array handed out over it; views of that array keep it alive
 
-    def __del__(self):
-        if getattr(self, "free", None) is not None and self.ptr:
-            self.free(self.ptr)
-
     def lend(self, n: int, dtype) -> np.ndarray:
-        mem = (C.c_char * (n * dtype.itemsize)).from_address(self.ptr.value)
-        mem.owner = self
-        a = np.frombuffer(mem, dtype, n)
+        a = np.frombuffer((C.c_char * (n * dtype.itemsize)).from_buffer(self.memory), dtype, n)
         self.array = weakref.ref(a)
         return a
 
@@ -227,23 +225,23 @@ class _PinnedBuffer:
 
 
 class _ResultArrays:
-    """The arrays infer() returns. From kPinnedFrom bytes on they lie in pinned memory, which the device copies the result into
-    directly: a fresh np.empty of that size is memory the kernel hands out page by page on first touch (measured: 2 GB/s, against
-    55 GB/s of the copy itself), and the result would have to be carried over from pinned memory besides. A buffer comes back when
-    the array over it (and every view of it) is gone, and is used again; a program that keeps more than kBuffers results of one
-    Session gets ordinary arrays from then on, so pinned memory stays bounded by kBuffers results per Session."""
-    kPinnedFrom, kBuffers = 128 << 10, 3
+    """The arrays infer() returns. From kKeptFrom bytes on their memory is used again: a fresh np.empty of that size is memory the kernel
+    hands out page by page on first touch (measured: 2 GB/s, against 55 GB/s of the copy). A buffer comes back when the array over it
+    (and every view of it) is gone; a program that keeps more than kBuffers results of one Session gets ordinary arrays from then on, so
+    what a Session holds on to stays bounded. The memory is ordinary memory, not pinned: a copy that a program starts out of a result on
+    a stream of its own has read it by the time the call returns, however soon the array is gone and its memory the next result's."""
+    kKeptFrom, kBuffers = 128 << 10, 3
 
     def __init__(self):
         self.buffers = []
         self.lock = threading.Lock()
 
     def new(self, n: int, dtype) -> np.ndarray:
-        if n * 8 < self.kPinnedFrom:
+        if n * 8 < self.kKeptFrom:
             return np.empty(n, dtype)
         dtype = np.dtype(dtype)
         nbytes = n * dtype.itemsize
-        if nbytes < self.kPinnedFrom:
+        if nbytes < self.kKeptFrom:
             return np.empty(n, dtype)
         with self.lock:
             spare = None
@@ -255,10 +253,7 @@ class _ResultArrays:
             if spare is not None:
                 self.buffers.remove(spare)      # too small for this batch: its place goes to a larger one
             if len(self.buffers) < self.kBuffers:
-                try:
-                    b = _PinnedBuffer(nbytes)
-                except capi.SofieCudaError:
-                    return np.empty(n, dtype)   # no pinned memory to be had: the result is carried over by the host
+                b = _Buffer(nbytes)
                 self.buffers.append(b)
                 return b.lend(n, dtype)
         return np.empty(n, dtype)

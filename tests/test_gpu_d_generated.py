@@ -330,7 +330,7 @@ def test_batch_sharded_over_sessions_with_the_helper(cuda_device, tmp_path):
 def test_batch_cut_into_ranges_of_samples(key, batch, dynamic, cuda_device):
     """Batches that do not split into equal parts, from 4 MB of input on: infer() cuts them into ranges (the last one short). The result
     is that of the whole batch (the same model emitted with one upload), from pageable and from pinned memory, into a fresh array, into
-    memory of the caller, and for more results kept alive than a Session lends pinned buffers for."""
+    memory of the caller, and for more results kept alive than a Session keeps buffers for."""
     import torch
     build = configs.resblock_f32 if key == "RES" else configs.BUILDERS[key]
     m, x = build(batch=batch)
@@ -382,3 +382,40 @@ def test_ranges_of_a_network_whose_layers_shrink(dynamic, cuda_device):
     assert capi_slice_rows(batch, x[0].nbytes) < batch
     for _ in range(200):
         assert np.array_equal(s.infer(x).view(np.uint32), whole.view(np.uint32))
+
+
+def test_a_result_that_is_gone_may_still_be_on_its_way_to_the_device(cuda_device):
+    """A program copies a result to the device without waiting, on a stream that is busy, and drops it; the next results take its memory.
+    What arrives is the result that was copied."""
+    import torch
+    m, x = configs.mlp_i8(batch=2048)
+    s = generated.session_from_model(m, "c3_b2048_gone")
+    inputs = [np.ascontiguousarray(x * k) for k in (1., -1., 0.5, -0.5)]
+    want = [s.infer(i).copy() for i in inputs]
+    busy = torch.randn(6000, 6000, device=cuda_device)
+    side = torch.cuda.Stream()
+    for _ in range(3):
+        arrived = []
+        with torch.cuda.stream(side):
+            for i in inputs:
+                busy @ busy
+                y = s.infer(i)
+                assert not torch.from_numpy(y).is_pinned()
+                arrived.append(torch.from_numpy(y).to(cuda_device, non_blocking=True))
+                arrived.append(torch.from_numpy(y[100:]).to(cuda_device, non_blocking=True))
+                del y
+        torch.cuda.synchronize()
+        for k, w in enumerate(want):
+            assert np.array_equal(arrived[2 * k].cpu().numpy(), w) and np.array_equal(arrived[2 * k + 1].cpu().numpy(), w[100:])
+
+
+def test_results_of_one_part_and_more_reach_ordinary_memory(cuda_device):
+    """Results carried over by the host: below one piece, one piece, a few, in uneven pieces, and parts of a batch."""
+    for batch in (20, 200, 257, 513, 1000, 2047, 4099):
+        m, x = configs.mlp_i8(batch=batch)
+        s = generated.session_from_model(m, f"c3_b{batch}_carry")
+        import torch
+        pinned = torch.empty(batch * 256, pin_memory=True).numpy()
+        s.infer(x, pinned)
+        out = np.full(batch * 256, np.nan, np.float32)
+        assert np.array_equal(s.infer(x, out).view(np.uint32), pinned.view(np.uint32))
