@@ -599,10 +599,9 @@ __global__ void quantize_e4m3_kernel(const In *__restrict__ X, uint8_t *__restri
    }
 }
 
-// Eight elements per thread and step: 16- or 32-byte loads, one 8-byte store.
-// x / scale for a value that is rounded to E4M3 next, by multiplication where that gives the same byte (see the comment at the
-// definition in the FP8 GEMM's epilogue: only values within a few units of an fp32 number with 19 zero bits need the division).
-// Eight IEEE divisions per thread made the kernel instruction bound.
+// x / scale for a value that is rounded to E4M3 next, by multiplication where that gives the same byte: every rounding boundary of E4M3
+// is an fp32 number whose low 19 bits are zero, and only a product within a few units of one can round to the other side. Eight IEEE
+// divisions per thread made the kernel below instruction bound.
 __device__ __forceinline__ float div_for_e4m3(float x, float scale, float inv_scale)
 {
    const float q = __fmul_rn(x, inv_scale);
@@ -610,6 +609,7 @@ __device__ __forceinline__ float div_for_e4m3(float x, float scale, float inv_sc
    return q;
 }
 
+// Eight elements per thread and step: 16- or 32-byte loads, one 8-byte store.
 template <typename In>
 __global__ void quantize_e4m3_vec8_kernel(const In *__restrict__ X, uint8_t *__restrict__ Y, size_t n8, float scale_in,
                                           const float *__restrict__ scale_dev)
