@@ -93,6 +93,7 @@ uint32_t *device_status_word(cudaStream_t stream)
 constexpr int kStagingSlots = 8;
 constexpr size_t kStagingSlot = size_t(2) << 20;
 constexpr size_t kStagingBytes = kStagingSlots * kStagingSlot;
+constexpr size_t kPastCaches = size_t(32) << 20; // a result from which on the host's caches hold no useful part of it
 
 struct sofie_cuda_ctx {
    int device = 0;
@@ -592,7 +593,7 @@ int sofie_cuda_selftest_host_copy(void *dst, const void *src, size_t bytes, size
    HostPool pool(threads - 1);
    for (int r = 0; r < repeats; r++)
       for (size_t done = 0; done < bytes; done += chunk)
-         pool.copy(static_cast<char *>(dst) + done, static_cast<const char *>(src) + done, bytes - done < chunk ? bytes - done : chunk);
+         pool.copy(static_cast<char *>(dst) + done, static_cast<const char *>(src) + done, bytes - done < chunk ? bytes - done : chunk, r % 2 != 0);
    return SOFIE_CUDA_OK;
 }
 
@@ -858,7 +859,7 @@ int sofie_cuda_ctx_result_end(sofie_cuda_ctx *ctx, void **host)
       if (l.parts > 1)
          for (int i = 0; i < l.parts; i++) { // each part as soon as it has landed, under the copies of the later ones
             SOFIE_CUDA_TRY(cudaEventSynchronize(ctx->landed_event[i]));
-            ctx->host_pool->copy(l.out + l.offset[i], l.land + l.offset[i], l.count[i]);
+            ctx->host_pool->copy(l.out + l.offset[i], l.land + l.offset[i], l.count[i], l.bytes >= kPastCaches);
          }
    }
    SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
@@ -869,7 +870,7 @@ int sofie_cuda_ctx_result_end(sofie_cuda_ctx *ctx, void **host)
    for (auto &slot : ctx->slots) copying = copying || (slot.busy && slot.stream == ctx->copy_stream);
    if (copying) SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->copy_stream));
    slots_free(ctx);
-   if (carry && l.parts == 1) ctx->host_pool->copy(l.out + l.offset[0], l.land + l.offset[0], l.count[0]);
+   if (carry && l.parts == 1) ctx->host_pool->copy(l.out + l.offset[0], l.land + l.offset[0], l.count[0], l.bytes >= kPastCaches);
    release_pool(ctx);
    if (l.mapped && l.out) std::memcpy(l.out, l.mapped, l.bytes);
    *host = l.out ? l.out : (l.mapped ? const_cast<char *>(l.mapped) : l.land);

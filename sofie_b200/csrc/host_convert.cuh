@@ -8,6 +8,9 @@
 #include <cstddef>
 #include <cstdint>
 #include <cstring>
+#if defined(__x86_64__)
+#include <immintrin.h>
+#endif
 
 namespace sofie {
 
@@ -63,6 +66,33 @@ __attribute__((always_inline)) inline void host_quantize_e4m3_loop(uint8_t *__re
       const uint32_t code = (a < 0.015625f ? small : normal) | sign;
       y[i] = (uint8_t)(v == v ? code : 0x7Fu);
    }
+}
+
+// A copy past the caches, for results larger than they are: the lines of the destination are not fetched first. FP8 chain on 8192 rows
+// (134 MB of results) 5.1 -> 4.35 ms per call on hosts whose memory gives about 85 GB/s.
+#if defined(__x86_64__)
+__attribute__((target("avx"), noinline)) inline void host_stream_avx(char *dst, const char *src, size_t bytes)
+{
+   size_t head = (64 - (reinterpret_cast<uintptr_t>(dst) & 63)) & 63;
+   if (head > bytes) head = bytes;
+   std::memcpy(dst, src, head);
+   size_t i = head;
+   for (; i + 64 <= bytes; i += 64) {
+      const __m256i a = _mm256_loadu_si256(reinterpret_cast<const __m256i *>(src + i)), b = _mm256_loadu_si256(reinterpret_cast<const __m256i *>(src + i + 32));
+      _mm256_stream_si256(reinterpret_cast<__m256i *>(dst + i), a);
+      _mm256_stream_si256(reinterpret_cast<__m256i *>(dst + i + 32), b);
+   }
+   std::memcpy(dst + i, src + i, bytes - i);
+   _mm_sfence(); // before another thread is told that the piece is done
+}
+#endif
+inline void host_stream_copy(void *dst, const void *src, size_t bytes)
+{
+#if defined(__x86_64__)
+   static const bool avx = __builtin_cpu_supports("avx");
+   if (avx) return host_stream_avx(static_cast<char *>(dst), static_cast<const char *>(src), bytes);
+#endif
+   std::memcpy(dst, src, bytes);
 }
 
 #if defined(__x86_64__)

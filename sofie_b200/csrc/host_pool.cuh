@@ -11,6 +11,8 @@
 #include <thread>
 #include <vector>
 
+#include "host_convert.cuh"
+
 namespace sofie {
 
 // A job is cut into numbered pieces that the caller and the helpers claim one after the other, so a helper that is still
@@ -80,13 +82,14 @@ public:
    size_t threads() const { return threads_.size() + 1; }
 
    // A copy below kAloneBytes is the caller's alone: two threads' hand-over costs as much as it saves.
-   void copy(void *dst, const void *src, size_t bytes)
+   // past_caches: the destination is part of something larger than the host's caches.
+   void copy(void *dst, const void *src, size_t bytes, bool past_caches = false)
    {
       if (threads_.empty() || bytes < kAloneBytes) {
          std::memcpy(dst, src, bytes);
          return;
       }
-      CopyJob job{static_cast<char *>(dst), static_cast<const char *>(src), bytes, kPieceBytes};
+      CopyJob job{static_cast<char *>(dst), static_cast<const char *>(src), bytes, kPieceBytes, past_caches};
       // enough pieces that every thread gets several, each still long enough for the prefetchers
       while (job.piece > size_t(32) << 10 && bytes / job.piece < 3 * (threads_.size() + 1)) job.piece >>= 1;
       run(copy_piece, &job, (bytes + job.piece - 1) / job.piece);
@@ -100,12 +103,14 @@ private:
       char *dst;
       const char *src;
       size_t bytes, piece;
+      bool past_caches;
    };
    static void copy_piece(void *arg, size_t i)
    {
       const CopyJob &j = *static_cast<CopyJob *>(arg);
-      const size_t off = i * j.piece;
-      std::memcpy(j.dst + off, j.src + off, j.bytes - off < j.piece ? j.bytes - off : j.piece);
+      const size_t off = i * j.piece, n = j.bytes - off < j.piece ? j.bytes - off : j.piece;
+      if (j.past_caches) host_stream_copy(j.dst + off, j.src + off, n);
+      else std::memcpy(j.dst + off, j.src + off, n);
    }
    static void relax()
    {

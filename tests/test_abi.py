@@ -217,3 +217,14 @@ def test_helper_threads_that_cannot_be_started_are_done_without(tmp_path):
         "print('ok')\n")
     r = subprocess.run([sys.executable, "-c", script, str(ROOT)], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip().endswith("ok"), (r.returncode, r.stdout[-2000:])
+
+
+@pytest.mark.parametrize("nbytes,dst_at,src_at,threads", [(1 << 20, 0, 0, 4), ((1 << 20) + 1, 1, 0, 3), ((5 << 20) - 63, 63, 17, 4), (98304, 16, 3, 2), (300001, 40, 40, 6)])
+def test_host_copy_past_the_caches(nbytes, dst_at, src_at, threads):
+    """Large results are carried with stores past the caches: any size and any alignment of either side, no byte beyond the end."""
+    import numpy as np
+    src = np.random.default_rng(nbytes).integers(0, 256, nbytes + 64, dtype=np.uint8)
+    dst = np.full(nbytes + 128, 7, np.uint8)
+    capi.call("sofie_cuda_selftest_host_copy", dst.ctypes.data + dst_at, src.ctypes.data + src_at, nbytes, 1 << 22, threads, 2)
+    assert np.array_equal(dst[dst_at:dst_at + nbytes], src[src_at:src_at + nbytes])
+    assert (dst[:dst_at] == 7).all() and (dst[dst_at + nbytes:] == 7).all()
