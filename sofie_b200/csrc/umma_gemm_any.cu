@@ -4,8 +4,8 @@
 // bits), and the six products of parts that reach into 24 bits are summed by the tensor core, the leading ones apart from the others
 // (what is dropped is below 2^-25 of a product). The tensor core's sums truncate, so they are added to fp32 registers every few stages:
 // every 96 elements of K below K = 256, where a chain of FMAs has made few roundings too, every 128 up to K = 1023, every 256 from there.
-// Error against float64 over that of the chain of FMAs, N(0,1) operands: 0.57 at K = 8, 0.4 to 0.6 at K = 128, 0.2 to 0.4 at K = 800,
-// below 0.3 beyond; the same with operands of one sign: 0.66, 0.9, 0.4, 0.3. (Two TF32 parts, 22 bits, and sums of 256, N(0,1): 1.7, 1.7, 1.5, 0.6 to 0.9.)
+// Error against float64 over that of the chain of FMAs, N(0,1) operands: at most 0.57 below K = 32, 0.62 below 96, 0.55 below 256, 0.44 below
+// 1024, 0.39 beyond; operands of one sign: 0.68, 0.95, 0.84, 0.72, 0.71. (Two TF32 parts, 22 bits, and sums of 256, N(0,1): 1.7 up to K = 256.)
 // Infinities, NaNs and the ends of fp32's range give what the chain gives (any_doubtful below).
 //   * sixteen worker warps read the operands themselves, split them in registers and write the parts where the MMA's swizzled K-major
 //     descriptors expect them. A unit of work is eight consecutive K of one row: two 16-byte loads, eight scalar loads (rows that are
