@@ -26,6 +26,8 @@ int launch_gemm_e4m3_umma(cudaStream_t, const sofie_fp8_gemm_desc &, const uint8
                           uint16_t *, uint8_t *, float *Yf32, const float *a_scale_dev = nullptr);
 int launch_conv2d_f32_simt(cudaStream_t, const ConvGeom &, const float *, const float *, const float *, float *);
 int launch_conv2d_f32_umma(cudaStream_t, const ConvGeom &, const float *, const float *, const float *, float *);
+// half-precision parts, 16 or 32 input channels (umma_conv_half.cu): -1 when the shape is not its own
+int launch_conv2d_f32_half(cudaStream_t, const ConvGeom &, const float *, const float *, const float *, float *);
 int launch_qconv2d_simt(cudaStream_t, const ConvGeom &, const uint8_t *, const int8_t *, const float *, const int32_t *,
                         int x_zp, int y_zp, uint8_t *);
 int launch_qconv2d_umma(cudaStream_t, const ConvGeom &, const uint8_t *, const int8_t *, const float *, const int32_t *,

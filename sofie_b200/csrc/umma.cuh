@@ -153,7 +153,7 @@ __device__ __forceinline__ void tc_commit(uint64_t *bar)
                 : "memory");
 }
 
-enum Kind { kTF32 = 0, kI8 = 1, kF8 = 2, kBF16 = 3 };
+enum Kind { kTF32 = 0, kI8 = 1, kF8 = 2, kBF16 = 3, kF16 = 4 };
 
 template <int KIND>
 __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
@@ -164,7 +164,7 @@ __device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a_desc, uint64_
                    "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
                    "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
                    : "memory");
-   } else if constexpr (KIND == kBF16) { // both operands
+   } else if constexpr (KIND == kBF16 || KIND == kF16) { // both operands of the one type
       asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
                    "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
@@ -293,6 +293,30 @@ __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&r)[CH])
    if constexpr (CH == 32) tmem_ld_32x32(taddr, r);
    else tmem_ld_32x16(taddr, r);
 }
+// CH columns of the 32 lanes in the 16x256b shape: thread t gets, of every eight columns, 2 (t % 4) and the next one, of lane t / 4 in the
+// first two of four registers and of lane t / 4 + 8 in the others; lanes 0..15 in the first CH / 2 registers, lanes 16..31 in the rest.
+template <int CH>
+__device__ __forceinline__ void tmem_ld_16x256(uint32_t taddr, uint32_t (&r)[CH])
+{
+   static_assert(CH == 16 || CH == 32, "chunk of 16 or 32 columns");
+#pragma unroll
+   for (int half = 0; half < 2; half++) {
+      const uint32_t addr = taddr + ((uint32_t)(16 * half) << 16);
+      uint32_t *d = r + half * (CH / 2);
+      if constexpr (CH == 16)
+         asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7])
+                      : "r"(addr)
+                      : "memory");
+      else
+         asm volatile("tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+                      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                      : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]), "=r"(d[4]), "=r"(d[5]), "=r"(d[6]), "=r"(d[7]), "=r"(d[8]),
+                        "=r"(d[9]), "=r"(d[10]), "=r"(d[11]), "=r"(d[12]), "=r"(d[13]), "=r"(d[14]), "=r"(d[15])
+                      : "r"(addr)
+                      : "memory");
+   }
+}
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // ---- descriptors -------------------------------------------------------------------------------
@@ -351,10 +375,45 @@ template <int KIND>
 __host__ __device__ constexpr uint32_t make_idesc(int M, int N)
 {
    uint32_t c_fmt = (KIND == kI8) ? 2u : 1u;
-   uint32_t a_fmt = (KIND == kTF32) ? 2u : (KIND == kBF16 ? 1u : 0u);                     // tf32 | bf16 | uint8 | e4m3
-   uint32_t b_fmt = (KIND == kTF32) ? 2u : ((KIND == kI8 || KIND == kBF16) ? 1u : 0u);    // tf32 | bf16 | int8  | e4m3
+   uint32_t a_fmt = (KIND == kTF32) ? 2u : (KIND == kBF16 ? 1u : 0u);                     // tf32 | bf16 | uint8, f16, e4m3
+   uint32_t b_fmt = (KIND == kTF32) ? 2u : ((KIND == kI8 || KIND == kBF16) ? 1u : 0u);    // tf32 | bf16 | int8  | f16, e4m3
    return (c_fmt << 4) | (a_fmt << 7) | (b_fmt << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+
+// ---- tile order of the convolutions -------------------------------------------------------------
+// Walks the tiles start, start + step, ... of an (image groups x tile rows x tile columns) grid with
+// adds and compares only: the roles call it once per tile on their critical path.
+struct TileWalker {
+   int n, th, tw;    // current tile: image group, tile row, tile column
+   int dn, dth, dtw; // the stride in the same digits
+   int tilesH, tilesW;
+   __device__ __forceinline__ void init(int start, int step, int tiles_h, int tiles_w)
+   {
+      tilesH = tiles_h;
+      tilesW = tiles_w;
+      const int per_image = tiles_h * tiles_w;
+      n = start / per_image;
+      th = (start % per_image) / tiles_w;
+      tw = start % tiles_w;
+      dn = step / per_image;
+      dth = (step % per_image) / tiles_w;
+      dtw = step % tiles_w;
+   }
+   __device__ __forceinline__ void next()
+   {
+      tw += dtw;
+      if (tw >= tilesW) {
+         tw -= tilesW;
+         th++;
+      }
+      th += dth;
+      if (th >= tilesH) {
+         th -= tilesH;
+         n++;
+      }
+      n += dn;
+   }
+};
 
 // ---- host: tensor-map encoding through the driver entry point (no link-time libcuda) ----------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,

@@ -47,40 +47,6 @@ constexpr int kConvIssuerB = 2 + kConvEpilogueWarpsI8;           // int8: warp o
 constexpr int kConvThreadsI8 = (3 + kConvEpilogueWarpsI8) * 32;
 constexpr int kConvThreadsTF32 = (2 + kConvEpilogueWarps + kConvConverterWarps) * 32;
 
-// Walks the tiles start, start + step, ... of an (image groups x tile rows x tile columns) grid with
-// adds and compares only: the roles call it once per tile on their critical path.
-struct TileWalker {
-   int n, th, tw;    // current tile: image group, tile row, tile column
-   int dn, dth, dtw; // the stride in the same digits
-   int tilesH, tilesW;
-   __device__ __forceinline__ void init(int start, int step, int tiles_h, int tiles_w)
-   {
-      tilesH = tiles_h;
-      tilesW = tiles_w;
-      const int per_image = tiles_h * tiles_w;
-      n = start / per_image;
-      th = (start % per_image) / tiles_w;
-      tw = start % tiles_w;
-      dn = step / per_image;
-      dth = (step % per_image) / tiles_w;
-      dtw = step % tiles_w;
-   }
-   __device__ __forceinline__ void next()
-   {
-      tw += dtw;
-      if (tw >= tilesW) {
-         tw -= tilesW;
-         th++;
-      }
-      th += dth;
-      if (th >= tilesH) {
-         th -= tilesH;
-         n++;
-      }
-      n += dn;
-   }
-};
-
 // The part of the epilogue one warp does for one finished tile: read its 32 TMEM lanes (pixels) for
 // its share of the output channels, add the NACC partial accumulators, apply bias / Relu or the
 // requantisation, reduce 2x2 windows by shuffles when pooling is fused, and store NHWC.
@@ -1011,6 +977,10 @@ static int launch_conv(cudaStream_t s, const ConvGeom &g, const void *X, const v
       return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "TMA needs 16-byte aligned tensors");
    const int BN = g.Cout <= 32 ? 32 : (g.Cout <= 64 ? 64 : 128);
    if (conv_variant() != 1) {
+      if constexpr (KIND == kTF32) {
+         const int hrc = launch_conv2d_f32_half(s, g, static_cast<const float *>(X), static_cast<const float *>(Wp), ep.bias, ep.Yf);
+         if (hrc >= 0) return hrc;
+      }
       const int prc = try_launch_conv_patch<KIND>(s, g, X, Wp, ep, BN);
       if (prc >= 0) return prc;
    }

@@ -201,6 +201,51 @@ def test_conv3x3_f32_tcgen05(case):
     assert rel_err(y.cpu().numpy().transpose(0, 3, 1, 2), ref) <= 1e-5
 
 
+# fp32 convolutions in half-precision parts: 16 and 32 channels, every width class of the output, odd tile counts, ragged channels
+# (values that the parts hold, values that send tiles or all of them to the FMA chains, infinities and NaN)
+@pytest.mark.parametrize("values", ["normal", "one sign", "image scales", "pixel scales", "tap scales", "specials"])
+@pytest.mark.parametrize("N,C,H,W,Cout,relu,pool", [(3, 16, 16, 8, 20, 0, 0), (2, 16, 48, 24, 64, 1, 2), (150, 32, 16, 16, 64, 0, 2), (1, 32, 16, 40, 33, 1, 2),
+                                                    (5, 32, 32, 16, 30, 0, 0), (3, 16, 32, 32, 100, 0, 2), (2, 16, 16, 16, 128, 1, 0), (1, 16, 16, 8, 1, 0, 2)])
+def test_conv3x3_f32_in_half_precision_parts(N, C, H, W, Cout, relu, pool, values):
+    rng = np.random.default_rng(N + C + H + W + Cout)
+    x, w, b = rng.standard_normal((N, C, H, W)), rng.standard_normal((Cout, C, 3, 3)), rng.standard_normal(Cout)
+    if values == "one sign":
+        x, w = np.abs(x), np.abs(w)
+    if values == "image scales":
+        x *= 2.0 ** rng.integers(-40, 40, (N, 1, 1, 1))
+    if values == "pixel scales":
+        x *= 2.0 ** rng.integers(-30, 30, (N, 1, H, W))
+    if values == "tap scales":
+        w *= 2.0 ** rng.integers(-30, 30, (Cout, 1, 3, 3))
+    if values == "specials":
+        for v in (np.inf, -np.inf, np.nan, 3e38, 1e-39):
+            x[rng.integers(N), rng.integers(C), rng.integers(H), rng.integers(W)] = v
+    x, w, b = (a.astype(np.float32) for a in (x, w, b))
+    y = ops.conv2d_f32(dev(x.transpose(0, 2, 3, 1)), ops.conv2d_pack_f32(dev(w)), dev(b), shape=x.shape, pad=(1, 1), relu=bool(relu), pool=pool,
+                       x_layout=capi.LAYOUT_NHWC, y_layout=capi.LAYOUT_NHWC, w_packed=True, kernel=(3, 3))
+    assert ops.last_engine() == capi.ENGINE_TCGEN05
+    y = y.cpu().double().view(N, H // max(pool, 1), W // max(pool, 1), Cout).permute(0, 3, 1, 2)
+    xd, wd, bd = (torch.from_numpy(a).double() for a in (x, w, b))
+    conv = torch.nn.functional.conv2d
+    ref = conv(xd, wd, bd, padding=1)
+    ref = ref.float().double()      # sums beyond fp32's range are infinite
+    # a product of the parts is off by 2^-22 of the largest channel of its pixel times the weight, every MMA's sum by one truncation
+    size = conv(xd.abs().nan_to_num(0, 0).amax(1, keepdim=True).expand_as(xd), wd.abs(), bd.abs(), padding=1) if values == "pixel scales" else \
+        conv(xd.abs().nan_to_num(0, 0), wd.abs(), bd.abs(), padding=1)
+    if relu:
+        ref = torch.where(ref > 0, ref, 0.0)
+    if pool:
+        # a NaN is passed over, as a comparison with it is false
+        ref = torch.where(ref.isnan(), -torch.inf, ref)
+        ref, size = torch.nn.functional.max_pool2d(ref, 2), torch.nn.functional.max_pool2d(size, 2)
+    finite = ref.isfinite()
+    steps = 2 * 9 * C // 16 + 4
+    assert ((y - ref).abs()[finite] <= steps * 2.0 ** -23 * size[finite]).all()
+    if pool:    # windows of nothing but NaNs
+        finite |= y.isnan()
+    assert torch.equal(y[~finite].float().nan_to_num(2.0, 1.0, -1.0), ref[~finite].float().nan_to_num(2.0, 1.0, -1.0))
+
+
 @pytest.mark.parametrize("case", [(3, 32, 32, 32, 64, 1, 2), (7, 64, 16, 16, 64, 1, 2), (9, 64, 8, 8, 128, 1, 2), (2, 32, 16, 16, 40, 0, 0),
                                   (130, 32, 32, 32, 64, 1, 2), (3, 128, 16, 16, 128, 1, 2), (2, 256, 16, 16, 32, 0, 0),
                                   (2, 128, 32, 16, 64, 1, 0), (5, 32, 16, 16, 24, 1, 2),
