@@ -403,24 +403,20 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
    if (warp == 0) {
       // ---------------- TMA producer ----------------
-      // lane 0 waits for the free slot and posts the byte count; lanes 0 and 1 issue the A and the B
-      // copy in parallel (issuing a tensor copy costs the issuing thread a few hundred cycles)
+      // One thread does all of it: two lanes that issue the two copies, with the hand-over of the wait between them, made a stage 2 to 6 %
+      // longer (4000 x 4096 x 4096 E4M3 56.3 -> 53.0 us)
       griddep_wait(); // A is the previous kernel's output
       int g = 0, s = 0;
       uint32_t ph = 0;
-      bool ok = true;
+      bool ok = lane == 0;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
          const int m0 = (tile / tiles_n) * kBM, n0 = (tile % tiles_n) * BN;
          for (int kb = 0; kb < num_kb; kb++, g++, ring_next(s, ph, S)) {
-            if (lane == 0) {
-               ok = SOFIE_PROF_WAIT(mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g));
-               if (ok) mbar_expect_tx(&full_bar[s], L::kATile + L::kBTile);
-            }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            ok = SOFIE_PROF_WAIT(mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g));
             if (!ok) break;
-            if (lane == 0) tma_load_2d(a_hi(s), &tmA, kb * KE, m0, &full_bar[s]);
-            else if (lane == 1) tma_load_2d(b_hi(s), &tmB, kb * KE, n0, &full_bar[s]);
-            __syncwarp();
+            mbar_expect_tx(&full_bar[s], L::kATile + L::kBTile);
+            tma_load_2d(a_hi(s), &tmA, kb * KE, m0, &full_bar[s]);
+            tma_load_2d(b_hi(s), &tmB, kb * KE, n0, &full_bar[s]);
          }
       }
    } else if (warp == 1) {
@@ -664,21 +660,17 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       griddep_wait(); // A is the previous kernel's output
       int g = 0, s = 0;
       uint32_t ph = 0;
-      bool ok = true;
+      bool ok = lane == 0;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
          const int m0 = (tile / tiles_n) * (2 * kBM) + (int)rank * kBM;
          const int n0 = (tile % tiles_n) * kPairBN + (int)rank * kBM;
          for (int kb = 0; kb < num_kb; kb++, g++, ring_next(s, ph, S)) {
-            if (lane == 0) {
-               ok = SOFIE_PROF_WAIT(mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g));
-               if (ok && rank == 0) mbar_expect_tx(&full_bar[s], 2 * kPairStageBytes);
-            }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            ok = SOFIE_PROF_WAIT(mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g));
             if (!ok) break;
+            if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * kPairStageBytes);
             const uint32_t full_leader = mapa_shared(smem_u32(&full_bar[s]), 0);
-            if (lane == 0) tma_load_2d_pair(a_tile(s), &tmA, kb * kStageK, m0, full_leader);
-            else if (lane == 1) tma_load_2d_pair(b_tile(s), &tmB, kb * kStageK, n0, full_leader);
-            __syncwarp();
+            tma_load_2d_pair(a_tile(s), &tmA, kb * kStageK, m0, full_leader);
+            tma_load_2d_pair(b_tile(s), &tmB, kb * kStageK, n0, full_leader);
          }
       }
    } else if (warp == 1) {
@@ -762,6 +754,178 @@ static int launch_pair(cudaStream_t s, const CUtensorMap &tmA, const CUtensorMap
    return SOFIE_CUDA_OK;
 }
 
+// ================================================================================================
+// Split kernel for the 8-bit kinds: a cluster of CS CTAs shares ONE 128 x BN tile, each taking a part of K, where the tiles alone would
+// leave most SMs idle (a decode-sized batch against wide weights: 128 x 4096 x 4096 has 32 tiles of 128 columns). What bounds such
+// a product is the copy of the operands into the SMs that take part, some 45 bytes a clock each. The ranks' partial tiles are exchanged
+// through distributed shared memory: rank c % CS adds up and finishes the columns 32 c .. 32 c + 31, to which the others send their part as
+// [4 columns][row] pieces of 16 bytes (no two lanes of a quarter warp meet in a bank). The pieces lie in the pipeline's stages, which
+// are free once every rank's MMAs are done: that is what the first of the two cluster barriers is for.
+template <int KIND, int BN>
+__global__ void __launch_bounds__((2 + kGemmEpilogueWarps8) * 32, 1)
+umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmEpilogue ep, int M, int N, int K, int CS,
+                       int S, uint32_t *status)
+{
+   static_assert(KIND == kI8 || KIND == kF8, "8-bit kinds");
+   using L = GemmSmem<KIND, BN>;
+   constexpr int EPI_WARPS = kGemmEpilogueWarps8, CHUNKS = BN / 32;
+   constexpr uint32_t TMEM_COLS = BN;
+   constexpr int kPieceBytes = kBM * 32 * 4;
+   extern __shared__ unsigned char smem_raw[];
+   unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+   __shared__ uint64_t full_bar[kGemmMaxStages], empty_bar[kGemmMaxStages], tmem_full;
+   __shared__ uint32_t tmem_base_holder;
+   __shared__ volatile uint32_t abort_flag;
+   __shared__ __align__(16) float s_cf[18][64];
+
+   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+   griddep_launch_dependents();
+   const int rank = (int)cluster_ctarank(), tile = blockIdx.x / CS;
+   const int tiles_n = (N + BN - 1) / BN;
+   const int m0 = (tile / tiles_n) * kBM, n0 = (tile % tiles_n) * BN;
+   const int num_kb = (K + kStageK - 1) / kStageK, kb0 = num_kb * rank / CS, kb1 = num_kb * (rank + 1) / CS;
+   auto a_tile = [&](int s) { return smem + (size_t)s * L::kStageBytes; };
+   auto b_tile = [&](int s) { return smem + (size_t)s * L::kStageBytes + L::kATile; };
+
+   if (threadIdx.x == 0) {
+      for (int s = 0; s < kGemmMaxStages; s++) {
+         mbar_init(&full_bar[s], 1);
+         mbar_init(&empty_bar[s], 1);
+      }
+      mbar_init(&tmem_full, 1);
+      abort_flag = 0;
+      fence_mbar_init();
+      prefetch_tensormap(&tmA);
+      prefetch_tensormap(&tmB);
+   }
+   if (warp == 1) {
+      tmem_alloc(&tmem_base_holder, TMEM_COLS);
+      tmem_relinquish();
+   }
+   tc_fence_before();
+   __syncthreads();
+   tc_fence_after();
+   const uint32_t tmem_base = tmem_base_holder;
+   const int lane_base = (warp & 3) * 32, group = (warp - 2) >> 2; // epilogue warps: a lane quarter, every fourth chunk of 32 columns
+   const uint32_t t_row = tmem_base + ((uint32_t)lane_base << 16);
+
+   if (warp == 0) {
+      griddep_wait(); // A is the previous kernel's output
+      int s = 0;
+      uint32_t ph = 0;
+      for (int kb = kb0; lane == 0 && kb < kb1; kb++, ring_next(s, ph, S)) {
+         if (!mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, kb)) break;
+         mbar_expect_tx(&full_bar[s], L::kATile + L::kBTile);
+         tma_load_2d(a_tile(s), &tmA, kb * kStageK, m0, &full_bar[s]);
+         tma_load_2d(b_tile(s), &tmB, kb * kStageK, n0, &full_bar[s]);
+      }
+   } else if (warp == 1) {
+      if (lane == 0) {
+         constexpr uint32_t idesc = make_idesc<KIND>(kBM, BN);
+         int s = 0;
+         uint32_t ph = 0;
+         bool ok = true;
+         for (int kb = kb0; kb < kb1; kb++, ring_next(s, ph, S)) {
+            ok = mbar_wait(&full_bar[s], ph, &abort_flag, status, kStatusWaitFull, kb);
+            if (!ok) break;
+            tc_fence_after();
+            const uint64_t da = make_smem_desc(smem_u32(a_tile(s)), kStageK), db = make_smem_desc(smem_u32(b_tile(s)), kStageK);
+#pragma unroll
+            for (int k = 0; k < kStageK / kMmaK; k++) {
+               const uint64_t koff = (uint64_t)(k * (kMmaK >> 4));
+               tc_mma<KIND>(tmem_base, da + koff, db + koff, idesc, (kb == kb0 && k == 0) ? 0u : 1u);
+            }
+            tc_commit(&empty_bar[s]);
+         }
+         if (ok) tc_commit(&tmem_full);
+      }
+   } else {
+      mbar_wait(&tmem_full, 0, &abort_flag, status, kStatusWaitAccum, 0x3000);
+      tc_fence_after();
+   }
+   __syncwarp();
+   cluster_sync_all(); // every rank's MMAs are done: the stages are free to take the others' pieces
+   if (warp >= 2 && !abort_flag) {
+#pragma unroll 1
+      for (int c = group; c < CHUNKS; c += EPI_WARPS / 4) {
+         const int owner = c % CS;
+         if (owner == rank || n0 + 32 * c >= N) continue;
+         uint32_t r[32];
+         tmem_ld_32x32(t_row + (uint32_t)(32 * c), r);
+         tmem_ld_wait();
+         const int from = rank < owner ? rank : rank - 1;
+         const uint32_t dst = mapa_shared(smem_u32(smem + (size_t)((c / CS) * (CS - 1) + from) * kPieceBytes), (uint32_t)owner) + (uint32_t)(lane_base + lane) * 16;
+#pragma unroll
+         for (int j4 = 0; j4 < 8; j4++)
+            asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)(j4 * kBM * 16)), "r"(r[4 * j4]), "r"(r[4 * j4 + 1]),
+                         "r"(r[4 * j4 + 2]), "r"(r[4 * j4 + 3])
+                         : "memory");
+      }
+   }
+   __syncwarp();
+   cluster_sync_all(); // the pieces have arrived
+   if (warp >= 2 && !abort_flag) {
+      const int row = m0 + lane_base + lane;
+#pragma unroll 1
+      for (int own = group, c = rank + group * CS; c < CHUNKS; own += EPI_WARPS / 4, c += (EPI_WARPS / 4) * CS) {
+         if (n0 + 32 * c >= N) break;
+         uint32_t r[32];
+         tmem_ld_32x32(t_row + (uint32_t)(32 * c), r);
+         tmem_ld_wait();
+         for (int from = 0; from < CS - 1; from++) {
+            const uint4 *piece = reinterpret_cast<const uint4 *>(smem + (size_t)(own * (CS - 1) + from) * kPieceBytes) + lane_base + lane;
+#pragma unroll
+            for (int j4 = 0; j4 < 8; j4++) {
+               const uint4 v = piece[j4 * kBM];
+               const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+               for (int t = 0; t < 4; t++) {
+                  if constexpr (KIND == kI8) r[4 * j4 + t] += x[t];
+                  else r[4 * j4 + t] = __float_as_uint(__uint_as_float(r[4 * j4 + t]) + __uint_as_float(x[t]));
+               }
+            }
+         }
+         store_row_chunk<KIND>(ep, r, row, row < M, n0 + 32 * c, N, s_cf[warp], lane);
+      }
+   }
+   tc_fence_before();
+   __syncthreads();
+   if (warp == 1) {
+      __syncwarp();
+      tc_fence_after();
+      tmem_dealloc(tmem_base, TMEM_COLS);
+   }
+}
+
+template <int KIND, int BN>
+static int launch_split(cudaStream_t s, const CUtensorMap &tmA, const CUtensorMap &tmB, const GemmEpilogue &ep, int M, int N, int K, int CS)
+{
+   using L = GemmSmem<KIND, BN>;
+   int stages = (200 * 1024) / L::kStageBytes;
+   if (stages > kGemmMaxStages) stages = kGemmMaxStages;
+   auto kern = umma_gemm_split_kernel<KIND, BN>;
+   const int smem = stages * L::kStageBytes + 1024;
+   SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), smem));
+   uint32_t *status = device_status_word(s);
+   if (!status) return fail(SOFIE_CUDA_ERR_CUDA, "cannot allocate the device status word");
+   cudaLaunchConfig_t cfg = {};
+   cfg.gridDim = dim3(CS * ceil_div(N, BN) * ceil_div(M, kBM));
+   cfg.blockDim = dim3((2 + kGemmEpilogueWarps8) * 32);
+   cfg.dynamicSmemBytes = smem;
+   cfg.stream = s;
+   cudaLaunchAttribute attr[2];
+   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+   attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+   attr[1].id = cudaLaunchAttributeClusterDimension;
+   attr[1].val.clusterDim.x = (unsigned)CS;
+   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+   cfg.attrs = attr;
+   cfg.numAttrs = 2;
+   SOFIE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, ep, M, N, K, CS, stages, status));
+   set_last_engine(SOFIE_ENGINE_TCGEN05);
+   return SOFIE_CUDA_OK;
+}
+
 // SOFIE_CUDA_GEMM_PAIR=0 keeps every shape on the single-CTA kernel (used to compare the two).
 static bool pair_enabled()
 {
@@ -789,6 +953,29 @@ static int launch_one(cudaStream_t s, const CUtensorMap &tmA, const CUtensorMap 
    return SOFIE_CUDA_OK;
 }
 
+// Tile width and CTAs that share a tile's K for the 8-bit kinds, by the time they take in ns: a stage (128 of K), a round of tiles, the fill
+// and drain of one tile, the exchange within a cluster (fitted to 43 products of 1 to 65536 rows, each at every width and cluster size).
+// A stage costs almost the same at every width, so one round of wide tiles beats two of narrow ones (690 x 4096 x 4096 27.7 -> 18.7 us),
+// and where even narrow tiles leave SMs idle K is shared (128 x 4096 x 4096 15.4 -> 11.5 us, 300 x 4096 x 4096 25.3 -> 15.1,
+// 512 x 256 x 2048 11.0 -> 9.0; 1000 x 1024 x 512 is left at 64 columns, 5.9 us against 7.7 shared by two).
+// Clusters of two / four found room for 148 / 140 CTAs at a time; shared tiles get one round.
+static void choose_tile(int M, int N, int K, int &BN, int &split)
+{
+   static const int widths[3] = {64, 128, 256}, stage[3] = {295, 305, 340}, tile[3] = {700, 1300, 2600};
+   const long long tm = ceil_div(M, kBM), kb = ceil_div(K, kStageK);
+   long long best = -1;
+   for (int w = 0; w < 3; w++) {
+      if (w > 0 && widths[w] / 2 >= N) break; // more than half of the tile would be padding
+      const long long tiles = tm * ceil_div(N, widths[w]), chunks = widths[w] / 32;
+      for (int q = 1; q <= 4; q *= 2) {
+         if (q > 1 && (kb < 2 * q || tiles * q > (q == 2 ? kNumSMs : 140))) break;
+         const long long rounds = (tiles * q + kNumSMs - 1) / kNumSMs;
+         const long long time = rounds * (ceil_div((int)kb, q) * stage[w] + 700) + tile[w] / q + (q > 1 ? 1700 + 500 * (chunks - chunks / q) : 0);
+         if (best < 0 || time < best) best = time, BN = widths[w], split = q;
+      }
+   }
+}
+
 template <int KIND>
 static int launch_umma_gemm(cudaStream_t s, const void *A, const void *B, const GemmEpilogue &ep, int M, int N, int K)
 {
@@ -797,9 +984,8 @@ static int launch_umma_gemm(cudaStream_t s, const void *A, const void *B, const 
    if (((size_t)K * ES) % 16 != 0 || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
       return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "TMA needs 16-byte aligned rows (K*%d %% 16 == 0) and bases", ES);
    // fp32 keeps the tile's running sum in registers (promotion), which bounds its width at 64 columns
-   int BN = N <= 32 ? 32 : ((N <= 64 || KIND == kTF32) ? 64 : (N <= 128 ? 128 : 256));
-   // wide tiles are the efficient ones, but not when they leave most SMs without a tile
-   while (BN > 64 && (long long)ceil_div(M, kBM) * ceil_div(N, BN) < (kNumSMs * 4) / 5) BN /= 2;
+   int BN = N <= 32 ? 32 : 64, split = 1;
+   if constexpr (KIND != kTF32) if (N > 32) choose_tile(M, N, K, BN, split);
    CUtensorMap tmA, tmB;
    const CUtensorMapDataType dt = (KIND == kTF32) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
    uint64_t dimsA[2] = {(uint64_t)K, (uint64_t)M}, dimsB[2] = {(uint64_t)K, (uint64_t)N};
@@ -824,6 +1010,11 @@ static int launch_umma_gemm(cudaStream_t s, const void *A, const void *B, const 
       if (BN == 32) return launch_one<KIND, 32>(s, tmA, tmB, ep, M, N, K);
       return launch_one<KIND, 64>(s, tmA, tmB, ep, M, N, K);
    } else {
+      if (split > 1) {
+         if (BN == 64) return launch_split<KIND, 64>(s, tmA, tmB, ep, M, N, K, split);
+         if (BN == 128) return launch_split<KIND, 128>(s, tmA, tmB, ep, M, N, K, split);
+         return launch_split<KIND, 256>(s, tmA, tmB, ep, M, N, K, split);
+      }
       switch (BN) {
       case 32: return launch_one<KIND, 32>(s, tmA, tmB, ep, M, N, K);
       case 64: return launch_one<KIND, 64>(s, tmA, tmB, ep, M, N, K);

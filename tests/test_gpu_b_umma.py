@@ -95,6 +95,33 @@ def test_qlinear_matmul_tcgen05_bit_exact(M, N, K, relu, zp):
     assert len(np.unique(ref)) > 20
 
 
+# few tiles and a long K: four or two CTAs of a cluster share a tile of 64, 128 or 256 columns; ranks with uneven parts of K (17 and 33
+# stages), with no columns of their own (64 columns, four ranks) and with columns beyond N
+@pytest.mark.parametrize("M,N,K", [(5, 70, 2096), (257, 64, 4096), (130, 300, 4112), (128, 4096, 4096), (300, 4090, 4112)])
+def test_8_bit_products_that_share_k(M, N, K):
+    rng = np.random.default_rng(M + N + K)
+    A, W = rng.integers(0, 256, (M, K)).astype(np.uint8), rng.integers(-127, 128, (N, K)).astype(np.int8)
+    acc = (A.astype(np.float64) @ W.astype(np.float64).T).astype(np.int64)     # exact: below 2^53
+    ws = rng.uniform(0.001, 0.01, N).astype(np.float32)
+    y_scale = 0.02 * np.sqrt(K) * 0.3
+    mult, corr = ops.qlinear_prepare(W, True, 0.02, 3, ws, y_scale, None, "cuda")
+    ref = (acc - 3 * W.sum(1, dtype=np.int64)).astype(np.float32) * mult.cpu().numpy()
+    ref = np.clip(np.rint(ref) + 128, 0, 255).astype(np.uint8)
+    y = ops.qlinear_matmul(dev(A), dev(W), mult, corr, w_is_nk=True, y_zp=128)
+    assert ops.last_engine() == capi.ENGINE_TCGEN05
+    assert np.array_equal(y.cpu().numpy(), ref) and len(np.unique(ref)) > 20
+    Aq = o.quantize_e4m3(rng.standard_normal((M, K)).astype(np.float32), 0.01)
+    Wq = o.quantize_e4m3(rng.standard_normal((N, K)).astype(np.float32), 0.01)
+    bias = rng.standard_normal(N).astype(np.float32)
+    Y, Yq = ops.gemm_e4m3(dev(Aq), dev(Wq), dev(bias), a_scale=0.01, w_scale=0.01, q_scale=0.05)
+    table = torch.arange(256, dtype=torch.uint8).view(torch.float8_e4m3fn).double().numpy()
+    a, w = table[Aq] * 0.01, table[Wq] * 0.01
+    exact, size = a @ w.T + bias, np.abs(a) @ np.abs(w).T + np.abs(bias)
+    # one rounding to bfloat16 of a sum whose tensor-core additions (32 of K each) truncate
+    assert (np.abs(Y.double().cpu().numpy() - exact) <= 2.0 ** -8 * np.abs(exact) + (K / 32 + 8) * 2.0 ** -23 * size).all()
+    assert np.array_equal(Yq.cpu().numpy(), o.quantize_e4m3(Y.float().cpu().numpy(), 0.05))
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 128, 128), (70, 45, 144), (1000, 512, 4096), (256, 4096, 512)])
 def test_gemm_e4m3_tcgen05(M, N, K):
     rng = np.random.default_rng(K + M)
