@@ -39,6 +39,8 @@ int launch_qconv2d_umma_pooled(cudaStream_t, const ConvGeom &, const uint8_t *, 
 int launch_mlp_f32_umma(cudaStream_t, const sofie_mlp_desc *, const float *, const float *const *, const float *const *, float *);
 // first-layer kernels (conv_first.cu): -1 when the shape is not theirs
 int launch_conv2d_f32_first(cudaStream_t, const ConvGeom &, const float *, const float *, const float *, float *);
+// 3x3 of any layout and size on the CUDA cores (conv3x3_direct.cu): -1 when the shape is not its own
+int launch_conv2d_f32_direct3x3(cudaStream_t, const ConvGeom &, const float *, const float *, const float *, float *);
 int launch_qconv2d_first(cudaStream_t, const ConvGeom &, const uint8_t *, const int8_t *, const float *, const int32_t *,
                          int x_zp, int y_zp, uint8_t *);
 // split-K skinny GEMM (splitk_gemm.cu)

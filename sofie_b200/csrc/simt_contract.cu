@@ -219,7 +219,8 @@ int launch_conv_direct(cudaStream_t s, const ConvGeom &g, const TX *X, const TW 
 int launch_conv2d_f32_simt(cudaStream_t s, const ConvGeom &g, const float *X, const float *W, const float *bias,
                            float *Y)
 {
-   const int rc = launch_conv2d_f32_first(s, g, X, W, bias, Y);
+   int rc = launch_conv2d_f32_first(s, g, X, W, bias, Y);
+   if (rc < 0) rc = launch_conv2d_f32_direct3x3(s, g, X, W, bias, Y);
    if (rc >= 0) return rc;
    return launch_conv_direct<float, float, float, float, EpiF32>(s, g, X, W, EpiF32{bias}, 0, Y);
 }

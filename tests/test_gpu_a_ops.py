@@ -137,6 +137,35 @@ CONV_CASES = [
 ]
 
 
+# 3x3 / stride 1 / pad 1 on the CUDA cores: channels around a chunk of four and one group of sixteen outputs, images around the 16 x 16 and 16 x 32
+# tiles (the last one is too small for them), rows of whole words or not, both layouts on either side, fused pooling of odd sizes, a NaN and infinities
+@pytest.mark.parametrize("pool", [0, 2])
+@pytest.mark.parametrize("N,C,H,W,Cout,x_nhwc,y_nhwc", [(3, 8, 16, 16, 16, 0, 0), (2, 16, 17, 33, 17, 0, 1), (400, 5, 8, 9, 3, 0, 0), (2, 6, 31, 64, 40, 0, 0),
+                                                        (2, 128, 16, 20, 8, 0, 1), (3, 12, 20, 18, 24, 1, 1), (1, 7, 6, 12, 16, 1, 0), (1, 9, 5, 60, 5, 0, 0), (2, 7, 3, 5, 9, 0, 0)])
+def test_conv3x3_f32_direct(N, C, H, W, Cout, x_nhwc, y_nhwc, pool):
+    rng = np.random.default_rng(N + C + H + W + Cout)
+    X, Wt, b = (rng.standard_normal(s).astype(np.float32) for s in ((N, C, H, W), (Cout, C, 3, 3), (Cout,)))
+    for relu in (False, True):
+        for special in (False, True):
+            if special:
+                X[0, 0, 0, 0], X[-1, -1, -1, -1], X[0, C // 2, H // 2, W // 2] = np.nan, np.inf, -np.inf
+            ref = o.conv2d_f32(X, Wt, b, pad=(1, 1), relu=relu)
+            if pool:
+                r = ref[:, :, :H // 2 * 2, :W // 2 * 2].reshape(N, Cout, H // 2, 2, W // 2, 2)
+                ref = r[:, :, :, 0, :, 0].copy()
+                for y, x in ((0, 1), (1, 0), (1, 1)):
+                    v = r[:, :, :, y, :, x]
+                    ref = np.where(v > ref, v, ref)
+            y = ops.conv2d_f32(dev(X.transpose(0, 2, 3, 1) if x_nhwc else X), dev(Wt), dev(b), shape=X.shape, pad=(1, 1), relu=relu, pool=pool,
+                               x_layout=x_nhwc, y_layout=y_nhwc, kernel=(3, 3)).cpu().numpy()
+            y = y.reshape((N, *ref.shape[2:], Cout)).transpose(0, 3, 1, 2) if y_nhwc else y.reshape(ref.shape)
+            finite = np.isfinite(ref)
+            assert (np.abs(y[finite] - ref[finite]) <= FP32_TOL * np.abs(ref[finite]).max(initial=0)).all()
+            assert np.array_equal(y[~finite], ref[~finite], equal_nan=True)
+        X = rng.standard_normal(X.shape).astype(np.float32)
+
+
+
 @pytest.mark.parametrize("case", CONV_CASES)
 def test_conv2d_f32_nchw(case):
     N, C, H, W, Cout, k, pad, stride, dil, group = case
