@@ -224,6 +224,20 @@ def test_conv_transpose2d_f32(case):
     assert y.shape == ref.shape and rel_err(y, ref) <= FP32_TOL
 
 
+# direct ConvTranspose: filters in one piece and in several (25 taps, 70 channels), four and eight channels a thread, channel counts off the multiples
+# of 4 and 16, strides with empty residues, and filters too large for shared memory
+@pytest.mark.parametrize("N,C,H,W,Cout,k,stride,pad,dil,out_pad", [(3, 70, 5, 7, 9, (5, 5), (2, 2), (2, 2), (1, 1), (1, 1)), (130, 17, 3, 2, 4, (2, 2), (2, 3), (0, 0), (1, 1), (0, 2)),
+                                                                   (2, 16, 6, 11, 3, (3, 3), (1, 4), (1, 1), (2, 1), (0, 3)), (1, 3, 4, 4, 20, (1, 7), (3, 1), (0, 3), (1, 1), (2, 0)),
+                                                                   (1, 2, 2, 3, 8, (33, 33), (1, 1), (0, 0), (1, 1), (0, 0)), (2, 40, 9, 9, 16, (4, 4), (2, 2), (1, 1), (1, 1), (0, 0))])
+def test_conv_transpose2d_f32_direct(N, C, H, W, Cout, k, stride, pad, dil, out_pad):
+    rng = np.random.default_rng(N + C + H + W + Cout)
+    X, Wt, b = (rng.standard_normal(s).astype(np.float32) for s in ((N, C, H, W), (C, Cout, *k), (Cout,)))
+    ref = o.conv_transpose2d_f32(X, Wt, b, pad=pad, stride=stride, dil=dil, out_pad=out_pad)
+    y = ops.conv_transpose2d_f32(dev(X), dev(Wt), dev(b), pad=pad, stride=stride, dil=dil, out_pad=out_pad).cpu().numpy()
+    assert rel_err(y, ref) <= FP32_TOL
+
+
+
 @pytest.mark.parametrize("case", [
     # N, C, H, W, Cout, k, pad, stride, dil, out_pad, bias, relu
     (4, 32, 16, 16, 16, (4, 4), (1, 1), (2, 2), (1, 1), (0, 0), True, True),       # the usual 2x upsampling layer of a decoder
