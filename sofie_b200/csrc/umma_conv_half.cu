@@ -291,9 +291,11 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
       }
       constexpr int GT = kHalfConvGroupWarps * 32, UNITS = kHalfPatchPixels * UPP, PER = (UNITS + GT - 1) / GT;
       const int t = gw * 32 + lane;
+      // a warp whose wait gave up goes on to the group's barrier, where the four leave together: nobody waits there for one that has left
+      bool ok = true;
       for (int lt = group; blockIdx.x + (long long)lt * gridDim.x < p.num_tiles; lt += kHalfConvGroups) {
          const int s = lt % SLOTS;
-         if (!SOFIE_PROF_WAIT(mbar_wait(&raw_full[s], (uint32_t)(lt / SLOTS) & 1u, &abort_flag, status, kStatusWaitFull, 0x6000 + lt))) break;
+         ok = ok && SOFIE_PROF_WAIT(mbar_wait(&raw_full[s], (uint32_t)(lt / SLOTS) & 1u, &abort_flag, status, kStatusWaitFull, 0x6000 + lt));
          float v[PER][8];
          // 32 bytes a unit: the lanes of a quarter warp read different halves of their units at a time, so that no banks collide
          const float4 *raw = reinterpret_cast<const float4 *>(raws + (size_t)s * RAW);
@@ -325,7 +327,12 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
             mbar_arrive(&raw_empty[s]); // the patch is in registers
             red[gw] = make_uint2(largest, smallest);
          }
-         asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(GT) : "memory");
+         uint32_t all_ok;
+         asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                      : "=r"(all_ok)
+                      : "r"(ok ? 1u : 0u), "r"(1 + group), "n"(GT)
+                      : "memory");
+         if (!all_ok) break;
 #pragma unroll
          for (int i = 0; i < kHalfConvGroupWarps; i++) {
             const uint2 o = red[i];
@@ -334,14 +341,14 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
          }
          float scale, inverse;
          const bool fits = half_scale(largest, smallest + 1, scale, inverse);
-         if (!SOFIE_PROF_WAIT(mbar_wait(&op_empty[s], ((uint32_t)(lt / SLOTS) & 1u) ^ 1u, &abort_flag, status, kStatusWaitEmpty, 0x7000 + lt))) break;
+         ok = SOFIE_PROF_WAIT(mbar_wait(&op_empty[s], ((uint32_t)(lt / SLOTS) & 1u) ^ 1u, &abort_flag, status, kStatusWaitEmpty, 0x7000 + lt));
          // read by the epilogue after the tile's MMAs, which wait for this group's arrivals below
          if (t == 0) s_xinv[lt % kHalfScales] = fits ? inverse : 0.f;
          unsigned char *op = ops + (size_t)s * 2 * PART;
 #pragma unroll
          for (int i = 0; i < PER; i++) {
             const int u = t + i * GT;
-            if (u < UNITS) {
+            if (ok && u < UNITS) {
                uint4 hi, lo;
                half_split(v[i], scale, hi, lo);
                const uint32_t off = half_swizzled<RB>((uint32_t)u * 16);
@@ -351,7 +358,7 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
          }
          fence_proxy_async();
          __syncwarp();
-         if (lane == 0) mbar_arrive(&op_full[s]);
+         if (ok && lane == 0) mbar_arrive(&op_full[s]);
       }
    } else {
       // ---------------- epilogue: warps 2..9, two per lane quarter ----------------
