@@ -7,21 +7,23 @@
 //
 // Half precision has 5 bits of exponent, so the parts are formed of SCALED values: a patch is multiplied by the power of two that brings
 // its largest magnitude into [2^14, 2^15), every output channel's weights by one of their own, and the epilogue multiplies the sums by the
-// inverse powers (exact). A part then ends at 2^-25 after scaling: a value keeps 22 bits down to 2^-17 of its patch's largest, and
-// loses one per power of two from there. A pixel all of whose channels are that small (but not all zero) would be held to fewer bits than
-// TF32 parts hold it to, so the converters look for one: such a tile, and any with an infinity, a NaN or a largest value outside
-// 2^-100 .. 2^100, is computed by the epilogue warps as chains of fp32 FMAs from global memory. The same holds for all tiles when the
-// weights of a channel have such a spread (groups of eight of a tap taken together). In data without wild spreads no tile comes to it.
-// Error against float64 (2-norm), N(0,1) operands: 3.8e-7 at 16 and 6.8e-7 at 32 channels, where TF32 parts gave 7.0e-7 and 1.28e-6 (their trailing
-// part is truncated, these are rounded, and the sums take half as many steps); operands of one sign 7.3e-7 and 1.75e-6 (1.05e-6 and 2.4e-6).
-// 8192 images 16 -> 32 at 32 x 32 with MaxPool 498 -> 326 us, 32 -> 64 at 16 x 16 371 -> 203 us; unpooled 2048 x 16 -> 32 176 -> 150 us. A tile taken
-// as FMA chains costs about ten of the others.
+// product of the inverse powers (exact). A trailing part is multiplied by another 2^11 before it is rounded, so that it lies where its leading part
+// does and not 2^11 below, at the end of half precision's range (the scaled residual of H. Ootomo and R. Yokota, "Recovering single precision accuracy
+// from Tensor Cores while surpassing the FP32 theoretical peak performance", 2022); the products with one trailing factor have sums of their own, which
+// the epilogue multiplies by 2^-11. A value whose scaled magnitude is 2^-14 or more is then held to 2^-22 of itself, as two TF32 parts hold it; a
+// smaller one to 2^-36 after scaling. The converters look for a value as small as that, at EVERY value of the patch and not at the largest of
+// a pixel or a channel: its neighbours may meet weights that are zero. A tile that has one, and any with an infinity or a NaN, is computed
+// by the epilogue warps as chains of fp32 FMAs from global memory; all tiles are when the weights of an output channel span more than that, or when the
+// two scales together leave fp32's range. The largest of a patch may be 2^28 times its smallest, beside zeros, before any of this happens.
+// Error against float64 (2-norm), N(0,1) operands: 2.1e-7 at 16 and 3.7e-7 at 32 channels, where TF32 parts gave 7.0e-7 and 1.28e-6 (their trailing
+// part is truncated, these are rounded, and the sums take half as many steps); operands of one sign 6.1e-7 and 1.4e-6 (1.05e-6 and 2.4e-6).
+// 8192 images 16 -> 32 at 32 x 32 with MaxPool 490 -> 332 us, 32 -> 64 at 16 x 16 367 -> 205 us; unpooled 2048 x 16 -> 32 172 -> 143 us. A tile taken
+// as FMA chains costs about sixty of the others (45 us).
 //
 // A tile is 16 x 8 pixels of one image; one TMA box brings its 18 x 10 patch (zero fill outside the image) as fp32 rows; two groups of four
 // converter warps take the patches in turn, find the largest magnitude, split the values and write both parts as K-major swizzled
 // rows, from which each of the 9 taps is a start address (see the haloed-patch kernel). One MMA multiplies the leading parts of the
-// pixels with [leading | trailing] weights (2 * BN columns), one the trailing parts with the leading weights; the epilogue adds the two
-// halves of the accumulator. A TMEM buffer goes back to the issuers as soon as it has been read, before pooling and stores. Pooled tiles are
+// pixels with [leading | trailing] weights (2 * BN columns), one the trailing parts with the leading weights, into the second BN columns. A TMEM buffer goes back to the issuers as soon as it has been read, before pooling and stores. Pooled tiles are
 // read in the shape that puts a pixel and the one below it in one thread: a third of the shuffles, which wait for the shared-memory
 // pipe the MMAs keep busy (the epilogue set the kernel's time with them: 375 instead of 326 us).
 // Waiting with one lane and a vote, or with test_wait, instead of whole warps on try_wait: 5 to 25 % slower.
@@ -42,7 +44,8 @@ constexpr int kHalfIssuerB = 2 + kHalfEpiWarps + kHalfConvWarps;
 constexpr int kHalfThreads = (kHalfIssuerB + 1) * 32;
 constexpr int kHalfMaxSlots = 4;
 constexpr int kHalfScales = 16;       // ring of tile scales: more than the tiles between a converter and the epilogue (slots + TMEM buffers)
-constexpr uint32_t kHalfSpread = 17;  // a pixel's largest channel may be 2^-17 of the patch's largest (see above)
+constexpr uint32_t kHalfSpread = 28;  // a value may be 2^-28 of the patch's largest (see above)
+constexpr float kHalfTrailing = 2048.f; // trailing parts are held times 2^11
 
 __host__ __device__ constexpr int half_part_bytes(int C) { return (kHalfPatchPixels * 2 * C + 1023) / 1024 * 1024; } // a patch's leading or trailing parts
 __host__ __device__ constexpr int half_raw_bytes(int C) { return kHalfPatchPixels * 4 * C; }
@@ -69,16 +72,20 @@ __device__ __forceinline__ uint32_t half_swizzled(uint32_t off)
    return off ^ ((off >> 3) & (RB == 32 ? 0x10u : 0x30u));
 }
 
-// Eight fp32 values times a power of two as 16 bytes of leading halves and 16 bytes of what those leave, rounded to nearest even.
+// Eight fp32 values times a power of two as 16 bytes of leading halves and 16 bytes of 2^11 times what those leave, rounded to nearest even.
 __device__ __forceinline__ void half_split(const float (&v)[8], float scale, uint4 &hi, uint4 &lo)
 {
    uint32_t h[4], l[4];
+   const uint64_t scale2 = pack_f32x2(scale, scale), minus_one2 = pack_f32x2(-1.f, -1.f), trailing2 = pack_f32x2(kHalfTrailing, kHalfTrailing);
 #pragma unroll
    for (int i = 0; i < 4; i++) {
-      const float a = v[2 * i] * scale, b = v[2 * i + 1] * scale;
+      const uint64_t v2 = fma_f32x2(pack_f32x2(v[2 * i], v[2 * i + 1]), scale2, 0);
+      float a, b;
+      unpack_f32x2(v2, a, b);
       const __half2 p = __floats2half2_rn(a, b);
       const float2 back = __half22float2(p);
-      const __half2 q = __floats2half2_rn(a - back.x, b - back.y);
+      unpack_f32x2(fma_f32x2(fma_f32x2(pack_f32x2(back.x, back.y), minus_one2, v2), trailing2, 0), a, b); // the difference is exact
+      const __half2 q = __floats2half2_rn(a, b);
       h[i] = *reinterpret_cast<const uint32_t *>(&p);
       l[i] = *reinterpret_cast<const uint32_t *>(&q);
    }
@@ -86,25 +93,29 @@ __device__ __forceinline__ void half_split(const float (&v)[8], float scale, uin
    lo = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
-__device__ __forceinline__ uint32_t half_largest(const float (&v)[8])
+// Largest magnitude of eight values, and the smallest of those that are not zero less one, as twice the magnitude's bits (no sign).
+__device__ __forceinline__ void half_extremes(const float (&v)[8], uint32_t &largest, uint32_t &smallest)
 {
-   uint32_t m = 0;
 #pragma unroll
-   for (int i = 0; i < 8; i++) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
-   return m;
+   for (int i = 0; i < 8; i++) {
+      const uint32_t m = __float_as_uint(v[i]) << 1;
+      largest = max(largest, m);
+      smallest = __viaddmin_u32(m, 0xffffffffu, smallest);
+   }
 }
 
-// The scale that brings `largest` (bits of a magnitude) into [2^14, 2^15), and its inverse; false when the values have to be taken as
-// fp32: largest is not finite or beyond the ends of the range, or the smallest of the groups' largest is more than 2^17 below it.
+// The scale that brings the largest magnitude into [2^14, 2^15), or 2^126 where that is less, and its inverse; false when the parts would not hold
+// the values (see the head of this file). Everything fits under 2^126: subnormal values are multiples of 2^-23 then, which two halves hold exactly.
 __device__ __forceinline__ bool half_scale(uint32_t largest, uint32_t smallest, float &scale, float &inverse)
 {
-   const uint32_t e = largest >> 23;
+   const uint32_t e = largest >> 24, e_small = (smallest + 1) >> 24;
    scale = inverse = 1.f;
    if (largest == 0) return true;
-   if (e > 227 || e < 27) return false;
-   scale = __uint_as_float((268u - e) << 23);
-   inverse = __uint_as_float((e - 14u) << 23);
-   return e - (smallest >> 23) <= kHalfSpread;
+   if (e == 255) return false;
+   const uint32_t lift = e > 15 ? e : 15;
+   scale = __uint_as_float((268u - lift) << 23);
+   inverse = __uint_as_float((lift - 14u) << 23);
+   return e <= 15 || (e_small > 0 && e - e_small <= kHalfSpread);
 }
 
 // Output pixel (h, w) of image n as chains of fp32 FMAs, without bias: J channels from c on, consecutive ones or (PAIRS) two of every eight.
@@ -236,7 +247,7 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
                for (int k = 0; k < KSTEPS; k++) {
                   const uint32_t a = (uint32_t)(((tap / 3) * kHalfPatchW + tap % 3) * RB + k * 32), b = (uint32_t)(tap * W_ITEM + k * 32);
                   tc_mma<kF16>(d, adesc(a), bdesc(b), idesc_wide, (tap | k) ? 1u : 0u); // leading x [leading | trailing]
-                  tc_mma<kF16>(d, adesc(a + PART), bdesc(b), idesc, 1u);                // trailing x leading
+                  tc_mma<kF16>(d + BN, adesc(a + PART), bdesc(b), idesc, 1u);           // trailing x leading
                }
             }
             tc_commit(&op_empty[s]);
@@ -257,14 +268,12 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
             if (row >= p.Cout) a = b = make_float4(0.f, 0.f, 0.f, 0.f);
             v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
          };
-         uint32_t largest = 0, smallest = 0xffffffffu; // smallest: of the units that are not all zero, less one
+         uint32_t largest = 0, smallest = 0xffffffffu;
 #pragma unroll 4
          for (int u = sub; u < UNITS; u += TPR) {
             float v[8];
             load(u, v);
-            const uint32_t m = half_largest(v);
-            largest = max(largest, m);
-            smallest = min(smallest, m - 1);
+            half_extremes(v, largest, smallest);
          }
 #pragma unroll
          for (int o = 1; o < TPR; o <<= 1) {
@@ -272,7 +281,7 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
             smallest = min(smallest, __shfl_xor_sync(0xffffffffu, smallest, o));
          }
          float scale, inverse;
-         if (!half_scale(largest, smallest + 1, scale, inverse)) w_spread = 1;
+         if (!half_scale(largest, smallest, scale, inverse)) w_spread = 1;
          if (sub == 0) s_winv[row] = inverse;
 #pragma unroll 4
          for (int u = sub; u < UNITS; u += TPR) {
@@ -311,15 +320,9 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
             v[i][0] = swap ? b.x : a.x; v[i][1] = swap ? b.y : a.y; v[i][2] = swap ? b.z : a.z; v[i][3] = swap ? b.w : a.w;
             v[i][4] = swap ? a.x : b.x; v[i][5] = swap ? a.y : b.y; v[i][6] = swap ? a.z : b.z; v[i][7] = swap ? a.w : b.w;
          }
-         uint32_t largest = 0, smallest = 0xffffffffu; // smallest: of the pixels that are not all zero, less one
+         uint32_t largest = 0, smallest = 0xffffffffu;
 #pragma unroll
-         for (int i = 0; i < PER; i++) {
-            uint32_t m = half_largest(v[i]);
-            largest = max(largest, m);
-#pragma unroll
-            for (int o = 1; o < UPP; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-            smallest = min(smallest, m - 1);
-         }
+         for (int i = 0; i < PER; i++) half_extremes(v[i], largest, smallest);
          largest = __reduce_max_sync(0xffffffffu, largest);
          smallest = __reduce_min_sync(0xffffffffu, smallest);
          uint2 *red = s_red[group][(lt >> 1) & 1];
@@ -340,7 +343,7 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
             smallest = min(smallest, o.y);
          }
          float scale, inverse;
-         const bool fits = half_scale(largest, smallest + 1, scale, inverse);
+         const bool fits = half_scale(largest, smallest, scale, inverse);
          ok = SOFIE_PROF_WAIT(mbar_wait(&op_empty[s], ((uint32_t)(lt / SLOTS) & 1u) ^ 1u, &abort_flag, status, kStatusWaitEmpty, 0x7000 + lt));
          // read by the epilogue after the tile's MMAs, which wait for this group's arrivals below
          if (t == 0) s_xinv[lt % kHalfScales] = fits ? inverse : 0.f;
@@ -369,6 +372,13 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
       // the weights' scales and verdict are the converters'
       bool ok = SOFIE_PROF_WAIT(mbar_wait(&w_ready, 0, &abort_flag, status, kStatusWaitConv, 0x5000));
       const bool w_exact = w_spread != 0;
+      // largest and smallest inverse scale of a channel's weights (positive: ordered as their bits are)
+      uint32_t w_low = 0x7f800000u, w_high = 0;
+      for (int c = lane; c < BN; c += 32) {
+         w_low = min(w_low, __float_as_uint(s_winv[c]));
+         w_high = max(w_high, __float_as_uint(s_winv[c]));
+      }
+      const float winv_low = __uint_as_float(__reduce_min_sync(0xffffffffu, w_low)), winv_high = __uint_as_float(__reduce_max_sync(0xffffffffu, w_high));
       // pooled: this lane's channels are 2 (lane % 4), +1 of every eight, its window is lane / 8 of pooled row lane_base / 16 + (lane / 4) % 2
       const int c2 = 2 * (lane & 3);
       const bool second = (lane & 4) != 0;
@@ -389,7 +399,8 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
          if (!ok) break;
          tc_fence_after();
          const float xinv = s_xinv[lt % kHalfScales];
-         const bool exact = w_exact || xinv == 0.f;
+         // a product of the inverse scales may be subnormal (an exact power of two all the same), but neither zero nor infinite
+         const bool exact = w_exact || !(xinv * winv_low > 0.f && xinv * winv_high < __uint_as_float(0x7f800000u));
          const uint32_t t_row = tmem_base + ((uint32_t)lane_base << 16) + (uint32_t)(buf * 2 * BN);
 #pragma unroll 1
          for (int c0 = c_begin; c0 < c_begin + CW; c0 += CH) {
@@ -406,7 +417,7 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
                }
                tmem_ld_wait();
 #pragma unroll
-               for (int j = 0; j < CH; j++) r[j] = __uint_as_float(a[j]) + __uint_as_float(b[j]);
+               for (int j = 0; j < CH; j++) r[j] = fmaf(__uint_as_float(b[j]), 1.f / kHalfTrailing, __uint_as_float(a[j]));
             }
             if (c0 + CH == c_begin + CW) { // all of this warp's columns have been read: the buffer is the issuers' again
                tc_fence_before();
@@ -415,9 +426,9 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, HalfConvParams
             }
             if (c0 >= p.Cout) continue;
             if (exact) griddep_wait(); // this thread reads the activations itself
-            // sum x the two inverse scales, one after the other (their product may leave fp32's range), + bias, Relu
+            // sum x the two inverse scales (rounded once) + bias, Relu
             auto finish = [&](float sum, float winv, float bias) {
-               const float v = fmaf(sum * xinv, winv, bias);
+               const float v = fmaf(sum, xinv * winv, bias);
                return p.relu ? relu_ref(v) : v;
             };
             if constexpr (POOL) {

@@ -229,8 +229,11 @@ def test_conv3x3_f32_tcgen05(case):
 
 
 # fp32 convolutions in half-precision parts: 16 and 32 channels, every width class of the output, odd tile counts, ragged channels
-# (values that the parts hold, values that send tiles or all of them to the FMA chains, infinities and NaN)
-@pytest.mark.parametrize("values", ["normal", "one sign", "image scales", "pixel scales", "tap scales", "specials"])
+# (values that the parts hold, values that they do not -- scales that differ from channel to channel, in a pixel's neighbourhood, from tap
+# to tap, beside weights that are zero or undo them --, filters that have died out, infinities and NaN)
+@pytest.mark.parametrize("values", ["normal", "one sign", "image scales", "pixel scales", "tap scales", "channels 2^8", "channels 2^16", "channels 2^24", "channels 2^28",
+                                    "channels 2^32", "channels 2^40", "channel blocks", "wide channel, no weights", "one place per image", "decayed channel", "dead filters",
+                                    "sparse decades", "smallest", "specials"])
 @pytest.mark.parametrize("N,C,H,W,Cout,relu,pool", [(3, 16, 16, 8, 20, 0, 0), (2, 16, 48, 24, 64, 1, 2), (150, 32, 16, 16, 64, 0, 2), (1, 32, 16, 40, 33, 1, 2),
                                                     (5, 32, 32, 16, 30, 0, 0), (3, 16, 32, 32, 100, 0, 2), (2, 16, 16, 16, 128, 1, 0), (1, 16, 16, 8, 1, 0, 2)])
 def test_conv3x3_f32_in_half_precision_parts(N, C, H, W, Cout, relu, pool, values):
@@ -244,6 +247,35 @@ def test_conv3x3_f32_in_half_precision_parts(N, C, H, W, Cout, relu, pool, value
         x *= 2.0 ** rng.integers(-30, 30, (N, 1, H, W))
     if values == "tap scales":
         w *= 2.0 ** rng.integers(-30, 30, (Cout, 1, 3, 3))
+    if values.startswith("channels") or values == "channel blocks":      # every product of the size it would have without the scales
+        e = float(values[values.find("^") + 1:]) if "^" in values else 30.0
+        scale = 2.0 ** np.round(np.linspace(0, e, C) if "^" in values else np.repeat([0, e / 3, e], C)[::3])
+        scale = (rng.permutation(scale) if "^" in values else scale)[:, None, None]
+        x, w = x * scale, w / scale
+    if values == "wide channel, no weights":
+        x[:, 3] *= 2.0 ** 26
+        x[N // 2:, 3] *= 2.0 ** 10
+        w[:, 3] = 0
+    if values == "one place per image":                                  # large there in every channel, and everywhere in a channel nobody reads
+        d = np.abs(np.arange(H)[:, None] - rng.integers(0, H, (N, 1, 1, 1))) + np.abs(np.arange(W)[None] - rng.integers(0, W, (N, 1, 1, 1)))
+        x *= 2.0 ** (-3.0 * d)
+        x[:, 0], w[:, 0] = 1, 0
+    if values == "decayed channel":                                      # weights of a channel that nobody used; half the images do
+        w[:, 5] *= 2.0 ** -70
+        w[:, 9:] *= rng.random((Cout, C - 9, 1, 1)) < 0.9
+        x[N // 2:, np.arange(C) != 5] = 0
+    if values == "dead filters":
+        w[0] *= 2.0 ** -40
+        w[Cout // 2] *= 2.0 ** -118
+        w[Cout // 3] *= 2.0 ** -135
+        w[Cout // 4] = 0
+        b[[0, Cout // 2, Cout // 3, Cout // 4]] = 0
+    if values == "sparse decades":
+        x = 10.0 ** rng.uniform(-9, 0, x.shape) * (rng.random((N, 1, H, W)) < 0.05)
+        x[:, :, : H // 2, : W // 2] = 0
+    if values == "smallest":                                             # down to the smallest normal numbers and the subnormal ones
+        x *= 2.0 ** rng.integers(-126, -90, (N, 1, H // 8, W // 8)).repeat(8, 2).repeat(8, 3)
+        w *= 2.0 ** rng.integers(60, 90, (Cout, 1, 1, 1))
     if values == "specials":
         for v in (np.inf, -np.inf, np.nan, 3e38, 1e-39):
             x[rng.integers(N), rng.integers(C), rng.integers(H), rng.integers(W)] = v
@@ -256,20 +288,19 @@ def test_conv3x3_f32_in_half_precision_parts(N, C, H, W, Cout, relu, pool, value
     conv = torch.nn.functional.conv2d
     ref = conv(xd, wd, bd, padding=1)
     ref = ref.float().double()      # sums beyond fp32's range are infinite
-    # a product of the parts is off by 2^-22 of the largest channel of its pixel times the weight, every MMA's sum by one truncation
-    size = conv(xd.abs().nan_to_num(0, 0).amax(1, keepdim=True).expand_as(xd), wd.abs(), bd.abs(), padding=1) if values == "pixel scales" else \
-        conv(xd.abs().nan_to_num(0, 0), wd.abs(), bd.abs(), padding=1)
+    # every product is off by 2^-22 of itself, every MMA's sum by one truncation
+    size = conv(xd.abs().nan_to_num(0, 0), wd.abs(), bd.abs(), padding=1)
     if relu:
         ref = torch.where(ref > 0, ref, 0.0)
     if pool:
-        # a NaN is passed over, as a comparison with it is false
+        # a NaN is passed over, as a comparison with it is false, unless the window holds nothing else
+        nan = -torch.nn.functional.max_pool2d(-ref.isnan().double(), 2) == 1
         ref = torch.where(ref.isnan(), -torch.inf, ref)
         ref, size = torch.nn.functional.max_pool2d(ref, 2), torch.nn.functional.max_pool2d(size, 2)
+        ref[nan] = torch.nan
     finite = ref.isfinite()
     steps = 2 * 9 * C // 16 + 4
-    assert ((y - ref).abs()[finite] <= steps * 2.0 ** -23 * size[finite]).all()
-    if pool:    # windows of nothing but NaNs
-        finite |= y.isnan()
+    assert ((y - ref).abs()[finite] <= steps * 2.0 ** -23 * size[finite] + 2.0 ** -149).all()
     assert torch.equal(y[~finite].float().nan_to_num(2.0, 1.0, -1.0), ref[~finite].float().nan_to_num(2.0, 1.0, -1.0))
 
 
