@@ -304,6 +304,34 @@ def test_conv3x3_f32_in_half_precision_parts(N, C, H, W, Cout, relu, pool, value
     assert torch.equal(y[~finite].float().nan_to_num(2.0, 1.0, -1.0), ref[~finite].float().nan_to_num(2.0, 1.0, -1.0))
 
 
+# many tiles a CTA, plain ones and such that take one pass, several or chains, in turn: their rings of slots, accumulators and patches come round
+@pytest.mark.parametrize("wide_weights", [0, 1])
+@pytest.mark.parametrize("N,C,H,W,Cout,pool", [(700, 16, 32, 32, 32, 2), (900, 32, 16, 32, 64, 0), (500, 16, 32, 32, 128, 2), (1700, 32, 16, 16, 24, 0)])
+def test_conv3x3_f32_in_half_precision_parts_many_tiles(N, C, H, W, Cout, pool, wide_weights):
+    g = torch.Generator(device="cuda").manual_seed(N + C + Cout)
+    x, w = torch.randn(N, C, H, W, device="cuda", generator=g), torch.randn(Cout, C, 3, 3, device="cuda", generator=g)
+    kind = torch.randint(0, 6, (N,), device="cuda", generator=g)
+    scale = lambda low, high, *shape: 2.0 ** torch.randint(low, high, shape, device="cuda", generator=g).float()
+    x = torch.where((kind == 1)[:, None, None, None], x * scale(-60, 60, N, 1, H, W), x)       # several passes
+    x = torch.where((kind == 2)[:, None, None, None], x * scale(-35, 1, N, C, H, W), x)        # one value or the other is lost
+    x[kind == 3, 3, 5, 5] = torch.inf
+    x[kind == 4, 2, 9, 2] = torch.nan
+    if wide_weights:
+        w *= scale(-40, 1, Cout, C, 3, 3)
+    y = ops.conv2d_f32(x.permute(0, 2, 3, 1).contiguous(), ops.conv2d_pack_f32(w), None, shape=x.shape, pad=(1, 1), pool=pool, x_layout=capi.LAYOUT_NHWC,
+                       y_layout=capi.LAYOUT_NHWC, w_packed=True, kernel=(3, 3))
+    y = y.double().view(N, H // max(pool, 1), W // max(pool, 1), Cout).permute(0, 3, 1, 2)
+    conv, pool2 = torch.nn.functional.conv2d, torch.nn.functional.max_pool2d
+    ref, size = conv(x.double(), w.double(), padding=1), conv(x.double().abs().nan_to_num(0, 0), w.double().abs(), padding=1)
+    if pool:
+        nan = -pool2(-ref.isnan().double(), 2) == 1
+        ref, size = pool2(torch.where(ref.isnan(), -torch.inf, ref), 2), pool2(size, 2)
+        ref[nan] = torch.nan
+    finite = ref.isfinite()
+    assert ((y - ref).abs()[finite] <= (2 * 9 * C // 16 + 4) * 2.0 ** -23 * size[finite]).all()
+    assert torch.equal(y[~finite].nan_to_num(2.0, 1.0, -1.0), ref[~finite].nan_to_num(2.0, 1.0, -1.0))
+
+
 @pytest.mark.parametrize("case", [(3, 32, 32, 32, 64, 1, 2), (7, 64, 16, 16, 64, 1, 2), (9, 64, 8, 8, 128, 1, 2), (2, 32, 16, 16, 40, 0, 0),
                                   (130, 32, 32, 32, 64, 1, 2), (3, 128, 16, 16, 128, 1, 2), (2, 256, 16, 16, 32, 0, 0),
                                   (2, 128, 32, 16, 64, 1, 0), (5, 32, 16, 16, 24, 1, 2),
