@@ -97,7 +97,9 @@ def test_qlinear_matmul_tcgen05_bit_exact(M, N, K, relu, zp):
 
 # few tiles and a long K: four or two CTAs of a cluster share a tile of 64, 128 or 256 columns; ranks with uneven parts of K (17 and 33
 # stages), with no columns of their own (64 columns, four ranks) and with columns beyond N
-@pytest.mark.parametrize("M,N,K", [(5, 70, 2096), (257, 64, 4096), (130, 300, 4112), (128, 4096, 4096), (300, 4090, 4112)])
+@pytest.mark.parametrize("M,N,K", [(5, 70, 2096), (257, 64, 4096), (130, 300, 4112), (128, 4096, 4096), (300, 4090, 4112),
+                                   # rows that are stored value by value: K shared for the sake of the stores, two rounds of narrow tiles
+                                   (1009, 131, 768), (340, 1919, 1744), (723, 1855, 96)])
 def test_8_bit_products_that_share_k(M, N, K):
     rng = np.random.default_rng(M + N + K)
     A, W = rng.integers(0, 256, (M, K)).astype(np.uint8), rng.integers(-127, 128, (N, K)).astype(np.int8)
