@@ -8,7 +8,7 @@
 // broadcast) feeds 16 packed FMAs and a warp stores whole lines of a 16-channel NHWC tensor. Every output is one chain of FMAs, two
 // channels at a time (each product and sum is rounded as the scalar ones are).
 // 1024 images of 16 x 16: 8 -> 16 channels 89 -> 28 us, 16 -> 16 164 -> 46; 256 x 64 -> 64 at 56 x 56 8369 -> 1795 (12.6 of the 37 TMAC/s of the
-// FMA units: the copies, the duplicated inputs of the packed FMAs and 12 warps an SM); a Session of a residual block on 1024 images 477 -> 297.
+// FMA units: the copies, the duplicated inputs of the packed FMAs and 12 warps an SM); a Session of a residual block on 1024 images 477 -> 291.
 #include "contract.cuh"
 
 namespace sofie {
@@ -204,10 +204,19 @@ int launch_conv2d_f32_direct3x3(cudaStream_t s, const ConvGeom &g, const float *
    if (g.C > 128 || (g.pool != 0 && g.pool != 2) || g.N < 1 || ceil_div(g.Cout, kDcOut) > 65535) return -1;
    const int chunks = ceil_div(g.C, kDcChunk);
    const bool vec = !g.x_nhwc && g.W % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0, wide = g.oW > 16;
-   // images that fill less than a quarter of their tiles stay with one thread per output: 1000 x 32 -> 32 at 7 x 7 141 us against 190 here, at 8 x 8
-   // (24 channels, NHWC) 145 against 136
-   const long long tiled = (long long)ceil_div(g.oH, kDcRows) * ceil_div(g.oW, wide ? 32 : 16) * kDcRows * (wide ? 32 : 16);
-   if (4LL * g.oH * g.oW < tiled) return -1;
+   // Images that fill less than a quarter of their tiles stay with one thread per output: 1000 x 32 -> 32 at 7 x 7 141 us against 190 here, at 8 x 8
+   // (24 channels, NHWC) 145 against 136. So do those that fill less than 0.6 of them where it is faster by the time in us that either takes, fitted
+   // to 200 calls of 1 to 1024 images (to 14 and 12 %; three of them are 6 to 16 % slower here all the same): few channels, whose time here is copies and indexes (32 x 5 -> 61 at 43 x 9 14.0 us against 22.3;
+   // 133 x 15 -> 103 at 65 x 6 212 against 248). Few tiles are not a reason: one image of 16 x 16, 128 -> 16 channels takes 235 us there and 124 here.
+   const long long groups = ceil_div(g.Cout, kDcOut), tiles = (long long)ceil_div(g.oH, kDcRows) * ceil_div(g.oW, wide ? 32 : 16), area = kDcRows * (wide ? 32 : 16);
+   const long long outputs = (long long)g.oH * g.oW;
+   if (4 * outputs < tiles * area) return -1;
+   if (5 * outputs < 3 * tiles * area) {
+      const double positions = 1e-6 * g.N * outputs, units = 1e-3 * g.N * tiles * groups * (wide ? 2 : 1);
+      const double general = 1.9 + 1.69 * g.C + positions * (25 * groups * g.C + 2.6 * g.Cout);
+      const double here = 2.5 + chunks * (vec ? 3.5 : 4.7) + units * (chunks * (vec ? 5.1 : 8.1) + 4.8);
+      if (1.05 * general <= here) return -1;
+   }
 #define SOFIE_DIRECT(P, G) return vec ? launch_direct<P, G, true>(s, g, X, W, bias, Y, chunks) : launch_direct<P, G, false>(s, g, X, W, bias, Y, chunks)
    if (g.pool == 2) {
       if (wide) SOFIE_DIRECT(2, 2);

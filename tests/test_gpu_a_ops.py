@@ -141,7 +141,8 @@ CONV_CASES = [
 # tiles (the last one is too small for them), rows of whole words or not, both layouts on either side, fused pooling of odd sizes, a NaN and infinities
 @pytest.mark.parametrize("pool", [0, 2])
 @pytest.mark.parametrize("N,C,H,W,Cout,x_nhwc,y_nhwc", [(3, 8, 16, 16, 16, 0, 0), (2, 16, 17, 33, 17, 0, 1), (400, 5, 8, 9, 3, 0, 0), (2, 6, 31, 64, 40, 0, 0),
-                                                        (2, 128, 16, 20, 8, 0, 1), (3, 12, 20, 18, 24, 1, 1), (1, 7, 6, 12, 16, 1, 0), (1, 9, 5, 60, 5, 0, 0), (2, 7, 3, 5, 9, 0, 0)])
+                                                        (2, 128, 16, 20, 8, 0, 1), (3, 12, 20, 18, 24, 1, 1), (1, 7, 6, 12, 16, 1, 0), (1, 9, 5, 60, 5, 0, 0), (2, 7, 3, 5, 9, 0, 0),
+                                                        (32, 5, 43, 9, 61, 0, 0), (20, 18, 8, 22, 33, 0, 0)])
 def test_conv3x3_f32_direct(N, C, H, W, Cout, x_nhwc, y_nhwc, pool):
     rng = np.random.default_rng(N + C + H + W + Cout)
     X, Wt, b = (rng.standard_normal(s).astype(np.float32) for s in ((N, C, H, W), (Cout, C, 3, 3), (Cout,)))
