@@ -72,10 +72,13 @@ conv_transpose2d_f32_kernel(sofie_conv_transpose2d_desc d, int oH, int oW, size_
 // A thread owns one output pixel and OC output channels. Threads are numbered by the column's residue modulo the stride before the column,
 // so that a warp's pixels share their taps (no divergence) and read neighbouring input pixels; the filters of the block's channels are
 // staged [channel][tap][OC], CK input channels at a time, and read as 16-byte broadcasts. A channel's product goes to one of four sums by the
-// channel's number modulo four: chains a quarter as long, whose error against float64 is about half of one chain's.
+// channel's number modulo four (those past the last multiple of four to the first): chains a quarter as long, whose error against float64 is about half of one chain's.
 // Against one thread per pixel and four channels with the filters from global memory: 32 -> 16 channels, 2 x 2 / 2 on 12 x 12, 1 / 64 / 1024 images 25 -> 9,
 // 55 -> 14, 785 -> 138 us; 16 -> 16, 3 x 3 / 1 on 64 x 64, 16 images 104 -> 27; error against float64 1.04e-7 -> 7.0e-8 and 2.1e-7 -> 1.2e-7. The product form
 // below is nearer to float64 still where it takes the tensor cores' three-part kernel, and stays where the caller asks for it.
+// At stride one with one input channel (or two and one tap) there is nothing to share, and as long as one wave of threads does, the pixel's thread with
+// the filters from global memory is there first: 8 x 8, one channel, 7 x 7 taps 18.4 us against 21.8, 3 x 3 5.4 against 6.1. Two channels and 3 x 3: 6.8
+// against 6.1; 64 images of 28 x 28, 1 -> 16 channels, 3 x 3: 17.4 against 13.0.
 constexpr int kPhaseThreads = 128;
 constexpr int kPhaseFilterBytes = 32 * 1024;
 template <int OC>
@@ -178,10 +181,11 @@ int launch_phase(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, i
 }
 int launch_direct(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, int oW, const float *X, const float *W, const float *bias, float *Y)
 {
-   const int rc = d.Cout <= 4 ? launch_phase<4>(s, d, oH, oW, X, W, bias, Y) : launch_phase<8>(s, d, oH, oW, X, W, bias, Y);
-   if (rc >= 0) return rc;
-   // filters of which not four channels fit beside one another, 2^31 outputs or more
    const size_t total = (size_t)d.N * ((d.Cout + kOcPerThread - 1) / kOcPerThread) * oH * oW;
+   const bool alone = d.stride_h == 1 && d.stride_w == 1 && d.C * min(d.kH * d.kW, 2) <= 2 && total <= 1u << 17;
+   const int rc = alone ? -1 : d.Cout <= 4 ? launch_phase<4>(s, d, oH, oW, X, W, bias, Y) : launch_phase<8>(s, d, oH, oW, X, W, bias, Y);
+   if (rc >= 0) return rc;
+   // also: filters of which not four channels fit beside one another, 2^31 outputs or more
    conv_transpose2d_f32_kernel<<<grid_for(total), kThreads, 0, s>>>(d, oH, oW, total, X, W, bias, Y);
    SOFIE_LAUNCH_CHECK("conv_transpose2d_f32_kernel");
    set_last_engine(SOFIE_ENGINE_SIMT);

@@ -229,7 +229,9 @@ def test_conv_transpose2d_f32(case):
 # of 4 and 16, strides with empty residues, and filters too large for shared memory
 @pytest.mark.parametrize("N,C,H,W,Cout,k,stride,pad,dil,out_pad", [(3, 70, 5, 7, 9, (5, 5), (2, 2), (2, 2), (1, 1), (1, 1)), (130, 17, 3, 2, 4, (2, 2), (2, 3), (0, 0), (1, 1), (0, 2)),
                                                                    (2, 16, 6, 11, 3, (3, 3), (1, 4), (1, 1), (2, 1), (0, 3)), (1, 3, 4, 4, 20, (1, 7), (3, 1), (0, 3), (1, 1), (2, 0)),
-                                                                   (1, 2, 2, 3, 8, (33, 33), (1, 1), (0, 0), (1, 1), (0, 0)), (2, 40, 9, 9, 16, (4, 4), (2, 2), (1, 1), (1, 1), (0, 0))])
+                                                                   (1, 2, 2, 3, 8, (33, 33), (1, 1), (0, 0), (1, 1), (0, 0)), (2, 40, 9, 9, 16, (4, 4), (2, 2), (1, 1), (1, 1), (0, 0)),
+                                                                   (4, 1, 32, 32, 9, (3, 5), (1, 1), (1, 0), (1, 2), (0, 0)), (60, 2, 8, 8, 3, (1, 1), (1, 1), (0, 0), (1, 1), (0, 0)),
+                                                                   (70, 1, 28, 28, 16, (2, 2), (1, 1), (0, 0), (1, 1), (0, 0))])
 def test_conv_transpose2d_f32_direct(N, C, H, W, Cout, k, stride, pad, dil, out_pad):
     rng = np.random.default_rng(N + C + H + W + Cout)
     X, Wt, b = (rng.standard_normal(s).astype(np.float32) for s in ((N, C, H, W), (C, Cout, *k), (Cout,)))
