@@ -849,14 +849,20 @@ template <int KIND, int BN>
 static int try_launch_conv_patch_bn(cudaStream_t s, const ConvGeom &g, const void *X, const void *Wp, const ConvEpilogue &ep)
 {
    constexpr int ES = (KIND == kTF32) ? 4 : 1;
+   // fp32 tiles of this size with 16 channels, or with 32 to at most 64, are the half-precision kernel's
+   constexpr bool kWith16 = KIND != kTF32, kWith32 = KIND != kTF32 || BN == 128;
    switch (g.C * ES) {
    case 32: return launch_conv_patch<KIND, BN, 1, 1>(s, g, X, Wp, ep);
-   case 64: return launch_conv_patch<KIND, BN, 2, 1>(s, g, X, Wp, ep);
-   case 128: {
-      // narrower stages when the resident weights leave room for fewer than two of the wide ones
-      const int rc = launch_conv_patch<KIND, BN, 4, 1>(s, g, X, Wp, ep);
-      return rc != -1 ? rc : launch_conv_patch<KIND, BN, 2, 2>(s, g, X, Wp, ep);
-   }
+   case 64:
+      if constexpr (kWith16) return launch_conv_patch<KIND, BN, 2, 1>(s, g, X, Wp, ep);
+      return -1;
+   case 128:
+      if constexpr (kWith32) {
+         // narrower stages when the resident weights leave room for fewer than two of the wide ones
+         const int rc = launch_conv_patch<KIND, BN, 4, 1>(s, g, X, Wp, ep);
+         return rc != -1 ? rc : launch_conv_patch<KIND, BN, 2, 2>(s, g, X, Wp, ep);
+      }
+      return -1;
    case 256: {
       const int rc = launch_conv_patch<KIND, BN, 4, 2>(s, g, X, Wp, ep);
       return rc != -1 ? rc : launch_conv_patch<KIND, BN, 2, 4>(s, g, X, Wp, ep);
