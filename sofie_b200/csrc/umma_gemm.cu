@@ -975,7 +975,7 @@ static void choose_tile(int M, int N, int K, int scalar, int &BN, int &split)
          if (q > 1 && (kb < 2 * q || tiles * q > (q == 2 ? kNumSMs : 140))) break;
          const long long rounds = (tiles * q + kNumSMs - 1) / kNumSMs;
          const long long store = (long long)scalar * stores[ceil_div<long long>(chunks, q)] * (M < kBM ? M : kBM) / kBM;
-         const long long time = rounds * (ceil_div((int)kb, q) * stage[w] + 700 + store) + tile[w] / q + (q > 1 ? 1700 + 500 * (chunks - chunks / q) + 1200 * scalar : 0);
+         const long long time = rounds * (ceil_div<long long>(kb, q) * stage[w] + 700 + store) + tile[w] / q + (q > 1 ? 1700 + 500 * (chunks - chunks / q) + 1200 * scalar : 0);
          if (best < 0 || time < best) best = time, BN = widths[w], split = q;
       }
    }
