@@ -1,8 +1,8 @@
 // What the host does to a model input on its way into pinned memory: copy it, or quantise it while it copies. A quantised
 // network reads its float input once, to quantise it; the host has to touch every one of those floats anyway when they lie in
 // pageable memory, and what it puts on the wire is then a quarter of the bytes. The loops are plain C for the compiler to
-// vectorise, with the IEEE division of the operator's definition (an AVX-512 core does 11 GB/s of floats; the memory of the host
-// is the limit from eight cores on), and give the bytes the device kernels give (quantize_u8_*, quantize_e4m3_* in eltwise.cu).
+// vectorise, with the IEEE division of the operator's definition (an AVX-512 core does 11 GB/s of floats, fourteen of a 16-core host 100
+// together; eight do 66), and give the bytes the device kernels give (quantize_u8_*, quantize_e4m3_* in eltwise.cu).
 #pragma once
 
 #include <cstddef>

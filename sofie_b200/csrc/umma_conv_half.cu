@@ -24,7 +24,8 @@
 // - Two scales whose product leaves fp32's range are applied one after the other.
 // Error against float64 (2-norm), N(0,1) operands: 2.1e-7 at 16 and 3.7e-7 at 32 channels, where TF32 parts gave 7.0e-7 and 1.28e-6 (their trailing
 // part is truncated, these are rounded, and the sums take half as many steps); operands of one sign 6.1e-7 and 1.4e-6 (1.05e-6 and 2.4e-6).
-// 8192 images 16 -> 32 at 32 x 32 with MaxPool 490 -> 332 us, 32 -> 64 at 16 x 16 367 -> 206 us; unpooled 2048 x 16 -> 32 172 -> 145 us. Of the first:
+// 8192 images 16 -> 32 at 32 x 32 with MaxPool 490 -> 332 us, 32 -> 64 at 16 x 16 365 -> 209 us; unpooled 2048 x 16 -> 32 165 -> 144 us; one image
+// 4.1 -> 4.0 and 5.5 -> 4.8 us when the kernel has just run, about 1 us more behind others (its instructions come from L2 then). Of the first:
 // channels 2^8 ... 2^40 apart 360; values down to 2^-28 of the largest and below in every patch 403; weights of a channel decayed to 1e-12 425; two
 // passes for every tile 1.5 ms, for images of exp(-r^2 / 8) 2.0, one infinity in each image 2.6 (as chains of FMAs in the epilogue, one scale and no check
 // of single sums, the last four took 20 ms, 10 for the infinities).
@@ -33,8 +34,9 @@
 // converter warps take the patches in turn, find the largest magnitude, split the values and write both parts as K-major swizzled
 // rows, from which each of the 9 taps is a start address (see the haloed-patch kernel). One MMA multiplies the leading parts of the
 // pixels with [leading | trailing] weights (2 * BN columns), one the trailing parts with the leading weights, into the second BN columns.
-// A TMEM buffer goes back to the issuers as soon as it has been read, before pooling and stores. Pooled tiles are read in the shape that puts a pixel and the one below it in one thread: a third of the shuffles, which wait for the shared-memory
-// pipe the MMAs keep busy (the epilogue set the kernel's time with them: 375 instead of 326 us).
+// A TMEM buffer goes back to the issuers as soon as it has been read, before pooling and stores. Pooled tiles are read in the shape that puts
+// a pixel and the one below it in one thread: a third of the shuffles, which wait for the shared-memory pipe the MMAs keep busy (the epilogue
+// set the kernel's time with them: 375 instead of 326 us).
 // Waiting with one lane and a vote, or with test_wait, instead of whole warps on try_wait: 5 to 25 % slower.
 #include "umma.cuh"
 #include "contract.cuh"
