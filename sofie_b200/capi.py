@@ -135,6 +135,7 @@ SIGNATURES = {
     "sofie_cuda_last_engine": [],
     "sofie_cuda_set_engine": [C.c_int],
     "sofie_cuda_gemm_f32": [vp, C.POINTER(GemmF32Desc), vp, vp, vp, vp],
+    "sofie_cuda_gemm_f32_ws": [vp, C.POINTER(GemmF32Desc), vp, vp, vp, vp, vp, sz],
     "sofie_cuda_gemm_f32_batched": [vp, C.POINTER(GemmF32Desc), vp, vp, vp, vp, i32, C.c_int64, C.c_int64, C.c_int64],
     "sofie_cuda_gemm_f32_splitk_static": [vp, C.POINTER(GemmF32Desc), vp, vp, vp, vp],
     "sofie_cuda_transpose_f32": [vp, vp, vp, i32, i32],
@@ -180,6 +181,7 @@ SIGNATURES = {
 STRING_GETTERS = {"sofie_cuda_strerror": [C.c_int], "sofie_cuda_last_error": []}
 SIZE_GETTERS = {"sofie_cuda_slice_rows": [sz, sz, sz, sz],
                 "sofie_cuda_mlp_f32_smem": [C.POINTER(MlpDesc)],
+                "sofie_cuda_gemm_f32_workspace": [C.POINTER(GemmF32Desc)],
                 "sofie_cuda_conv_transpose2d_f32_gemm_scratch": [C.POINTER(ConvTranspose2dDesc)]}
 MLP_MAX_LAYERS, MLP_MAX_WIDTH, MLP_MAX_SMEM = 8, 256, 200 * 1024
 

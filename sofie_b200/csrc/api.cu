@@ -48,8 +48,18 @@ using namespace sofie;
 
 extern "C" {
 
-int sofie_cuda_gemm_f32(void *stream, const sofie_gemm_f32_desc *d, const float *A, const float *B, const float *C,
-                        float *Y)
+int sofie_cuda_gemm_f32(void *stream, const sofie_gemm_f32_desc *d, const float *A, const float *B, const float *C, float *Y)
+{
+   return sofie_cuda_gemm_f32_ws(stream, d, A, B, C, Y, nullptr, 0);
+}
+
+size_t sofie_cuda_gemm_f32_workspace(const sofie_gemm_f32_desc *d)
+{
+   if (!d || d->M <= 0 || d->N <= 0 || d->K <= 0 || forced_engine() == SOFIE_ENGINE_SIMT) return 0;
+   return gemm_f32_parts_bytes(*d);
+}
+
+int sofie_cuda_gemm_f32_ws(void *stream, const sofie_gemm_f32_desc *d, const float *A, const float *B, const float *C, float *Y, void *workspace, size_t bytes)
 {
    SOFIE_REQUIRE(d != nullptr, "NULL descriptor");
    SOFIE_REQUIRE(d->M >= 0 && d->N > 0 && d->K > 0, "bad GEMM shape %d x %d x %d", d->M, d->N, d->K);
@@ -58,6 +68,10 @@ int sofie_cuda_gemm_f32(void *stream, const sofie_gemm_f32_desc *d, const float 
    if (d->M == 0) return SOFIE_CUDA_OK; // an empty batch has no rows to compute (and may have NULL A / Y)
    SOFIE_REQUIRE(A && B && Y, "NULL tensor");
    cudaStream_t s = as_stream(stream);
+   if (workspace && forced_engine() != SOFIE_ENGINE_SIMT) {
+      const int rc = launch_gemm_f32_parts(s, *d, A, B, C, Y, workspace, bytes);
+      if (rc != SOFIE_CUDA_ERR_UNSUPPORTED) return rc;
+   }
    // few rows, few columns, long K: split K over the grid, instead of running on two or three SMs. The tensor-core kernel is the faster one
    // from about 800 rows on (1000 x 10 x 4096 14.6 against 21.8 us, 24 x 10 x 4096 13.6 against 7.1), but split-K's many short chains are
    // the more precise: 1.0e-7 from float64 at K = 1500 against 1.2e-7, and 0.5e-7 against 1.8e-7 with operands of one sign.

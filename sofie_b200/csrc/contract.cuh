@@ -16,6 +16,11 @@ int launch_gemm_f32_umma(cudaStream_t, const sofie_gemm_f32_desc &, const float 
 // any layout, alignment and K; long K split over a cluster (umma_gemm_any.cu). tma: operands the TMA kernel takes too; others are refused
 // where the CUDA-core kernel is the faster one
 int launch_gemm_f32_any(cudaStream_t, const sofie_gemm_f32_desc &, bool tma, const float *, const float *, const float *, float *);
+// the time in ns that such a product is estimated to take there or on the CUDA cores, whichever is faster
+long long gemm_f32_whole_ns(const sofie_gemm_f32_desc &, bool tma);
+// the same out of operands split into a workspace first (umma_gemm_parts.cu): UNSUPPORTED without one of gemm_f32_parts_bytes (0: not its shape)
+size_t gemm_f32_parts_bytes(const sofie_gemm_f32_desc &);
+int launch_gemm_f32_parts(cudaStream_t, const sofie_gemm_f32_desc &, const float *, const float *, const float *, float *, void *workspace, size_t bytes);
 int launch_qgemm_simt(cudaStream_t, const sofie_qgemm_desc &, const uint8_t *, const int8_t *, const float *,
                       const int32_t *, uint8_t *, float *Yf32, float dq_scale);
 int launch_qgemm_umma(cudaStream_t, const sofie_qgemm_desc &, const uint8_t *, const int8_t *, const float *,

@@ -19,16 +19,13 @@
 //     writes a S-th of the rows out of all of them (distributed shared memory, fixed order). No scratch buffer, one launch.
 // What bounds it is the workers' chain of loading, splitting and storing; the MMAs of a stage take 770 clocks at 128 columns.
 // The tile goes out through shared memory, so stores (and a bias of the output's shape) are contiguous along rows for every N.
-#include "umma.cuh"
+#include "gemm_parts.cuh"
 #include "contract.cuh"
 
 namespace sofie {
 namespace umma {
 namespace {
 
-constexpr int kAnyBM = 128;             // rows of the tile = TMEM lanes
-constexpr int kAnyKE = 32;              // floats of K per stage: one 64-byte swizzle row of each of the three parts
-constexpr int kAnyRow = kAnyKE * 2;
 constexpr int kAnyWorkers = 16 * 32;
 // Groups of worker warps that take the stages in turn. Four were 5 to 10 % faster at 32 columns with a long K and as much slower with a
 // short one (the pipeline takes longer to start), and spilled at 64 columns.
@@ -47,31 +44,6 @@ struct AnySmem {
    static_assert(kB % 512 == 0, "parts start on whole swizzle atoms");
    static constexpr int kBytes = kStages * kStage + 1024;
 };
-
-// How an operand of `rows` x K is read.
-enum AnyMode { kVecK = 0, kScalarK = 1, kRowsContiguous = 2 };
-struct AnyOperand {
-   const float *p;
-   long long ld; // distance of rows (kVecK, kScalarK) or of consecutive K (kRowsContiguous)
-   int rows, mode;
-};
-
-// Two values in three bfloat16 parts each, packed: round, take off, twice. Both remainders are exact, and the second has at most
-// seven bits, so that its upper half is all of it: p0 + p1 + p2 is the value itself.
-__device__ __forceinline__ uint32_t any_part(float lo, float hi)
-{
-   uint32_t p;
-   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p) : "f"(hi), "f"(lo)); // the first source lands in the upper half
-   return p;
-}
-__device__ __forceinline__ void any_split(float x, float y, uint32_t &p0, uint32_t &p1, uint32_t &p2)
-{
-   p0 = any_part(x, y);
-   x -= __uint_as_float(p0 << 16), y -= __uint_as_float(p0 & 0xFFFF0000u);
-   p1 = any_part(x, y);
-   x -= __uint_as_float(p1 << 16), y -= __uint_as_float(p1 & 0xFFFF0000u);
-   p2 = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
-}
 
 // One thread's share of the tiles of an operand with R rows: U units, a unit being K chunk `c` (eight floats) of row `r`.
 //   K contiguous: four lanes cover the 128 bytes of one row; the thread's units are T / 4 rows apart, in the same chunk.
@@ -164,44 +136,7 @@ struct AnyLoader {
    }
 };
 
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr)
-{
-   float4 v;
-   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
-   return v;
-}
-__device__ __forceinline__ float ld_cluster_f1(uint32_t addr)
-{
-   float v;
-   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
-   return v;
-}
 __device__ __forceinline__ void workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kAnyWorkers) : "memory"); }
-
-struct AnyEpilogue {
-   float alpha, beta;
-   const float *C;
-   float *Y;
-   int bias_kind, relu, vec; // vec: rows of Y (and of a full C) start on 16-byte boundaries
-   int unit;                 // stages added up in one TMEM buffer (the tensor core's sums truncate) before they are promoted
-};
-
-__device__ __forceinline__ float any_finish(const AnyEpilogue &ep, float v, float c)
-{
-   v = ep.alpha * v;
-   if (ep.bias_kind) v += ep.beta * c;
-   return ep.relu ? relu_ref(v) : v;
-}
-
-// The parts of an operand that is infinite, not a number or above the largest bfloat16 do not add up to it (Inf - Inf, Inf x 0), and
-// those of one below 2^-110 lose bits to bfloat16's range. The first kind shows in the sum, the second where the sum is tiny too
-// (and not where a factor above 2^14 or more lifts it back into the range; an operand below 2^-134 counts as zero). Such a sum is
-// doubtful: it is taken again as the chain of FMAs that the CUDA-core kernel forms, term by term.
-__device__ __forceinline__ bool any_doubtful(float v)
-{
-   const uint32_t e = __float_as_uint(v) & 0x7FFFFFFFu, tiny = 31u << 23; // 2^-96
-   return e - tiny >= 0x7F800000u - tiny && e != 0u;
-}
 
 // any_write below for a tile with doubtful sums.
 template <int BN>
@@ -509,17 +444,9 @@ int launch_any(cudaStream_t s, const AnyOperand &A, const AnyOperand &B, const A
    return SOFIE_CUDA_OK;
 }
 
-} // namespace
-} // namespace umma
-
-int launch_gemm_f32_any(cudaStream_t s, const sofie_gemm_f32_desc &d, bool tma, const float *A, const float *B, const float *C, float *Y)
+// Time of a product on this kernel in ns, at its best tile width and cluster size.
+long long any_ns(const sofie_gemm_f32_desc &d, int &BN, int &S)
 {
-   using namespace umma;
-   auto aligned = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-   const bool vec_k = d.K % 4 == 0;
-   const AnyOperand a{A, d.transA ? d.M : d.K, d.M, d.transA ? kRowsContiguous : (vec_k && aligned(A) ? kVecK : kScalarK)};
-   const AnyOperand b{B, d.transB ? d.K : d.N, d.N, !d.transB ? kRowsContiguous : (vec_k && aligned(B) ? kVecK : kScalarK)};
-   const AnyEpilogue ep{d.alpha, d.beta, C, Y, d.bias_kind, d.relu, d.N % 4 == 0 && aligned(Y) && (d.bias_kind != 2 || aligned(C)), d.K >= 1024 ? 8 : (d.K >= 256 ? 4 : 3)};
    const int tm = ceil_div(d.M, kAnyBM), nkb = ceil_div(d.K, kAnyKE);
    // Tile width and clusters along K by the time they take, in ns (fitted to 450 products, each at every width and cluster size): a stage
    // of 32 K, a tile's start and end, the exchange within a cluster, and what the write-out takes more where rows of Y are not whole
@@ -529,7 +456,7 @@ int launch_gemm_f32_any(cudaStream_t s, const sofie_gemm_f32_desc &d, bool tma, 
                     room[4] = {kNumSMs, kNumSMs, 140, 104};
    const bool vec = d.N % 4 == 0, full = d.bias_kind == 2;
    const long long bias = full ? (long long)d.M * d.N / 750 : 0;
-   int BN = 32, S = 1;
+   BN = 32, S = 1;
    long long best = -1;
    for (int w = 0; w < 3; w++) {
       if (widths[w] > 32 && widths[w] / 2 >= d.N) continue; // more than half of the tile would be padding
@@ -541,15 +468,43 @@ int launch_gemm_f32_any(cudaStream_t s, const sofie_gemm_f32_desc &d, bool tma, 
          if (best < 0 || time < best) best = time, BN = widths[w], S = q;
       }
    }
+   return best;
+}
+// ... and on the CUDA-core kernel.
+long long simt_ns(const sofie_gemm_f32_desc &d)
+{
+   const long long blocks = (long long)ceil_div(d.M, 64) * ceil_div(d.N, 64), steps = ceil_div(d.K, 16);
+   const long long alone = 1900 * steps * ((blocks + 3 * kNumSMs - 1) / (3 * kNumSMs));
+   const long long filled = ((d.transB ? 645 : 445) * steps + 800 + (d.bias_kind == 2 ? 330 : 0)) * blocks / kNumSMs;
+   return 2200 + (alone > filled ? alone : filled);
+}
+
+} // namespace
+} // namespace umma
+
+long long gemm_f32_whole_ns(const sofie_gemm_f32_desc &d, bool tma)
+{
+   int BN, S;
+   const long long any = umma::any_ns(d, BN, S), simt = umma::simt_ns(d);
+   return tma || simt > any ? any : simt;
+}
+
+int launch_gemm_f32_any(cudaStream_t s, const sofie_gemm_f32_desc &d, bool tma, const float *A, const float *B, const float *C, float *Y)
+{
+   using namespace umma;
+   auto aligned = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+   const bool vec_k = d.K % 4 == 0;
+   const AnyOperand a{A, d.transA ? d.M : d.K, d.M, d.transA ? kRowsContiguous : (vec_k && aligned(A) ? kVecK : kScalarK)};
+   const AnyOperand b{B, d.transB ? d.K : d.N, d.N, !d.transB ? kRowsContiguous : (vec_k && aligned(B) ? kVecK : kScalarK)};
+   const AnyEpilogue ep{d.alpha, d.beta, C, Y, d.bias_kind, d.relu, d.N % 4 == 0 && aligned(Y) && (d.bias_kind != 2 || aligned(C)), d.K >= 1024 ? 8 : (d.K >= 256 ? 4 : 3)};
+   int BN, S;
+   const long long best = any_ns(d, BN, S);
    // What TMA cannot fetch has the CUDA-core kernel beside it: blocks of 64 x 64, steps of 16 K that take 1.9 us alone and 0.45 us (0.65 with
    // B stored [N,K]) apart on an SM full of them, whose outputs leave while other blocks compute. It wins where the output is what
    // counts: 16384 x 4093 x 8 with a full bias 163 us against 580, 16384 x 777 x 64 81 against 144; 1000 x 777 x 1333 211 against 38. Over
    // 620 products the choice is 0.9 % above the faster of the two in the mean, and never more than 5 % above the CUDA-core kernel.
    if (!tma && forced_engine() != SOFIE_ENGINE_TCGEN05) {
-      const long long blocks = (long long)ceil_div(d.M, 64) * ceil_div(d.N, 64), steps = ceil_div(d.K, 16);
-      const long long alone = 1900 * steps * ((blocks + 3 * kNumSMs - 1) / (3 * kNumSMs));
-      const long long filled = ((d.transB ? 645 : 445) * steps + 800 + (full ? 330 : 0)) * blocks / kNumSMs;
-      if (2200 + (alone > filled ? alone : filled) < best) return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "faster on the CUDA cores");
+      if (simt_ns(d) < best) return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "faster on the CUDA cores");
    }
    if (BN == 128) return launch_any<128>(s, a, b, ep, d.K, S);
    if (BN == 64) return launch_any<64>(s, a, b, ep, d.K, S);

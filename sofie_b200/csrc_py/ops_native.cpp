@@ -165,7 +165,17 @@ PyObject *gemm_f32(Args a)
    void *const s = stream();
    const float *pA = as<float>(A), *pB = as<float>(B), *pC = as<float>(a[2]);
    float *pY = as<float>(Y);
-   SOFIE_CALL(sofie_cuda_gemm_f32, s, &d, pA, pB, pC, pY);
+   // a workspace where one makes the product faster, from torch's pool of this stream; without memory for it the product does without
+   const size_t bytes = sofie_cuda_gemm_f32_workspace(&d);
+   at::Tensor workspace;
+   if (bytes) {
+      try {
+         workspace = make({(int64_t)bytes}, at::kByte, A);
+      } catch (const c10::OutOfMemoryError &) {
+      }
+   }
+   void *const w = workspace.defined() ? workspace.data_ptr() : nullptr;
+   SOFIE_CALL(sofie_cuda_gemm_f32_ws, s, &d, pA, pB, pC, pY, w, w ? bytes : 0);
    return THPVariable_Wrap(Y);
 }
 

@@ -489,3 +489,48 @@ def test_gemm_f32_takes_the_faster_kernel_where_tma_cannot_fetch(M, N, K, tA, tB
     if engine == capi.ENGINE_SIMT:
         ops.set_engine(capi.ENGINE_SIMT)
         assert torch.equal(y, ops.gemm_f32(A, B, C_, transA=tA, transB=tB, alpha=0.75, beta=1.5))
+
+
+# one tile and several per CTA, every tile width, K shared by 1, 2, 4 and 8 ranks, units of 3, 4 and 8 stages with remainders, ragged and whole rows of Y
+@pytest.mark.parametrize("M,N,K,bias", [(2049, 513, 257, 1), (1000, 777, 1333, 2), (64, 60, 4100, 0), (5000, 330, 95, 2), (1024, 1024, 1024, 1), (390, 2052, 600, 0),
+                                        (4200, 330, 2050, 1), (130, 1290, 3000, 2), (20000, 129, 65, 0), (12100, 520, 140, 1), (36, 3000, 3905, 2), (900, 2500, 64, 0)])
+def test_gemm_f32_of_operands_split_beforehand(M, N, K, bias):
+    """The workspace form against float64 and the chain of FMAs (whose 2-norm error is the bound), for every layout and an unaligned base; rows
+    of values the parts do not hold give what the chain gives; without the workspace the call is the plain one."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    lib = capi.load()
+
+    def place(t, offset):
+        buf = torch.empty(t.numel() + 4, device="cuda")
+        return buf[offset: offset + t.numel()].view(t.shape).copy_(t)
+    taken = 0
+    for i, (tA, tB) in enumerate(((0, 0), (0, 1), (1, 0), (1, 1))):
+        A = place(torch.randn((K, M) if tA else (M, K), device="cuda", generator=g), i % 2)
+        B = place(torch.randn((N, K) if tB else (K, N), device="cuda", generator=g) * K ** -0.5, i // 2)
+        C_ = {0: None, 1: torch.randn(N, device="cuda", generator=g), 2: torch.randn(M, N, device="cuda", generator=g)}[bias]
+        a, b = (A.t() if tA else A), (B.t() if tB else B)
+        a[5, 7], a[6, K - 1], a[9] = float("inf"), float("nan"), a[9] * 1e-35
+        d = capi.GemmF32Desc(M, N, K, tA, tB, 0.75, 1.5, bias, i % 2)
+        nbytes = lib.sofie_cuda_gemm_f32_workspace(C.byref(d))
+        taken += nbytes > 0
+
+        def product(engine, size):
+            ops.set_engine(engine)
+            w = torch.empty(max(size, 1), dtype=torch.uint8, device="cuda")
+            Y = torch.full((M, N), 7.0, device="cuda")
+            capi.call("sofie_cuda_gemm_f32_ws", ops._stream(), C.byref(d), *[C.c_void_p(0 if t is None else t.data_ptr()) for t in (A, B, C_, Y)], C.c_void_p(w.data_ptr()), size)
+            return Y
+        chain, plain = product(capi.ENGINE_SIMT, nbytes), product(capi.ENGINE_TCGEN05, nbytes - 1 if nbytes else 0)
+        y = product(capi.ENGINE_TCGEN05, nbytes)
+        assert ops.last_engine() == capi.ENGINE_TCGEN05
+        exact = 0.75 * (a.double() @ b.double()) + (0 if C_ is None else 1.5 * C_.double())
+        if i % 2:
+            exact = torch.where(exact > 0, exact, 0.)
+        for odd in (5, 6):
+            assert torch.equal(y[odd].nan_to_num(1.), chain[odd].nan_to_num(1.)) and torch.equal(y[odd].isnan(), chain[odd].isnan())
+        if bias == 0:
+            assert torch.equal(y[9], chain[9])
+        rows = [r for r in range(M) if r not in (5, 6, 9)]
+        off = [float((t[rows].double() - exact[rows]).norm()) for t in (y, chain, plain)]
+        assert off[0] <= off[1] * 1.02 and off[2] <= off[1] * 1.02      # K = 64 .. 95: all of them round a handful of times
+    assert taken == 4
