@@ -96,14 +96,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
 // The issuers' form has no way out, since a branch behind the wait costs 45 to 90 clocks a stage: a wait that runs out (about a
 // second) leaves `gave_up` set, which makes the later ones return at once; the warp walks on over whatever the stages hold to the end of its
 // loop and then reports with finish(). Copies are not issued that way: a role that writes shared memory stops (mbar_wait_warp).
+constexpr uint32_t kPollLimit = 1u << 18; // polls of a barrier that nothing happens to take 7800 clocks each: about a second
 struct WarpWait {
    uint32_t gave_up = 0;
    __device__ __forceinline__ void operator()(uint64_t *bar, uint32_t parity)
    {
-      const uint32_t start = clock();
-      uint32_t limit = gave_up ? 0u : (uint32_t)kWaitLimitCycles;
-      while (!__any_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity)) && limit) limit = __any_sync(0xFFFFFFFFu, (uint32_t)clock() - start >= limit) ? 0u : limit;
-      gave_up |= limit == 0u;
+      uint32_t n = gave_up;
+      while (!__any_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity)) && ++n < kPollLimit) {}
+      gave_up |= n & kPollLimit;
    }
    // After the role's loop: true when all waits came through. Otherwise the give-up is reported and the MMAs under way are waited for
    // (`drain`: a barrier of one arrival that nothing else uses).
@@ -179,6 +179,27 @@ __device__ __forceinline__ void warp_expect_tx(uint64_t *bar, uint32_t bytes)
    asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xFFFFFFFF;\n\t@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
                 "r"(bytes)
                 : "memory");
+}
+#define SOFIE_WARP_TMA(rank, coords, ...)                                                                                                \
+   asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xFFFFFFFF;\n\t"                                                               \
+                "@e cp.async.bulk.tensor." rank ".shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {" coords "}], [%2];\n\t}" ::"r"(smem_u32(dst)), \
+                "l"(map), "r"(smem_u32(bar)), __VA_ARGS__                                                                                \
+                : "memory")
+__device__ __forceinline__ void warp_tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar)
+{
+   SOFIE_WARP_TMA("2d", "%3, %4", "r"(x), "r"(y));
+}
+__device__ __forceinline__ void warp_tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar)
+{
+   SOFIE_WARP_TMA("3d", "%3, %4, %5", "r"(x), "r"(y), "r"(z));
+}
+__device__ __forceinline__ void warp_tma_load_4d(void *dst, const CUtensorMap *map, int x, int y, int z, int w, uint64_t *bar)
+{
+   SOFIE_WARP_TMA("4d", "%3, %4, %5, %6", "r"(x), "r"(y), "r"(z), "r"(w));
+}
+__device__ __forceinline__ void warp_tma_load_5d(void *dst, const CUtensorMap *map, int x, int y, int z, int w, int v, uint64_t *bar)
+{
+   SOFIE_WARP_TMA("5d", "%3, %4, %5, %6, %7", "r"(x), "r"(y), "r"(z), "r"(w), "r"(v));
 }
 // `bytes` (a multiple of 16) from a 16-byte aligned address
 __device__ __forceinline__ void warp_bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
@@ -301,10 +322,11 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr)
 }
 // Tensor copy into this CTA's shared memory whose completion bytes are counted on a barrier that may
 // lie in the peer CTA (cluster address).
-__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, int x, int y, uint32_t bar_cluster_addr)
+__device__ __forceinline__ void warp_tma_load_2d_pair(void *dst, const CUtensorMap *map, int x, int y, uint32_t bar_cluster_addr)
 {
-   asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-                ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(bar_cluster_addr)
+   asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xFFFFFFFF;\n\t"
+                "@e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}" ::"r"(smem_u32(dst)),
+                "l"(map), "r"(x), "r"(y), "r"(bar_cluster_addr)
                 : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t *smem_result, uint32_t ncols)
@@ -322,27 +344,19 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 }
 // Arrive on the barrier at this shared-memory offset in every CTA of `cta_mask` once all MMAs issued
 // so far by this thread have completed.
-__device__ __forceinline__ void tc_commit_pair(uint64_t *bar, uint16_t cta_mask)
+__device__ __forceinline__ void warp_commit_pair(uint64_t *bar, uint16_t cta_mask)
 {
-   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+   asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xFFFFFFFF;\n\t"
+                "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
                 "h"(cta_mask)
                 : "memory");
 }
 template <int KIND>
-__device__ __forceinline__ void tc_mma_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
+__device__ __forceinline__ void warp_mma_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate)
 {
    static_assert(KIND == kI8 || KIND == kF8, "pair MMAs are built for the 8-bit kinds");
-   if constexpr (KIND == kI8) {
-      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                   "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-                   "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-                   : "memory");
-   } else {
-      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                   "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-                   "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-                   : "memory");
-   }
+   if constexpr (KIND == kI8) SOFIE_WARP_MMA("2", "i8");
+   else SOFIE_WARP_MMA("2", "f8f6f4");
 }
 
 // 32 lanes x 32 columns of 32-bit accumulators: thread t of the warp receives lane (base + t),

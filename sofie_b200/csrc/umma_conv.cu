@@ -243,7 +243,7 @@ umma_conv3x3_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
    constexpr int EPI_WARPS = KIND == kI8 ? kConvEpilogueWarpsI8 : kConvEpilogueWarps;
    extern __shared__ unsigned char smem_raw[];
    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-   __shared__ uint64_t full_bar[kConvMaxStages], conv_bar[kConvMaxStages], empty_bar[kConvMaxStages], tmem_full[NBUF], tmem_empty[NBUF], w_full;
+   __shared__ uint64_t full_bar[kConvMaxStages], conv_bar[kConvMaxStages], empty_bar[kConvMaxStages], tmem_full[NBUF], tmem_empty[NBUF], w_full, drain_bar[2];
    __shared__ uint32_t tmem_base_holder;
    __shared__ volatile uint32_t abort_flag;
    __shared__ float s_bias[128], s_mult[128]; // per output channel, zero / one beyond Cout
@@ -281,6 +281,7 @@ umma_conv3x3_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
          mbar_init(&tmem_empty[b], EPI_WARPS);
       }
       mbar_init(&w_full, 1);
+      for (int i = 0; i < 2; i++) mbar_init(&drain_bar[i], 1);
       abort_flag = 0;
       fence_mbar_init();
       prefetch_tensormap(&tmX);
@@ -298,9 +299,6 @@ umma_conv3x3_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
 
    if (warp == 0) {
       // ---------------- TMA producer ----------------
-      // Issuing a tensor copy costs the issuing thread a few hundred cycles, so the 2 x TPS copies of
-      // a stage are issued by 2 x TPS lanes in parallel; lane 0 waits for the free slot and posts the
-      // expected byte count (the phase cannot complete before that arrive, whatever the order).
       if constexpr (RW) {
          // the weights are constants: fetched before the previous kernel's output is waited for
          if (lane == 0) mbar_expect_tx(&w_full, (uint32_t)(9 * tg.chunks * B_TILE));
@@ -319,82 +317,73 @@ umma_conv3x3_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
       for (int tile = blockIdx.x; tile < tg.num_tiles && ok; tile += gridDim.x, tw.next()) {
          const int n0 = tw.n * tg.tileN, h0 = tw.th * tg.tileH, w0 = tw.tw * tg.tileW;
          for (int st = 0; st < stages_per_tile; st++, g++, ring_next(s, ph, S)) {
-            if (lane == 0) {
-               ok = SOFIE_PROF_WAIT(mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g));
-               if (ok) mbar_expect_tx(&full_bar[s], TPS * (RW ? A_TILE : A_TILE + B_TILE));
-            }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            ok = SOFIE_PROF_WAIT(mbar_wait_warp(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g));
             if (!ok) break;
-            if (RW ? lane < TPS : lane < 2 * TPS) {
-               const int k = RW ? lane : lane >> 1;
+            warp_expect_tx(&full_bar[s], TPS * (RW ? A_TILE : A_TILE + B_TILE));
+#pragma unroll
+            for (int k = 0; k < TPS; k++) {
                const int item = st * TPS + k;
                const int tap = tg.chunks == 1 ? item : item / tg.chunks, ch = tg.chunks == 1 ? 0 : item % tg.chunks;
                const int r = tap / 3, sx = tap - 3 * r;
                // x coordinate (channels) is a multiple of CBE, i.e. of 16 bytes; the spatial
                // coordinates may be -1 or reach H / W: those elements read as zero
-               if (!RW && (lane & 1)) tma_load_2d(b_hi(s, k), &tmW, tap * tg.C + ch * CBE, 0, &full_bar[s]);
-               else tma_load_4d(a_hi(s, k), &tmX, ch * CBE, w0 + sx - 1, h0 + r - 1, n0, &full_bar[s]);
+               warp_tma_load_4d(a_hi(s, k), &tmX, ch * CBE, w0 + sx - 1, h0 + r - 1, n0, &full_bar[s]);
+               if constexpr (!RW) warp_tma_load_2d(b_hi(s, k), &tmW, tap * tg.C + ch * CBE, 0, &full_bar[s]);
             }
-            __syncwarp();
          }
       }
    } else if (warp == 1 || (KIND == kI8 && warp == kConvIssuerB)) {
       // ---------------- MMA issuers ----------------
-      // int8: two threads of different warps take the tiles alternately (an MMA costs the thread that issues
-      // it more clocks than it occupies the tensor pipe); fp32: one thread.
+      // int8: two warps take the tiles alternately (the hand-over between two tiles leaves the pipe idle otherwise); fp32: one.
       const int issuer = warp == 1 ? 0 : 1;
-      if (lane == 0) {
-         constexpr uint32_t idesc = make_idesc<KIND>(128, BN);
-         int g = 0, lt = 0, s = 0;
-         uint32_t ph = 0;
-         bool ok = true;
-         if constexpr (RW) ok = SOFIE_PROF_WAIT(mbar_wait(&w_full, 0, &abort_flag, status, kStatusWaitFull, 0x4000));
-         for (int tile = blockIdx.x; tile < tg.num_tiles && ok; tile += gridDim.x, lt++) {
-            const int buf = lt & (NBUF - 1);
-            if (KIND == kI8 && (lt & 1) != issuer) {
-               // the other issuer's tile: step over its stages, still seeing each of them become ready (a parity
-               // wait tells only the last two phases of a barrier apart, so no phase of a shared slot is skipped)
-               for (int st = 0; st < stages_per_tile && ok; st++, g++, ring_next(s, ph, S))
-                  ok = SOFIE_PROF_WAIT(mbar_wait(&full_bar[s], ph, &abort_flag, status, kStatusWaitFull, g));
-               continue;
-            }
-            if (!SOFIE_PROF_WAIT(mbar_wait(&tmem_empty[buf], ((lt / NBUF) & 1) ^ 1, &abort_flag, status, kStatusWaitAccum, 0x2000 + lt))) break;
+      constexpr uint32_t idesc = make_idesc<KIND>(128, BN);
+      int lt = 0, s = 0;
+      uint32_t ph = 0;
+      WarpWait wait;
+      if constexpr (RW) wait(&w_full, 0);
+      for (int tile = blockIdx.x; tile < tg.num_tiles; tile += gridDim.x, lt++) {
+         const int buf = lt & (NBUF - 1);
+         if (KIND == kI8 && (lt & 1) != issuer) {
+            // the other issuer's tile: step over its stages, still seeing each of them become ready (a parity
+            // wait tells only the last two phases of a barrier apart, so no phase of a shared slot is skipped)
+            for (int st = 0; st < stages_per_tile; st++, ring_next(s, ph, S)) wait(&full_bar[s], ph);
+            continue;
+         }
+         wait(&tmem_empty[buf], ((lt / NBUF) & 1) ^ 1);
+         tc_fence_after();
+         const uint32_t d_base = tmem_base + (uint32_t)(buf * NACC * BN);
+         int mma_idx = 0; // MMAs issued for this tile
+         for (int st = 0; st < stages_per_tile; st++, ring_next(s, ph, S)) {
+            wait(KIND == kTF32 ? &conv_bar[s] : &full_bar[s], ph);
             tc_fence_after();
-            const uint32_t d_base = tmem_base + (uint32_t)(buf * NACC * BN);
-            int mma_idx = 0; // MMAs issued for this tile
-            for (int st = 0; st < stages_per_tile; st++, g++, ring_next(s, ph, S)) {
-               ok = SOFIE_PROF_WAIT((KIND == kTF32) ? mbar_wait(&conv_bar[s], ph, &abort_flag, status, kStatusWaitConv, g)
-                                                    : mbar_wait(&full_bar[s], ph, &abort_flag, status, kStatusWaitFull, g));
-               if (!ok) break;
-               tc_fence_after();
 #pragma unroll
-               for (int sub = 0; sub < TPS; sub++) {
-                  const uint64_t da = make_smem_desc(smem_u32(a_hi(s, sub)), CB);
-                  const uint64_t db = make_smem_desc(smem_u32(RW ? w_smem + (size_t)(st * TPS + sub) * B_TILE : b_hi(s, sub)), CB);
+            for (int sub = 0; sub < TPS; sub++) {
+               const uint64_t da = make_smem_desc(smem_u32(a_hi(s, sub)), CB);
+               const uint64_t db = make_smem_desc(smem_u32(RW ? w_smem + (size_t)(st * TPS + sub) * B_TILE : b_hi(s, sub)), CB);
 #pragma unroll
-                  for (int k = 0; k < CB / 32; k++) {
-                     const uint64_t koff = (uint64_t)(k * 2); // 32 bytes of K = 2 units of 16 bytes
-                     // the first MMA into each accumulator overwrites it, the later ones add
-                     auto issue = [&](uint64_t adesc, uint64_t bdesc) {
-                        tc_mma<KIND>(d_base + (uint32_t)((mma_idx % NACC) * BN), adesc, bdesc, idesc, mma_idx >= NACC ? 1u : 0u);
-                        mma_idx++;
-                     };
-                     if constexpr (KIND == kTF32) {
-                        const uint64_t dal = make_smem_desc(smem_u32(a_lo(s, sub)), CB);
-                        const uint64_t dbl = make_smem_desc(smem_u32(b_lo(s, sub)), CB);
-                        issue(dal + koff, db + koff);
-                        issue(da + koff, dbl + koff);
-                        issue(da + koff, db + koff);
-                     } else {
-                        issue(da + koff, db + koff);
-                     }
+               for (int k = 0; k < CB / 32; k++) {
+                  const uint64_t koff = (uint64_t)(k * 2); // 32 bytes of K = 2 units of 16 bytes
+                  // the first MMA into each accumulator overwrites it, the later ones add
+                  auto issue = [&](uint64_t adesc, uint64_t bdesc) {
+                     warp_mma<KIND>(d_base + (uint32_t)((mma_idx % NACC) * BN), adesc, bdesc, idesc, mma_idx >= NACC ? 1u : 0u);
+                     mma_idx++;
+                  };
+                  if constexpr (KIND == kTF32) {
+                     const uint64_t dal = make_smem_desc(smem_u32(a_lo(s, sub)), CB);
+                     const uint64_t dbl = make_smem_desc(smem_u32(b_lo(s, sub)), CB);
+                     issue(dal + koff, db + koff);
+                     issue(da + koff, dbl + koff);
+                     issue(da + koff, db + koff);
+                  } else {
+                     issue(da + koff, db + koff);
                   }
                }
-               tc_commit(&empty_bar[s]);
             }
-            if (ok) tc_commit(&tmem_full[buf]);
+            warp_commit(&empty_bar[s]);
          }
+         warp_commit(&tmem_full[buf]);
       }
+      wait.finish(&drain_bar[issuer], &abort_flag, status, kStatusWaitFull, lt);
    } else if (KIND == kTF32 && warp >= 2 + EPI_WARPS) {
       // ---------------- converter warps (kTF32): hi/lo split of each stage ----------------
       if constexpr (KIND == kTF32) {
@@ -547,7 +536,7 @@ umma_conv3x3_patch_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
    extern __shared__ unsigned char smem_raw[];
    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
    __shared__ uint64_t full_bar[kPatchMaxStages], conv_bar[kPatchMaxStages], empty_bar[kPatchMaxStages], tmem_full[NBUF], tmem_empty[NBUF];
-   __shared__ uint64_t w_full, w_conv;
+   __shared__ uint64_t w_full, w_conv, drain_bar[4];
    __shared__ uint32_t tmem_base_holder;
    __shared__ volatile uint32_t abort_flag;
    __shared__ float s_bias[128], s_mult[128];
@@ -581,6 +570,7 @@ umma_conv3x3_patch_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
       }
       mbar_init(&w_full, 1);
       mbar_init(&w_conv, CONV_WARPS * 32);
+      for (int i = 0; i < 4; i++) mbar_init(&drain_bar[i], 1);
       abort_flag = 0;
       fence_mbar_init();
       prefetch_tensormap(&tmX);
@@ -618,59 +608,50 @@ umma_conv3x3_patch_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
       for (int tile = blockIdx.x; tile < tg.num_tiles && ok; tile += gridDim.x, tw.next()) {
          const int n0 = tw.n * tg.tileN, h0 = tw.th * tg.tileH, w0 = tw.tw * tg.tileW;
          for (int grp = 0; grp < G; grp++, g++, ring_next(s, ph, S)) {
-            if (lane == 0) {
-               ok = SOFIE_PROF_WAIT(mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g));
-               if (ok) mbar_expect_tx(&full_bar[s], (uint32_t)(kPatchPixels * PB));
-            }
-            ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+            ok = SOFIE_PROF_WAIT(mbar_wait_warp(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g));
             if (!ok) break;
+            warp_expect_tx(&full_bar[s], (uint32_t)(kPatchPixels * PB));
             // ONE box per stage: PB bytes of channels of every pixel of the haloed patch (channel coordinate = a multiple of
             // PB bytes; rows and columns start at -1: zero fill), written with the swizzle of its row length
-            if (lane == 0) tma_load_4d(slot_hi(s), &tmX, grp * (PB / ES), w0 - 1, h0 - 1, n0, &full_bar[s]);
-            __syncwarp();
+            warp_tma_load_4d(slot_hi(s), &tmX, grp * (PB / ES), w0 - 1, h0 - 1, n0, &full_bar[s]);
          }
       }
    } else if (warp == 1 || warp >= kPatchIssuerB) {
       // ---------------- MMA issuers ----------------
-      // Threads of different warps take the tiles of this CTA in turn (the accumulator buffers go round
-      // with the tile count): while one waits for its barriers and commits, the others keep the tensor
-      // pipe fed, which a single thread cannot -- an MMA costs the thread that issues it more clocks than
-      // it occupies the pipe, and its hand-over work between two tiles leaves the pipe idle.
+      // Different warps take the tiles of this CTA in turn (the accumulator buffers go round with the tile
+      // count): while one waits for its barriers and commits, the others keep the tensor pipe fed, which one
+      // alone cannot: its hand-over work between two tiles leaves the pipe idle.
       const int issuer = warp == 1 ? 0 : warp - kPatchIssuerB + 1;
       const int ni = pl.issuers < NBUF ? pl.issuers : NBUF; // a buffer is never shared by two issuers
-      if (lane == 0 && issuer < ni) {
+      if (issuer < ni) {
          constexpr uint32_t idesc = make_idesc<KIND>(128, BN);
          constexpr uint32_t idesc_wide = make_idesc<KIND>(128, NACC * BN);
-         bool ok = SOFIE_PROF_WAIT((KIND == kTF32) ? mbar_wait(&w_conv, 0, &abort_flag, status, kStatusWaitConv, 0x4000)
-                                                   : mbar_wait(&w_full, 0, &abort_flag, status, kStatusWaitFull, 0x4000));
+         WarpWait wait;
+         wait(KIND == kTF32 ? &w_conv : &w_full, 0);
          tc_fence_after();
-         // The issuing thread is the pacemaker of the whole CTA, so everything that can be is folded
+         // The issuing warp is the pacemaker of the whole CTA, so everything that can be is folded
          // at compile time: each MMA costs it one 32-bit add per descriptor. The address field (bits
          // 0..13, in units of 16 bytes) never carries out of its field.
          const uint64_t db0 = make_smem_desc(smem_u32(w_smem), CBK);
          const uint32_t b_hi_word = (uint32_t)(db0 >> 32), b_lo_word = (uint32_t)db0;
          const uint32_t lo16 = pl.stage_bytes >> 4; // hi -> lo copy of a slot, in 16-byte units
-         int g = 0, lt = 0, s = 0;
+         int lt = 0, s = 0;
          uint32_t ph = 0;
-         for (int tile = blockIdx.x; tile < tg.num_tiles && ok; tile += gridDim.x, lt++) {
+         for (int tile = blockIdx.x; tile < tg.num_tiles; tile += gridDim.x, lt++) {
             const int buf = lt & (NBUF - 1);
             if ((lt & (ni - 1)) != issuer) {
                // The other issuer's tile: step over its stages of the ring, but still see each of them
                // become ready. A parity wait only tells the last two phases of a barrier apart, so a
                // thread that skipped a phase of a slot it shares with the other issuer could take an
                // old completion for the one it waits for.
-               for (int grp = 0; grp < G && ok; grp++, g++, ring_next(s, ph, S))
-                  ok = SOFIE_PROF_WAIT((KIND == kTF32) ? mbar_wait(&conv_bar[s], ph, &abort_flag, status, kStatusWaitConv, g)
-                                                       : mbar_wait(&full_bar[s], ph, &abort_flag, status, kStatusWaitFull, g));
+               for (int grp = 0; grp < G; grp++, ring_next(s, ph, S)) wait(KIND == kTF32 ? &conv_bar[s] : &full_bar[s], ph);
                continue;
             }
-            if (!SOFIE_PROF_WAIT(mbar_wait(&tmem_empty[buf], ((lt / NBUF) & 1) ^ 1, &abort_flag, status, kStatusWaitAccum, 0x2000 + lt))) break;
+            wait(&tmem_empty[buf], ((lt / NBUF) & 1) ^ 1);
             const uint32_t d = tmem_base + (uint32_t)(buf * NACC * BN);
 #pragma unroll
-            for (int grp = 0; grp < G; grp++, g++, ring_next(s, ph, S)) {
-               ok = SOFIE_PROF_WAIT((KIND == kTF32) ? mbar_wait(&conv_bar[s], ph, &abort_flag, status, kStatusWaitConv, g)
-                                                    : mbar_wait(&full_bar[s], ph, &abort_flag, status, kStatusWaitFull, g));
-               if (!ok) break;
+            for (int grp = 0; grp < G; grp++, ring_next(s, ph, S)) {
+               wait(KIND == kTF32 ? &conv_bar[s] : &full_bar[s], ph);
                tc_fence_after();
                // K-major rows of PB bytes in the swizzle TMA wrote them with; the eight pixels of a tile row are one 8-row
                // group, the next group is one PATCH row further (not 8 rows: the swizzle is a function of the absolute
@@ -688,17 +669,18 @@ umma_conv3x3_patch_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
                      const uint32_t b16 = (uint32_t)((tap * CHUNKS + kb / CBK) * (COPIES * B_TILE) + kb % CBK) >> 4;
                      const uint32_t acc = (grp | tap | kk) ? 1u : 0u;
                      if constexpr (KIND == kTF32) {
-                        tc_mma<KIND>(d, adesc(a16), bdesc(b16), idesc_wide, acc);     // hi x [hi | lo]
-                        tc_mma<KIND>(d, adesc(a16 + lo16), bdesc(b16), idesc, 1u);     // lo x hi
+                        warp_mma<KIND>(d, adesc(a16), bdesc(b16), idesc_wide, acc);     // hi x [hi | lo]
+                        warp_mma<KIND>(d, adesc(a16 + lo16), bdesc(b16), idesc, 1u);     // lo x hi
                      } else {
-                        tc_mma<KIND>(d, adesc(a16), bdesc(b16), idesc, acc);
+                        warp_mma<KIND>(d, adesc(a16), bdesc(b16), idesc, acc);
                      }
                   }
                }
-               tc_commit(&empty_bar[s]);
+               warp_commit(&empty_bar[s]);
             }
-            if (ok) tc_commit(&tmem_full[buf]);
+            warp_commit(&tmem_full[buf]);
          }
+         wait.finish(&drain_bar[issuer], &abort_flag, status, kStatusWaitFull, lt);
       }
    } else if (KIND == kTF32 && warp >= 2 + EPI_WARPS && warp < 2 + EPI_WARPS + CONV_WARPS) {
       // ---------------- converter warps (kTF32): hi/lo split, weights once, then each slot ----------------

@@ -358,7 +358,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
    extern __shared__ unsigned char smem_raw[];
    // 1024-byte alignment: the 128B swizzle pattern repeats every 1024 bytes and is address based.
    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-   __shared__ uint64_t full_bar[kGemmMaxStages], conv_bar[kGemmMaxStages], empty_bar[kGemmMaxStages], tmem_full[2], tmem_empty[2];
+   __shared__ uint64_t full_bar[kGemmMaxStages], conv_bar[kGemmMaxStages], empty_bar[kGemmMaxStages], tmem_full[2], tmem_empty[2], drain_bar;
    __shared__ uint32_t tmem_base_holder;
    __shared__ volatile uint32_t abort_flag;
    __shared__ __align__(16) float s_cf[18][64]; // per-warp hand-over of the per-column epilogue constants
@@ -387,6 +387,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
          mbar_init(&tmem_full[b], 1);
          mbar_init(&tmem_empty[b], EPI_WARPS);
       }
+      mbar_init(&drain_bar, 1);
       abort_flag = 0;
       fence_mbar_init();
       prefetch_tensormap(&tmA);
@@ -403,67 +404,61 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
    if (warp == 0) {
       // ---------------- TMA producer ----------------
-      // One thread does all of it: two lanes that issue the two copies, with the hand-over of the wait between them, made a stage 2 to 6 %
+      // One lane does all of it: two lanes that issue the two copies, with the hand-over of the wait between them, made a stage 2 to 6 %
       // longer (4000 x 4096 x 4096 E4M3 56.3 -> 53.0 us)
       griddep_wait(); // A is the previous kernel's output
       int g = 0, s = 0;
       uint32_t ph = 0;
-      bool ok = lane == 0;
+      bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
          const int m0 = (tile / tiles_n) * kBM, n0 = (tile % tiles_n) * BN;
          for (int kb = 0; kb < num_kb; kb++, g++, ring_next(s, ph, S)) {
-            ok = SOFIE_PROF_WAIT(mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g));
+            ok = SOFIE_PROF_WAIT(mbar_wait_warp(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g));
             if (!ok) break;
-            mbar_expect_tx(&full_bar[s], L::kATile + L::kBTile);
-            tma_load_2d(a_hi(s), &tmA, kb * KE, m0, &full_bar[s]);
-            tma_load_2d(b_hi(s), &tmB, kb * KE, n0, &full_bar[s]);
+            warp_expect_tx(&full_bar[s], L::kATile + L::kBTile);
+            warp_tma_load_2d(a_hi(s), &tmA, kb * KE, m0, &full_bar[s]);
+            warp_tma_load_2d(b_hi(s), &tmB, kb * KE, n0, &full_bar[s]);
          }
       }
    } else if (warp == 1) {
       // ---------------- MMA issuer ----------------
-      if (lane == 0) {
-         constexpr uint32_t idesc = make_idesc<KIND>(kBM, BN);
-         int g = 0, u = 0, s = 0;
-         uint32_t ph = 0;
-         bool ok = true;
-         for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-            for (int c = 0; c < units_per_tile && ok; c++, u++) {
-               const int buf = u & 1;
-               if (!SOFIE_PROF_WAIT(mbar_wait(&tmem_empty[buf], ((u >> 1) & 1) ^ 1, &abort_flag, status, kStatusWaitAccum, 0x1000 + u))) {
-                  ok = false;
-                  break;
-               }
+      constexpr uint32_t idesc = make_idesc<KIND>(kBM, BN);
+      int u = 0, s = 0;
+      uint32_t ph = 0;
+      WarpWait wait;
+      for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x) {
+         for (int c = 0; c < units_per_tile; c++, u++) {
+            const int buf = u & 1;
+            wait(&tmem_empty[buf], ((u >> 1) & 1) ^ 1);
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
+            const int kb_end = min(num_kb, (c + 1) * chunk_kb);
+            for (int kb = c * chunk_kb; kb < kb_end; kb++, ring_next(s, ph, S)) {
+               wait(KIND == kTF32 ? &conv_bar[s] : &full_bar[s], ph);
                tc_fence_after();
-               const uint32_t d_tmem = tmem_base + (uint32_t)(buf * BN);
-               const int kb_end = min(num_kb, (c + 1) * chunk_kb);
-               for (int kb = c * chunk_kb; kb < kb_end; kb++, g++, ring_next(s, ph, S)) {
-                  ok = SOFIE_PROF_WAIT((KIND == kTF32) ? mbar_wait(&conv_bar[s], ph, &abort_flag, status, kStatusWaitConv, g)
-                                                       : mbar_wait(&full_bar[s], ph, &abort_flag, status, kStatusWaitFull, g));
-                  if (!ok) break;
-                  tc_fence_after();
-                  const uint64_t da = make_smem_desc(smem_u32(a_hi(s)), kStageK);
-                  const uint64_t db = make_smem_desc(smem_u32(b_hi(s)), kStageK);
+               const uint64_t da = make_smem_desc(smem_u32(a_hi(s)), kStageK);
+               const uint64_t db = make_smem_desc(smem_u32(b_hi(s)), kStageK);
 #pragma unroll
-                  for (int k = 0; k < kStageK / kMmaK; k++) {
-                     // advancing K inside the swizzle row: +32 bytes = +2 in the (>>4) address field
-                     const uint64_t koff = (uint64_t)(k * (kMmaK >> 4));
-                     const uint32_t accumulate = (kb == c * chunk_kb && k == 0) ? 0u : 1u;
-                     if constexpr (KIND == kTF32) {
-                        const uint64_t dal = make_smem_desc(smem_u32(a_lo(s)), kStageK);
-                        const uint64_t dbl = make_smem_desc(smem_u32(b_lo(s)), kStageK);
-                        tc_mma<KIND>(d_tmem, dal + koff, db + koff, idesc, accumulate);
-                        tc_mma<KIND>(d_tmem, da + koff, dbl + koff, idesc, 1);
-                        tc_mma<KIND>(d_tmem, da + koff, db + koff, idesc, 1);
-                     } else {
-                        tc_mma<KIND>(d_tmem, da + koff, db + koff, idesc, accumulate);
-                     }
+               for (int k = 0; k < kStageK / kMmaK; k++) {
+                  // advancing K inside the swizzle row: +32 bytes = +2 in the (>>4) address field
+                  const uint64_t koff = (uint64_t)(k * (kMmaK >> 4));
+                  const uint32_t accumulate = (kb == c * chunk_kb && k == 0) ? 0u : 1u;
+                  if constexpr (KIND == kTF32) {
+                     const uint64_t dal = make_smem_desc(smem_u32(a_lo(s)), kStageK);
+                     const uint64_t dbl = make_smem_desc(smem_u32(b_lo(s)), kStageK);
+                     warp_mma<KIND>(d_tmem, dal + koff, db + koff, idesc, accumulate);
+                     warp_mma<KIND>(d_tmem, da + koff, dbl + koff, idesc, 1);
+                     warp_mma<KIND>(d_tmem, da + koff, db + koff, idesc, 1);
+                  } else {
+                     warp_mma<KIND>(d_tmem, da + koff, db + koff, idesc, accumulate);
                   }
-                  tc_commit(&empty_bar[s]); // the stage is free once these MMAs have read it
                }
-               if (ok) tc_commit(&tmem_full[buf]);
+               warp_commit(&empty_bar[s]); // the stage is free once these MMAs have read it
             }
+            warp_commit(&tmem_full[buf]);
          }
       }
+      wait.finish(&drain_bar, &abort_flag, status, kStatusWaitFull, u);
    } else if (warp >= 2 + EPI_WARPS) {
       // ---------------- converter warps (kTF32): hi / lo split of every stage ----------------
       if constexpr (KIND == kTF32) {
@@ -614,7 +609,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
    constexpr int EPI_WARPS = kGemmEpilogueWarps8;
    extern __shared__ unsigned char smem_raw[];
    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-   __shared__ uint64_t full_bar[S], empty_bar[S], tmem_full[2], tmem_empty[2];
+   __shared__ uint64_t full_bar[S], empty_bar[S], tmem_full[2], tmem_empty[2], drain_bar;
    __shared__ uint32_t tmem_base_holder;
    __shared__ volatile uint32_t abort_flag;
    __shared__ __align__(16) float s_cf[18][64]; // per-warp hand-over of the per-column epilogue constants
@@ -640,6 +635,7 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
          mbar_init(&tmem_full[b], 1);
          mbar_init(&tmem_empty[b], 2 * EPI_WARPS);
       }
+      mbar_init(&drain_bar, 1);
       abort_flag = 0;
       fence_mbar_init();
       prefetch_tensormap(&tmA);
@@ -660,45 +656,50 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       griddep_wait(); // A is the previous kernel's output
       int g = 0, s = 0;
       uint32_t ph = 0;
-      bool ok = lane == 0;
+      bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
          const int m0 = (tile / tiles_n) * (2 * kBM) + (int)rank * kBM;
          const int n0 = (tile % tiles_n) * kPairBN + (int)rank * kBM;
          for (int kb = 0; kb < num_kb; kb++, g++, ring_next(s, ph, S)) {
-            ok = SOFIE_PROF_WAIT(mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g));
+            ok = SOFIE_PROF_WAIT(mbar_wait_warp(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g));
             if (!ok) break;
-            if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * kPairStageBytes);
+            if (rank == 0) warp_expect_tx(&full_bar[s], 2 * kPairStageBytes);
             const uint32_t full_leader = mapa_shared(smem_u32(&full_bar[s]), 0);
-            tma_load_2d_pair(a_tile(s), &tmA, kb * kStageK, m0, full_leader);
-            tma_load_2d_pair(b_tile(s), &tmB, kb * kStageK, n0, full_leader);
+            warp_tma_load_2d_pair(a_tile(s), &tmA, kb * kStageK, m0, full_leader);
+            warp_tma_load_2d_pair(b_tile(s), &tmB, kb * kStageK, n0, full_leader);
          }
       }
    } else if (warp == 1) {
       // ---------------- MMA issuer (leader CTA only) ----------------
-      if (lane == 0 && rank == 0) {
+      if (rank == 0) {
          constexpr uint32_t idesc = make_idesc<KIND>(2 * kBM, kPairBN);
-         int g = 0, u = 0, s = 0;
+         int u = 0, s = 0;
          uint32_t ph = 0;
-         bool ok = true;
-         for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, u++) {
+         WarpWait wait;
+         for (int tile = pair; tile < num_tiles; tile += num_pairs, u++) {
             const int buf = u & 1;
-            if (!SOFIE_PROF_WAIT(mbar_wait(&tmem_empty[buf], ((u >> 1) & 1) ^ 1, &abort_flag, status, kStatusWaitAccum, 0x1000 + u))) break;
+            wait(&tmem_empty[buf], ((u >> 1) & 1) ^ 1);
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + (uint32_t)(buf * kPairBN);
-            for (int kb = 0; kb < num_kb; kb++, g++, ring_next(s, ph, S)) {
-               ok = SOFIE_PROF_WAIT(mbar_wait(&full_bar[s], ph, &abort_flag, status, kStatusWaitFull, g));
-               if (!ok) break;
+            for (int kb = 0; kb < num_kb; kb++, ring_next(s, ph, S)) {
+               wait(&full_bar[s], ph);
                tc_fence_after();
                const uint64_t da = make_smem_desc(smem_u32(a_tile(s)), kStageK);
                const uint64_t db = make_smem_desc(smem_u32(b_tile(s)), kStageK);
 #pragma unroll
                for (int k = 0; k < kStageK / kMmaK; k++) {
                   const uint64_t koff = (uint64_t)(k * (kMmaK >> 4));
-                  tc_mma_pair<KIND>(d_tmem, da + koff, db + koff, idesc, (kb == 0 && k == 0) ? 0u : 1u);
+                  warp_mma_pair<KIND>(d_tmem, da + koff, db + koff, idesc, (kb == 0 && k == 0) ? 0u : 1u);
                }
-               tc_commit_pair(&empty_bar[s], 3); // both CTAs' slots are free once these MMAs have read them
+               warp_commit_pair(&empty_bar[s], 3); // both CTAs' slots are free once these MMAs have read them
             }
-            if (ok) tc_commit_pair(&tmem_full[buf], 3);
+            warp_commit_pair(&tmem_full[buf], 3);
+         }
+         if (wait.gave_up) { // what is under way ends before the tensor memory is given back
+            if (lane == 0 && !abort_flag) mbar_give_up(&abort_flag, status, kStatusWaitFull, u);
+            __syncwarp();
+            warp_commit_pair(&drain_bar, 1);
+            for (int n = 0; !__any_sync(0xFFFFFFFFu, mbar_try_wait(&drain_bar, 0)) && ++n < 4096;) {}
          }
       }
    } else {
@@ -773,7 +774,7 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
    constexpr int kPieceBytes = kBM * 32 * 4;
    extern __shared__ unsigned char smem_raw[];
    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-   __shared__ uint64_t full_bar[kGemmMaxStages], empty_bar[kGemmMaxStages], tmem_full;
+   __shared__ uint64_t full_bar[kGemmMaxStages], empty_bar[kGemmMaxStages], tmem_full, drain_bar;
    __shared__ uint32_t tmem_base_holder;
    __shared__ volatile uint32_t abort_flag;
    __shared__ __align__(16) float s_cf[18][64];
@@ -793,6 +794,7 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
          mbar_init(&empty_bar[s], 1);
       }
       mbar_init(&tmem_full, 1);
+      mbar_init(&drain_bar, 1);
       abort_flag = 0;
       fence_mbar_init();
       prefetch_tensormap(&tmA);
@@ -813,32 +815,30 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       griddep_wait(); // A is the previous kernel's output
       int s = 0;
       uint32_t ph = 0;
-      for (int kb = kb0; lane == 0 && kb < kb1; kb++, ring_next(s, ph, S)) {
-         if (!mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, kb)) break;
-         mbar_expect_tx(&full_bar[s], L::kATile + L::kBTile);
-         tma_load_2d(a_tile(s), &tmA, kb * kStageK, m0, &full_bar[s]);
-         tma_load_2d(b_tile(s), &tmB, kb * kStageK, n0, &full_bar[s]);
+      for (int kb = kb0; kb < kb1; kb++, ring_next(s, ph, S)) {
+         if (!mbar_wait_warp(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, kb)) break;
+         warp_expect_tx(&full_bar[s], L::kATile + L::kBTile);
+         warp_tma_load_2d(a_tile(s), &tmA, kb * kStageK, m0, &full_bar[s]);
+         warp_tma_load_2d(b_tile(s), &tmB, kb * kStageK, n0, &full_bar[s]);
       }
    } else if (warp == 1) {
-      if (lane == 0) {
-         constexpr uint32_t idesc = make_idesc<KIND>(kBM, BN);
-         int s = 0;
-         uint32_t ph = 0;
-         bool ok = true;
-         for (int kb = kb0; kb < kb1; kb++, ring_next(s, ph, S)) {
-            ok = mbar_wait(&full_bar[s], ph, &abort_flag, status, kStatusWaitFull, kb);
-            if (!ok) break;
-            tc_fence_after();
-            const uint64_t da = make_smem_desc(smem_u32(a_tile(s)), kStageK), db = make_smem_desc(smem_u32(b_tile(s)), kStageK);
+      constexpr uint32_t idesc = make_idesc<KIND>(kBM, BN);
+      int s = 0;
+      uint32_t ph = 0;
+      WarpWait wait;
+      for (int kb = kb0; kb < kb1; kb++, ring_next(s, ph, S)) {
+         wait(&full_bar[s], ph);
+         tc_fence_after();
+         const uint64_t da = make_smem_desc(smem_u32(a_tile(s)), kStageK), db = make_smem_desc(smem_u32(b_tile(s)), kStageK);
 #pragma unroll
-            for (int k = 0; k < kStageK / kMmaK; k++) {
-               const uint64_t koff = (uint64_t)(k * (kMmaK >> 4));
-               tc_mma<KIND>(tmem_base, da + koff, db + koff, idesc, (kb == kb0 && k == 0) ? 0u : 1u);
-            }
-            tc_commit(&empty_bar[s]);
+         for (int k = 0; k < kStageK / kMmaK; k++) {
+            const uint64_t koff = (uint64_t)(k * (kMmaK >> 4));
+            warp_mma<KIND>(tmem_base, da + koff, db + koff, idesc, (kb == kb0 && k == 0) ? 0u : 1u);
          }
-         if (ok) tc_commit(&tmem_full);
+         warp_commit(&empty_bar[s]);
       }
+      warp_commit(&tmem_full);
+      wait.finish(&drain_bar, &abort_flag, status, kStatusWaitFull, kb1);
    } else {
       mbar_wait(&tmem_full, 0, &abort_flag, status, kStatusWaitAccum, 0x3000);
       tc_fence_after();

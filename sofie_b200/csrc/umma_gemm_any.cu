@@ -217,7 +217,7 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
    extern __shared__ unsigned char smem_raw[];
    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
    float *tile_out = reinterpret_cast<float *>(smem);
-   __shared__ uint64_t full_bar[kAnyMaxStages], empty_bar[kAnyMaxStages], tmem_full[2], tmem_empty[2];
+   __shared__ uint64_t full_bar[kAnyMaxStages], empty_bar[kAnyMaxStages], tmem_full[2], tmem_empty[2], drain_bar;
    __shared__ uint32_t tmem_base_holder;
    __shared__ volatile uint32_t abort_flag, doubt_flag; // doubt_flag: a sum of this CTA's tile is doubtful
 
@@ -244,6 +244,7 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
          mbar_init(&tmem_full[b], 1);
          mbar_init(&tmem_empty[b], kAnyWorkers / 32);
       }
+      mbar_init(&drain_bar, 1);
       abort_flag = 0;
       doubt_flag = 0;
       fence_mbar_init();
@@ -354,25 +355,21 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
          workers_sync(); // the tile has been read: its place is the stages' again
          if (threadIdx.x == 0) doubt_flag = 0; // set again behind the next tile's first workers_sync
       }
-   } else if (lane == 0) {
+   } else {
       // ---------------- MMA issuer ----------------
       constexpr uint32_t idesc_wide = make_idesc<kBF16>(kAnyBM, 2 * BN), idesc = make_idesc<kBF16>(kAnyBM, BN);
-      int s = 0, u = 0, g = 0;
+      int s = 0, u = 0;
       uint32_t ph = 0;
-      bool ok = true;
-      for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
-         for (int kc = 0; kc < kbn && ok; kc += unit_stages, u++) {
+      WarpWait wait;
+      for (int tile = tile0; tile < num_tiles; tile += tile_step) {
+         for (int kc = 0; kc < kbn; kc += unit_stages, u++) {
             const int buf = u & 1;
-            if (!SOFIE_PROF_WAIT(mbar_wait(&tmem_empty[buf], ((u >> 1) & 1) ^ 1, &abort_flag, status, kStatusWaitAccum, 0x1000 + u))) {
-               ok = false;
-               break;
-            }
+            wait(&tmem_empty[buf], ((u >> 1) & 1) ^ 1);
             tc_fence_after();
             const uint32_t d_tmem = tmem_base + (uint32_t)(buf * 2 * BN);
             const int kce = min(kbn, kc + unit_stages);
-            for (int kb = kc; kb < kce; kb++, g++, ring_next(s, ph, L::kStages)) {
-               ok = SOFIE_PROF_WAIT(mbar_wait(&full_bar[s], ph, &abort_flag, status, kStatusWaitConv, g));
-               if (!ok) break;
+            for (int kb = kc; kb < kce; kb++, ring_next(s, ph, L::kStages)) {
+               wait(&full_bar[s], ph);
                tc_fence_after();
                const uint64_t da0 = make_smem_desc(smem_u32(a_part(s, 0)), kAnyRow), da1 = make_smem_desc(smem_u32(a_part(s, 1)), kAnyRow);
                const uint64_t da2 = make_smem_desc(smem_u32(a_part(s, 2)), kAnyRow), db0 = make_smem_desc(smem_u32(b_part(s, 0)), kAnyRow);
@@ -380,17 +377,18 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
 #pragma unroll
                for (int k = 0; k < 2; k++) {
                   const uint64_t koff = (uint64_t)(2 * k);
-                  tc_mma<kBF16>(d_tmem, da0 + koff, db0 + koff, idesc_wide, (kb == kc && k == 0) ? 0u : 1u); // and the second part of B behind it
-                  tc_mma<kBF16>(d_tmem + BN, da1 + koff, db0 + koff, idesc, 1);
-                  tc_mma<kBF16>(d_tmem + BN, da1 + koff, db1 + koff, idesc, 1);
-                  tc_mma<kBF16>(d_tmem + BN, da0 + koff, db2 + koff, idesc, 1);
-                  tc_mma<kBF16>(d_tmem + BN, da2 + koff, db0 + koff, idesc, 1);
+                  warp_mma<kBF16>(d_tmem, da0 + koff, db0 + koff, idesc_wide, (kb == kc && k == 0) ? 0u : 1u); // and the second part of B behind it
+                  warp_mma<kBF16>(d_tmem + BN, da1 + koff, db0 + koff, idesc, 1);
+                  warp_mma<kBF16>(d_tmem + BN, da1 + koff, db1 + koff, idesc, 1);
+                  warp_mma<kBF16>(d_tmem + BN, da0 + koff, db2 + koff, idesc, 1);
+                  warp_mma<kBF16>(d_tmem + BN, da2 + koff, db0 + koff, idesc, 1);
                }
-               tc_commit(&empty_bar[s]);
+               warp_commit(&empty_bar[s]);
             }
-            if (ok) tc_commit(&tmem_full[buf]);
+            warp_commit(&tmem_full[buf]);
          }
       }
+      wait.finish(&drain_bar, &abort_flag, status, kStatusWaitConv, u);
    }
    SOFIE_PROF_REPORT(warp < kAnyWorkers / 32 ? "worker" : "mma");
    if (S > 1) {
