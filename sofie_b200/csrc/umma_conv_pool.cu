@@ -29,8 +29,7 @@
 //
 // Roles (21 warps, one persistent CTA per SM): warp 0 TMA producer; warps 1, 18, 19, 20 MMA issuers, one per
 // window position (an MMA of 64 columns occupies the tensor core for 48 clocks, its 6 KB of operands at 128
-// bytes per clock, but costs the thread that issues it 80 to 90: four threads issuing side by side keep
-// the pipe full, and all four work on the same tile, so a tile finishes as early as it can); warps 2..17
+// bytes per clock; all four work on the same tile, so a tile finishes as early as it can); warps 2..17
 // epilogue in two groups of eight that take the tiles alternately (group 0 drains TMEM buffer 0 while group 1
 // drains buffer 1: the latency of one tile's TMEM reads hides behind the other's arithmetic), two warps per
 // lane quarter, 32 channels each. Every wait is bounded (umma::mbar_wait).
@@ -99,14 +98,22 @@ struct PoolConvParams {
    uint8_t *Y;            // [N][H/2][W/2][Cout]
 };
 
-// Requantisation to a zero point of 0: q = clamp(rne(acc * mult), 0, 255) is ONE conversion with round-to-nearest-even and
-// saturation to the uint8 range (the lower bound 0 is also the Relu of a quantised value, so `relu` changes nothing here).
-// Same value as requant_u8(acc, mult, 0, relu), three instructions instead of seven.
-__device__ __forceinline__ uint32_t requant_u8_zp0(int acc, float mult)
+// Requantisation to a zero point of 0, four values at a time: q = clamp(rne(acc * mult), 0, 255) (the lower bound 0 is also the Relu of a
+// quantised value, so `relu` changes nothing here). What bounds these epilogues is the ALU pipe, half as wide as the FMA pipe, and the
+// conversions between integers and floats are its work. So they are done by multiplications: a product scaled by 2^-149, the smallest
+// subnormal, is rounded to nearest even to an integer in its bits, and cvt.pack saturates and packs two of them; and an integer in [0, 2^23)
+// read as a float is itself times 2^-149. The product before the rounding is that of requant_u8(), scaled by a power of two: exact while
+// it is not subnormal, far below 0.5 then. (5 ALU instructions a value, the four-way maximum among them, became 2.5: first layer of 16384 images
+// 332 -> 292 us.)
+constexpr float kTwo100 = 1.2676506002282294e30f;   // 2^100
+constexpr float kTwoM100 = 7.888609052210118e-31f;  // 2^-100
+constexpr float kLargestMult = 1048576.f;           // multipliers up to here stay finite times 2^100
+__device__ __forceinline__ uint32_t pack4_u8(const float (&p)[4]) // of products times 2^-149
 {
-   uint32_t q;
-   asm("cvt.rni.sat.u8.f32 %0, %1;" : "=r"(q) : "f"(__fmul_rn(__int2float_rn(acc), mult)));
-   return q;
+   uint32_t w;
+   asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(__float_as_int(p[3])), "r"(__float_as_int(p[2])), "r"(0));
+   asm("cvt.pack.sat.u8.s32.b32 %0, %1, %2, %3;" : "=r"(w) : "r"(__float_as_int(p[1])), "r"(__float_as_int(p[0])), "r"(w));
+   return w;
 }
 
 // The epilogue of both kernels of this file: the sixteen epilogue warps form NBUF groups that take the tiles in turn,
@@ -115,7 +122,8 @@ __device__ __forceinline__ uint32_t requant_u8_zp0(int acc, float mult)
 // channels). More buffers in flight hide more of the fixed latency of a tile's trip through the barriers, which is
 // what bounds a kernel whose tiles carry little arithmetic. lane = pooling window; its four accumulators lie BN
 // columns apart.
-template <int BN, int NBUF>
+// SMALL: sums without bias lie in (-2^23, 2^23).
+template <int BN, int NBUF, bool SMALL>
 __device__ __forceinline__ void pool_epilogue_warp(const PoolConvParams &p, const float *s_mult, const int *s_qbias, bool pool_first,
                                                    uint32_t tmem_base, uint64_t *tmem_full, uint64_t *tmem_empty,
                                                    volatile uint32_t *abort_flag, uint32_t *status, int warp, int lane)
@@ -143,50 +151,75 @@ __device__ __forceinline__ void pool_epilogue_warp(const PoolConvParams &p, cons
          const int c0 = half * CW + piece * 16;
          if (c0 >= p.Cout) break;
          const uint32_t t_row = tmem_base + ((uint32_t)lane_base << 16) + (uint32_t)(buf * 4 * BN + c0);
-         int q[16];
+         uint32_t w4[4];
          if (pool_first) {
-            uint32_t a[16], b[16];
-            tmem_ld_32x16(t_row, a);
-            tmem_ld_32x16(t_row + BN, b);
-            tmem_ld_wait();
+            uint32_t a[16], b[16], c[16];
+            if (SMALL && p.y_zp == 0 && p.qbias == nullptr) {
+               tmem_ld_32x16(t_row, a);
+               tmem_ld_32x16(t_row + BN, b);
+               tmem_ld_32x16(t_row + 2 * BN, c);
+               tmem_ld_wait();
 #pragma unroll
-            for (int j = 0; j < 16; j++) a[j] = (uint32_t)max((int)a[j], (int)b[j]);
-            uint32_t c[16];
-            tmem_ld_32x16(t_row + 2 * BN, b);
-            tmem_ld_32x16(t_row + 3 * BN, c);
-            tmem_ld_wait();
-            // four channels at a time: their multipliers (and biases) are one 16-byte shared load each (c0 is a multiple of 16)
-            // four copies of the loop, chosen by two uniform branches outside it: a layer without bias does not pay an addition
-            // per value, and the choice between the two requantisation forms is not made (or both computed) per value
-            auto finish = [&](auto with_bias, auto zero_point_0) {
+               for (int j = 0; j < 16; j++) a[j] = (uint32_t)__vimax3_s32((int)a[j], (int)b[j], (int)c[j]);
+               tmem_ld_32x16(t_row + 3 * BN, b);
+               tmem_ld_wait();
 #pragma unroll
                for (int j4 = 0; j4 < 4; j4++) {
-                  const float4 m4 = reinterpret_cast<const float4 *>(s_mult + c0)[j4];
+                  const float4 m4 = reinterpret_cast<const float4 *>(s_mult + 64 + c0)[j4]; // times 2^100
                   const float mu[4] = {m4.x, m4.y, m4.z, m4.w};
-                  int bi[4] = {0, 0, 0, 0};
-                  if constexpr (decltype(with_bias)::value) {
-                     const int4 b4 = reinterpret_cast<const int4 *>(s_qbias + c0)[j4];
-                     bi[0] = b4.x; bi[1] = b4.y; bi[2] = b4.z; bi[3] = b4.w;
-                  }
+                  float v[4];
 #pragma unroll
-                  for (int t = 0; t < 4; t++) {
-                     const int j = 4 * j4 + t;
-                     int m = __vimax3_s32((int)a[j], (int)b[j], (int)c[j]);
-                     if constexpr (decltype(with_bias)::value) m += bi[t];
-                     if constexpr (decltype(zero_point_0)::value) q[j] = (int)requant_u8_zp0(m, mu[t]);
-                     else q[j] = requant_u8(m, mu[t], p.y_zp, p.relu);
-                  }
+                  for (int t = 0; t < 4; t++)
+                     v[t] = __fmul_rn(__fmul_rn(__int_as_float(__vimax3_s32((int)a[4 * j4 + t], (int)b[4 * j4 + t], 0)), mu[t]), kTwoM100);
+                  w4[j4] = pack4_u8(v);
                }
-            };
-            if (p.y_zp == 0) {
-               if (p.qbias != nullptr) finish(std::true_type{}, std::true_type{});
-               else finish(std::false_type{}, std::true_type{});
             } else {
-               if (p.qbias != nullptr) finish(std::true_type{}, std::false_type{});
-               else finish(std::false_type{}, std::false_type{});
+               tmem_ld_32x16(t_row, a);
+               tmem_ld_32x16(t_row + BN, b);
+               tmem_ld_wait();
+#pragma unroll
+               for (int j = 0; j < 16; j++) a[j] = (uint32_t)max((int)a[j], (int)b[j]);
+               tmem_ld_32x16(t_row + 2 * BN, b);
+               tmem_ld_32x16(t_row + 3 * BN, c);
+               tmem_ld_wait();
+               // four channels at a time: their multipliers (and biases) are one 16-byte shared load each (c0 is a multiple of 16)
+               // four copies of the loop, chosen by two uniform branches outside it: a layer without bias does not pay an addition
+               // per value, and the choice between the two requantisation forms is not made (or both computed) per value
+               auto finish = [&](auto with_bias, auto zero_point_0) {
+#pragma unroll
+                  for (int j4 = 0; j4 < 4; j4++) {
+                     const float4 m4 = reinterpret_cast<const float4 *>(s_mult + c0)[j4];
+                     const float mu[4] = {m4.x, m4.y, m4.z, m4.w};
+                     int bi[4] = {0, 0, 0, 0};
+                     if constexpr (decltype(with_bias)::value) {
+                        const int4 b4 = reinterpret_cast<const int4 *>(s_qbias + c0)[j4];
+                        bi[0] = b4.x; bi[1] = b4.y; bi[2] = b4.z; bi[3] = b4.w;
+                     }
+                     float v[4];
+                     uint32_t w = 0;
+#pragma unroll
+                     for (int t = 0; t < 4; t++) {
+                        const int j = 4 * j4 + t;
+                        int m = __vimax3_s32((int)a[j], (int)b[j], (int)c[j]);
+                        if constexpr (decltype(with_bias)::value) m += bi[t];
+                        if constexpr (decltype(zero_point_0)::value) v[t] = __fmul_rn(__fmul_rn(__int2float_rn(m), mu[t]), __int_as_float(1));
+                        else w |= (uint32_t)requant_u8(m, mu[t], p.y_zp, p.relu) << (8 * t);
+                     }
+                     if constexpr (decltype(zero_point_0)::value) w = pack4_u8(v);
+                     w4[j4] = w;
+                  }
+               };
+               if (p.y_zp == 0) {
+                  if (p.qbias != nullptr) finish(std::true_type{}, std::true_type{});
+                  else finish(std::false_type{}, std::true_type{});
+               } else {
+                  if (p.qbias != nullptr) finish(std::true_type{}, std::false_type{});
+                  else finish(std::false_type{}, std::false_type{});
+               }
             }
          } else {
             // a negative multiplier reverses the order: requantise the four pixels, then take the maximum
+            int q[16];
 #pragma unroll
             for (int pos = 0; pos < 4; pos++) {
                uint32_t a[16];
@@ -198,11 +231,10 @@ __device__ __forceinline__ void pool_epilogue_warp(const PoolConvParams &p, cons
                   q[j] = pos ? max(q[j], v) : v;
                }
             }
-         }
-         uint32_t w4[4];
 #pragma unroll
-         for (int j = 0; j < 4; j++)
-            w4[j] = (uint32_t)q[4 * j] | ((uint32_t)q[4 * j + 1] << 8) | ((uint32_t)q[4 * j + 2] << 16) | ((uint32_t)q[4 * j + 3] << 24);
+            for (int j = 0; j < 4; j++)
+               w4[j] = (uint32_t)q[4 * j] | ((uint32_t)q[4 * j + 1] << 8) | ((uint32_t)q[4 * j + 2] << 16) | ((uint32_t)q[4 * j + 3] << 24);
+         }
          *reinterpret_cast<uint4 *>(yrow + c0) = make_uint4(w4[0], w4[1], w4[2], w4[3]);   // Cout % 16 == 0: aligned
       }
       tc_fence_before();
@@ -226,7 +258,7 @@ umma_qconv3x3_pool_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
    constexpr uint32_t TMEM_COLS = 8 * BN;                   // two buffers of four accumulators
    extern __shared__ unsigned char smem_raw[];
    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-   __shared__ uint64_t full_bar[kPoolMaxStages], empty_bar[kPoolMaxStages], tmem_full[2], tmem_empty[2], w_full;
+   __shared__ uint64_t full_bar[kPoolMaxStages], empty_bar[kPoolMaxStages], tmem_full[2], tmem_empty[2], w_full, drain_bar[4];
    __shared__ uint32_t tmem_base_holder;
    __shared__ volatile uint32_t abort_flag;
    __shared__ __align__(16) float s_mult[64];
@@ -239,7 +271,7 @@ umma_qconv3x3_pool_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
       const bool in = c < p.Cout;
       s_mult[c] = in ? p.mult[c] : 0.f;
       s_qbias[c] = (in && p.qbias) ? p.qbias[c] : 0;
-      if (in && !(p.mult[c] >= 0.f)) negative_mult = 1;
+      if (in && !(p.mult[c] >= 0.f && p.mult[c] <= kLargestMult)) negative_mult = 1; // or too large for the short form
    }
    const int S = p.stages;
    unsigned char *w_smem = smem;
@@ -255,6 +287,7 @@ umma_qconv3x3_pool_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
          mbar_init(&tmem_empty[b], kPoolEpiWarps / 2);
       }
       mbar_init(&w_full, 1);
+      for (int i = 0; i < 4; i++) mbar_init(&drain_bar[i], 1);
       abort_flag = 0;
       fence_mbar_init();
       prefetch_tensormap(&tmX);
@@ -286,71 +319,61 @@ umma_qconv3x3_pool_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
       for (int tile = blockIdx.x, g = 0; tile < p.num_tiles && ok; tile += gridDim.x, g++, ring_next(s, ph, S)) {
          const int n = tile / per_image, rem = tile - n * per_image;
          const int h0 = (rem / p.tilesW) * kPoolTileH, w0 = (rem % p.tilesW) * kPoolTileW;
-         if (lane == 0) {
-            ok = mbar_wait(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g);
-            if (ok) mbar_expect_tx(&full_bar[s], (uint32_t)(2 * kPoolBoxPixels * PB));
-         }
-         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+         ok = mbar_wait_warp(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g);
          if (!ok) break;
-         if (lane < 2) {
-            // box b = 0: patch columns w0-1, w0+1, ... (odd image columns, from pair w0/2 - 1);
-            // box b = 1: patch columns w0, w0+2, ...   (even image columns, from pair w0/2).
-            // A box row is one pixel with all its PB bytes of channels, written with the swizzle of that row length.
-            const int b = lane;
-            asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-                         ::"r"(smem_u32(slots + (size_t)s * p.stage_bytes + (size_t)b * BOX_STRIDE)),
-                         "l"(&tmX), "r"(0), "r"(b ? 0 : 1), "r"(b ? w0 / 2 : w0 / 2 - 1), "r"(h0 - 1), "r"(n),
-                         "r"(smem_u32(&full_bar[s]))
-                         : "memory");
-         }
-         __syncwarp();
+         warp_expect_tx(&full_bar[s], (uint32_t)(2 * kPoolBoxPixels * PB));
+         // box 0: patch columns w0-1, w0+1, ... (odd image columns, from pair w0/2 - 1);
+         // box 1: patch columns w0, w0+2, ...   (even image columns, from pair w0/2).
+         // A box row is one pixel with all its PB bytes of channels, written with the swizzle of that row length.
+         unsigned char *slot = slots + (size_t)s * p.stage_bytes;
+         warp_tma_load_5d(slot, &tmX, 0, 1, w0 / 2 - 1, h0 - 1, n, &full_bar[s]);
+         warp_tma_load_5d(slot + BOX_STRIDE, &tmX, 0, 0, w0 / 2, h0 - 1, n, &full_bar[s]);
       }
    } else if (warp == 1 || warp >= kPoolFirstExtraIssuer) {
-      // ---------------- MMA issuers: thread `pos` issues the nine taps of window position pos of every tile ----------------
+      // ---------------- MMA issuers: warp `pos` issues the nine taps of window position pos of every tile ----------------
       const int pos = warp == 1 ? 0 : warp - kPoolFirstExtraIssuer + 1;
-      if (lane == 0) {
-         constexpr uint32_t idesc = make_idesc<kI8>(128, BN);
-         bool ok = mbar_wait(&w_full, 0, &abort_flag, status, kStatusWaitFull, 0x4000);
+      constexpr uint32_t idesc = make_idesc<kI8>(128, BN);
+      WarpWait wait;
+      wait(&w_full, 0);
+      tc_fence_after();
+      const uint64_t db0 = make_smem_desc(smem_u32(w_smem), CBK);
+      const uint32_t b_hi_word = (uint32_t)(db0 >> 32), b_lo_word = (uint32_t)db0;
+      // start of this position's operand for tap (r,s), in 16-byte units: box (dx+s) & 1, patch row dy+r, column (dx+s) >> 1
+      uint32_t a_off[9];
+#pragma unroll
+      for (int tap = 0; tap < 9; tap++) {
+         const int row = (pos >> 1) + tap / 3, e = (pos & 1) + tap % 3;
+         a_off[tap] = (uint32_t)((e & 1) * BOX_STRIDE + (row * kPoolCols + (e >> 1)) * PB) >> 4;
+      }
+      int s = 0, lt = 0;
+      uint32_t ph = 0;
+      for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, lt++, ring_next(s, ph, S)) {
+         const int buf = lt & 1;
+         wait(&full_bar[s], ph);
+         wait(&tmem_empty[buf], ((lt >> 1) & 1) ^ 1);
          tc_fence_after();
-         const uint64_t db0 = make_smem_desc(smem_u32(w_smem), CBK);
-         const uint32_t b_hi_word = (uint32_t)(db0 >> 32), b_lo_word = (uint32_t)db0;
-         // start of this position's operand for tap (r,s), in 16-byte units: box (dx+s) & 1, patch row dy+r, column (dx+s) >> 1
-         uint32_t a_off[9];
+         const uint32_t d = tmem_base + (uint32_t)(buf * 4 * BN + pos * BN);
+         // swizzled K-major rows of PB bytes; the eight windows of a tile row are eight consecutive pixels of a box row, the
+         // next tile row of windows is two patch rows further (make_smem_desc_rows: any start row, any group stride)
+         const uint64_t da0 = make_smem_desc_rows(smem_u32(slots + (size_t)s * p.stage_bytes), PB, 2 * kPoolCols * PB);
+         const uint32_t a_hi_word = (uint32_t)(da0 >> 32), a_lo_word = (uint32_t)da0;
 #pragma unroll
          for (int tap = 0; tap < 9; tap++) {
-            const int row = (pos >> 1) + tap / 3, e = (pos & 1) + tap % 3;
-            a_off[tap] = (uint32_t)((e & 1) * BOX_STRIDE + (row * kPoolCols + (e >> 1)) * PB) >> 4;
-         }
-         int s = 0, lt = 0;
-         uint32_t ph = 0;
-         for (int tile = blockIdx.x; tile < p.num_tiles && ok; tile += gridDim.x, lt++, ring_next(s, ph, S)) {
-            const int buf = lt & 1;
-            ok = mbar_wait(&full_bar[s], ph, &abort_flag, status, kStatusWaitFull, lt);
-            if (!ok) break;
-            if (!mbar_wait(&tmem_empty[buf], ((lt >> 1) & 1) ^ 1, &abort_flag, status, kStatusWaitAccum, 0x2000 + lt)) break;
-            tc_fence_after();
-            const uint32_t d = tmem_base + (uint32_t)(buf * 4 * BN + pos * BN);
-            // swizzled K-major rows of PB bytes; the eight windows of a tile row are eight consecutive pixels of a box row, the
-            // next tile row of windows is two patch rows further (make_smem_desc_rows: any start row, any group stride)
-            const uint64_t da0 = make_smem_desc_rows(smem_u32(slots + (size_t)s * p.stage_bytes), PB, 2 * kPoolCols * PB);
-            const uint32_t a_hi_word = (uint32_t)(da0 >> 32), a_lo_word = (uint32_t)da0;
 #pragma unroll
-            for (int tap = 0; tap < 9; tap++) {
-#pragma unroll
-               for (int kk = 0; kk < KPS; kk++) {
-                  const int kb = kk * 32;
-                  const uint32_t b16 = (uint32_t)((tap * CHUNKS + kb / CBK) * B_TILE + kb % CBK) >> 4;
-                  const uint64_t bdesc = ((uint64_t)b_hi_word << 32) | (uint64_t)(b_lo_word + b16);
-                  const uint64_t adesc = ((uint64_t)a_hi_word << 32) | (uint64_t)(a_lo_word + a_off[tap] + (uint32_t)(kk * 2));
-                  tc_mma<kI8>(d, adesc, bdesc, idesc, (tap | kk) ? 1u : 0u);
-               }
+            for (int kk = 0; kk < KPS; kk++) {
+               const int kb = kk * 32;
+               const uint32_t b16 = (uint32_t)((tap * CHUNKS + kb / CBK) * B_TILE + kb % CBK) >> 4;
+               const uint64_t bdesc = ((uint64_t)b_hi_word << 32) | (uint64_t)(b_lo_word + b16);
+               const uint64_t adesc = ((uint64_t)a_hi_word << 32) | (uint64_t)(a_lo_word + a_off[tap] + (uint32_t)(kk * 2));
+               warp_mma<kI8>(d, adesc, bdesc, idesc, (tap | kk) ? 1u : 0u);
             }
-            tc_commit(&empty_bar[s]);
-            tc_commit(&tmem_full[buf]);
          }
+         warp_commit(&empty_bar[s]);
+         warp_commit(&tmem_full[buf]);
       }
+      wait.finish(&drain_bar[pos], &abort_flag, status, kStatusWaitFull, lt);
    } else if (warp < 2 + kPoolEpiWarps) {
-      pool_epilogue_warp<BN, 2>(p, s_mult, s_qbias, pool_first, tmem_base, tmem_full, tmem_empty, &abort_flag, status, warp, lane);
+      pool_epilogue_warp<BN, 2, (288 * KPS * 255 * 128 < 1 << 23)>(p, s_mult, s_qbias, pool_first, tmem_base, tmem_full, tmem_empty, &abort_flag, status, warp, lane);
    }
    tc_fence_before();
    __syncthreads();
@@ -366,19 +389,19 @@ umma_qconv3x3_pool_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
 // First layer (ONE input channel) of the same shape class, on the same tensor-memory pooling: with C = 1 a tap is a
 // single byte, far below the 16 bytes of K a shared-memory operand row needs, so here -- and only here -- the operand is
 // written out: four builder warps (one thread per pooling window) read the window's 4 x 4 input bytes from the staged
-// input rows and store, for each of the four window positions, the 9 taps of that position as one 16-byte operand row
-// (bytes 9..15 zero). K = 32 for 8-bit MMAs: the upper 16 bytes of every row of A and of the weights are ONE shared block
-// of zeros that each descriptor's leading byte offset points at. A tile is four MMAs (128 windows x BN channels x 32),
-// issued by one thread; its epilogue is the one above. The input rows of a tile (34 x 48 bytes: the tile's 18 columns
-// start at byte 15 so that the TMA box starts on a 16-byte boundary of the image row, as the copy engine requires)
+// input rows and store them as they are, one 16-byte operand row. The taps of the four window positions are sixteen-byte rows
+// of weights with zeros where a position does not reach, 4 x BN of them, so that ONE MMA of 4 x BN columns makes all four accumulators:
+// 64 clocks at BN = 32 where four MMAs over the nine taps of each position took 160 and the builders wrote, and permuted, four times as much.
+// K = 32 for 8-bit MMAs: the upper 16 bytes of every row of A and of the weights are ONE shared block
+// of zeros that each descriptor's leading byte offset points at. The epilogue is the one above. The input rows of a tile (34 x 48 bytes: the
+// tile's 18 columns start at byte 15 so that the TMA box starts on a 16-byte boundary of the image row, as the copy engine requires)
 // arrive by one TMA box per tile; out-of-image bytes are the zero fill = the padding value (input zero point 0).
-// Two threads issue (even and odd tiles): a tile's two waits, four MMAs and two commits cost one thread about as long as
-// the tile's epilogue takes, and the thread that issues is the pacemaker of everything behind it.
+// Two warps issue (even and odd tiles): the issuer is the pacemaker of everything behind it.
 //   warp 0 producer | warps 1 and 26 MMA issuers | warps 2..17 epilogue | warps 18..25 operand builders (two groups of four)
 constexpr int kFirstRawPitch = 48;                                  // bytes per staged input row
 constexpr int kFirstRawBytes = kPoolRows * kFirstRawPitch;          // 1632
 constexpr int kFirstRawStride = (kFirstRawBytes + 127) / 128 * 128; // 1664
-constexpr int kFirstABytes = 4 * 2048;                              // four positions x 128 rows x 16 bytes
+constexpr int kFirstABytes = 2048;                                  // 128 rows x 16 bytes
 constexpr int kFirstStages = 4;
 constexpr int kFirstBuilderGroups = 2;   // groups of four builder warps that take the tiles alternately
 constexpr int kFirstThreads = (19 + 4 * kFirstBuilderGroups) * 32;
@@ -393,15 +416,15 @@ umma_qconv3x3_first_pool_kernel(const __grid_constant__ CUtensorMap tmX, const i
    constexpr uint32_t TMEM_COLS = 512;
    extern __shared__ unsigned char smem_raw[];
    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-   // layout: [A slots: S x 8 KB][raw slots: S x 1664][weights: BN x 16][zeros: 2 KB]
+   // layout: [A slots: S x 2 KB][raw slots: S x 1664][weights: 4 x BN x 16][zeros: as much]
    unsigned char *a_slots = smem;
    unsigned char *raw_slots = a_slots + kFirstStages * kFirstABytes;
    unsigned char *w_smem = raw_slots + kFirstStages * kFirstRawStride;
-   unsigned char *zeros = w_smem + 1024;
-   __shared__ uint64_t raw_full[kFirstStages], raw_empty[kFirstStages], a_full[kFirstStages], a_empty[kFirstStages], tmem_full[4], tmem_empty[4];
+   unsigned char *zeros = w_smem + 4 * BN * 16;
+   __shared__ uint64_t raw_full[kFirstStages], raw_empty[kFirstStages], a_full[kFirstStages], a_empty[kFirstStages], tmem_full[4], tmem_empty[4], drain_bar[2];
    __shared__ uint32_t tmem_base_holder;
    __shared__ volatile uint32_t abort_flag;
-   __shared__ __align__(16) float s_mult[64];
+   __shared__ __align__(16) float s_mult[128]; // and behind them the same times 2^100
    __shared__ __align__(16) int s_qbias[64];
 
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -410,15 +433,18 @@ umma_qconv3x3_first_pool_kernel(const __grid_constant__ CUtensorMap tmX, const i
    for (int c = threadIdx.x; c < 64; c += blockDim.x) {
       const bool in = c < p.Cout;
       s_mult[c] = in ? p.mult[c] : 0.f;
+      s_mult[64 + c] = s_mult[c] * kTwo100;
       s_qbias[c] = (in && p.qbias) ? p.qbias[c] : 0;
-      if (in && !(p.mult[c] >= 0.f)) negative_mult = 1;
+      if (in && !(p.mult[c] >= 0.f && p.mult[c] <= kLargestMult)) negative_mult = 1; // or too large for the short form
    }
-   // weights: row n = its nine taps and seven zeros (no-swizzle K-major: 8 rows of 16 bytes per core matrix); zero block
-   for (int i = threadIdx.x; i < BN * 16; i += blockDim.x) {
-      const int n = i >> 4, k = i & 15;
-      w_smem[i] = (n < p.Cout && k < 9) ? (unsigned char)W[n * 9 + k] : 0;
+   // weights: row (position, channel) = the channel's nine taps at the position's place in the window's 4 x 4 bytes (no-swizzle K-major: 8
+   // rows of 16 bytes per core matrix); zero block
+   static_assert(4 * BN * 16 >= kFirstABytes, "the zeros stand for the upper half of either operand");
+   for (int i = threadIdx.x; i < 4 * BN * 16; i += blockDim.x) {
+      const int pos = i / (BN * 16), n = (i >> 4) % BN, r = ((i >> 2) & 3) - (pos >> 1), t = (i & 3) - (pos & 1);
+      w_smem[i] = (n < p.Cout && r >= 0 && r < 3 && t >= 0 && t < 3) ? (unsigned char)W[n * 9 + r * 3 + t] : 0;
+      zeros[i] = 0;
    }
-   for (int i = threadIdx.x; i < 2048 / 4; i += blockDim.x) reinterpret_cast<uint32_t *>(zeros)[i] = 0u;
    if (threadIdx.x == 0) {
       for (int s = 0; s < kFirstStages; s++) {
          mbar_init(&raw_full[s], 1);
@@ -430,6 +456,7 @@ umma_qconv3x3_first_pool_kernel(const __grid_constant__ CUtensorMap tmX, const i
          mbar_init(&tmem_full[b], 1);
          mbar_init(&tmem_empty[b], kPoolEpiWarps / NBUF);
       }
+      for (int i = 0; i < 2; i++) mbar_init(&drain_bar[i], 1);
       abort_flag = 0;
       fence_mbar_init();
       prefetch_tensormap(&tmX);
@@ -448,50 +475,41 @@ umma_qconv3x3_first_pool_kernel(const __grid_constant__ CUtensorMap tmX, const i
    if (warp == 0) {
       // ---------------- TMA producer: the 34 input rows of a tile ----------------
       griddep_wait(); // the input is the previous kernel's output
-      if (lane == 0) {
-         PoolTileWalker tw;
-         tw.init(blockIdx.x, gridDim.x, p.tilesH, p.tilesW);
-         int s = 0;
-         uint32_t ph = 0;
-         for (int tile = blockIdx.x, g = 0; tile < p.num_tiles; tile += gridDim.x, g++, ring_next(s, ph, S), tw.next()) {
-            if (!mbar_wait(&raw_empty[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g)) break;
-            mbar_expect_tx(&raw_full[s], kFirstRawBytes);
-            // box {48 bytes, 34 rows, 1 image} from column w0 - 16 (a 16-byte boundary), row h0 - 1
-            asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-                         ::"r"(smem_u32(raw_slots + (size_t)s * kFirstRawStride)), "l"(&tmX), "r"(tw.tw * kPoolTileW - 16),
-                         "r"(tw.th * kPoolTileH - 1), "r"(tw.n), "r"(smem_u32(&raw_full[s]))
-                         : "memory");
-         }
+      PoolTileWalker tw;
+      tw.init(blockIdx.x, gridDim.x, p.tilesH, p.tilesW);
+      int s = 0;
+      uint32_t ph = 0;
+      for (int tile = blockIdx.x, g = 0; tile < p.num_tiles; tile += gridDim.x, g++, ring_next(s, ph, S), tw.next()) {
+         if (!mbar_wait_warp(&raw_empty[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g)) break;
+         warp_expect_tx(&raw_full[s], kFirstRawBytes);
+         // box {48 bytes, 34 rows, 1 image} from column w0 - 16 (a 16-byte boundary), row h0 - 1
+         warp_tma_load_3d(raw_slots + (size_t)s * kFirstRawStride, &tmX, tw.tw * kPoolTileW - 16, tw.th * kPoolTileH - 1, tw.n, &raw_full[s]);
       }
    } else if (warp == 1 || warp == kFirstIssuerB) {
-      // ---------------- MMA issuers: four MMAs per tile, one per window position; even tiles warp 1, odd tiles warp 22 ----------------
+      // ---------------- MMA issuers: one MMA per tile; even tiles warp 1, odd tiles the last warp ----------------
       // (an even number of operand slots and of TMEM buffers: each of them always meets the same issuer)
-      if (lane == 0) {
-         constexpr uint32_t idesc = make_idesc<kI8>(128, BN);
-         const uint32_t zero_addr = smem_u32(zeros);
-         const uint64_t bdesc = make_smem_desc_noswizzle(smem_u32(w_smem), zero_addr - smem_u32(w_smem), 128);
-         // descriptor of the operand at a_slots (slot 0, position 0); one at `off` bytes further has its address field
-         // (bits 0-13, 16-byte units) larger and its leading byte offset (bits 16-29: the distance to the zero block) smaller
-         const uint64_t da0 = make_smem_desc_noswizzle(smem_u32(a_slots), zero_addr - smem_u32(a_slots), 128);
-         const uint32_t a_hi_word = (uint32_t)(da0 >> 32), a_lo_word = (uint32_t)da0;
-         for (int lt = (warp == 1 ? 0 : 1); blockIdx.x + (long long)lt * gridDim.x < p.num_tiles; lt += 2) {
-            const int s = lt % S, buf = lt % NBUF;
-            if (!mbar_wait(&a_full[s], (uint32_t)(lt / S) & 1u, &abort_flag, status, kStatusWaitFull, lt)) break;
-            if (!mbar_wait(&tmem_empty[buf], (((uint32_t)(lt / NBUF)) & 1u) ^ 1u, &abort_flag, status, kStatusWaitAccum, 0x2000 + lt)) break;
-            tc_fence_after();
-            const uint32_t d = tmem_base + (uint32_t)(buf * 4 * BN);
-            const uint32_t lo_slot = a_lo_word + (uint32_t)(s * (kFirstABytes >> 4)) * (1u - 65536u);
-#pragma unroll
-            for (int pos = 0; pos < 4; pos++) {
-               const uint32_t lo = lo_slot + (uint32_t)(pos * (2048 >> 4)) * (1u - 65536u);
-               tc_mma<kI8>(d + (uint32_t)(pos * BN), ((uint64_t)a_hi_word << 32) | lo, bdesc, idesc, 0u);
-            }
-            tc_commit(&a_empty[s]);
-            tc_commit(&tmem_full[buf]);
-         }
+      constexpr uint32_t idesc = make_idesc<kI8>(128, 4 * BN);
+      const uint32_t zero_addr = smem_u32(zeros);
+      const uint64_t bdesc = make_smem_desc_noswizzle(smem_u32(w_smem), zero_addr - smem_u32(w_smem), 128);
+      // descriptor of the operand in slot 0; one at `off` bytes further has its address field
+      // (bits 0-13, 16-byte units) larger and its leading byte offset (bits 16-29: the distance to the zero block) smaller
+      const uint64_t da0 = make_smem_desc_noswizzle(smem_u32(a_slots), zero_addr - smem_u32(a_slots), 128);
+      const uint32_t a_hi_word = (uint32_t)(da0 >> 32), a_lo_word = (uint32_t)da0;
+      WarpWait wait;
+      for (int lt = (warp == 1 ? 0 : 1); blockIdx.x + (long long)lt * gridDim.x < p.num_tiles; lt += 2) {
+         const int s = lt % S, buf = lt % NBUF;
+         wait(&a_full[s], (uint32_t)(lt / S) & 1u);
+         wait(&tmem_empty[buf], (((uint32_t)(lt / NBUF)) & 1u) ^ 1u);
+         tc_fence_after();
+         const uint32_t d = tmem_base + (uint32_t)(buf * 4 * BN);
+         const uint32_t lo = a_lo_word + (uint32_t)(s * (kFirstABytes >> 4)) * (1u - 65536u);
+         warp_mma<kI8>(d, ((uint64_t)a_hi_word << 32) | lo, bdesc, idesc, 0u);
+         warp_commit(&a_empty[s]);
+         warp_commit(&tmem_full[buf]);
       }
+      wait.finish(&drain_bar[warp == 1 ? 0 : 1], &abort_flag, status, kStatusWaitFull, 0x4000);
    } else if (warp < 2 + kPoolEpiWarps) {
-      pool_epilogue_warp<BN, NBUF>(p, s_mult, s_qbias, pool_first, tmem_base, tmem_full, tmem_empty, &abort_flag, status, warp, lane);
+      pool_epilogue_warp<BN, NBUF, true>(p, s_mult, s_qbias, pool_first, tmem_base, tmem_full, tmem_empty, &abort_flag, status, warp, lane);
    } else {
       // ---------------- operand builders: thread = pooling window (py, px) of the tile ----------------
       // Two groups of four warps take the tiles alternately (the number of slots is even: a slot always meets the same group):
@@ -518,19 +536,7 @@ umma_qconv3x3_first_pool_kernel(const __grid_constant__ CUtensorMap tmX, const i
          __syncwarp();
          if (lane == 0) mbar_arrive(&raw_empty[s]);   // the staged rows are in registers
          if (!mbar_wait(&a_empty[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, 0x7000 + g)) break;
-         unsigned char *a_slot = a_slots + (size_t)s * kFirstABytes + t * 16;
-#pragma unroll
-         for (int pos = 0; pos < 4; pos++) {
-            const int dy = pos >> 1, dx = pos & 1;
-            // taps (r,s) in the order r*3+s: rows dy..dy+2 of the window, columns dx..dx+2
-            // k = 0..3: columns dx, dx+1, dx+2 of window row dy, column dx of row dy+1
-            const uint32_t w0 = __byte_perm(r[dy], r[dy + 1], dx ? 0x5321u : 0x4210u);
-            // k = 4..7: columns dx+1, dx+2 of row dy+1, columns dx, dx+1 of row dy+2
-            const uint32_t w1 = __byte_perm(r[dy + 1], r[dy + 2], dx ? 0x6532u : 0x5421u);
-            // k = 8: column dx+2 of row dy+2; k = 9..15 are zero
-            const uint32_t w2 = (r[dy + 2] >> (8 * (dx + 2))) & 0xffu;
-            *reinterpret_cast<uint4 *>(a_slot + pos * 2048) = make_uint4(w0, w1, w2, 0u);
-         }
+         *reinterpret_cast<uint4 *>(a_slots + (size_t)s * kFirstABytes + t * 16) = make_uint4(r[0], r[1], r[2], r[3]);
          fence_proxy_async();
          __syncwarp();
          if (lane == 0) mbar_arrive(&a_full[s]);
@@ -562,7 +568,7 @@ int launch_first_pool_conv(cudaStream_t s, const ConvGeom &g, const uint8_t *X, 
    uint32_t xbox[3] = {(uint32_t)kFirstRawPitch, (uint32_t)kPoolRows, 1u};
    int rc = make_tensor_map(&tmX, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, X, xdims, xstr, xbox, 0);
    if (rc) return rc;
-   const int smem = kFirstStages * (kFirstABytes + kFirstRawStride) + 1024 + 2048 + 1024;
+   const int smem = kFirstStages * (kFirstABytes + kFirstRawStride) + 2 * 4 * BN * 16 + 1024;
    uint32_t *status = device_status_word(s);
    if (!status) return fail(SOFIE_CUDA_ERR_CUDA, "cannot allocate the device status word");
    const int grid = p.num_tiles < kNumSMs ? p.num_tiles : kNumSMs;

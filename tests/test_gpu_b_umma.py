@@ -534,3 +534,30 @@ def test_gemm_f32_of_operands_split_beforehand(M, N, K, bias):
         off = [float((t[rows].double() - exact[rows]).norm()) for t in (y, chain, plain)]
         assert off[0] <= off[1] * 1.02 and off[2] <= off[1] * 1.02      # K = 64 .. 95: all of them round a handful of times
     assert taken == 4
+
+
+# the form without conversions (zero point 0; one input channel without bias, and 32 with one): multipliers of zero, subnormal and far below one,
+# such that most products are ties, that saturate everything, the largest that stay with it (2^20) and larger ones
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("C,Cout", [(1, 32), (1, 64), (1, 16), (32, 64)])
+def test_qconv_pooled_requantisation_at_its_edges(C, Cout, bias):
+    g = torch.Generator(device="cuda").manual_seed(C + Cout)
+    N, H, W = 3, 64, 32
+    X = torch.randint(0, 256, (N, C, H, W), device="cuda", generator=g, dtype=torch.uint8)
+    X[0] = 255
+    Wt = torch.randint(-128, 128, (Cout, C, 3, 3), device="cuda", generator=g, dtype=torch.int8)
+    Wt[1], Wt[2] = 127, -128                                    # the largest sums there are
+    exact = torch.nn.functional.conv2d(X.double(), Wt.double(), padding=1)
+    b = torch.randint(-2000, 2000, (Cout,), device="cuda", generator=g, dtype=torch.int32) if bias else None
+    if bias:
+        exact = exact + b.double()[:, None, None]
+    for values in ([0.0, 2.0 ** -140, 2.0 ** -126, 1e-30, 2.0 ** -24, 3e-5], [0.5, 0.25, 0.125, 1.5, 0.0625, 2.0 ** -9], [1e-3, 7.3e-4, 255.5 / 291465, 1.0, 2.0 ** 20, 1000.0],
+                   [1e-3, 2.0 ** 20 + 1, 2.0 ** 40, 3e38, 0.0, 0.02]):
+        mult = torch.tensor(values, device="cuda").repeat(Cout // 6 + 1)[:Cout].contiguous()
+        q = (exact.float() * mult[:, None, None]).round().clamp(0, 255)      # one rounding to fp32, then to the nearest even integer
+        ref = torch.nn.functional.max_pool2d(q, 2).permute(0, 2, 3, 1).to(torch.uint8)
+        ops.set_engine(0)
+        y = ops.qlinear_conv2d(X.permute(0, 2, 3, 1).contiguous(), ops.qconv2d_pack_i8(Wt), mult, b, shape=X.shape, pad=(1, 1), relu=True, pool=2,
+                               x_layout=capi.LAYOUT_NHWC, y_layout=capi.LAYOUT_NHWC, w_packed=True, kernel=(3, 3))
+        assert ops.last_engine() == capi.ENGINE_TCGEN05
+        assert torch.equal(y.view(ref.shape), ref)
