@@ -24,20 +24,22 @@
 // - Two scales whose product leaves fp32's range are applied one after the other.
 // Error against float64 (2-norm), N(0,1) operands: 2.1e-7 at 16 and 3.7e-7 at 32 channels, where TF32 parts gave 7.0e-7 and 1.28e-6 (their trailing
 // part is truncated, these are rounded, and the sums take half as many steps); operands of one sign 6.1e-7 and 1.4e-6 (1.05e-6 and 2.4e-6).
-// 8192 images 16 -> 32 at 32 x 32 with MaxPool 490 -> 332 us, 32 -> 64 at 16 x 16 365 -> 209 us; unpooled 2048 x 16 -> 32 165 -> 144 us; one image
+// 8192 images 16 -> 32 at 32 x 32 with MaxPool 490 -> 320 us, 32 -> 64 at 16 x 16 365 -> 187 us; unpooled 2048 x 16 -> 32 165 -> 144 us; one image
 // 4.1 -> 4.0 and 5.5 -> 4.8 us when the kernel has just run, about 1 us more behind others (its instructions come from L2 then). Of the first:
 // channels 2^8 ... 2^40 apart 360; values down to 2^-28 of the largest and below in every patch 403; weights of a channel decayed to 1e-12 425; two
 // passes for every tile 1.5 ms, for images of exp(-r^2 / 8) 2.0, one infinity in each image 2.6 (as chains of FMAs in the epilogue, one scale and no check
 // of single sums, the last four took 20 ms, 10 for the infinities).
 //
-// A tile is 16 x 8 pixels of one image; one TMA box brings its 18 x 10 patch (zero fill outside the image) as fp32 rows; two groups of four
-// converter warps take the patches in turn, find the largest magnitude, split the values and write both parts as K-major swizzled
+// A tile is 16 x 8 pixels of one image; one TMA box brings its 18 x 10 patch (zero fill outside the image) as fp32 rows; two or three groups of
+// four converter warps take the patches in turn, find the largest magnitude, split the values and write both parts as K-major swizzled
 // rows, from which each of the 9 taps is a start address (see the haloed-patch kernel). One MMA multiplies the leading parts of the
 // pixels with [leading | trailing] weights (2 * BN columns), one the trailing parts with the leading weights, into the second BN columns.
 // A TMEM buffer goes back to the issuers as soon as it has been read, before pooling and stores. Pooled tiles are read in the shape that puts
 // a pixel and the one below it in one thread: a third of the shuffles, which wait for the shared-memory pipe the MMAs keep busy (the epilogue
 // set the kernel's time with them: 375 instead of 326 us).
-// Waiting with one lane and a vote, or with test_wait, instead of whole warps on try_wait: 5 to 25 % slower.
+// Waiting with one lane and a vote, or with test_wait, instead of whole warps on try_wait: 5 to 25 % slower. Sixteen epilogue warps on four tiles
+// at 32 columns, or four converter groups: 339 and 342 us; the roles then wait for the shared memory, of which a tile moves 134 KB, 1050 of its
+// 1370 clocks.
 #include "umma.cuh"
 #include "contract.cuh"
 #include <cuda_fp16.h>
@@ -49,11 +51,10 @@ namespace {
 constexpr int kHalfTileH = 16, kHalfTileW = 8;
 constexpr int kHalfPatchH = kHalfTileH + 2, kHalfPatchW = kHalfTileW + 2;
 constexpr int kHalfPatchPixels = kHalfPatchH * kHalfPatchW;
-constexpr int kHalfEpiWarps = 8, kHalfConvGroups = 2, kHalfConvGroupWarps = 4;
-constexpr int kHalfConvWarps = kHalfConvGroups * kHalfConvGroupWarps;
-constexpr int kHalfIssuerB = 2 + kHalfEpiWarps + kHalfConvWarps;
-constexpr int kHalfThreads = (kHalfIssuerB + 1) * 32;
-constexpr int kHalfMaxSlots = 4;
+constexpr int kHalfEpiWarps = 8, kHalfConvGroupWarps = 4;
+constexpr int kHalfCarefulGroups = 2; // groups that convert the careful tiles
+constexpr int kHalfMaxSlots = 6;
+constexpr int kHalfWeightWarps = 8;   // converter warps that prepare the weights
 constexpr int kHalfScales = 16;       // ring of tile scales: more than the tiles between a converter and the epilogue (slots + TMEM buffers)
 constexpr uint32_t kHalfSpread = 28;  // a value may be 2^-28 of the patch's largest (see above)
 constexpr float kHalfTrailing = 2048.f; // trailing parts are held times 2^11
@@ -73,11 +74,19 @@ __host__ __device__ constexpr int half_buffers(int BN) { return 512 / (2 * BN) >
 __host__ __device__ constexpr int half_part_bytes(int C) { return (kHalfPatchPixels * 2 * C + 1023) / 1024 * 1024; } // a patch's leading or trailing parts
 __host__ __device__ constexpr int half_raw_bytes(int C) { return kHalfPatchPixels * 4 * C; }
 __host__ __device__ constexpr int half_weight_bytes(int BN, int C) { return 9 * 2 * BN * 2 * C; }
-// patches in flight as fp32, and as many as parts: four or two, so that a slot always meets the same converter group and the same issuer
-__host__ __device__ constexpr int half_slots(int BN, int C)
-{
-   return 220 * 1024 - half_weight_bytes(BN, C) >= 4 * (half_raw_bytes(C) + 2 * half_part_bytes(C)) ? 4 : 2;
-}
+// Converter groups, which take the patches in turn: a patch's way through one (load, largest magnitude, barrier, split, store) is latency.
+// Patches in flight as fp32, and as many as parts: a multiple of the groups and of the two issuers, so that a slot always meets the same ones.
+__host__ __device__ constexpr int half_room(int BN, int C) { return (220 * 1024 - half_weight_bytes(BN, C)) / (half_raw_bytes(C) + 2 * half_part_bytes(C)); }
+__host__ __device__ constexpr int half_groups(int BN, int C) { return half_room(BN, C) >= 6 ? 3 : 2; }
+__host__ __device__ constexpr int half_slots(int BN, int C) { return half_room(BN, C) >= 6 ? 6 : (half_room(BN, C) >= 4 ? 4 : 2); }
+// slots of one group of careful tiles: the rings of passes and patches below are sized for two
+__host__ __device__ constexpr int half_careful_slots(int BN, int C) { return half_slots(BN, C) >= 4 ? 2 : 1; }
+// Epilogue warps of a tile: with 32 columns four, which read all of them, and the other four take the next tile. (Eight warps with 16 columns
+// each, all of them on every tile, set the kernel's time: 1200 clocks of latency a tile.)
+__host__ __device__ constexpr int half_epilogue_groups(int BN) { return BN == 32 ? 2 : 1; }
+__host__ __device__ constexpr int half_conv_warps(int BN, int C) { return half_groups(BN, C) * kHalfConvGroupWarps; }
+__host__ __device__ constexpr int half_issuer_b(int BN, int C) { return 2 + kHalfEpiWarps + half_conv_warps(BN, C); }
+__host__ __device__ constexpr int half_threads(int BN, int C) { return (half_issuer_b(BN, C) + 1) * 32; }
 
 struct HalfConvParams {
    const float *X, *W, *bias; // NHWC, [Cout][3][3][C], [Cout] or nullptr
@@ -90,7 +99,7 @@ struct HalfConvParams {
 template <int BN, int C>
 struct HalfShared {
    uint64_t raw_full[kHalfMaxSlots], raw_empty[kHalfMaxSlots], op_full[kHalfMaxSlots], op_empty[kHalfMaxSlots];
-   uint64_t tmem_full[half_buffers(BN)], tmem_empty[half_buffers(BN)], w_ready;
+   uint64_t tmem_full[half_buffers(BN)], tmem_empty[half_buffers(BN)], w_ready, drain[2];
    uint64_t careful_op_full[kHalfMaxSlots], careful_op_empty[kHalfMaxSlots]; // of the careful tiles' slots and accumulators
    uint64_t careful_tmem_full[half_buffers(BN)], careful_tmem_empty[half_buffers(BN)];
    uint32_t tmem_base;
@@ -103,14 +112,14 @@ struct HalfShared {
    __align__(16) float stands[BN];           // a sum of this size stands although values or weights have lost something (0: no weights, it always does)
    uint32_t row_found[BN];
    volatile float x_inv[kHalfScales];        // inverse scale of a tile's patch, negative when some of its values have lost something; 0: a careful tile
-   uint2 red[kHalfConvGroups][2][kHalfConvGroupWarps];
+   uint2 red[half_groups(BN, C)][2][kHalfConvGroupWarps];
    uint32_t any_notes, notes[kHalfNoteWords];
    // Careful tiles, by converter group: of its passes in turn, and the bits of the patches' units of its tiles in turn. A pass or a patch is written when
    // the MMAs of at most the second last pass before it are done, which waited until the epilogue had read the second last accumulator before
    // that: four passes, and six tiles, are in use at most.
-   volatile float careful_inv[kHalfConvGroups][4];
-   volatile uint32_t careful_found[kHalfConvGroups][4];
-   uint32_t nonzero[kHalfConvGroups][8][kHalfBitWords], infinite[kHalfConvGroups][8][kHalfBitWords], nan[kHalfConvGroups][8][kHalfBitWords];
+   volatile float careful_inv[kHalfCarefulGroups][4];
+   volatile uint32_t careful_found[kHalfCarefulGroups][4];
+   uint32_t nonzero[kHalfCarefulGroups][8][kHalfBitWords], infinite[kHalfCarefulGroups][8][kHalfBitWords], nan[kHalfCarefulGroups][8][kHalfBitWords];
 };
 
 // Offset of a 16-byte piece in rows of RB bytes as the MMA's swizzle expects it (the region starts on a 1024-byte boundary).
@@ -298,8 +307,8 @@ __device__ __forceinline__ void half_issue(uint32_t d, uint32_t op, uint32_t w)
 #pragma unroll
       for (int k = 0; k < KSTEPS; k++) {
          const uint32_t a = (uint32_t)(((tap / 3) * kHalfPatchW + tap % 3) * RB + k * 32), b = (uint32_t)(tap * W_ITEM + k * 32);
-         tc_mma<kF16>(d, adesc(a), bdesc(b), idesc_wide, (tap | k) ? 1u : 0u); // leading x [leading | trailing]
-         tc_mma<kF16>(d + BN, adesc(a + PART), bdesc(b), idesc, 1u);           // trailing x leading
+         warp_mma<kF16>(d, adesc(a), bdesc(b), idesc_wide, (tap | k) ? 1u : 0u); // leading x [leading | trailing]
+         warp_mma<kF16>(d + BN, adesc(a + PART), bdesc(b), idesc, 1u);           // trailing x leading
       }
    }
 }
@@ -399,7 +408,7 @@ __device__ __forceinline__ void half_careful_convert(const HalfConvParams &p, Ha
          float scale, inverse;
          more = half_scale(largest, smallest, scale, inverse) == kHalfWide;
          const uint32_t e = largest >> 24, below = e > 15 ? max((int)e - (int)kHalfSpread, 1) : 0; // exponents under this wait for the next pass
-         const HalfPlace slot(group, q, half_slots(BN, C) / 2);
+         const HalfPlace slot(group, q, half_careful_slots(BN, C));
          const bool ok = (state & kHalfOk) && mbar_wait(&sh.careful_op_empty[slot.at], slot.phase ^ 1u, &sh.abort_flag, status, kStatusWaitEmpty, 0xa000 + lt);
          if (!ok) state &= ~kHalfOk; // and on to the group's next exchange
          if (t == 0) {
@@ -556,34 +565,32 @@ __device__ __noinline__ void half_careful_tiles(const HalfConvParams &p, HalfSha
    const HalfNotes notes = {sh.notes, tiles, HalfNotes::shift_for(tiles), (sh.w_found & kHalfSpecial) != 0};
    griddep_wait(); // the activations are read by these threads themselves
    if (warp == 1) {
-      if (lane == 0) {
-         int count = 0, q[2] = {0, 0};
-         for (int lt = notes.from(0); lt < notes.tiles; lt = notes.from(lt + 1), count++) {
-            const int group = count & 1;
-            bool more = true;
-            for (; more; q[group]++) {
-               const HalfPlace slot(group, q[group], half_slots(BN, C) / 2), buf(group, q[group], half_buffers(BN) / 2);
-               if (!mbar_wait(&sh.careful_op_full[slot.at], slot.phase, &sh.abort_flag, status, kStatusWaitConv, 0xb000 + lt) ||
-                   !mbar_wait(&sh.careful_tmem_empty[buf.at], buf.phase ^ 1u, &sh.abort_flag, status, kStatusWaitAccum, 0xb000 + lt))
-                  return;
-               more = sh.careful_found[group][q[group] & 3] & kHalfWide;
-               tc_fence_after();
-               half_issue<BN, C>(sh.tmem_base + (uint32_t)(buf.at * 2 * BN), smem_u32(ops + (size_t)slot.at * 2 * half_part_bytes(C)), smem_u32(w_smem));
-               tc_commit(&sh.careful_op_empty[slot.at]);
-               tc_commit(&sh.careful_tmem_full[buf.at]);
-            }
+      int count = 0, q[2] = {0, 0};
+      for (int lt = notes.from(0); lt < notes.tiles; lt = notes.from(lt + 1), count++) {
+         const int group = count & 1;
+         bool more = true;
+         for (; more; q[group]++) {
+            const HalfPlace slot(group, q[group], half_careful_slots(BN, C)), buf(group, q[group], half_buffers(BN) / 2);
+            if (!mbar_wait_warp(&sh.careful_op_full[slot.at], slot.phase, &sh.abort_flag, status, kStatusWaitConv, 0xb000 + lt) ||
+                !mbar_wait_warp(&sh.careful_tmem_empty[buf.at], buf.phase ^ 1u, &sh.abort_flag, status, kStatusWaitAccum, 0xb000 + lt))
+               return;
+            more = __any_sync(0xFFFFFFFFu, sh.careful_found[group][q[group] & 3] & kHalfWide);
+            tc_fence_after();
+            half_issue<BN, C>(sh.tmem_base + (uint32_t)(buf.at * 2 * BN), smem_u32(ops + (size_t)slot.at * 2 * half_part_bytes(C)), smem_u32(w_smem));
+            warp_commit(&sh.careful_op_empty[slot.at]);
+            warp_commit(&sh.careful_tmem_full[buf.at]);
          }
       }
    } else if (warp >= 2 && warp < 2 + kHalfEpiWarps) {
       half_careful_epilogue<BN, C, POOL>(p, sh, notes, sh.tmem_base + ((uint32_t)((warp & 3) * 32) << 16), warp, lane, status);
-   } else if (warp >= 2 + kHalfEpiWarps && warp < kHalfIssuerB) {
+   } else if (warp >= 2 + kHalfEpiWarps && warp < 2 + kHalfEpiWarps + kHalfCarefulGroups * kHalfConvGroupWarps) {
       const int cw = warp - 2 - kHalfEpiWarps, group = cw / kHalfConvGroupWarps;
       half_careful_convert<BN, C>(p, sh, notes, ops, group, cw % kHalfConvGroupWarps, lane, status);
    }
 }
 
 template <int BN, int C, bool POOL>
-__global__ void __launch_bounds__(kHalfThreads, 1)
+__global__ void __launch_bounds__(half_threads(BN, C), 1)
 umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ HalfConvParams p, uint32_t *status)
 {
    constexpr int RB = 2 * C;                       // bytes of an operand row: one pixel's or one (tap, output channel)'s halves
@@ -591,9 +598,10 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
    constexpr int UPP = C / 8;                      // units of eight channels per pixel
    constexpr int W_ITEM = 2 * BN * RB;             // one tap's weights: BN leading rows, BN trailing rows
    constexpr int NBUF = half_buffers(BN);
-   constexpr int SLOTS = half_slots(BN, C);
+   constexpr int SLOTS = half_slots(BN, C), GROUPS = half_groups(BN, C), ISSUER_B = half_issuer_b(BN, C), EPI_GROUPS = half_epilogue_groups(BN);
+   static_assert(SLOTS % GROUPS == 0, "a slot always meets the same converter group");
    constexpr uint32_t TMEM_COLS = NBUF * 2 * BN;
-   constexpr int CW = BN / 2;                      // channels per epilogue warp (two warps a lane quarter)
+   constexpr int CW = BN / 2 * EPI_GROUPS;         // channels per epilogue warp
    constexpr int CH = CW >= 32 ? 32 : CW;
    extern __shared__ unsigned char smem_raw[];
    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -605,7 +613,7 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
    SOFIE_PROF_DECL
    griddep_launch_dependents(); // the next kernel may set itself up while this one runs
-   for (int c = threadIdx.x; c < BN; c += kHalfThreads) sh.bias[c] = (c < p.Cout && p.bias) ? p.bias[c] : 0.f;
+   for (int c = threadIdx.x; c < BN; c += half_threads(BN, C)) sh.bias[c] = (c < p.Cout && p.bias) ? p.bias[c] : 0.f;
    if (threadIdx.x < C) sh.w_largest[threadIdx.x] = 0;
    if (threadIdx.x < kHalfNoteWords) sh.notes[threadIdx.x] = 0;
    if (threadIdx.x == 0) {
@@ -619,11 +627,12 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
       }
       for (int b = 0; b < NBUF; b++) {
          mbar_init(&sh.tmem_full[b], 1);
-         mbar_init(&sh.tmem_empty[b], kHalfEpiWarps);
+         mbar_init(&sh.tmem_empty[b], kHalfEpiWarps / EPI_GROUPS);
          mbar_init(&sh.careful_tmem_full[b], 1);
          mbar_init(&sh.careful_tmem_empty[b], kHalfEpiWarps);
       }
-      mbar_init(&sh.w_ready, kHalfConvWarps);
+      mbar_init(&sh.w_ready, kHalfWeightWarps);
+      for (int i = 0; i < 2; i++) mbar_init(&sh.drain[i], 1);
       sh.abort_flag = 0;
       sh.w_found = sh.any_notes = 0;
       fence_mbar_init();
@@ -642,46 +651,46 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
    if (warp == 0) {
       // ---------------- TMA producer: one box per tile ----------------
       griddep_wait(); // the activations are the previous kernel's output
-      if (lane == 0) {
-         TileWalker tw;
-         tw.init(blockIdx.x, gridDim.x, p.tilesH, p.tilesW);
-         int s = 0, g = 0;
-         uint32_t ph = 0;
-         for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, g++, ring_next(s, ph, SLOTS), tw.next()) {
-            // from the second round of slots on: when the weights send all tiles to the careful form, nobody looks at the patches
-            if (g == SLOTS && mbar_wait(&sh.w_ready, 0, &sh.abort_flag, status, kStatusWaitConv, 0x8000) && (sh.w_found & kHalfSpecial)) break;
-            if (!SOFIE_PROF_WAIT(mbar_wait(&sh.raw_empty[s], ph ^ 1, &sh.abort_flag, status, kStatusWaitEmpty, g))) break;
-            mbar_expect_tx(&sh.raw_full[s], RAW);
-            // rows and columns start at -1: zero fill; the channel coordinate is 0
-            tma_load_4d(raws + (size_t)s * RAW, &tmX, 0, tw.tw * kHalfTileW - 1, tw.th * kHalfTileH - 1, tw.n, &sh.raw_full[s]);
-         }
-         // the copies of patches that nobody looks at end before the kernel does
-         if (mbar_wait(&sh.w_ready, 0, &sh.abort_flag, status, kStatusWaitConv, 0x8000) && (sh.w_found & kHalfSpecial))
-            for (int i = 0; i < g && i < SLOTS; i++) mbar_wait(&sh.raw_full[i], 0, &sh.abort_flag, status, kStatusWaitFull, 0x8000);
+      TileWalker tw;
+      tw.init(blockIdx.x, gridDim.x, p.tilesH, p.tilesW);
+      int s = 0, g = 0;
+      uint32_t ph = 0;
+      // when the weights send all tiles to the careful form, nobody looks at the patches
+      auto unread = [&] { return __all_sync(0xFFFFFFFFu, mbar_wait(&sh.w_ready, 0, &sh.abort_flag, status, kStatusWaitConv, 0x8000) && (sh.w_found & kHalfSpecial)); };
+      for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, g++, ring_next(s, ph, SLOTS), tw.next()) {
+         if (g == SLOTS && unread()) break; // from the second round of slots on
+         if (!SOFIE_PROF_WAIT(mbar_wait_warp(&sh.raw_empty[s], ph ^ 1, &sh.abort_flag, status, kStatusWaitEmpty, g))) break;
+         warp_expect_tx(&sh.raw_full[s], RAW);
+         // rows and columns start at -1: zero fill; the channel coordinate is 0
+         warp_tma_load_4d(raws + (size_t)s * RAW, &tmX, 0, tw.tw * kHalfTileW - 1, tw.th * kHalfTileH - 1, tw.n, &sh.raw_full[s]);
       }
-   } else if (warp == 1 || warp == kHalfIssuerB) {
-      // ---------------- MMA issuers: even and odd tiles ----------------
-      if (lane == 0) {
-         bool ok = SOFIE_PROF_WAIT(mbar_wait(&sh.w_ready, 0, &sh.abort_flag, status, kStatusWaitConv, 0x4000)) && !(sh.w_found & kHalfSpecial);
-         const uint32_t w = smem_u32(w_smem);
-         const int step = gridDim.x;
-         for (int lt = warp == 1 ? 0 : 1; ok && blockIdx.x + (long long)lt * step < p.num_tiles; lt += 2) {
-            const int s = lt % SLOTS, buf = lt % NBUF;
-            ok = SOFIE_PROF_WAIT(mbar_wait(&sh.op_full[s], (uint32_t)(lt / SLOTS) & 1u, &sh.abort_flag, status, kStatusWaitConv, lt)) &&
-                 SOFIE_PROF_WAIT(mbar_wait(&sh.tmem_empty[buf], ((uint32_t)(lt / NBUF) & 1u) ^ 1u, &sh.abort_flag, status, kStatusWaitAccum, 0x2000 + lt));
-            if (!ok) break;
-            tc_fence_after();
-            half_issue<BN, C>(tmem_base + (uint32_t)(buf * 2 * BN), smem_u32(ops + (size_t)s * 2 * PART), w);
-            tc_commit(&sh.op_empty[s]);
-            tc_commit(&sh.tmem_full[buf]);
-         }
+      // the copies of patches that nobody looks at end before the kernel does
+      if (unread())
+         for (int i = 0; i < g && i < SLOTS; i++) mbar_wait(&sh.raw_full[i], 0, &sh.abort_flag, status, kStatusWaitFull, 0x8000);
+   } else if (warp == 1 || warp == ISSUER_B) {
+      // ---------------- MMA issuers: all tiles, or even and odd ones ----------------
+      // one of them keeps the pipe full with 36 MMAs a tile (32 channels: 185 us instead of 199), two do with 18 (320 instead of 338)
+      constexpr int ISSUERS = C == 32 ? 1 : 2;
+      const bool plain = __all_sync(0xFFFFFFFFu, SOFIE_PROF_WAIT(mbar_wait(&sh.w_ready, 0, &sh.abort_flag, status, kStatusWaitConv, 0x4000)) && !(sh.w_found & kHalfSpecial));
+      const uint32_t w = smem_u32(w_smem);
+      const int step = gridDim.x, parity = warp == 1 ? 0 : 1;
+      WarpWait wait;
+      for (int lt = parity; plain && parity < ISSUERS && blockIdx.x + (long long)lt * step < p.num_tiles; lt += ISSUERS) {
+         const int s = lt % SLOTS, buf = lt % NBUF;
+         wait(&sh.op_full[s], (uint32_t)(lt / SLOTS) & 1u);
+         wait(&sh.tmem_empty[buf], ((uint32_t)(lt / NBUF) & 1u) ^ 1u);
+         tc_fence_after();
+         half_issue<BN, C>(tmem_base + (uint32_t)(buf * 2 * BN), smem_u32(ops + (size_t)s * 2 * PART), w);
+         warp_commit(&sh.op_empty[s]);
+         warp_commit(&sh.tmem_full[buf]);
       }
+      wait.finish(&sh.drain[parity], &sh.abort_flag, status, kStatusWaitConv, 0x2000);
    } else if (warp >= 2 + kHalfEpiWarps) {
       // ---------------- converters ----------------
       const int cw = warp - 2 - kHalfEpiWarps, group = cw / kHalfConvGroupWarps, gw = cw % kHalfConvGroupWarps;
-      {
-         // the weights, once per CTA, by all converter warps: TPR neighbouring threads a row, each with the units of the same eight channels
-         constexpr int TPR = kHalfConvWarps * 32 / BN, UNITS = 9 * UPP, PER = (UNITS + TPR - 1) / TPR;
+      if (cw < kHalfWeightWarps) {
+         // the weights, once per CTA, by the first converter warps: TPR neighbouring threads a row, each with the units of the same eight channels
+         constexpr int TPR = kHalfWeightWarps * 32 / BN, UNITS = 9 * UPP, PER = (UNITS + TPR - 1) / TPR;
          static_assert(TPR >= 1 && 32 % TPR == 0, "the threads of a row are in one warp");
          static_assert(TPR % UPP == 0, "a thread's units are of the same channels");
          const int t = cw * 32 + lane, row = t / TPR, sub = t % TPR, c_first = sub % UPP * 8;
@@ -708,7 +717,7 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
             for (int o = UPP; o < 32; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
             if (lane < UPP) atomicMax(&sh.w_largest[c_first + j], m);
          }
-         asm volatile("bar.sync %0, %1;" ::"n"(1 + kHalfConvGroups), "n"(kHalfConvWarps * 32) : "memory");
+         asm volatile("bar.sync %0, %1;" ::"n"(1 + GROUPS), "n"(kHalfWeightWarps * 32) : "memory");
          const uint32_t all = sh.w_largest[lane % C], high = __reduce_max_sync(0xffffffffu, all), low = __reduce_min_sync(0xffffffffu, all), e_high = max(high >> 24, 1u);
          if (high != 0 && e_high < 255 && (low == 0 || e_high - max(low >> 24, 1u) > kHalfChannelSpread)) {
             auto below = [&](uint32_t largest) { return min(e_high - max(largest >> 24, 1u), kHalfChannelFactor); }; // powers of two
@@ -764,7 +773,7 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
       uint32_t state = mbar_wait(&sh.w_ready, 0, &sh.abort_flag, status, kStatusWaitConv, 0x8000) ? kHalfOk : 0, none = 0;
       const bool factors = sh.w_factors != 0, go = !(sh.w_found & kHalfSpecial);
       if (!go) half_exchange(sh, group, gw, lane, state, none, none); // a warp whose wait gave up may not know that, and goes on to an exchange
-      for (int lt = group; go && lt < tiles; lt += kHalfConvGroups) {
+      for (int lt = group; go && lt < tiles; lt += GROUPS) {
          const int s = lt % SLOTS;
          if (!((state & kHalfOk) && SOFIE_PROF_WAIT(mbar_wait(&sh.raw_full[s], (uint32_t)(lt / SLOTS) & 1u, &sh.abort_flag, status, kStatusWaitFull, 0x6000 + lt)))) state = state & ~kHalfOk;
          float v[PER][8];
@@ -829,11 +838,11 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
          if (ok && lane == 0) mbar_arrive(&sh.op_full[s]);
       }
    } else {
-      // ---------------- epilogue: warps 2..9, two per lane quarter ----------------
-      const int c_begin = ((warp - 2) >> 2) * CW;
-      const int lane_base = (warp & 3) * 32;
+      // ---------------- epilogue: warps 2..9, two per lane quarter, on the same tile or on two in turn ----------------
+      const int egroup = EPI_GROUPS == 2 ? (warp - 2) >> 2 : 0, c_begin = EPI_GROUPS == 2 ? 0 : ((warp - 2) >> 2) * CW;
+      const int lane_base = (warp & 3) * 32, step = EPI_GROUPS * gridDim.x;
       TileWalker tw;
-      tw.init(blockIdx.x, gridDim.x, p.tilesH, p.tilesW);
+      tw.init(blockIdx.x + egroup * gridDim.x, step, p.tilesH, p.tilesW);
       // the weights' scales and verdict are the converters'
       bool ok = SOFIE_PROF_WAIT(mbar_wait(&sh.w_ready, 0, &sh.abort_flag, status, kStatusWaitConv, 0x5000)) && !(sh.w_found & kHalfSpecial);
       // largest and smallest inverse scale of a channel's weights (positive: ordered as their bits are)
@@ -858,8 +867,8 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
       load_constants(c_begin);
       const int note_shift = HalfNotes::shift_for(tiles);
       const bool w_lossy = sh.w_found != 0;
-      int lt = 0;
-      for (int tile = blockIdx.x; ok && tile < p.num_tiles; tile += gridDim.x, lt++, tw.next()) {
+      int lt = egroup;
+      for (int tile = blockIdx.x + egroup * gridDim.x; ok && tile < p.num_tiles; tile += step, lt += EPI_GROUPS, tw.next()) {
          const int buf = lt % NBUF;
          ok = SOFIE_PROF_WAIT(mbar_wait(&sh.tmem_full[buf], (uint32_t)(lt / NBUF) & 1u, &sh.abort_flag, status, kStatusWaitAccum, 0x3000 + lt));
          if (!ok) break;
@@ -948,7 +957,7 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
          }
       }
    }
-   SOFIE_PROF_REPORT(warp == 0 ? "producer" : (warp == 1 || warp == kHalfIssuerB ? "mma" : (warp < 2 + kHalfEpiWarps ? "epilogue" : "converter")));
+   SOFIE_PROF_REPORT(warp == 0 ? "producer" : (warp == 1 || warp == ISSUER_B ? "mma" : (warp < 2 + kHalfEpiWarps ? "epilogue" : "converter")));
    tc_fence_before();
    __syncthreads();
    if ((sh.any_notes || (sh.w_found & kHalfSpecial)) && !sh.abort_flag) {
@@ -987,7 +996,7 @@ int launch_half(cudaStream_t s, const ConvGeom &g, const float *X, const float *
    const int grid = p.num_tiles < kNumSMs ? p.num_tiles : kNumSMs;
    auto kern = umma_conv3x3_half_kernel<BN, C, POOL>;
    SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), smem));
-   SOFIE_CUDA_TRY(launch_dependent(kern, dim3(grid), dim3(kHalfThreads), smem, s, tmX, p, status));
+   SOFIE_CUDA_TRY(launch_dependent(kern, dim3(grid), dim3(half_threads(BN, C)), smem, s, tmX, p, status));
    SOFIE_LAUNCH_CHECK("umma_conv3x3_half_kernel");
    set_last_engine(SOFIE_ENGINE_TCGEN05);
    return SOFIE_CUDA_OK;
