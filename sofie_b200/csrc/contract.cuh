@@ -12,6 +12,9 @@ struct ConvGeom {
 };
 
 int launch_gemm_f32_simt(cudaStream_t, const sofie_gemm_f32_desc &, const float *, const float *, const float *, float *);
+// few FMAs, any layout
+bool gemm_f32_tiny_ok(const sofie_gemm_f32_desc &);
+int launch_gemm_f32_tiny(cudaStream_t, const sofie_gemm_f32_desc &, const float *, const float *, const float *, float *);
 int launch_gemm_f32_umma(cudaStream_t, const sofie_gemm_f32_desc &, const float *, const float *, const float *, float *);
 // any layout, alignment and K; long K split over a cluster (umma_gemm_any.cu). tma: operands the TMA kernel takes too; others are refused
 // where the CUDA-core kernel is the faster one

@@ -74,6 +74,93 @@ gemm_f32_simt_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, const f
    }
 }
 
+// Products of few FMAs, whatever the layout: what bounds them is latency. The kernel above walks K in steps of 16 with a round trip to memory
+// and two barriers each (2 x 1 x 427 34 us), the tensor-core kernels set themselves up (6 to 8 us). Here T lanes share an output, each with every
+// T-th term of K, all loads of eight terms issued together, and add up their sums in pairs: 2 x 1 x 427 2.7 us, 5 x 2 x 166 21.7 -> 2.3,
+// 2 x 119 x 66 12.1 -> 2.6. Sums carry what products and additions round off in a second
+// word (T. Ogita, S. M. Rump and S. Oishi, "Accurate sum and dot product", 2005), which costs nothing here: no other kernel's are closer. (In 64 bits
+// the same took 71 us for 1 x 1 x 16384.)
+struct TwoSum {
+   float s = 0.f, c = 0.f; // s is the ordinary sum
+   __device__ __forceinline__ void add(float x)
+   {
+      const float t = __fadd_rn(s, x), z = __fsub_rn(t, s);
+      c = __fadd_rn(c, __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(x, z)));
+      s = t;
+   }
+   __device__ __forceinline__ void add_product(float x, float y)
+   {
+      const float p = __fmul_rn(x, y);
+      add(p);
+      c = __fadd_rn(c, __fmaf_rn(x, y, -p));
+   }
+};
+template <int T>
+__global__ void __launch_bounds__(128)
+gemm_f32_tiny_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, const float *__restrict__ B, const float *C, float *Y)
+{
+   griddep_launch_dependents();
+   griddep_wait(); // the operands may be the previous kernel's output
+   const int i = (blockIdx.x * 128 + threadIdx.x) / T, t = threadIdx.x % T;
+   const bool live = i < d.M * d.N;
+   const int m = live ? i / d.N : 0, n = live ? i - m * d.N : 0;
+   const long long as = d.transA ? d.M : 1, bs = d.transB ? 1 : d.N;
+   const float *a = A + (d.transA ? m : (long long)m * d.K) + t * as, *b = B + (d.transB ? (long long)n * d.K : n) + t * bs;
+   const float c = d.bias_kind == 0 || !live ? 0.f : C[d.bias_kind == 1 ? n : i];
+   TwoSum acc;
+   for (int k = t; k < d.K; k += 8 * T, a += 8 * T * as, b += 8 * T * bs) {
+      float x[8], y[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+         const bool in = k + j * T < d.K;
+         x[j] = in ? a[j * T * as] : 0.f;
+         y[j] = in ? b[j * T * bs] : 0.f;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; j++) acc.add_product(x[j], y[j]);
+   }
+#pragma unroll
+   for (int o = T / 2; o > 0; o /= 2) {
+      const float s = __shfl_down_sync(0xFFFFFFFFu, acc.s, o, T), c = __shfl_down_sync(0xFFFFFFFFu, acc.c, o, T);
+      acc.add(s);
+      acc.c += c;
+   }
+   if (t == 0 && live) {
+      float sum = acc.s + acc.c;
+      if (!(fabsf(sum) < __uint_as_float(0x7F800000u))) { // infinities, NaNs, and what overflows: as the chain of FMAs
+         sum = 0.f;
+         a = A + (d.transA ? m : (long long)m * d.K), b = B + (d.transB ? (long long)n * d.K : n);
+         for (int k = 0; k < d.K; k++, a += as, b += bs) sum = fmaf(*a, *b, sum);
+      }
+      float y = d.alpha * sum;
+      if (d.bias_kind) y += d.beta * c;
+      Y[i] = d.relu ? relu_ref(y) : y;
+   }
+}
+
+// Up to 2^18 FMAs, of 8192 terms at most: from there on the loads count, which are not shared (2^19: 1.4 to 1.7 times as fast in the mean, but
+// half as fast in the worst case; up to 2^18 1.2 to 4 times, 2.4 in the mean, over 420 products of every layout). A longer K is taken where the
+// kernel above would.
+bool gemm_f32_tiny_ok(const sofie_gemm_f32_desc &d)
+{
+   const long long fmas = (long long)d.M * d.N * d.K;
+   return (long long)d.M * d.N <= 1 << 18 && fmas <= 1 << 18 && (d.K <= 8192 || fmas <= 32768);
+}
+
+int launch_gemm_f32_tiny(cudaStream_t s, const sofie_gemm_f32_desc &d, const float *A, const float *B, const float *C, float *Y)
+{
+   const int outputs = d.M * d.N;
+   auto launch = [&](auto lanes) {
+      constexpr int T = decltype(lanes)::value;
+      return launch_dependent(gemm_f32_tiny_kernel<T>, dim3(ceil_div(outputs * T, 128)), dim3(128), 0, s, d, A, B, C, Y);
+   };
+   // as many lanes as keep a lane's terms to one batch of loads
+   SOFIE_CUDA_TRY(d.K <= 8 ? launch(std::integral_constant<int, 1>{}) : d.K <= 32 ? launch(std::integral_constant<int, 4>{}) :
+                  d.K <= 128 ? launch(std::integral_constant<int, 16>{}) : launch(std::integral_constant<int, 32>{}));
+   set_last_engine(SOFIE_ENGINE_SIMT);
+   return SOFIE_CUDA_OK;
+}
+
 int launch_gemm_f32_simt(cudaStream_t s, const sofie_gemm_f32_desc &d, const float *A, const float *B, const float *C,
                          float *Y)
 {

@@ -1042,7 +1042,7 @@ int launch_gemm_f32_umma(cudaStream_t s, const sofie_gemm_f32_desc &d, const flo
    auto aligned = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
    const bool tma = !d.transA && d.transB && d.K % 4 == 0 && aligned(A) && aligned(B); // rows TMA can fetch
    if (!tma && (long long)d.M * d.N * d.K <= 32768)
-      return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "a product this small of rows TMA cannot fetch is faster on the CUDA cores (3.2 against 3.5 us)");
+      return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "a product this small of rows TMA cannot fetch has kernels on the CUDA cores");
    // The kernel below overlaps a tile's epilogue with the next one's MMAs, which pays where a CTA has several tiles and each is short:
    // 100000 x 10 x 128 20 us against 29, 100000 x 128 x 128 48 against 54. Longer K or fewer tiles are the other kernel's, whose
    // stages are cheaper and which splits K -- unless the rows of Y are short, which this kernel's threads write one each: 500 x 1 x 12 3.8 us

@@ -517,7 +517,7 @@ PartsPlan parts_plan(const sofie_gemm_f32_desc &d)
    PartsPlan p;
    const int tm = ceil_div(d.M, kAnyBM), nkb = ceil_div(d.K, kAnyKE);
    const bool full = d.bias_kind == 2, tma = !d.transA && d.transB && d.K % 4 == 0;
-   if (d.M < 32 || d.N < 32) return p;  // hardly a tile: not measured, and the skinny products have more precise kernels
+   if (d.M < 32 || d.N < 32 || (!forced_engine() && gemm_f32_tiny_ok(d))) return p;  // hardly a tile: not measured, and the skinny products have more precise kernels
    if (d.K < 48) return p; // the writes of Y count, and short K leaves the split little to save: 16384 x 4093 x 8 169 us either way
    const long long split = 4560 + 1817 * (((long long)d.M + d.N) * nkb * kAnyKE) / 1000000, out = 1361 * ((long long)d.M * d.N * (full ? 2 : 1)) / 1000000;
    long long best = -1;

@@ -885,3 +885,35 @@ def test_skinny_products_stay_with_split_k(M, N, K, transB):
     assert ops.last_engine() == capi.ENGINE_SIMT
     exact = A.double() @ (B.double().t() if transB else B.double())
     assert float((y.double() - exact).norm() / exact.norm()) <= 2.5e-7     # chains of at most some hundred terms
+
+
+# 1, 4, 16 and 32 lanes an output, one batch of terms and more, the last block and the last group of lanes partly empty, the largest it takes
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (3, 5, 8), (7, 3, 9), (64, 512, 8), (11, 13, 32), (5, 7, 33), (9, 11, 128), (3, 3, 129), (2, 1, 427), (1, 1, 8192), (31, 33, 256), (1, 32, 8191),
+                                   (512, 512, 1), (4, 500, 131), (1, 1, 20000)])
+def test_gemm_f32_of_few_fmas(M, N, K):
+    """Rounded a handful of times in all (the sum, alpha, beta, the bias), for every layout; infinities and NaNs as a chain of FMAs gives them."""
+    g = torch.Generator(device="cuda").manual_seed(M * N + K)
+    for tA in (0, 1):
+        for tB in (0, 1):
+            for bias in (0, 1, 2):
+                if tB and N <= 16 and K >= 1024:
+                    continue                                         # the row kernel's
+                ops.set_engine(0)
+                A = torch.randn((K, M) if tA else (M, K), device="cuda", generator=g)
+                B = torch.randn((N, K) if tB else (K, N), device="cuda", generator=g)
+                C_ = {0: None, 1: torch.randn(N, device="cuda", generator=g), 2: torch.randn(M, N, device="cuda", generator=g)}[bias]
+                a, b = (A.t() if tA else A).double(), (B.t() if tB else B).double()
+                c = 0 if C_ is None else 1.5 * C_.double().view(-1, N)
+                ref = 0.75 * (a @ b) + c
+                out = C_.clone() if bias == 2 and tA else None       # the bias and the result may be the same memory
+                y = ops.gemm_f32(A, B, C_ if out is None else out, transA=tA, transB=tB, alpha=0.75, beta=1.5, out=out)
+                assert ((y.double() - ref).abs() <= 4 * 2.0 ** -24 * ((0.75 * (a @ b)).abs() + (c.abs() if bias else 0)) + 2.0 ** -45).all()
+                if N <= 16 and K >= 1024:
+                    continue                                         # the CUDA cores' own kernel for these is not one chain
+                A.view(-1)[0], B.view(-1)[-1] = float("inf"), float("nan") if M * N > 1 else 3e38
+                y = ops.gemm_f32(A, B, C_, transA=tA, transB=tB)
+                ops.set_engine(capi.ENGINE_SIMT)
+                chain = ops.gemm_f32(A, B, C_, transA=tA, transB=tB)
+                ops.set_engine(0)
+                odd = ~chain.isfinite()
+                assert torch.equal(y.isfinite(), ~odd) and torch.equal(y[odd].nan_to_num(1., 2., 3.), chain[odd].nan_to_num(1., 2., 3.))
