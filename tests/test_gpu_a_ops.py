@@ -917,3 +917,18 @@ def test_gemm_f32_of_few_fmas(M, N, K):
                 ops.set_engine(0)
                 odd = ~chain.isfinite()
                 assert torch.equal(y.isfinite(), ~odd) and torch.equal(y[odd].nan_to_num(1., 2., 3.), chain[odd].nan_to_num(1., 2., 3.))
+
+
+# as many groups of eight channels as blocks beside a tile, or all of them in one; the last group partly empty
+@pytest.mark.parametrize("N,C,H,W,Cout,pool", [(2, 3, 12, 12, 30, 0), (70, 1, 17, 40, 64, 2), (75, 4, 16, 32, 64, 0), (5, 2, 33, 9, 9, 2), (600, 3, 16, 16, 8, 0)])
+@pytest.mark.parametrize("nhwc", [0, 1])
+def test_first_conv_f32_channel_groups(N, C, H, W, Cout, pool, nhwc):
+    g = torch.Generator(device="cuda").manual_seed(N + Cout)
+    x, w, b = (torch.randn(s, device="cuda", generator=g) for s in ((N, C, H, W), (Cout, C, 3, 3), (Cout,)))
+    y = ops.conv2d_f32(x.permute(0, 2, 3, 1).contiguous() if nhwc else x, w, b, shape=(N, C, H, W), pad=(1, 1), relu=True, pool=pool, x_layout=nhwc, y_layout=capi.LAYOUT_NHWC)
+    ref = torch.nn.functional.conv2d(x.double(), w.double(), b.double(), padding=1).relu()
+    if pool:
+        ref = torch.nn.functional.max_pool2d(ref, 2)
+    # a chain of 9 C products: each of them and each partial sum is off by 2^-24 of at most the sum of sizes
+    size = torch.nn.functional.conv2d(x.double().abs(), w.double().abs(), b.double().abs(), padding=1).amax()
+    assert (y.view(N, ref.shape[2], ref.shape[3], Cout).permute(0, 3, 1, 2).double() - ref).abs().max() <= (9 * C + 2) * 2.0 ** -24 * size
