@@ -93,10 +93,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
 // outcome the compiler gathers them from the active lanes one by one. Ten MMAs of a stage of 128 x 64 x 16 (128 x 128 x 16) with their
 // wait, commit and copies: 979 (980) clocks from one lane, 601 (786) from a warp, 548 (769) without any wait.
 //
-// The issuers' form has no way out, since a branch behind the wait costs 45 to 90 clocks a stage: a wait that runs out (about a
-// second) leaves `gave_up` set, which makes the later ones return at once; the warp walks on over whatever the stages hold to the end of its
+// The issuers' form has no way out, since a branch behind the wait costs 45 to 90 clocks a stage: a wait that runs out (a few
+// seconds) leaves `gave_up` set, which makes the later ones return at once; the warp walks on over whatever the stages hold to the end of its
 // loop and then reports with finish(). Copies are not issued that way: a role that writes shared memory stops (mbar_wait_warp).
-constexpr uint32_t kPollLimit = 1u << 18; // polls of a barrier that nothing happens to take 7800 clocks each: about a second
+constexpr uint32_t kPollLimit = 1u << 20; // a poll takes some 300 clocks, 7800 on a barrier that nothing happens to: four seconds at most
 struct WarpWait {
    uint32_t gave_up = 0;
    __device__ __forceinline__ void operator()(uint64_t *bar, uint32_t parity)
@@ -159,13 +159,6 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, i
 {
    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                 ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-                : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(void *dst, const CUtensorMap *map, int x, int y, int z, int w,
-                                            uint64_t *bar)
-{
-   asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-                ::"r"(smem_u32(dst)), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(smem_u32(bar))
                 : "memory");
 }
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map)

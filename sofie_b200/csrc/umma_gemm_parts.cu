@@ -219,6 +219,10 @@ __device__ __forceinline__ void parts_write(const AnyEpilogue &ep, const float *
    }
 }
 
+// A full C is read once, at the end of a tile, from memory: its lines are asked for when the tile begins (1000 x 777 x 1333 with new inputs every
+// pass 27.1 -> 25.7 us).
+__device__ __forceinline__ void parts_prefetch(const float *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // The end of a tile that a cluster shares: every rank adds up and writes its rows out of all partial tiles (distributed shared memory, in the
 // order of the ranks). With the loads of a thread's whole share issued together, as for a tile of one CTA, it took longer (320 x 1239 x 2149 26.0
 // instead of 23.8 us).
@@ -328,6 +332,18 @@ umma_gemm_parts_kernel(AnyOperand A, AnyOperand B, PartsLayout pa, PartsLayout p
       int u = 0;
       bool ok = true;
       for (int tile = tile0; tile < num_tiles && ok; tile += tile_step) {
+         if (ep.bias_kind == 2) { // the 32 rows and COLS columns that this warp has, or its share of the rank's rows
+            const int m0 = (tile / tiles_n) * kAnyBM, n0 = (tile % tiles_n) * BN;
+            if (S == 1) {
+               const int row = min(m0 + lane_base + lane, M - 1), col = min(n0 + col_base, N - 1);
+               parts_prefetch(ep.C + (size_t)row * N + col);
+               parts_prefetch(ep.C + (size_t)row * N + min(col + COLS - 1, N - 1));
+            } else {
+               constexpr int LINES = BN / 32 + 1;
+               for (int i = threadIdx.x; i < kAnyBM / S * LINES; i += L::kWriters)
+                  parts_prefetch(ep.C + (size_t)min(m0 + rank * (kAnyBM / S) + i / LINES, M - 1) * N + min(n0 + min(i % LINES * 32, BN - 1), N - 1));
+            }
+         }
          float acc[COLS];
 #pragma unroll
          for (int j = 0; j < COLS; j++) acc[j] = 0.f;
@@ -493,7 +509,7 @@ struct PartsPlan {
 // where rows of Y are not whole 16-byte words and where C is of Y's shape), under which the next tile's stages run, or the exchange within
 // a cluster; at least the writes of Y. Clusters of 4 / 8 found room for 132 / 96 CTAs at a time.
 // Against the other kernels' estimate, which is 20 % low in the mean: the split pays from about 2^20 outputs or 2^24 FMAs a tile on. 1000 x 777 x
-// 1333 with A transposed and a full bias 39 -> 25 us, 4096 x 4096 x 2048 522 -> 302, 785 x 2853 x 683 64 -> 35, 16384 x 777 x 64 59 -> 32; of the 2800
+// 1333 with A transposed and a full bias 39 -> 25.7 us, 4096 x 4096 x 2048 522 -> 302, 785 x 2853 x 683 64 -> 35, 16384 x 777 x 64 59 -> 32; of the 2800
 // (M and N from 48 on) it takes three in five, and 0.3 % of them are more than 3 % slower.
 PartsPlan parts_plan(const sofie_gemm_f32_desc &d)
 {
