@@ -161,6 +161,12 @@ int sofie_cuda_device_check(int device);
  * when `reached_exit_device` is not NULL, stores 1 there as its last action. Nothing faults or hangs;
  * the following sofie_cuda_ctx_check / sofie_cuda_ctx_fetch reports SOFIE_CUDA_ERR_DEVICE once. */
 int sofie_cuda_selftest_wait_timeout(void *stream, int64_t limit_cycles, uint32_t *reached_exit_device);
+/* The same for the waits of the warps that issue copies and MMAs: one CTA copies eight stages of 4096 bytes from `src_device` (16-byte aligned)
+ * into a ring of two and multiplies each. In the fourth the issuing warp (role 1) or the copying warp (role 2) waits on a barrier nothing arrives
+ * on, with the caller's limit; with role 0 nobody does. The others leave through the CTA's abort flag, the issuer by a limit of its own.
+ * out_device, five words: 1 as the last action | stages copied | 1 when the accumulator was handed to the reading warp with the sums of
+ * 32 x 8 times the first byte (2: other sums) | 1 when the issuing warp gave up | 1 when every copy had landed. */
+int sofie_cuda_selftest_warp_waits(void *stream, int32_t role, int64_t limit_cycles, const void *src_device, uint32_t *out_device);
 /* Self test of the threaded host copy that carries pageable inputs into the pinned staging ring (no
  * counterpart in the reference; needs no GPU): copies `bytes` bytes from src to dst `repeats` times in
  * chunks of `chunk` bytes with `threads` threads (the caller and threads - 1 helpers), exactly as

@@ -112,6 +112,7 @@ SIGNATURES = {
     "sofie_cuda_ctx_check": [vp],
     "sofie_cuda_device_check": [C.c_int],
     "sofie_cuda_selftest_wait_timeout": [vp, C.c_int64, vp],
+    "sofie_cuda_selftest_warp_waits": [vp, i32, C.c_int64, vp, vp],
     "sofie_cuda_selftest_host_copy": [vp, vp, C.c_size_t, C.c_size_t, C.c_int, C.c_int],
     "sofie_cuda_ctx_timers": [vp, C.c_int],
     "sofie_cuda_ctx_timed": [vp],

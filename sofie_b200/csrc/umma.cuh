@@ -1,8 +1,9 @@
 // sm_100a building blocks used by the tensor-core kernels: mbarrier, TMA (cp.async.bulk.tensor,
 // never with cluster multicast), tcgen05 (TMEM allocation, MMA, commit, load) and the descriptors
-// they take. Every wait is bounded: a wait that runs out records a code in the device status word
-// and reports failure to its caller, which then leaves the kernel through the normal exit path
-// (TMEM released), so the context stays usable.
+// they take. Every wait is bounded, by the clock (about a second) or, in the warps that issue MMAs, by a count of
+// polls (0.2 to 4 seconds): a wait that runs out records a code in the device status word, and its role hands
+// nothing on and leaves the kernel through the normal exit path (copies and MMAs under way waited for, TMEM
+// released), so the context stays usable.
 #pragma once
 
 #include <cuda.h>
@@ -93,37 +94,61 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
 // outcome the compiler gathers them from the active lanes one by one. Ten MMAs of a stage of 128 x 64 x 16 (128 x 128 x 16) with their
 // wait, commit and copies: 979 (980) clocks from one lane, 601 (786) from a warp, 548 (769) without any wait.
 //
-// The issuers' form has no way out, since a branch behind the wait costs 45 to 90 clocks a stage: a wait that runs out (a few
-// seconds) leaves `gave_up` set, which makes the later ones return at once; the warp walks on over whatever the stages hold to the end of its
-// loop and then reports with finish(). Copies are not issued that way: a role that writes shared memory stops (mbar_wait_warp).
+// The issuers' form has no way out and nothing but polls in its loop: a branch behind the wait costs 45 to 90 clocks a stage, a look at the clock
+// or at the abort flag between polls, however rare, or a store to the flag beside the commit 4 to 9 % of a product of narrow tiles or of a pooled
+// convolution. A wait that runs out leaves `gave_up` set, which makes the later ones return at once; the warp walks on over whatever the stages hold
+// to the end of its loop, but its commits (commit() below) do nothing, so that no other role takes a stage or an accumulator for finished: they stand
+// until finish() raises the CTA's abort flag and reports. Roles that write shared memory or results stop (mbar_wait_warp).
+// The vote is __all_sync: a vote orders no memory accesses, so every lane, the elected one among them, sees the phase for itself.
 constexpr uint32_t kPollLimit = 1u << 20; // a poll takes some 300 clocks, 7800 on a barrier that nothing happens to: four seconds at most
 struct WarpWait {
+   uint32_t limit = kPollLimit; // a power of two
    uint32_t gave_up = 0;
    __device__ __forceinline__ void operator()(uint64_t *bar, uint32_t parity)
    {
       uint32_t n = gave_up;
-      while (!__any_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity)) && ++n < kPollLimit) {}
-      gave_up |= n & kPollLimit;
+      while (!__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity)) && ++n < limit) {}
+      gave_up |= n & limit;
    }
-   // After the role's loop: true when all waits came through. Otherwise the give-up is reported and the MMAs under way are waited for
-   // (`drain`: a barrier of one arrival that nothing else uses).
-   __device__ __forceinline__ bool finish(uint64_t *drain, volatile uint32_t *abort_flag, uint32_t *status, uint32_t code, uint32_t detail);
+   // Arrives on the barrier once all MMAs issued so far by this warp have completed; not after a wait that gave up.
+   __device__ __forceinline__ void commit(uint64_t *bar);
+   // After the role's loop: a wait that gave up is reported, and the MMAs under way end before the tensor memory is given back (`drain`: a barrier of
+   // one arrival that nothing else uses).
+   __device__ __forceinline__ void finish(uint64_t *drain, volatile uint32_t *abort_flag, uint32_t *status, uint32_t code, uint32_t detail);
 };
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, volatile uint32_t *abort_flag, uint32_t *status, uint32_t code,
-                                               uint32_t detail)
+                                               uint32_t detail, long long limit_cycles = kWaitLimitCycles)
 {
-   if (__any_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+   if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
    const long long start = clock64();
    while (true) {
 #pragma unroll 1
       for (int spin = 0; spin < 16; spin++)
-         if (__any_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+         if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
       if (__any_sync(0xFFFFFFFFu, *abort_flag != 0u)) return false;
-      if (__any_sync(0xFFFFFFFFu, clock64() - start > kWaitLimitCycles)) {
+      if (__any_sync(0xFFFFFFFFu, clock64() - start > limit_cycles)) {
          if ((threadIdx.x & 31) == 0) mbar_give_up(abort_flag, status, code, detail);
          __syncwarp();
          return false;
       }
+   }
+}
+// A wait for what the hardware has under way when a role ends: at most some milliseconds, then the block leaves all the same.
+__device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity)
+{
+   for (int n = 0; n < 4096 && !__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity)); n++) {}
+}
+// What a warp that issues copies does at its end: the copies under way land before the block leaves its shared memory. (Without a wait that
+// gave up somewhere they have been consumed, or are about to be.) slot and phase: of the ring of `stages`, behind the last of `issued` stages.
+__device__ __forceinline__ void drain_copies(uint64_t *full_bar, int slot, uint32_t phase, int issued, int stages)
+{
+   const int n = issued < stages ? issued : stages;
+   slot -= n; // the oldest first: all but the last have landed by then, and this role is done when that one has
+   if (slot < 0) slot += stages, phase ^= 1u;
+#pragma unroll 1
+   for (int i = 0; i < n; i++) {
+      mbar_drain(&full_bar[slot], phase);
+      if (++slot == stages) slot = 0, phase ^= 1u;
    }
 }
 
@@ -235,14 +260,19 @@ __device__ __forceinline__ void warp_commit(uint64_t *bar)
                 : "memory");
 }
 
-__device__ __forceinline__ bool WarpWait::finish(uint64_t *drain, volatile uint32_t *abort_flag, uint32_t *status, uint32_t code, uint32_t detail)
+__device__ __forceinline__ void WarpWait::commit(uint64_t *bar)
 {
-   if (!gave_up) return true;
-   if ((threadIdx.x & 31) == 0 && !*abort_flag) mbar_give_up(abort_flag, status, code, detail);
+   asm volatile("{\n\t.reg .pred e, g;\n\tsetp.eq.u32 g, %1, 0;\n\telect.sync _|e, 0xFFFFFFFF;\n\tand.pred e, e, g;\n\t"
+                "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(gave_up)
+                : "memory");
+}
+__device__ __forceinline__ void WarpWait::finish(uint64_t *drain, volatile uint32_t *abort_flag, uint32_t *status, uint32_t code, uint32_t detail)
+{
+   if (!gave_up) return;
+   if ((threadIdx.x & 31) == 0) mbar_give_up(abort_flag, status, code, detail);
    __syncwarp();
    warp_commit(drain);
-   for (int n = 0; !__any_sync(0xFFFFFFFFu, mbar_try_wait(drain, 0)) && ++n < 4096;) {}
-   return false;
+   mbar_drain(drain, 0);
 }
 
 enum Kind { kTF32 = 0, kI8 = 1, kF8 = 2, kBF16 = 3, kF16 = 4 };
@@ -337,11 +367,11 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 }
 // Arrive on the barrier at this shared-memory offset in every CTA of `cta_mask` once all MMAs issued
 // so far by this thread have completed.
-__device__ __forceinline__ void warp_commit_pair(uint64_t *bar, uint16_t cta_mask)
+__device__ __forceinline__ void warp_commit_pair(uint64_t *bar, uint16_t cta_mask, uint32_t gave_up) // see WarpWait::commit()
 {
-   asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xFFFFFFFF;\n\t"
+   asm volatile("{\n\t.reg .pred e, g;\n\tsetp.eq.u32 g, %2, 0;\n\telect.sync _|e, 0xFFFFFFFF;\n\tand.pred e, e, g;\n\t"
                 "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(smem_u32(bar)),
-                "h"(cta_mask)
+                "h"(cta_mask), "r"(gave_up)
                 : "memory");
 }
 template <int KIND>

@@ -332,6 +332,8 @@ umma_conv3x3_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
             }
          }
       }
+      if constexpr (RW) mbar_drain(&w_full, 0);
+      drain_copies(full_bar, s, ph, g, S);
    } else if (warp == 1 || (KIND == kI8 && warp == kConvIssuerB)) {
       // ---------------- MMA issuers ----------------
       // int8: two warps take the tiles alternately (the hand-over between two tiles leaves the pipe idle otherwise); fp32: one.
@@ -379,9 +381,9 @@ umma_conv3x3_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
                   }
                }
             }
-            warp_commit(&empty_bar[s]);
+            wait.commit(&empty_bar[s]);
          }
-         warp_commit(&tmem_full[buf]);
+         wait.commit(&tmem_full[buf]);
       }
       wait.finish(&drain_bar[issuer], &abort_flag, status, kStatusWaitFull, lt);
    } else if (KIND == kTF32 && warp >= 2 + EPI_WARPS) {
@@ -452,7 +454,7 @@ umma_conv3x3_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_consta
       }
    }
    SOFIE_PROF_REPORT(warp == 0 ? "producer" : ((warp == 1 || (KIND == kI8 && warp == kConvIssuerB)) ? "mma" : (warp < 2 + EPI_WARPS ? "epilogue" : "converter")));
-   // A wait gives up only after about a second, long after every copy and MMA of this CTA landed.
+   // no copy or MMA is under way any more: the roles that issue them wait for them before they end
    tc_fence_before();
    __syncthreads();
    if (warp == 1) {
@@ -616,6 +618,8 @@ umma_conv3x3_patch_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
             warp_tma_load_4d(slot_hi(s), &tmX, grp * (PB / ES), w0 - 1, h0 - 1, n0, &full_bar[s]);
          }
       }
+      mbar_drain(&w_full, 0);
+      drain_copies(full_bar, s, ph, g, S);
    } else if (warp == 1 || warp >= kPatchIssuerB) {
       // ---------------- MMA issuers ----------------
       // Different warps take the tiles of this CTA in turn (the accumulator buffers go round with the tile
@@ -676,9 +680,9 @@ umma_conv3x3_patch_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
                      }
                   }
                }
-               warp_commit(&empty_bar[s]);
+               wait.commit(&empty_bar[s]);
             }
-            warp_commit(&tmem_full[buf]);
+            wait.commit(&tmem_full[buf]);
          }
          wait.finish(&drain_bar[issuer], &abort_flag, status, kStatusWaitFull, lt);
       }

@@ -572,8 +572,11 @@ __device__ __noinline__ void half_careful_tiles(const HalfConvParams &p, HalfSha
          for (; more; q[group]++) {
             const HalfPlace slot(group, q[group], half_careful_slots(BN, C)), buf(group, q[group], half_buffers(BN) / 2);
             if (!mbar_wait_warp(&sh.careful_op_full[slot.at], slot.phase, &sh.abort_flag, status, kStatusWaitConv, 0xb000 + lt) ||
-                !mbar_wait_warp(&sh.careful_tmem_empty[buf.at], buf.phase ^ 1u, &sh.abort_flag, status, kStatusWaitAccum, 0xb000 + lt))
+                !mbar_wait_warp(&sh.careful_tmem_empty[buf.at], buf.phase ^ 1u, &sh.abort_flag, status, kStatusWaitAccum, 0xb000 + lt)) {
+               warp_commit(&sh.drain[0]); // what is under way ends before the tensor memory is given back
+               mbar_drain(&sh.drain[0], 0);
                return;
+            }
             more = __any_sync(0xFFFFFFFFu, sh.careful_found[group][q[group] & 3] & kHalfWide);
             tc_fence_after();
             half_issue<BN, C>(sh.tmem_base + (uint32_t)(buf.at * 2 * BN), smem_u32(ops + (size_t)slot.at * 2 * half_part_bytes(C)), smem_u32(w_smem));
@@ -664,9 +667,7 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
          // rows and columns start at -1: zero fill; the channel coordinate is 0
          warp_tma_load_4d(raws + (size_t)s * RAW, &tmX, 0, tw.tw * kHalfTileW - 1, tw.th * kHalfTileH - 1, tw.n, &sh.raw_full[s]);
       }
-      // the copies of patches that nobody looks at end before the kernel does
-      if (unread())
-         for (int i = 0; i < g && i < SLOTS; i++) mbar_wait(&sh.raw_full[i], 0, &sh.abort_flag, status, kStatusWaitFull, 0x8000);
+      drain_copies(sh.raw_full, s, ph, g, SLOTS); // and of patches that nobody looks at
    } else if (warp == 1 || warp == ISSUER_B) {
       // ---------------- MMA issuers: all tiles, or even and odd ones ----------------
       // one of them keeps the pipe full with 36 MMAs a tile (32 channels: 185 us instead of 199), two do with 18 (320 instead of 338)
@@ -681,8 +682,8 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
          wait(&sh.tmem_empty[buf], ((uint32_t)(lt / NBUF) & 1u) ^ 1u);
          tc_fence_after();
          half_issue<BN, C>(tmem_base + (uint32_t)(buf * 2 * BN), smem_u32(ops + (size_t)s * 2 * PART), w);
-         warp_commit(&sh.op_empty[s]);
-         warp_commit(&sh.tmem_full[buf]);
+         wait.commit(&sh.op_empty[s]);
+         wait.commit(&sh.tmem_full[buf]);
       }
       wait.finish(&sh.drain[parity], &sh.abort_flag, status, kStatusWaitConv, 0x2000);
    } else if (warp >= 2 + kHalfEpiWarps) {

@@ -313,10 +313,10 @@ umma_qconv3x3_pool_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
          tma_load_2d(w_smem + (size_t)item * B_TILE, &tmW, tap * p.C + ch * CBK, 0, &w_full);
       }
       griddep_wait(); // the activations are the previous kernel's output
-      int s = 0;
+      int s = 0, g = 0;
       uint32_t ph = 0;
       bool ok = true;
-      for (int tile = blockIdx.x, g = 0; tile < p.num_tiles && ok; tile += gridDim.x, g++, ring_next(s, ph, S)) {
+      for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, g++, ring_next(s, ph, S)) {
          const int n = tile / per_image, rem = tile - n * per_image;
          const int h0 = (rem / p.tilesW) * kPoolTileH, w0 = (rem % p.tilesW) * kPoolTileW;
          ok = mbar_wait_warp(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g);
@@ -329,6 +329,8 @@ umma_qconv3x3_pool_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
          warp_tma_load_5d(slot, &tmX, 0, 1, w0 / 2 - 1, h0 - 1, n, &full_bar[s]);
          warp_tma_load_5d(slot + BOX_STRIDE, &tmX, 0, 0, w0 / 2, h0 - 1, n, &full_bar[s]);
       }
+      mbar_drain(&w_full, 0);
+      drain_copies(full_bar, s, ph, g, S);
    } else if (warp == 1 || warp >= kPoolFirstExtraIssuer) {
       // ---------------- MMA issuers: warp `pos` issues the nine taps of window position pos of every tile ----------------
       const int pos = warp == 1 ? 0 : warp - kPoolFirstExtraIssuer + 1;
@@ -368,8 +370,8 @@ umma_qconv3x3_pool_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
                warp_mma<kI8>(d, adesc, bdesc, idesc, (tap | kk) ? 1u : 0u);
             }
          }
-         warp_commit(&empty_bar[s]);
-         warp_commit(&tmem_full[buf]);
+         wait.commit(&empty_bar[s]);
+         wait.commit(&tmem_full[buf]);
       }
       wait.finish(&drain_bar[pos], &abort_flag, status, kStatusWaitFull, lt);
    } else if (warp < 2 + kPoolEpiWarps) {
@@ -477,14 +479,15 @@ umma_qconv3x3_first_pool_kernel(const __grid_constant__ CUtensorMap tmX, const i
       griddep_wait(); // the input is the previous kernel's output
       PoolTileWalker tw;
       tw.init(blockIdx.x, gridDim.x, p.tilesH, p.tilesW);
-      int s = 0;
+      int s = 0, g = 0;
       uint32_t ph = 0;
-      for (int tile = blockIdx.x, g = 0; tile < p.num_tiles; tile += gridDim.x, g++, ring_next(s, ph, S), tw.next()) {
+      for (int tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, g++, ring_next(s, ph, S), tw.next()) {
          if (!mbar_wait_warp(&raw_empty[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, g)) break;
          warp_expect_tx(&raw_full[s], kFirstRawBytes);
          // box {48 bytes, 34 rows, 1 image} from column w0 - 16 (a 16-byte boundary), row h0 - 1
          warp_tma_load_3d(raw_slots + (size_t)s * kFirstRawStride, &tmX, tw.tw * kPoolTileW - 16, tw.th * kPoolTileH - 1, tw.n, &raw_full[s]);
       }
+      drain_copies(raw_full, s, ph, g, S);
    } else if (warp == 1 || warp == kFirstIssuerB) {
       // ---------------- MMA issuers: one MMA per tile; even tiles warp 1, odd tiles the last warp ----------------
       // (an even number of operand slots and of TMEM buffers: each of them always meets the same issuer)
@@ -504,8 +507,8 @@ umma_qconv3x3_first_pool_kernel(const __grid_constant__ CUtensorMap tmX, const i
          const uint32_t d = tmem_base + (uint32_t)(buf * 4 * BN);
          const uint32_t lo = a_lo_word + (uint32_t)(s * (kFirstABytes >> 4)) * (1u - 65536u);
          warp_mma<kI8>(d, ((uint64_t)a_hi_word << 32) | lo, bdesc, idesc, 0u);
-         warp_commit(&a_empty[s]);
-         warp_commit(&tmem_full[buf]);
+         wait.commit(&a_empty[s]);
+         wait.commit(&tmem_full[buf]);
       }
       wait.finish(&drain_bar[warp == 1 ? 0 : 1], &abort_flag, status, kStatusWaitFull, 0x4000);
    } else if (warp < 2 + kPoolEpiWarps) {

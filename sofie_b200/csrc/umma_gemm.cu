@@ -420,6 +420,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             warp_tma_load_2d(b_hi(s), &tmB, kb * KE, n0, &full_bar[s]);
          }
       }
+      drain_copies(full_bar, s, ph, g, S);
    } else if (warp == 1) {
       // ---------------- MMA issuer ----------------
       constexpr uint32_t idesc = make_idesc<KIND>(kBM, BN);
@@ -453,9 +454,9 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
                      warp_mma<KIND>(d_tmem, da + koff, db + koff, idesc, accumulate);
                   }
                }
-               warp_commit(&empty_bar[s]); // the stage is free once these MMAs have read it
+               wait.commit(&empty_bar[s]); // the stage is free once these MMAs have read it
             }
-            warp_commit(&tmem_full[buf]);
+            wait.commit(&tmem_full[buf]);
          }
       }
       wait.finish(&drain_bar, &abort_flag, status, kStatusWaitFull, u);
@@ -570,8 +571,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
    }
    SOFIE_PROF_REPORT(warp == 0 ? "producer" : (warp == 1 ? "mma" : (warp < 2 + EPI_WARPS ? "epilogue" : "converter")));
-   // A wait only gives up after about a second, long after every copy and MMA this CTA issued has
-   // landed, so nothing is in flight when the TMEM columns are released below.
+   // no copy or MMA is under way any more: the roles that issue them wait for them before they end
    tc_fence_before();
    __syncthreads();
    if (warp == 1) {
@@ -669,6 +669,9 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
             warp_tma_load_2d_pair(b_tile(s), &tmB, kb * kStageK, n0, full_leader);
          }
       }
+      // Both CTAs' copies count on the leader's barriers. (After a give-up the peer may have filled slots that the leader's producer had not
+      // posted yet: it did so while slots were still given back, a wait's limit before any wait ran out.)
+      if (rank == 0) drain_copies(full_bar, s, ph, g, S);
    } else if (warp == 1) {
       // ---------------- MMA issuer (leader CTA only) ----------------
       if (rank == 0) {
@@ -691,15 +694,15 @@ umma_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                   const uint64_t koff = (uint64_t)(k * (kMmaK >> 4));
                   warp_mma_pair<KIND>(d_tmem, da + koff, db + koff, idesc, (kb == 0 && k == 0) ? 0u : 1u);
                }
-               warp_commit_pair(&empty_bar[s], 3); // both CTAs' slots are free once these MMAs have read them
+               warp_commit_pair(&empty_bar[s], 3, wait.gave_up); // both CTAs' slots are free once these MMAs have read them
             }
-            warp_commit_pair(&tmem_full[buf], 3);
+            warp_commit_pair(&tmem_full[buf], 3, wait.gave_up);
          }
          if (wait.gave_up) { // what is under way ends before the tensor memory is given back
-            if (lane == 0 && !abort_flag) mbar_give_up(&abort_flag, status, kStatusWaitFull, u);
+            if (lane == 0) mbar_give_up(&abort_flag, status, kStatusWaitFull, u);
             __syncwarp();
-            warp_commit_pair(&drain_bar, 1);
-            for (int n = 0; !__any_sync(0xFFFFFFFFu, mbar_try_wait(&drain_bar, 0)) && ++n < 4096;) {}
+            warp_commit_pair(&drain_bar, 1, 0);
+            mbar_drain(&drain_bar, 0);
          }
       }
    } else {
@@ -811,15 +814,16 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
    const int lane_base = (warp & 3) * 32, group = (warp - 2) >> 2; // epilogue warps: a lane quarter, every fourth chunk of 32 columns
    const uint32_t t_row = tmem_base + ((uint32_t)lane_base << 16);
 
+   int s = 0, issued = 0;
+   uint32_t ph = 0;
    if (warp == 0) {
       griddep_wait(); // A is the previous kernel's output
-      int s = 0;
-      uint32_t ph = 0;
       for (int kb = kb0; kb < kb1; kb++, ring_next(s, ph, S)) {
          if (!mbar_wait_warp(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, kb)) break;
          warp_expect_tx(&full_bar[s], L::kATile + L::kBTile);
          warp_tma_load_2d(a_tile(s), &tmA, kb * kStageK, m0, &full_bar[s]);
          warp_tma_load_2d(b_tile(s), &tmB, kb * kStageK, n0, &full_bar[s]);
+         issued++;
       }
    } else if (warp == 1) {
       constexpr uint32_t idesc = make_idesc<KIND>(kBM, BN);
@@ -835,9 +839,9 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
             const uint64_t koff = (uint64_t)(k * (kMmaK >> 4));
             warp_mma<KIND>(tmem_base, da + koff, db + koff, idesc, (kb == kb0 && k == 0) ? 0u : 1u);
          }
-         warp_commit(&empty_bar[s]);
+         wait.commit(&empty_bar[s]);
       }
-      warp_commit(&tmem_full);
+      wait.commit(&tmem_full);
       wait.finish(&drain_bar, &abort_flag, status, kStatusWaitFull, kb1);
    } else {
       mbar_wait(&tmem_full, 0, &abort_flag, status, kStatusWaitAccum, 0x3000);
@@ -845,6 +849,7 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
    }
    __syncwarp();
    cluster_sync_all(); // every rank's MMAs are done: the stages are free to take the others' pieces
+   if (warp == 0 && abort_flag) drain_copies(full_bar, s, ph, issued, S);
    if (warp >= 2 && !abort_flag) {
 #pragma unroll 1
       for (int c = group; c < CHUNKS; c += EPI_WARPS / 4) {

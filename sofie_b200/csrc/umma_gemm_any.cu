@@ -383,9 +383,9 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
                   warp_mma<kBF16>(d_tmem + BN, da0 + koff, db2 + koff, idesc, 1);
                   warp_mma<kBF16>(d_tmem + BN, da2 + koff, db0 + koff, idesc, 1);
                }
-               warp_commit(&empty_bar[s]);
+               wait.commit(&empty_bar[s]);
             }
-            warp_commit(&tmem_full[buf]);
+            wait.commit(&tmem_full[buf]);
          }
       }
       wait.finish(&drain_bar, &abort_flag, status, kStatusWaitConv, u);

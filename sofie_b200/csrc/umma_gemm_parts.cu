@@ -410,11 +410,7 @@ umma_gemm_parts_kernel(AnyOperand A, AnyOperand B, PartsLayout pa, PartsLayout p
             warp_bulk_load(smem + s * L::kStage + 3 * L::kA, b, 3 * L::kB, &full_bar[s]);
          }
       }
-      // after a give-up: the copies under way end before the block does
-      for (int i = g < L::kStages ? g : L::kStages; !ok && i > 0; i--) {
-         if (s-- == 0) s = L::kStages - 1, ph ^= 1u;
-         for (int n = 0; n < 1000 && !mbar_try_wait(&full_bar[s], ph); n++) {}
-      }
+      drain_copies(full_bar, s, ph, g, L::kStages);
    } else {
       // ---------------- MMA issuer ----------------
       constexpr uint32_t idesc_wide = make_idesc<kBF16>(kAnyBM, 2 * BN), idesc = make_idesc<kBF16>(kAnyBM, BN);
@@ -444,9 +440,9 @@ umma_gemm_parts_kernel(AnyOperand A, AnyOperand B, PartsLayout pa, PartsLayout p
                   warp_mma<kBF16>(d_tmem + BN, da0 + koff, db2 + koff, idesc, 1);
                   warp_mma<kBF16>(d_tmem + BN, da2 + koff, db0 + koff, idesc, 1);
                }
-               warp_commit(&empty_bar[s]);
+               wait.commit(&empty_bar[s]);
             }
-            warp_commit(&tmem_full[buf]);
+            wait.commit(&tmem_full[buf]);
          }
       }
       wait.finish(&drain_bar, &abort_flag, status, kStatusWaitFull, u);

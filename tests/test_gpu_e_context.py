@@ -55,6 +55,33 @@ def test_bounded_wait_runs_out_reports_once_and_the_context_stays_usable(cuda_de
         capi.call("sofie_cuda_ctx_destroy", b)
 
 
+@pytest.mark.parametrize("role,copied,detail", [(0, 8, None), (1, 5, "0x7e5c"), (2, 3, "0x7e59")])
+def test_waits_of_whole_warps_run_out(cuda_device, role, copied, detail):
+    """A warp whose wait ran out hands nothing on: the copying role gets no slot back from it (stages 0 to 4 of eight fit before that), the
+    reading role no accumulator; both leave at once, and the kernel ends behind the last copy and reports."""
+    ctx, stream = _ctx()
+    try:
+        src, out = torch.full((4096,), 3, dtype=torch.uint8, device=cuda_device), torch.zeros(5, dtype=torch.int32, device=cuda_device)
+        torch.cuda.synchronize()
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        external = torch.cuda.ExternalStream(stream.value)
+        a.record(external)
+        capi.call("sofie_cuda_selftest_warp_waits", stream, role, 200_000, C.c_void_p(src.data_ptr()), C.c_void_p(out.data_ptr()))
+        b.record(external)
+        if role:
+            with pytest.raises(capi.SofieCudaError) as e:
+                capi.call("sofie_cuda_ctx_check", ctx)
+            assert e.value.status == capi.ERR_DEVICE and "0x1ff" in str(e.value) and detail in str(e.value)
+        capi.call("sofie_cuda_ctx_check", ctx)
+        assert out.tolist() == [1, copied, 0 if role else 1, 1 if role else 0, 1]
+        assert a.elapsed_time(b) < (800 if role == 2 else 100)  # ms; the other roles' own limits: a second, and a quarter for the issuer
+        for args in ((3, 1000, src, out), (1, 10**12, src, out), (1, 1000, src[1:], out)):
+            with pytest.raises(capi.SofieCudaError):
+                capi.call("sofie_cuda_selftest_warp_waits", stream, args[0], args[1], *[C.c_void_p(t.data_ptr()) for t in args[2:]])
+    finally:
+        capi.call("sofie_cuda_ctx_destroy", ctx)
+
+
 def test_fetch_reports_a_kernel_that_gave_up(cuda_device):
     ctx, stream = _ctx()
     try:
