@@ -77,13 +77,15 @@ __host__ __device__ constexpr int half_weight_bytes(int BN, int C) { return 9 * 
 // Converter groups, which take the patches in turn: a patch's way through one (load, largest magnitude, barrier, split, store) is latency.
 // Patches in flight as fp32, and as many as parts: a multiple of the groups and of the two issuers, so that a slot always meets the same ones.
 __host__ __device__ constexpr int half_room(int BN, int C) { return (220 * 1024 - half_weight_bytes(BN, C)) / (half_raw_bytes(C) + 2 * half_part_bytes(C)); }
-__host__ __device__ constexpr int half_groups(int BN, int C) { return half_room(BN, C) >= 6 ? 3 : 2; }
+// (A third group where six patches fit gains at 32 columns only: with 64 it made the pooled layer 60.6 -> 64.4 us, 1024 images of 16 channels.)
+__host__ __device__ constexpr int half_groups(int BN, int C) { return BN == 32 && half_room(BN, C) >= 6 ? 3 : 2; }
 __host__ __device__ constexpr int half_slots(int BN, int C) { return half_room(BN, C) >= 6 ? 6 : (half_room(BN, C) >= 4 ? 4 : 2); }
 // slots of one group of careful tiles: the rings of passes and patches below are sized for two
 __host__ __device__ constexpr int half_careful_slots(int BN, int C) { return half_slots(BN, C) >= 4 ? 2 : 1; }
-// Epilogue warps of a tile: with 32 columns four, which read all of them, and the other four take the next tile. (Eight warps with 16 columns
-// each, all of them on every tile, set the kernel's time: 1200 clocks of latency a tile.)
-__host__ __device__ constexpr int half_epilogue_groups(int BN) { return BN == 32 ? 2 : 1; }
+// Epilogue warps of a pooled tile: with 32 columns four, which read all of them, and the other four take the next tile. (Eight warps with 16 columns
+// each, all of them on every tile, set the kernel's time: 1200 clocks of latency a tile.) Unpooled tiles write four times as much, which is what bounds
+// them, and eight warps write it sooner: 1024 x 16 x 32 x 32 to 16 channels 91 -> 47 us (with the words below).
+__host__ __device__ constexpr int half_epilogue_groups(int BN, bool POOL) { return BN == 32 && POOL ? 2 : 1; }
 __host__ __device__ constexpr int half_conv_warps(int BN, int C) { return half_groups(BN, C) * kHalfConvGroupWarps; }
 __host__ __device__ constexpr int half_issuer_b(int BN, int C) { return 2 + kHalfEpiWarps + half_conv_warps(BN, C); }
 __host__ __device__ constexpr int half_threads(int BN, int C) { return (half_issuer_b(BN, C) + 1) * 32; }
@@ -217,7 +219,7 @@ __device__ __forceinline__ bool half_window(const uint32_t *bits, int row, int c
    return (found & ((1u << (3 * C / 8)) - 1)) != 0;
 }
 
-// Two output channels of a pooled pixel / sixteen of a pixel
+// Two output channels of a pooled pixel / CH of a pixel
 __device__ __forceinline__ void half_store_pair(float *y, int c, int Cout, bool pairs, float v0, float v1)
 {
    if (pairs) {
@@ -227,16 +229,27 @@ __device__ __forceinline__ void half_store_pair(float *y, int c, int Cout, bool 
       if (c + 1 < Cout) y[1] = v1;
    }
 }
+// Whole 32-byte sectors where the row is aligned, else words of four channels as far as they go: 1024 x 16 x 32 x 32 to 64 channels 130 us in words,
+// 106 in sectors; to 28 channels 176 us where a row that is not whole went out value by value, 59 in words.
 template <int CH>
 __device__ __forceinline__ void half_store_row(float *y, int c, int Cout, const float (&r)[CH])
 {
-   if (c + CH <= Cout && (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
+   const uint32_t at = (uint32_t)reinterpret_cast<uintptr_t>(y);
+   if (c + CH <= Cout && (at & 31) == 0) {
 #pragma unroll
-      for (int j = 0; j < CH; j += 4) *reinterpret_cast<float4 *>(y + j) = make_float4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+      for (int j = 0; j < CH; j += 8)
+         asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(y + j), "f"(r[j]), "f"(r[j + 1]), "f"(r[j + 2]), "f"(r[j + 3]),
+                      "f"(r[j + 4]), "f"(r[j + 5]), "f"(r[j + 6]), "f"(r[j + 7])
+                      : "memory");
    } else {
+      const bool words = (at & 15) == 0;
 #pragma unroll
-      for (int j = 0; j < CH; j++)
-         if (c + j < Cout) y[j] = r[j];
+      for (int j = 0; j < CH; j += 4)
+         if (words && c + j + 4 <= Cout) *reinterpret_cast<float4 *>(y + j) = make_float4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+         else
+#pragma unroll
+            for (int i = j; i < j + 4; i++)
+               if (c + i < Cout) y[i] = r[i];
    }
 }
 
@@ -601,7 +614,7 @@ umma_conv3x3_half_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_c
    constexpr int UPP = C / 8;                      // units of eight channels per pixel
    constexpr int W_ITEM = 2 * BN * RB;             // one tap's weights: BN leading rows, BN trailing rows
    constexpr int NBUF = half_buffers(BN);
-   constexpr int SLOTS = half_slots(BN, C), GROUPS = half_groups(BN, C), ISSUER_B = half_issuer_b(BN, C), EPI_GROUPS = half_epilogue_groups(BN);
+   constexpr int SLOTS = half_slots(BN, C), GROUPS = half_groups(BN, C), ISSUER_B = half_issuer_b(BN, C), EPI_GROUPS = half_epilogue_groups(BN, POOL);
    static_assert(SLOTS % GROUPS == 0, "a slot always meets the same converter group");
    constexpr uint32_t TMEM_COLS = NBUF * 2 * BN;
    constexpr int CW = BN / 2 * EPI_GROUPS;         // channels per epilogue warp

@@ -306,6 +306,28 @@ def test_conv3x3_f32_in_half_precision_parts(N, C, H, W, Cout, relu, pool, value
     assert torch.equal(y[~finite].float().nan_to_num(2.0, 1.0, -1.0), ref[~finite].float().nan_to_num(2.0, 1.0, -1.0))
 
 
+# how a row of channels leaves: whole sectors, words of four, single values, the last of them partly, and every alignment of the result
+@pytest.mark.parametrize("Cout", [1, 4, 6, 8, 12, 16, 17, 20, 24, 28, 31, 32, 36, 40, 56, 64, 72])
+@pytest.mark.parametrize("C", [16, 32])
+def test_conv3x3_f32_in_half_precision_parts_rows_of_channels(C, Cout):
+    g = torch.Generator(device="cuda").manual_seed(C + Cout)
+    N, H, W = 3, 32, 24
+    x, w, b = (torch.randn(s, device="cuda", generator=g) for s in ((N, C, H, W), (Cout, C, 3, 3), (Cout,)))
+    x[1, 3, 4, 5] = 2.0 ** 40                                            # a tile of the careful form, whose rows leave by sixteen channels
+    ref, size = (torch.nn.functional.conv2d(f(x.double()), f(w.double()), f(b.double()), padding=1).permute(0, 2, 3, 1) for f in (lambda t: t, torch.abs))
+    X, P = x.permute(0, 2, 3, 1).contiguous(), ops.conv2d_pack_f32(w)
+    first = None
+    for offset in (0, 1, 2, 4):                                          # floats past a 256-byte boundary
+        whole = torch.full((N * H * W * Cout + 16,), 7.0, device="cuda")
+        y = whole[offset: offset + N * H * W * Cout]
+        ops.conv2d_f32(X, P, b, shape=x.shape, pad=(1, 1), x_layout=1, y_layout=1, w_packed=True, kernel=(3, 3), out=y.view(N, H, W, Cout))
+        assert ops.last_engine() == capi.ENGINE_TCGEN05
+        assert (whole[:offset] == 7).all() and (whole[offset + y.numel():] == 7).all()
+        first = y.clone() if first is None else first
+        assert torch.equal(y, first)
+    assert ((first.view(ref.shape).double() - ref).abs() <= (2 * 9 * C // 16 + 4) * 2.0 ** -23 * size).all()
+
+
 # many tiles a CTA, plain ones and such that take one pass, several or chains, in turn: their rings of slots, accumulators and patches come round
 @pytest.mark.parametrize("wide_weights", [0, 1])
 @pytest.mark.parametrize("N,C,H,W,Cout,pool", [(700, 16, 32, 32, 32, 2), (900, 32, 16, 32, 64, 0), (500, 16, 32, 32, 128, 2), (1700, 32, 16, 16, 24, 0)])
