@@ -77,7 +77,8 @@ gemm_f32_simt_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, const f
 // Products of few FMAs, whatever the layout: what bounds them is latency. The kernel above walks K in steps of 16 with a round trip to memory
 // and two barriers each (2 x 1 x 427 34 us), the tensor-core kernels set themselves up (6 to 8 us). Here T lanes share an output, each with every
 // T-th term of K, all loads of eight terms issued together, and add up their sums in pairs: 2 x 1 x 427 2.7 us, 5 x 2 x 166 21.7 -> 2.3,
-// 2 x 119 x 66 12.1 -> 2.6. Sums carry what products and additions round off in a second
+// 2 x 119 x 66 12.1 -> 2.6. From 1024 terms on a lane of 32 would have more than four such batches, 0.3 us each one after the other, and the split-K
+// kernel would be the faster one: a block of 256 shares the output (3 x 6 x 7858 11.5 -> 5.1 us, split-K 5.9; 1 x 2 x 5995 8.7 -> 4.1, split-K 4.3). Sums carry what products and additions round off in a second
 // word (T. Ogita, S. M. Rump and S. Oishi, "Accurate sum and dot product", 2005), which costs nothing here: no other kernel's are closer. (In 64 bits
 // the same took 71 us for 1 x 1 x 16384.)
 struct TwoSum {
@@ -96,12 +97,12 @@ struct TwoSum {
    }
 };
 template <int T>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(T > 128 ? T : 128)
 gemm_f32_tiny_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, const float *__restrict__ B, const float *C, float *Y)
 {
    griddep_launch_dependents();
    griddep_wait(); // the operands may be the previous kernel's output
-   const int i = (blockIdx.x * 128 + threadIdx.x) / T, t = threadIdx.x % T;
+   const int i = (blockIdx.x * (T > 128 ? T : 128) + threadIdx.x) / T, t = threadIdx.x % T;
    const bool live = i < d.M * d.N;
    const int m = live ? i / d.N : 0, n = live ? i - m * d.N : 0;
    const long long as = d.transA ? d.M : 1, bs = d.transB ? 1 : d.N;
@@ -119,11 +120,21 @@ gemm_f32_tiny_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, const f
 #pragma unroll
       for (int j = 0; j < 8; j++) acc.add_product(x[j], y[j]);
    }
-#pragma unroll
-   for (int o = T / 2; o > 0; o /= 2) {
-      const float s = __shfl_down_sync(0xFFFFFFFFu, acc.s, o, T), c = __shfl_down_sync(0xFFFFFFFFu, acc.c, o, T);
-      acc.add(s);
-      acc.c += c;
+   auto add_up = [&](int lanes) { // of a group of lanes, into its first
+      for (int o = lanes / 2; o > 0; o /= 2) {
+         const float s = __shfl_down_sync(0xFFFFFFFFu, acc.s, o, lanes), r = __shfl_down_sync(0xFFFFFFFFu, acc.c, o, lanes);
+         acc.add(s);
+         acc.c += r;
+      }
+   };
+   add_up(T > 32 ? 32 : T);
+   if constexpr (T > 32) { // an output is a block's: the sums of its warps
+      __shared__ float2 warps[T / 32];
+      if (t % 32 == 0) warps[t / 32] = make_float2(acc.s, acc.c);
+      __syncthreads();
+      if (t >= 32) return;
+      acc.s = warps[t % (T / 32)].x, acc.c = warps[t % (T / 32)].y;
+      add_up(T / 32);
    }
    if (t == 0 && live) {
       float sum = acc.s + acc.c;
@@ -151,12 +162,12 @@ int launch_gemm_f32_tiny(cudaStream_t s, const sofie_gemm_f32_desc &d, const flo
 {
    const int outputs = d.M * d.N;
    auto launch = [&](auto lanes) {
-      constexpr int T = decltype(lanes)::value;
-      return launch_dependent(gemm_f32_tiny_kernel<T>, dim3(ceil_div(outputs * T, 128)), dim3(128), 0, s, d, A, B, C, Y);
+      constexpr int T = decltype(lanes)::value, threads = T > 128 ? T : 128;
+      return launch_dependent(gemm_f32_tiny_kernel<T>, dim3(ceil_div(outputs * T, threads)), dim3(threads), 0, s, d, A, B, C, Y);
    };
-   // as many lanes as keep a lane's terms to one batch of loads
+   // as many lanes as keep a lane's terms to one batch of loads; 256 for 740 to 1024 terms of a hundred outputs and more are up to 10 % slower than 32
    SOFIE_CUDA_TRY(d.K <= 8 ? launch(std::integral_constant<int, 1>{}) : d.K <= 32 ? launch(std::integral_constant<int, 4>{}) :
-                  d.K <= 128 ? launch(std::integral_constant<int, 16>{}) : launch(std::integral_constant<int, 32>{}));
+                  d.K <= 128 ? launch(std::integral_constant<int, 16>{}) : d.K <= 1024 ? launch(std::integral_constant<int, 32>{}) : launch(std::integral_constant<int, 256>{}));
    set_last_engine(SOFIE_ENGINE_SIMT);
    return SOFIE_CUDA_OK;
 }

@@ -919,6 +919,25 @@ def test_gemm_f32_of_few_fmas(M, N, K):
                 assert torch.equal(y.isfinite(), ~odd) and torch.equal(y[odd].nan_to_num(1., 2., 3.), chain[odd].nan_to_num(1., 2., 3.))
 
 
+# an output shared by a block: one batch of loads and many, the last term and the last batch alone, one output and the most there can be
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1025), (3, 5, 2048), (2, 9, 2049), (16, 15, 1091), (1, 32, 8192), (255, 1, 1028), (4, 8, 4097)])
+@pytest.mark.parametrize("tA,tB", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_gemm_f32_of_few_fmas_and_many_terms(M, N, K, tA, tB):
+    if tB and not tA and K % 4 == 0 and N <= 16:
+        pytest.skip("the row kernel's")
+    g = torch.Generator(device="cuda").manual_seed(M * N + K)
+    A, B = torch.randn((K, M) if tA else (M, K), device="cuda", generator=g), torch.randn((N, K) if tB else (K, N), device="cuda", generator=g)
+    c = torch.randn(M, N, device="cuda", generator=g)
+    ops.set_engine(0)
+    y = ops.gemm_f32(A, B, c, transA=tA, transB=tB, alpha=0.75, beta=1.5)
+    product = (A.t() if tA else A).double() @ (B.t() if tB else B).double()
+    # the sum, alpha, beta and the bias round once each; the second word is good to K 2^-24 of what it holds
+    assert ((y.double() - (0.75 * product + 1.5 * c.double())).abs() <= 4 * 2.0 ** -24 * ((0.75 * product).abs() + 1.5 * c.double().abs()) + K * K * 2.0 ** -48).all()
+    A.view(-1)[0] = float("inf")                                     # the first row's sums are infinite, the others as they were
+    z = ops.gemm_f32(A, B, c, transA=tA, transB=tB, alpha=0.75, beta=1.5)
+    assert torch.equal(z[0], (B.t() if tB else B)[0].sign() * float("inf")) and torch.equal(z[1:], y[1:])
+
+
 # as many groups of eight channels as blocks beside a tile, or all of them in one; the last group partly empty
 @pytest.mark.parametrize("N,C,H,W,Cout,pool", [(2, 3, 12, 12, 30, 0), (70, 1, 17, 40, 64, 2), (75, 4, 16, 32, 64, 0), (5, 2, 33, 9, 9, 2), (600, 3, 16, 16, 8, 0)])
 @pytest.mark.parametrize("nhwc", [0, 1])
