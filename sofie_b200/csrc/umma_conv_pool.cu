@@ -122,9 +122,10 @@ __device__ __forceinline__ uint32_t pack4_u8(const float (&p)[4]) // of products
 // channels). More buffers in flight hide more of the fixed latency of a tile's trip through the barriers, which is
 // what bounds a kernel whose tiles carry little arithmetic. lane = pooling window; its four accumulators lie BN
 // columns apart.
-// SMALL: sums without bias lie in (-2^23, 2^23).
+// SMALL: sums without bias lie in (-2^23, 2^23) -- nine taps of one channel do, of 32 channels (9400320 at most) they do not --, and the multipliers
+// times 2^100 stand behind the multipliers.
 template <int BN, int NBUF, bool SMALL>
-__device__ __forceinline__ void pool_epilogue_warp(const PoolConvParams &p, const float *s_mult, const int *s_qbias, bool pool_first,
+__device__ __forceinline__ void pool_epilogue_warp(const PoolConvParams &p, const float (&s_mult)[SMALL ? 128 : 64], const int *s_qbias, bool pool_first,
                                                    uint32_t tmem_base, uint64_t *tmem_full, uint64_t *tmem_empty,
                                                    volatile uint32_t *abort_flag, uint32_t *status, int warp, int lane)
 {
@@ -375,7 +376,7 @@ umma_qconv3x3_pool_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_
       }
       wait.finish(&drain_bar[pos], &abort_flag, status, kStatusWaitFull, lt);
    } else if (warp < 2 + kPoolEpiWarps) {
-      pool_epilogue_warp<BN, 2, (288 * KPS * 255 * 128 < 1 << 23)>(p, s_mult, s_qbias, pool_first, tmem_base, tmem_full, tmem_empty, &abort_flag, status, warp, lane);
+      pool_epilogue_warp<BN, 2, false>(p, s_mult, s_qbias, pool_first, tmem_base, tmem_full, tmem_empty, &abort_flag, status, warp, lane);
    }
    tc_fence_before();
    __syncthreads();
