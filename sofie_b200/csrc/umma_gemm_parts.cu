@@ -506,7 +506,9 @@ struct PartsPlan {
 // a cluster; at least the writes of Y. Clusters of 4 / 8 found room for 132 / 96 CTAs at a time.
 // Against the other kernels' estimate, which is 20 % low in the mean: the split pays from about 2^20 outputs or 2^24 FMAs a tile on. 1000 x 777 x
 // 1333 with A transposed and a full bias 39 -> 25.7 us, 4096 x 4096 x 2048 522 -> 302, 785 x 2853 x 683 64 -> 35, 16384 x 777 x 64 59 -> 32; of the 2800
-// (M and N from 48 on) it takes three in five, and 0.3 % of them are more than 3 % slower.
+// (M and N from 48 on) it takes three in five, and 0.3 % of them are more than 3 % slower. With 32 to 47 rows
+// or columns it takes a fifth of 260, 0.84 of the other kernels' time in the mean, but below K = 256 six of 12 took 3 to 15 % longer (41 x 17142 x 180 14.6 us
+// without, 16.7 with): those are left to the others.
 PartsPlan parts_plan(const sofie_gemm_f32_desc &d)
 {
    static const int widths[4] = {128, 96, 64, 32}, stage[4] = {505, 441, 404, 347}, end[4] = {1908, 1421, 586, 214}, room[4] = {kNumSMs, kNumSMs, 132, 96};
@@ -514,6 +516,7 @@ PartsPlan parts_plan(const sofie_gemm_f32_desc &d)
    const int tm = ceil_div(d.M, kAnyBM), nkb = ceil_div(d.K, kAnyKE);
    const bool full = d.bias_kind == 2, tma = !d.transA && d.transB && d.K % 4 == 0;
    if (d.M < 32 || d.N < 32 || (!forced_engine() && gemm_f32_tiny_ok(d))) return p;  // hardly a tile: not measured, and the skinny products have more precise kernels
+   if (d.K < 256 && (d.M < 48 || d.N < 48)) return p;
    if (d.K < 48) return p; // the writes of Y count, and short K leaves the split little to save: 16384 x 4093 x 8 169 us either way
    const long long split = 4560 + 1817 * (((long long)d.M + d.N) * nkb * kAnyKE) / 1000000, out = 1361 * ((long long)d.M * d.N * (full ? 2 : 1)) / 1000000;
    long long best = -1;

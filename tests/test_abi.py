@@ -65,6 +65,16 @@ def test_status_strings_and_argument_errors():
         capi.call("sofie_cuda_set_engine", 7)
 
 
+@pytest.mark.parametrize("M,N,K,taken", [(41, 17142, 180, 0), (17142, 41, 255, 0), (36, 3000, 3905, 1), (172, 33, 3880, 1), (48, 17142, 180, 1), (31, 3000, 3905, 0),
+                                         (1000, 777, 1333, 1), (16384, 4093, 8, 0), (64, 64, 64, 0), (8192, 8192, 8192, 1), (65536, 65536, 4096, 0)])
+def test_workspace_is_asked_for_where_the_split_was_measured_to_pay(M, N, K, taken):
+    """Six bytes a value of whole tiles of A and B, 1 GiB at most; from 32 rows and columns on, below 48 from K = 256 on."""
+    d = capi.GemmF32Desc(M, N, K, 1, 0, 1.0, 1.0, 2, 0)
+    nbytes = capi.load().sofie_cuda_gemm_f32_workspace(C.byref(d))
+    assert (nbytes > 0) == bool(taken) and nbytes <= 1 << 30
+    assert not taken or 6 * K * (M + N) <= nbytes <= 6 * (K + 31) * (M + 127 + N + 127)
+
+
 def test_no_gpu_means_loud_failure_not_cpu_fallback():
     """Without a device the context cannot be created; nothing computes on the CPU instead."""
     import torch
