@@ -229,8 +229,8 @@ typedef struct sofie_gemm_f32_desc {
 int sofie_cuda_gemm_f32(void *stream, const sofie_gemm_f32_desc *desc, const float *A, const float *B,
                         const float *C, float *Y);
 /* The same product for a caller that has device memory to spare for the duration of the call: _workspace gives the bytes (256-byte
- * aligned memory) with which it is faster, 0 where a workspace gains nothing; _ws takes them. With less, or NULL, _ws is
- * sofie_cuda_gemm_f32. Same inputs, results and errors. */
+ * aligned memory, at most 1 GiB) with which it is faster, 0 where a workspace gains nothing; _ws takes them. With less, or NULL, _ws is
+ * sofie_cuda_gemm_f32. Same inputs, errors and error bound; the two run different kernels, whose results may differ in their last bits. */
 size_t sofie_cuda_gemm_f32_workspace(const sofie_gemm_f32_desc *desc);
 int sofie_cuda_gemm_f32_ws(void *stream, const sofie_gemm_f32_desc *desc, const float *A, const float *B, const float *C, float *Y,
                            void *workspace, size_t bytes);

@@ -147,7 +147,7 @@ void require(bool ok, const char *what)
    if (!ok) raise(PyExc_AssertionError, what);
 }
 
-// A, B, C, transA, transB, alpha, beta, relu, out
+// A, B, C, transA, transB, alpha, beta, relu, out, workspace
 PyObject *gemm_f32(Args a)
 {
    const at::Tensor &A = tensor(a[0]), &B = tensor(a[1]);
@@ -166,7 +166,7 @@ PyObject *gemm_f32(Args a)
    const float *pA = as<float>(A), *pB = as<float>(B), *pC = as<float>(a[2]);
    float *pY = as<float>(Y);
    // a workspace where one makes the product faster, from torch's pool of this stream; without memory for it the product does without
-   const size_t bytes = sofie_cuda_gemm_f32_workspace(&d);
+   const size_t bytes = truth(a[9]) ? sofie_cuda_gemm_f32_workspace(&d) : 0;
    at::Tensor workspace;
    if (bytes) {
       try {
@@ -506,7 +506,7 @@ PyObject *entry(PyObject *, PyObject *const *args, Py_ssize_t n)
 }
 
 #define SOFIE_ENTRY(name, n) {#name, (PyCFunction)(void (*)(void))entry<name, n>, METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {SOFIE_ENTRY(gemm_f32, 9),       SOFIE_ENTRY(conv2d_f32, 15),     SOFIE_ENTRY(qlinear_conv2d, 15), SOFIE_ENTRY(relu_f32, 2),
+PyMethodDef methods[] = {SOFIE_ENTRY(gemm_f32, 10),       SOFIE_ENTRY(conv2d_f32, 15),     SOFIE_ENTRY(qlinear_conv2d, 15), SOFIE_ENTRY(relu_f32, 2),
                          SOFIE_ENTRY(unary_f32, 3),      SOFIE_ENTRY(binary_f32, 3),      SOFIE_ENTRY(batchnorm_f32, 9),   SOFIE_ENTRY(pool2d_f32, 8),
                          SOFIE_ENTRY(maxpool2d_u8, 5),   SOFIE_ENTRY(softmax_f32, 2),     SOFIE_ENTRY(change_layout, 2),   SOFIE_ENTRY(quantize_u8, 3),
                          SOFIE_ENTRY(dequantize_u8, 3),  SOFIE_ENTRY(quantize_e4m3, 2),   SOFIE_ENTRY(qlinear_matmul, 8),  SOFIE_ENTRY(gemm_e4m3, 9),

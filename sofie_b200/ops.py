@@ -46,9 +46,13 @@ def last_engine() -> int:
     return capi.load().sofie_cuda_last_engine()
 
 
-def gemm_f32(A, B, C_=None, *, transA=0, transB=0, alpha=1.0, beta=1.0, relu=False, out=None):
-    """ONNX Gemm / MatMul: Y = alpha*op(A)*op(B) + beta*broadcast(C), optional Relu."""
-    return _native().gemm_f32(A, B, C_, transA, transB, alpha, beta, relu, out)
+def gemm_f32(A, B, C_=None, *, transA=0, transB=0, alpha=1.0, beta=1.0, relu=False, out=None, workspace=True):
+    """ONNX Gemm / MatMul: Y = alpha*op(A)*op(B) + beta*broadcast(C), optional Relu.
+
+    Where it makes the product faster, six bytes per value of A and B (1 GiB at most) are taken from torch's pool for the duration of the call; when torch
+    has no memory for them the product does without. With workspace=False nothing but the result is allocated. The two forms round differently within
+    the same error bound."""
+    return _native().gemm_f32(A, B, C_, transA, transB, alpha, beta, relu, out, workspace)
 
 
 def conv_out_hw(H, W, kH, kW, pad, stride, dil=(1, 1)):

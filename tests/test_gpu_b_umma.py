@@ -558,6 +558,60 @@ def test_gemm_f32_of_operands_split_beforehand(M, N, K, bias):
     assert taken == 4
 
 
+@pytest.mark.parametrize("M,N,K,bias", [(1000, 777, 1333, 2), (64, 60, 4100, 0), (2049, 513, 257, 1), (36, 3000, 3905, 2)])
+@pytest.mark.parametrize("tA,tB", [(0, 0), (1, 1)])
+def test_gemm_f32_workspace_and_without(M, N, K, bias, tA, tB):
+    """The workspace is written as far as it was asked for and no further, under the automatic dispatch too; one byte less, none, a base that is not aligned,
+    workspace=False and no memory left are the plain call, bit for bit, and take nothing."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    lib = capi.load()
+    A, B = torch.randn((K, M) if tA else (M, K), device="cuda", generator=g), torch.randn((N, K) if tB else (K, N), device="cuda", generator=g)
+    C_ = {0: None, 1: torch.randn(N, device="cuda", generator=g), 2: torch.randn(M, N, device="cuda", generator=g)}[bias]
+    d = capi.GemmF32Desc(M, N, K, tA, tB, 0.75, 1.5, bias, 0)
+    pointers = [C.c_void_p(0 if t is None else t.data_ptr()) for t in (A, B, C_)]
+    for engine in (0, capi.ENGINE_TCGEN05):
+        ops.set_engine(engine)
+        nbytes = lib.sofie_cuda_gemm_f32_workspace(C.byref(d))
+        assert nbytes > 0
+        whole = torch.full((nbytes + 8192,), 0xA5, dtype=torch.uint8, device="cuda")
+
+        def product(offset, size):
+            Y = torch.full((M, N), 7.0, device="cuda")
+            capi.call("sofie_cuda_gemm_f32_ws", ops._stream(), C.byref(d), *pointers, C.c_void_p(Y.data_ptr()), C.c_void_p(whole.data_ptr() + offset), size)
+            return Y
+        plain = torch.full((M, N), 7.0, device="cuda")
+        capi.call("sofie_cuda_gemm_f32", ops._stream(), C.byref(d), *pointers, C.c_void_p(plain.data_ptr()))
+        for short in (product(4096, nbytes - 1), product(4096, 0), product(4096 + 64, nbytes)):
+            assert torch.equal(short, plain) and (whole == 0xA5).all()
+        exact = 0.75 * ((A.t() if tA else A).double() @ (B.t() if tB else B).double()) + (0 if C_ is None else 1.5 * C_.double())
+        y = product(4096, nbytes)
+        assert float((y.double() - exact).norm() / exact.norm()) <= 2.5e-7
+        assert (whole[:4096] == 0xA5).all() and (whole[4096 + nbytes:] == 0xA5).all() and not (whole[4096:4096 + nbytes] == 0xA5).all()
+        call = lambda **kw: ops.gemm_f32(A, B, C_, transA=tA, transB=tB, alpha=0.75, beta=1.5, **kw)
+        assert torch.equal(call(), y)
+        out = torch.empty(M, N, device="cuda")
+        taken = torch.cuda.memory_stats()["allocation.all.allocated"]
+        call(out=out, workspace=False)
+        assert torch.cuda.memory_stats()["allocation.all.allocated"] == taken
+        assert torch.equal(out, plain)
+        del y, whole
+        torch.cuda.empty_cache()
+        out.fill_(7.0)
+        hold = []
+        try:                                                             # no more than there is now, and that is held
+            torch.cuda.set_per_process_memory_fraction(torch.cuda.memory_reserved() / torch.cuda.get_device_properties(0).total_memory)
+            for size in (1 << 24, 1 << 21, 1 << 18):
+                with pytest.raises(torch.OutOfMemoryError):
+                    while True:
+                        hold.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            call(out=out)
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        del hold
+        assert torch.equal(out, plain)
+    ops.set_engine(0)
+
+
 # the form without conversions (zero point 0; one input channel without bias, and 32 with one): multipliers of zero, subnormal and far below one,
 # such that most products are ties, that saturate everything, the largest that stay with it (2^20) and larger ones
 @pytest.mark.parametrize("bias", [False, True])
