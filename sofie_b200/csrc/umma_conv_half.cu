@@ -24,11 +24,13 @@
 // - Two scales whose product leaves fp32's range are applied one after the other.
 // Error against float64 (2-norm), N(0,1) operands: 2.1e-7 at 16 and 3.7e-7 at 32 channels, where TF32 parts gave 7.0e-7 and 1.28e-6 (their trailing
 // part is truncated, these are rounded, and the sums take half as many steps); operands of one sign 6.1e-7 and 1.4e-6 (1.05e-6 and 2.4e-6).
-// 8192 images 16 -> 32 at 32 x 32 with MaxPool 490 -> 320 us, 32 -> 64 at 16 x 16 365 -> 187 us; unpooled 2048 x 16 -> 32 165 -> 144 us; one image
+// 8192 images 16 -> 32 at 32 x 32 with MaxPool 490 -> 322 us, 32 -> 64 at 16 x 16 365 -> 189 us; unpooled 2048 x 16 -> 32 165 -> 120 us; one image
 // 4.1 -> 4.0 and 5.5 -> 4.8 us when the kernel has just run, about 1 us more behind others (its instructions come from L2 then). Of the first:
-// channels 2^8 ... 2^40 apart 360; values down to 2^-28 of the largest and below in every patch 403; weights of a channel decayed to 1e-12 425; two
-// passes for every tile 1.5 ms, for images of exp(-r^2 / 8) 2.0, one infinity in each image 2.6 (as chains of FMAs in the epilogue, one scale and no check
-// of single sums, the last four took 20 ms, 10 for the infinities).
+// channels 2^8 ... 2^40 apart 340; values down to 2^-28 of the largest and below in every patch 436; weights of a channel decayed to 1e-12 460; two
+// passes for every tile 1.6 ms, for images of exp(-r^2 / 8) 1.9, one infinity in each image 3.4 (as chains of FMAs in the epilogue, one scale and no check
+// of single sums, the last four took 20 ms, 10 for the infinities). With two converter groups and all epilogue warps on every tile, in 96 registers and 115 KB,
+// these were 332, 360, 403, 427 us, 1.5, 2.0 and 2.6 ms: the check of single sums holds a tile longer now, and the chains have 80 registers and a
+// smaller L1 cache (parts packed closer, 159 KB: 3.07 ms, but 324 us; the check out of the epilogue's own sums: 413 us, but 335).
 //
 // A tile is 16 x 8 pixels of one image; one TMA box brings its 18 x 10 patch (zero fill outside the image) as fp32 rows; two or three groups of
 // four converter warps take the patches in turn, find the largest magnitude, split the values and write both parts as K-major swizzled
