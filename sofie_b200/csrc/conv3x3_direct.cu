@@ -195,6 +195,157 @@ int launch_direct(cudaStream_t s, const ConvGeom &g, const float *X, const float
    return SOFIE_CUDA_OK;
 }
 
+// ---- few tiles: the input channels of a tile shared out between the block's warps ------------------------------------------------
+// The kernel above walks a tile's channels one after the other in two warps: one image of 16 x 16 takes as long as 800 do (8 -> 16 channels 11.8 us,
+// 16 -> 16 17.5), most of it round trips. Here a block of eight warps owns 4 RH rows x 16 columns x 16 output channels; a warp takes four of the
+// rows and every (8 / RH)-th channel, a thread four outputs below one another x eight channels, and the sums of the 8 / RH warps meet in shared memory.
+// All of up to 32 channels' inputs and weights are one round trip of asynchronous copies. Chains are shorter than the other kernel's, sums no less exact.
+constexpr int kDsThreads = 256, kDsChunk = 32, kDsPitch = 24, kDsWPitch = 20; // 20: a warp's weights in four banks apart, 16 bytes aligned
+__host__ __device__ constexpr int ds_channel(int RH) { return (4 * RH + 2) * kDsPitch + 4; } // + 4: neighbouring channels start in other banks
+__host__ __device__ constexpr int ds_out(int RH) { return 4 * RH * 16 + 2; }
+__host__ __device__ constexpr int ds_partial(int RH) { return kDcOut * ds_out(RH); }
+
+template <int POOL, int RH, bool VEC>
+__global__ void __launch_bounds__(kDsThreads, 2)
+conv3x3_split_f32_kernel(ConvGeom g, const float *__restrict__ X, const float *__restrict__ Wt, const float *__restrict__ bias, float *__restrict__ Y, FastDiv tiles_x,
+                         FastDiv tiles_y, int chunk)
+{
+   constexpr int KS = 8 / RH, ROWS = 4 * RH + 2, CST = ds_channel(RH), OST = ds_out(RH);
+   extern __shared__ __align__(16) float smem[];
+   float *tile = smem;                 // [channel][row][column], from column w0 - 4 on
+   float *s_w = smem + chunk * CST;    // [channel][tap][16], rows of kDsWPitch
+   float *partial = smem;              // [sharer][output channel][row][column], where the inputs and weights were
+   __shared__ float s_bias[kDcOut];
+   griddep_launch_dependents();
+   griddep_wait();
+   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, oc_base = blockIdx.y * kDcOut, outs = min(kDcOut, g.Cout - oc_base);
+   if (tid < kDcOut) s_bias[tid] = tid < outs && bias ? __ldg(bias + oc_base + tid) : 0.f;
+   uint32_t tx, ty;
+   const uint32_t n = tiles_y.divmod(tiles_x.divmod(blockIdx.x, tx), ty);
+   const int h0 = (int)ty * 4 * RH, w0 = (int)tx * 16;
+   const int col = lane >> 1, oc_local = (lane & 1) * 8, half = warp / KS, sharer = warp % KS;
+   uint64_t acc2[4][4]; // two neighbouring channels each
+#pragma unroll
+   for (int q = 0; q < 4; q++)
+#pragma unroll
+      for (int o = 0; o < 4; o++) acc2[q][o] = 0;
+   for (int c0 = 0; c0 < g.C; c0 += chunk) {
+      const int ck = min(chunk, g.C - c0);
+      if (c0) __syncthreads(); // the chunk before this one is no longer read
+      auto copy4 = [](float *dst, const float *src, int bytes) {
+         asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+      };
+      if constexpr (VEC) {
+         constexpr int WORDS = kDsPitch / 4;
+         for (int i = tid; i < ck * ROWS * WORDS; i += kDsThreads) {
+            const int c = i / (ROWS * WORDS), p = i % (ROWS * WORDS), r = p / WORDS, w = p % WORDS;
+            const int ih = h0 - 1 + r, iw = w0 - 4 + 4 * w;
+            const bool in = ih >= 0 && ih < g.H && iw >= 0 && iw < g.W;
+            const float *src = in ? X + (((size_t)n * g.C + c0 + c) * g.H + ih) * g.W + iw : X;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(tile + c * CST + 4 * p)), "l"(src), "r"(in ? 16 : 0) : "memory");
+         }
+      } else {
+         constexpr int COLS = 18;
+         for (int i = tid; i < ck * ROWS * COLS; i += kDsThreads) {
+            // the index that is contiguous in memory runs fastest
+            const int c = g.x_nhwc ? i % ck : i / (ROWS * COLS), p = g.x_nhwc ? i / ck : i % (ROWS * COLS);
+            const int r = p / COLS, k = p % COLS, ih = h0 - 1 + r, iw = w0 - 1 + k;
+            const bool in = ih >= 0 && ih < g.H && iw >= 0 && iw < g.W;
+            const size_t at = g.x_nhwc ? (((size_t)n * g.H + ih) * g.W + iw) * g.C + c0 + c : (((size_t)n * g.C + c0 + c) * g.H + ih) * g.W + iw;
+            copy4(tile + c * CST + r * kDsPitch + 3 + k, in ? X + at : X, in ? 4 : 0);
+         }
+      }
+      // a filter's weights of these channels are consecutive in memory, tap by tap or channel by channel
+      for (int i = tid; i < kDcOut * ck * 9; i += kDsThreads) {
+         const int o = i / (ck * 9), e = i - o * (ck * 9);
+         const int c = g.w_packed ? e % ck : e / 9, rt = g.w_packed ? e / ck : e % 9;
+         copy4(s_w + (c * 9 + rt) * kDsWPitch + o, o < outs ? Wt + dc_weight_index(g, oc_base + o, c0 + c, rt) : Wt, o < outs ? 4 : 0);
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+      const float *in = tile + half * 4 * kDsPitch + col + 3;
+#pragma unroll 1
+      for (int c = sharer; c < ck; c += KS) {
+         uint64_t win[6][3]; // the inputs under the four outputs, each twice
+#pragma unroll
+         for (int r = 0; r < 6; r++)
+#pragma unroll
+            for (int t = 0; t < 3; t++) {
+               const float v = in[c * CST + r * kDsPitch + t];
+               win[r][t] = pack_f32x2(v, v);
+            }
+         const float *w = s_w + c * 9 * kDsWPitch + oc_local;
+#pragma unroll
+         for (int rt = 0; rt < 9; rt++)
+#pragma unroll
+            for (int o4 = 0; o4 < 2; o4++) {
+               const ulonglong2 wv = *reinterpret_cast<const ulonglong2 *>(w + rt * kDsWPitch + 4 * o4);
+#pragma unroll
+               for (int q = 0; q < 4; q++) {
+                  acc2[q][2 * o4] = fma_f32x2(win[q + rt / 3][rt % 3], wv.x, acc2[q][2 * o4]);
+                  acc2[q][2 * o4 + 1] = fma_f32x2(win[q + rt / 3][rt % 3], wv.y, acc2[q][2 * o4 + 1]);
+               }
+            }
+      }
+   }
+   __syncthreads(); // inputs and weights are no longer read
+   {
+      float *p = partial + sharer * ds_partial(RH) + oc_local * OST + half * 64 + col;
+#pragma unroll
+      for (int q = 0; q < 4; q++)
+#pragma unroll
+         for (int o = 0; o < 4; o++) {
+            float a, b;
+            unpack_f32x2(acc2[q][o], a, b);
+            p[2 * o * OST + q * 16] = a;
+            p[(2 * o + 1) * OST + q * 16] = b;
+         }
+   }
+   __syncthreads();
+   // one output of the convolution
+   auto output = [&](int o, int row, int column) {
+      const float *p = partial + o * OST + row * 16 + column;
+      float v = p[0];
+#pragma unroll
+      for (int k = 1; k < KS; k++) v += p[k * ds_partial(RH)];
+      v += s_bias[o];
+      return g.relu ? relu_ref(v) : v;
+   };
+   constexpr int SIDE = POOL == 2 ? 2 : 1, PR = 4 * RH / SIDE, PC = 16 / SIDE;
+   for (int i = tid; i < PR * PC * kDcOut; i += kDsThreads) {
+      // threads along what is contiguous in Y
+      const int o = g.y_nhwc ? i % kDcOut : i / (PR * PC), p = g.y_nhwc ? i / kDcOut : i % (PR * PC);
+      const int pr = p / PC, pc = p % PC, ph = h0 / SIDE + pr, pw = w0 / SIDE + pc;
+      if (o >= outs || ph >= g.pH || pw >= g.pW) continue;
+      float v = output(o, SIDE * pr, SIDE * pc);
+      if constexpr (POOL == 2) {
+         // the comparisons v > best from the window's first pixel on: a NaN counts there and is passed over elsewhere
+#pragma unroll
+         for (int k = 1; k < 4; k++) {
+            const float u = output(o, 2 * pr + k / 2, 2 * pc + k % 2);
+            v = u > v ? u : v;
+         }
+      }
+      Y[g.y_nhwc ? (((size_t)n * g.pH + ph) * g.pW + pw) * g.Cout + oc_base + o : (((size_t)n * g.Cout + oc_base + o) * g.pH + ph) * g.pW + pw] = v;
+   }
+}
+
+// -1 when the grid would not hold the tiles
+template <int POOL, int RH, bool VEC>
+int launch_split(cudaStream_t s, const ConvGeom &g, const float *X, const float *W, const float *bias, float *Y)
+{
+   const int tiles_x = ceil_div(g.oW, 16), tiles_y = ceil_div(g.oH, 4 * RH), chunk = g.C < kDsChunk ? g.C : kDsChunk;
+   const long long tiles = (long long)g.N * tiles_x * tiles_y;
+   if (tiles >= 1ll << 31) return -1;
+   const int staged = chunk * (ds_channel(RH) + 9 * kDsWPitch), sums = 8 / RH * ds_partial(RH), smem = (staged > sums ? staged : sums) * (int)sizeof(float);
+   auto kern = conv3x3_split_f32_kernel<POOL, RH, VEC>;
+   SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), smem));
+   SOFIE_CUDA_TRY(launch_dependent(kern, dim3((unsigned)tiles, ceil_div(g.Cout, kDcOut)), dim3(kDsThreads), smem, s, g, X, W, bias, Y, FastDiv(tiles_x), FastDiv(tiles_y), chunk));
+   SOFIE_LAUNCH_CHECK("conv3x3_split_f32_kernel");
+   set_last_engine(SOFIE_ENGINE_SIMT);
+   return SOFIE_CUDA_OK;
+}
+
 } // namespace
 
 // 3x3 / stride 1 / pad 1 / group 1 with at most 128 input channels (their weights for 16 outputs are 72 KB): -1 for any other shape.
@@ -204,19 +355,41 @@ int launch_conv2d_f32_direct3x3(cudaStream_t s, const ConvGeom &g, const float *
    if (g.C > 128 || (g.pool != 0 && g.pool != 2) || g.N < 1 || ceil_div(g.Cout, kDcOut) > 65535) return -1;
    const int chunks = ceil_div(g.C, kDcChunk);
    const bool vec = !g.x_nhwc && g.W % 4 == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0, wide = g.oW > 16;
-   // Images that fill less than a quarter of their tiles stay with one thread per output: 1000 x 32 -> 32 at 7 x 7 141 us against 190 here, at 8 x 8
+   // Images that fill less than a quarter of the large tiles stay with one thread per output: 1000 x 32 -> 32 at 7 x 7 141 us against 190 here, at 8 x 8
    // (24 channels, NHWC) 145 against 136. So do those that fill less than 0.6 of them where it is faster by the time in us that either takes, fitted
    // to 200 calls of 1 to 1024 images (to 14 and 12 %; three of them are 6 to 16 % slower here all the same): few channels, whose time here is copies and indexes (32 x 5 -> 61 at 43 x 9 14.0 us against 22.3;
-   // 133 x 15 -> 103 at 65 x 6 212 against 248). Few tiles are not a reason: one image of 16 x 16, 128 -> 16 channels takes 235 us there and 124 here.
+   // 133 x 15 -> 103 at 65 x 6 212 against 248).
    const long long groups = ceil_div(g.Cout, kDcOut), tiles = (long long)ceil_div(g.oH, kDcRows) * ceil_div(g.oW, wide ? 32 : 16), area = kDcRows * (wide ? 32 : 16);
    const long long outputs = (long long)g.oH * g.oW;
-   if (4 * outputs < tiles * area) return -1;
-   if (5 * outputs < 3 * tiles * area) {
-      const double positions = 1e-6 * g.N * outputs, units = 1e-3 * g.N * tiles * groups * (wide ? 2 : 1);
-      const double general = 1.9 + 1.69 * g.C + positions * (25 * groups * g.C + 2.6 * g.Cout);
-      const double here = 2.5 + chunks * (vec ? 3.5 : 4.7) + units * (chunks * (vec ? 5.1 : 8.1) + 4.8);
-      if (1.05 * general <= here) return -1;
+   const double positions = 1e-6 * g.N * outputs, units = (double)g.N * tiles * groups * (wide ? 2 : 1);
+   const double general = 1.9 + 1.69 * g.C + positions * (25 * groups * g.C + 2.6 * g.Cout);
+   const double sparse = 2.5 + chunks * (vec ? 3.5 : 4.7) + 1e-3 * units * (chunks * (vec ? 5.1 : 8.1) + 4.8);
+   const bool filled = 5 * outputs >= 3 * tiles * area;
+   const bool large = 4 * outputs >= tiles * area && (filled || 1.05 * general > sparse);
+   // Shared channels take what is estimated faster that way by a twentieth: the first block of an SM costs its round trips, each further one its work.
+   // (us, by channels; 8 RH = 1, 2, 4; 16 -> 16 channels of 16 x 16, 1 / 128 / 512 / 1024 images: 4.9 / 12.0 / 38 / 74, 5.8 / 8.6 / 27 / 51, 8.2 / 11.7 / 24 / 41, large tiles 19.6 / 20.2 / 34 / 44.)
+   double best = large ? (filled ? (vec ? 1.0 : 1.1) * (2.5 + 4.3 * chunks + (units > kNumSMs ? units / kNumSMs - 1 : 0) * 0.29 * g.C) : sparse) : general;
+   best *= 0.95;
+   int share = 0;
+   for (int i = 0; i < 3; i++) {
+      static const double first[3] = {0.17, 0.235, 0.35}, more[3] = {0.145, 0.21, 0.35}, fixed[3] = {0.5, 0.7, 0.8};
+      const double blocks = (double)g.N * ceil_div(g.oH, 4 << i) * ceil_div(g.oW, 16) * groups;
+      const double time = (vec ? 1.0 : 1.25) * (2.4 + first[i] * g.C + (blocks > kNumSMs ? blocks / kNumSMs - 1 : 0) * (fixed[i] + more[i] * g.C));
+      if (time < best) best = time, share = 1 << i;
    }
+#define SOFIE_SPLIT(P, R) rc = vec ? launch_split<P, R, true>(s, g, X, W, bias, Y) : launch_split<P, R, false>(s, g, X, W, bias, Y)
+   int rc = -1;
+   if (g.pool == 2) {
+      if (share == 1) SOFIE_SPLIT(2, 1);
+      if (share == 2) SOFIE_SPLIT(2, 2);
+      if (share == 4) SOFIE_SPLIT(2, 4);
+   } else {
+      if (share == 1) SOFIE_SPLIT(0, 1);
+      if (share == 2) SOFIE_SPLIT(0, 2);
+      if (share == 4) SOFIE_SPLIT(0, 4);
+   }
+#undef SOFIE_SPLIT
+   if (rc >= 0 || !large) return rc;
 #define SOFIE_DIRECT(P, G) return vec ? launch_direct<P, G, true>(s, g, X, W, bias, Y, chunks) : launch_direct<P, G, false>(s, g, X, W, bias, Y, chunks)
    if (g.pool == 2) {
       if (wide) SOFIE_DIRECT(2, 2);

@@ -167,6 +167,32 @@ def test_conv3x3_f32_direct(N, C, H, W, Cout, x_nhwc, y_nhwc, pool):
 
 
 
+# 3x3 convolutions whose input channels are shared between a block's warps: one, two and four groups of four rows, channels in one piece and in several (70), fewer
+# channels than warps, images smaller than a tile and ragged ones, every layout, pooled odd extents; NaN and infinities pool as the comparisons do
+@pytest.mark.parametrize("N,C,H,W,Cout,pool,x_nhwc,y_nhwc,packed", [(1, 70, 5, 17, 20, 0, 0, 0, 0), (2, 33, 9, 33, 7, 2, 1, 0, 1), (128, 16, 16, 16, 16, 0, 0, 1, 0), (600, 8, 13, 16, 16, 2, 0, 0, 1),
+                                                                    (1, 5, 1, 3, 1, 0, 1, 1, 0), (40, 24, 7, 7, 33, 0, 1, 1, 1), (300, 16, 17, 20, 5, 2, 0, 1, 0)])
+def test_conv2d_f32_shared_channels(N, C, H, W, Cout, pool, x_nhwc, y_nhwc, packed):
+    rng = np.random.default_rng(N + C + H + W + Cout)
+    X, Wt, b = (rng.standard_normal(s).astype(np.float32) for s in ((N, C, H, W), (Cout, C, 3, 3), (Cout,)))
+    X[0, 0, 0, 0], X[-1, -1, -1, -1] = np.nan, np.inf
+    ref = o.conv2d_f32(X, Wt, b, pad=(1, 1), relu=False)
+    if pool:
+        r = ref[:, :, :H // 2 * 2, :W // 2 * 2].reshape(N, Cout, H // 2, 2, W // 2, 2)
+        ref = r[:, :, :, 0, :, 0].copy()
+        for y, x in ((0, 1), (1, 0), (1, 1)):
+            ref = np.where(r[:, :, :, y, :, x] > ref, r[:, :, :, y, :, x], ref)
+    capi.call("sofie_cuda_set_engine", 1)   # images of whole tiles are the tensor cores' otherwise
+    try:
+        y = ops.conv2d_f32(dev(X.transpose(0, 2, 3, 1) if x_nhwc else X), ops.conv2d_pack_f32(dev(Wt)) if packed else dev(Wt), dev(b), shape=X.shape, pad=(1, 1), pool=pool,
+                           x_layout=x_nhwc, y_layout=y_nhwc, kernel=(3, 3), w_packed=bool(packed)).cpu().numpy()
+    finally:
+        capi.call("sofie_cuda_set_engine", 0)
+    y = y.reshape((N, *ref.shape[2:], Cout)).transpose(0, 3, 1, 2) if y_nhwc else y.reshape(ref.shape)
+    finite = np.isfinite(ref)
+    assert (np.abs(y[finite] - ref[finite]) <= FP32_TOL * np.abs(ref[finite]).max(initial=0)).all()
+    assert np.array_equal(y[~finite], ref[~finite], equal_nan=True)
+
+
 @pytest.mark.parametrize("case", CONV_CASES)
 def test_conv2d_f32_nchw(case):
     N, C, H, W, Cout, k, pad, stride, dil, group = case
