@@ -192,6 +192,196 @@ int launch_direct(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, 
    return SOFIE_CUDA_OK;
 }
 
+// ---- few products an output: one launch, sums in 64 bits ----------------------------------------------------------
+// The product form below is four launches and writes every tap's product to memory and reads it back; where an output has few products those are its time, and the
+// direct form above waits for one channel's filters and inputs after the other's. Here a block owns a band of output rows of one image and OC output channels: the band's
+// inputs and the filters are converted to double once, on their way into shared memory, and a thread sums four channels of PX outputs in double, so that the result is the exact
+// sum rounded once (error against float64 2.5e-8; 3.5e-8 to 1.3e-7 the product form, 4.3e-8 to 5.5e-8 the direct one). A warp's outputs share their phase (row and column
+// modulo the strides) and so their taps; OC / 4 neighbouring lanes share an output's inputs.
+// What bounds it: round trips and instructions at few warps an SM (19 % of the issue slots at 64 images), from some hundred images on the reads out of shared memory
+// (2 clk a 16-byte broadcast, 2 an input: 34 of the 64 DFMA/clk at PX = 4). 32 -> 16 channels, 2 x 2 / 2 on 12 x 12, 1 / 64 / 1024 images: 13.6 -> 5.3, 16.3 -> 10.6, 103 -> 85 us against
+// the product form; 16 -> 3, 3 x 3 / 2 on 24 x 24: 12.9 -> 6.4, 21.5 -> 13.9, 184 -> 117. Its channels in registers two or four at a time: the same or slower (96, 127 at 1024).
+constexpr int kSumThreads = 256;
+constexpr int kSumBytes = 96 * 1024; // of shared memory: two blocks an SM
+struct SumGeom {
+   sofie_conv_transpose2d_desc d;
+   int oH, oW, bands, steps, lines; // bands of an image, steps (times the stride: output rows) of a band, input rows it may read
+};
+
+__host__ __device__ inline int floor_div(int a, int b) { return a >= 0 ? a / b : -((b - 1 - a) / b); }
+
+template <int OC, int PX>
+__global__ void __launch_bounds__(kSumThreads, 2)
+conv_transpose_sum_kernel(SumGeom g, FastDiv bands, FastDiv columns, FastDiv taps, FastDiv phase_units, FastDiv phase_columns, int line, const float *__restrict__ X, const float *__restrict__ Wt,
+                          const float *__restrict__ bias, float *__restrict__ Y)
+{
+   extern __shared__ __align__(16) double staged[];
+   const sofie_conv_transpose2d_desc &d = g.d;
+   griddep_launch_dependents();
+   griddep_wait();
+   const int oc0 = blockIdx.y * OC, outs = min(OC, d.Cout - oc0);
+   // [channel][tap][OC], [channel][row][column]; of every filter row (column) the phase that it is a tap of and how far below the output's step its input lies
+   double *filters = staged, *inputs = staged + d.C * (int)taps.d * OC;
+   int2 *tap_rows = reinterpret_cast<int2 *>(inputs + d.C * line), *tap_columns = tap_rows + d.kH;
+   for (int i = threadIdx.x; i < d.kH + d.kW; i += kSumThreads) {
+      const bool column = i >= d.kH;
+      const int stride = column ? d.stride_w : d.stride_h, at = column ? (i - d.kH) * d.dil_w - d.pad_w : i * d.dil_h - d.pad_h, step = floor_div(at, stride);
+      tap_rows[i] = make_int2(at - step * stride, -step);
+   }
+   uint32_t band;
+   const uint32_t n = bands.divmod(blockIdx.x, band);
+   const int oh0 = (int)band * g.steps * d.stride_h, rows = min(g.steps * d.stride_h, g.oH - oh0);
+   // input rows that an output row of the band has a tap on
+   const int first = max(0, floor_div(oh0 + d.pad_h - (d.kH - 1) * d.dil_h, d.stride_h)), last = min(d.H - 1, (oh0 + rows - 1 + d.pad_h) / d.stride_h);
+   const int lines = max(0, last - first + 1);
+   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+   // half of the warps fetch the filters, half the inputs: a warp walks the consecutive values of every fourth input channel, eight loads under way
+   auto stage = [&](int span, auto source, auto store) {
+      int c = warp & 3, base = 0;
+      auto next = [&] {
+         base += 32;
+         if (base >= span) base = 0, c += 4;
+      };
+      while (c < d.C) {
+         const int c0 = c, base0 = base;
+         float v[8];
+#pragma unroll
+         for (int k = 0; k < 8; k++, next()) v[k] = c < d.C && base + lane < span ? __ldg(source(c) + base + lane) : 0.f;
+         c = c0, base = base0;
+#pragma unroll
+         for (int k = 0; k < 8; k++, next())
+            if (c < d.C && base + lane < span) store(c, base + lane, (double)v[k]);
+      }
+   };
+   if (warp < 4) {
+      stage(outs * (int)taps.d, [&](int c) { return Wt + ((size_t)c * d.Cout + oc0) * taps.d; }, // the block's filters of an input channel are consecutive
+            [&](int c, int e, double v) {
+               uint32_t tap;
+               const uint32_t j = taps.divmod((uint32_t)e, tap);
+               filters[(c * taps.d + tap) * OC + j] = v;
+            });
+      if (outs < OC)
+         for (int i = threadIdx.x; i < d.C * (int)taps.d; i += kSumThreads / 2)
+            for (int j = outs; j < OC; j++) filters[i * OC + j] = 0.0;
+   } else if (lines > 0) {
+      // a channel's rows are consecutive in X and here
+      const float *x = X + ((size_t)n * d.C * d.H + first) * d.W;
+      stage(lines * d.W, [&](int c) { return x + (size_t)c * d.H * d.W; }, [&](int c, int e, double v) { inputs[c * line + e] = v; });
+   }
+   __syncthreads();
+   constexpr int LG = OC / 4, PXW = 32 / LG * PX; // lanes that share an output's channels, positions of a warp
+   const int oc = lane % LG * 4, units = (int)phase_units.d;
+   for (int u = warp; u < units * d.stride_h * d.stride_w; u += kSumThreads / 32) {
+      uint32_t rw, in_phase;
+      const int rh = (int)phase_columns.divmod(phase_units.divmod((uint32_t)u, in_phase), rw), i0 = (int)in_phase * PXW + lane / LG;
+      int step_h[PX], step_w[PX]; // the output is in row stride * step + phase
+      double acc[PX][4];
+#pragma unroll
+      for (int q = 0; q < PX; q++) {
+         uint32_t column;
+         step_h[q] = (int)band * g.steps + (int)columns.divmod((uint32_t)(i0 + q * (32 / LG)), column);
+         step_w[q] = (int)column;
+#pragma unroll
+         for (int j = 0; j < 4; j++) acc[q][j] = 0.0;
+      }
+      for (int r = 0; r < d.kH; r++) {
+         const int2 row = tap_rows[r];
+         if (row.x != rh) continue;
+         for (int s = 0; s < d.kW; s++) {
+            const int2 across = tap_columns[s];
+            if (across.x != (int)rw) continue;
+            const double *w = filters + (r * d.kW + s) * OC + oc;
+            const double *x[PX];
+            bool in[PX];
+            bool any = false;
+#pragma unroll
+            for (int q = 0; q < PX; q++) {
+               const int ih = step_h[q] + row.y, iw = step_w[q] + across.y;
+               in[q] = ih >= first && ih <= last && iw >= 0 && iw < d.W;
+               x[q] = inputs + (in[q] ? (ih - first) * d.W + iw : 0);
+               any = any || in[q];
+            }
+            if (!any) continue;
+#pragma unroll 4
+            for (int c = 0; c < d.C; c++) {
+               const double2 f0 = *reinterpret_cast<const double2 *>(w), f1 = *reinterpret_cast<const double2 *>(w + 2);
+               w += taps.d * OC;
+#pragma unroll
+               for (int q = 0; q < PX; q++) {
+                  const double v = *x[q];
+                  x[q] += line;
+                  if (in[q]) { // a tap outside is no product: an infinite weight does not count there
+                     acc[q][0] = fma(v, f0.x, acc[q][0]);
+                     acc[q][1] = fma(v, f0.y, acc[q][1]);
+                     acc[q][2] = fma(v, f1.x, acc[q][2]);
+                     acc[q][3] = fma(v, f1.y, acc[q][3]);
+                  }
+               }
+            }
+         }
+      }
+#pragma unroll
+      for (int q = 0; q < PX; q++) {
+         const int oh = d.stride_h * step_h[q] + rh, ow = d.stride_w * step_w[q] + (int)rw;
+         if (oh >= oh0 + rows || ow >= g.oW) continue;
+#pragma unroll
+         for (int j = 0; j < 4; j++) {
+            if (oc + j < outs) {
+               float v = (float)(acc[q][j] + (bias ? (double)__ldg(bias + oc0 + oc + j) : 0.0));
+               if (d.relu) v = relu_ref(v);
+               Y[(((size_t)n * d.Cout + oc0 + oc + j) * g.oH + oh) * g.oW + ow] = v;
+            }
+         }
+      }
+   }
+}
+
+// -1 where the filters and one row of outputs' inputs do not fit in shared memory
+template <int OC, int PX>
+int launch_sum(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, int oW, int per, const float *X, const float *W, const float *bias, float *Y)
+{
+   const int groups = ceil_div(d.Cout, OC), steps = ceil_div(oH, d.stride_h), columns = ceil_div(oW, d.stride_w), halo = ceil_div((d.kH - 1) * d.dil_h, d.stride_h) + 1;
+   const size_t filters = (size_t)d.C * d.kH * d.kW * OC * sizeof(double), row = (size_t)d.C * d.W * sizeof(double);
+   if (groups > 65535 || filters + row * (1 + halo) > kSumBytes || d.kH + d.kW > 1024 || (long long)d.kH * d.dil_h > 1 << 20 || (long long)d.pad_h + oH > 1 << 28 || (long long)d.pad_w + oW > 1 << 28) return -1;
+   const int fit = (int)((kSumBytes - filters) / row) - halo;
+   if (per > fit) per = fit;
+   SumGeom g = {d, oH, oW, ceil_div(steps, per), per, per + halo};
+   if ((long long)d.N * g.bands >= 1ll << 31) return -1;
+   const size_t smem = filters + row * g.lines + (d.kH + d.kW) * sizeof(int2);
+   auto kern = conv_transpose_sum_kernel<OC, PX>;
+   SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), (int)smem));
+   SOFIE_CUDA_TRY(launch_dependent(kern, dim3((unsigned)(d.N * (long long)g.bands), groups), dim3(kSumThreads), smem, s, g, FastDiv(g.bands), FastDiv(columns), FastDiv(d.kH * d.kW), FastDiv(ceil_div(per * columns, 128 / OC * PX)), FastDiv(d.stride_w),
+                                   g.lines * d.W, X, W, bias, Y));
+   SOFIE_LAUNCH_CHECK("conv_transpose_sum_kernel");
+   set_last_engine(SOFIE_ENGINE_SIMT);
+   return SOFIE_CUDA_OK;
+}
+
+// -1 where an output has more products, or they do not fit
+int launch_few_products(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, int oW, const float *X, const float *W, const float *bias, float *Y)
+{
+   // Up to 48 products an output, counted without borders. 64 -> 32 channels, 2 x 2 / 2 (64 products) on 256 images of 8 x 8: 44 us here, 30 in the product form; 32 -> 16, 4 x 4 / 2
+   // (128) on 64 of 16 x 16: 29 and 31; 16 -> 16, 3 x 3 / 1 (144) on 64 of 64 x 64: 101 here, 84 in the direct form.
+   if ((long long)d.C * d.kH * d.kW > 48ll * d.stride_h * d.stride_w || forced_engine() == SOFIE_ENGINE_TCGEN05) return -1;
+   // Bands for two blocks an SM, as far as the rows go: what a block costs beside its sums is its start (64 images, 32 -> 16 channels: 4 bands an image 11.5 us, 6 15.1, 12 19.3, 2 16.6).
+   // Of the outputs a thread can take the most that leave every warp some.
+   const int OC = d.Cout <= 4 ? 4 : d.Cout <= 8 ? 8 : 16, steps = ceil_div(oH, d.stride_h), columns = ceil_div(oW, d.stride_w);
+   const long long wanted = 2 * kNumSMs / ((long long)d.N * ceil_div(d.Cout, OC));
+   const int per = ceil_div(steps, (int)(wanted < 1 ? 1 : (wanted > steps ? steps : wanted)));
+   auto units = [&](int q) { return (long long)d.stride_h * d.stride_w * ceil_div((long long)per * columns, 128ll / OC * q); };
+   const int px = units(4) >= kSumThreads / 32 ? 4 : units(2) >= kSumThreads / 32 ? 2 : 1;
+#define SOFIE_SUM(C, P) return launch_sum<C, P>(s, d, oH, oW, per, X, W, bias, Y)
+#define SOFIE_SUM_OC(P) \
+   if (OC == 4) SOFIE_SUM(4, P); \
+   if (OC == 8) SOFIE_SUM(8, P); \
+   SOFIE_SUM(16, P)
+   if (px == 1) { SOFIE_SUM_OC(1); }
+   if (px == 2) { SOFIE_SUM_OC(2); }
+   SOFIE_SUM_OC(4);
+#undef SOFIE_SUM_OC
+#undef SOFIE_SUM
+}
+
 // ---- the product form: one GEMM over all images on the tensor cores, then a gather -------------------------------
 // The reference computes, per image, filter^T [Cout*kH*kW, C] x image [C, H*W] with sgemm_ and scatters the columns
 // into the output (col2im). Here the images are brought to channel-last once, so ALL of them are one K-major operand:
@@ -300,6 +490,8 @@ extern "C" int sofie_cuda_conv_transpose2d_f32_gemm(void *stream, const sofie_co
    SOFIE_REQUIRE(scratch_bytes >= need, "scratch of %zu bytes, %zu needed", scratch_bytes, need);
    SOFIE_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 255) == 0, "scratch must be 256-byte aligned");
    cudaStream_t s = as_stream(stream);
+   const int few = launch_few_products(s, *d, (int)oH, (int)oW, X, W, bias, Y);
+   if (few >= 0) return few;
    const size_t pixels = (size_t)d->N * d->H * d->W;
    const int taps = d->kH * d->kW;
    float *Xt = static_cast<float *>(scratch);
@@ -330,5 +522,7 @@ extern "C" int sofie_cuda_conv_transpose2d_f32(void *stream, const sofie_conv_tr
    if (rc) return rc;
    if (d->N == 0) return SOFIE_CUDA_OK;
    SOFIE_REQUIRE(X && W && Y, "NULL tensor");
+   const int few = launch_few_products(as_stream(stream), *d, (int)oH, (int)oW, X, W, bias, Y);
+   if (few >= 0) return few;
    return launch_direct(as_stream(stream), *d, (int)oH, (int)oW, X, W, bias, Y);
 }

@@ -267,6 +267,29 @@ def test_conv_transpose2d_f32_direct(N, C, H, W, Cout, k, stride, pad, dil, out_
 
 
 
+# ConvTranspose of few products an output: many bands an image and one, steps that do not divide, four / eight / sixteen channels and two groups of them, one to four outputs a
+# thread, strides beyond the filter (outputs without a tap), dilation, inputs cut by the pads. The sums are exact to double's rounding: the result is theirs, rounded once.
+@pytest.mark.parametrize("N,C,H,W,Cout,k,stride,pad,dil,out_pad", [(1, 32, 12, 12, 16, (2, 2), (2, 2), (0, 0), (1, 1), (0, 0)), (64, 16, 24, 24, 3, (3, 3), (2, 2), (1, 1), (1, 1), (1, 1)),
+                                                                   (300, 5, 7, 9, 8, (3, 2), (2, 3), (1, 0), (2, 1), (1, 2)), (37, 20, 5, 33, 19, (1, 5), (1, 4), (0, 2), (1, 1), (0, 3)),
+                                                                   (3, 40, 6, 5, 4, (1, 1), (3, 2), (0, 0), (1, 1), (2, 1)), (2, 1, 40, 3, 17, (5, 5), (1, 1), (4, 2), (1, 1), (0, 0))])
+def test_conv_transpose2d_f32_few_products(N, C, H, W, Cout, k, stride, pad, dil, out_pad):
+    rng = np.random.default_rng(N + C + H + W + Cout)
+    X, Wt, b = (rng.standard_normal(s).astype(np.float32) for s in ((N, C, H, W), (C, Cout, *k), (Cout,)))
+    Wt[0, 0, 0, 0] = np.inf   # counts only where the tap lies on the input
+    args = dict(stride=stride, padding=pad, dilation=dil, output_padding=out_pad)
+    # (the infinity apart: a library may multiply it with padding)
+    finite = torch.from_numpy(np.where(np.isinf(Wt), 0, Wt)).double()
+    ref = torch.nn.functional.conv_transpose2d(torch.from_numpy(X).double(), finite, torch.from_numpy(b).double(), **args).numpy()
+    size = torch.nn.functional.conv_transpose2d(torch.from_numpy(abs(X)).double(), finite.abs(), torch.from_numpy(abs(b)).double(), **args).numpy()
+    one = np.zeros_like(Wt)
+    one[0, 0, 0, 0] = 1
+    hit = o.conv_transpose2d_f32(X, one, None, pad=pad, stride=stride, dil=dil, out_pad=out_pad)
+    for product_form in ((False, True) if C >= 16 and C % 4 == 0 else (False,)):
+        y = ops.conv_transpose2d_f32(dev(X), dev(Wt), dev(b), pad=pad, stride=stride, dil=dil, out_pad=out_pad, product_form=product_form).cpu().numpy()
+        assert np.array_equal(np.isinf(y), hit != 0) and np.array_equal(np.sign(y[hit != 0]), np.sign(hit[hit != 0]))
+        assert (np.abs(y - ref)[hit == 0] <= (2.0 ** -24 * 1.01 * np.abs(ref) + 1e-13 * size)[hit == 0]).all()
+
+
 @pytest.mark.parametrize("case", [
     # N, C, H, W, Cout, k, pad, stride, dil, out_pad, bias, relu
     (4, 32, 16, 16, 16, (4, 4), (1, 1), (2, 2), (1, 1), (0, 0), True, True),       # the usual 2x upsampling layer of a decoder
