@@ -259,6 +259,101 @@ int launch_mlp(cudaStream_t stream, MlpParams &p, int floats, int maxact, const 
    return SOFIE_CUDA_OK;
 }
 
+// ---- few rows: the weights in registers ---------------------------------------------------------------------------
+// With a row or two a block each weight is used once or twice: staging them in shared memory is half of such a call. Here S lanes share an output's sum and a thread
+// holds its pieces of the weights of all (up to three) layers in registers, asked for at once and beside the inputs, which come the longest way (across PCIe where a Session
+// leaves them in host memory); what remains of a layer is its sum, two to five shuffles and a barrier. What bounds it: the launch and two round trips, then the
+// weights' way out of L2. 64 -> 128 -> 128 -> 10, launch and wait, inputs and results in host memory: 1 row 17.4 -> 14.5 us, 128 20.4 -> 18.0, 256 21.6 -> 19.4; a Session on 1 / 64 / 128 /
+// 256 rows 22.1 -> 18.1, 23.8 -> 22.2, 30.7 -> 23.7, 32.5 -> 27.8. From three rows a block on it is no faster (400 rows 35.2 both, 592 35.2 against 37.4: its reads of the rows).
+// A cluster of 2, 4 or 8 blocks that shares the outputs and writes them to each other's shared memory saves one to two us of a row's and loses from 64 rows on.
+constexpr int kRegThreads = 512, kRegPieces = 8, kRegRows = 2;
+struct RegParams {
+   int M, rows, ld;
+   int K[3], N[3], S[3], pieces[3], relu[3];
+   const float *W[3], *B[3];
+};
+
+template <int NL>
+__global__ void __launch_bounds__(kRegThreads, 1) mlp_registers_f32_kernel(RegParams p, const float *__restrict__ X, float *__restrict__ Y)
+{
+   extern __shared__ __align__(16) float sm[]; // the inputs of every layer, [row][ld], zeros behind them
+   const int tid = threadIdx.x, m0 = blockIdx.x * p.rows, rows = min(p.rows, p.M - m0), L4 = p.ld >> 2;
+   for (int i = tid; i < rows * L4; i += kRegThreads) {
+      const int r = i / L4, k = 4 * (i - r * L4);
+      const bool in = k < p.K[0];
+      cp_async16(sm + r * p.ld + k, X + (size_t)(m0 + r) * p.K[0] + (in ? k : 0), in);
+   }
+   float4 w[NL][kRegPieces];
+   float b[NL];
+#pragma unroll
+   for (int l = 0; l < NL; l++) {
+      const int S = p.S[l], n = tid / S;
+      const bool ok = n < p.N[l];
+      const float4 *row = reinterpret_cast<const float4 *>(p.W[l] + (size_t)(ok ? n : 0) * p.K[l]);
+      b[l] = ok && p.B[l] ? __ldg(p.B[l] + n) : 0.f;
+#pragma unroll
+      for (int i = 0; i < kRegPieces; i++) {
+         const int k = (tid & (S - 1)) + S * i;
+         w[l][i] = ok && 4 * k < p.K[l] ? __ldg(row + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+   }
+   for (int i = tid; i < (NL - 1) * p.rows * p.ld; i += kRegThreads) sm[p.rows * p.ld + i] = 0.f;
+   cp_async_wait_all();
+   __syncthreads();
+#pragma unroll
+   for (int l = 0; l < NL; l++) {
+      const int S = p.S[l], s = tid & (S - 1), n = tid / S, pieces = p.pieces[l], N = p.N[l];
+      const float *in = sm + l * p.rows * p.ld + 4 * s;
+      if ((tid & ~31) / S < N) // some output of this warp
+         for (int r = 0; r < rows; r++) {
+            float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < kRegPieces; i++)
+               if (i < pieces) {
+                  const float4 x = *reinterpret_cast<const float4 *>(in + r * p.ld + 4 * S * i);
+                  c.x = fmaf(x.x, w[l][i].x, c.x);
+                  c.y = fmaf(x.y, w[l][i].y, c.y);
+                  c.z = fmaf(x.z, w[l][i].z, c.z);
+                  c.w = fmaf(x.w, w[l][i].w, c.w);
+               }
+            float v = (c.x + c.y) + (c.z + c.w);
+            for (int d = 1; d < S; d *= 2) v += __shfl_xor_sync(0xffffffffu, v, d);
+            v += b[l];
+            if (p.relu[l]) v = relu_ref(v);
+            if (s == 0 && n < N) {
+               if (l + 1 < NL) sm[((l + 1) * p.rows + r) * p.ld + n] = v;
+               else Y[(size_t)(m0 + r) * N + n] = v;
+            }
+         }
+      if (l + 1 < NL) __syncthreads();
+   }
+}
+
+// -1 for more rows or layers, and for weights that are not read in 16-byte pieces or of which a thread would hold more than kRegPieces a layer
+int launch_mlp_registers(cudaStream_t stream, const MlpParams &m, const float *X, float *Y)
+{
+   const sofie_mlp_desc &d = m.d;
+   if (d.layers > 3 || d.M > kRegRows * kNumSMs || !m.x_vec) return -1;
+   RegParams p = {};
+   p.M = d.M;
+   p.rows = ceil_div(d.M, kNumSMs);
+   for (int l = 0; l < d.layers; l++) {
+      int S = 32;
+      while (S > 1 && S * d.dims[l + 1] > kRegThreads) S >>= 1;
+      p.K[l] = d.dims[l], p.N[l] = d.dims[l + 1], p.S[l] = S, p.pieces[l] = ceil_div(ceil_div(d.dims[l], 4), S), p.relu[l] = d.relu[l];
+      p.W[l] = m.W[l], p.B[l] = m.B[l];
+      if (!m.w_vec[l] || S * p.N[l] > kRegThreads || p.pieces[l] > kRegPieces) return -1;
+      if (p.ld < 4 * S * p.pieces[l]) p.ld = 4 * S * p.pieces[l];
+   }
+   const size_t smem = (size_t)d.layers * p.rows * p.ld * sizeof(float); // at most 3 x 2 x 256 floats
+   const int blocks = ceil_div(d.M, p.rows);
+   if (d.layers == 1) mlp_registers_f32_kernel<1><<<blocks, kRegThreads, smem, stream>>>(p, X, Y);
+   else if (d.layers == 2) mlp_registers_f32_kernel<2><<<blocks, kRegThreads, smem, stream>>>(p, X, Y);
+   else mlp_registers_f32_kernel<3><<<blocks, kRegThreads, smem, stream>>>(p, X, Y);
+   SOFIE_LAUNCH_CHECK("mlp_registers_f32_kernel");
+   return SOFIE_CUDA_OK;
+}
+
 } // namespace
 } // namespace sofie
 
@@ -314,9 +409,11 @@ extern "C" int sofie_cuda_mlp_f32(void *stream, const sofie_mlp_desc *d, const f
       if (rc >= 0) return rc;
       return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "these layer widths are not served by the tensor-core chain");
    }
+   set_last_engine(SOFIE_ENGINE_SIMT);
+   const int few = launch_mlp_registers(s, p, X, Y);
+   if (few >= 0) return few;
    int rows = 32;
    while (rows > 8 && (d->M + rows - 1) / rows < kNumSMs) rows >>= 1;
-   set_last_engine(SOFIE_ENGINE_SIMT);
    if (rows == 32) return launch_mlp<32>(s, p, floats, maxact, X, Y);
    if (rows == 16) return launch_mlp<16>(s, p, floats, maxact, X, Y);
    return launch_mlp<8>(s, p, floats, maxact, X, Y);

@@ -752,8 +752,8 @@ static std::string ByteCount(const std::vector<size_t> &shape, ETensorType t)
 
 // results up to this size are written by the kernels straight into mapped host memory
 static constexpr size_t kHostOutputMaxBytes = 64 * 1024;
-// inputs up to this size can be read from there (64 rows of 64 floats: 0.3 us of PCIe beside the 1.2 of its latency)
-static constexpr size_t kHostInputMaxBytes = 16 * 1024;
+// inputs up to this size can be read from there (256 rows of 64 floats: 5 us beside the same rows out of device memory, where a kernel of its own that fetches them first takes 7)
+static constexpr size_t kHostInputMaxBytes = 64 * 1024;
 
 void RModel::GenerateSessionMembers()
 {

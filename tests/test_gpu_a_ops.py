@@ -102,6 +102,25 @@ def test_mlp_f32_fused_chain(M, dims, relu, nk, bias, engine):
     assert y.shape == ref.shape and rel_err(y, ref) <= FP32_TOL
 
 
+# rows that take the kernel with its weights in registers: one and two a block, the first beyond; pieces that end inside a lane's share (K = 20, 36), one lane to thirty-two an
+# output, an infinite input (zeros behind a row's inputs are no products of it), one to three layers
+@pytest.mark.parametrize("M,dims", [(1, (64, 128, 128, 10)), (148, (64, 128, 128, 10)), (149, (20, 36, 7)), (296, (256, 16, 64, 3)), (297, (64, 128, 128, 10)), (3, (256, 1)), (5, (16, 256, 4)),
+                                    (2, (4, 100, 128, 33))])
+def test_mlp_f32_few_rows(M, dims):
+    rng = np.random.default_rng(M + len(dims))
+    x = rng.standard_normal((M, dims[0])).astype(np.float32)
+    Ws = [(np.abs(rng.standard_normal((n, k))) / np.sqrt(k)).astype(np.float32) for k, n in zip(dims[:-1], dims[1:])]
+    Bs = [rng.standard_normal(n).astype(np.float32) for n in dims[1:]]
+    relu, nk = [1] * (len(dims) - 2) + [0], [1] * (len(dims) - 1)
+    if M > 1:
+        x[M - 1, dims[0] - 1] = np.inf
+    ref = _mlp_reference(x, Ws, Bs, relu, nk)
+    y = ops.mlp_f32(dev(x), [dev(W) for W in Ws], [dev(b) for b in Bs], relu, nk).cpu().numpy()
+    finite = np.isfinite(ref)
+    assert np.array_equal(y[~finite], ref[~finite], equal_nan=True) and (M == 1 or not finite.all())
+    assert np.abs(y[finite] - ref[finite]).max() <= FP32_TOL * np.abs(ref[finite]).max()
+
+
 def test_mlp_f32_limits_and_empty_batch():
     W = torch.zeros((8, 300), device="cuda")
     with pytest.raises(capi.SofieCudaError) as e:
