@@ -67,6 +67,13 @@ constexpr int kNumSMs = 148; // B200
 // a kernel that was launched the ordinary way. SOFIE_CUDA_PDL=0 turns the attribute off.
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A read of what an earlier kernel wrote, behind griddep_wait(): a load the compiler takes for one of constant data (__ldg, or through a restrict pointer) may move before it.
+__device__ __forceinline__ float load_dependent(const float *p)
+{
+   float v;
+   asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+   return v;
+}
 bool pdl_enabled();
 
 template <typename... KArgs, typename... Args>

@@ -246,7 +246,7 @@ conv_transpose_sum_kernel(SumGeom g, FastDiv bands, FastDiv columns, FastDiv tap
          const int c0 = c, base0 = base;
          float v[8];
 #pragma unroll
-         for (int k = 0; k < 8; k++, next()) v[k] = c < d.C && base + lane < span ? __ldg(source(c) + base + lane) : 0.f;
+         for (int k = 0; k < 8; k++, next()) v[k] = c < d.C && base + lane < span ? load_dependent(source(c) + base + lane) : 0.f;
          c = c0, base = base0;
 #pragma unroll
          for (int k = 0; k < 8; k++, next())
