@@ -74,6 +74,132 @@ gemm_f32_simt_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, const f
    }
 }
 
+// ---- outputs of few terms (K <= 32) --------------------------------------------------------------
+// What the kernel above spends on a large output of few terms is instructions: it walks K in steps of 16 between barriers for 64 x 64 outputs, and each staged value and
+// each stored one has its own indexes. Here a block keeps its BN columns of B, all K of them, and walks tiles of BM rows, the next tile's A on its way under this one; a warp's
+// BM / 8 rows read A as broadcasts of four rows and feed packed FMAs (two rows each, in the order of k and rounded as the scalar ones: the same sums), and a lane's columns are
+// 32 apart, so that a warp stores whole lines of any alignment. Bound by issue slots still (16 instructions for 32 outputs of 9 terms; 36 without the walk). Against the kernel
+// above: 9602 x 3820 x 9 83 -> 38 us (its bytes take 23), 16384 x 4093 x 8 with a full C 169 -> 106 (83), 13028 x 2481 x 14 73 -> 42, 12399 x 459 x 23 28 -> 20, 728 x 2032 x 10 7.7 -> 6.1.
+// Tiles of 128 rows: 41, 119, 45, 19, 6.8.
+constexpr int kFewThreads = 256, kFewK = 32, kFewRows = 64;
+template <int BN, int BIAS>
+__global__ void __launch_bounds__(kFewThreads, 3)
+gemm_f32_few_terms_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, const float *__restrict__ B, const float *C, float *Y, uint32_t tiles_m, uint32_t sharers, FastDiv columns,
+                          FastDiv terms)
+{
+   constexpr int BM = kFewRows, ROWS = BM / 8, COLS = BN / 32, PA = BM + 4, PB = BN + 1, BATCH = 4; // rows of C under way
+   extern __shared__ __align__(16) float few[];
+   float *Bs = few + 2 * d.K * PA; // [k][column]; few: two tiles [k][row]
+   const int tid = threadIdx.x, lane = tid & 31, row0 = (tid >> 5) * ROWS, K = d.K;
+   uint32_t tn;
+   const uint32_t sharer = columns.divmod(blockIdx.x, tn);
+   const int n0 = (int)tn * BN;
+   // EXTENT rows or columns from `first` on, of `count`, into [k][extent]; threads along what is contiguous in memory
+   auto stage = [&](float *dst, int pitch, int extent, const float *src, bool k_contiguous, int first, int count) {
+      for (int i = tid; i < extent * K; i += kFewThreads) {
+         uint32_t k, e;
+         if (k_contiguous) e = terms.divmod((uint32_t)i, k);
+         else k = (uint32_t)i / (uint32_t)extent, e = (uint32_t)i % (uint32_t)extent; // a power of two
+         const bool in = first + (int)e < count;
+         const float *from = src + (in ? (k_contiguous ? (size_t)first * K + i : (size_t)k * count + first + e) : 0);
+         asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst + k * pitch + e)), "l"(from), "r"(in ? 4 : 0) : "memory");
+      }
+   };
+   stage(Bs, PB, BN, B, d.transB, n0, d.N);
+   stage(few, PA, BM, A, !d.transA, (int)sharer * BM, d.M);
+   asm volatile("cp.async.commit_group;" ::: "memory");
+   bool in[COLS];
+   float bias[COLS];
+#pragma unroll
+   for (int j = 0; j < COLS; j++) {
+      in[j] = n0 + lane + 32 * j < d.N;
+      bias[j] = BIAS == 1 && in[j] ? d.beta * C[n0 + lane + 32 * j] : 0.f;
+   }
+   int buf = 0;
+   for (uint32_t t = sharer; t < tiles_m; t += sharers, buf ^= 1) {
+      const int m0 = (int)t * BM;
+      __syncthreads(); // the tile before this one is no longer read
+      if (t + sharers < tiles_m) stage(few + (buf ^ 1) * K * PA, PA, BM, A, !d.transA, (int)(t + sharers) * BM, d.M);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+      __syncthreads();
+      uint64_t acc[ROWS / 2][COLS]; // two rows each
+#pragma unroll
+      for (int i = 0; i < ROWS / 2; i++)
+#pragma unroll
+         for (int j = 0; j < COLS; j++) acc[i][j] = 0;
+      const float *a_k = few + buf * K * PA + row0, *b_k = Bs + lane;
+#pragma unroll 2
+      for (int k = 0; k < K; k++, a_k += PA, b_k += PB) {
+         uint64_t b[COLS];
+#pragma unroll
+         for (int j = 0; j < COLS; j++) b[j] = pack_f32x2(b_k[32 * j], b_k[32 * j]);
+#pragma unroll
+         for (int i = 0; i < ROWS / 4; i++) {
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(a_k + 4 * i);
+#pragma unroll
+            for (int j = 0; j < COLS; j++) {
+               acc[2 * i][j] = fma_f32x2(a.x, b[j], acc[2 * i][j]);
+               acc[2 * i + 1][j] = fma_f32x2(a.y, b[j], acc[2 * i + 1][j]);
+            }
+         }
+      }
+      const int rows = min(ROWS, d.M - m0 - row0);
+      size_t at = (size_t)(m0 + row0) * d.N + n0 + lane;
+#pragma unroll
+      for (int i = 0; i < ROWS; i += BATCH) {
+         float c[BATCH][COLS]; // read before the first of them is written: Y may be C
+         if (BIAS == 2) {
+#pragma unroll
+            for (int r = 0; r < BATCH; r++)
+#pragma unroll
+               for (int j = 0; j < COLS; j++) c[r][j] = i + r < rows && in[j] ? C[at + (size_t)r * d.N + 32 * j] : 0.f;
+         }
+#pragma unroll
+         for (int r = 0; r < BATCH; r++, at += d.N) {
+            if (i + r >= rows) break;
+#pragma unroll
+            for (int j = 0; j < COLS; j++) {
+               float lo, hi;
+               unpack_f32x2(acc[(i + r) / 2][j], lo, hi);
+               float y = d.alpha * ((i + r) % 2 ? hi : lo);
+               if (BIAS == 1) y += bias[j];
+               if (BIAS == 2) y = fmaf(d.beta, c[r][j], y);
+               if (d.relu) y = relu_ref(y);
+               if (in[j]) Y[at + 32 * j] = y;
+            }
+         }
+      }
+   }
+}
+
+template <int BN>
+int launch_few_terms(cudaStream_t s, const sofie_gemm_f32_desc &d, const float *A, const float *B, const float *C, float *Y)
+{
+   constexpr int BM = kFewRows;
+   const int tiles_n = ceil_div(d.N, BN), tiles_m = ceil_div(d.M, BM), smem = d.K * (2 * (BM + 4) + BN + 1) * (int)sizeof(float);
+   long long sharers = 3ll * kNumSMs / tiles_n; // blocks that share a column of tiles: three an SM are resident
+   sharers = sharers < 1 ? 1 : (sharers > tiles_m ? tiles_m : sharers);
+   auto go = [&](auto kind) -> int {
+      auto kern = gemm_f32_few_terms_kernel<BN, decltype(kind)::value>;
+      SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), smem));
+      kern<<<(unsigned)(sharers * tiles_n), kFewThreads, smem, s>>>(d, A, B, C, Y, (uint32_t)tiles_m, (uint32_t)sharers, FastDiv(tiles_n), FastDiv(d.K));
+      SOFIE_LAUNCH_CHECK("gemm_f32_few_terms_kernel");
+      set_last_engine(SOFIE_ENGINE_SIMT);
+      return SOFIE_CUDA_OK;
+   };
+   return d.bias_kind == 0 ? go(std::integral_constant<int, 0>{}) : d.bias_kind == 1 ? go(std::integral_constant<int, 1>{}) : go(std::integral_constant<int, 2>{});
+}
+
+static int launch_gemm_f32_few_terms(cudaStream_t s, const sofie_gemm_f32_desc &d, const float *A, const float *B, const float *C, float *Y)
+{
+   // the widest tile that still gives every SM one; 64 x 64 against 64 x 32: 287 x 1457 x 8 (115 tiles) 3.5 us both, 78 x 1574 x 16 (50) 4.2 against 3.6
+   const long long tall = ceil_div(d.M, kFewRows);
+   if (tall * ceil_div(d.N, 128) >= kNumSMs) return launch_few_terms<128>(s, d, A, B, C, Y);
+   if (tall * ceil_div(d.N, 64) >= 64) return launch_few_terms<64>(s, d, A, B, C, Y);
+   return launch_few_terms<32>(s, d, A, B, C, Y);
+}
+
 // Products of few FMAs, whatever the layout: what bounds them is latency. The kernel above walks K in steps of 16 with a round trip to memory
 // and two barriers each (2 x 1 x 427 34 us), the tensor-core kernels set themselves up (6 to 8 us). Here T lanes share an output, each with every
 // T-th term of K, all loads of eight terms issued together, and add up their sums in pairs: 2 x 1 x 427 2.7 us, 5 x 2 x 166 21.7 -> 2.3,
@@ -175,6 +301,7 @@ int launch_gemm_f32_tiny(cudaStream_t s, const sofie_gemm_f32_desc &d, const flo
 int launch_gemm_f32_simt(cudaStream_t s, const sofie_gemm_f32_desc &d, const float *A, const float *B, const float *C,
                          float *Y)
 {
+   if (d.K <= kFewK) return launch_gemm_f32_few_terms(s, d, A, B, C, Y);
    dim3 grid(ceil_div(d.N, 64), ceil_div(d.M, 64));
    if (d.transA && d.transB) gemm_f32_simt_kernel<true, true><<<grid, 256, 0, s>>>(d, A, B, C, Y);
    else if (d.transA) gemm_f32_simt_kernel<true, false><<<grid, 256, 0, s>>>(d, A, B, C, Y);

@@ -1054,6 +1054,11 @@ int launch_gemm_f32_umma(cudaStream_t s, const sofie_gemm_f32_desc &d, const flo
    // against 5.4, 327 x 2 x 120 5.6 against 6.7, but 163 x 52 x 104 7.8 against 6.1 and 17 x 1 x 236 8.0 against 6.2.
    const bool few_tiles = (long long)ceil_div(d.M, umma::kBM) * ceil_div(d.N, 64) < 2 * kNumSMs, short_rows = d.N <= 24 && d.K < 224;
    if (!tma || d.K >= 1024 || (few_tiles && !short_rows)) return launch_gemm_f32_any(s, d, tma, A, B, C, Y);
+   // Up to 32 terms an output is written in less time by the CUDA-core kernel for that, and is nearer to float64 (two TF32 parts 0.7 to 2.5e-7, FMA chains 0.4 to 1.0e-7): 12538 x 3278 x 8
+   // 163 -> 39 us, 11548 x 1127 x 12 69 -> 19, 6986 x 2034 x 20 61 -> 27, 9637 x 1461 x 28 with a full C 109 -> 44. Rows of whole 16-byte words of 28 terms and more are faster here:
+   // 2545 x 4044 x 32 24 us against 30, 7881 x 908 x 28 20.2 against 22.2; of 24 terms 6561 x 1268 21.6 against 20.0.
+   if (d.K <= 32 && d.N > 24 && !(d.N % 4 == 0 && d.K >= 28 && d.bias_kind != 2) && forced_engine() != SOFIE_ENGINE_TCGEN05)
+      return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "a large output of few terms has a kernel on the CUDA cores");
    umma::GemmEpilogue ep = {};
    ep.alpha = d.alpha;
    ep.beta = d.beta;

@@ -102,6 +102,32 @@ def test_mlp_f32_fused_chain(M, dims, relu, nk, bias, engine):
     assert y.shape == ref.shape and rel_err(y, ref) <= FP32_TOL
 
 
+# products of up to 32 terms on the CUDA cores: tiles of 128, 64 and 32 columns, one tile and several walked by a block, last rows and columns, K of one and of the largest
+@pytest.mark.parametrize("M,N,K,tA,tB", [(9610, 133, 9, 1, 1), (65, 4000, 32, 0, 0), (700, 1000, 31, 0, 1), (64, 64, 1, 1, 0), (1, 1, 32, 0, 1), (5, 4093, 8, 1, 1), (1000, 33, 17, 0, 0), (20000, 257, 2, 1, 0)])
+@pytest.mark.parametrize("bias_kind,relu", [(0, 0), (1, 1), (2, 0)])
+def test_gemm_f32_few_terms(M, N, K, tA, tB, bias_kind, relu):
+    rng = np.random.default_rng(M + N + K)
+    A, B = rng.standard_normal((K, M) if tA else (M, K)).astype(np.float32), rng.standard_normal((N, K) if tB else (K, N)).astype(np.float32)
+    bias = {0: None, 1: rng.standard_normal(N).astype(np.float32), 2: rng.standard_normal((M, N)).astype(np.float32)}[bias_kind]
+    a, b = (A.T if tA else A).astype(np.float64), (B if not tB else B.T).astype(np.float64)
+    ref, size = 0.75 * (a @ b) + (0 if bias is None else 1.5 * bias), 0.75 * (abs(a) @ abs(b)) + (0 if bias is None else 1.5 * abs(bias))
+    ref = np.maximum(ref, 0) if relu else ref
+    capi.call("sofie_cuda_set_engine", 1)
+    try:
+        Cd = None if bias is None else dev(bias)
+        y = ops.gemm_f32(dev(A), dev(B), Cd, transA=tA, transB=tB, alpha=0.75, beta=1.5, relu=bool(relu))
+        in_place = None
+        if bias_kind == 2:   # Y may be C
+            d = capi.GemmF32Desc(M, N, K, tA, tB, 0.75, 1.5, 2, relu)
+            Ad, Bd, in_place = dev(A), dev(B), Cd.clone()
+            capi.call("sofie_cuda_gemm_f32", None, C.byref(d), C.c_void_p(Ad.data_ptr()), C.c_void_p(Bd.data_ptr()), C.c_void_p(in_place.data_ptr()), C.c_void_p(in_place.data_ptr()))
+            torch.cuda.synchronize()
+    finally:
+        capi.call("sofie_cuda_set_engine", 0)
+    for got in (y, in_place):
+        assert got is None or (np.abs(got.cpu().numpy() - ref) <= (K + 3) * 2.0 ** -24 * size).all()   # a chain of K FMAs, then alpha, beta and the sum
+
+
 # rows that take the kernel with its weights in registers: one and two a block, the first beyond; pieces that end inside a lane's share (K = 20, 36), one lane to thirty-two an
 # output, an infinite input (zeros behind a row's inputs are no products of it), one to three layers
 @pytest.mark.parametrize("M,dims", [(1, (64, 128, 128, 10)), (148, (64, 128, 128, 10)), (149, (20, 36, 7)), (296, (256, 16, 64, 3)), (297, (64, 128, 128, 10)), (3, (256, 1)), (5, (16, 256, 4)),
