@@ -12,6 +12,9 @@ struct ConvGeom {
 };
 
 int launch_gemm_f32_simt(cudaStream_t, const sofie_gemm_f32_desc &, const float *, const float *, const float *, float *);
+// at most 8 rows or columns, any layout (gemm_skinny.cu)
+bool gemm_f32_skinny_ok(const sofie_gemm_f32_desc &);
+int launch_gemm_f32_skinny(cudaStream_t, const sofie_gemm_f32_desc &, const float *, const float *, const float *, float *);
 // few FMAs, any layout
 bool gemm_f32_tiny_ok(const sofie_gemm_f32_desc &);
 int launch_gemm_f32_tiny(cudaStream_t, const sofie_gemm_f32_desc &, const float *, const float *, const float *, float *);

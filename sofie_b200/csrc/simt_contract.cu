@@ -301,7 +301,8 @@ int launch_gemm_f32_tiny(cudaStream_t s, const sofie_gemm_f32_desc &d, const flo
 int launch_gemm_f32_simt(cudaStream_t s, const sofie_gemm_f32_desc &d, const float *A, const float *B, const float *C,
                          float *Y)
 {
-   if (d.K <= kFewK) return launch_gemm_f32_few_terms(s, d, A, B, C, Y);
+   // (up to eight columns a block of one step is as soon done: 16377 x 2 x 10 4.8 us against 5.3)
+   if (d.K <= kFewK && d.M > 8 && d.N > 8) return launch_gemm_f32_few_terms(s, d, A, B, C, Y);
    dim3 grid(ceil_div(d.N, 64), ceil_div(d.M, 64));
    if (d.transA && d.transB) gemm_f32_simt_kernel<true, true><<<grid, 256, 0, s>>>(d, A, B, C, Y);
    else if (d.transA) gemm_f32_simt_kernel<true, false><<<grid, 256, 0, s>>>(d, A, B, C, Y);

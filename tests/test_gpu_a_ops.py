@@ -103,7 +103,7 @@ def test_mlp_f32_fused_chain(M, dims, relu, nk, bias, engine):
 
 
 # products of up to 32 terms on the CUDA cores: tiles of 128, 64 and 32 columns, one tile and several walked by a block, last rows and columns, K of one and of the largest
-@pytest.mark.parametrize("M,N,K,tA,tB", [(9610, 133, 9, 1, 1), (65, 4000, 32, 0, 0), (700, 1000, 31, 0, 1), (64, 64, 1, 1, 0), (1, 1, 32, 0, 1), (5, 4093, 8, 1, 1), (1000, 33, 17, 0, 0), (20000, 257, 2, 1, 0)])
+@pytest.mark.parametrize("M,N,K,tA,tB", [(9610, 133, 9, 1, 1), (65, 4000, 32, 0, 0), (700, 1000, 31, 0, 1), (64, 64, 1, 1, 0), (9, 9, 32, 0, 1), (5, 4093, 8, 1, 1), (1000, 33, 17, 0, 0), (20000, 257, 2, 1, 0)])
 @pytest.mark.parametrize("bias_kind,relu", [(0, 0), (1, 1), (2, 0)])
 def test_gemm_f32_few_terms(M, N, K, tA, tB, bias_kind, relu):
     rng = np.random.default_rng(M + N + K)
@@ -126,6 +126,25 @@ def test_gemm_f32_few_terms(M, N, K, tA, tB, bias_kind, relu):
         capi.call("sofie_cuda_set_engine", 0)
     for got in (y, in_place):
         assert got is None or (np.abs(got.cpu().numpy() - ref) <= (K + 3) * 2.0 ** -24 * size).all()   # a chain of K FMAs, then alpha, beta and the sum
+
+
+# products of at most eight rows or columns: the long operand's rows or its K contiguous, whole 16-byte words and not, one block to a K and clusters of two to eight, last slices
+# shorter than the others, several chunks of the short operand, one to eight of its rows; infinities stay in their rows and columns
+@pytest.mark.parametrize("M,N,K,tA,tB", [(6317, 2, 3797, 1, 0), (2, 3731, 2897, 0, 0), (5, 2378, 516, 0, 1), (4099, 8, 1001, 0, 1), (1, 1001, 4100, 0, 0), (300, 3, 1024, 0, 0), (8, 8, 4097, 1, 1),
+                                         (20000, 1, 64, 0, 1), (7, 9000, 68, 1, 1), (700, 5, 1300, 1, 1), (4, 130, 777, 0, 1)])
+@pytest.mark.parametrize("bias_kind", [0, 1, 2])
+def test_gemm_f32_skinny(M, N, K, tA, tB, bias_kind):
+    rng = np.random.default_rng(M + N + K)
+    A, B = rng.standard_normal((K, M) if tA else (M, K)).astype(np.float32), rng.standard_normal((N, K) if tB else (K, N)).astype(np.float32)
+    bias = {0: None, 1: rng.standard_normal(N).astype(np.float32), 2: rng.standard_normal((M, N)).astype(np.float32)}[bias_kind]
+    a, b = (A.T if tA else A), (B if not tB else B.T)   # views of what the kernel gets
+    a[M - 1, K - 1] = np.inf
+    ref = 0.75 * (a[:M - 1].astype(np.float64) @ b.astype(np.float64)) + (0 if bias is None else 1.5 * (bias if bias_kind == 1 else bias[:M - 1]))
+    size = 0.75 * (abs(a[:M - 1]).astype(np.float64) @ abs(b).astype(np.float64)) + (0 if bias is None else 1.5 * abs(bias if bias_kind == 1 else bias[:M - 1]))
+    y = ops.gemm_f32(dev(A), dev(B), None if bias is None else dev(bias), transA=tA, transB=tB, alpha=0.75, beta=1.5).cpu().numpy()
+    assert np.array_equal(y[M - 1], np.where(b[K - 1] > 0, np.inf, -np.inf))
+    # a lane's chain and the adding up: fewer roundings than one chain of K has, each of at most half a unit of the sum of the sizes
+    assert (np.abs(y[:M - 1] - ref) <= (K / 8 + 24) * 2.0 ** -24 * size).all()
 
 
 # rows that take the kernel with its weights in registers: one and two a block, the first beyond; pieces that end inside a lane's share (K = 20, 36), one lane to thirty-two an
