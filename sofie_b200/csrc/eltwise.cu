@@ -163,6 +163,45 @@ __global__ void pool2x2_f32_nchw_kernel(const float *__restrict__ X, float *__re
       reinterpret_cast<float2 *>(Y + (size_t)row * (W >> 1))[q] = o;
    }
 }
+// The same window on NCHW images of any size (a last odd row or column is passed over): one output at a time, the loads of four outputs under way. 777 images of 3 x 91 x 85
+// 27.0 -> 13.6 us, 1533 of 24 x 16 x 42 39.9 -> 22.8 against the kernel for any window.
+template <bool AVG>
+__global__ void pool2x2_f32_any_kernel(const float *__restrict__ X, float *__restrict__ Y, unsigned total, FastDiv ow, FastDiv oh, int H, int W)
+{
+   constexpr int U = 4;
+   griddep_launch_dependents();
+   griddep_wait(); // X is the previous kernel's output
+   const unsigned nthreads = gridDim.x * blockDim.x;
+   for (unsigned long long i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (unsigned long long)U * nthreads) {
+      float v[U][4];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+         const unsigned long long idx = i + (unsigned long long)u * nthreads;
+         if (idx < total) {
+            uint32_t col, row;
+            const uint32_t plane = oh.divmod(ow.divmod((uint32_t)idx, col), row);
+            const float *w = X + ((size_t)plane * H + 2 * row) * W + 2 * col;
+            v[u][0] = w[0], v[u][1] = w[1], v[u][2] = w[W], v[u][3] = w[W + 1];
+         }
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+         const unsigned long long idx = i + (unsigned long long)u * nthreads;
+         if (idx < total) {
+            float o;
+            if (AVG) {
+               o = (((v[u][0] + v[u][1]) + v[u][2]) + v[u][3]) / 4.f; // the window's elements in the order the reference adds them
+            } else {
+               o = -INFINITY;
+#pragma unroll
+               for (int k = 0; k < 4; k++)
+                  if (v[u][k] > o) o = v[u][k];
+            }
+            Y[idx] = o;
+         }
+      }
+   }
+}
 template <bool AVG>
 __global__ void pool2x2_f32_nhwc_kernel(const float *__restrict__ X, float *__restrict__ Y, unsigned rows /* N*oH */, int oW, int C)
 {
@@ -318,6 +357,49 @@ __global__ void softmax_rows_reg1_kernel(const float *__restrict__ X, float *__r
       }
    }
 }
+// Rows of more than 384 values that are not read in words: four warps share one, so that a thread holds up to 16 of its values instead of 64 and four times as many rows' loads
+// fit on an SM: 9000 rows of 1997 76 -> 43 us.
+template <int V>
+__global__ void __launch_bounds__(kThreads) softmax_rows_shared_kernel(const float *__restrict__ X, float *__restrict__ Y, size_t rows, int len)
+{
+   __shared__ float s_max[kThreads / 32], s_sum[kThreads / 32];
+   const int t = threadIdx.x & 127, warp = threadIdx.x >> 5, first = warp & ~3;
+   for (size_t r0 = blockIdx.x * (size_t)(kThreads / 128); r0 < rows; r0 += (size_t)gridDim.x * (kThreads / 128)) {
+      const size_t r = r0 + (threadIdx.x >> 7);
+      const bool live = r < rows;
+      const float *x = X + (live ? r : 0) * len;
+      float v[V], vmax = -INFINITY;
+#pragma unroll
+      for (int i = 0; i < V; i++) {
+         const int k = t + 128 * i;
+         if (live && k < len) {
+            v[i] = __ldg(x + k);
+            vmax = fmaxf(vmax, v[i]);
+         }
+      }
+      for (int o = 16; o; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+      if ((threadIdx.x & 31) == 0) s_max[warp] = vmax;
+      __syncthreads();
+      vmax = fmaxf(fmaxf(s_max[first], s_max[first + 1]), fmaxf(s_max[first + 2], s_max[first + 3]));
+      float sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < V; i++)
+         if (live && t + 128 * i < len) {
+            v[i] = expf(v[i] - vmax);
+            sum += v[i];
+         }
+      for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if ((threadIdx.x & 31) == 0) s_sum[warp] = sum;
+      __syncthreads();
+      sum = (s_sum[first] + s_sum[first + 1]) + (s_sum[first + 2] + s_sum[first + 3]);
+      float *y = Y + r * len;
+#pragma unroll
+      for (int i = 0; i < V; i++) {
+         const int k = t + 128 * i;
+         if (live && k < len) y[k] = v[i] / sum;
+      }
+   }
+}
 // inner == 1, rows of at most 32 values (class scores): a block takes 256 consecutive rows, copies them into shared memory
 // with coalesced loads (row pitch padded to an odd number of words), one thread works on one row, and the block copies
 // the results out coalesced. No division in the copy loops: row and column advance incrementally.
@@ -431,12 +513,18 @@ __global__ void __launch_bounds__(kThreads) layout_few_channels_kernel(const T *
    const int run = 1 << log_run, p0 = blockIdx.x << log_run, n = min(run, P - p0), pitch = run + 1, flat = n * C, planes = C << log_run;
    const T *src = in + image * (size_t)P * C;
    T *dst = out + image * (size_t)P * C;
+   // a float goes into the tile by an asynchronous copy: no registers hold it, all of a thread's are under way (777 images of 3 x 91 x 85 40 -> 28 us)
+   auto fetch = [](T *at, const T *from) {
+      if constexpr (sizeof(T) == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(at)), "l"(from) : "memory");
+      else *at = *from;
+   };
    if (TO_NHWC) {
 #pragma unroll 8
       for (int i = threadIdx.x; i < planes; i += kThreads) {
          const int c = i >> log_run, p = i & (run - 1);
-         if (p < n) tile[c * pitch + p] = src[(size_t)c * P + p0 + p];
+         if (p < n) fetch(tile + c * pitch + p, src + (size_t)c * P + p0 + p);
       }
+      asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();
       T *y = dst + (size_t)p0 * C;
 #pragma unroll 4
@@ -451,13 +539,70 @@ __global__ void __launch_bounds__(kThreads) layout_few_channels_kernel(const T *
       for (int i = threadIdx.x; i < flat; i += kThreads) {
          uint32_t c;
          const uint32_t p = channels.divmod((uint32_t)i, c);
-         tile[c * pitch + p] = x[i];
+         fetch(tile + c * pitch + p, x + i);
       }
+      asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();
 #pragma unroll 4
       for (int i = threadIdx.x; i < planes; i += kThreads) {
          const int c = i >> log_run, p = i & (run - 1);
          if (p < n) dst[(size_t)c * P + p0 + p] = tile[c * pitch + p];
+      }
+   }
+}
+// The same for floats in images of whole 16-byte words (P a multiple of 4): words on both sides, the tile's rows words apart. What bounds the form above is the number of loads and
+// stores: 512 images of 16 x 64 x 64 58 -> 42 us (its bytes take 41), 1533 of 24 x 16 x 42 56 -> 40 (30).
+template <bool TO_NHWC>
+__global__ void __launch_bounds__(kThreads) layout_few_channels_words_kernel(const float *__restrict__ in, float *__restrict__ out, int P, int C, int log_run, FastDiv channels)
+{
+   __shared__ __align__(16) float tile[kLayoutTile + 4 * 64];
+   griddep_launch_dependents();
+   griddep_wait();
+   const size_t image = blockIdx.y + (size_t)gridDim.y * blockIdx.z;
+   const int run = 1 << log_run, p0 = blockIdx.x << log_run, n = min(run, P - p0), pitch = run + 4, flat = n * C / 4, planes = C << (log_run - 2);
+   const float *src = in + image * (size_t)P * C;
+   float *dst = out + image * (size_t)P * C;
+   // the elements of word i of the pixels' channels
+   auto places = [&](int i, int(&at)[4]) {
+      uint32_t c;
+      uint32_t p = channels.divmod(4u * (uint32_t)i, c);
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+         at[e] = (int)c * pitch + (int)p;
+         if (++c == (uint32_t)C) c = 0, p++;
+      }
+   };
+   if (TO_NHWC) {
+#pragma unroll 4
+      for (int i = threadIdx.x; i < planes; i += kThreads) {
+         const int c = i >> (log_run - 2), p = (i & (run / 4 - 1)) * 4;
+         if (p < n) *reinterpret_cast<float4 *>(tile + c * pitch + p) = *reinterpret_cast<const float4 *>(src + (size_t)c * P + p0 + p);
+      }
+      __syncthreads();
+      float4 *y = reinterpret_cast<float4 *>(dst + (size_t)p0 * C);
+#pragma unroll 4
+      for (int i = threadIdx.x; i < flat; i += kThreads) {
+         int at[4];
+         places(i, at);
+         y[i] = make_float4(tile[at[0]], tile[at[1]], tile[at[2]], tile[at[3]]);
+      }
+   } else {
+      const float4 *x = reinterpret_cast<const float4 *>(src + (size_t)p0 * C);
+#pragma unroll 4
+      for (int i = threadIdx.x; i < flat; i += kThreads) {
+         int at[4];
+         places(i, at);
+         const float4 v = x[i];
+         tile[at[0]] = v.x;
+         tile[at[1]] = v.y;
+         tile[at[2]] = v.z;
+         tile[at[3]] = v.w;
+      }
+      __syncthreads();
+#pragma unroll 4
+      for (int i = threadIdx.x; i < planes; i += kThreads) {
+         const int c = i >> (log_run - 2), p = (i & (run / 4 - 1)) * 4;
+         if (p < n) *reinterpret_cast<float4 *>(dst + (size_t)c * P + p0 + p) = *reinterpret_cast<const float4 *>(tile + c * pitch + p);
       }
    }
 }
@@ -477,6 +622,12 @@ static int launch_layout(cudaStream_t s, const T *in, T *out, int N, int C, int 
       const int whole = N / y * y;
       int rc = launch_layout<T, TO_NHWC>(s, in, out, whole, C, P);
       return rc ? rc : launch_layout<T, TO_NHWC>(s, in + (size_t)whole * C * P, out + (size_t)whole * C * P, N - whole, C, P);
+   }
+   if constexpr (sizeof(T) == 4) {
+      if (P % 4 == 0 && aligned16(in) && aligned16(out)) {
+         SOFIE_CUDA_TRY(launch_dependent(layout_few_channels_words_kernel<TO_NHWC>, grid, dim3(kThreads), 0, s, in, out, P, C, log_run, FastDiv((uint32_t)C)));
+         return SOFIE_CUDA_OK;
+      }
    }
    SOFIE_CUDA_TRY(launch_dependent(layout_few_channels_kernel<T, TO_NHWC>, grid, dim3(kThreads), 0, s, in, out, P, C, log_run, FastDiv((uint32_t)C)));
    return SOFIE_CUDA_OK;
@@ -515,24 +666,22 @@ __device__ __forceinline__ uint8_t quant_u8(float x, float scale, float inv_scal
    return (uint8_t)(__float2int_rn(r) + zp);
 }
 
-// Sixteen elements per thread and step: four 16-byte loads in flight, one 16-byte store.
-__global__ void quantize_u8_vec16_kernel(const float *__restrict__ X, uint8_t *__restrict__ Y, size_t n16, float scale, float inv_scale,
-                                         int zp)
+// Eight elements per thread and step: a lane's two 16-byte loads are a sector, one 8-byte store. 134 MB 30.2 -> 27.2 us (sixteen a step, whose four loads are 64 bytes apart
+// from lane to lane, before).
+__global__ void quantize_u8_vec8_kernel(const float *__restrict__ X, uint8_t *__restrict__ Y, size_t n8, float scale, float inv_scale, int zp)
 {
    griddep_launch_dependents();
    griddep_wait(); // X is the previous kernel's output
    const size_t nthreads = (size_t)gridDim.x * blockDim.x;
 #pragma unroll 2
-   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n16; i += nthreads) {
-      float4 v[4];
+   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n8; i += nthreads) {
+      const float4 v[2] = {reinterpret_cast<const float4 *>(X)[2 * i], reinterpret_cast<const float4 *>(X)[2 * i + 1]};
+      uint32_t w[2];
 #pragma unroll
-      for (int j = 0; j < 4; j++) v[j] = reinterpret_cast<const float4 *>(X)[4 * i + j];
-      uint32_t w[4];
-#pragma unroll
-      for (int j = 0; j < 4; j++)
+      for (int j = 0; j < 2; j++)
          w[j] = (uint32_t)quant_u8(v[j].x, scale, inv_scale, zp) | ((uint32_t)quant_u8(v[j].y, scale, inv_scale, zp) << 8) |
                 ((uint32_t)quant_u8(v[j].z, scale, inv_scale, zp) << 16) | ((uint32_t)quant_u8(v[j].w, scale, inv_scale, zp) << 24);
-      reinterpret_cast<uint4 *>(Y)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+      reinterpret_cast<uint2 *>(Y)[i] = make_uint2(w[0], w[1]);
    }
 }
 
@@ -554,6 +703,7 @@ __global__ void quantize_u8_kernel(const float *__restrict__ X, uint8_t *__restr
    for (size_t i = n4 * 4 + tid; i < n; i += nthreads) Y[i] = quant_u8(X[i], scale, inv_scale, zp);
 }
 
+// (Eight elements a step with two 16-byte stores: 134 MB 44 us against 32; with one store of a whole sector 30, smaller tensors up to 8 % slower.)
 __global__ void dequantize_u8_kernel(const uint8_t *__restrict__ X, float *__restrict__ Y, size_t n, float scale,
                                      int zp, bool vec)
 {
@@ -777,6 +927,10 @@ int sofie_cuda_pool2d_f32(void *stream, const sofie_pool2d_desc *d, const float 
       const unsigned rows = (unsigned)((size_t)d->N * oH);
       if (d->mode == 0) pool2x2_f32_nhwc_kernel<false><<<grid_for(total / 4), kThreads, 0, s>>>(X, Y, rows, oW, d->C);
       else pool2x2_f32_nhwc_kernel<true><<<grid_for(total / 4), kThreads, 0, s>>>(X, Y, rows, oW, d->C);
+   } else if (d->kH == 2 && d->kW == 2 && d->stride_h == 2 && d->stride_w == 2 && !d->pads[0] && !d->pads[1] && !d->pads[2] && !d->pads[3] && d->layout != SOFIE_LAYOUT_NHWC &&
+              total < (1u << 31)) {
+      auto kernel = d->mode == 0 ? pool2x2_f32_any_kernel<false> : pool2x2_f32_any_kernel<true>;
+      SOFIE_CUDA_TRY(launch_dependent(kernel, dim3(grid_for(total)), dim3(kThreads), 0, s, X, Y, (unsigned)total, FastDiv((uint32_t)oW), FastDiv((uint32_t)oH), d->H, d->W));
    } else {
       const bool small = total < (1u << 31);
       const PoolCoords pc = small ? PoolCoords{FastDiv((uint32_t)oW), FastDiv((uint32_t)oH), FastDiv((uint32_t)d->C)} : PoolCoords();
@@ -823,10 +977,10 @@ int sofie_cuda_softmax_f32(void *stream, const float *X, float *Y, size_t outer,
       softmax_rows_reg1_kernel<4><<<grid_for(outer * 32), kThreads, 0, s>>>(X, Y, outer, (int)axis_len);
    else if (inner == 1 && axis_len <= 32 * 12)
       softmax_rows_reg1_kernel<12><<<grid_for(outer * 32), kThreads, 0, s>>>(X, Y, outer, (int)axis_len);
-   else if (inner == 1 && axis_len <= 32 * 32)
-      softmax_rows_reg1_kernel<32><<<grid_for(outer * 32), kThreads, 0, s>>>(X, Y, outer, (int)axis_len);
-   else if (inner == 1 && axis_len <= 32 * 64)
-      softmax_rows_reg1_kernel<64><<<grid_for(outer * 32), kThreads, 0, s>>>(X, Y, outer, (int)axis_len);
+   else if (inner == 1 && axis_len <= 128 * 8)
+      softmax_rows_shared_kernel<8><<<grid_for(outer * 128), kThreads, 0, s>>>(X, Y, outer, (int)axis_len);
+   else if (inner == 1 && axis_len <= 128 * 16)
+      softmax_rows_shared_kernel<16><<<grid_for(outer * 128), kThreads, 0, s>>>(X, Y, outer, (int)axis_len);
    else if (inner == 1)
       softmax_rows_kernel<<<grid_for(outer * 32), kThreads, 0, s>>>(X, Y, outer, axis_len);
    else
@@ -876,13 +1030,13 @@ int sofie_cuda_quantize_u8(void *stream, const float *X, uint8_t *Y, size_t n, f
    SOFIE_REQUIRE(scale > 0.f && zp >= 0 && zp <= 255, "bad quantisation parameters");
    if (n == 0) return SOFIE_CUDA_OK;
    const float inv_scale = 1.0f / scale;
-   if (aligned16(X) && aligned16(Y) && n >= 16) {
-      // the bulk sixteen elements at a time, the ragged end (fewer than 16 elements) with the scalar kernel
-      const size_t n16 = n / 16;
-      SOFIE_CUDA_TRY(launch_dependent(quantize_u8_vec16_kernel, dim3(grid_for(n16)), dim3(kThreads), 0, as_stream(stream), X, Y, n16, scale, inv_scale, (int)zp));
-      X += n16 * 16;
-      Y += n16 * 16;
-      n -= n16 * 16;
+   if (aligned16(X) && (reinterpret_cast<uintptr_t>(Y) & 7) == 0 && n >= 8) {
+      // the bulk eight elements at a time, the ragged end with the scalar kernel
+      const size_t n8 = n / 8;
+      SOFIE_CUDA_TRY(launch_dependent(quantize_u8_vec8_kernel, dim3(grid_for(n8)), dim3(kThreads), 0, as_stream(stream), X, Y, n8, scale, inv_scale, (int)zp));
+      X += n8 * 8;
+      Y += n8 * 8;
+      n -= n8 * 8;
       if (n == 0) return SOFIE_CUDA_OK;
    }
    bool vec = aligned16(X) && (reinterpret_cast<uintptr_t>(Y) & 3) == 0;

@@ -147,6 +147,45 @@ def test_gemm_f32_skinny(M, N, K, tA, tB, bias_kind):
     assert (np.abs(y[:M - 1] - ref) <= (K / 8 + 24) * 2.0 ** -24 * size).all()
 
 
+# images of whole 16-byte words, whose layout changes word by word, and others: channels that divide a word, that do not, and all 64; runs of pixels that end early; and back
+@pytest.mark.parametrize("N,C,H,W", [(3, 16, 8, 8), (2, 3, 10, 14), (2, 24, 16, 42), (1, 64, 6, 6), (5, 7, 2, 2), (2, 2, 64, 67), (2, 5, 9, 11), (1, 63, 37, 4)])
+def test_layout_words(N, C, H, W):
+    x = torch.randn((N, C, H, W), device="cuda")
+    y = ops.nchw_to_nhwc(x)
+    assert torch.equal(y, x.permute(0, 2, 3, 1).contiguous())
+    back = torch.empty_like(x)
+    capi.call("sofie_cuda_nhwc_to_nchw_f32", None, C_ptr(y), C_ptr(back), N, C, H, W)
+    torch.cuda.synchronize()
+    assert torch.equal(back, x)
+
+
+def C_ptr(t):
+    return C.c_void_p(t.data_ptr())
+
+
+# the 2 x 2 window on images of odd sizes (a last row or column left over), more outputs than a pass of the grid's; NaN as the comparisons have it
+@pytest.mark.parametrize("N,Ch,H,W", [(1, 1, 2, 2), (2, 3, 7, 9), (777, 3, 91, 85), (3, 5, 6, 42), (2, 2, 3, 2)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_pool2x2_any_size(N, Ch, H, W, mode):
+    x = np.random.default_rng(N + H).standard_normal((N, Ch, H, W)).astype(np.float32)
+    x[0, 0, 0, 1] = np.nan
+    ref = o.pool2d_f32(x, mode, (2, 2), (2, 2))
+    y = ops.pool2d_f32(dev(x), mode=mode).cpu().numpy()
+    assert np.array_equal(y, ref.reshape(y.shape), equal_nan=True)
+
+
+# rows shared by four warps, up to eight and sixteen values a thread, an odd number of rows; sums of `len` terms and an exponential of a few units
+@pytest.mark.parametrize("rows,length", [(3, 385), (7, 1000 + 1), (5, 1025), (2, 2047), (1200, 611)])
+def test_softmax_shared_rows(rows, length):
+    x = torch.randn((rows, length), device="cuda") * 3
+    x[0, 5] = -float("inf")
+    ref = torch.softmax(x.double(), 1)
+    y = ops.softmax_f32(x).double()
+    # relative: the rounding of x - max, which the exponential carries on; exp to 2 ulp, sums of up to 16 and 7 more, the division
+    bound = 2.0 ** -24 * ((x - x.max(1, keepdim=True).values).double().abs().clamp_max(200) + 4 + 23 + 1)
+    assert ((y - ref).abs() <= bound * ref + 1e-37).all()
+
+
 # rows that take the kernel with its weights in registers: one and two a block, the first beyond; pieces that end inside a lane's share (K = 20, 36), one lane to thirty-two an
 # output, an infinite input (zeros behind a row's inputs are no products of it), one to three layers
 @pytest.mark.parametrize("M,dims", [(1, (64, 128, 128, 10)), (148, (64, 128, 128, 10)), (149, (20, 36, 7)), (296, (256, 16, 64, 3)), (297, (64, 128, 128, 10)), (3, (256, 1)), (5, (16, 256, 4)),
