@@ -391,3 +391,21 @@ def test_results_land_in_pieces(cuda_device, nbytes):
         capi.call("sofie_cuda_ctx_check", ctx)
     finally:
         capi.call("sofie_cuda_ctx_destroy", ctx)
+
+
+@pytest.mark.parametrize("nbytes", [3, 524288, 524288 + 19, 700001, 1 << 20, (1 << 20) + 1, 3 << 20])
+def test_inputs_from_pageable_memory(cuda_device, nbytes):
+    """One kernel's fetch, two of them with a ragged end, and the copies above: the same bytes, nothing beside them, twice with other bytes."""
+    rng = np.random.default_rng(nbytes)
+    dst = torch.zeros(nbytes + 64, dtype=torch.uint8, device=cuda_device)
+    torch.cuda.synchronize()
+    ctx, _ = _ctx()
+    try:
+        for _ in range(2):
+            x = rng.integers(1, 256, nbytes, dtype=np.uint8)
+            capi.call("sofie_cuda_ctx_h2d", ctx, C.c_void_p(dst.data_ptr()), C.c_void_p(x.ctypes.data), C.c_size_t(nbytes))
+            capi.call("sofie_cuda_ctx_check", ctx)
+            got = dst.cpu().numpy()
+            assert np.array_equal(got[:nbytes], x) and not got[nbytes:].any()
+    finally:
+        capi.call("sofie_cuda_ctx_destroy", ctx)
