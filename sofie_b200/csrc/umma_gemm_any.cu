@@ -22,6 +22,8 @@
 #include "gemm_parts.cuh"
 #include "contract.cuh"
 
+#include <utility>
+
 namespace sofie {
 namespace umma {
 namespace {
@@ -158,8 +160,9 @@ __device__ __forceinline__ void any_write_checked(const AnyOperand &A, const Any
 #pragma unroll 1
          for (int k = 0; k < K; k++, a += as, b += bs) v = fmaf(*a, *b, v);
       }
-      const float bias = ep.bias_kind == 1 ? ep.C[col] : (ep.bias_kind == 2 ? ep.C[(size_t)row * B.rows + col] : 0.f);
-      ep.Y[(size_t)row * B.rows + col] = any_finish(ep, v, bias);
+      const size_t y = ep.turned ? (size_t)col * A.rows + row : (size_t)row * B.rows + col;
+      const float bias = ep.bias_kind == 1 ? ep.C[ep.turned ? row : col] : (ep.bias_kind == 2 ? ep.C[y] : 0.f);
+      ep.Y[y] = any_finish(ep, v, bias);
    }
 }
 
@@ -191,16 +194,19 @@ __device__ __forceinline__ void any_write(const AnyEpilogue &ep, const float *ti
             make_float4(any_finish(ep, v.x, b.x), any_finish(ep, v.y, b.y), any_finish(ep, v.z, b.z), any_finish(ep, v.w, b.w));
       }
    } else {
+      const int log_rows = __ffs(rows) - 1; // a power of two
 #pragma unroll 4
       for (int i = threadIdx.x; i < rows * BN; i += kAnyWorkers) {
-         const int r = r0 + i / BN, c = i % BN, row = m0 + r, col = n0 + c;
+         // threads along what is contiguous in Y
+         const int r = r0 + (ep.turned ? i & (rows - 1) : i / BN), c = ep.turned ? i >> log_rows : i % BN, row = m0 + r, col = n0 + c;
          if (row >= M || col >= N) continue;
-         const float b = ep.bias_kind == 1 ? ep.C[col] : (ep.bias_kind == 2 ? ep.C[(size_t)row * N + col] : 0.f);
+         const size_t y = ep.turned ? (size_t)col * M + row : (size_t)row * N + col;
+         const float b = ep.bias_kind == 1 ? ep.C[ep.turned ? row : col] : (ep.bias_kind == 2 ? ep.C[y] : 0.f);
          float v = 0.f;
          if (S == 1) v = tile[r * P + c];
          else
             for (int q = 0; q < S; q++) v += ld_cluster_f1(mapa_shared(base + (uint32_t)(r * P + c) * 4, (uint32_t)q));
-         ep.Y[(size_t)row * N + col] = any_finish(ep, v, b);
+         ep.Y[y] = any_finish(ep, v, b);
       }
    }
 }
@@ -443,8 +449,10 @@ int launch_any(cudaStream_t s, const AnyOperand &A, const AnyOperand &B, const A
 }
 
 // Time of a product on this kernel in ns, at its best tile width and cluster size.
-long long any_ns(const sofie_gemm_f32_desc &d, int &BN, int &S)
+long long any_ns(const sofie_gemm_f32_desc &desc, bool turned, int &BN, int &S)
 {
+   sofie_gemm_f32_desc d = desc;
+   if (turned) d.M = desc.N, d.N = desc.M;
    const int tm = ceil_div(d.M, kAnyBM), nkb = ceil_div(d.K, kAnyKE);
    // Tile width and clusters along K by the time they take, in ns (fitted to 450 products, each at every width and cluster size): a stage
    // of 32 K, a tile's start and end, the exchange within a cluster, and what the write-out takes more where rows of Y are not whole
@@ -452,7 +460,7 @@ long long any_ns(const sofie_gemm_f32_desc &d, int &BN, int &S)
    // 148 / 140 / 104 CTAs at a time.
    static const int widths[3] = {128, 64, 32}, stage[3] = {1210, 700, 750}, tile[3] = {4100, 2300, 1500}, scalar[3] = {2000, 1000, 470}, scalar_full[3] = {3500, 1600, 950},
                     room[4] = {kNumSMs, kNumSMs, 140, 104};
-   const bool vec = d.N % 4 == 0, full = d.bias_kind == 2;
+   const bool vec = d.N % 4 == 0 && !turned, full = d.bias_kind == 2;
    const long long bias = full ? (long long)d.M * d.N / 750 : 0;
    BN = 32, S = 1;
    long long best = -1;
@@ -467,6 +475,18 @@ long long any_ns(const sofie_gemm_f32_desc &d, int &BN, int &S)
       }
    }
    return best;
+}
+// Up to 31 rows fill a quarter of a tile of 128; the rest of it is zeros that are loaded, split and multiplied too. As the columns of a tile they fill it, and the long side makes the rows:
+// the same parts and products, written along the tile's rows. 30 x 1109 x 1819 28.3 -> 13.5 us, 18 x 2378 x 2513 32.7 -> 23.3, 9 x 2327 x 1695 24.2 -> 16.6. Taken where the estimate
+// says 0.7 of the time, and from K = 512 on, since these write word by word (31 x 3359 x 472 12.5 -> 13.3 us, 23 x 2937 x 405 1.04 of the time). From 32 rows on operands split beforehand are the faster ones (64 x 2533 x 3026 31 us, turned 41).
+long long any_best_ns(const sofie_gemm_f32_desc &d, bool &turned, int &BN, int &S)
+{
+   int other_BN, other_S;
+   const long long straight = any_ns(d, false, BN, S), other = d.M < 32 && d.K >= 512 ? any_ns(d, true, other_BN, other_S) : straight;
+   turned = 10 * other < 7 * straight;
+   if (!turned) return straight;
+   BN = other_BN, S = other_S;
+   return other;
 }
 // ... and on the CUDA-core kernel.
 long long simt_ns(const sofie_gemm_f32_desc &d)
@@ -483,7 +503,8 @@ long long simt_ns(const sofie_gemm_f32_desc &d)
 long long gemm_f32_whole_ns(const sofie_gemm_f32_desc &d, bool tma)
 {
    int BN, S;
-   const long long any = umma::any_ns(d, BN, S), simt = umma::simt_ns(d);
+   bool turned;
+   const long long any = umma::any_best_ns(d, turned, BN, S), simt = umma::simt_ns(d);
    return tma || simt > any ? any : simt;
 }
 
@@ -492,11 +513,16 @@ int launch_gemm_f32_any(cudaStream_t s, const sofie_gemm_f32_desc &d, bool tma, 
    using namespace umma;
    auto aligned = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
    const bool vec_k = d.K % 4 == 0;
-   const AnyOperand a{A, d.transA ? d.M : d.K, d.M, d.transA ? kRowsContiguous : (vec_k && aligned(A) ? kVecK : kScalarK)};
-   const AnyOperand b{B, d.transB ? d.K : d.N, d.N, !d.transB ? kRowsContiguous : (vec_k && aligned(B) ? kVecK : kScalarK)};
-   const AnyEpilogue ep{d.alpha, d.beta, C, Y, d.bias_kind, d.relu, d.N % 4 == 0 && aligned(Y) && (d.bias_kind != 2 || aligned(C)), d.K >= 1024 ? 8 : (d.K >= 256 ? 4 : 3)};
+   AnyOperand a{A, d.transA ? d.M : d.K, d.M, d.transA ? kRowsContiguous : (vec_k && aligned(A) ? kVecK : kScalarK)};
+   AnyOperand b{B, d.transB ? d.K : d.N, d.N, !d.transB ? kRowsContiguous : (vec_k && aligned(B) ? kVecK : kScalarK)};
+   AnyEpilogue ep{d.alpha, d.beta, C, Y, d.bias_kind, d.relu, d.N % 4 == 0 && aligned(Y) && (d.bias_kind != 2 || aligned(C)), d.K >= 1024 ? 8 : (d.K >= 256 ? 4 : 3)};
    int BN, S;
-   const long long best = any_ns(d, BN, S);
+   bool turned;
+   const long long best = any_best_ns(d, turned, BN, S);
+   if (turned) {
+      std::swap(a, b);
+      ep.turned = 1, ep.vec = 0;
+   }
    // What TMA cannot fetch has the CUDA-core kernel beside it: blocks of 64 x 64, steps of 16 K that take 1.9 us alone and 0.45 us (0.65 with
    // B stored [N,K]) apart on an SM full of them, whose outputs leave while other blocks compute. It wins where the output is what
    // counts: 16384 x 4093 x 8 with a full bias 163 us against 580, 16384 x 777 x 64 81 against 144; 1000 x 777 x 1333 211 against 38. Over

@@ -187,6 +187,28 @@ def test_softmax_shared_rows(rows, length):
     assert ((y - ref).abs() <= bound * ref + 1e-37).all()
 
 
+# few rows that are the columns of the tensor-core kernel's tiles: one tile and several of them a way, K split over clusters and not, both orders of both operands; an infinite value, whose
+# row is taken again term by term
+@pytest.mark.parametrize("M,N,K,tA,tB", [(30, 1109, 1819, 0, 0), (18, 2378, 2513, 0, 1), (9, 2327, 1695, 1, 1), (26, 2498, 2312, 1, 0), (31, 3384, 4090, 0, 0), (17, 2780, 967, 0, 0)])
+@pytest.mark.parametrize("bias_kind", [0, 1, 2])
+def test_gemm_f32_turned(M, N, K, tA, tB, bias_kind):
+    ops.set_engine(0)
+    rng = np.random.default_rng(M + N + K)
+    A, B = rng.standard_normal((K, M) if tA else (M, K)).astype(np.float32), rng.standard_normal((N, K) if tB else (K, N)).astype(np.float32)
+    bias = {0: None, 1: rng.standard_normal(N).astype(np.float32), 2: rng.standard_normal((M, N)).astype(np.float32)}[bias_kind]
+    a, b = (A.T if tA else A), (B if not tB else B.T)   # views of what the kernel gets
+    for infinite in (False, True):
+        if infinite:
+            a[M - 1, K - 1] = np.inf
+        rows = M - 1 if infinite else M
+        ref = 0.75 * (a[:rows].astype(np.float64) @ b.astype(np.float64)) + (0 if bias is None else 1.5 * (bias if bias_kind == 1 else bias[:rows]))
+        y = ops.gemm_f32(dev(A), dev(B), None if bias is None else dev(bias), transA=tA, transB=tB, alpha=0.75, beta=1.5, workspace=False).cpu().numpy()
+        assert ops.last_engine() == capi.ENGINE_TCGEN05
+        if infinite:
+            assert np.array_equal(y[M - 1], np.where(b[K - 1] > 0, np.inf, -np.inf))
+        assert rel_err(y[:rows], ref) <= FP32_TOL
+
+
 # rows that take the kernel with its weights in registers: one and two a block, the first beyond; pieces that end inside a lane's share (K = 20, 36), one lane to thirty-two an
 # output, an infinite input (zeros behind a row's inputs are no products of it), one to three layers
 @pytest.mark.parametrize("M,dims", [(1, (64, 128, 128, 10)), (148, (64, 128, 128, 10)), (149, (20, 36, 7)), (296, (256, 16, 64, 3)), (297, (64, 128, 128, 10)), (3, (256, 1)), (5, (16, 256, 4)),
