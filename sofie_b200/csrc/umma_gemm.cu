@@ -765,16 +765,23 @@ static int launch_pair(cudaStream_t s, const CUtensorMap &tmA, const CUtensorMap
 // through distributed shared memory: rank c % CS adds up and finishes the columns 32 c .. 32 c + 31, to which the others send their part as
 // [4 columns][row] pieces of 16 bytes (no two lanes of a quarter warp meet in a bank). The pieces lie in the pipeline's stages, which
 // are free once every rank's MMAs are done: that is what the first of the two cluster barriers is for.
-template <int KIND, int BN>
+//
+// FEW: a product of few rows. TMA would fill the tile of A up with zeros, which costs shared memory's time like data does and more (16 x 4096 x 4096 took longer than
+// 64 x 4096 x 4096), so only the rows there are, up to the next eight, are copied: a stage is that much shorter, and the rows of the MMAs' tile beyond them are whatever
+// follows in shared memory. Their sums are never read. E4M3, 4096 x 4096, with 8 / 24 / 40 / 80 rows: 11.7 -> 8.7 us, 11.7 -> 9.0, 10.0 -> 9.3, 10.1 -> 9.9; int8 9.6 -> 6.5, 9.5 -> 6.6,
+// 7.8 -> 7.1, 7.9 -> 7.5. From 100 rows on the stages of a fixed size are 2 % faster. What is left at 16 rows: 2.4 us for the weights (7 TB/s) and 4 that any K costs (launch, first copy,
+// two barriers of the cluster, the finish).
+template <int KIND, int BN, bool FEW>
 __global__ void __launch_bounds__((2 + kGemmEpilogueWarps8) * 32, 1)
 umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, GemmEpilogue ep, int M, int N, int K, int CS,
-                       int S, uint32_t *status)
+                       int S, int a_box, uint32_t *status)
 {
    static_assert(KIND == kI8 || KIND == kF8, "8-bit kinds");
    using L = GemmSmem<KIND, BN>;
    constexpr int EPI_WARPS = kGemmEpilogueWarps8, CHUNKS = BN / 32;
    constexpr uint32_t TMEM_COLS = BN;
    constexpr int kPieceBytes = kBM * 32 * 4;
+   const int a_bytes = FEW ? a_box : L::kATile; // of a stage
    extern __shared__ unsigned char smem_raw[];
    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
    __shared__ uint64_t full_bar[kGemmMaxStages], empty_bar[kGemmMaxStages], tmem_full, drain_bar;
@@ -788,8 +795,8 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
    const int tiles_n = (N + BN - 1) / BN;
    const int m0 = (tile / tiles_n) * kBM, n0 = (tile % tiles_n) * BN;
    const int num_kb = (K + kStageK - 1) / kStageK, kb0 = num_kb * rank / CS, kb1 = num_kb * (rank + 1) / CS;
-   auto a_tile = [&](int s) { return smem + (size_t)s * L::kStageBytes; };
-   auto b_tile = [&](int s) { return smem + (size_t)s * L::kStageBytes + L::kATile; };
+   auto a_tile = [&](int s) { return smem + (size_t)s * (a_bytes + L::kBTile); };
+   auto b_tile = [&](int s) { return smem + (size_t)s * (a_bytes + L::kBTile) + a_bytes; };
 
    if (threadIdx.x == 0) {
       for (int s = 0; s < kGemmMaxStages; s++) {
@@ -820,7 +827,7 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       griddep_wait(); // A is the previous kernel's output
       for (int kb = kb0; kb < kb1; kb++, ring_next(s, ph, S)) {
          if (!mbar_wait_warp(&empty_bar[s], ph ^ 1, &abort_flag, status, kStatusWaitEmpty, kb)) break;
-         warp_expect_tx(&full_bar[s], L::kATile + L::kBTile);
+         warp_expect_tx(&full_bar[s], a_bytes + L::kBTile);
          warp_tma_load_2d(a_tile(s), &tmA, kb * kStageK, m0, &full_bar[s]);
          warp_tma_load_2d(b_tile(s), &tmB, kb * kStageK, n0, &full_bar[s]);
          issued++;
@@ -850,7 +857,7 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
    __syncwarp();
    cluster_sync_all(); // every rank's MMAs are done: the stages are free to take the others' pieces
    if (warp == 0 && abort_flag) drain_copies(full_bar, s, ph, issued, S);
-   if (warp >= 2 && !abort_flag) {
+   if (warp >= 2 && !abort_flag && (!FEW || lane_base < M)) {
 #pragma unroll 1
       for (int c = group; c < CHUNKS; c += EPI_WARPS / 4) {
          const int owner = c % CS;
@@ -869,7 +876,7 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
    }
    __syncwarp();
    cluster_sync_all(); // the pieces have arrived
-   if (warp >= 2 && !abort_flag) {
+   if (warp >= 2 && !abort_flag && (!FEW || lane_base < M)) {
       const int row = m0 + lane_base + lane;
 #pragma unroll 1
       for (int own = group, c = rank + group * CS; c < CHUNKS; own += EPI_WARPS / 4, c += (EPI_WARPS / 4) * CS) {
@@ -902,14 +909,21 @@ umma_gemm_split_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
    }
 }
 
-template <int KIND, int BN>
+constexpr int kFewRows = 80;
+// Rows of A that the split kernel copies to a stage: whole groups of the swizzle's eight.
+static int split_rows(int M) { return M <= kFewRows ? (M + 7) / 8 * 8 : kBM; }
+
+template <int KIND, int BN, bool FEW>
 static int launch_split(cudaStream_t s, const CUtensorMap &tmA, const CUtensorMap &tmB, const GemmEpilogue &ep, int M, int N, int K, int CS)
 {
    using L = GemmSmem<KIND, BN>;
-   int stages = (200 * 1024) / L::kStageBytes;
+   const int a_bytes = split_rows(M) * kStageK, stage_bytes = a_bytes + L::kBTile;
+   int stages = (200 * 1024) / stage_bytes;
    if (stages > kGemmMaxStages) stages = kGemmMaxStages;
-   auto kern = umma_gemm_split_kernel<KIND, BN>;
-   const int smem = stages * L::kStageBytes + 1024;
+   auto kern = umma_gemm_split_kernel<KIND, BN, FEW>;
+   // The MMAs read whole tiles of A, the last stage's too. And the others' partial sums have room: 48 KB at 64 and 128 columns, where eight stages of FEW have 72 and 136
+   // at least, 96 KB at 256.
+   const int smem = stages * stage_bytes + (stage_bytes < L::kATile ? L::kATile - stage_bytes : 0) + 1024;
    SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), smem));
    uint32_t *status = device_status_word(s);
    if (!status) return fail(SOFIE_CUDA_ERR_CUDA, "cannot allocate the device status word");
@@ -926,7 +940,7 @@ static int launch_split(cudaStream_t s, const CUtensorMap &tmA, const CUtensorMa
    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
    cfg.attrs = attr;
    cfg.numAttrs = 2;
-   SOFIE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, ep, M, N, K, CS, stages, status));
+   SOFIE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tmA, tmB, ep, M, N, K, CS, stages, a_bytes, status));
    set_last_engine(SOFIE_ENGINE_TCGEN05);
    return SOFIE_CUDA_OK;
 }
@@ -1003,7 +1017,7 @@ static int launch_umma_gemm(cudaStream_t s, const void *A, const void *B, const 
    const CUtensorMapDataType dt = (KIND == kTF32) ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
    uint64_t dimsA[2] = {(uint64_t)K, (uint64_t)M}, dimsB[2] = {(uint64_t)K, (uint64_t)N};
    uint64_t stride[1] = {(uint64_t)K * ES};
-   uint32_t boxA[2] = {(uint32_t)(kStageK / ES), (uint32_t)kBM}, boxB[2] = {(uint32_t)(kStageK / ES), (uint32_t)BN};
+   uint32_t boxA[2] = {(uint32_t)(kStageK / ES), (uint32_t)(split > 1 ? split_rows(M) : kBM)}, boxB[2] = {(uint32_t)(kStageK / ES), (uint32_t)BN};
    int rc = make_tensor_map(&tmA, dt, 2, A, dimsA, stride, boxA, 128);
    if (rc) return rc;
    rc = make_tensor_map(&tmB, dt, 2, B, dimsB, stride, boxB, 128);
@@ -1024,9 +1038,14 @@ static int launch_umma_gemm(cudaStream_t s, const void *A, const void *B, const 
       return launch_one<KIND, 64>(s, tmA, tmB, ep, M, N, K);
    } else {
       if (split > 1) {
-         if (BN == 64) return launch_split<KIND, 64>(s, tmA, tmB, ep, M, N, K, split);
-         if (BN == 128) return launch_split<KIND, 128>(s, tmA, tmB, ep, M, N, K, split);
-         return launch_split<KIND, 256>(s, tmA, tmB, ep, M, N, K, split);
+         if (split_rows(M) < kBM) {
+            if (BN == 64) return launch_split<KIND, 64, true>(s, tmA, tmB, ep, M, N, K, split);
+            if (BN == 128) return launch_split<KIND, 128, true>(s, tmA, tmB, ep, M, N, K, split);
+            return launch_split<KIND, 256, true>(s, tmA, tmB, ep, M, N, K, split);
+         }
+         if (BN == 64) return launch_split<KIND, 64, false>(s, tmA, tmB, ep, M, N, K, split);
+         if (BN == 128) return launch_split<KIND, 128, false>(s, tmA, tmB, ep, M, N, K, split);
+         return launch_split<KIND, 256, false>(s, tmA, tmB, ep, M, N, K, split);
       }
       switch (BN) {
       case 32: return launch_one<KIND, 32>(s, tmA, tmB, ep, M, N, K);

@@ -124,6 +124,12 @@ def test_8_bit_products_that_share_k(M, N, K):
     assert np.array_equal(Yq.cpu().numpy(), o.quantize_e4m3(Y.float().cpu().numpy(), 0.05))
 
 
+# up to 80 rows only those are copied: one, eight, a group of eight begun, the last count of the kind and the first beyond, at each tile width and cluster size
+@pytest.mark.parametrize("M,N,K", [(1, 64, 4096), (8, 70, 2096), (9, 4090, 4112), (33, 4096, 4096), (80, 8190, 4096), (17, 16300, 4096), (81, 4096, 4096)])
+def test_8_bit_products_of_few_rows_that_share_k(M, N, K):
+    test_8_bit_products_that_share_k(M, N, K)
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 128, 128), (70, 45, 144), (1000, 512, 4096), (256, 4096, 512)])
 def test_gemm_e4m3_tcgen05(M, N, K):
     rng = np.random.default_rng(K + M)
