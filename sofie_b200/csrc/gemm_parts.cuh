@@ -43,7 +43,6 @@ struct AnyEpilogue {
    float *Y;
    int bias_kind, relu, vec; // vec: rows of Y (and of a full C) start on 16-byte boundaries
    int unit;                 // stages added up in one TMEM buffer (the tensor core's sums truncate) before they are promoted
-   int turned = 0;           // the tile's rows are Y's columns: the operands have changed places (umma_gemm_any.cu; vec is 0)
 };
 
 __device__ __forceinline__ float any_finish(const AnyEpilogue &ep, float v, float c)

@@ -22,8 +22,6 @@
 #include "gemm_parts.cuh"
 #include "contract.cuh"
 
-#include <utility>
-
 namespace sofie {
 namespace umma {
 namespace {
@@ -141,7 +139,7 @@ struct AnyLoader {
 __device__ __forceinline__ void workers_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kAnyWorkers) : "memory"); }
 
 // any_write below for a tile with doubtful sums.
-template <int BN>
+template <int BN, bool TURNED>
 __device__ __forceinline__ void any_write_checked(const AnyOperand &A, const AnyOperand &B, int K, const AnyEpilogue &ep, const float *tile, int S, int r0, int rows, int m0, int n0)
 {
    constexpr int P = AnySmem<BN>::kPitch;
@@ -160,19 +158,20 @@ __device__ __forceinline__ void any_write_checked(const AnyOperand &A, const Any
 #pragma unroll 1
          for (int k = 0; k < K; k++, a += as, b += bs) v = fmaf(*a, *b, v);
       }
-      const size_t y = ep.turned ? (size_t)col * A.rows + row : (size_t)row * B.rows + col;
-      const float bias = ep.bias_kind == 1 ? ep.C[ep.turned ? row : col] : (ep.bias_kind == 2 ? ep.C[y] : 0.f);
+      const size_t y = TURNED ? (size_t)col * A.rows + row : (size_t)row * B.rows + col;
+      const float bias = ep.bias_kind == 1 ? ep.C[TURNED ? row : col] : (ep.bias_kind == 2 ? ep.C[y] : 0.f);
       ep.Y[y] = any_finish(ep, v, bias);
    }
 }
 
-// Rows [r0, r0 + rows) of the tile at (m0, n0), the sum of the S partial tiles, to global memory.
-template <int BN>
+// Rows [r0, r0 + rows) of the tile at (m0, n0), the sum of the S partial tiles, to global memory. TURNED: the operands have changed places, the tile's rows are Y's columns;
+// a flag in the place of the template's cost every other product 0.2 us.
+template <int BN, bool TURNED>
 __device__ __forceinline__ void any_write(const AnyEpilogue &ep, const float *tile, int S, int r0, int rows, int m0, int n0, int M, int N)
 {
    constexpr int P = AnySmem<BN>::kPitch;
    const uint32_t base = smem_u32(tile);
-   if (ep.vec) {
+   if (!TURNED && ep.vec) {
 #pragma unroll 2
       for (int i = threadIdx.x; i < rows * (BN / 4); i += kAnyWorkers) {
          const int r = r0 + i / (BN / 4), c = (i % (BN / 4)) * 4, row = m0 + r, col = n0 + c;
@@ -198,10 +197,10 @@ __device__ __forceinline__ void any_write(const AnyEpilogue &ep, const float *ti
 #pragma unroll 4
       for (int i = threadIdx.x; i < rows * BN; i += kAnyWorkers) {
          // threads along what is contiguous in Y
-         const int r = r0 + (ep.turned ? i & (rows - 1) : i / BN), c = ep.turned ? i >> log_rows : i % BN, row = m0 + r, col = n0 + c;
+         const int r = r0 + (TURNED ? i & (rows - 1) : i / BN), c = TURNED ? i >> log_rows : i % BN, row = m0 + r, col = n0 + c;
          if (row >= M || col >= N) continue;
-         const size_t y = ep.turned ? (size_t)col * M + row : (size_t)row * N + col;
-         const float b = ep.bias_kind == 1 ? ep.C[ep.turned ? row : col] : (ep.bias_kind == 2 ? ep.C[y] : 0.f);
+         const size_t y = TURNED ? (size_t)col * M + row : (size_t)row * N + col;
+         const float b = ep.bias_kind == 1 ? ep.C[TURNED ? row : col] : (ep.bias_kind == 2 ? ep.C[y] : 0.f);
          float v = 0.f;
          if (S == 1) v = tile[r * P + c];
          else
@@ -212,7 +211,7 @@ __device__ __forceinline__ void any_write(const AnyEpilogue &ep, const float *ti
 }
 
 // Grid: S x min(tiles, SMs / S) CTAs in clusters of S; with S = 1 a CTA walks tiles (N fastest), with S > 1 it has one.
-template <int BN>
+template <int BN, bool TURNED>
 __global__ void __launch_bounds__(kAnyThreads, 1)
 umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, uint32_t *status)
 {
@@ -355,8 +354,8 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
          workers_sync();
          if (S > 1) break; // one tile per cluster: it is summed up below
          if (!abort_flag) {
-            if (doubt_flag) any_write_checked<BN>(A, B, K, ep, tile_out, 1, 0, kAnyBM, m0, n0);
-            else any_write<BN>(ep, tile_out, 1, 0, kAnyBM, m0, n0, M, N);
+            if (doubt_flag) any_write_checked<BN, TURNED>(A, B, K, ep, tile_out, 1, 0, kAnyBM, m0, n0);
+            else any_write<BN, TURNED>(ep, tile_out, 1, 0, kAnyBM, m0, n0, M, N);
          }
          workers_sync(); // the tile has been read: its place is the stages' again
          if (threadIdx.x == 0) doubt_flag = 0; // set again behind the next tile's first workers_sync
@@ -405,8 +404,8 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
          uint32_t doubt = 0;
          for (int q = 0; q < S; q++) doubt |= __float_as_uint(ld_cluster_f1(mapa_shared(smem_u32(const_cast<uint32_t *>(&doubt_flag)), (uint32_t)q)));
          const int r0 = rank * (kAnyBM / S), m0 = (tile0 / tiles_n) * kAnyBM, n0 = (tile0 % tiles_n) * BN;
-         if (doubt) any_write_checked<BN>(A, B, K, ep, tile_out, S, r0, kAnyBM / S, m0, n0);
-         else any_write<BN>(ep, tile_out, S, r0, kAnyBM / S, m0, n0, M, N);
+         if (doubt) any_write_checked<BN, TURNED>(A, B, K, ep, tile_out, S, r0, kAnyBM / S, m0, n0);
+         else any_write<BN, TURNED>(ep, tile_out, S, r0, kAnyBM / S, m0, n0, M, N);
       }
       __syncwarp();
       cluster_sync_all(); // nobody leaves while its tile is still read
@@ -420,11 +419,11 @@ umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, u
    }
 }
 
-template <int BN>
+template <int BN, bool TURNED = false>
 int launch_any(cudaStream_t s, const AnyOperand &A, const AnyOperand &B, const AnyEpilogue &ep, int K, int S)
 {
    using L = AnySmem<BN>;
-   auto kern = umma_gemm_any_kernel<BN>;
+   auto kern = umma_gemm_any_kernel<BN, TURNED>;
    SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), L::kBytes));
    uint32_t *status = device_status_word(s);
    if (!status) return fail(SOFIE_CUDA_ERR_CUDA, "cannot allocate the device status word");
@@ -513,16 +512,12 @@ int launch_gemm_f32_any(cudaStream_t s, const sofie_gemm_f32_desc &d, bool tma, 
    using namespace umma;
    auto aligned = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
    const bool vec_k = d.K % 4 == 0;
-   AnyOperand a{A, d.transA ? d.M : d.K, d.M, d.transA ? kRowsContiguous : (vec_k && aligned(A) ? kVecK : kScalarK)};
-   AnyOperand b{B, d.transB ? d.K : d.N, d.N, !d.transB ? kRowsContiguous : (vec_k && aligned(B) ? kVecK : kScalarK)};
-   AnyEpilogue ep{d.alpha, d.beta, C, Y, d.bias_kind, d.relu, d.N % 4 == 0 && aligned(Y) && (d.bias_kind != 2 || aligned(C)), d.K >= 1024 ? 8 : (d.K >= 256 ? 4 : 3)};
+   const AnyOperand a{A, d.transA ? d.M : d.K, d.M, d.transA ? kRowsContiguous : (vec_k && aligned(A) ? kVecK : kScalarK)};
+   const AnyOperand b{B, d.transB ? d.K : d.N, d.N, !d.transB ? kRowsContiguous : (vec_k && aligned(B) ? kVecK : kScalarK)};
+   const AnyEpilogue ep{d.alpha, d.beta, C, Y, d.bias_kind, d.relu, d.N % 4 == 0 && aligned(Y) && (d.bias_kind != 2 || aligned(C)), d.K >= 1024 ? 8 : (d.K >= 256 ? 4 : 3)};
    int BN, S;
    bool turned;
    const long long best = any_best_ns(d, turned, BN, S);
-   if (turned) {
-      std::swap(a, b);
-      ep.turned = 1, ep.vec = 0;
-   }
    // What TMA cannot fetch has the CUDA-core kernel beside it: blocks of 64 x 64, steps of 16 K that take 1.9 us alone and 0.45 us (0.65 with
    // B stored [N,K]) apart on an SM full of them, whose outputs leave while other blocks compute. It wins where the output is what
    // counts: 16384 x 4093 x 8 with a full bias 163 us against 580, 16384 x 777 x 64 81 against 144; 1000 x 777 x 1333 211 against 38. Over
@@ -530,6 +525,7 @@ int launch_gemm_f32_any(cudaStream_t s, const sofie_gemm_f32_desc &d, bool tma, 
    if (!tma && forced_engine() != SOFIE_ENGINE_TCGEN05) {
       if (simt_ns(d) < best) return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "faster on the CUDA cores");
    }
+   if (turned) return launch_any<32, true>(s, b, a, ep, d.K, S); // (a wider tile would be half padding)
    if (BN == 128) return launch_any<128>(s, a, b, ep, d.K, S);
    if (BN == 64) return launch_any<64>(s, a, b, ep, d.K, S);
    return launch_any<32>(s, a, b, ep, d.K, S);
