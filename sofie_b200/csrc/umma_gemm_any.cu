@@ -28,8 +28,9 @@ namespace {
 
 constexpr int kAnyWorkers = 16 * 32;
 // Groups of worker warps that take the stages in turn. Four were 5 to 10 % faster at 32 columns with a long K and as much slower with a
-// short one (the pipeline takes longer to start), and spilled at 64 columns.
-constexpr int kAnyGroups = 2;
+// short one (the pipeline takes longer to start), and spilled at 64 columns. Turned tiles (K >= 512, below) have four: 27 x 2512 x 3682 28.1 -> 26.2 us, 13 x 1652 x 2420 13.6 -> 12.9,
+// 15 x 1446 x 1006 10.4 -> 10.7.
+constexpr int kAnyGroups = 2, kAnyTurnedGroups = 4;
 constexpr int kAnyThreads = kAnyWorkers + 32; // and the warp that issues the MMAs
 constexpr int kAnyMaxStages = 5;
 
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(kAnyThreads, 1)
 umma_gemm_any_kernel(AnyOperand A, AnyOperand B, AnyEpilogue ep, int K, int S, uint32_t *status)
 {
    using L = AnySmem<BN>;
-   constexpr int G = kAnyGroups, GT = kAnyWorkers / G; // groups and their threads
+   constexpr int G = TURNED ? kAnyTurnedGroups : kAnyGroups, GT = kAnyWorkers / G; // groups and their threads
    constexpr int QUARTER = BN / 4;       // columns of the tile a worker warp adds up
    constexpr uint32_t TMEM_COLS = 4 * BN; // two buffers of [the leading products | the smaller ones]
    extern __shared__ unsigned char smem_raw[];
@@ -476,13 +477,14 @@ long long any_ns(const sofie_gemm_f32_desc &desc, bool turned, int &BN, int &S)
    return best;
 }
 // Up to 31 rows fill a quarter of a tile of 128; the rest of it is zeros that are loaded, split and multiplied too. As the columns of a tile they fill it, and the long side makes the rows:
-// the same parts and products, written along the tile's rows. 30 x 1109 x 1819 28.3 -> 13.5 us, 18 x 2378 x 2513 32.7 -> 23.3, 9 x 2327 x 1695 24.2 -> 16.6. Taken where the estimate
-// says 0.7 of the time, and from K = 512 on, since these write word by word (31 x 3359 x 472 12.5 -> 13.3 us, 23 x 2937 x 405 1.04 of the time). From 32 rows on operands split beforehand are the faster ones (64 x 2533 x 3026 31 us, turned 41).
+// the same parts and products, written along the tile's rows. 30 x 1109 x 1819 28.3 -> 13.1 us, 18 x 2378 x 2513 32.7 -> 23.1, 9 x 2327 x 1695 24.2 -> 16.7. Taken where the estimate
+// says 0.8 of the time: of 148 products timed each way the 44 below it took 0.65 to 1.00, the others 0.91 to 1.47 (but for four). From K = 512 on, since these write word by word
+// (31 x 3359 x 472 12.5 -> 13.3 us). From 32 rows on operands split beforehand are the faster ones (64 x 2533 x 3026 31 us, turned 41).
 long long any_best_ns(const sofie_gemm_f32_desc &d, bool &turned, int &BN, int &S)
 {
    int other_BN, other_S;
    const long long straight = any_ns(d, false, BN, S), other = d.M < 32 && d.K >= 512 ? any_ns(d, true, other_BN, other_S) : straight;
-   turned = 10 * other < 7 * straight;
+   turned = 10 * other < 8 * straight;
    if (!turned) return straight;
    BN = other_BN, S = other_S;
    return other;
