@@ -143,6 +143,10 @@ inline cudaError_t allow_smem(const void *kernel, int bytes)
    return err;
 }
 
+// CTAs of kernels of one CTA an SM (their shared memory takes more than half of one) that run at a time in clusters of 2, 4 or 8: it differs from card to card with the SMs that its
+// processing clusters have (132 and 140 of 148 were seen at four, 104 and 120 at eight), and a tile too many costs a whole round. Asked for once a device.
+int cluster_room(int size);
+
 // ---- requantisation recipe shared by every int8 kernel -------------------------------------------
 // q = clamp(rne((float)acc * mult), qmin - zp, qmax - zp) + zp, with no FMA contraction, so a CPU
 // evaluating nearbyintf((float)acc * mult) under the default rounding mode gets the same bits.

@@ -456,10 +456,10 @@ long long any_ns(const sofie_gemm_f32_desc &desc, bool turned, int &BN, int &S)
    const int tm = ceil_div(d.M, kAnyBM), nkb = ceil_div(d.K, kAnyKE);
    // Tile width and clusters along K by the time they take, in ns (fitted to 450 products, each at every width and cluster size): a stage
    // of 32 K, a tile's start and end, the exchange within a cluster, and what the write-out takes more where rows of Y are not whole
-   // 16-byte words and where a bias of Y's shape is read. Nothing overlaps a CTA's write-out. Clusters of 2 / 4 / 8 found room for
-   // 148 / 140 / 104 CTAs at a time.
-   static const int widths[3] = {128, 64, 32}, stage[3] = {1210, 700, 750}, tile[3] = {4100, 2300, 1500}, scalar[3] = {2000, 1000, 470}, scalar_full[3] = {3500, 1600, 950},
-                    room[4] = {kNumSMs, kNumSMs, 140, 104};
+   // 16-byte words and where a bias of Y's shape is read. Nothing overlaps a CTA's write-out. Clusters that the card has no room for wait for a
+   // round to end: with 140 CTAs taken for granted at four, where it has 132, 14 x 2144 x 1368 took 22.6 us (13.4 turned) and 19 x 2227 x 740 19.9 (12.1).
+   static const int widths[3] = {128, 64, 32}, stage[3] = {1210, 700, 750}, tile[3] = {4100, 2300, 1500}, scalar[3] = {2000, 1000, 470}, scalar_full[3] = {3500, 1600, 950};
+   const int room[4] = {kNumSMs, cluster_room(2), cluster_room(4), cluster_room(8)};
    const bool vec = d.N % 4 == 0 && !turned, full = d.bias_kind == 2;
    const long long bias = full ? (long long)d.M * d.N / 750 : 0;
    BN = 32, S = 1;

@@ -189,7 +189,8 @@ def test_softmax_shared_rows(rows, length):
 
 # few rows that are the columns of the tensor-core kernel's tiles: one tile and several of them a way, K split over clusters and not, both orders of both operands; an infinite value, whose
 # row is taken again term by term
-@pytest.mark.parametrize("M,N,K,tA,tB", [(30, 1109, 1819, 0, 0), (18, 2378, 2513, 0, 1), (9, 2327, 1695, 1, 1), (26, 2498, 2312, 1, 0), (31, 3384, 4090, 0, 0), (17, 2780, 967, 0, 0)])
+@pytest.mark.parametrize("M,N,K,tA,tB", [(30, 1109, 1819, 0, 0), (18, 2378, 2513, 0, 1), (9, 2327, 1695, 1, 1), (26, 2498, 2312, 1, 0), (31, 3384, 4090, 0, 0), (17, 2780, 967, 0, 0),
+                                         (14, 2144, 1368, 0, 1), (31, 2238, 1277, 1, 0)])   # straight they would be 136 and 140 CTAs in fours
 @pytest.mark.parametrize("bias_kind", [0, 1, 2])
 def test_gemm_f32_turned(M, N, K, tA, tB, bias_kind):
     ops.set_engine(0)

@@ -125,7 +125,8 @@ def test_8_bit_products_that_share_k(M, N, K):
 
 
 # up to 80 rows only those are copied: one, eight, a group of eight begun, the last count of the kind and the first beyond, at each tile width and cluster size
-@pytest.mark.parametrize("M,N,K", [(1, 64, 4096), (8, 70, 2096), (9, 4090, 4112), (33, 4096, 4096), (80, 8190, 4096), (17, 16300, 4096), (81, 4096, 4096)])
+@pytest.mark.parametrize("M,N,K", [(1, 64, 4096), (8, 70, 2096), (9, 4090, 4112), (33, 4096, 4096), (80, 8190, 4096), (17, 16300, 4096), (81, 4096, 4096),
+                                   (100, 4480, 2048), (130, 2176, 4096)])   # and 140 and 136 CTAs in fours, for which not every card has room at a time
 def test_8_bit_products_of_few_rows_that_share_k(M, N, K):
     test_8_bit_products_that_share_k(M, N, K)
 
