@@ -144,8 +144,12 @@ inline cudaError_t allow_smem(const void *kernel, int bytes)
 }
 
 // CTAs of kernels of one CTA an SM (their shared memory takes more than half of one) that run at a time in clusters of 2, 4 or 8: it differs from card to card with the SMs that its
-// processing clusters have (132 and 140 of 148 were seen at four, 104 and 120 at eight), and a tile too many costs a whole round. Asked for once a device.
-int cluster_room(int size);
+// processing clusters have (132 and 140 of 148 were seen at four, 104 and 120 at eight), and a tile too many costs a whole round. Asked for once a device; a launcher takes them once
+// a call, since looking up the device costs each of its callers host time.
+struct ClusterRoom {
+   int ctas[4]; // in clusters of 1, 2, 4 and 8
+};
+ClusterRoom cluster_room();
 
 // ---- requantisation recipe shared by every int8 kernel -------------------------------------------
 // q = clamp(rne((float)acc * mult), qmin - zp, qmax - zp) + zp, with no FMA contraction, so a CPU

@@ -986,13 +986,14 @@ static void choose_tile(int M, int N, int K, int scalar, int &BN, int &split)
 {
    static const int widths[3] = {64, 128, 256}, stage[3] = {295, 305, 340}, tile[3] = {700, 1300, 2600};
    static const int stores[9] = {0, 3400, 7400, 0, 16500, 0, 0, 0, 32000}; // 128 rows of 1, 2, 4, 8 chunks of 32 columns
+   const ClusterRoom room = cluster_room();
    const long long tm = ceil_div(M, kBM), kb = ceil_div(K, kStageK);
    long long best = -1;
    for (int w = 0; w < 3; w++) {
       if (w > 0 && widths[w] / 2 >= N) break; // more than half of the tile would be padding
       const long long tiles = tm * ceil_div(N, widths[w]), chunks = widths[w] / 32;
       for (int q = 1; q <= 4; q *= 2) {
-         if (q > 1 && (kb < 2 * q || tiles * q > cluster_room(q))) break;
+         if (q > 1 && (kb < 2 * q || tiles * q > room.ctas[q / 2])) break;
          const long long rounds = (tiles * q + kNumSMs - 1) / kNumSMs;
          const long long store = (long long)scalar * stores[ceil_div<long long>(chunks, q)] * (M < kBM ? M : kBM) / kBM;
          const long long time = rounds * (ceil_div<long long>(kb, q) * stage[w] + 700 + store) + tile[w] / q + (q > 1 ? 1700 + 500 * (chunks - chunks / q) + 1200 * scalar : 0);
