@@ -513,6 +513,7 @@ constexpr size_t kPullMaxBytes = size_t(512) << 10;
 // call, 0.8 MB (98 of the residual block) 75 -> 68, 1 MB (4096 rows of the perceptron) 90 -> 80; 1.2 MB no difference, 1.6 MB 95 -> 100; ranges of an input, with results on their
 // way out beside them, 284 -> 319 (int8 perceptron, 8192 rows).
 constexpr size_t kPullTwiceBytes = size_t(1) << 20;
+// Its words are of 16 bytes: a piece behind a fill that was begun ahead, of a length its caller chose, need not start on one and is copied.
 constexpr int kPullThreads = 256;
 __global__ void __launch_bounds__(kPullThreads) pull_kernel(const uint4 *__restrict__ src, uint4 *__restrict__ dst, uint32_t n16, const uint8_t *__restrict__ src1,
                                                             uint8_t *__restrict__ dst1, uint32_t rest)
@@ -560,7 +561,7 @@ static int stage_slots(sofie_cuda_ctx *ctx, const HostConvert &how, void *dst, c
       const size_t next = done + now->bytes;
       if (next < bytes && (rc = begin_fill(ctx, how, src + next * how.ratio(), bytes - next < step ? bytes - next : step, &cur))) return rc;
       if (ctx->fail_copy > 0 && --ctx->fail_copy == 0) rc = fail(SOFIE_CUDA_ERR_CUDA, "staged copy refused (self test)");
-      else if (small) rc = pull(stream, static_cast<char *>(dst) + done, now->mem, now->bytes);
+      else if (small && done % 16 == 0) rc = pull(stream, static_cast<char *>(dst) + done, now->mem, now->bytes);
       else SOFIE_CUDA_TRY(cudaMemcpyAsync(static_cast<char *>(dst) + done, now->mem, now->bytes, cudaMemcpyHostToDevice, stream));
       if (rc) return rc;
       now->slot->busy = true;

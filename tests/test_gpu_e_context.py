@@ -409,3 +409,28 @@ def test_inputs_from_pageable_memory(cuda_device, nbytes):
             assert np.array_equal(got[:nbytes], x) and not got[nbytes:].any()
     finally:
         capi.call("sofie_cuda_ctx_destroy", ctx)
+
+
+@pytest.mark.parametrize("part", [None, 0])
+@pytest.mark.parametrize("ahead,nbytes", [(1, 4096), (1001, 4096), (1001, 300000), (4096, 300000), (4100, 700001), (16, 17), (2 << 20, 3 << 20)])
+def test_a_fill_ahead_that_is_shorter_than_its_copy(cuda_device, ahead, nbytes, part):
+    """The helpers were started on fewer bytes than the copy takes, on whatever number the caller named: the pieces behind it begin on no boundary."""
+    rng = np.random.default_rng(ahead + nbytes)
+    dst = torch.zeros(nbytes + 64, dtype=torch.uint8, device=cuda_device)
+    torch.cuda.synchronize()
+    ctx, _ = _ctx()
+    try:
+        for _ in range(2):
+            x = rng.integers(1, 256, nbytes, dtype=np.uint8)
+            capi.call("sofie_cuda_ctx_stage_ahead", ctx, C.c_void_p(x.ctypes.data), C.c_size_t(ahead), 0, 1.0, 0)
+            args = (ctx, C.c_void_p(dst.data_ptr()), C.c_void_p(x.ctypes.data), C.c_size_t(nbytes))
+            if part is None:
+                capi.call("sofie_cuda_ctx_h2d", *args)
+            else:
+                capi.call("sofie_cuda_ctx_h2d_part", *args, part)
+                capi.call("sofie_cuda_ctx_wait_part", ctx, part)
+            capi.call("sofie_cuda_ctx_check", ctx)
+            got = dst.cpu().numpy()
+            assert np.array_equal(got[:nbytes], x) and not got[nbytes:].any()
+    finally:
+        capi.call("sofie_cuda_ctx_destroy", ctx)
