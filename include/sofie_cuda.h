@@ -123,7 +123,7 @@ int sofie_cuda_ctx_fetch(sofie_cuda_ctx *ctx, const void *src_device, size_t byt
  * fills from the context's pinned buffer; or NULL: anywhere) and its size; _part copies `bytes` bytes at `offset` of it, once
  * the work enqueued so far is done -- a part that is not the whole runs on a stream of its own, under later parts' kernels and
  * input copies; _end waits, reports a kernel that gave up as sofie_cuda_ctx_fetch does, and returns the address (out_host, or
- * pinned memory of the context that stays valid until the next result). At most SOFIE_CUDA_MAX_PARTS parts. */
+ * pinned memory of the context that stays valid until the next result). At most SOFIE_CUDA_MAX_PARTS parts, whatever their sizes. */
 int sofie_cuda_ctx_result_begin(sofie_cuda_ctx *ctx, void *out_host, size_t bytes);
 int sofie_cuda_ctx_result_part(sofie_cuda_ctx *ctx, const void *src_device, size_t offset, size_t bytes);
 int sofie_cuda_ctx_result_end(sofie_cuda_ctx *ctx, void **host);

@@ -131,6 +131,7 @@ constexpr int kStagingSlots = 8;
 constexpr size_t kStagingSlot = size_t(2) << 20;
 constexpr size_t kStagingBytes = kStagingSlots * kStagingSlot;
 constexpr size_t kLandInPieces = size_t(5) << 19; // a result that lands in one piece below this (sofie_cuda_ctx_result_part)
+constexpr int kLandings = 2 * SOFIE_CUDA_MAX_PARTS - 1; // copies of a result: a whole one's pieces and seven parts more
 constexpr size_t kPastCaches = size_t(32) << 20; // a result from which on the host's caches hold no useful part of it
 
 struct sofie_cuda_ctx {
@@ -167,12 +168,13 @@ struct sofie_cuda_ctx {
       char *land = nullptr;   // pinned memory the copies write: out, or `result`
       const char *mapped = nullptr; // the kernels wrote it to host memory themselves
       size_t bytes = 0;
-      int parts = 0;
-      size_t offset[SOFIE_CUDA_MAX_PARTS], count[SOFIE_CUDA_MAX_PARTS];
+      int parts = 0;  // the caller's
+      int pieces = 0; // copies: a part, or (one part only, the whole) a piece of it
+      size_t offset[kLandings], count[kLandings];
    } landing;
    cudaStream_t result_stream = nullptr; // results that are copied part by part, under the kernels of later parts
    cudaEvent_t ready_event = nullptr;    // a part's kernels are done
-   cudaEvent_t landed_event[SOFIE_CUDA_MAX_PARTS] = {};
+   cudaEvent_t landed_event[kLandings] = {};
    struct Captured {
       cudaGraph_t graph = nullptr;
       cudaGraphExec_t exec = nullptr;
@@ -882,7 +884,7 @@ int sofie_cuda_ctx_result_part(sofie_cuda_ctx *ctx, const void *src, size_t offs
    // tens of MB that the cores have just read runs at a quarter of the link's rate).
    const bool carried = l.out && l.land != l.out;
    size_t pieces = 1;
-   if (carried && bytes == l.bytes && l.parts == 0 && bytes >= kLandInPieces) {
+   if (carried && bytes == l.bytes && l.pieces == 0 && bytes >= kLandInPieces) {
       pieces = bytes / (size_t(2) << 20);
       pieces = pieces < 2 ? 2 : (pieces > SOFIE_CUDA_MAX_PARTS ? SOFIE_CUDA_MAX_PARTS : pieces);
    }
@@ -890,14 +892,15 @@ int sofie_cuda_ctx_result_part(sofie_cuda_ctx *ctx, const void *src, size_t offs
    for (size_t at = 0; at < bytes; at += piece) {
       const size_t n = bytes - at < piece ? bytes - at : piece;
       SOFIE_CUDA_TRY(cudaMemcpyAsync(l.land + offset + at, s8 + at, n, cudaMemcpyDeviceToHost, stream));
-      if (carried && n != l.bytes) {
-         cudaEvent_t &e = ctx->landed_event[l.parts];
+      if (carried && (n != l.bytes || l.pieces > 0)) {
+         cudaEvent_t &e = ctx->landed_event[l.pieces];
          if (!e) SOFIE_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
          SOFIE_CUDA_TRY(cudaEventRecord(e, stream));
       }
-      l.offset[l.parts] = offset + at;
-      l.count[l.parts++] = n;
+      l.offset[l.pieces] = offset + at;
+      l.count[l.pieces++] = n;
    }
+   l.parts++;
    return SOFIE_CUDA_OK;
 }
 
@@ -912,9 +915,10 @@ int sofie_cuda_ctx_result_end(sofie_cuda_ctx *ctx, void **host)
    if (carry) {
       int rc = ensure_pool(ctx);
       if (rc) return rc;
-      if (l.parts > 1)
-         for (int i = 0; i < l.parts; i++) { // each part as soon as it has landed, under the copies of the later ones
-            SOFIE_CUDA_TRY(cudaEventSynchronize(ctx->landed_event[i]));
+      if (l.pieces > 1)
+         for (int i = 0; i < l.pieces; i++) { // each as soon as it has landed, under the copies of the later ones
+            if (i == 0 && l.count[0] == l.bytes) SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->stream)); // the whole at once, and parts of it again
+            else SOFIE_CUDA_TRY(cudaEventSynchronize(ctx->landed_event[i]));
             ctx->host_pool->copy(l.out + l.offset[i], l.land + l.offset[i], l.count[i], l.bytes >= kPastCaches);
          }
    }
@@ -926,7 +930,7 @@ int sofie_cuda_ctx_result_end(sofie_cuda_ctx *ctx, void **host)
    for (auto &slot : ctx->slots) copying = copying || (slot.busy && slot.stream == ctx->copy_stream);
    if (copying) SOFIE_CUDA_TRY(cudaStreamSynchronize(ctx->copy_stream));
    slots_free(ctx);
-   if (carry && l.parts == 1) ctx->host_pool->copy(l.out + l.offset[0], l.land + l.offset[0], l.count[0], l.bytes >= kPastCaches);
+   if (carry && l.pieces == 1) ctx->host_pool->copy(l.out + l.offset[0], l.land + l.offset[0], l.count[0], l.bytes >= kPastCaches);
    release_pool(ctx);
    if (l.mapped && l.out) std::memcpy(l.out, l.mapped, l.bytes);
    *host = l.out ? l.out : (l.mapped ? const_cast<char *>(l.mapped) : l.land);
