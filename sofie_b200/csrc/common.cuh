@@ -143,13 +143,10 @@ inline cudaError_t allow_smem(const void *kernel, int bytes)
    return err;
 }
 
-// CTAs of kernels of one CTA an SM (their shared memory takes more than half of one) that run at a time in clusters of 2, 4 or 8: it differs from card to card with the SMs that its
-// processing clusters have (132 and 140 of 148 were seen at four, 104 and 120 at eight), and a tile too many costs a whole round. Asked for once a device; a launcher takes them once
-// a call, since looking up the device costs each of its callers host time.
-struct ClusterRoom {
-   int ctas[4]; // in clusters of 1, 2, 4 and 8
-};
-ClusterRoom cluster_room();
+// CTAs of kernels of one CTA an SM (their shared memory takes more than half of one) that run at a time in clusters of 1, 2, 4 and 8, for the estimates that cut a product along K. Cards
+// differ with the SMs that their processing clusters have (132 and 140 of 148 were seen at four, 104 and 120 at eight), and a cluster too many costs a whole round: the least seen. One
+// figure for every card, not the one a product runs on, since the cut decides the last bits of its sums: a model gives the same result on all of them.
+constexpr int kClusterRoom[4] = {kNumSMs, kNumSMs, 132, 104};
 
 // ---- requantisation recipe shared by every int8 kernel -------------------------------------------
 // q = clamp(rne((float)acc * mult), qmin - zp, qmax - zp) + zp, with no FMA contraction, so a CPU

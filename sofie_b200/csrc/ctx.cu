@@ -9,7 +9,6 @@
 #include "host_convert.cuh"
 #include "host_pool.cuh"
 
-#include <atomic>
 #include <cstdlib>
 #include <memory>
 #include <utility>
@@ -68,42 +67,6 @@ void unregister_stream_status(cudaStream_t stream)
          g_stream_status.erase(g_stream_status.begin() + i);
          return;
       }
-}
-
-__global__ void __launch_bounds__(128, 1) cluster_room_kernel() {}
-
-ClusterRoom cluster_room()
-{
-   static constexpr int kDevices = 64;
-   static std::atomic<int> asked[kDevices][3]; // 0: not yet
-   ClusterRoom room = {{kNumSMs, kNumSMs, 132, 104}};
-   int dev = -1;
-   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return room;
-   for (int i = 0; i < 3; i++) {
-      int n = asked[dev][i].load(std::memory_order_relaxed);
-      if (!n) {
-         constexpr int smem = 150 * 1024;
-         const int size = 2 << i;
-         cudaLaunchAttribute attr = {};
-         attr.id = cudaLaunchAttributeClusterDimension;
-         attr.val.clusterDim.x = (unsigned)size;
-         attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-         cudaLaunchConfig_t cfg = {};
-         cfg.gridDim = dim3(size * kNumSMs);
-         cfg.blockDim = dim3(128);
-         cfg.dynamicSmemBytes = smem;
-         cfg.attrs = &attr;
-         cfg.numAttrs = 1;
-         if (allow_smem(reinterpret_cast<const void *>(cluster_room_kernel), smem) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, cluster_room_kernel, &cfg) != cudaSuccess || n < 1) {
-            cudaGetLastError();
-            continue;
-         }
-         n = n * size < kNumSMs ? n * size : kNumSMs;
-         asked[dev][i].store(n, std::memory_order_relaxed);
-      }
-      room.ctas[i + 1] = n;
-   }
-   return room;
 }
 
 uint32_t *device_status_word(cudaStream_t stream)

@@ -977,7 +977,7 @@ static int launch_one(cudaStream_t s, const CUtensorMap &tmA, const CUtensorMap 
 // A stage costs almost the same at every width, so one round of wide tiles beats two of narrow ones (690 x 4096 x 4096 27.7 -> 18.7 us),
 // and where even narrow tiles leave SMs idle K is shared (128 x 4096 x 4096 15.4 -> 11.5 us, 300 x 4096 x 4096 25.3 -> 15.1,
 // 512 x 256 x 2048 11.0 -> 9.0; 1000 x 1024 x 512 is left at 64 columns, 5.9 us against 7.7 shared by two).
-// Shared tiles get one round of what the card has room for: a cluster more than fits waits for the others to end (int8, with 140 CTAs at four taken for granted and room for 132:
+// Shared tiles get one round of kClusterRoom: a cluster more than the card has room for waits for the others to end (int8, with 140 CTAs at four taken for granted and room for 132:
 // 130 x 4352 x 4096 18.9 us, now 8.8; 100 x 8704 x 4096 19.2, now 8.9).
 // `scalar` outputs have rows that are no multiple of 16 bytes and are stored value by value: the stores of a CTA's columns are then most of a short
 // product's time, and more than proportional to their number (723 x 1855 x 80 25.1 us in one round of 128 columns, 19.3 in two of 64; 1009 x 131 x 768
@@ -986,14 +986,13 @@ static void choose_tile(int M, int N, int K, int scalar, int &BN, int &split)
 {
    static const int widths[3] = {64, 128, 256}, stage[3] = {295, 305, 340}, tile[3] = {700, 1300, 2600};
    static const int stores[9] = {0, 3400, 7400, 0, 16500, 0, 0, 0, 32000}; // 128 rows of 1, 2, 4, 8 chunks of 32 columns
-   const ClusterRoom room = cluster_room();
    const long long tm = ceil_div(M, kBM), kb = ceil_div(K, kStageK);
    long long best = -1;
    for (int w = 0; w < 3; w++) {
       if (w > 0 && widths[w] / 2 >= N) break; // more than half of the tile would be padding
       const long long tiles = tm * ceil_div(N, widths[w]), chunks = widths[w] / 32;
       for (int q = 1; q <= 4; q *= 2) {
-         if (q > 1 && (kb < 2 * q || tiles * q > room.ctas[q / 2])) break;
+         if (q > 1 && (kb < 2 * q || tiles * q > kClusterRoom[q / 2])) break;
          const long long rounds = (tiles * q + kNumSMs - 1) / kNumSMs;
          const long long store = (long long)scalar * stores[ceil_div<long long>(chunks, q)] * (M < kBM ? M : kBM) / kBM;
          const long long time = rounds * (ceil_div<long long>(kb, q) * stage[w] + 700 + store) + tile[w] / q + (q > 1 ? 1700 + 500 * (chunks - chunks / q) + 1200 * scalar : 0);

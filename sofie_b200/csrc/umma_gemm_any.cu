@@ -449,7 +449,7 @@ int launch_any(cudaStream_t s, const AnyOperand &A, const AnyOperand &B, const A
 }
 
 // Time of a product on this kernel in ns, at its best tile width and cluster size.
-long long any_ns(const sofie_gemm_f32_desc &desc, const ClusterRoom &room, bool turned, int &BN, int &S)
+long long any_ns(const sofie_gemm_f32_desc &desc, bool turned, int &BN, int &S)
 {
    sofie_gemm_f32_desc d = desc;
    if (turned) d.M = desc.N, d.N = desc.M;
@@ -468,7 +468,7 @@ long long any_ns(const sofie_gemm_f32_desc &desc, const ClusterRoom &room, bool 
       const long long tiles = (long long)tm * ceil_div(d.N, widths[w]);
       const int out = vec ? 0 : scalar[w] + (full ? scalar_full[w] : 0);
       for (int i = 0, q = 1; i < 4 && (q == 1 || (nkb >= 2 * q && tiles * q <= 3 * kNumSMs)); i++, q *= 2) {
-         const long long waves = (tiles * q + room.ctas[i] - 1) / room.ctas[i];
+         const long long waves = (tiles * q + kClusterRoom[i] - 1) / kClusterRoom[i];
          const long long time = 1400 + bias + waves * ((long long)ceil_div(nkb, q) * stage[w] + tile[w] + out / q + (q > 1 ? 2100 : 0));
          if (best < 0 || time < best) best = time, BN = widths[w], S = q;
       }
@@ -481,9 +481,8 @@ long long any_ns(const sofie_gemm_f32_desc &desc, const ClusterRoom &room, bool 
 // (31 x 3359 x 472 12.5 -> 13.3 us). From 32 rows on operands split beforehand are the faster ones (64 x 2533 x 3026 31 us, turned 41).
 long long any_best_ns(const sofie_gemm_f32_desc &d, bool &turned, int &BN, int &S)
 {
-   const ClusterRoom room = cluster_room();
    int other_BN, other_S;
-   const long long straight = any_ns(d, room, false, BN, S), other = d.M < 32 && d.K >= 512 ? any_ns(d, room, true, other_BN, other_S) : straight;
+   const long long straight = any_ns(d, false, BN, S), other = d.M < 32 && d.K >= 512 ? any_ns(d, true, other_BN, other_S) : straight;
    turned = 10 * other < 8 * straight;
    if (!turned) return straight;
    BN = other_BN, S = other_S;

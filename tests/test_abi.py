@@ -238,3 +238,10 @@ def test_host_copy_past_the_caches(nbytes, dst_at, src_at, threads):
     capi.call("sofie_cuda_selftest_host_copy", dst.ctypes.data + dst_at, src.ctypes.data + src_at, nbytes, 1 << 22, threads, 2)
     assert np.array_equal(dst[dst_at:dst_at + nbytes], src[src_at:src_at + nbytes])
     assert (dst[:dst_at] == 7).all() and (dst[dst_at + nbytes:] == 7).all()
+
+
+def test_the_cut_of_a_product_does_not_depend_on_the_card():
+    """The last bits of a product's sums follow from how it is cut along K: no launcher asks the card it runs on how many clusters it has room for."""
+    for p in sorted((ROOT / "sofie_b200" / "csrc").glob("*.cu*")):
+        for query in ("cudaOccupancyMaxActive", "cudaDeviceGetAttribute", "cudaGetDeviceProperties"):
+            assert query not in p.read_text(), f"{p.name}: {query}"
