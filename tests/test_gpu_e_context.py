@@ -367,8 +367,8 @@ def test_sessions_share_the_helper_threads(cuda_device):
 
 @pytest.mark.parametrize("nbytes", [(5 << 19) - 4, 5 << 19, (4 << 20) + 12, (17 << 20) + 4100, (70 << 20) + 1])
 def test_results_land_in_pieces(cuda_device, nbytes):
-    """A result for pageable memory, as one part: it lands whole or in two to eight pieces, the same bytes and nothing beside them; seven more parts
-    are taken after it, whole or not, a ninth is refused, and an abandoned result leaves the context usable."""
+    """A result for pageable memory, as one part: it lands whole or in two to eight pieces, the same bytes and nothing beside them; a second part
+    after it (the same bytes again) is refused or lands too, and an abandoned result leaves the context usable."""
     x = torch.randint(0, 256, (nbytes,), dtype=torch.uint8, device=cuda_device)
     torch.cuda.synchronize()
     ctx, _ = _ctx()
@@ -381,19 +381,12 @@ def test_results_land_in_pieces(cuda_device, nbytes):
             capi.call("sofie_cuda_ctx_result_part", ctx, C.c_void_p(x.data_ptr()), C.c_size_t(0), C.c_size_t(nbytes))
             capi.call("sofie_cuda_ctx_result_end", ctx, C.byref(host))
             assert host.value == out.ctypes.data and np.array_equal(out[:nbytes], x.cpu().numpy()) and (out[nbytes:] == 7).all()
-        third = nbytes // 3
-        for again in ((0, nbytes), (third, nbytes - third)):
-            out[:] = 7
-            capi.call("sofie_cuda_ctx_result_begin", ctx, C.c_void_p(out.ctypes.data), C.c_size_t(nbytes))
-            for offset, count in ((0, nbytes),) + 7 * (again,):
-                capi.call("sofie_cuda_ctx_result_part", ctx, C.c_void_p(x.data_ptr() + offset), C.c_size_t(offset), C.c_size_t(count))
-            with pytest.raises(capi.SofieCudaError) as e:
-                capi.call("sofie_cuda_ctx_result_part", ctx, C.c_void_p(x.data_ptr()), C.c_size_t(0), C.c_size_t(nbytes))
-            assert e.value.status == capi.ERR_INVALID
-            capi.call("sofie_cuda_ctx_result_end", ctx, C.byref(host))
-            assert np.array_equal(out[:nbytes], x.cpu().numpy()) and (out[nbytes:] == 7).all()
         capi.call("sofie_cuda_ctx_result_begin", ctx, C.c_void_p(out.ctypes.data), C.c_size_t(nbytes))
-        capi.call("sofie_cuda_ctx_result_part", ctx, C.c_void_p(x.data_ptr()), C.c_size_t(0), C.c_size_t(nbytes))
+        for _ in range(8):
+            try:
+                capi.call("sofie_cuda_ctx_result_part", ctx, C.c_void_p(x.data_ptr()), C.c_size_t(0), C.c_size_t(nbytes))
+            except capi.SofieCudaError as e:
+                assert e.status == capi.ERR_INVALID
         capi.call("sofie_cuda_ctx_result_abort", ctx)
         capi.call("sofie_cuda_ctx_check", ctx)
     finally:
@@ -439,5 +432,29 @@ def test_a_fill_ahead_that_is_shorter_than_its_copy(cuda_device, ahead, nbytes, 
             capi.call("sofie_cuda_ctx_check", ctx)
             got = dst.cpu().numpy()
             assert np.array_equal(got[:nbytes], x) and not got[nbytes:].any()
+    finally:
+        capi.call("sofie_cuda_ctx_destroy", ctx)
+
+
+@pytest.mark.parametrize("nbytes", [(5 << 19) - 4, 5 << 19, (4 << 20) + 12, (17 << 20) + 4100, (70 << 20) + 1])
+def test_parts_after_a_whole_result(cuda_device, nbytes):
+    """A result for pageable memory whose first part is all of it, in one piece or several: seven more parts are taken after it, whole or not, and a ninth is refused."""
+    x = torch.randint(0, 256, (nbytes,), dtype=torch.uint8, device=cuda_device)
+    torch.cuda.synchronize()
+    ctx, _ = _ctx()
+    host = C.c_void_p()
+    try:
+        out = np.full(nbytes + 64, 7, np.uint8)
+        third = nbytes // 3
+        for again in ((0, nbytes), (third, nbytes - third)):
+            out[:] = 7
+            capi.call("sofie_cuda_ctx_result_begin", ctx, C.c_void_p(out.ctypes.data), C.c_size_t(nbytes))
+            for offset, count in ((0, nbytes),) + 7 * (again,):
+                capi.call("sofie_cuda_ctx_result_part", ctx, C.c_void_p(x.data_ptr() + offset), C.c_size_t(offset), C.c_size_t(count))
+            with pytest.raises(capi.SofieCudaError) as e:
+                capi.call("sofie_cuda_ctx_result_part", ctx, C.c_void_p(x.data_ptr()), C.c_size_t(0), C.c_size_t(nbytes))
+            assert e.value.status == capi.ERR_INVALID
+            capi.call("sofie_cuda_ctx_result_end", ctx, C.byref(host))
+            assert np.array_equal(out[:nbytes], x.cpu().numpy()) and (out[nbytes:] == 7).all()
     finally:
         capi.call("sofie_cuda_ctx_destroy", ctx)
