@@ -1,4 +1,4 @@
-// fp32 products with at most 8 rows or columns (of more than 32 terms and more FMAs than gemm_f32_tiny_kernel's), any layout.
+// fp32 products with at most 8 rows or columns (from 64 terms on, of more FMAs than gemm_f32_tiny_kernel's), any layout.
 //
 // One operand is long (R rows), the other short (S <= 8). What bounds such a product is the long operand's way out of memory, as long as enough of it is asked for at
 // once; the tile kernels leave most SMs idle or pad S to their tile, and the split-K pair are two launches. Every value of the long operand is one thread's alone here, so it comes
@@ -6,9 +6,11 @@
 //   neighbouring rows are neighbours in memory: a lane owns RT rows, the warps take k in turn, the short operand is read as broadcasts (packed FMAs of two columns)
 //   rows contiguous in k: the lanes take k in turn, a warp owns RT rows, its sums are added up by a butterfly that leaves each lane some of them
 // K is cut over a cluster of up to eight blocks, whose sums meet through distributed shared memory: each block adds up and writes its share of the outputs. Chains are
-// 32 terms long at most where lanes own rows and K / (32 x cluster) where they share them, so that no other kernel but the compensated one for few FMAs is nearer to float64 (0.9 to 1.1 of the kernels' that took these products, 0.6 of one
-// chain's). 140 drawn products: 0.60 of the time in the mean; 2 x 3731 x 2897 31 -> 11.4 us, 6317 x 2 x 3797 (A transposed) 44 -> 23 (its bytes take 15), 5 x 2378 x 2513 30 -> 14.7,
-// 9640 x 7 x 1000 24 -> 17, 3027 x 4 x 108 6.6 -> 3.2. 9 to 16 columns are no faster (1.0 in the mean: the short operand's reads), nor are tiles of the long operand in shared memory.
+// 16 or 32 terms long, a chunk's are added up before they join the sum of the chunks, and the last additions (of the lanes that hold a row's terms, of the blocks) are in 64 bits and rounded once: of 160 drawn products none was
+// further from float64 than on the kernels that took them before (0.70 of their error in the mean, 0.31 with operands of one sign); with all of it in 32 bits some were by a tenth, and the chains of rows contiguous in k
+// grew with K. It costs 2 % of the time in the mean, 15 % at most (6 x 1069 x 820, B stored [N,K]: 5.3 -> 6.1 us).
+// The drawn products take 0.69 of those kernels' time in the mean; 2 x 3731 x 2897 31 -> 10.3 us, 6317 x 2 x 3797 (A transposed) 45 -> 23 (its bytes take 15), 5 x 2378 x 2513 27 -> 12.6 (B stored [N,K] 30 -> 15.0),
+// 9640 x 7 x 1000 24 -> 17.4, 3027 x 4 x 108 6.3 -> 3.2. 9 to 16 columns are no faster (1.0 in the mean: the short operand's reads), nor are tiles of the long operand in shared memory.
 #include "contract.cuh"
 
 namespace sofie {
@@ -28,7 +30,7 @@ struct SkinnyArgs {
 
 // Rows r0 .. r0 + rows of the result out of the blocks' sums [row][SP + 1], threads along what is contiguous in Y.
 template <int SP>
-__device__ __forceinline__ void skinny_output(const SkinnyArgs &g, const float *sums, int r0, int rows, uint32_t rank, uint32_t ranks)
+__device__ __forceinline__ void skinny_output(const SkinnyArgs &g, const double *sums, int r0, int rows, uint32_t rank, uint32_t ranks)
 {
    if (ranks > 1) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
    else __syncthreads();
@@ -36,23 +38,24 @@ __device__ __forceinline__ void skinny_output(const SkinnyArgs &g, const float *
    for (int i = threadIdx.x + (int)rank * kSkThreads; i < total; i += (int)ranks * kSkThreads) {
       const bool along_s = g.y_s == 1;
       const int r = along_s ? i / g.S : i % rows, s = along_s ? i - r * g.S : i / rows;
-      const float *at = sums + r * (SP + 1) + s;
-      float part[8]; // of the blocks that share K, added up in pairs
+      const double *at = sums + r * (SP + 1) + s;
+      double sum = 0.0; // over the blocks that share K
       const uint32_t local = (uint32_t)__cvta_generic_to_shared(at);
 #pragma unroll
       for (uint32_t c = 0; c < 8; c++) {
          uint32_t remote;
-         part[c] = 0.f;
+         double part = 0.0;
          if (c < ranks) {
             asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(c));
-            asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(part[c]) : "r"(remote) : "memory");
+            asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(part) : "r"(remote) : "memory");
          }
+         sum += part;
       }
-      const float sum = ((part[0] + part[1]) + (part[2] + part[3])) + ((part[4] + part[5]) + (part[6] + part[7]));
       const long long y = (r0 + r) * g.y_r + s * g.y_s;
-      float out = g.alpha * sum;
-      if (g.bias_kind == 1) out += g.beta * g.C[g.bias_long ? r0 + r : s];
-      else if (g.bias_kind == 2) out += g.beta * g.C[y];
+      double full = g.alpha * sum;
+      if (g.bias_kind == 1) full += (double)g.beta * g.C[g.bias_long ? r0 + r : s];
+      else if (g.bias_kind == 2) full += (double)g.beta * g.C[y];
+      const float out = (float)full;
       g.Y[y] = g.relu ? relu_ref(out) : out;
    }
    if (ranks > 1) asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory"); // no block ends while its sums are read
@@ -91,7 +94,7 @@ __global__ void __launch_bounds__(kSkThreads, 2) gemm_f32_skinny_lanes_kernel(Sk
 {
    constexpr int U = kSkLoads / RT, ROWS = 32 * RT, CHAINS = 16 / SP; // k under way; sums of every CHAINS-th of them
    __shared__ __align__(16) float q[kSkChunk * SP > kSkWarps / 2 * RT * SP * 32 ? kSkChunk * SP : kSkWarps / 2 * RT * SP * 32]; // later: half of the warps' sums
-   __shared__ float sums[ROWS * (SP + 1)];
+   __shared__ double sums[ROWS * (SP + 1)];
    griddep_launch_dependents();
    griddep_wait(); // the operands may be the previous kernel's output
    uint32_t rank, ranks;
@@ -193,7 +196,7 @@ __global__ void __launch_bounds__(kSkThreads, 2) gemm_f32_skinny_rows_kernel(Ski
 {
    constexpr int U = kSkLoads / RT / W, STEP = 32 * W, STRIDE = U * STEP, CHUNK = kSkChunk, PITCH = CHUNK + 4, N = RT * SP, ROWS = kSkWarps * RT;
    __shared__ __align__(16) float q[SP * PITCH]; // [s][k]
-   __shared__ float sums[ROWS * (SP + 1)];
+   __shared__ double sums[ROWS * (SP + 1)];
    griddep_launch_dependents();
    griddep_wait();
    uint32_t rank, ranks;
@@ -222,9 +225,9 @@ __global__ void __launch_bounds__(kSkThreads, 2) gemm_f32_skinny_rows_kernel(Ski
          }
       }
    };
-   float acc[N];
+   float chain[N], sum[N]; // of this chunk's terms; of the chunks before it
 #pragma unroll
-   for (int j = 0; j < N; j++) acc[j] = 0.f;
+   for (int j = 0; j < N; j++) chain[j] = sum[j] = 0.f;
    float v[2][U][RT][W];
    static_assert(CHUNK % (2 * STRIDE) == 0, "two steps at a time");
    load(v[0], k_begin);
@@ -249,7 +252,7 @@ __global__ void __launch_bounds__(kSkThreads, 2) gemm_f32_skinny_rows_kernel(Ski
 #pragma unroll
                for (int i = 0; i < RT; i++)
 #pragma unroll
-                  for (int e = 0; e < W; e++) acc[i * SP + s] = fmaf(now[u][i][e], w[e], acc[i * SP + s]);
+                  for (int e = 0; e < W; e++) chain[i * SP + s] = fmaf(now[u][i][e], w[e], chain[i * SP + s]);
             }
          }
       };
@@ -258,30 +261,39 @@ __global__ void __launch_bounds__(kSkThreads, 2) gemm_f32_skinny_rows_kernel(Ski
          step(v[0], v[1], k0);
          step(v[1], v[0], k0 + STRIDE); // zeros behind k_end
       }
-   }
-   // a butterfly over the lanes: while a lane has several sums it sends half of them and keeps the other half
-   int kept = N, at = 0;
 #pragma unroll
-   for (int o = 16; o > 0; o >>= 1) {
+      for (int j = 0; j < N; j++) {
+         sum[j] += chain[j];
+         chain[j] = 0.f;
+      }
+   }
+   // a butterfly over the lanes: while a lane has several sums it sends half of them and keeps the other half; the last three steps, where a rounding counts most, in 64 bits
+   int kept = N, at = 0;
+   auto halve = [&](auto *v, int o) {
       const bool up = lane & o;
       if (kept > 1) {
          kept >>= 1;
 #pragma unroll
          for (int j = 0; j < N / 2; j++)
             if (j < kept) {
-               const float send = up ? acc[j] : acc[j + kept], keep = up ? acc[j + kept] : acc[j];
-               acc[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+               const auto send = up ? v[j] : v[j + kept], keep = up ? v[j + kept] : v[j];
+               v[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
             }
          at += up ? kept : 0;
       } else {
-         acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);
+         v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
       }
-   }
+   };
+   halve(sum, 16);
+   halve(sum, 8);
+   double acc[N / 4];
 #pragma unroll
-   for (int j = 0; j < (N > 32 ? N / 32 : 1); j++) {
-      const int e = at + j;
-      sums[(first + e / SP) * (SP + 1) + e % SP] = acc[j];
-   }
+   for (int j = 0; j < N / 4; j++) acc[j] = sum[j];
+   static_assert(N == 16 || N == 32, "four sums a lane after the first steps, or eight");
+   halve(acc, 4);
+   halve(acc, 2);
+   halve(acc, 1);
+   sums[(first + at / SP) * (SP + 1) + at % SP] = acc[0];
    skinny_output<SP>(g, sums, r0, min(ROWS, g.R - r0), rank, ranks);
 }
 
@@ -325,8 +337,16 @@ int launch_skinny(cudaStream_t s, SkinnyArgs &g, bool k_contiguous)
 
 bool gemm_f32_skinny_ok(const sofie_gemm_f32_desc &d)
 {
-   // from 64 terms on: below, the adding up of the partial sums is most of the error (9750 x 1 x 35 5.5e-8 from float64 against 4.0e-8)
-   return (d.M <= 8 || d.N <= 8) && d.K >= 64;
+   // from 64 terms on: below, the adding up of the partial sums is most of the error (9750 x 1 x 35 5.5e-8 from float64 against 4.0e-8). Up to 2^20: a sum is of K / 4096 chunks' sums then,
+   // and no more have been compared with the other kernels' (at 262144 terms 0.5 to 0.6 of their error)
+   if ((d.M > 8 && d.N > 8) || d.K < 64 || d.K > 1 << 20) return false;
+   // K is shared by eight blocks at most, which leaves most SMs idle where the long side is not long: split-K, whose slabs are 64, keeps what it is faster at. 8 x 8 x 65536 15.6 us there, 46 here, 1 x 4 x 16385
+   // 6.5 and 12, 100 x 8 x 32768 20.5 and 25.7, but 250 x 8 x 32768 32.6 and 27.8, 100 x 8 x 8192 12.1 and 8.8; rows read value by value turn earlier: 8 x 8 x 8193 8.6 and 10.9, 32 x 8 x 3001
+   // 5.3 and 5.7, 250 x 8 x 16385 (B stored [N,K]) 16.2 and 16.7.
+   if (!splitk_shape_ok(d)) return true;
+   const bool long_a = d.M >= d.N, k_contiguous = long_a ? !d.transA : d.transB, by_value = k_contiguous && d.K % 4 != 0;
+   const int longer = long_a ? d.M : d.N;
+   return d.K <= (by_value && longer <= 64 ? 2560 : 8192) || longer > (by_value ? 256 : 160);
 }
 
 int launch_gemm_f32_skinny(cudaStream_t s, const sofie_gemm_f32_desc &d, const float *A, const float *B, const float *C, float *Y)

@@ -148,6 +148,37 @@ def test_gemm_f32_skinny(M, N, K, tA, tB, bias_kind):
     assert (np.abs(y[:M - 1] - ref) <= (K / 8 + 24) * 2.0 ** -24 * size).all()
 
 
+# long and ordinary K, where lanes share a row's terms (one by one, in words, and in rows of whole words whose base is four bytes off) and where they own rows
+@pytest.mark.parametrize("M,N,K,tA,tB,shift", [(1000, 1, 65537, 0, 0, 0), (3, 300, 65536, 0, 1, 0), (300, 4, 20000, 0, 0, 1), (2222, 7, 1876, 0, 0, 0), (1, 1000, 65536, 0, 0, 0), (700, 5, 1300, 1, 1, 1), (8, 1999, 1000, 1, 1, 1),
+                                               (64, 8, 4096, 0, 0, 0), (8, 8, 65537, 0, 0, 0), (256, 3, 16385, 0, 1, 0)])   # the last two are split-K's
+def test_gemm_f32_skinny_precision(M, N, K, tA, tB, shift):
+    ops.set_engine(0)
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    rows = (not tA) if M >= N else tB
+    split_k = K > 8192 and max(M, N) <= 256
+    if split_k:      # of at most 64 slabs, 32 lanes each: a lane's chain, the lanes, the slabs
+        roundings = K / 64 / 32 / 2 + 1 + 5 + 64 / 2 + 1
+    elif rows:       # a chain of 16 terms a chunk, the chunks of a block's K (all of it, a half, ... an eighth), two steps of 32-bit additions, the last rounding
+        roundings = 16 / 2 + K / 8 / 512 / 2 * (8 if max(M, N) > 4000 else 4 if max(M, N) > 2000 else 2) + 2 + 1
+    else:            # a chain of up to 32, two pairs of chains, the chunks, the warps, the last rounding
+        roundings = 32 / 2 + 2 + K / 8 / 512 / 2 * (8 if max(M, N) > 4000 else 4 if max(M, N) > 2000 else 2) + 3 + 1
+    for sign in (False, True):
+        ab = []
+        for shape in ((K, M) if tA else (M, K), (N, K) if tB else (K, N)):
+            x = torch.empty(shape[0] * shape[1] + shift, device="cuda").normal_(generator=g)
+            ab.append((x.abs() if sign else x)[shift:].view(shape))
+        y = ops.gemm_f32(*ab, transA=tA, transB=tB).double()
+        assert ops.last_engine() == capi.ENGINE_SIMT
+        a, b = (ab[0].t() if tA else ab[0]).double(), (ab[1].t() if tB else ab[1]).double()
+        exact = a @ b
+        error = float((y - exact).norm())
+        if sign:     # the sums of the last steps are nearly all there is: the result's rounding, two steps of additions (three of lanes that own rows), of slabs as many as there are
+            assert error <= 2.0 ** -24 * (roundings if split_k else 3) ** 0.5 * float(exact.norm())
+        else:        # independent roundings of at most 2^-24 of a partial sum, evenly spread
+            size = float(((a * a) @ (b * b)).sum().sqrt())
+            assert error <= 2.0 ** -24 / 3 ** 0.5 * roundings ** 0.5 * size
+
+
 # images of whole 16-byte words, whose layout changes word by word, and others: channels that divide a word, that do not, and all 64; runs of pixels that end early; and back
 @pytest.mark.parametrize("N,C,H,W", [(3, 16, 8, 8), (2, 3, 10, 14), (2, 24, 16, 42), (1, 64, 6, 6), (5, 7, 2, 2), (2, 2, 64, 67), (2, 5, 9, 11), (1, 63, 37, 4)])
 def test_layout_words(N, C, H, W):
