@@ -128,6 +128,12 @@ def test_gemm_f32_few_terms(M, N, K, tA, tB, bias_kind, relu):
         assert got is None or (np.abs(got.cpu().numpy() - ref) <= (K + 3) * 2.0 ** -24 * size).all()   # a chain of K FMAs, then alpha, beta and the sum
 
 
+# few columns of many rows take a tile no wider than they need, the sums are the same: up to 32, 64 and more columns, a step behind each
+@pytest.mark.parametrize("M,N,K,tA", [(11732, 19, 14, 1), (9600, 32, 5, 0), (9600, 33, 5, 1), (9500, 64, 32, 0), (9500, 65, 3, 1)])
+def test_gemm_f32_few_terms_of_few_columns(M, N, K, tA):
+    test_gemm_f32_few_terms(M, N, K, tA, 0, 2, 1)
+
+
 # products of at most eight rows or columns: the long operand's rows or its K contiguous, whole 16-byte words and not, one block to a K and clusters of two to eight, last slices
 # shorter than the others, several chunks of the short operand, one to eight of its rows; infinities stay in their rows and columns
 @pytest.mark.parametrize("M,N,K,tA,tB", [(6317, 2, 3797, 1, 0), (2, 3731, 2897, 0, 0), (5, 2378, 516, 0, 1), (4099, 8, 1001, 0, 1), (1, 1001, 4100, 0, 0), (300, 3, 1024, 0, 0), (8, 8, 4097, 1, 1),
