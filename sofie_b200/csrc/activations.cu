@@ -49,7 +49,7 @@ template <int OP>
 __global__ void __launch_bounds__(kActThreads) unary_f32_kernel(float alpha, const float *__restrict__ X, float *__restrict__ Y, size_t n, bool vec)
 {
    griddep_launch_dependents();
-   griddep_wait(); // X is the previous kernel's output
+   griddep_wait(X); // X is the previous kernel's output
    const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nthreads = (size_t)gridDim.x * blockDim.x;
    const size_t n4 = vec ? n / 4 : 0;
    // four loads under way before the first value is worked on: with two, functions of twenty instructions a value kept too few (sigmoid of 134 MB 59.4 -> 47.0 us, part
@@ -96,7 +96,7 @@ __global__ void binary_same_f32_kernel(int op, const float *__restrict__ A, cons
                                        int vec)
 {
    griddep_launch_dependents();
-   griddep_wait();
+   griddep_wait(A, B);
    const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nthreads = (size_t)gridDim.x * blockDim.x;
    const size_t n4 = vec == 4 ? n / 4 : 0, n8 = vec == 8 ? n / 8 : 0;
 #pragma unroll 2
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kActThreads) binary_bcast_f32_kernel(BcastDims
                                                                       uint32_t n, bool vec)
 {
    griddep_launch_dependents();
-   griddep_wait();
+   griddep_wait(A, B);
    const uint32_t nthreads = gridDim.x * blockDim.x;
    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += nthreads * 4) {
       uint32_t c[4], rem = i, ao = 0, bo = 0;
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kActThreads) binary_bcast_f32_kernel(BcastDims
 __global__ void binary_bcast_large_f32_kernel(sofie_binary_desc d, const float *__restrict__ A, const float *__restrict__ B, float *__restrict__ Y, size_t n)
 {
    griddep_launch_dependents();
-   griddep_wait();
+   griddep_wait(A, B);
    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
       size_t rem = i, ao = 0, bo = 0;
 #pragma unroll
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kActThreads) batchnorm_f32_kernel(FastDiv inne
                                                                    const float *__restrict__ bias, const float *__restrict__ mean, float *__restrict__ Y, uint32_t n, int relu, bool vec)
 {
    griddep_launch_dependents();
-   griddep_wait();
+   griddep_wait(X, scale, bias, mean);
    const uint32_t nthreads = gridDim.x * blockDim.x;
    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += nthreads * 4) {
       uint32_t in, c;
@@ -259,7 +259,7 @@ __global__ void batchnorm_large_f32_kernel(sofie_batchnorm_desc d, const float *
                                            const float *__restrict__ bias, const float *__restrict__ mean, float *__restrict__ Y, size_t n)
 {
    griddep_launch_dependents();
-   griddep_wait();
+   griddep_wait(X, scale, bias, mean);
    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
       const int c = d.layout == SOFIE_LAYOUT_NHWC ? (int)(i % (size_t)d.C) : (int)((i / (size_t)d.HW) % (size_t)d.C);
       Y[i] = batchnorm_apply(X[i], mean[c], scale[c], bias[c], d.relu);

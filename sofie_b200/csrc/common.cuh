@@ -66,8 +66,17 @@ constexpr int kNumSMs = 148; // B200
 // constant data (weights, biases, descriptors) is touched before it. Both instructions are no-ops in
 // a kernel that was launched the ordinary way. SOFIE_CUDA_PDL=0 turns the attribute off.
 __device__ __forceinline__ void griddep_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// A read of what an earlier kernel wrote, behind griddep_wait(): a load the compiler takes for one of constant data (__ldg, or through a restrict pointer) may move before it.
+// `dependent`: the kernel's restrict pointers to what it reads behind the wait. What such a pointer leads to no statement of the kernel can write, so the compiler may take a load through it before the
+// wait (and one of __ldg through any pointer); behind an empty statement that might have changed the pointer itself it may not.
+template <typename P>
+__device__ __forceinline__ void may_have_changed(P &pointer) { asm volatile("" : "+l"(pointer)); }
+template <typename... P>
+__device__ __forceinline__ void griddep_wait(P &...dependent)
+{
+   asm volatile("griddepcontrol.wait;" ::: "memory");
+   (may_have_changed(dependent), ...);
+}
+// A read of what an earlier kernel wrote that stays where it is written.
 __device__ __forceinline__ float load_dependent(const float *p)
 {
    float v;

@@ -35,7 +35,7 @@ conv3x3_direct_f32_kernel(ConvGeom g, const float *__restrict__ X, const float *
    float *s_w = smem + 2 * dc_tile_floats(GROUPS);        // [channel][tap][16]
    __shared__ float s_bias[kDcOut];
    griddep_launch_dependents();
-   griddep_wait();
+   griddep_wait(X, Wt, bias);
    const int tid = threadIdx.x, oc_base = blockIdx.y * kDcOut;
    for (int i = tid; i < chunks * kDcChunk * 9 * kDcOut; i += THREADS) {
       const int o = i % kDcOut, rt = i / kDcOut % 9, c = i / (9 * kDcOut);
@@ -217,7 +217,7 @@ conv3x3_split_f32_kernel(ConvGeom g, const float *__restrict__ X, const float *_
    float *partial = smem;              // [sharer][output channel][row][column], where the inputs and weights were
    __shared__ float s_bias[kDcOut];
    griddep_launch_dependents();
-   griddep_wait();
+   griddep_wait(X, Wt, bias);
    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, oc_base = blockIdx.y * kDcOut, outs = min(kDcOut, g.Cout - oc_base);
    if (tid < kDcOut) s_bias[tid] = tid < outs && bias ? __ldg(bias + oc_base + tid) : 0.f;
    uint32_t tx, ty;

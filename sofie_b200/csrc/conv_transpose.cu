@@ -218,7 +218,7 @@ conv_transpose_sum_kernel(SumGeom g, FastDiv bands, FastDiv columns, FastDiv tap
    extern __shared__ __align__(16) double staged[];
    const sofie_conv_transpose2d_desc &d = g.d;
    griddep_launch_dependents();
-   griddep_wait();
+   griddep_wait(X, Wt, bias);
    const int oc0 = blockIdx.y * OC, outs = min(OC, d.Cout - oc0);
    // [channel][tap][OC], [channel][row][column]; of every filter row (column) the phase that it is a tap of and how far below the output's step its input lies
    double *filters = staged, *inputs = staged + d.C * (int)taps.d * OC;

@@ -28,7 +28,7 @@ inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 
 __global__ void relu_f32_vec4(const float4 *__restrict__ X, float4 *__restrict__ Y, size_t n4)
 {
    griddep_launch_dependents();
-   griddep_wait(); // X is the previous kernel's output
+   griddep_wait(X); // X is the previous kernel's output
    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n4; i += (size_t)gridDim.x * blockDim.x) {
       float4 v = X[i];
       v.x = relu_ref(v.x);
@@ -41,7 +41,7 @@ __global__ void relu_f32_vec4(const float4 *__restrict__ X, float4 *__restrict__
 __global__ void relu_f32_scalar(const float *__restrict__ X, float *__restrict__ Y, size_t begin, size_t n)
 {
    griddep_launch_dependents();
-   griddep_wait(); // X is the previous kernel's output
+   griddep_wait(X); // X is the previous kernel's output
    for (size_t i = begin + blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
       Y[i] = relu_ref(X[i]);
 }
@@ -87,7 +87,7 @@ __global__ void pool2d_f32_kernel(sofie_pool2d_desc d, PoolCoords pc, bool small
                                   float *__restrict__ Y)
 {
    griddep_launch_dependents();
-   griddep_wait();
+   griddep_wait(X);
    const size_t total = (size_t)d.N * d.C * oH * oW;
    const bool do_pad = d.pads[0] || d.pads[1] || d.pads[2] || d.pads[3];
    const size_t step_h = NHWC ? (size_t)d.W * d.C : (size_t)d.W, step_w = NHWC ? (size_t)d.C : 1;
@@ -170,7 +170,7 @@ __global__ void pool2x2_f32_any_kernel(const float *__restrict__ X, float *__res
 {
    constexpr int U = 4;
    griddep_launch_dependents();
-   griddep_wait(); // X is the previous kernel's output
+   griddep_wait(X); // X is the previous kernel's output
    const unsigned nthreads = gridDim.x * blockDim.x;
    for (unsigned long long i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (unsigned long long)U * nthreads) {
       float v[U][4];
@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(kThreads) layout_few_channels_kernel(const T *
 {
    __shared__ T tile[kLayoutTile + 64];
    griddep_launch_dependents();
-   griddep_wait();
+   griddep_wait(in);
    const size_t image = blockIdx.y + (size_t)gridDim.y * blockIdx.z;
    const int run = 1 << log_run, p0 = blockIdx.x << log_run, n = min(run, P - p0), pitch = run + 1, flat = n * C, planes = C << log_run;
    const T *src = in + image * (size_t)P * C;
@@ -551,13 +551,13 @@ __global__ void __launch_bounds__(kThreads) layout_few_channels_kernel(const T *
    }
 }
 // The same for floats in images of whole 16-byte words (P a multiple of 4): words on both sides, the tile's rows words apart. What bounds the form above is the number of loads and
-// stores: 512 images of 16 x 64 x 64 58 -> 42 us (its bytes take 41), 1533 of 24 x 16 x 42 56 -> 40 (30).
+// stores: 512 images of 16 x 64 x 64 58 -> 42 us (its bytes take 41), 1533 of 24 x 16 x 42 56 -> 32 (30; 41 with words that passed through registers one by one), back 39 -> 31.
 template <bool TO_NHWC>
 __global__ void __launch_bounds__(kThreads) layout_few_channels_words_kernel(const float *__restrict__ in, float *__restrict__ out, int P, int C, int log_run, FastDiv channels)
 {
    __shared__ __align__(16) float tile[kLayoutTile + 4 * 64];
    griddep_launch_dependents();
-   griddep_wait();
+   griddep_wait(in);
    const size_t image = blockIdx.y + (size_t)gridDim.y * blockIdx.z;
    const int run = 1 << log_run, p0 = blockIdx.x << log_run, n = min(run, P - p0), pitch = run + 4, flat = n * C / 4, planes = C << (log_run - 2);
    const float *src = in + image * (size_t)P * C;
@@ -576,8 +576,9 @@ __global__ void __launch_bounds__(kThreads) layout_few_channels_words_kernel(con
 #pragma unroll 4
       for (int i = threadIdx.x; i < planes; i += kThreads) {
          const int c = i >> (log_run - 2), p = (i & (run / 4 - 1)) * 4;
-         if (p < n) *reinterpret_cast<float4 *>(tile + c * pitch + p) = *reinterpret_cast<const float4 *>(src + (size_t)c * P + p0 + p);
+         if (p < n) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(tile + c * pitch + p)), "l"(src + (size_t)c * P + p0 + p));
       }
+      asm volatile("cp.async.wait_all;" ::: "memory");
       __syncthreads();
       float4 *y = reinterpret_cast<float4 *>(dst + (size_t)p0 * C);
 #pragma unroll 4
@@ -588,15 +589,21 @@ __global__ void __launch_bounds__(kThreads) layout_few_channels_words_kernel(con
       }
    } else {
       const float4 *x = reinterpret_cast<const float4 *>(src + (size_t)p0 * C);
-#pragma unroll 4
-      for (int i = threadIdx.x; i < flat; i += kThreads) {
-         int at[4];
-         places(i, at);
-         const float4 v = x[i];
-         tile[at[0]] = v.x;
-         tile[at[1]] = v.y;
-         tile[at[2]] = v.z;
-         tile[at[3]] = v.w;
+      for (int i0 = threadIdx.x; i0 < flat; i0 += 4 * kThreads) {
+         float4 v[4];
+#pragma unroll
+         for (int k = 0; k < 4; k++)
+            if (i0 + k * kThreads < flat) v[k] = x[i0 + k * kThreads];
+#pragma unroll
+         for (int k = 0; k < 4; k++)
+            if (i0 + k * kThreads < flat) {
+               int at[4];
+               places(i0 + k * kThreads, at);
+               tile[at[0]] = v[k].x;
+               tile[at[1]] = v[k].y;
+               tile[at[2]] = v[k].z;
+               tile[at[3]] = v[k].w;
+            }
       }
       __syncthreads();
 #pragma unroll 4
@@ -671,7 +678,7 @@ __device__ __forceinline__ uint8_t quant_u8(float x, float scale, float inv_scal
 __global__ void quantize_u8_vec8_kernel(const float *__restrict__ X, uint8_t *__restrict__ Y, size_t n8, float scale, float inv_scale, int zp)
 {
    griddep_launch_dependents();
-   griddep_wait(); // X is the previous kernel's output
+   griddep_wait(X); // X is the previous kernel's output
    const size_t nthreads = (size_t)gridDim.x * blockDim.x;
 #pragma unroll 2
    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n8; i += nthreads) {
@@ -689,7 +696,7 @@ __global__ void quantize_u8_kernel(const float *__restrict__ X, uint8_t *__restr
                                    bool vec)
 {
    griddep_launch_dependents();
-   griddep_wait(); // X is the previous kernel's output
+   griddep_wait(X); // X is the previous kernel's output
    const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nthreads = (size_t)gridDim.x * blockDim.x;
    size_t n4 = vec ? n / 4 : 0;
    // several independent 16-byte loads in flight per thread
@@ -708,16 +715,22 @@ __global__ void dequantize_u8_kernel(const uint8_t *__restrict__ X, float *__res
                                      int zp, bool vec)
 {
    griddep_launch_dependents();
-   griddep_wait(); // X is the previous kernel's output
+   griddep_wait(X); // X is the previous kernel's output
    const size_t tid = blockIdx.x * (size_t)blockDim.x + threadIdx.x, nthreads = (size_t)gridDim.x * blockDim.x;
    size_t n4 = vec ? n / 4 : 0;
-#pragma unroll 4
-   for (size_t i = tid; i < n4; i += nthreads) {
-      uchar4 q = reinterpret_cast<const uchar4 *>(X)[i];
-      float4 v = make_float4(__fmul_rn((float)((int)q.x - zp), scale), __fmul_rn((float)((int)q.y - zp), scale),
-                             __fmul_rn((float)((int)q.z - zp), scale), __fmul_rn((float)((int)q.w - zp), scale));
-      reinterpret_cast<float4 *>(Y)[i] = v;
+   auto value = [&](uchar4 q) {
+      return make_float4(__fmul_rn((float)((int)q.x - zp), scale), __fmul_rn((float)((int)q.y - zp), scale),
+                         __fmul_rn((float)((int)q.z - zp), scale), __fmul_rn((float)((int)q.w - zp), scale));
+   };
+   size_t i4 = tid;
+   for (; i4 + 3 * nthreads < n4; i4 += 4 * nthreads) { // four loads under way before the first store
+      uchar4 q[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) q[k] = reinterpret_cast<const uchar4 *>(X)[i4 + k * nthreads];
+#pragma unroll
+      for (int k = 0; k < 4; k++) reinterpret_cast<float4 *>(Y)[i4 + k * nthreads] = value(q[k]);
    }
+   for (; i4 < n4; i4 += nthreads) reinterpret_cast<float4 *>(Y)[i4] = value(reinterpret_cast<const uchar4 *>(X)[i4]);
    for (size_t i = n4 * 4 + tid; i < n; i += nthreads) Y[i] = __fmul_rn((float)((int)X[i] - zp), scale);
 }
 
@@ -730,7 +743,7 @@ __device__ __forceinline__ uint8_t to_e4m3(float x)
 __global__ void dequantize_e4m3_kernel(const uint8_t *__restrict__ X, float *__restrict__ Y, size_t n, float scale)
 {
    griddep_launch_dependents();
-   griddep_wait(); // X is the previous kernel's output
+   griddep_wait(X); // X is the previous kernel's output
    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
       Y[i] = __fmul_rn(__half2float(__half(__nv_cvt_fp8_to_halfraw(X[i], __NV_E4M3))), scale);
 }
@@ -765,7 +778,7 @@ __global__ void quantize_e4m3_vec8_kernel(const In *__restrict__ X, uint8_t *__r
                                           const float *__restrict__ scale_dev)
 {
    griddep_launch_dependents();
-   griddep_wait(); // X (and a scale on the device) come from the previous kernels
+   griddep_wait(X, scale_dev); // X (and a scale on the device) come from the previous kernels
    const float scale = scale_dev ? *scale_dev : scale_in;
    const float inv = __fdiv_rn(1.f, scale);
    const size_t nthreads = (size_t)gridDim.x * blockDim.x;

@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(T > 128 ? T : 128)
 gemm_f32_tiny_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, const float *__restrict__ B, const float *C, float *Y)
 {
    griddep_launch_dependents();
-   griddep_wait(); // the operands may be the previous kernel's output
+   griddep_wait(A, B); // the operands may be the previous kernel's output
    const int i = (blockIdx.x * (T > 128 ? T : 128) + threadIdx.x) / T, t = threadIdx.x % T;
    const bool live = i < d.M * d.N;
    const int m = live ? i / d.N : 0, n = live ? i - m * d.N : 0;

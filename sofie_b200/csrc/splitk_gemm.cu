@@ -29,7 +29,7 @@ gemm_f32_splitk_partial_kernel(int M, int N, int K, int slab, const float *__res
    __shared__ __align__(16) float bs[kSplitKMaxN * kSplitKChunk];
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    griddep_launch_dependents();
-   griddep_wait(); // A (and possibly B) are the previous kernel's output; nothing worth doing before it
+   griddep_wait(A, B); // A (and possibly B) are the previous kernel's output; nothing worth doing before it
    const int m = blockIdx.x * kSplitKWarps + warp;
    const int s = blockIdx.y;
    const int k0 = s * slab, k1 = min(K, k0 + slab);
@@ -89,7 +89,7 @@ __global__ void gemm_f32_splitk_reduce_kernel(sofie_gemm_f32_desc d, int splits,
 {
    const size_t total = (size_t)d.M * d.N;
    griddep_launch_dependents();
-   griddep_wait(); // the partial sums of the kernel before
+   griddep_wait(partial, C); // the partial sums of the kernel before
    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
       float sum = 0.f;
       for (int s = 0; s < splits; s++) sum += partial[(size_t)s * total + i];
@@ -120,7 +120,7 @@ gemm_f32_rowblock_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, con
    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
    const int m0 = blockIdx.x * ROWS, K = d.K;
    griddep_launch_dependents();
-   griddep_wait(); // A is the previous kernel's output
+   griddep_wait(A, B, C); // A is the previous kernel's output
    float acc[ROWS][NN];
 #pragma unroll
    for (int r = 0; r < ROWS; r++)
@@ -186,7 +186,7 @@ gemm_f32_rows_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, const f
    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); // known to be the same in all lanes
    const int m0 = (blockIdx.x * 8 + warp) * ROWS, K = d.K;
    griddep_launch_dependents();
-   griddep_wait(); // A is the previous kernel's output
+   griddep_wait(A, B, C); // A is the previous kernel's output
    auto copy_b = [&](int k0, int buf) {
       for (int i = threadIdx.x; i < NN * (kRowsChunk / 4); i += 256) {
          const int n = i / (kRowsChunk / 4), k = k0 + 4 * (i % (kRowsChunk / 4));

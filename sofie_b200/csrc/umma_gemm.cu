@@ -245,7 +245,7 @@ __device__ __forceinline__ void store_row_chunk(const GemmEpilogue &ep, const ui
       // longer than its MMAs at K = 1024 and slowed them at K = 4096. 65536 x 4096 x 4096 1083 -> 836 us (2031 -> 2632 TFLOP/s),
       // 262144 x 1024 x 1024 988 -> 304 us; back to back the first one runs into the power limit (1198 -> 948 us).
       uint32_t hb[16], qb[8];
-      const float scale = ep.a_scale_dev ? __fmul_rn(__ldg(ep.a_scale_dev), ep.w_scale) : ep.scale;
+      const float scale = ep.a_scale_dev ? __fmul_rn(load_dependent(ep.a_scale_dev), ep.w_scale) : ep.scale;
       const uint64_t inv2 = pack_f32x2(ep.q_inv, ep.q_inv);
       const float off_zero = ep.relu ? copysignf(1e-30f, ep.q_inv) : -0.f;
       const uint64_t off2 = pack_f32x2(off_zero, off_zero);

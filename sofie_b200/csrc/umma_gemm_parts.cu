@@ -115,7 +115,7 @@ split_parts_kernel(AnyOperand A, AnyOperand B, PartsLayout pa, PartsLayout pb, i
 {
    __shared__ float buf[kSplitThreads / 32 * 16 * 33];
    griddep_launch_dependents();
-   griddep_wait(); // the operands may be the previous kernel's output, the workspace may still be read by it
+   griddep_wait(A.p, B.p); // the operands may be the previous kernel's output, the workspace may still be read by it
    const int g = blockIdx.x, kb0 = blockIdx.y * kSplitStages;
    if (g < groups_a) split_block(A, pa, K, nkb, g * kSplitRows, kb0, buf);
    else split_block(B, pb, K, nkb, (g - groups_a) * kSplitRows, kb0, buf);

@@ -209,7 +209,7 @@ umma_mlp_kernel(MlpTcPlan pl, const float *__restrict__ X, float *__restrict__ Y
          g.vec = x_vec != 0;
          return g;
       };
-      griddep_wait(); // X is the previous kernel's output
+      griddep_wait(X); // X is the previous kernel's output
       float4 xv[XPRE];
       stage_load<NTA, XPRE>(x_geom(blockIdx.x), t, 0, xv);
       for (int slab = blockIdx.x; slab < slabs; slab += gridDim.x) {

@@ -245,3 +245,27 @@ def test_the_cut_of_a_product_does_not_depend_on_the_card():
     for p in sorted((ROOT / "sofie_b200" / "csrc").glob("*.cu*")):
         for query in ("cudaOccupancyMaxActive", "cudaDeviceGetAttribute", "cudaGetDeviceProperties"):
             assert query not in p.read_text(), f"{p.name}: {query}"
+
+
+def test_what_an_earlier_kernel_wrote_is_read_behind_the_wait_for_it():
+    """A load through a restrict pointer of a kernel may move before griddep_wait(), unless the pointer is one of its arguments; so may __ldg of a pointer that the kernel did not wait with."""
+    weights = {"umma_qconv3x3_first_pool_kernel": {"W"}}   # read before the wait, on purpose
+    waiting = 0
+    for p in sorted((ROOT / "sofie_b200" / "csrc").glob("*.cu*")):
+        text = re.sub(r"//[^\n]*", "", p.read_text())
+        for m in re.finditer(r"__global__", text):
+            start = text.index("{", m.end())
+            depth, end = 0, start
+            while end == start or depth:
+                depth += {"{": 1, "}": -1}.get(text[end], 0)
+                end += 1
+            head, body = text[m.end():start], text[start:end]
+            waits = re.findall(r"griddep_wait\(([^)]*)\)", body)
+            if not waits:
+                continue
+            waiting += 1
+            name = re.findall(r"(\w+)\s*\(", re.sub(r"__launch_bounds__\([^)]*\)+", "", head))[0]
+            read = {q for q in re.findall(r"const\s+[\w:]+\s*\*\s*__restrict__\s*(\w+)", head)} - weights.get(name, set())
+            named = {a.strip() for a in ",".join(waits).split(",")}
+            assert read <= named, f"{p.name}: {name} reads {sorted(read - named)} through a restrict pointer behind its wait"
+    assert waiting > 30
