@@ -76,6 +76,25 @@ __device__ __forceinline__ void griddep_wait(P &...dependent)
    asm volatile("griddepcontrol.wait;" ::: "memory");
    (may_have_changed(dependent), ...);
 }
+// A load through such a pointer that may move freely behind the wait, before stores too (what the pointer leads to does not change any more): where a loop's loads are to be under way together.
+__device__ __forceinline__ uint8_t load_settled(const uint8_t *p)
+{
+   uint32_t v;
+   asm("ld.global.u8 %0, [%1];" : "=r"(v) : "l"(p));
+   return (uint8_t)v;
+}
+__device__ __forceinline__ float load_settled(const float *p)
+{
+   float v;
+   asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+   return v;
+}
+__device__ __forceinline__ float4 load_settled(const float4 *p)
+{
+   float4 v;
+   asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+   return v;
+}
 // A read of what an earlier kernel wrote that stays where it is written.
 __device__ __forceinline__ float load_dependent(const float *p)
 {

@@ -39,7 +39,10 @@ conv3x3_direct_f32_kernel(ConvGeom g, const float *__restrict__ X, const float *
    const int tid = threadIdx.x, oc_base = blockIdx.y * kDcOut;
    for (int i = tid; i < chunks * kDcChunk * 9 * kDcOut; i += THREADS) {
       const int o = i % kDcOut, rt = i / kDcOut % 9, c = i / (9 * kDcOut);
-      s_w[i] = c < g.C && oc_base + o < g.Cout ? __ldg(Wt + dc_weight_index(g, oc_base + o, c, rt)) : 0.f;
+      const bool in = c < g.C && oc_base + o < g.Cout;
+      // (waited for with the first tile)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(s_w + i)), "l"(in ? Wt + dc_weight_index(g, oc_base + o, c, rt) : Wt), "r"(in ? 4 : 0)
+                   : "memory");
    }
    if (tid < kDcOut) s_bias[tid] = oc_base + tid < g.Cout && bias ? __ldg(bias + oc_base + tid) : 0.f;
    auto origin = [&](long long id, int &n, int &h0, int &w0) {

@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(kThreads) layout_few_channels_kernel(const T *
    // a float goes into the tile by an asynchronous copy: no registers hold it, all of a thread's are under way (777 images of 3 x 91 x 85 40 -> 28 us)
    auto fetch = [](T *at, const T *from) {
       if constexpr (sizeof(T) == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(at)), "l"(from) : "memory");
-      else *at = *from;
+      else *at = load_settled(from);
    };
    if (TO_NHWC) {
 #pragma unroll 8
