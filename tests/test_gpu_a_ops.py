@@ -247,6 +247,27 @@ def test_gemm_f32_turned(M, N, K, tA, tB, bias_kind):
         assert rel_err(y[:rows], ref) <= FP32_TOL
 
 
+# ... and no further from float64 than the chain of FMAs that the CUDA-core kernel forms for the same product
+@pytest.mark.parametrize("M,N,K,tA,tB", [(30, 1109, 1819, 0, 0), (18, 2378, 2513, 0, 1), (31, 2238, 1277, 1, 0), (17, 2780, 967, 0, 0)])
+def test_gemm_f32_turned_is_as_precise_as_a_chain(M, N, K, tA, tB):
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    for sign in (False, True):
+        A, B = torch.randn((K, M) if tA else (M, K), device="cuda", generator=g), torch.randn((N, K) if tB else (K, N), device="cuda", generator=g)
+        if sign:
+            A, B = A.abs(), B.abs()
+        exact = (A.t() if tA else A).double() @ (B.t() if tB else B).double()
+        error = {}
+        for engine in (1, 0):
+            ops.set_engine(engine)
+            try:
+                y = ops.gemm_f32(A, B, transA=tA, transB=tB, workspace=False)
+                assert ops.last_engine() == (capi.ENGINE_SIMT if engine else capi.ENGINE_TCGEN05)
+            finally:
+                ops.set_engine(0)
+            error[engine] = float((y.double() - exact).norm())
+        assert error[0] <= error[1]
+
+
 # rows that take the kernel with its weights in registers: one and two a block, the first beyond; pieces that end inside a lane's share (K = 20, 36), one lane to thirty-two an
 # output, an infinite input (zeros behind a row's inputs are no products of it), one to three layers
 @pytest.mark.parametrize("M,dims", [(1, (64, 128, 128, 10)), (148, (64, 128, 128, 10)), (149, (20, 36, 7)), (296, (256, 16, 64, 3)), (297, (64, 128, 128, 10)), (3, (256, 1)), (5, (16, 256, 4)),
@@ -355,6 +376,24 @@ def test_conv2d_f32_shared_channels(N, C, H, W, Cout, pool, x_nhwc, y_nhwc, pack
     finite = np.isfinite(ref)
     assert (np.abs(y[finite] - ref[finite]) <= FP32_TOL * np.abs(ref[finite]).max(initial=0)).all()
     assert np.array_equal(y[~finite], ref[~finite], equal_nan=True)
+
+
+# whole 16-byte rows whose base is four bytes off are copied value by value
+@pytest.mark.parametrize("N,C,H,W,Cout,pool", [(1, 8, 16, 16, 16, 0), (40, 24, 8, 20, 33, 2), (600, 33, 12, 16, 7, 0)])
+def test_conv2d_f32_shared_channels_of_unaligned_images(N, C, H, W, Cout, pool):
+    g = torch.Generator(device="cuda").manual_seed(N + C)
+    X, Wt, b = (torch.randn(s, device="cuda", generator=g) for s in ((N, C, H, W), (Cout, C, 3, 3), (Cout,)))
+    shifted = torch.empty(X.numel() + 1, device="cuda")[1:].view(X.shape).copy_(X)
+    capi.call("sofie_cuda_set_engine", 1)
+    try:
+        args = dict(shape=X.shape, pad=(1, 1), pool=pool, kernel=(3, 3))
+        y, of_shifted = ops.conv2d_f32(X, Wt, b, **args), ops.conv2d_f32(shifted, Wt, b, **args)
+    finally:
+        capi.call("sofie_cuda_set_engine", 0)
+    ref = torch.nn.functional.conv2d(X.double(), Wt.double(), b.double(), padding=1)
+    ref = torch.nn.functional.max_pool2d(ref, 2) if pool else ref
+    for out in (y, of_shifted):
+        assert float((out.double().view(ref.shape) - ref).abs().max()) <= FP32_TOL * float(ref.abs().max())
 
 
 @pytest.mark.parametrize("case", CONV_CASES)
