@@ -198,8 +198,8 @@ int launch_direct(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, 
 // inputs and the filters are converted to double once, on their way into shared memory, and a thread sums four channels of PX outputs in double, so that the result is the exact
 // sum rounded once (error against float64 2.5e-8; 3.5e-8 to 1.3e-7 the product form, 4.3e-8 to 5.5e-8 the direct one). A warp's outputs share their phase (row and column
 // modulo the strides) and so their taps; OC / 4 neighbouring lanes share an output's inputs.
-// What bounds it: round trips and instructions at few warps an SM (19 % of the issue slots at 64 images), from some hundred images on the reads out of shared memory
-// (2 clk a 16-byte broadcast, 2 an input: 34 of the 64 DFMA/clk at PX = 4). 32 -> 16 channels, 2 x 2 / 2 on 12 x 12, 1 / 64 / 1024 images: 13.6 -> 5.3, 16.3 -> 10.6, 103 -> 85 us against
+// What bounds it: round trips at sixteen warps an SM, to L2 while a block stages and to shared memory while it sums; no pipe is busy, at 64 images or at 1024 (issue slots 31 and 29 %, fp64
+// 15 and 16 %, shared memory 17 and 23 %). 32 -> 16 channels, 2 x 2 / 2 on 12 x 12, 1 / 64 / 1024 images: 13.6 -> 5.3, 16.3 -> 10.6, 103 -> 85 us against
 // the product form; 16 -> 3, 3 x 3 / 2 on 24 x 24: 12.9 -> 6.4, 21.5 -> 13.9, 184 -> 117. Its channels in registers two or four at a time: the same or slower (96, 127 at 1024).
 constexpr int kSumThreads = 256;
 constexpr int kSumBytes = 96 * 1024; // of shared memory: two blocks an SM

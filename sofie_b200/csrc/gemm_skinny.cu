@@ -299,7 +299,8 @@ __global__ void __launch_bounds__(kSkThreads, 2) gemm_f32_skinny_rows_kernel(Ski
 
 int launch_clustered(cudaStream_t s, void (*kern)(SkinnyArgs), SkinnyArgs &g, int rows, int slice)
 {
-   // as many blocks to a K as leave under 300 of them and slices of `slice` at least
+   // As many blocks to a K as leave under 300 of them (two an SM are resident) and slices of `slice` at least. Of 160 drawn products 27 take another cut with 150, 1.24 of the time in their mean (0.79 to 1.64),
+   // 23 with 600, 1.25 (0.85 to 2.06).
    const int groups = ceil_div(g.R, rows);
    int ranks = 1;
    while (ranks < 8 && (long long)groups * ranks * 2 < 300 && g.K / (ranks * 2) >= slice) ranks *= 2;

@@ -78,7 +78,7 @@ gemm_f32_simt_kernel(sofie_gemm_f32_desc d, const float *__restrict__ A, const f
 // What the kernel above spends on a large output of few terms is instructions: it walks K in steps of 16 between barriers for 64 x 64 outputs, and each staged value and
 // each stored one has its own indexes. Here a block keeps its BN columns of B, all K of them, and walks tiles of BM rows, the next tile's A on its way under this one; a warp's
 // BM / 8 rows read A as broadcasts of four rows and feed packed FMAs (two rows each, in the order of k and rounded as the scalar ones: the same sums), and a lane's columns are
-// 32 apart, so that a warp stores whole lines of any alignment. Bound by issue slots still (16 instructions for 32 outputs of 9 terms; 36 without the walk). Against the kernel
+// 32 apart, so that a warp stores whole lines of any alignment. Bound by issue slots still (20 instructions for 32 outputs of 9 terms, 63 % of the slots). Against the kernel
 // above: 9602 x 3820 x 9 83 -> 38 us (its bytes take 23), 16384 x 4093 x 8 with a full C 169 -> 106 (83), 13028 x 2481 x 14 73 -> 42, 12399 x 459 x 23 28 -> 20, 728 x 2032 x 10 7.7 -> 6.1.
 // Tiles of 128 rows: 41, 119, 45, 19, 6.8.
 constexpr int kFewThreads = 256, kFewK = 32, kFewRows = 64;

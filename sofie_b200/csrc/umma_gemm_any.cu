@@ -521,8 +521,9 @@ int launch_gemm_f32_any(cudaStream_t s, const sofie_gemm_f32_desc &d, bool tma, 
    const long long best = any_best_ns(d, turned, BN, S);
    // What TMA cannot fetch has the CUDA-core kernel beside it: blocks of 64 x 64, steps of 16 K that take 1.9 us alone and 0.45 us (0.65 with
    // B stored [N,K]) apart on an SM full of them, whose outputs leave while other blocks compute. It wins where the output is what
-   // counts: 16384 x 4093 x 8 with a full bias 163 us against 580, 16384 x 777 x 64 81 against 144; 1000 x 777 x 1333 211 against 38. Over
-   // 620 products the choice is 0.9 % above the faster of the two in the mean, and never more than 5 % above the CUDA-core kernel.
+   // counts: 16384 x 777 x 64 81 us against 144; 1000 x 777 x 1333 211 against 38. Over
+   // 620 products the choice is 0.9 % above the faster of the two in the mean, and never more than 5 % above the CUDA-core kernel. Up to 32 terms the CUDA cores' kernel is another and up to 1.9 times as fast
+   // as estimated (16384 x 4093 x 8 with a full bias 106 us, 580 here; 2310 x 3543 x 17 15 and 28): what the estimate leaves on this kernel stays here all the same, where its error is half (0.4 to 0.8) of a chain's.
    if (!tma && forced_engine() != SOFIE_ENGINE_TCGEN05) {
       if (simt_ns(d) < best) return fail(SOFIE_CUDA_ERR_UNSUPPORTED, "faster on the CUDA cores");
    }

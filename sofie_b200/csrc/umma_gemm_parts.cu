@@ -503,7 +503,7 @@ struct PartsPlan {
 // Tile width and clusters along K by the time they take, in ns, fitted to 22700 runs of 2800 products (each at every width and cluster size; the
 // choice is 1.2 % above the best of them in the mean): both launches, the split of (M + N) x K values, a stage of 32 K, a tile's end (longer
 // where rows of Y are not whole 16-byte words and where C is of Y's shape), under which the next tile's stages run, or the exchange within
-// a cluster; at least the writes of Y. Clusters of 4 / 8 found room for 132 / 96 CTAs at a time.
+// a cluster; at least the writes of Y. `room` is what clusters of 1 / 2 / 4 / 8 found at the time of the fit, the same on every card as kClusterRoom is.
 // Against the other kernels' estimate, which is 20 % low in the mean: the split pays from about 2^20 outputs or 2^24 FMAs a tile on. 1000 x 777 x
 // 1333 with A transposed and a full bias 39 -> 25.7 us, 4096 x 4096 x 2048 522 -> 302, 785 x 2853 x 683 64 -> 35, 16384 x 777 x 64 59 -> 32; of the 2800
 // (M and N from 48 on) it takes three in five, and 0.3 % of them are more than 3 % slower. With 32 to 47 rows
