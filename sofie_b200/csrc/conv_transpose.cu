@@ -7,6 +7,9 @@
 // X [N,C,H,W], W [C,Cout,kH,kW] (the ONNX layout), Y [N,Cout,oH,oW], fp32 FMA, taps in (r, s, ic) order.
 #include "common.cuh"
 
+#include <algorithm>
+#include <type_traits>
+
 namespace sofie {
 namespace {
 
@@ -79,31 +82,32 @@ conv_transpose2d_f32_kernel(sofie_conv_transpose2d_desc d, int oH, int oW, size_
 // At stride one with one input channel (or two and one tap) there is nothing to share, and as long as one wave of threads does, the pixel's thread with
 // the filters from global memory is there first: 8 x 8, one channel, 7 x 7 taps 18.4 us against 21.8, 3 x 3 5.4 against 6.1. Two channels and 3 x 3: 6.8
 // against 6.1; 64 images of 28 x 28, 1 -> 16 channels, 3 x 3: 17.4 against 13.0.
+// EXACT: sums in 64 bits, in one chain, for layers of few products an output (launch_few_products); fewer channels a thread where threads are few. With the divisions by the strides as multiplications it takes 0.81 to 0.98
+// of the time that sums in 32 bits took with divisions, by the number of blocks; those take 0.93 of it on 900 layers of more products. Four chains in 64 bits: 1.15 of one's time.
 constexpr int kPhaseThreads = 128;
 constexpr int kPhaseFilterBytes = 32 * 1024;
-template <int OC>
+template <int OC, bool EXACT>
 __global__ void __launch_bounds__(kPhaseThreads)
-conv_transpose_phase_kernel(sofie_conv_transpose2d_desc d, int oH, int oW, uint32_t columns, uint32_t positions, int CK, const float *__restrict__ X,
+conv_transpose_phase_kernel(sofie_conv_transpose2d_desc d, int oW, FastDiv columns, FastDiv strides_h, FastDiv strides_w, FastDiv rows, uint32_t positions, int CK, const float *__restrict__ X,
                             const float *__restrict__ Wt, const float *__restrict__ bias, float *__restrict__ Y)
 {
-   extern __shared__ __align__(16) float filters[];
-   const size_t in_hw = (size_t)d.H * d.W, out_hw = (size_t)oH * oW;
+   using T = std::conditional_t<EXACT, double, float>;
+   constexpr int CHAINS = EXACT ? 1 : 4;
+   extern __shared__ __align__(16) unsigned char phase_smem[];
+   T *filters = reinterpret_cast<T *>(phase_smem);
+   const size_t in_hw = (size_t)d.H * d.W, out_hw = (size_t)rows.d * oW;
    const int taps = d.kH * d.kW, oc0 = blockIdx.y * OC;
    // (n, oh, residue, column) of the thread, in 32 bits (more positions than that are the other kernel's)
-   uint32_t t = blockIdx.x * (uint32_t)kPhaseThreads + threadIdx.x;
+   uint32_t t = blockIdx.x * (uint32_t)kPhaseThreads + threadIdx.x, column, phase, row;
    bool active = t < positions;
-   const int column = (int)(t % columns);
-   t /= columns;
-   const int ow = column * d.stride_w + (int)(t % d.stride_w);
-   t /= d.stride_w;
-   const int oh = (int)(t % oH);
-   const size_t n = t / oH;
+   const size_t n = rows.divmod(strides_w.divmod(columns.divmod(t, column), phase), row);
+   const int ow = (int)column * d.stride_w + (int)phase, oh = (int)row;
    active = active && ow < oW;
-   float acc[4][OC];
+   T acc[CHAINS][OC];
 #pragma unroll
-   for (int k = 0; k < 4; k++)
+   for (int k = 0; k < CHAINS; k++)
 #pragma unroll
-      for (int j = 0; j < OC; j++) acc[k][j] = 0.f;
+      for (int j = 0; j < OC; j++) acc[k][j] = 0;
    const float *x = X + (active ? n : 0) * d.C * in_hw;
    for (int c0 = 0; c0 < d.C; c0 += CK) {
       const int ck = min(CK, d.C - c0);
@@ -116,24 +120,34 @@ conv_transpose_phase_kernel(sofie_conv_transpose2d_desc d, int oH, int oW, uint3
       if (!active) continue;
       for (int r = 0; r < d.kH; r++) {
          const int th = oh + d.pad_h - r * d.dil_h;
-         if (th < 0 || th % d.stride_h) continue;
-         const int ih = th / d.stride_h;
-         if (ih >= d.H) continue;
+         if (th < 0) continue;
+         uint32_t rest;
+         const int ih = (int)strides_h.divmod((uint32_t)th, rest);
+         if (rest || ih >= d.H) continue;
          for (int s = 0; s < d.kW; s++) {
             const int tw = ow + d.pad_w - s * d.dil_w;
-            if (tw < 0 || tw % d.stride_w) continue;
-            const int iw = tw / d.stride_w;
-            if (iw >= d.W) continue;
+            if (tw < 0) continue;
+            const int iw = (int)strides_w.divmod((uint32_t)tw, rest);
+            if (rest || iw >= d.W) continue;
             const float *xp = x + (size_t)c0 * in_hw + (size_t)ih * d.W + iw;
-            const float *wp = filters + (r * d.kW + s) * OC;
-            auto add = [&](float v, const float *w, float(&a)[OC]) {
+            const T *wp = filters + (r * d.kW + s) * OC;
+            auto add = [&](float v, const T *w, T(&a)[OC]) {
+               if constexpr (EXACT) {
 #pragma unroll
-               for (int j = 0; j < OC; j += 4) {
-                  const float4 f = *reinterpret_cast<const float4 *>(w + j);
-                  a[j] = fmaf(v, f.x, a[j]);
-                  a[j + 1] = fmaf(v, f.y, a[j + 1]);
-                  a[j + 2] = fmaf(v, f.z, a[j + 2]);
-                  a[j + 3] = fmaf(v, f.w, a[j + 3]);
+                  for (int j = 0; j < OC; j += 2) {
+                     const double2 f = *reinterpret_cast<const double2 *>(w + j);
+                     a[j] = fma((double)v, f.x, a[j]);
+                     a[j + 1] = fma((double)v, f.y, a[j + 1]);
+                  }
+               } else {
+#pragma unroll
+                  for (int j = 0; j < OC; j += 4) {
+                     const float4 f = *reinterpret_cast<const float4 *>(w + j);
+                     a[j] = fmaf(v, f.x, a[j]);
+                     a[j + 1] = fmaf(v, f.y, a[j + 1]);
+                     a[j + 2] = fmaf(v, f.z, a[j + 2]);
+                     a[j + 3] = fmaf(v, f.w, a[j + 3]);
+                  }
                }
             };
             int c = 0;
@@ -142,14 +156,14 @@ conv_transpose_phase_kernel(sofie_conv_transpose2d_desc d, int oH, int oW, uint3
 #pragma unroll
                for (int k = 0; k < 16; k++) v[k] = __ldg(xp + (size_t)(c + k) * in_hw);
 #pragma unroll
-               for (int k = 0; k < 16; k++) add(v[k], wp + (c + k) * taps * OC, acc[k & 3]);
+               for (int k = 0; k < 16; k++) add(v[k], wp + (c + k) * taps * OC, acc[k % CHAINS]);
             }
             for (; c + 4 <= ck; c += 4) {
                float v[4];
 #pragma unroll
                for (int k = 0; k < 4; k++) v[k] = __ldg(xp + (size_t)(c + k) * in_hw);
 #pragma unroll
-               for (int k = 0; k < 4; k++) add(v[k], wp + (c + k) * taps * OC, acc[k]);
+               for (int k = 0; k < 4; k++) add(v[k], wp + (c + k) * taps * OC, acc[k % CHAINS]);
             }
             for (; c < ck; c++) add(__ldg(xp + (size_t)c * in_hw), wp + c * taps * OC, acc[0]);
          }
@@ -159,31 +173,50 @@ conv_transpose_phase_kernel(sofie_conv_transpose2d_desc d, int oH, int oW, uint3
 #pragma unroll
    for (int j = 0; j < OC; j++) {
       if (oc0 + j < d.Cout) {
-         float v = ((acc[0][j] + acc[1][j]) + (acc[2][j] + acc[3][j])) + (bias ? __ldg(bias + oc0 + j) : 0.f);
+         float v;
+         if constexpr (EXACT) v = (float)(acc[0][j] + (bias ? (double)__ldg(bias + oc0 + j) : 0.0));
+         else v = ((acc[0][j] + acc[1][j]) + (acc[2][j] + acc[3][j])) + (bias ? __ldg(bias + oc0 + j) : 0.f);
          if (d.relu) v = relu_ref(v);
          Y[(n * d.Cout + oc0 + j) * out_hw + (size_t)oh * oW + ow] = v;
       }
    }
 }
 
-template <int OC>
+template <int OC, bool EXACT>
 int launch_phase(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, int oW, const float *X, const float *W, const float *bias, float *Y)
 {
    const int columns = ceil_div(oW, d.stride_w);
-   const size_t positions = (size_t)d.N * oH * d.stride_w * columns, channel = (size_t)d.kH * d.kW * OC * sizeof(float);
+   const size_t positions = (size_t)d.N * oH * d.stride_w * columns, channel = (size_t)d.kH * d.kW * OC * (EXACT ? sizeof(double) : sizeof(float));
    const int fit = (int)(kPhaseFilterBytes / channel), CK = fit >= d.C ? d.C : fit / 4 * 4;
    const size_t blocks = ceil_div<size_t>(positions, kPhaseThreads);
    if (CK < 1 || positions > 0x7FFFFFFFu || ceil_div(d.Cout, OC) > 65535) return -1;
-   conv_transpose_phase_kernel<OC><<<dim3((unsigned)blocks, ceil_div(d.Cout, OC)), kPhaseThreads, CK * channel, s>>>(d, oH, oW, (uint32_t)columns, (uint32_t)positions, CK, X, W, bias, Y);
+   conv_transpose_phase_kernel<OC, EXACT><<<dim3((unsigned)blocks, ceil_div(d.Cout, OC)), kPhaseThreads, CK * channel, s>>>(d, oW, FastDiv(columns), FastDiv(d.stride_h), FastDiv(d.stride_w), FastDiv(oH), (uint32_t)positions, CK, X,
+                                                                                                                                           W, bias, Y);
    SOFIE_LAUNCH_CHECK("conv_transpose_phase_kernel");
    set_last_engine(SOFIE_ENGINE_SIMT);
    return SOFIE_CUDA_OK;
 }
+// Channels of a thread where sums are in 64 bits: as many as leave two blocks an SM, down to two
+int phase_channels(const sofie_conv_transpose2d_desc &d, int oH, int oW)
+{
+   const size_t blocks = ceil_div<size_t>((size_t)d.N * oH * d.stride_w * ceil_div(oW, d.stride_w), kPhaseThreads);
+   for (int OC = d.Cout <= 4 ? 4 : 8; OC > 2; OC /= 2)
+      if (blocks * ceil_div(d.Cout, OC) >= 2 * kNumSMs) return OC;
+   return d.Cout <= 4 ? 2 : 4;
+}
+int launch_phase_exact(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, int oW, const float *X, const float *W, const float *bias, float *Y)
+{
+   const int OC = phase_channels(d, oH, oW);
+   if (OC == 2) return launch_phase<2, true>(s, d, oH, oW, X, W, bias, Y);
+   if (OC == 4) return launch_phase<4, true>(s, d, oH, oW, X, W, bias, Y);
+   return launch_phase<8, true>(s, d, oH, oW, X, W, bias, Y);
+}
+
 int launch_direct(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, int oW, const float *X, const float *W, const float *bias, float *Y)
 {
    const size_t total = (size_t)d.N * ((d.Cout + kOcPerThread - 1) / kOcPerThread) * oH * oW;
    const bool alone = d.stride_h == 1 && d.stride_w == 1 && d.C * min(d.kH * d.kW, 2) <= 2 && total <= 1u << 17;
-   const int rc = alone ? -1 : d.Cout <= 4 ? launch_phase<4>(s, d, oH, oW, X, W, bias, Y) : launch_phase<8>(s, d, oH, oW, X, W, bias, Y);
+   const int rc = alone ? -1 : d.Cout <= 4 ? launch_phase<4, false>(s, d, oH, oW, X, W, bias, Y) : launch_phase<8, false>(s, d, oH, oW, X, W, bias, Y);
    if (rc >= 0) return rc;
    // also: filters of which not four channels fit beside one another, 2^31 outputs or more
    conv_transpose2d_f32_kernel<<<grid_for(total), kThreads, 0, s>>>(d, oH, oW, total, X, W, bias, Y);
@@ -197,7 +230,7 @@ int launch_direct(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, 
 // direct form above waits for one channel's filters and inputs after the other's. Here a block owns a band of output rows of one image and OC output channels: the band's
 // inputs and the filters are converted to double once, on their way into shared memory, and a thread sums four channels of PX outputs in double, so that the result is the exact
 // sum rounded once (error against float64 2.5e-8; 3.5e-8 to 1.3e-7 the product form, 4.3e-8 to 5.5e-8 the direct one). A warp's outputs share their phase (row and column
-// modulo the strides) and so their taps; OC / 4 neighbouring lanes share an output's inputs.
+// modulo the strides) and so their taps; OC / 4 neighbouring lanes share an output's inputs. Or the direct form runs, its sums in 64 bits too (launch_few_products).
 // What bounds it: round trips at sixteen warps an SM, to L2 while a block stages and to shared memory while it sums; no pipe is busy, at 64 images or at 1024 (issue slots 31 and 29 %, fp64
 // 15 and 16 %, shared memory 17 and 23 %). 32 -> 16 channels, 2 x 2 / 2 on 12 x 12, 1 / 64 / 1024 images: 13.6 -> 5.3, 16.3 -> 10.6, 103 -> 85 us against
 // the product form; 16 -> 3, 3 x 3 / 2 on 24 x 24: 12.9 -> 6.4, 21.5 -> 13.9, 184 -> 117. Its channels in registers two or four at a time: the same or slower (96, 127 at 1024).
@@ -336,47 +369,93 @@ conv_transpose_sum_kernel(SumGeom g, FastDiv bands, FastDiv columns, FastDiv tap
    }
 }
 
-// -1 where the filters and one row of outputs' inputs do not fit in shared memory
-template <int OC, int PX>
-int launch_sum(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, int oW, int per, const float *X, const float *W, const float *bias, float *Y)
+// How the kernel would cut a layer up; fits: the filters and one row of outputs' inputs do in shared memory
+struct SumPlan {
+   bool fits = false;
+   int OC, PX, per, columns, halo, bands, groups;
+   size_t filters, row; // bytes: the filters, an input row of all channels
+};
+
+SumPlan plan_sum(const sofie_conv_transpose2d_desc &d, int oH, int oW)
 {
-   const int groups = ceil_div(d.Cout, OC), steps = ceil_div(oH, d.stride_h), columns = ceil_div(oW, d.stride_w), halo = ceil_div((d.kH - 1) * d.dil_h, d.stride_h) + 1;
-   const size_t filters = (size_t)d.C * d.kH * d.kW * OC * sizeof(double), row = (size_t)d.C * d.W * sizeof(double);
-   if (groups > 65535 || filters + row * (1 + halo) > kSumBytes || d.kH + d.kW > 1024 || (long long)d.kH * d.dil_h > 1 << 20 || (long long)d.pad_h + oH > 1 << 28 || (long long)d.pad_w + oW > 1 << 28) return -1;
-   const int fit = (int)((kSumBytes - filters) / row) - halo;
-   if (per > fit) per = fit;
-   SumGeom g = {d, oH, oW, ceil_div(steps, per), per, per + halo};
-   if ((long long)d.N * g.bands >= 1ll << 31) return -1;
-   const size_t smem = filters + row * g.lines + (d.kH + d.kW) * sizeof(int2);
+   SumPlan p;
+   p.OC = d.Cout <= 4 ? 4 : d.Cout <= 8 ? 8 : 16;
+   p.groups = ceil_div(d.Cout, p.OC), p.columns = ceil_div(oW, d.stride_w), p.halo = ceil_div((d.kH - 1) * d.dil_h, d.stride_h) + 1;
+   p.filters = (size_t)d.C * d.kH * d.kW * p.OC * sizeof(double), p.row = (size_t)d.C * d.W * sizeof(double);
+   if (p.groups > 65535 || p.filters + p.row * (1 + p.halo) > kSumBytes || d.kH + d.kW > 1024 || (long long)d.kH * d.dil_h > 1 << 20 || (long long)d.pad_h + oH > 1 << 28 || (long long)d.pad_w + oW > 1 << 28) return p;
+   // Bands for two blocks an SM, as far as the rows go: what a block costs beside its sums is its start (64 images, 32 -> 16 channels: 4 bands an image 11.5 us, 6 15.1, 12 19.3, 2 16.6).
+   // Of the outputs a thread can take the most that leave every warp some.
+   const int steps = ceil_div(oH, d.stride_h);
+   const long long wanted = 2 * kNumSMs / ((long long)d.N * p.groups);
+   p.per = ceil_div(steps, (int)(wanted < 1 ? 1 : (wanted > steps ? steps : wanted)));
+   auto units = [&](int q) { return (long long)d.stride_h * d.stride_w * ceil_div((long long)p.per * p.columns, 128ll / p.OC * q); };
+   p.PX = units(4) >= kSumThreads / 32 ? 4 : units(2) >= kSumThreads / 32 ? 2 : 1;
+   const int fit = (int)((kSumBytes - p.filters) / p.row) - p.halo;
+   if (p.per > fit) p.per = fit;
+   p.bands = ceil_div(steps, p.per);
+   p.fits = (long long)d.N * p.bands < 1ll << 31 && (long long)p.per * p.columns < 1 << 30;
+   return p;
+}
+
+template <int OC, int PX>
+int launch_sum(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, int oW, const SumPlan &p, const float *X, const float *W, const float *bias, float *Y)
+{
+   const SumGeom g = {d, oH, oW, p.bands, p.per, p.per + p.halo};
+   const size_t smem = p.filters + p.row * g.lines + (d.kH + d.kW) * sizeof(int2);
    auto kern = conv_transpose_sum_kernel<OC, PX>;
    SOFIE_CUDA_TRY(allow_smem(reinterpret_cast<const void *>(kern), (int)smem));
-   SOFIE_CUDA_TRY(launch_dependent(kern, dim3((unsigned)(d.N * (long long)g.bands), groups), dim3(kSumThreads), smem, s, g, FastDiv(g.bands), FastDiv(columns), FastDiv(d.kH * d.kW), FastDiv(ceil_div(per * columns, 128 / OC * PX)), FastDiv(d.stride_w),
-                                   g.lines * d.W, X, W, bias, Y));
+   SOFIE_CUDA_TRY(launch_dependent(kern, dim3((unsigned)(d.N * (long long)g.bands), p.groups), dim3(kSumThreads), smem, s, g, FastDiv(g.bands), FastDiv(p.columns), FastDiv(d.kH * d.kW), FastDiv(ceil_div(p.per * p.columns, 128 / OC * PX)),
+                                   FastDiv(d.stride_w), g.lines * d.W, X, W, bias, Y));
    SOFIE_LAUNCH_CHECK("conv_transpose_sum_kernel");
    set_last_engine(SOFIE_ENGINE_SIMT);
    return SOFIE_CUDA_OK;
 }
 
-// -1 where an output has more products, or they do not fit
-int launch_few_products(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, int oW, const float *X, const float *W, const float *bias, float *Y)
+// Layers of up to 48 products an output, counted without borders: sums in 64 bits, by the kernel above or by the direct form, whichever takes less time by an estimate. -1 where an output has more, where
+// neither can, and (product_form) where the product form is the faster one.
+int launch_few_products(cudaStream_t s, const sofie_conv_transpose2d_desc &d, int oH, int oW, bool product_form, const float *X, const float *W, const float *bias, float *Y)
 {
-   // Up to 48 products an output, counted without borders. 64 -> 32 channels, 2 x 2 / 2 (64 products) on 256 images of 8 x 8: 44 us here, 30 in the product form; 32 -> 16, 4 x 4 / 2
-   // (128) on 64 of 16 x 16: 29 and 31; 16 -> 16, 3 x 3 / 1 (144) on 64 of 64 x 64: 101 here, 84 in the direct form.
+   // 64 -> 32 channels, 2 x 2 / 2 (64 products) on 256 images of 8 x 8: 44 us here, 30 in the product form; 32 -> 16, 4 x 4 / 2 (128) on 64 of 16 x 16: 29 and 31; 16 -> 16, 3 x 3 / 1 (144) on
+   // 64 of 64 x 64: 101 here, 84 in the direct form.
    if ((long long)d.C * d.kH * d.kW > 48ll * d.stride_h * d.stride_w || forced_engine() == SOFIE_ENGINE_TCGEN05) return -1;
-   // Bands for two blocks an SM, as far as the rows go: what a block costs beside its sums is its start (64 images, 32 -> 16 channels: 4 bands an image 11.5 us, 6 15.1, 12 19.3, 2 16.6).
-   // Of the outputs a thread can take the most that leave every warp some.
-   const int OC = d.Cout <= 4 ? 4 : d.Cout <= 8 ? 8 : 16, steps = ceil_div(oH, d.stride_h), columns = ceil_div(oW, d.stride_w);
-   const long long wanted = 2 * kNumSMs / ((long long)d.N * ceil_div(d.Cout, OC));
-   const int per = ceil_div(steps, (int)(wanted < 1 ? 1 : (wanted > steps ? steps : wanted)));
-   auto units = [&](int q) { return (long long)d.stride_h * d.stride_w * ceil_div((long long)per * columns, 128ll / OC * q); };
-   const int px = units(4) >= kSumThreads / 32 ? 4 : units(2) >= kSumThreads / 32 ? 2 : 1;
-#define SOFIE_SUM(C, P) return launch_sum<C, P>(s, d, oH, oW, per, X, W, bias, Y)
+   // Times in us, fitted to 8900 layers of 1 to 4096 images (to 13, 20 and 19 %): blocks beyond what is resident at a time count, the first round's round trips do not shrink. Many small images, few products and large
+   // strides are the direct form's (1 x 1 images, 4 x 4 / 2, 2 -> 49 channels, 3899 of them 8.5 us against 167), longer sums this kernel's. Of 2500 other layers the choice takes 0.77 of the time of the direct form with sums in
+   // 32 bits in the mean, 2.7 % of them above 1.2 (with this kernel for all of them 0.88, 20 % above 1.2, up to 28 times the time); against the product form 0.70, one of 172 above 1.2.
+   const int taps = d.kH * d.kW;
+   const double outputs = 1e-4 * d.N * d.Cout * oH * oW, products = std::min((double)taps / (d.stride_h * d.stride_w), (double)d.H * d.W * taps / ((double)oH * oW)) * d.C; // of an output
+   const SumPlan p = plan_sum(d, oH, oW);
+   double sum = 1e30;
+   if (p.fits) {
+      const double blocks = (double)d.N * p.bands * p.groups, rounds = std::max(1.0, blocks / (2 * kNumSMs));
+      const double units = std::max(1.0, (double)d.stride_h * d.stride_w * ceil_div((long long)p.per * p.columns, 128ll / p.OC * p.PX) / (kSumThreads / 32)); // a warp's
+      const double walk = ceil_div(d.C, 4) * std::max(ceil_div(taps * std::min(d.Cout, p.OC), 32), ceil_div(std::min(p.per + p.halo, d.H) * d.W, 32)) / 8.0;
+      sum = 0.98 + rounds * (1.88 + 1.2 * walk + units * (0.042 * taps + 0.0196 * products * (p.PX + 1) + 0.097 * p.PX)) + 0.029 * outputs;
+   }
+   double phase;
+   {
+      const int OC = phase_channels(d, oH, oW);
+      const double blocks = (double)ceil_div<size_t>((size_t)d.N * oH * d.stride_w * p.columns, kPhaseThreads) * ceil_div(d.Cout, OC), share = blocks / kNumSMs;
+      const size_t channel = (size_t)taps * OC * sizeof(double);
+      const int fit = (int)(kPhaseFilterBytes / channel), CK = fit >= d.C ? d.C : fit / 4 * 4;
+      const double rounds = std::max(1.0, share / std::min<size_t>(12, 227 * 1024 / (CK * channel + 1024)));
+      const double stage = (double)d.C * taps * OC / kPhaseThreads, tests = d.kH + (double)d.kH / d.stride_h * d.kW;
+      const double trips = (double)ceil_div(d.kH, d.stride_h) * ceil_div(d.kW, d.stride_w) * (d.C / 16 + d.C % 16 / 4 + d.C % 4);
+      phase = 2.82 + rounds * (0.868 * stage + 0.103 * tests + 0.069 * trips) + share * (0.107 + 0.0123 * stage + 0.0185 * tests + 0.0032 * products * OC) + 0.0115 * outputs;
+      if (CK < 1) phase = 1e30;
+   }
+   const bool here = sum < phase;
+   if (product_form) {
+      const double pixels = 1e-5 * d.N * d.H * d.W, columns = (double)taps * d.Cout;
+      if (std::min(sum, phase) >= 0.85 * (10.2 + pixels * (0.413 * d.C + 0.721 * columns + 0.00407 * columns * d.C) + 0.0313 * outputs)) return -1;
+   }
+   if (!here) return launch_phase_exact(s, d, oH, oW, X, W, bias, Y);
+#define SOFIE_SUM(C, P) return launch_sum<C, P>(s, d, oH, oW, p, X, W, bias, Y)
 #define SOFIE_SUM_OC(P) \
-   if (OC == 4) SOFIE_SUM(4, P); \
-   if (OC == 8) SOFIE_SUM(8, P); \
+   if (p.OC == 4) SOFIE_SUM(4, P); \
+   if (p.OC == 8) SOFIE_SUM(8, P); \
    SOFIE_SUM(16, P)
-   if (px == 1) { SOFIE_SUM_OC(1); }
-   if (px == 2) { SOFIE_SUM_OC(2); }
+   if (p.PX == 1) { SOFIE_SUM_OC(1); }
+   if (p.PX == 2) { SOFIE_SUM_OC(2); }
    SOFIE_SUM_OC(4);
 #undef SOFIE_SUM_OC
 #undef SOFIE_SUM
@@ -490,7 +569,7 @@ extern "C" int sofie_cuda_conv_transpose2d_f32_gemm(void *stream, const sofie_co
    SOFIE_REQUIRE(scratch_bytes >= need, "scratch of %zu bytes, %zu needed", scratch_bytes, need);
    SOFIE_REQUIRE((reinterpret_cast<uintptr_t>(scratch) & 255) == 0, "scratch must be 256-byte aligned");
    cudaStream_t s = as_stream(stream);
-   const int few = launch_few_products(s, *d, (int)oH, (int)oW, X, W, bias, Y);
+   const int few = launch_few_products(s, *d, (int)oH, (int)oW, true, X, W, bias, Y);
    if (few >= 0) return few;
    const size_t pixels = (size_t)d->N * d->H * d->W;
    const int taps = d->kH * d->kW;
@@ -522,7 +601,7 @@ extern "C" int sofie_cuda_conv_transpose2d_f32(void *stream, const sofie_conv_tr
    if (rc) return rc;
    if (d->N == 0) return SOFIE_CUDA_OK;
    SOFIE_REQUIRE(X && W && Y, "NULL tensor");
-   const int few = launch_few_products(as_stream(stream), *d, (int)oH, (int)oW, X, W, bias, Y);
+   const int few = launch_few_products(as_stream(stream), *d, (int)oH, (int)oW, false, X, W, bias, Y);
    if (few >= 0) return few;
    return launch_direct(as_stream(stream), *d, (int)oH, (int)oW, X, W, bias, Y);
 }

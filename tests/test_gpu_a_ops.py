@@ -493,6 +493,28 @@ def test_conv_transpose2d_f32_few_products(N, C, H, W, Cout, k, stride, pad, dil
         assert (np.abs(y - ref)[hit == 0] <= (2.0 ** -24 * 1.01 * np.abs(ref) + 1e-13 * size)[hit == 0]).all()
 
 
+# ... and those the direct form takes, with sums in 64 bits: two, four and eight channels a thread and a last group that is not full, filters in one piece and in several, inputs of one pixel,
+# strides beyond the filter, a position more than whole blocks
+@pytest.mark.parametrize("N,C,H,W,Cout,k,stride,pad,dil,out_pad", [(700, 2, 1, 1, 49, (4, 4), (2, 2), (1, 1), (1, 1), (0, 0)), (3, 75, 17, 51, 2, (2, 1), (2, 3), (1, 0), (2, 2), (0, 0)),
+                                                                   (11, 60, 40, 40, 20, (1, 1), (3, 1), (0, 0), (1, 2), (0, 0)), (129, 1, 3, 3, 1, (2, 2), (1, 1), (0, 0), (1, 1), (0, 0)),
+                                                                   (5, 256, 9, 30, 9, (1, 3), (4, 4), (0, 1), (1, 1), (0, 1)), (613, 20, 2, 2, 43, (3, 3), (4, 4), (1, 0), (1, 1), (0, 0))])
+def test_conv_transpose2d_f32_few_products_direct(N, C, H, W, Cout, k, stride, pad, dil, out_pad):
+    # (the other entry point's product form, with its own rounding, takes some of them)
+    rng = np.random.default_rng(N + C + H + W + Cout)
+    X, Wt, b = (rng.standard_normal(s).astype(np.float32) for s in ((N, C, H, W), (C, Cout, *k), (Cout,)))
+    Wt[0, 0, 0, 0] = np.inf   # counts only where the tap lies on the input
+    args = dict(stride=stride, padding=pad, dilation=dil, output_padding=out_pad)
+    finite = torch.from_numpy(np.where(np.isinf(Wt), 0, Wt)).double()
+    ref = torch.nn.functional.conv_transpose2d(torch.from_numpy(X).double(), finite, torch.from_numpy(b).double(), **args).numpy()
+    size = torch.nn.functional.conv_transpose2d(torch.from_numpy(abs(X)).double(), finite.abs(), torch.from_numpy(abs(b)).double(), **args).numpy()
+    one = np.zeros_like(Wt)
+    one[0, 0, 0, 0] = 1
+    hit = o.conv_transpose2d_f32(X, one, None, pad=pad, stride=stride, dil=dil, out_pad=out_pad)
+    y = ops.conv_transpose2d_f32(dev(X), dev(Wt), dev(b), pad=pad, stride=stride, dil=dil, out_pad=out_pad).cpu().numpy()
+    assert np.array_equal(np.isinf(y), hit != 0) and np.array_equal(np.sign(y[hit != 0]), np.sign(hit[hit != 0]))
+    assert (np.abs(y - ref)[hit == 0] <= (2.0 ** -24 * 1.01 * np.abs(ref) + 1e-13 * size)[hit == 0]).all()
+
+
 @pytest.mark.parametrize("case", [
     # N, C, H, W, Cout, k, pad, stride, dil, out_pad, bias, relu
     (4, 32, 16, 16, 16, (4, 4), (1, 1), (2, 2), (1, 1), (0, 0), True, True),       # the usual 2x upsampling layer of a decoder
