@@ -365,7 +365,9 @@ int launch_conv2d_f32_direct3x3(cudaStream_t s, const ConvGeom &g, const float *
    const long long groups = ceil_div(g.Cout, kDcOut), tiles = (long long)ceil_div(g.oH, kDcRows) * ceil_div(g.oW, wide ? 32 : 16), area = kDcRows * (wide ? 32 : 16);
    const long long outputs = (long long)g.oH * g.oW;
    const double positions = 1e-6 * g.N * outputs, units = (double)g.N * tiles * groups * (wide ? 2 : 1);
-   const double general = 1.9 + 1.69 * g.C + positions * (25 * groups * g.C + 2.6 * g.Cout);
+   // images of one row: a third of the taps lie on them (447 x 84 -> 39 at 1 x 7 90 us, 144 with shared channels, which were estimated faster without this factor)
+   const double inside = g.oH > 1 ? 1.0 : (g.oW > 1 ? 0.65 : 0.5);
+   const double general = 1.9 + inside * (1.69 * g.C + positions * 25 * groups * g.C) + positions * 2.6 * g.Cout;
    const double sparse = 2.5 + chunks * (vec ? 3.5 : 4.7) + 1e-3 * units * (chunks * (vec ? 5.1 : 8.1) + 4.8);
    const bool filled = 5 * outputs >= 3 * tiles * area;
    const bool large = 4 * outputs >= tiles * area && (filled || 1.05 * general > sparse);
