@@ -131,8 +131,9 @@ public:
       if (!fNB.empty()) model.UseOnDevice(fNB);
       // With 16 or more input channels the operator is lowered as the reference lowers it -- a filter GEMM, here one for
       // all images and on the tensor cores, followed by the gather form of col2im -- and needs a slice of the arena for
-      // the products (alive during this operator only). It is there for layers of few products too, which take one kernel and
-      // no slice unless the tensor cores are asked for: that choice is made when the Session runs. Not with a run-time batch: part of the slice (the re-ordered
+      // the products (alive during this operator only). It is there for layers of few products too, which mostly take one
+      // kernel and no slice: that choice is made when the Session runs, and falls to the product form where the tensor cores
+      // are asked for. Not with a run-time batch: part of the slice (the re-ordered
       // filters) does not scale with the batch.
       const sofie_conv_transpose2d_desc d = Desc();
       fProductsBytes = model.RunTimeBatch() ? 0 : sofie_conv_transpose2d_gemm_scratch_bytes(&d);
