@@ -341,6 +341,7 @@ bool gemm_f32_skinny_ok(const sofie_gemm_f32_desc &d)
    // from 64 terms on: below, the adding up of the partial sums is most of the error (9750 x 1 x 35 5.5e-8 from float64 against 4.0e-8). Up to 2^20: a sum is of K / 4096 chunks' sums then,
    // and no more have been compared with the other kernels' (at 262144 terms 0.5 to 0.6 of their error)
    if ((d.M > 8 && d.N > 8) || d.K < 64 || d.K > 1 << 20) return false;
+   // Of five to eight columns, 12000 rows and more and up to 300 terms the kernel of two TF32 parts took less time (16384 x 8 x 92 5.9 us, 8.6 here; 16384 x 5 x 272 10.3 and 11.9) with 1.2 to 1.7 times the error: they stay.
    // K is shared by eight blocks at most, which leaves most SMs idle where the long side is not long: split-K, whose slabs are 64, keeps what it is faster at. 8 x 8 x 65536 15.6 us there, 46 here, 1 x 4 x 16385
    // 6.5 and 12, 100 x 8 x 32768 20.5 and 25.7, but 250 x 8 x 32768 32.6 and 27.8, 100 x 8 x 8192 12.1 and 8.8; rows read value by value turn earlier: 8 x 8 x 8193 8.6 and 10.9, 32 x 8 x 3001
    // 5.3 and 5.7, 250 x 8 x 16385 (B stored [N,K]) 16.2 and 16.7.
